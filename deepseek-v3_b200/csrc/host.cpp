@@ -1,0 +1,477 @@
+// Native host path of the Python operators: argument checks, output allocation and the call into libdsv3_b200.so in
+// one CPython call each.
+//
+// Why it exists: a decode-sized operator runs for 2-8 us on a B200, while the same call through ctypes (device guard,
+// stream lookup, three or four framework calls for the outputs, pointer conversions) kept the host busy for 14-20 us,
+// so every small call was bound by its own launch.  Here a call costs the two allocations and the launch itself.
+// The extension adds nothing to the C ABI: it fills in the same arguments a C host would.
+//
+// Threads and streams: every entry point is called with the GIL held and releases it only around the library call;
+// the split-K workspaces are keyed on (device, stream), and calls that share one are ordered by their stream.
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include <ATen/core/Tensor.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/DefaultDtype.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <array>
+#include <exception>
+#include <vector>
+
+#include "dsv3_b200.h"
+
+namespace {
+
+PyObject* g_error_class = nullptr;   // dsv3_b200.Dsv3Error
+
+PyObject* g_oom_class = nullptr;     // torch.OutOfMemoryError
+
+// A Python exception is already set.
+struct PythonError {};
+
+[[noreturn]] void raise(PyObject* type, const char* msg) {
+    PyErr_SetString(type, msg);
+    throw PythonError{};
+}
+
+void require(bool cond, const char* assertion) {
+    if (!cond) raise(PyExc_AssertionError, assertion);
+}
+
+void check(int status) {
+    if (status == DSV3_OK) return;
+    PyObject* msg = PyUnicode_FromFormat("%s (%d): %s", dsv3_strerror(status), status, dsv3_last_error());
+    if (msg) {
+        PyObject* exc = PyObject_CallFunction(g_error_class, "iO", status, msg);
+        Py_DECREF(msg);
+        if (exc) {
+            PyErr_SetObject(g_error_class, exc);
+            Py_DECREF(exc);
+        }
+    }
+    throw PythonError{};
+}
+
+const at::Tensor& tensor_arg(PyObject* o) {
+    if (!THPVariable_Check(o)) raise(PyExc_TypeError, "expected a torch.Tensor");
+    return THPVariable_Unpack(o);
+}
+
+int scale_fmt_arg(PyObject* o) {
+    return (PyUnicode_Check(o) && PyUnicode_CompareWithASCIIString(o, "ue8m0") == 0) ? DSV3_SCALE_FMT_UE8M0
+                                                                                     : DSV3_SCALE_FMT_FP32;
+}
+
+// All tensors of a call live on one CUDA device; returns it.
+template <typename... Ts>
+c10::Device require_cuda(const at::Tensor& first, const Ts&... rest) {
+    const c10::Device dev = first.device();
+    const at::Tensor* all[] = {&first, &rest...};
+    for (const at::Tensor* t : all) {
+        if (!t->is_cuda()) {
+            PyErr_Format(PyExc_RuntimeError, "dsv3_b200 runs on CUDA tensors only (there is no CPU path); got a %s tensor",
+                         c10::DeviceTypeName(t->device().type(), true).c_str());
+            throw PythonError{};
+        }
+        if (t->device() != dev) raise(PyExc_RuntimeError, "all tensors of one call must be on the same device");
+    }
+    return dev;
+}
+
+void require_bf16_default() {
+    const auto dt = c10::get_default_dtype_as_scalartype();
+    if (dt != at::kBFloat16) {
+        PyErr_Format(PyExc_NotImplementedError,
+                     "the CUDA path writes bfloat16 only; call torch.set_default_dtype(torch.bfloat16) as every entry point of "
+                     "the reference does (default dtype is %s)", c10::toString(dt));
+        throw PythonError{};
+    }
+}
+
+at::Tensor new_cuda(at::IntArrayRef sizes, at::ScalarType dt, c10::Device dev) {
+    return at::detail::empty_cuda(sizes, dt, dev, std::nullopt);
+}
+
+// `like`'s sizes with the last one replaced.
+at::Tensor new_cuda_last(const at::Tensor& like, int64_t last, at::ScalarType dt) {
+    c10::SmallVector<int64_t, 6> sizes(like.sizes().begin(), like.sizes().end());
+    if (sizes.empty()) sizes.push_back(last); else sizes.back() = last;
+    return new_cuda(sizes, dt, like.device());
+}
+
+int64_t last_dim(const at::Tensor& t) {
+    if (t.dim() == 0) raise(PyExc_IndexError, "Dimension specified as -1 but tensor has no dimensions");
+    return t.sizes().back();
+}
+
+PyObject* wrap(at::Tensor t) { return THPVariable_Wrap(std::move(t)); }
+
+PyObject* wrap_pair(at::Tensor a, at::Tensor b) {
+    PyObject* first = wrap(std::move(a));
+    PyObject* second = first ? wrap(std::move(b)) : nullptr;
+    PyObject* tup = second ? PyTuple_New(2) : nullptr;
+    if (!tup) {
+        Py_XDECREF(first);
+        Py_XDECREF(second);
+        return nullptr;
+    }
+    PyTuple_SET_ITEM(tup, 0, first);
+    PyTuple_SET_ITEM(tup, 1, second);
+    return tup;
+}
+
+// Runs a library call with the tensors' device current and without the GIL; raises what it reports.
+template <typename F>
+void call_library(c10::Device dev, F&& f) {
+    c10::cuda::OptionalCUDAGuard guard;
+    if (dev.index() != c10::cuda::current_device()) guard.set_device(dev);
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    int status;
+    {
+        PyThreadState* save = PyEval_SaveThread();
+        status = f(static_cast<dsv3_stream_t>(stream));
+        PyEval_RestoreThread(save);
+    }
+    check(status);
+}
+
+// ------------------------------------------------------------------ split-K workspaces, one per (device, stream)
+struct Workspace {
+    int device;
+    cudaStream_t stream;
+    at::Tensor mem;
+};
+// (never destroyed: at process exit the CUDA context may already be gone)
+std::vector<Workspace>& g_workspaces = *new std::vector<Workspace>;
+// Smaller predecessors of a grown workspace: a captured graph may still refer to them.  Sizes at least double, so
+// together they stay below the size of the live one.
+std::vector<at::Tensor>& g_retired = *new std::vector<at::Tensor>;
+
+// The header of a workspace must be zero on first use; every call leaves it zero again.
+const at::Tensor& workspace(c10::Device dev, size_t bytes) {
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
+    Workspace* slot = nullptr;
+    for (Workspace& w : g_workspaces)
+        if (w.device == dev.index() && w.stream == stream) slot = &w;
+    if (slot && static_cast<size_t>(slot->mem.numel()) >= bytes) return slot->mem;
+    int64_t size = std::max<int64_t>(static_cast<int64_t>(bytes), 16ll << 20);
+    if (slot) size = std::max<int64_t>(size, 2 * slot->mem.numel());
+    c10::cuda::OptionalCUDAGuard guard(dev);
+    at::Tensor mem = new_cuda({size}, at::kByte, dev);
+    if (cudaMemsetAsync(mem.data_ptr(), 0, DSV3_WORKSPACE_HEADER_BYTES, stream) != cudaSuccess)
+        raise(PyExc_RuntimeError, "could not clear the header of a new split-K workspace");
+    if (slot) {
+        g_retired.push_back(slot->mem);
+        slot->mem = mem;
+        return slot->mem;
+    }
+    g_workspaces.push_back({dev.index(), stream, mem});
+    return g_workspaces.back().mem;
+}
+
+// ------------------------------------------------------------------ operators
+std::pair<at::Tensor, at::Tensor> quantise(const at::Tensor& x, int64_t block, int fmt) {
+    require(x.is_contiguous(), "Input tensor must be contiguous");
+    const int64_t K = last_dim(x);
+    if (block <= 0 || K % block != 0) {
+        PyErr_Format(PyExc_AssertionError, "Last dimension size must be divisible by block_size (block_size=%lld)",
+                     static_cast<long long>(block));
+        throw PythonError{};
+    }
+    const c10::Device dev = require_cuda(x);
+    if (x.scalar_type() != at::kBFloat16) {
+        PyErr_Format(PyExc_NotImplementedError, "act_quant takes bfloat16 activations (got %s)", c10::toString(x.scalar_type()));
+        throw PythonError{};
+    }
+    at::Tensor y = new_cuda(x.sizes(), at::kFloat8_e4m3fn, dev);
+    at::Tensor s = new_cuda_last(x, K / block, at::kFloat);
+    const int64_t rows = K ? x.numel() / K : 0;
+    const void* xp = x.const_data_ptr();
+    void* yp = y.data_ptr();
+    float* sp = static_cast<float*>(s.data_ptr());
+    call_library(dev, [&](dsv3_stream_t st) { return dsv3_act_quant(xp, rows, K, static_cast<int>(block), fmt, yp, sp, st); });
+    return {std::move(y), std::move(s)};
+}
+
+at::Tensor gemm(const at::Tensor& a, const at::Tensor& a_s, const at::Tensor& b, const at::Tensor& b_s) {
+    require(a.is_contiguous() && b.is_contiguous(), "Input tensors must be contiguous");
+    require(a_s.is_contiguous() && b_s.is_contiguous(), "Scaling factor tensors must be contiguous");
+    const c10::Device dev = require_cuda(a, a_s, b, b_s);
+    if (a.element_size() != 1 || b.element_size() != 1 || a_s.scalar_type() != at::kFloat || b_s.scalar_type() != at::kFloat)
+        raise(PyExc_NotImplementedError, "fp8_gemm takes 1-byte FP8 operands and float32 scales");
+    const int64_t K = last_dim(a);
+    if (K == 0) raise(PyExc_ZeroDivisionError, "integer division or modulo by zero");
+    const int64_t M = a.numel() / K, N = b.size(0);
+    require_bf16_default();
+    at::Tensor c = new_cuda_last(a, N, at::kBFloat16);
+    const size_t need = dsv3_fp8_gemm_workspace_bytes(M, N, K);
+    void* ws = nullptr;
+    size_t ws_bytes = 0;
+    if (need) {
+        const at::Tensor& w = workspace(dev, need);
+        ws = w.data_ptr();
+        ws_bytes = static_cast<size_t>(w.numel());
+    }
+    const void *ap = a.const_data_ptr(), *bp = b.const_data_ptr();
+    const float *asp = static_cast<const float*>(a_s.const_data_ptr()), *bsp = static_cast<const float*>(b_s.const_data_ptr());
+    void* cp = c.data_ptr();
+    call_library(dev, [&](dsv3_stream_t st) { return dsv3_fp8_gemm(ap, asp, bp, bsp, M, N, K, cp, ws, ws_bytes, st); });
+    return c;
+}
+
+at::Tensor linear_small(const at::Tensor& x, const at::Tensor& w, const at::Tensor& s, int fmt) {
+    require(x.is_contiguous() && w.is_contiguous() && s.is_contiguous(), "Input tensors must be contiguous");
+    const c10::Device dev = require_cuda(x, w, s);
+    if (x.scalar_type() != at::kBFloat16 || w.element_size() != 1 || s.scalar_type() != at::kFloat)
+        raise(PyExc_NotImplementedError, "fp8_linear takes bfloat16 activations, a 1-byte FP8 weight and float32 scales");
+    const int64_t K = last_dim(x);
+    const int64_t M = K ? x.numel() / K : 0, N = w.size(0);
+    require_bf16_default();
+    at::Tensor c = new_cuda_last(x, N, at::kBFloat16);
+    const void *xp = x.const_data_ptr(), *wp = w.const_data_ptr();
+    const float* sp = static_cast<const float*>(s.const_data_ptr());
+    void* cp = c.data_ptr();
+    call_library(dev, [&](dsv3_stream_t st) { return dsv3_fp8_linear(xp, M, K, wp, sp, N, fmt, cp, st); });
+    return c;
+}
+
+// ------------------------------------------------------------------ the FP8 branch of linear()
+// Quantisations of the two most recent activation tensors (see linear_seam.py for when an entry may be reused).
+struct Remembered {
+    c10::weak_intrusive_ptr<at::TensorImpl, c10::UndefinedTensorImpl> x;
+    const void* data;
+    c10::SmallVector<int64_t, 6> sizes;
+    int64_t version;          // -1: a tensor without a modification counter
+    int64_t block;
+    int fmt;
+    cudaStream_t stream;
+    at::Tensor q, s;
+};
+std::vector<Remembered>& g_memo = *new std::vector<Remembered>;     // at most two, most recent first
+PyObject* g_stats = nullptr;        // the seam's counters, a dict
+PyObject *g_key_calls, *g_key_reused, *g_key_fused, *g_attr_scale;
+
+void count(PyObject* key) {
+    PyObject* old = g_stats ? PyDict_GetItemWithError(g_stats, key) : nullptr;
+    if (!old) return;
+    PyObject* now = PyLong_FromLong(PyLong_AsLong(old) + 1);
+    if (!now || PyDict_SetItem(g_stats, key, now) != 0) PyErr_Clear();
+    Py_XDECREF(now);
+}
+
+std::pair<at::Tensor, at::Tensor> quantise_remembered(const at::Tensor& x, int64_t block, int fmt, bool assume_no_inplace) {
+    const bool counted = !x.is_inference();
+    if ((!counted && !assume_no_inplace) || !x.is_cuda()) {
+        count(g_key_calls);
+        return quantise(x, block, fmt);
+    }
+    const int64_t version = counted ? static_cast<int64_t>(x._version()) : -1;
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
+    for (size_t i = 0; i < g_memo.size(); ++i) {
+        Remembered& e = g_memo[i];
+        // a weak reference keeps the TensorImpl's address from being reused, so equal addresses mean the same tensor
+        if (e.x._unsafe_get_target() == x.unsafeGetTensorImpl() && e.version == version && e.data == x.const_data_ptr() &&
+            e.block == block && e.fmt == fmt && e.stream == stream && x.sizes() == at::IntArrayRef(e.sizes)) {
+            count(g_key_reused);
+            if (i) std::swap(g_memo[0], g_memo[i]);
+            return {g_memo[0].q, g_memo[0].s};
+        }
+    }
+    auto r = quantise(x, block, fmt);
+    count(g_key_calls);
+    if (g_memo.size() > 1) g_memo.pop_back();
+    g_memo.insert(g_memo.begin(), Remembered{decltype(Remembered::x)(x.getIntrusivePtr()), x.const_data_ptr(), {x.sizes().begin(), x.sizes().end()},
+                                             version, block, fmt, stream, r.first, r.second});
+    return r;
+}
+
+// ------------------------------------------------------------------ Python entry points
+void want_args(Py_ssize_t got, Py_ssize_t want) {
+    if (got != want) raise(PyExc_TypeError, "wrong number of arguments");
+}
+
+int64_t int_arg(PyObject* o) {
+    const long long v = PyLong_AsLongLong(o);
+    if (v == -1 && PyErr_Occurred()) throw PythonError{};
+    return v;
+}
+
+template <typename F>
+PyObject* guarded(F&& f) {
+    try {
+        return f();
+    } catch (const PythonError&) {
+        return nullptr;
+    } catch (const c10::OutOfMemoryError& e) {
+        PyErr_SetString(g_oom_class, e.what_without_backtrace());
+        return nullptr;
+    } catch (const std::exception& e) {
+        PyErr_SetString(PyExc_RuntimeError, e.what());
+        return nullptr;
+    }
+}
+
+PyObject* py_set_error_class(PyObject*, PyObject* cls) {
+    Py_XSETREF(g_error_class, Py_NewRef(cls));
+    Py_RETURN_NONE;
+}
+
+PyObject* py_act_quant(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        want_args(n, 3);
+        auto r = quantise(tensor_arg(args[0]), int_arg(args[1]), scale_fmt_arg(args[2]));
+        return wrap_pair(std::move(r.first), std::move(r.second));
+    });
+}
+
+PyObject* py_swiglu_quant(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        want_args(n, 3);
+        const at::Tensor &a = tensor_arg(args[0]), &b = tensor_arg(args[1]);
+        const int fmt = scale_fmt_arg(args[2]);
+        require(a.is_contiguous() && b.is_contiguous(), "Input tensors must be contiguous");
+        const int64_t K = last_dim(a);
+        require(a.sizes() == b.sizes() && K % 128 == 0, "a and b must have the same shape, last dimension divisible by 128");
+        const c10::Device dev = require_cuda(a, b);
+        if (a.scalar_type() != at::kBFloat16 || b.scalar_type() != at::kBFloat16)
+            raise(PyExc_NotImplementedError, "swiglu_quant takes bfloat16 tensors");
+        const int64_t rows = K ? a.numel() / K : 0;
+        at::Tensor y = new_cuda(a.sizes(), at::kFloat8_e4m3fn, dev);
+        at::Tensor s = new_cuda_last(a, K / 128, at::kFloat);
+        const void *ap = a.const_data_ptr(), *bp = b.const_data_ptr();
+        void* yp = y.data_ptr();
+        float* sp = static_cast<float*>(s.data_ptr());
+        call_library(dev, [&](dsv3_stream_t st) { return dsv3_swiglu_quant(ap, bp, rows, K, fmt, yp, sp, st); });
+        return wrap_pair(std::move(y), std::move(s));
+    });
+}
+
+PyObject* py_weight_dequant(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        want_args(n, 3);
+        const at::Tensor &x = tensor_arg(args[0]), &s = tensor_arg(args[1]);
+        const int64_t block = int_arg(args[2]);
+        require(x.is_contiguous() && s.is_contiguous(), "Input tensors must be contiguous");
+        require(x.dim() == 2 && s.dim() == 2, "Input tensors must have 2 dimensions");
+        const c10::Device dev = require_cuda(x, s);
+        if (x.element_size() != 1 || s.scalar_type() != at::kFloat)
+            raise(PyExc_NotImplementedError, "weight_dequant takes a 1-byte FP8 weight and float32 scales");
+        require_bf16_default();
+        at::Tensor y = new_cuda(x.sizes(), at::kBFloat16, dev);
+        const int64_t N = x.size(0), K = x.size(1);
+        const void* xp = x.const_data_ptr();
+        const float* sp = static_cast<const float*>(s.const_data_ptr());
+        void* yp = y.data_ptr();
+        call_library(dev, [&](dsv3_stream_t st) { return dsv3_weight_dequant(xp, sp, N, K, static_cast<int>(block), yp, st); });
+        return wrap(std::move(y));
+    });
+}
+
+PyObject* py_fp8_gemm(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        want_args(n, 4);
+        return wrap(gemm(tensor_arg(args[0]), tensor_arg(args[1]), tensor_arg(args[2]), tensor_arg(args[3])));
+    });
+}
+
+PyObject* py_fp8_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        want_args(n, 4);
+        return wrap(linear_small(tensor_arg(args[0]), tensor_arg(args[1]), tensor_arg(args[2]), scale_fmt_arg(args[3])));
+    });
+}
+
+// (x, weight, block_size, scale_fmt, assume_no_inplace, fused_max_rows, fused_max_bytes): linear()'s FP8 branch.
+PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        want_args(n, 7);
+        const at::Tensor &x = tensor_arg(args[0]), &w = tensor_arg(args[1]);
+        const int64_t block = int_arg(args[2]);
+        const int fmt = scale_fmt_arg(args[3]);
+        PyObject* scale_obj = PyObject_GetAttr(args[1], g_attr_scale);
+        if (!scale_obj) throw PythonError{};
+        at::Tensor scale;
+        if (THPVariable_Check(scale_obj)) scale = THPVariable_Unpack(scale_obj);
+        Py_DECREF(scale_obj);
+        if (!scale.defined()) raise(PyExc_TypeError, "weight.scale is not a tensor");
+        const int64_t K = last_dim(x), rows = K ? x.numel() / K : 0;
+        if (rows > 0 && rows <= int_arg(args[5]) && w.numel() <= int_arg(args[6]) && block == 128 && K % 128 == 0 &&
+            x.scalar_type() == at::kBFloat16 && x.is_contiguous()) {
+            count(g_key_fused);
+            return wrap(linear_small(x, w, scale, fmt));
+        }
+        auto q = quantise_remembered(x, block, fmt, PyObject_IsTrue(args[4]) == 1);
+        return wrap(gemm(q.first, q.second, w, scale));
+    });
+}
+
+// (x, block_size, scale_fmt, assume_no_inplace) -> (y, s), remembered
+PyObject* py_quantise_remembered(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        want_args(n, 4);
+        auto r = quantise_remembered(tensor_arg(args[0]), int_arg(args[1]), scale_fmt_arg(args[2]), PyObject_IsTrue(args[3]) == 1);
+        return wrap_pair(std::move(r.first), std::move(r.second));
+    });
+}
+
+PyObject* py_set_stats(PyObject*, PyObject* dict) {
+    Py_XSETREF(g_stats, Py_NewRef(dict));
+    Py_RETURN_NONE;
+}
+
+PyObject* py_forget(PyObject*, PyObject*) {
+    g_memo.clear();
+    Py_RETURN_NONE;
+}
+
+// After a bounded wait gave up, tickets may be left non-zero.
+PyObject* py_clear_workspaces(PyObject*, PyObject*) {
+    return guarded([&]() -> PyObject* {
+        for (Workspace& w : g_workspaces) {
+            c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(w.device));
+            if (cudaMemsetAsync(w.mem.data_ptr(), 0, DSV3_WORKSPACE_HEADER_BYTES, w.stream) != cudaSuccess)
+                raise(PyExc_RuntimeError, "could not clear the header of a split-K workspace");
+        }
+        Py_RETURN_NONE;
+    });
+}
+
+PyMethodDef methods[] = {
+    {"set_error_class", py_set_error_class, METH_O, "class raised for a non-zero status: cls(status, message)"},
+    {"act_quant", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_act_quant)), METH_FASTCALL, "(x, block_size, scale_fmt)"},
+    {"swiglu_quant", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_swiglu_quant)), METH_FASTCALL, "(a, b, scale_fmt)"},
+    {"weight_dequant", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_weight_dequant)), METH_FASTCALL, "(x, s, block_size)"},
+    {"fp8_gemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_fp8_gemm)), METH_FASTCALL, "(a, a_s, b, b_s)"},
+    {"fp8_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_fp8_linear)), METH_FASTCALL, "(x, weight, scale, scale_fmt)"},
+    {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_linear)), METH_FASTCALL,
+     "(x, weight, block_size, scale_fmt, assume_no_inplace, fused_max_rows, fused_max_bytes)"},
+    {"quantise_remembered", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_quantise_remembered)), METH_FASTCALL,
+     "(x, block_size, scale_fmt, assume_no_inplace)"},
+    {"set_stats", py_set_stats, METH_O, "dict whose counters linear() keeps"},
+    {"forget", py_forget, METH_NOARGS, "drop the remembered quantisations"},
+    {"clear_workspaces", py_clear_workspaces, METH_NOARGS, "zero the ticket headers of all split-K workspaces"},
+    {nullptr, nullptr, 0, nullptr},
+};
+
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_dsv3_host", "Native host path of the dsv3_b200 operators.", -1, methods,
+                          nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__dsv3_host(void) {
+    g_key_calls = PyUnicode_InternFromString("act_quant_calls");
+    g_key_reused = PyUnicode_InternFromString("act_quant_reused");
+    g_key_fused = PyUnicode_InternFromString("fused_linear_calls");
+    g_attr_scale = PyUnicode_InternFromString("scale");
+    PyObject* torch = PyImport_ImportModule("torch");
+    g_oom_class = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
+    Py_XDECREF(torch);
+    if (!g_oom_class) return nullptr;
+    if (!g_key_calls || !g_key_reused || !g_key_fused || !g_attr_scale) return nullptr;
+    return PyModule_Create(&module_def);
+}

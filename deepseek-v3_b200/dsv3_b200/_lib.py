@@ -1,16 +1,19 @@
-"""ctypes binding of libdsv3_b200.so (the C ABI declared in include/dsv3_b200.h).
+"""Bindings of libdsv3_b200.so (the C ABI declared in include/dsv3_b200.h): ctypes for set-up and rarely called entry
+points (``lib``), the CPython extension ``_dsv3_host.so`` for the operators (``host``).
 
-The library is built in-tree by ``deepseek-v3_b200/build.py``.  There is no other
-implementation behind these functions: if the shared object is missing the import
-fails, and tensors that are not on a CUDA device are rejected.
+Both are built in-tree by ``deepseek-v3_b200/build.py``.  There is no other implementation behind these functions: if
+a shared object is missing the import fails, and tensors that are not on a CUDA device are rejected.
 """
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(os.path.dirname(_HERE), "lib", "libdsv3_b200.so")
+HOST_PATH = os.path.join(os.path.dirname(_HERE), "lib", "_dsv3_host.so")
 
 OK = 0
 ERR_INVALID_ARGUMENT = -1
@@ -97,3 +100,18 @@ def check(status: int) -> None:
     if status != OK:
         detail = lib.dsv3_last_error().decode(errors="replace")
         raise Dsv3Error(status, f"{lib.dsv3_strerror(status).decode()} ({status}): {detail}")
+
+
+def _load_host():
+    if not os.path.exists(HOST_PATH):
+        raise ImportError(f"{HOST_PATH} is missing: build it with `python deepseek-v3_b200/build.py`")
+    import torch  # noqa: F401  (its libraries must be loaded before the extension that links against them)
+    loader = importlib.machinery.ExtensionFileLoader("_dsv3_host", HOST_PATH)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_dsv3_host", HOST_PATH, loader=loader))
+    loader.exec_module(module)
+
+    module.set_error_class(Dsv3Error)
+    return module
+
+
+host = _load_host()

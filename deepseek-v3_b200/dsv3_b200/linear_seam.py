@@ -26,48 +26,17 @@ does).
 """
 from __future__ import annotations
 
-import weakref
 from typing import Optional
 
 import torch
 import torch.nn.functional as F
 
-from .ops import (act_quant, fp8_gemm, fp8_linear, weight_dequant, FUSED_LINEAR_MAX_ROWS, FUSED_LINEAR_MAX_WEIGHT_BYTES,
-                  _stream)
+from ._lib import host
+from .ops import weight_dequant, FUSED_LINEAR_MAX_ROWS, FUSED_LINEAR_MAX_WEIGHT_BYTES
 
-_memo = []          # at most two entries, most recent first: dicts with ref / version / key / value
 stats = {"act_quant_calls": 0, "act_quant_reused": 0, "fused_linear_calls": 0}
 _assume_no_inplace = False
-
-
-def _version(x: torch.Tensor) -> Optional[int]:
-    """In-place modification counter, or None for tensors that have none (inference mode)."""
-    try:
-        return x._version
-    except RuntimeError:
-        return None
-
-
-def _quantised(x: torch.Tensor, block_size: int, scale_fmt: Optional[str]):
-    ver = _version(x)
-    if ver is None and not _assume_no_inplace:
-        stats["act_quant_calls"] += 1
-        return act_quant(x, block_size, scale_fmt)
-    key = (x.data_ptr(), tuple(x.shape), block_size, scale_fmt, _stream())
-    for i, e in enumerate(_memo):
-        if e["ref"]() is x and e["version"] == ver and e["key"] == key:
-            stats["act_quant_reused"] += 1
-            if i:
-                _memo.insert(0, _memo.pop(i))
-            return e["value"]
-    value = act_quant(x, block_size, scale_fmt)
-    stats["act_quant_calls"] += 1
-    try:
-        _memo.insert(0, dict(ref=weakref.ref(x), version=ver, key=key, value=value))
-        del _memo[2:]
-    except TypeError:           # tensor subclasses that cannot be weakly referenced: no memo
-        pass
-    return value
+host.set_stats(stats)
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,
@@ -77,15 +46,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         return F.linear(x, weight, bias)
     if gemm_impl == "bf16":
         return F.linear(x, weight_dequant(weight, weight.scale), bias)
-    K = x.size(-1)
-    rows = x.numel() // K if K else 0
-    if (0 < rows <= FUSED_LINEAR_MAX_ROWS and weight.numel() <= FUSED_LINEAR_MAX_WEIGHT_BYTES and block_size == 128
-            and K % 128 == 0 and x.dtype == torch.bfloat16 and x.is_contiguous()):
-        stats["fused_linear_calls"] += 1
-        y = fp8_linear(x, weight, weight.scale, scale_fmt)
-    else:
-        xq, xs = _quantised(x, block_size, scale_fmt)
-        y = fp8_gemm(xq, xs, weight, weight.scale)
+    y = host.linear(x, weight, block_size, scale_fmt, _assume_no_inplace, FUSED_LINEAR_MAX_ROWS, FUSED_LINEAR_MAX_WEIGHT_BYTES)
     if bias is not None:
         y += bias
     return y
@@ -105,5 +66,5 @@ def install_linear(model_module, assume_no_inplace: bool = False) -> None:
 
 
 def reset_memo() -> None:
-    del _memo[:]
+    host.forget()
     stats.update(act_quant_calls=0, act_quant_reused=0, fused_linear_calls=0)

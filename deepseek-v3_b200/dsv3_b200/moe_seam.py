@@ -18,8 +18,8 @@ from typing import List
 import torch
 
 from . import _lib
-from ._lib import lib
-from .linear_seam import _quantised
+from . import linear_seam
+from ._lib import host, lib
 from .ops import swiglu_quant, _stream
 
 
@@ -79,7 +79,7 @@ class GroupedExperts:
             _lib.check(lib.dsv3_moe_route(idx.data_ptr(), wf.data_ptr(), T, topk, self.start, n, seg.data_ptr(),
                                           tok.data_ptr(), pair_row.data_ptr(), pos_s.data_ptr(), w_s.data_ptr(), _stream()))
             # ---- quantise every token once, gather the rows in expert order
-            xq, xs = _quantised(x, 128, self.scale_fmt)
+            xq, xs = host.quantise_remembered(x, 128, self.scale_fmt, linear_seam._assume_no_inplace)
             xq_p = xq.view(torch.uint8).index_select(0, tok).view(torch.float8_e4m3fn)
             xs_p = xs.index_select(0, tok)
             # ---- w2(silu(w1 x) * w3 x), the bf16 rounding points of Expert.forward (model.py:633)

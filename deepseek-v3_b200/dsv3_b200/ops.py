@@ -8,17 +8,15 @@ device and nothing here falls back to another implementation.
 """
 from __future__ import annotations
 
-from typing import Dict, Optional, Tuple
+from typing import Optional, Tuple
 
 import torch
 
 from . import _lib
-from ._lib import lib
+from ._lib import host, lib
 
 KERNEL_AUTO, KERNEL_CUDA_CORE, KERNEL_TC_TOKEN_MAJOR, KERNEL_TC_WEIGHT_MAJOR, KERNEL_TC_TOKEN_PAIR, KERNEL_DECODE = 0, 1, 2, 3, 4, 5
 KERNEL_TC_TOKEN_PAIR_WIDE = 6
-
-_workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
 
 
 def _require_cuda(*tensors: torch.Tensor) -> torch.device:
@@ -36,29 +34,6 @@ def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
 
-def _out_dtype() -> torch.dtype:
-    dt = torch.get_default_dtype()
-    if dt != torch.bfloat16:
-        raise NotImplementedError(
-            "the CUDA path writes bfloat16 only; call torch.set_default_dtype(torch.bfloat16) "
-            f"as every entry point of the reference does (default dtype is {dt})")
-    return dt
-
-
-def _workspace(dev: torch.device, nbytes: int) -> Optional[torch.Tensor]:
-    """Scratch for split-K, one per (device, stream); its header must be zero on first use and
-    every call leaves it zero again."""
-    if nbytes == 0:
-        return None
-    key = (dev.index if dev.index is not None else torch.cuda.current_device(), _stream())
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        size = max(nbytes, 8 << 20)
-        ws = torch.zeros(size, dtype=torch.uint8, device=dev)
-        _workspaces[key] = ws
-    return ws
-
-
 def act_quant(x: torch.Tensor, block_size: int = 128, scale_fmt: Optional[str] = None
               ) -> Tuple[torch.Tensor, torch.Tensor]:
     """Block-wise FP8 quantisation of activations (kernel.py:38-57).
@@ -67,38 +42,13 @@ def act_quant(x: torch.Tensor, block_size: int = 128, scale_fmt: Optional[str] =
     ``[..., K // block_size]`` with ``s = max(amax, 1e-4) / 448`` per block (rounded up to a
     power of two when ``scale_fmt == "ue8m0"``).
     """
-    assert x.is_contiguous(), 'Input tensor must be contiguous'
-    assert x.size(-1) % block_size == 0, \
-        f'Last dimension size must be divisible by block_size (block_size={block_size})'
-    dev = _require_cuda(x)
-    if x.dtype != torch.bfloat16:
-        raise NotImplementedError(f"act_quant takes bfloat16 activations (got {x.dtype})")
-    y = torch.empty_like(x, dtype=torch.float8_e4m3fn)
-    s = x.new_empty(*x.size()[:-1], x.size(-1) // block_size, dtype=torch.float32)
-    K = x.size(-1)
-    rows = x.numel() // K if K else 0
-    with torch.cuda.device(dev):
-        _lib.check(lib.dsv3_act_quant(x.data_ptr(), rows, K, block_size, 1 if scale_fmt == "ue8m0" else 0,
-                                      y.data_ptr(), s.data_ptr(), _stream()))
-    return y, s
+    return host.act_quant(x, block_size, scale_fmt)
 
 
 def swiglu_quant(a: torch.Tensor, b: torch.Tensor, scale_fmt: Optional[str] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """``act_quant(F.silu(a) * b, 128, scale_fmt)`` in one launch (model.py:532 / 633 followed by :158-159), with the
     rounding points of the three-launch form; the bf16 product is never written."""
-    assert a.is_contiguous() and b.is_contiguous(), 'Input tensors must be contiguous'
-    assert a.shape == b.shape and a.size(-1) % 128 == 0, 'a and b must have the same shape, last dimension divisible by 128'
-    dev = _require_cuda(a, b)
-    if a.dtype != torch.bfloat16 or b.dtype != torch.bfloat16:
-        raise NotImplementedError("swiglu_quant takes bfloat16 tensors")
-    K = a.size(-1)
-    rows = a.numel() // K if K else 0
-    y = torch.empty_like(a, dtype=torch.float8_e4m3fn)
-    s = a.new_empty(*a.size()[:-1], K // 128, dtype=torch.float32)
-    with torch.cuda.device(dev):
-        _lib.check(lib.dsv3_swiglu_quant(a.data_ptr(), b.data_ptr(), rows, K, 1 if scale_fmt == "ue8m0" else 0,
-                                         y.data_ptr(), s.data_ptr(), _stream()))
-    return y, s
+    return host.swiglu_quant(a, b, scale_fmt)
 
 
 # Cache of de-quantised weights (off by default).  MLA.forward in "absorb" mode de-quantises wkv_b on every call of
@@ -135,25 +85,17 @@ def _version_or_none(t: torch.Tensor):
 
 def weight_dequant(x: torch.Tensor, s: torch.Tensor, block_size: int = 128) -> torch.Tensor:
     """De-quantise a block-scaled FP8 weight to the default dtype (kernel.py:89-110)."""
-    assert x.is_contiguous() and s.is_contiguous(), 'Input tensors must be contiguous'
-    assert x.dim() == 2 and s.dim() == 2, 'Input tensors must have 2 dimensions'
-    dev = _require_cuda(x, s)
-    if x.element_size() != 1 or s.dtype != torch.float32:
-        raise NotImplementedError("weight_dequant takes a 1-byte FP8 weight and float32 scales")
-    M, N = x.size()
     key = None
     if _dequant_cache is not None:
         vx, vs = _version_or_none(x), _version_or_none(s)
         if vx is not None and vs is not None:
-            key = (x.data_ptr(), s.data_ptr(), M, N, block_size, vx, vs, _out_dtype())
+            key = (x.data_ptr(), s.data_ptr(), tuple(x.shape), block_size, vx, vs, torch.get_default_dtype())
             hit = _dequant_cache.get(key)
             if hit is not None and hit[0]() is x:
                 _dequant_cache.move_to_end(key)
                 dequant_stats["hits"] += 1
                 return hit[1]
-    y = torch.empty_like(x, dtype=_out_dtype())
-    with torch.cuda.device(dev):
-        _lib.check(lib.dsv3_weight_dequant(x.data_ptr(), s.data_ptr(), M, N, block_size, y.data_ptr(), _stream()))
+    y = host.weight_dequant(x, s, block_size)
     dequant_stats["launches"] += 1
     if key is not None:
         import weakref
@@ -170,38 +112,13 @@ def weight_dequant(x: torch.Tensor, s: torch.Tensor, block_size: int = 128) -> t
 
 def fp8_gemm(a: torch.Tensor, a_s: torch.Tensor, b: torch.Tensor, b_s: torch.Tensor) -> torch.Tensor:
     """Block-scaled FP8 GEMM ``c = a @ b.T`` with fp32 accumulation (kernel.py:175-196)."""
-    assert a.is_contiguous() and b.is_contiguous(), 'Input tensors must be contiguous'
-    assert a_s.is_contiguous() and b_s.is_contiguous(), 'Scaling factor tensors must be contiguous'
-    dev = _require_cuda(a, a_s, b, b_s)
-    if a.element_size() != 1 or b.element_size() != 1 or a_s.dtype != torch.float32 or b_s.dtype != torch.float32:
-        raise NotImplementedError("fp8_gemm takes 1-byte FP8 operands and float32 scales")
-    K = a.size(-1)
-    M = a.numel() // K
-    N = b.size(0)
-    c = a.new_empty(*a.size()[:-1], N, dtype=_out_dtype())
-    with torch.cuda.device(dev):
-        ws = _workspace(dev, lib.dsv3_fp8_gemm_workspace_bytes(M, N, K))
-        _lib.check(lib.dsv3_fp8_gemm(a.data_ptr(), a_s.data_ptr(), b.data_ptr(), b_s.data_ptr(), M, N, K,
-                                     c.data_ptr(), ws.data_ptr() if ws is not None else None,
-                                     ws.numel() if ws is not None else 0, _stream()))
-    return c
+    return host.fp8_gemm(a, a_s, b, b_s)
 
 
 def fp8_linear(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, scale_fmt: Optional[str] = None) -> torch.Tensor:
     """``fp8_gemm(*act_quant(x, 128, scale_fmt), weight, scale)`` (model.py:158-160) in one launch, for at most 16
     rows: the activations are quantised in the GEMM's prologue.  Raises ``Dsv3Error`` (status -2) for other shapes."""
-    assert x.is_contiguous() and weight.is_contiguous() and scale.is_contiguous(), 'Input tensors must be contiguous'
-    dev = _require_cuda(x, weight, scale)
-    if x.dtype != torch.bfloat16 or weight.element_size() != 1 or scale.dtype != torch.float32:
-        raise NotImplementedError("fp8_linear takes bfloat16 activations, a 1-byte FP8 weight and float32 scales")
-    K = x.size(-1)
-    M = x.numel() // K if K else 0
-    N = weight.size(0)
-    c = x.new_empty(*x.size()[:-1], N, dtype=_out_dtype())
-    with torch.cuda.device(dev):
-        _lib.check(lib.dsv3_fp8_linear(x.data_ptr(), M, K, weight.data_ptr(), scale.data_ptr(), N,
-                                       1 if scale_fmt == "ue8m0" else 0, c.data_ptr(), _stream()))
-    return c
+    return host.fp8_linear(x, weight, scale, scale_fmt)
 
 
 # The kernel takes up to 16 rows; the seam uses it up to 4, where quantising the activations inside every CTA is
@@ -241,6 +158,5 @@ def check_device_status() -> None:
     detail = (ctypes.c_uint32 * 4)()
     rc = lib.dsv3_check_device_status(_stream(), ctypes.byref(detail))
     if rc != _lib.OK:
-        for ws in _workspaces.values():   # tickets may be left non-zero by an aborted launch
-            ws[: _lib.WORKSPACE_HEADER_BYTES].zero_()
+        host.clear_workspaces()           # tickets may be left non-zero by an aborted launch
         _lib.check(rc)
