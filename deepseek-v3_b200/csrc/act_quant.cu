@@ -90,17 +90,9 @@ __global__ void __launch_bounds__(kThreads) act_quant_generic_kernel(const uint4
 
 // SwiGLU followed by act_quant in one pass: h = bf16(bf16(silu(a)) * b), then h is quantised per 128 values.
 // Replaces the three launches `F.silu(w1(x)) * w3(x)` + act_quant in front of w2 (model.py:532, 633 and 158-159) and
-// keeps their rounding points: silu is evaluated in fp32 as a / (1 + exp(-a)) and rounded to bf16, the product is
+// keeps their rounding points: silu is evaluated in fp32 and rounded to bf16 (swiglu8), the product is
 // formed in fp32 and rounded to bf16 (what the framework's bf16 kernels do), and the quantisation of h is the
 // arithmetic of act_quant128_kernel.  h itself is never written.
-__device__ __forceinline__ uint32_t swiglu2(uint32_t a2, uint32_t b2) {
-    const float al = bf16_bits_to_float(a2 & 0xFFFFu), ah = __uint_as_float(a2 & 0xFFFF0000u);
-    const float bl = bf16_bits_to_float(b2 & 0xFFFFu), bh = __uint_as_float(b2 & 0xFFFF0000u);
-    const float sl = __bfloat162float(__float2bfloat16_rn(al / (1.0f + expf(-al))));
-    const float sh = __bfloat162float(__float2bfloat16_rn(ah / (1.0f + expf(-ah))));
-    return pack_bf16x2(sl * bl, sh * bh);
-}
-
 __global__ void __launch_bounds__(kThreads, 4) swiglu_quant128_kernel(const uint4* __restrict__ a, const uint4* __restrict__ b,
                                                                     uint2* __restrict__ y, float* __restrict__ s, int64_t nblk,
                                                                     int scale_fmt) {
@@ -118,8 +110,7 @@ __global__ void __launch_bounds__(kThreads, 4) swiglu_quant128_kernel(const uint
 #pragma unroll
     for (int u = 0; u < kUnroll; ++u) {
         const int64_t blk = b0 + u * (kThreads / 16);
-        const uint4 h = make_uint4(swiglu2(va[u].x, vb[u].x), swiglu2(va[u].y, vb[u].y), swiglu2(va[u].z, vb[u].z),
-                                   swiglu2(va[u].w, vb[u].w));
+        const uint4 h = swiglu8(va[u], vb[u]);
         float m = amax8(h);
         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));

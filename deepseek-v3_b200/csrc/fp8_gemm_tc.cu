@@ -38,7 +38,6 @@
 #include <cstring>
 #include <mutex>
 #include <type_traits>
-#include <vector>
 
 #include "common.cuh"
 #include "gemm_plan.cuh"
@@ -72,22 +71,15 @@ struct TcParams {
     int kc;                 // number of K chunks
     int tiles_p, tiles_q;
     int splits;
-    FastDiv div_splits, div_per_group, div_raster, div_tiles_p;   // for the work-item decoder
+    FastDiv div_splits, div_per_group, div_raster;   // for the work-item decoder
     int raster;             // token-major tiles: P tiles (token tiles) that share consecutive Q tiles in the work order
     int tma_store;          // token-major tiles: results leave through shared memory and a TMA store (needs N % 8 == 0)
     int num_items;          // tiles_p * tiles_q * splits
-    // Grouped mode (MoE experts; weight-major tiles only, no split-K): group e multiplies the activation
-    // rows [g_seg[e], g_seg[e+1]) with its own weight.  n_groups == 0 means one ordinary GEMM.
-    const CUtensorMap* g_tmaps;    // per-group weight tensor maps, in global memory
-    const float* const* g_bs;      // per-group weight scale pointers, in global memory
-    const int* g_seg;              // [n_groups + 1] row offsets, in global memory (written on the device)
-    int n_groups;
-    int g_slots;                   // upper bound on the number of token tiles over all groups
 };
 
 // K chunks of one weight-major work item whose scales fit the shared-memory table: 144 (K <= 18432) for
 // 16- and 32-token tiles, 72 for 64-token tiles (the same 18 KB, which leaves room for four 48 KB stages;
-// longer K is split, or uses the 32-token variant in grouped mode)
+// longer K is split)
 constexpr int scale_tab_chunks(int bn) { return bn >= 64 ? 72 : 144; }
 
 template <int BN, bool kSwap>
@@ -103,11 +95,10 @@ struct Cfg {
     static constexpr int kTmemUnits = kAccs / kUC;                          // unit products resident in TMEM
     // weight-major tiles: a_s * b_s of the item's chunks for the tile's BN tokens, [chunk][token]
     static constexpr int kScaleTabBytes = kSwap ? scale_tab_chunks(BN) * BN * 4 : 0;
-    static constexpr int kGroupTabBytes = kSwap ? 2048 : 0;   // grouped mode: token-tile prefix per group
     // token-major tiles: the 128 x 128 bf16 result tile is staged here (two 128-byte-swizzled 128 x 64 boxes)
     static constexpr int kStoreBytes = !kSwap ? kPRows * 128 * 2 : 0;
     static constexpr int kStagesRaw =
-        (232448 - 2048 - kStoreBytes - kScaleTabBytes - kGroupTabBytes) / kStageBytes;
+        (232448 - 2048 - kStoreBytes - kScaleTabBytes) / kStageBytes;
     static constexpr int kStagesCap = kStagesRaw > 10 ? 10 : kStagesRaw;
     // weight-major tiles: an even stage count, so that a stage always belongs to the same MMA issuer and
     // the issuer may probe its next full[] barrier (see the issuer loop)
@@ -115,7 +106,7 @@ struct Cfg {
     static constexpr int kTmemCols = kAccs * BN;  // 64..512, a power of two
     // tiles + result staging + tables + barriers + control words + slack for the 1024-byte alignment of the tiles
     static constexpr int kSmemBytes =
-        kStages * kStageBytes + kStoreBytes + kScaleTabBytes + kGroupTabBytes + 1024 + 1024;
+        kStages * kStageBytes + kStoreBytes + kScaleTabBytes + 1024 + 1024;
     static_assert(kSmemBytes <= 232448, "shared memory per CTA");
     static_assert(kStages >= 3, "at least three smem stages");
     static_assert(kTmemCols >= 32 && kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "TMEM columns");
@@ -127,43 +118,13 @@ struct Cfg {
 struct Item {
     int p_idx, q_idx, split, tile;
     int c0, c1;     // chunk range
-    int group;      // grouped mode: which weight
     int row0;       // weight-major tiles: first activation row of the tile
     int row_end;    // weight-major tiles: activation rows at and beyond this index are not part of the problem
 };
 
-constexpr int kMaxGroups = 256;
-
-// g_prefix (shared memory, grouped mode): g_prefix[e] = number of token tiles of the groups before e.
 template <int BN, bool kSwap>
-__device__ __forceinline__ Item decode_item(int item, const TcParams& p, const int* g_prefix) {
+__device__ __forceinline__ Item decode_item(int item, const TcParams& p) {
     Item it;
-    if (kSwap && p.n_groups > 0) {
-        // item -> (weight tile p_idx, token-tile slot); slot -> (group, tile within the group) by binary search
-        const int slot = static_cast<int>(fast_div(static_cast<uint32_t>(item), p.div_tiles_p));
-        it.p_idx = item - slot * p.tiles_p;
-        it.tile = item;
-        it.split = 0;
-        it.q_idx = 0;
-        int lo = 0, hi = p.n_groups;          // invariant: g_prefix[lo] <= slot, answer in [lo, hi)
-        if (slot >= g_prefix[p.n_groups]) {   // beyond the last real tile: an empty item
-            it.group = 0;
-            it.row0 = it.row_end = 0;
-            it.c0 = it.c1 = 0;
-            return it;
-        }
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (g_prefix[mid] <= slot) lo = mid; else hi = mid;
-        }
-        it.group = lo;
-        it.row0 = __ldg(p.g_seg + lo) + (slot - g_prefix[lo]) * BN;
-        it.row_end = __ldg(p.g_seg + lo + 1);
-        it.c0 = 0;
-        it.c1 = p.kc;
-        return it;
-    }
-    it.group = 0;
     it.tile = static_cast<int>(fast_div(static_cast<uint32_t>(item), p.div_splits));
     it.split = item - it.tile * p.splits;
     // work order: `raster` P tiles share consecutive Q tiles so that a wave re-uses both operands in L2
@@ -222,8 +183,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
     uint8_t* store_buf = gen_tiles + NS * C::kStageBytes;                       // 1024-byte aligned (swizzle atom)
     uint8_t* after_store = store_buf + C::kStoreBytes;
     float* sc_tab = reinterpret_cast<float*>(after_store);   // [chunk][token]
-    int* g_prefix = reinterpret_cast<int*>(after_store + C::kScaleTabBytes);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(after_store + C::kScaleTabBytes + C::kGroupTabBytes);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(after_store + C::kScaleTabBytes);
     Control* ctl = reinterpret_cast<Control*>(bars + 2 * NS + 2 * NT + 2);
     const uint32_t bar0 = smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
@@ -260,8 +220,8 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
     // the kernel before this one in the stream.  While waiting for that kernel, the producer thread pulls
     // the first weight boxes of this CTA's first work item into L2 (L2 is the point of coherence: should
     // the predecessor still be writing those weights, the later TMA loads see its data all the same).
-    if (threadIdx.x == 0 && p.n_groups == 0 && static_cast<int>(blockIdx.x) < p.num_items) {
-        const Item it = decode_item<BN, kSwap>(blockIdx.x, p, g_prefix);
+    if (threadIdx.x == 0 && static_cast<int>(blockIdx.x) < p.num_items) {
+        const Item it = decode_item<BN, kSwap>(blockIdx.x, p);
         const void* wmap = kSwap ? static_cast<const void*>(&tmap_p) : static_cast<const void*>(&tmap_q);
         const int wrow = kSwap ? it.p_idx * kPRows : it.q_idx * BN;
         const int n_pre = min(it.c1 - it.c0, NS * UC);
@@ -269,24 +229,6 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
     }
     griddep_launch_dependents();
     griddep_wait();
-    if constexpr (kSwap) {
-        if (p.n_groups > 0) {
-            // token tiles per group, then an exclusive prefix sum (n_groups <= kMaxGroups)
-            for (int e = threadIdx.x; e < p.n_groups; e += kNumThreads) {
-                const int cnt = __ldg(p.g_seg + e + 1) - __ldg(p.g_seg + e);
-                g_prefix[e + 1] = (cnt + BN - 1) / BN;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int run = 0;
-                g_prefix[0] = 0;
-                for (int e = 1; e <= p.n_groups; ++e) {
-                    run += g_prefix[e];
-                    g_prefix[e] = run;
-                }
-            }
-        }
-    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -309,11 +251,9 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
             uint32_t probe = 0;   // result of try_wait on empty[] for chunk g, issued one chunk earlier
             bool ok = true;
             for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
-                const Item it = decode_item<BN, kSwap>(item, p, g_prefix);
+                const Item it = decode_item<BN, kSwap>(item, p);
                 const int p_row = it.p_idx * kPRows;
                 const int q_row = kSwap ? it.row0 : it.q_idx * BN;
-                const void* map_p = (kSwap && p.n_groups > 0) ? static_cast<const void*>(p.g_tmaps + it.group)
-                                                               : static_cast<const void*>(&tmap_p);
                 const int n_units = (it.c1 - it.c0 + UC - 1) / UC;
                 for (int u = 0; u < n_units; ++u, ++g) {
                     const int s = g % NS;
@@ -326,7 +266,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                         mbar_arrive_expect_tx(full_bar(s), nch * C::kChunkBytes);
                         for (int j = 0; j < nch; ++j) {
                             const uint32_t dst = tiles + s * C::kStageBytes + j * C::kChunkBytes;
-                            tma_load_2d(dst, map_p, (k0 + j) * kChunk, p_row, full_bar(s));
+                            tma_load_2d(dst, &tmap_p, (k0 + j) * kChunk, p_row, full_bar(s));
                             tma_load_2d(dst + kPRows * kChunk, &tmap_q, (k0 + j) * kChunk, q_row, full_bar(s));
                         }
                     }
@@ -348,7 +288,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
             uint32_t probe_t = 0, probe_f = 0;   // probes of tempty[] / full[] for this issuer's next unit
             bool ok = true;
             for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
-                const Item it = decode_item<BN, kSwap>(item, p, g_prefix);
+                const Item it = decode_item<BN, kSwap>(item, p);
                 const int n_units = (it.c1 - it.c0 + UC - 1) / UC;
                 for (int u = 0; u < n_units; ++u, ++g) {
                     if (g % kIssuers != me) continue;
@@ -435,9 +375,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
         };
 
         for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
-            const Item it = decode_item<BN, kSwap>(item, p, g_prefix);
-            // grouped mode: slots beyond the last token tile carry no work; they cost a decode and nothing else
-            if (it.c1 <= it.c0) continue;
+            const Item it = decode_item<BN, kSwap>(item, p);
             const uint32_t item_cur = item_no++;
             float2 acc[CPT / 2];
 #pragma unroll
@@ -454,8 +392,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                 bs_ptr = p.b_s + static_cast<int64_t>(it.q_idx) * kc;          // BN == 128
             } else {
                 as_ptr = p.a_s;
-                const float* bs_base = (p.n_groups > 0) ? p.g_bs[it.group] : p.b_s;
-                bs_ptr = bs_base + static_cast<int64_t>(it.p_idx) * kc;        // 128 weight rows = one scale row
+                bs_ptr = p.b_s + static_cast<int64_t>(it.p_idx) * kc;        // 128 weight rows = one scale row
             }
             const int n_ch = it.c1 - it.c0;
             // Weight-major tiles: every thread needs a_s * b_s of all its tokens for every chunk; the
@@ -1016,13 +953,7 @@ int launch_fp8_gemm_tc(const void* a, const float* a_s, const void* b, const flo
     prm.div_splits = make_fast_div(static_cast<uint32_t>(prm.splits));
     prm.div_raster = make_fast_div(static_cast<uint32_t>(prm.raster));
     prm.div_per_group = make_fast_div(static_cast<uint32_t>(prm.raster) * static_cast<uint32_t>(prm.tiles_q));
-    prm.div_tiles_p = make_fast_div(static_cast<uint32_t>(prm.tiles_p));
     prm.num_items = pl.tiles_p * pl.tiles_q * pl.splits;   // < 2^31: checked by tc_plan
-    prm.g_tmaps = nullptr;
-    prm.g_bs = nullptr;
-    prm.g_seg = nullptr;
-    prm.n_groups = 0;
-    prm.g_slots = 0;
     if (pl.swap) {
         switch (pl.bn) {
             case 16: return launch_variant<16, true>(tp, tq, tc, prm, stream);
@@ -1036,103 +967,6 @@ int launch_fp8_gemm_tc(const void* a, const float* a_s, const void* b, const flo
     }
     set_last_error("fp8_gemm: no tcgen05 variant for tile width %d", pl.bn);
     return DSV3_ERR_UNSUPPORTED;
-}
-
-
-// ---------------------------------------------------------------------------------------------
-// Grouped GEMM (MoE experts): one launch, group e multiplies rows [seg[e], seg[e+1]) of `a` with its
-// own weight.  The table holds, in device memory, n tensor maps followed by n scale pointers.
-// ---------------------------------------------------------------------------------------------
-size_t group_table_bytes(int n) { return static_cast<size_t>(n) * (sizeof(CUtensorMap) + sizeof(const float*)); }
-
-int build_group_table(void* table_dev, const void* const* weights, const float* const* scales, int n, int64_t N,
-                      int64_t K, cudaStream_t stream) {
-    if (n <= 0 || n > kMaxGroups) {
-        set_last_error("group table: between 1 and %d groups are supported (got %d)", kMaxGroups, n);
-        return DSV3_ERR_UNSUPPORTED;
-    }
-    if ((K % 16) != 0 || (reinterpret_cast<uintptr_t>(table_dev) % 64) != 0) {
-        set_last_error("group table: needs K %% 16 == 0 and a 64-byte aligned table");
-        return DSV3_ERR_UNSUPPORTED;
-    }
-    std::vector<uint8_t> host(group_table_bytes(n));
-    CUtensorMap* maps = reinterpret_cast<CUtensorMap*>(host.data());
-    const float** sp = reinterpret_cast<const float**>(host.data() + static_cast<size_t>(n) * sizeof(CUtensorMap));
-    for (int e = 0; e < n; ++e) {
-        if (!weights[e] || !scales[e] || (reinterpret_cast<uintptr_t>(weights[e]) % 16) != 0) {
-            set_last_error("group table: weight %d is null or not 16-byte aligned", e);
-            return DSV3_ERR_INVALID_ARGUMENT;
-        }
-        CUtensorMap m;
-        const int rc = make_tmap(&m, weights[e], N, K, kPRows);
-        if (rc != DSV3_OK) return rc;
-        memcpy(maps + e, &m, sizeof(m));
-        sp[e] = scales[e];
-    }
-    DSV3_CUDA_TRY(cudaMemcpyAsync(table_dev, host.data(), host.size(), cudaMemcpyHostToDevice, stream));
-    DSV3_CUDA_TRY(cudaStreamSynchronize(stream));   // `host` goes out of scope
-    return DSV3_OK;
-}
-
-int launch_fp8_gemm_grouped(const void* table_dev, int n, const void* a, const float* a_s, const int* seg_dev,
-                            int64_t rows_total, int64_t rows_hint, int64_t N, int64_t K, void* c, cudaStream_t stream) {
-    if (rows_total <= 0 || N <= 0) return DSV3_OK;
-    if (!tc_supported(a, a, c, rows_total, N, K) || n <= 0 || n > kMaxGroups) {
-        set_last_error("grouped fp8_gemm: needs K %% 16 == 0, 16-byte aligned a and c, and 1..%d groups", kMaxGroups);
-        return DSV3_ERR_UNSUPPORTED;
-    }
-    const int kc = static_cast<int>((K + kChunk - 1) / kChunk);
-    if (kc > scale_tab_chunks(32)) {
-        set_last_error("grouped fp8_gemm: K = %lld exceeds %d (scale table of the weight-major kernel)",
-                       static_cast<long long>(K), scale_tab_chunks(32) * kChunk);
-        return DSV3_ERR_UNSUPPORTED;
-    }
-    // the counts themselves live on the device: the token tile is sized for the expected load per group
-    const int64_t expect = (rows_hint > 0 && rows_hint < rows_total) ? rows_hint : rows_total;
-    const int64_t avg = (expect + n - 1) / n;
-    int bn = avg <= 16 ? 16 : (avg <= 32 ? 32 : 64);
-    if (kc > scale_tab_chunks(bn)) bn = 32;                // the 64-token variant's table is shorter
-    CUtensorMap tq, dummy;
-    int rc;
-    if ((rc = make_tmap(&tq, a, rows_total, K, bn)) != DSV3_OK) return rc;
-    memset(&dummy, 0, sizeof(dummy));
-    TcParams prm;
-    prm.a_s = a_s;
-    prm.b_s = nullptr;
-    prm.c = static_cast<__nv_bfloat16*>(c);
-    prm.tickets = nullptr;
-    prm.partials = nullptr;
-    prm.status = status_device_ptr();
-    if (!prm.status) return DSV3_ERR_CUDA;
-    prm.M = rows_total;
-    prm.N = N;
-    prm.kc = kc;
-    prm.tiles_p = static_cast<int>((N + kPRows - 1) / kPRows);
-    prm.tiles_q = 1;
-    prm.splits = 1;
-    prm.raster = 8;
-    prm.tma_store = 0;
-    prm.div_splits = make_fast_div(1);
-    prm.div_raster = make_fast_div(8);
-    prm.div_per_group = make_fast_div(8);
-    prm.div_tiles_p = make_fast_div(static_cast<uint32_t>(prm.tiles_p));
-    prm.g_tmaps = static_cast<const CUtensorMap*>(table_dev);
-    prm.g_bs = reinterpret_cast<const float* const*>(static_cast<const uint8_t*>(table_dev) +
-                                                     static_cast<size_t>(n) * sizeof(CUtensorMap));
-    prm.g_seg = seg_dev;
-    prm.n_groups = n;
-    prm.g_slots = static_cast<int>((rows_total + bn - 1) / bn) + n;
-    const int64_t items = static_cast<int64_t>(prm.tiles_p) * prm.g_slots;
-    if (items >= (1ll << 31)) {
-        set_last_error("grouped fp8_gemm: too many work items");
-        return DSV3_ERR_UNSUPPORTED;
-    }
-    prm.num_items = static_cast<int>(items);
-    switch (bn) {
-        case 16: return launch_variant<16, true>(dummy, tq, dummy, prm, stream);
-        case 32: return launch_variant<32, true>(dummy, tq, dummy, prm, stream);
-        default: return launch_variant<64, true>(dummy, tq, dummy, prm, stream);
-    }
 }
 
 // ---------------------------------------------------------------------------------------------

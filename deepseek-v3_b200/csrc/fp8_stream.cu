@@ -1,0 +1,1058 @@
+// Weight-streaming FP8 GEMM for sm_100a: few tokens per weight, every weight byte read once.  Used for the expert
+// loop of an expert layer (all local experts in one launch per projection) and for w1 / w3 of a small MLP, optionally
+// with SwiGLU and the quantisation in front of w2 folded into the epilogue.
+//
+// Replaces the per-expert act_quant + fp8_gemm calls of MoE.forward, inference/model.py:683-689 and :633, and
+// `F.silu(w1(x)) * w3(x)` followed by w2's act_quant, model.py:532 and :158-159.
+//
+// What bounds it: HBM.  An SM's share of the copy bandwidth is 43 GB/s, one 32 KB pair of weight blocks per 0.75 us.
+//   * A tile is TWO 128-row weight blocks (rows 128 j.. of w1 and of w3; or two neighbouring blocks of one weight)
+//     against up to BN tokens: the token tile crosses from L2 once per 256 weight rows instead of once per 128, and
+//     both halves of a SwiGLU pair meet in the same thread's registers.
+//   * Weights are the M operand (128 TMEM lanes), tokens the N operand: a tile of 16 tokens costs 16 columns.
+//   * Uneven split: where whole tiles would leave the last round of SMs mostly idle, the (tile, K chunk) space is cut
+//     into equal contiguous ranges, one per CTA.  A CTA then has at most two partial tiles (the head and the tail of
+//     its range); they are parked as fp32 (valid tokens only) and the CTA that takes a tile's last ticket adds them
+//     in K order, so the result does not depend on timing and nothing spins.
+//
+// Roles: warp 0 TMA producer, warp 1 MMA issuer (both converged, one elected lane issues), warps 2-3 fill the ring of
+// token scales, warps 4..11 promotion.  Promotion group g (four warps) owns token columns [g BN/2, (g+1) BN/2) of BOTH
+// blocks; a thread owns one weight row.  Per chunk: acc = fma(dot * a_s, b_s, acc), the reference's order
+// (kernel.py:162).
+//
+// Every mbarrier wait is bounded (tc_wait.cuh); producers wait for the last commits onto their barriers before the
+// CTA leaves.
+#include <cuda.h>
+
+#include <cstring>
+#include <vector>
+
+#include "common.cuh"
+#include "gemm_plan.cuh"
+#include "quant_math.cuh"
+#include "tc_wait.cuh"
+
+namespace dsv3 {
+
+namespace {
+
+constexpr int kNumThreads = 384;
+constexpr int kFirstPromoWarp = 4;
+constexpr int kPromoThreads = 256;
+constexpr int kTabThreads = 64;
+constexpr int kRegsControl = 40;
+constexpr int kRegsPromo = 232;
+static_assert(128 * kRegsControl + 256 * kRegsPromo <= 384 * 168, "register pool");
+constexpr int kMaxGroups = kMaxGroupsOfTable;
+constexpr int kMinUnits = 3;        // a split range is at least this many 32 KB chunks
+
+template <int BN>
+struct SCfg {
+    static constexpr bool kRows = BN >= 32;                           // tokens on the M side (fp8_rows_kernel)
+    static constexpr int kBox = BN < 32 ? BN : 32;                    // token rows per TMA box
+    static constexpr int kTokBytes = BN * kChunk;
+    static constexpr int kStageBytes = kTokBytes + 2 * kPRows * kChunk;   // tokens and two weight blocks of one chunk
+    static constexpr int kStages = BN <= 32 ? 6 : (BN <= 64 ? 5 : 4);
+    static constexpr int kSlotCols = kRows ? 2 * kPRows : 2 * BN;     // TMEM columns of one chunk product
+    static constexpr int kSlots = kRows ? 2 : 8;
+    static constexpr int kTmemCols = kSlots * kSlotCols;
+    // weights on the M side: ring of token scales, per-warp maxima and final scales
+    static constexpr int kTabChunks = 16;                             // K chunks per slot of the scale ring
+    static constexpr int kTabBytes = kRows ? 0 : 2 * kTabChunks * BN * 4;
+    static constexpr int kRedBytes = kRows ? 0 : (4 + 1) * BN * 4;
+    // tokens on the M side: exchange of SwiGLU halves / staging of results
+    static constexpr int kXBytes = kRows ? 2 * BN * 128 : 0;
+    // barriers, control words, group prefix and scan
+    static constexpr int kCtlBytes = (2 * kStages + 2 * kSlots + 4) * 8 + static_cast<int>(sizeof(Control)) + (kMaxGroups + 1 + 8) * 4;
+    static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kTabBytes + kRedBytes + kXBytes + kCtlBytes;
+    static_assert(kStageBytes >= kPRows * kChunk + kTokBytes || !kRows, "the MMA's 128 token rows stay inside the stage");
+    static_assert(kSmemBytes <= 232448, "shared memory per CTA");
+    static_assert(kSmemBytes > 116 * 1024, "one CTA per SM");
+    static_assert(kTmemCols >= 32 && kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "TMEM columns");
+};
+
+struct StreamParams {
+    // weights: block b of a tile comes from map / scale set b
+    const CUtensorMap* g_map[2];        // grouped: per-group maps, in global memory
+    const float* const* g_scale[2];     // grouped: per-group scale pointers, in global memory
+    const float* scale[2];              // one group
+    const int* seg;                     // grouped: [n_groups + 1] row offsets, in global memory
+    int n_groups;                       // 0: one ordinary weight
+    int M;                              // rows when n_groups == 0
+    int kc, nblk, tiles_p;              // K chunks, 128-row blocks of a weight, tiles per token tile
+    const float* a_s;                   // token scales: a_s[row * as_row + chunk * as_chunk]
+    int64_t as_row, as_chunk;
+    // results
+    __nv_bfloat16* c;                   // plain: bf16 [rows, N]
+    int64_t N;
+    int vec_store;                      // rows of c are 16-byte aligned
+    uint8_t* hq;                        // SwiGLU: e4m3 [rows, N]
+    float* hs;                          // SwiGLU: hs[row * hs_row + block * hs_blk]
+    int64_t hs_row, hs_blk;
+    int scale_fmt;
+    // split tiles
+    float* partials;                    // [CTA][2][2 * BN / 4][128] float4, or null: whole tiles only
+    int* tickets;                       // one per CTA, zero on entry and on exit
+    unsigned int* status;
+};
+
+struct Seg {          // a range of K chunks of one tile
+    int tile, c0, c1;
+    int row0, ntok;   // token rows
+    int group, p;     // weight, tile within the weight
+};
+
+// The CTA's share of the work and how tiles are split; every CTA derives the same plan from the same numbers.
+struct Plan {
+    int n_tiles, kc, G;      // G: CTAs that take part
+    bool split;
+    int64_t units;
+    __device__ __forceinline__ int64_t begin(int cta) const { return units * cta / G; }
+    __device__ __forceinline__ int owner(int64_t u) const { return static_cast<int>(((u + 1) * G - 1) / units); }
+};
+
+__device__ __forceinline__ Plan make_plan(int n_tiles, int kc, int ctas, bool may_split) {
+    Plan pl;
+    pl.n_tiles = n_tiles;
+    pl.kc = kc;
+    pl.G = ctas;
+    pl.units = static_cast<int64_t>(n_tiles) * kc;
+    const int rounds = (n_tiles + ctas - 1) / ctas;
+    // whole tiles keep at least 15 of 16 CTA-rounds busy: splitting would only add the parked partial tiles
+    pl.split = may_split && n_tiles > 0 && static_cast<int64_t>(n_tiles) * 16 < static_cast<int64_t>(rounds) * ctas * 15;
+    if (pl.split) {
+        const int64_t g = pl.units / kMinUnits;
+        if (g < pl.G) pl.G = g < 1 ? 1 : static_cast<int>(g);
+    }
+    return pl;
+}
+
+// Iterates over the segments of a CTA.
+template <int BN>
+struct Walker {
+    const StreamParams& p;
+    const Plan& pl;
+    const int* prefix;       // shared memory: token tiles of the groups before each group
+    int64_t u, u1;           // split: next unit and end of the range; whole tiles: next tile
+    __device__ __forceinline__ Walker(const StreamParams& p_, const Plan& pl_, const int* prefix_) : p(p_), pl(pl_), prefix(prefix_) {
+        const int cta = static_cast<int>(blockIdx.x);
+        if (pl.split) {
+            u = cta < pl.G ? pl.begin(cta) : 0;
+            u1 = cta < pl.G ? pl.begin(cta + 1) : 0;
+        } else {
+            u = cta;
+            u1 = pl.n_tiles;
+        }
+    }
+    __device__ __forceinline__ bool next(Seg& s) {
+        if (u >= u1) return false;
+        if (pl.split) {
+            s.tile = static_cast<int>(u / pl.kc);
+            s.c0 = static_cast<int>(u - static_cast<int64_t>(s.tile) * pl.kc);
+            s.c1 = static_cast<int>(min(static_cast<int64_t>(pl.kc), s.c0 + (u1 - u)));
+            u += s.c1 - s.c0;
+        } else {
+            s.tile = static_cast<int>(u);
+            s.c0 = 0;
+            s.c1 = pl.kc;
+            u += pl.G;
+        }
+        if (p.n_groups > 0) {
+            // group by binary search over prefix * tiles_p; inside a group the token tile runs fastest, so CTAs that
+            // work side by side share the weight blocks
+            int lo = 0, hi = p.n_groups;
+            while (hi - lo > 1) {
+                const int mid = (lo + hi) >> 1;
+                if (prefix[mid] * p.tiles_p <= s.tile) lo = mid; else hi = mid;
+            }
+            const int nq = prefix[lo + 1] - prefix[lo];
+            const int r = s.tile - prefix[lo] * p.tiles_p;
+            s.group = lo;
+            s.p = nq == 1 ? r : r / nq;
+            const int q = r - s.p * nq;
+            const int e1 = __ldg(p.seg + lo + 1);
+            s.row0 = __ldg(p.seg + lo) + q * BN;
+            s.ntok = min(BN, e1 - s.row0);
+        } else {
+            const int nq = (p.M + BN - 1) / BN;
+            s.group = 0;
+            s.p = nq == 1 ? s.tile : s.tile / nq;
+            const int q = s.tile - s.p * nq;
+            s.row0 = q * BN;
+            s.ntok = min(BN, p.M - s.row0);
+        }
+        return true;
+    }
+};
+
+// Token tiles per group and their exclusive prefix sum over the groups, into shared memory (all threads of the CTA;
+// the caller synchronises before prefix[] is read).
+template <int BN>
+__device__ __forceinline__ void prefix_groups(const StreamParams& p, int* prefix, int* scan, int warp, int lane) {
+    int v = 0;
+    if (threadIdx.x < kMaxGroups) {
+        const int e = threadIdx.x;
+        if (e < p.n_groups) v = (__ldg(p.seg + e + 1) - __ldg(p.seg + e) + BN - 1) / BN;
+        int inc = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += t;
+        }
+        if (lane == 31) scan[warp] = inc;
+        v = inc - v;
+    }
+    __syncthreads();
+    if (threadIdx.x < kMaxGroups) {
+        for (int w = 0; w < warp; ++w) v += scan[w];
+        prefix[threadIdx.x] = v;
+    }
+    if (threadIdx.x == 0) {
+        int tot = 0;
+        for (int w = 0; w < kMaxGroups / 32; ++w) tot += scan[w];
+        prefix[kMaxGroups] = tot;        // groups beyond n_groups hold no tiles
+    }
+}
+
+// While the kernel before this one drains (programmatic dependent launch), the first weight boxes of an ordinary problem
+// come into L2 (the point of coherence: were the predecessor still writing them, the loads after the wait would see
+// its data all the same).  One thread.
+template <int BN, bool kSwiglu>
+__device__ __forceinline__ void prefetch_weights(const StreamParams& p, const void* w0, const void* w1, const int* prefix, int n) {
+    const Plan pl = make_plan(p.tiles_p * ((p.M + BN - 1) / BN), p.kc, static_cast<int>(gridDim.x), p.partials != nullptr);
+    Walker<BN> wk(p, pl, prefix);
+    Seg s;
+    if (wk.next(s)) {
+        const int r0 = (kSwiglu ? s.p : 2 * s.p) * kPRows;
+        for (int k = s.c0; k < min(s.c1, s.c0 + n); ++k) {
+            tma_prefetch_l2_2d(w0, k * kChunk, r0);
+            if (kSwiglu || 2 * s.p + 1 < p.nblk) tma_prefetch_l2_2d(w1, k * kChunk, kSwiglu ? r0 : r0 + kPRows);
+        }
+    }
+}
+
+// The TMA producer (one converged warp).  Stage: [BN token rows][block 0][block 1] of one K chunk; of the tokens only
+// the boxes that hold any of the tile's rows are fetched.
+template <int BN, bool kSwiglu>
+__device__ __forceinline__ void produce(const StreamParams& p, const Plan& pl, const int* prefix, const void* w0, const void* w1,
+                                        const void* ta, uint32_t tiles, uint32_t bar0, Control* ctl) {
+    using C = SCfg<BN>;
+    constexpr int NS = C::kStages;
+    Walker<BN> wk(p, pl, prefix);
+    Seg s;
+    uint32_t g = 0;
+    bool ok = true;
+    while (ok && wk.next(s)) {
+        const void* m0 = p.n_groups > 0 ? static_cast<const void*>(p.g_map[0] + s.group) : w0;
+        const void* m1 = p.n_groups > 0 ? static_cast<const void*>(p.g_map[1] + s.group) : w1;
+        const int r0 = (kSwiglu ? s.p : 2 * s.p) * kPRows;
+        const int r1 = kSwiglu ? r0 : r0 + kPRows;
+        const bool two = kSwiglu || 2 * s.p + 1 < p.nblk;
+        const int boxes = (s.ntok + C::kBox - 1) / C::kBox;
+        const uint32_t bytes = (two ? 2u : 1u) * kPRows * kChunk + static_cast<uint32_t>(boxes) * C::kBox * kChunk;
+        for (int k = s.c0; k < s.c1; ++k, ++g) {
+            const int st = g % NS;
+            const uint32_t full = bar0 + 8u * st, empty = bar0 + 8u * (NS + st);
+            ok = __all_sync(0xffffffffu, bounded_wait(empty, ((g / NS) & 1u) ^ 1u, ctl, p.status, 1, g));
+            if (!ok) break;
+            if (elect_one()) {
+                const uint32_t dst = tiles + st * C::kStageBytes;
+                mbar_arrive_expect_tx(full, bytes);
+                tma_load_2d(dst + C::kTokBytes, m0, k * kChunk, r0, full);
+                if (two) tma_load_2d(dst + C::kTokBytes + kPRows * kChunk, m1, k * kChunk, r1, full);
+                for (int b = 0; b < boxes; ++b) tma_load_2d(dst + b * C::kBox * kChunk, ta, k * kChunk, s.row0 + b * C::kBox, full);
+            }
+            __syncwarp();
+        }
+    }
+    // nothing else waits for the commits onto the empty[] barriers of the last chunks: none may be in flight
+    // when the CTA leaves (it would land in whatever CTA gets this shared memory next)
+    for (uint32_t d = (g > static_cast<uint32_t>(NS) ? g - NS : 0u); ok && d < g; ++d)
+        ok = __all_sync(0xffffffffu, bounded_wait(bar0 + 8u * (NS + d % NS), (d / NS) & 1u, ctl, p.status, 1, d));
+}
+
+// Ticket of a partial tile: parks are done; returns whether this CTA holds the tile's last ticket (promotion threads).
+__device__ __forceinline__ bool last_part(const StreamParams& p, Control* ctl, int first, int last) {
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    if (threadIdx.x == kFirstPromoWarp * 32) {
+        int tk;
+        // releases the parked tile (cumulative over the barrier) and acquires the other parts
+        asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(tk) : "l"(p.tickets + first) : "memory");
+        if (tk == last - first) p.tickets[first] = 0;
+        ctl->ticket[0] = tk;
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    const bool mine = ctl->ticket[0] == last - first;
+    asm volatile("bar.sync 1, 256;" ::: "memory");            // the slot may be overwritten from here on
+    return mine;
+}
+
+__device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_base, uint32_t cols) {
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (ctl->abort_flag) {
+        // give copies and MMAs that were already issued time to land before shared memory and TMEM are released
+        const uint64_t t0 = global_timer_ns();
+        while (global_timer_ns() - t0 < 200000ull) __nanosleep(1000);
+        __syncthreads();
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        tc_dealloc(tmem_base, cols);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// Up to 16 tokens per tile: weights on the M side.
+// ---------------------------------------------------------------------------------------------------------------------
+template <int BN, bool kSwiglu>
+__global__ void __launch_bounds__(kNumThreads, 1)
+fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
+                  const __grid_constant__ CUtensorMap tmap_a, const StreamParams p) {
+    using C = SCfg<BN>;
+    constexpr int NS = C::kStages, NT = C::kSlots, TC = C::kTabChunks;
+    constexpr int CT = BN / 2;             // token columns per promotion thread and block
+
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t tiles = (raw + 1023u) & ~1023u;
+    uint8_t* gen = smem_raw + (tiles - raw);
+    float* tab = reinterpret_cast<float*>(gen + NS * C::kStageBytes);                 // [2][TC][BN]
+    float* red = reinterpret_cast<float*>(gen + NS * C::kStageBytes + C::kTabBytes);  // [4][BN] maxima, then [BN] scales
+    uint64_t* bars = reinterpret_cast<uint64_t*>(gen + NS * C::kStageBytes + C::kTabBytes + C::kRedBytes);
+    Control* ctl = reinterpret_cast<Control*>(bars + 2 * NS + 2 * NT + 4);
+    int* prefix = reinterpret_cast<int*>(ctl + 1);
+    int* scan = prefix + kMaxGroups + 1;                                              // [8] warp totals
+    const uint32_t bar0 = smem_u32(bars);
+    auto full_bar = [&](int s) { return bar0 + 8u * s; };
+    auto empty_bar = [&](int s) { return bar0 + 8u * (NS + s); };
+    auto tfull_bar = [&](int s) { return bar0 + 8u * (2 * NS + s); };
+    auto tempty_bar = [&](int s) { return bar0 + 8u * (2 * NS + NT + s); };
+    auto sfull_bar = [&](int s) { return bar0 + 8u * (2 * NS + 2 * NT + s); };        // slot of the scale ring is filled
+    auto sempty_bar = [&](int s) { return bar0 + 8u * (2 * NS + 2 * NT + 2 + s); };
+
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+    const int lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < NS; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        for (int s = 0; s < NT; ++s) {
+            mbar_init(tfull_bar(s), 1);
+            mbar_init(tempty_bar(s), kPromoThreads / 32);
+        }
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(sfull_bar(s), kTabThreads);
+            mbar_init(sempty_bar(s), kPromoThreads / 32);
+        }
+        ctl->abort_flag = 0;
+        mbar_fence_init();
+        tma_prefetch_desc(&tmap_a);
+        if (p.n_groups == 0) {
+            tma_prefetch_desc(&tmap_w0);
+            tma_prefetch_desc(&tmap_w1);
+        }
+    }
+    if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
+    if (threadIdx.x == 0 && p.n_groups == 0) prefetch_weights<BN, kSwiglu>(p, &tmap_w0, &tmap_w1, prefix, NS);
+    griddep_launch_dependents();
+    griddep_wait();
+    if (p.n_groups > 0) prefix_groups<BN>(p, prefix, scan, warp, lane);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = ctl->tmem_base;
+    const int n_tiles = p.tiles_p * (p.n_groups > 0 ? prefix[kMaxGroups] : (p.M + BN - 1) / BN);
+    const Plan pl = make_plan(n_tiles, p.kc, static_cast<int>(gridDim.x), p.partials != nullptr);
+
+    if (warp == 0) {
+        produce<BN, kSwiglu>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a, tiles, bar0, ctl);
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMA issuer
+        constexpr uint32_t idesc = umma_idesc_e4m3_f32(kPRows, BN);
+        Walker<BN> wk(p, pl, prefix);
+        Seg s;
+        uint32_t g = 0;
+        bool ok = true;
+        while (ok && wk.next(s)) {
+            const bool two = kSwiglu || 2 * s.p + 1 < p.nblk;
+            for (int k = s.c0; k < s.c1; ++k, ++g) {
+                const int st = g % NS, ts = g % NT;
+                ok = __all_sync(0xffffffffu, bounded_wait(tempty_bar(ts), ((g / NT) & 1u) ^ 1u, ctl, p.status, 3, g) &&
+                                             bounded_wait(full_bar(st), (g / NS) & 1u, ctl, p.status, 2, g));
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t sp = tiles + st * C::kStageBytes;
+                const uint64_t dt = umma_desc_k_major_sw128(sp);
+                const uint64_t d0 = umma_desc_k_major_sw128(sp + C::kTokBytes);
+                const uint64_t d1 = umma_desc_k_major_sw128(sp + C::kTokBytes + kPRows * kChunk);
+                const uint32_t d_tmem = tmem_base + ts * C::kSlotCols;
+                if (elect_one()) {
+#pragma unroll
+                    for (int kk = 0; kk < kChunk / 32; ++kk) tc_mma_f8(d_tmem, d0 + 2u * kk, dt + 2u * kk, idesc, kk > 0 ? 1u : 0u);
+                    if (two) {
+#pragma unroll
+                        for (int kk = 0; kk < kChunk / 32; ++kk)
+                            tc_mma_f8(d_tmem + BN, d1 + 2u * kk, dt + 2u * kk, idesc, kk > 0 ? 1u : 0u);
+                    }
+                    tc_commit(empty_bar(st));
+                    tc_commit(tfull_bar(ts));
+                }
+                __syncwarp();
+            }
+        }
+    } else if (warp < kFirstPromoWarp) {
+        // ------------------------------------------------------------ token scales, TC chunks at a time
+        Walker<BN> wk(p, pl, prefix);
+        Seg s;
+        uint32_t t = 0;          // ring counter
+        bool ok = true;
+        const int tid = threadIdx.x - 64;
+        while (ok && wk.next(s)) {
+            for (int k = s.c0; k < s.c1; k += TC, ++t) {
+                const int sl = t & 1;
+                ok = __all_sync(0xffffffffu, bounded_wait(sempty_bar(sl), ((t >> 1) & 1u) ^ 1u, ctl, p.status, 7, t));
+                if (!ok) break;
+                const int n = min(TC, s.c1 - k);
+                float* dst = tab + sl * TC * BN;
+                // columns beyond ntok keep what they held: they multiply products nobody reads
+                for (int i = tid; i < n * BN; i += kTabThreads) {
+                    const int ch = i / BN, col = i - ch * BN;
+                    if (col < s.ntok) dst[i] = __ldg(p.a_s + (s.row0 + col) * p.as_row + (k + ch) * p.as_chunk);
+                }
+                mbar_arrive(sfull_bar(sl));
+            }
+        }
+    } else {
+        // ------------------------------------------------------------ promotion + epilogue
+        const int grp = (warp - kFirstPromoWarp) >> 2;
+        const int col0 = grp * CT;
+        const int quarter = warp & 3;
+        const int row = quarter * 32 + lane;                    // weight row within a block (TMEM lane)
+        const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + col0;
+        Walker<BN> wk(p, pl, prefix);
+        Seg s;
+        uint32_t g = 0, t = 0;
+        bool ok = true;
+        float2 acc[2][CT / 2];
+        uint32_t v[2 * CT];
+        // acc[b] += (v * a_s) * b_s over this thread's CT columns
+        auto fold = [&](const uint32_t* vv, const float* as, float bs, float2* a) {
+            const float2 b2 = make_float2(bs, bs);
+            const float4* as4 = reinterpret_cast<const float4*>(as);
+#pragma unroll
+            for (int j = 0; j < CT / 4; ++j) {
+                const float4 a4 = as4[j];
+                const float2 lo = __fmul2_rn(make_float2(__uint_as_float(vv[4 * j]), __uint_as_float(vv[4 * j + 1])), make_float2(a4.x, a4.y));
+                const float2 hi = __fmul2_rn(make_float2(__uint_as_float(vv[4 * j + 2]), __uint_as_float(vv[4 * j + 3])), make_float2(a4.z, a4.w));
+                a[2 * j] = __ffma2_rn(lo, b2, a[2 * j]);
+                a[2 * j + 1] = __ffma2_rn(hi, b2, a[2 * j + 1]);
+            }
+        };
+        auto load_cols = [&](uint32_t taddr, uint32_t* vv) {
+            if constexpr (CT == 8) tc_ld_x8(taddr, vv);
+            else tc_ld_x16(taddr, vv);
+        };
+        while (ok && wk.next(s)) {
+            const bool two = kSwiglu || 2 * s.p + 1 < p.nblk;
+            const float* b0 = (p.n_groups > 0 ? p.g_scale[0][s.group] : p.scale[0]) + static_cast<int64_t>(kSwiglu ? s.p : 2 * s.p) * p.kc;
+            const float* b1 = (p.n_groups > 0 ? p.g_scale[1][s.group] : p.scale[1]) +
+                              static_cast<int64_t>(kSwiglu ? s.p : (two ? 2 * s.p + 1 : 2 * s.p)) * p.kc;
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int j = 0; j < CT / 2; ++j) acc[b][j] = make_float2(0.0f, 0.0f);
+            float bs0 = __ldg(b0 + s.c0), bs1 = __ldg(b1 + s.c0);
+            int in_tab = 0;                         // chunk within the slot of the scale ring
+            const int n_ch = s.c1 - s.c0;
+            for (int k = 0; k < n_ch; ++k, ++g) {
+                const int sl = t & 1;
+                if (in_tab == 0) {
+                    ok = __all_sync(0xffffffffu, bounded_wait_lean(sfull_bar(sl), (t >> 1) & 1u, ctl, p.status, 8, t));
+                    if (!ok) break;
+                }
+                const float* as = tab + (sl * TC + in_tab) * BN + col0;
+                const int ts = g % NT;
+                ok = __all_sync(0xffffffffu, bounded_wait_lean(tfull_bar(ts), (g / NT) & 1u, ctl, p.status, 4, g));
+                if (!ok) break;
+                tc_fence_after();
+                const uint32_t taddr = t_lane + ts * C::kSlotCols;
+                load_cols(taddr, v);
+                load_cols(taddr + BN, v + CT);
+                const int kn = min(k + 1, n_ch - 1);                      // scales of the next chunk (the last re-reads its own)
+                const float nb0 = __ldg(b0 + s.c0 + kn), nb1 = __ldg(b1 + s.c0 + kn);
+                tc_wait_ld();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(tempty_bar(ts));
+                fold(v, as, bs0, acc[0]);
+                fold(v + CT, as, bs1, acc[1]);
+                bs0 = nb0;
+                bs1 = nb1;
+                if (++in_tab == TC || k == n_ch - 1) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(sempty_bar(sl));
+                    in_tab = 0;
+                    ++t;
+                }
+            }
+            if (!ok) break;
+
+            float* accf = reinterpret_cast<float*>(acc);                  // [2][CT]
+            const int my = min(max(s.ntok - col0, 0), CT);                // valid token columns of this thread
+            if (n_ch < p.kc) {
+                // part of a tile: park the valid columns, take a ticket; the last part of the tile adds all parts
+                // in K order and goes on to write the result
+                const int cta = static_cast<int>(blockIdx.x);
+                const int64_t ut = static_cast<int64_t>(s.tile) * pl.kc;
+                const int first = pl.owner(ut), last = pl.owner(ut + pl.kc - 1);
+                constexpr int kTileVec = 2 * BN / 4 * kPRows;             // float4 per parked tile
+                float4* base = reinterpret_cast<float4*>(p.partials) + (col0 / 4) * kPRows + row;
+                auto part = [&](int c) { return base + (static_cast<int64_t>(c) * 2 + (pl.begin(c) >= ut ? 0 : 1)) * kTileVec; };
+                {
+                    float4* dst = part(cta);
+#pragma unroll
+                    for (int b = 0; b < 2; ++b)
+#pragma unroll
+                        for (int j = 0; j < CT / 4; ++j)
+                            if (4 * j < my)
+                                __stcg(dst + (b * (BN / 4) + j) * kPRows, make_float4(accf[b * CT + 4 * j], accf[b * CT + 4 * j + 1],
+                                                                                      accf[b * CT + 4 * j + 2], accf[b * CT + 4 * j + 3]));
+                }
+                if (!last_part(p, ctl, first, last)) continue;
+#pragma unroll
+                for (int j = 0; j < 2 * CT; ++j) accf[j] = 0.0f;
+#pragma unroll 2
+                for (int c = first; c <= last; ++c) {
+                    const float4* src = part(c);
+#pragma unroll
+                    for (int b = 0; b < 2; ++b)
+#pragma unroll
+                        for (int j = 0; j < CT / 4; ++j)
+                            if (4 * j < my) {
+                                const float4 f = __ldcg(src + (b * (BN / 4) + j) * kPRows);
+                                accf[b * CT + 4 * j] += f.x;
+                                accf[b * CT + 4 * j + 1] += f.y;
+                                accf[b * CT + 4 * j + 2] += f.z;
+                                accf[b * CT + 4 * j + 3] += f.w;
+                            }
+                }
+            }
+            const int64_t tok0 = s.row0 + col0;
+            if constexpr (!kSwiglu) {
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const int64_t n = static_cast<int64_t>(2 * s.p + b) * kPRows + row;
+                    if (n < p.N) {
+#pragma unroll
+                        for (int j = 0; j < CT; ++j)
+                            if (j < my) p.c[(tok0 + j) * p.N + n] = __float2bfloat16_rn(accf[b * CT + j]);
+                    }
+                }
+            } else {
+                // h = bf16(bf16(silu(h1)) * h3), then act_quant over the tile's 128 columns of every token: the
+                // maximum is taken across the lanes of a warp and, through shared memory, across the group's warps.
+                float* gred = red + col0;
+#pragma unroll
+                for (int j = 0; j < CT; ++j) {
+                    if (j < my) {
+                        const float h1 = __bfloat162float(__float2bfloat16_rn(accf[j]));
+                        const float h3 = __bfloat162float(__float2bfloat16_rn(accf[CT + j]));
+                        const float h = __bfloat162float(__float2bfloat16_rn(silu_exact(h1) * h3));
+                        accf[j] = h;
+                        const float a = fabsf(h);
+                        const uint32_t m = __reduce_max_sync(0xffffffffu, a == a ? __float_as_uint(a) : 0u);
+                        if (lane == 0) gred[quarter * BN + j] = __uint_as_float(m);
+                    }
+                }
+                asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
+                const int gt = threadIdx.x & 127;
+                if (gt < my) {
+                    const float m = fmaxf(fmaxf(gred[gt], gred[BN + gt]), fmaxf(gred[2 * BN + gt], gred[3 * BN + gt]));
+                    const float sc = scale_from_amax(m, p.scale_fmt);
+                    gred[4 * BN + gt] = sc;
+                    p.hs[(tok0 + gt) * p.hs_row + s.p * p.hs_blk] = sc;
+                }
+                asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
+                uint8_t* out = p.hq + tok0 * p.N + static_cast<int64_t>(s.p) * kPRows + row;
+#pragma unroll
+                for (int j = 0; j < CT; ++j) {
+                    if (j < my) {
+                        const float sc = gred[4 * BN + j];
+                        const float qv = p.scale_fmt == DSV3_SCALE_FMT_FP32 ? __fmul_rn(accf[j], rcp_approx(sc)) : div_full(accf[j], sc);
+                        out[j * p.N] = static_cast<uint8_t>(cvt_e4m3x2(qv, 0.0f) & 0xFFu);
+                    }
+                }
+                // the next tile's maxima must not overtake this tile's scales
+                asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
+            }
+        }
+    }
+
+    teardown(ctl, warp, tmem_base, C::kTmemCols);
+}
+
+// ---------------------------------------------------------------------------------------------------------------------
+// 32, 64 or 128 tokens per tile: tokens on the M side (128 TMEM lanes, of which the tile's rows are used), the two weight
+// blocks side by side on the N side.
+//
+// Why the roles change: with weights on the M side a token's scale varies along a thread's registers, so every chunk
+// costs a shared-memory load per two FMAs and the SwiGLU epilogue needs maxima across 128 threads; for 64 and 128
+// tokens that, not HBM, was the bound (1100 cycles per chunk and 12000 per tile: 1983 us for w1 / w3 of 256 experts of
+// 7168 x 2048 with 16384 rows, where the weights take 1165 us).  Here a thread owns one token row and 128 columns of
+// one block: one scale product per chunk and thread, and a row's maximum is two threads' business.  The MMA costs 512
+// cycles per chunk whatever the number of tokens, which the 1300 cycles that the weights take to arrive hide.
+// ---------------------------------------------------------------------------------------------------------------------
+template <int BN, bool kSwiglu>
+__global__ void __launch_bounds__(kNumThreads, 1)
+fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
+                const __grid_constant__ CUtensorMap tmap_a, const StreamParams p) {
+    using C = SCfg<BN>;
+    constexpr int NS = C::kStages, NT = C::kSlots;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t raw = smem_u32(smem_raw);
+    const uint32_t tiles = (raw + 1023u) & ~1023u;
+    uint8_t* gen = smem_raw + (tiles - raw);
+    uint8_t* xbuf = gen + NS * C::kStageBytes;                                 // [2][BN][128 bytes]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(xbuf + C::kXBytes);
+    Control* ctl = reinterpret_cast<Control*>(bars + 2 * NS + 2 * NT);
+    int* prefix = reinterpret_cast<int*>(ctl + 1);
+    int* scan = prefix + kMaxGroups + 1;
+    const uint32_t bar0 = smem_u32(bars);
+    auto full_bar = [&](int s) { return bar0 + 8u * s; };
+    auto empty_bar = [&](int s) { return bar0 + 8u * (NS + s); };
+    auto tfull_bar = [&](int s) { return bar0 + 8u * (2 * NS + s); };
+    auto tempty_bar = [&](int s) { return bar0 + 8u * (2 * NS + NT + s); };
+
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+    const int lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < NS; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        for (int s = 0; s < NT; ++s) {
+            mbar_init(tfull_bar(s), 1);
+            mbar_init(tempty_bar(s), kPromoThreads / 32);
+        }
+        ctl->abort_flag = 0;
+        mbar_fence_init();
+        tma_prefetch_desc(&tmap_a);
+        if (p.n_groups == 0) {
+            tma_prefetch_desc(&tmap_w0);
+            tma_prefetch_desc(&tmap_w1);
+        }
+    }
+    if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
+    if (threadIdx.x == 0 && p.n_groups == 0) prefetch_weights<BN, kSwiglu>(p, &tmap_w0, &tmap_w1, prefix, NS);
+    griddep_launch_dependents();
+    griddep_wait();
+    if (p.n_groups > 0) prefix_groups<BN>(p, prefix, scan, warp, lane);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = ctl->tmem_base;
+    const int n_tiles = p.tiles_p * (p.n_groups > 0 ? prefix[kMaxGroups] : (p.M + BN - 1) / BN);
+    const Plan pl = make_plan(n_tiles, p.kc, static_cast<int>(gridDim.x), p.partials != nullptr);
+
+    if (warp < kFirstPromoWarp) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
+        if (warp == 0) {
+            produce<BN, kSwiglu>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a, tiles, bar0, ctl);
+        } else if (warp == 1) {
+            // -------------------------------------------------------- MMA issuer
+            Walker<BN> wk(p, pl, prefix);
+            Seg s;
+            uint32_t g = 0;
+            bool ok = true;
+            while (ok && wk.next(s)) {
+                const bool two = kSwiglu || 2 * s.p + 1 < p.nblk;
+                const uint32_t idesc = two ? umma_idesc_e4m3_f32(kPRows, 2 * kPRows) : umma_idesc_e4m3_f32(kPRows, kPRows);
+                for (int k = s.c0; k < s.c1; ++k, ++g) {
+                    const int st = g % NS, ts = g % NT;
+                    ok = __all_sync(0xffffffffu, bounded_wait(tempty_bar(ts), ((g / NT) & 1u) ^ 1u, ctl, p.status, 3, g) &&
+                                                 bounded_wait(full_bar(st), (g / NS) & 1u, ctl, p.status, 2, g));
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t sp = tiles + st * C::kStageBytes;
+                    // 128 token rows are multiplied; the rows beyond the tile's lie in the weight blocks behind the
+                    // tokens (still inside the stage) and produce lanes that nobody reads
+                    const uint64_t da = umma_desc_k_major_sw128(sp);
+                    const uint64_t db = umma_desc_k_major_sw128(sp + C::kTokBytes);
+                    const uint32_t d_tmem = tmem_base + ts * 256;
+                    if (elect_one()) {
+#pragma unroll
+                        for (int kk = 0; kk < kChunk / 32; ++kk) tc_mma_f8(d_tmem, da + 2u * kk, db + 2u * kk, idesc, kk > 0 ? 1u : 0u);
+                        tc_commit(empty_bar(st));
+                        tc_commit(tfull_bar(ts));
+                    }
+                    __syncwarp();
+                }
+            }
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsPromo));
+        // ------------------------------------------------------------ promotion + epilogue
+        const int grp = (warp - kFirstPromoWarp) >> 2;          // weight block
+        const int quarter = warp & 3;
+        const int row = quarter * 32 + lane;                    // token row of the tile (TMEM lane)
+        const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + grp * kPRows;
+        uint8_t* my_x = xbuf + grp * (BN * 128);                // this group's half of the exchange buffer
+        uint8_t* other_x = xbuf + (1 - grp) * (BN * 128);
+        Walker<BN> wk(p, pl, prefix);
+        Seg s, ahead;
+        uint32_t g = 0;
+        bool ok = true;
+        float2 acc[64];
+        uint32_t v[64];
+        auto fold = [&](float sc, int off) {
+            const float2 sc2 = make_float2(sc, sc);
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+                acc[off + j] = __ffma2_rn(make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), sc2, acc[off + j]);
+        };
+        auto release = [&](int ts) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(tempty_bar(ts));
+        };
+        // Scales of this row for four chunks are in flight or in registers, each register re-used for the chunk four
+        // further on: a chunk takes 0.3 us to fold, a load that misses L1 about
+        // 0.6 us, and with one chunk of look-ahead every chunk waited for it (1330 cycles instead of 700).  A tile's
+        // first scales are requested before the result of the tile before it is written.
+        const float *as = nullptr, *bs = nullptr;
+        float ra[4], rb;         // rb: the weight block's scale of the next chunk (32 chunks to a cache line: L1)
+        auto scales_of = [&](const Seg& q) {
+            const int blk = kSwiglu ? q.p : 2 * q.p + grp;
+            as = p.a_s + (q.row0 + min(row, q.ntok - 1)) * p.as_row + q.c0 * p.as_chunk;
+            bs = (p.n_groups > 0 ? p.g_scale[grp][q.group] : p.scale[grp]) + static_cast<int64_t>(min(blk, p.nblk - 1)) * p.kc + q.c0;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int k = min(i, q.c1 - q.c0 - 1);
+                ra[i] = __ldg(as + k * p.as_chunk);
+            }
+            rb = __ldg(bs);
+        };
+        bool more = wk.next(ahead);
+        if (more) scales_of(ahead);
+        while (ok && more) {
+            s = ahead;
+            const int blk = kSwiglu ? s.p : 2 * s.p + grp;
+            const bool active = quarter * 32 < s.ntok && blk < p.nblk;     // uniform in the warp
+            const int n_ch = s.c1 - s.c0;
+#pragma unroll
+            for (int j = 0; j < 64; ++j) acc[j] = make_float2(0.0f, 0.0f);
+            for (int k0 = 0; ok && k0 < n_ch; k0 += 4) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int k = k0 + i;
+                    if (!ok || k >= n_ch) break;
+                    const int ts = g % NT;
+                    ok = __all_sync(0xffffffffu, bounded_wait_lean(tfull_bar(ts), (g / NT) & 1u, ctl, p.status, 4, g));
+                    ++g;
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (!active) {
+                        release(ts);
+                        continue;
+                    }
+                    const uint32_t taddr = t_lane + ts * 256;
+                    tc_ld_x64(taddr, v);
+                    const float sc = ra[i] * rb;
+                    ra[i] = __ldg(as + min(k + 4, n_ch - 1) * p.as_chunk);
+                    rb = __ldg(bs + min(k + 1, n_ch - 1));
+                    tc_wait_ld();
+                    fold(sc, 0);
+                    tc_ld_x64(taddr + 64, v);
+                    tc_wait_ld();
+                    release(ts);
+                    fold(sc, 32);
+                }
+            }
+            if (!ok) break;
+            more = wk.next(ahead);
+            if (more) scales_of(ahead);
+
+            if (n_ch < p.kc) {
+                // part of a tile: park the valid rows, take a ticket; the last part of the tile adds all parts in K
+                // order and goes on to write the result
+                const int cta = static_cast<int>(blockIdx.x);
+                const int64_t ut = static_cast<int64_t>(s.tile) * pl.kc;
+                const int first = pl.owner(ut), last = pl.owner(ut + pl.kc - 1);
+                constexpr int kTileVec = 256 * BN / 4;                     // float4 per parked tile: [64 column groups][BN rows]
+                float4* base = reinterpret_cast<float4*>(p.partials) + grp * 32 * BN + row;
+                auto part = [&](int c) { return base + (static_cast<int64_t>(c) * 2 + (pl.begin(c) >= ut ? 0 : 1)) * kTileVec; };
+                const bool mine_row = active && row < s.ntok;
+                if (mine_row) {
+                    float4* dst = part(cta);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) __stcg(dst + j * BN, make_float4(acc[2 * j].x, acc[2 * j].y, acc[2 * j + 1].x, acc[2 * j + 1].y));
+                }
+                if (!last_part(p, ctl, first, last)) continue;
+#pragma unroll
+                for (int j = 0; j < 64; ++j) acc[j] = make_float2(0.0f, 0.0f);
+                if (mine_row) {
+                    for (int c = first; c <= last; ++c) {
+                        const float4* src = part(c);
+#pragma unroll
+                        for (int j0 = 0; j0 < 32; j0 += 16) {              // sixteen loads in flight
+                            float4 f[16];
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) f[j] = __ldcg(src + (j0 + j) * BN);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) {
+                                acc[2 * (j0 + j)] = __fadd2_rn(acc[2 * (j0 + j)], make_float2(f[j].x, f[j].y));
+                                acc[2 * (j0 + j) + 1] = __fadd2_rn(acc[2 * (j0 + j) + 1], make_float2(f[j].z, f[j].w));
+                            }
+                        }
+                    }
+                }
+            }
+            if (quarter * 32 >= s.ntok) continue;
+            if constexpr (!kSwiglu) {
+                if (!active) continue;
+                // 32 rows x 64 columns at a time through the warp's own 4 KB, so that global stores cover whole lines
+                uint8_t* wbuf = my_x + quarter * (32 * 128);
+                const int64_t n0 = static_cast<int64_t>(blk) * kPRows;
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    __syncwarp();
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const float2* a = acc + half * 32 + c * 4;
+                        *reinterpret_cast<uint4*>(wbuf + lane * 128 + ((c ^ (lane & 7)) << 4)) =
+                            make_uint4(pack_bf16x2(a[0].x, a[0].y), pack_bf16x2(a[1].x, a[1].y), pack_bf16x2(a[2].x, a[2].y), pack_bf16x2(a[3].x, a[3].y));
+                    }
+                    __syncwarp();
+                    const int piece = lane & 7;
+                    const int64_t n = n0 + half * 64 + piece * 8;
+#pragma unroll
+                    for (int r0 = 0; r0 < 32; r0 += 4) {
+                        const int r = r0 + (lane >> 3);
+                        if (quarter * 32 + r >= s.ntok) continue;
+                        const uint4 o = *reinterpret_cast<const uint4*>(wbuf + r * 128 + ((piece ^ (r & 7)) << 4));
+                        __nv_bfloat16* dst = p.c + (static_cast<int64_t>(s.row0) + quarter * 32 + r) * p.N + n;
+                        if (p.vec_store && n + 8 <= p.N) {
+                            *reinterpret_cast<uint4*>(dst) = o;
+                        } else {
+                            const uint32_t w4[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                            for (int e = 0; e < 8; ++e)
+                                if (n + e < p.N) reinterpret_cast<uint16_t*>(dst)[e] = static_cast<uint16_t>(w4[e >> 1] >> (16 * (e & 1)));
+                        }
+                    }
+                }
+            } else {
+                // h1 of a row sits in one group's thread, h3 in the other's: each gives the other half of its columns
+                // (bf16, as the operators would have written them) and computes h = bf16(bf16(silu(h1)) * h3) for the 64
+                // columns it keeps.  The two threads' maxima meet in the exchange slots they have just read.
+                const int give = 1 - grp;                                  // column half handed over
+                const uint32_t slot = static_cast<uint32_t>(row) * 128;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const float2* a = acc + c * 4;
+                    const float2* b = acc + 32 + c * 4;
+                    const uint4 lo = make_uint4(pack_bf16x2(a[0].x, a[0].y), pack_bf16x2(a[1].x, a[1].y), pack_bf16x2(a[2].x, a[2].y), pack_bf16x2(a[3].x, a[3].y));
+                    const uint4 hi = make_uint4(pack_bf16x2(b[0].x, b[0].y), pack_bf16x2(b[1].x, b[1].y), pack_bf16x2(b[2].x, b[2].y), pack_bf16x2(b[3].x, b[3].y));
+                    *reinterpret_cast<uint4*>(my_x + slot + ((c ^ (row & 7)) << 4)) = give ? hi : lo;
+                    v[4 * c] = give ? lo.x : hi.x;
+                    v[4 * c + 1] = give ? lo.y : hi.y;
+                    v[4 * c + 2] = give ? lo.z : hi.z;
+                    v[4 * c + 3] = give ? lo.w : hi.w;
+                }
+                asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
+                float m = 0.0f;
+                // Rolled loops over a register file that turns by one group per trip: unrolled, this epilogue was longer
+                // than the instruction cache holds and cost 8000-14000 cycles per tile.  (Rows beyond the tile's hold
+                // products of weights with weights: not worth silu's exact path.)
+                if (row < s.ntok) {
+#pragma unroll 1
+                    for (int c = 0; c < 8; ++c) {
+                        const uint4 mine = make_uint4(v[0], v[1], v[2], v[3]);
+                        const uint4 theirs = *reinterpret_cast<const uint4*>(other_x + slot + ((c ^ (row & 7)) << 4));
+                        const uint4 h = grp == 0 ? swiglu8(mine, theirs) : swiglu8(theirs, mine);
+#pragma unroll
+                        for (int e = 0; e < 28; ++e) v[e] = v[e + 4];
+                        v[28] = h.x;
+                        v[29] = h.y;
+                        v[30] = h.z;
+                        v[31] = h.w;
+                        m = fmaxf(m, amax8(h));
+                    }
+                }
+                // only this thread reads slot `row` of the other group's half
+                *reinterpret_cast<float*>(other_x + slot) = m;
+                asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
+                m = fmaxf(m, *reinterpret_cast<const float*>(my_x + slot));
+                if (row < s.ntok) {
+                    const float scale = scale_from_amax(m, p.scale_fmt);
+                    const int64_t tok = static_cast<int64_t>(s.row0) + row;
+                    if (grp == 0) p.hs[tok * p.hs_row + s.p * p.hs_blk] = scale;
+                    uint4* out = reinterpret_cast<uint4*>(p.hq + tok * p.N + static_cast<int64_t>(s.p) * kPRows + grp * 64);
+#pragma unroll 1
+                    for (int c = 0; c < 4; ++c) {
+                        const uint4 a = make_uint4(v[0], v[1], v[2], v[3]);
+                        const uint4 b = make_uint4(v[4], v[5], v[6], v[7]);
+#pragma unroll
+                        for (int e = 0; e < 24; ++e) v[e] = v[e + 8];
+                        uint2 qa, qb;
+                        if (p.scale_fmt == DSV3_SCALE_FMT_FP32) {
+                            qa = quant8<true>(a, scale);
+                            qb = quant8<true>(b, scale);
+                        } else {
+                            qa = quant8<false>(a, scale);
+                            qb = quant8<false>(b, scale);
+                        }
+                        out[c] = make_uint4(qa.x, qa.y, qb.x, qb.y);
+                    }
+                }
+            }
+        }
+    }
+    teardown(ctl, warp, tmem_base, C::kTmemCols);
+}
+
+template <int BN, bool kSwiglu>
+int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta, const StreamParams& prm, int64_t tiles_bound,
+                   cudaStream_t stream) {
+    using C = SCfg<BN>;
+    constexpr auto pick = [] {
+        if constexpr (C::kRows) return fp8_rows_kernel<BN, kSwiglu>;
+        else return fp8_stream_kernel<BN, kSwiglu>;
+    };
+    auto kern = pick();
+    static bool configured[64] = {};
+    int dev = 0;
+    DSV3_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) {
+        set_last_error("fp8_gemm: device ordinal %d is outside the supported range", dev);
+        return DSV3_ERR_UNSUPPORTED;
+    }
+    if (!configured[dev]) {
+        DSV3_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+        configured[dev] = true;
+    }
+    int64_t grid = num_sms();
+    const int64_t most = prm.partials ? tiles_bound * prm.kc : tiles_bound;      // no more CTAs than there can be work for
+    if (grid > most) grid = most;
+    DSV3_CUDA_TRY(launch_dependent(kern, dim3(static_cast<unsigned>(grid)), dim3(kNumThreads), C::kSmemBytes, stream, w0, w1, ta, prm));
+    return DSV3_OK;
+}
+
+}  // namespace
+
+// Token tile for an expected load per group: the smallest that holds it with room for uneven routing.  A group that
+// needs a second tile reads its weights a second time (from L2), which costs more than wider tiles do.
+int stream_tile(int64_t rows_per_group) {
+    return rows_per_group <= 4 ? 16 : (rows_per_group <= 14 ? 32 : (rows_per_group <= 32 ? 64 : 128));
+}
+
+size_t stream_workspace_bytes(int64_t rows_per_group) {
+    const int bn = stream_tile(rows_per_group);
+    return DSV3_WORKSPACE_HEADER_BYTES + static_cast<size_t>(num_sms()) * 2 * (2 * bn) * kPRows * sizeof(float);
+}
+
+int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
+    StreamParams prm;
+    memset(&prm, 0, sizeof(prm));
+    CUtensorMap w0, w1, ta;
+    memset(&w0, 0, sizeof(w0));
+    memset(&w1, 0, sizeof(w1));
+    int rc;
+    const int n = q.n_groups > 0 ? q.n_groups : 1;
+    const int bn = stream_tile((q.rows_expected + n - 1) / n);
+    const int box = bn < 32 ? bn : 32;
+    if ((rc = make_tmap(&ta, q.a, q.rows, q.K, box)) != DSV3_OK) return rc;
+    prm.kc = static_cast<int>((q.K + kChunk - 1) / kChunk);
+    prm.nblk = static_cast<int>((q.N + kPRows - 1) / kPRows);
+    prm.tiles_p = q.swiglu ? prm.nblk : (prm.nblk + 1) / 2;
+    if (q.n_groups > 0) {
+        for (int b = 0; b < 2; ++b) {
+            const void* tbl = (b == 1 && q.swiglu) ? q.table1 : q.table0;
+            prm.g_map[b] = static_cast<const CUtensorMap*>(tbl);
+            prm.g_scale[b] = reinterpret_cast<const float* const*>(static_cast<const uint8_t*>(tbl) + static_cast<size_t>(q.n_groups) * sizeof(CUtensorMap));
+        }
+        prm.seg = q.seg;
+    } else {
+        if ((rc = make_tmap(&w0, q.w0, q.N, q.K, kPRows)) != DSV3_OK) return rc;
+        if ((rc = make_tmap(&w1, q.swiglu ? q.w1 : q.w0, q.N, q.K, kPRows)) != DSV3_OK) return rc;
+        prm.scale[0] = q.w0_s;
+        prm.scale[1] = q.swiglu ? q.w1_s : q.w0_s;
+    }
+    prm.n_groups = q.n_groups;
+    prm.M = static_cast<int>(q.rows);
+    prm.a_s = q.a_s;
+    prm.as_row = q.as_row;
+    prm.as_chunk = q.as_chunk;
+    prm.c = static_cast<__nv_bfloat16*>(q.c);
+    prm.N = q.N;
+    prm.vec_store = (q.N % 8) == 0 && (reinterpret_cast<uintptr_t>(q.c) % 16) == 0;
+    prm.hq = static_cast<uint8_t*>(q.hq);
+    prm.hs = q.hs;
+    prm.hs_row = q.hs_row;
+    prm.hs_blk = q.hs_blk;
+    prm.scale_fmt = q.scale_fmt;
+    prm.status = status_device_ptr();
+    if (!prm.status) return DSV3_ERR_CUDA;
+    const size_t need = stream_workspace_bytes((q.rows_expected + n - 1) / n);
+    if (need > 0 && q.workspace && q.workspace_bytes >= need && (reinterpret_cast<uintptr_t>(q.workspace) % 256) == 0) {
+        prm.tickets = static_cast<int*>(q.workspace);
+        prm.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(q.workspace) + DSV3_WORKSPACE_HEADER_BYTES);
+    }
+    // token tiles: at most one partly filled tile per group on top of the full ones, and never more groups than rows
+    const int64_t slots = q.n_groups > 0 ? q.rows / bn + (q.n_groups < q.rows ? q.n_groups : q.rows) : (q.rows + bn - 1) / bn;
+    const int64_t tiles_bound = slots * prm.tiles_p;
+    if (tiles_bound * prm.kc >= (1ll << 31)) {
+        set_last_error("fp8 stream GEMM: %lld tiles of %d K chunks are more than the work-item counter holds",
+                       static_cast<long long>(tiles_bound), prm.kc);
+        return DSV3_ERR_UNSUPPORTED;
+    }
+#define DSV3_STREAM_CASE(BN_) \
+    case BN_: return q.swiglu ? launch_variant<BN_, true>(w0, w1, ta, prm, tiles_bound, stream) : launch_variant<BN_, false>(w0, w1, ta, prm, tiles_bound, stream)
+    switch (bn) {
+        DSV3_STREAM_CASE(16);
+        DSV3_STREAM_CASE(32);
+        DSV3_STREAM_CASE(64);
+        DSV3_STREAM_CASE(128);
+    }
+#undef DSV3_STREAM_CASE
+    return DSV3_ERR_UNSUPPORTED;
+}
+
+// The table holds, in device memory, n tensor maps followed by n scale pointers.
+size_t group_table_bytes(int n) { return static_cast<size_t>(n) * (sizeof(CUtensorMap) + sizeof(const float*)); }
+
+int build_group_table(void* table_dev, const void* const* weights, const float* const* scales, int n, int64_t N,
+                      int64_t K, cudaStream_t stream) {
+    if (n <= 0 || n > kMaxGroupsOfTable) {
+        set_last_error("group table: between 1 and %d groups are supported (got %d)", kMaxGroupsOfTable, n);
+        return DSV3_ERR_UNSUPPORTED;
+    }
+    if ((K % 16) != 0 || (reinterpret_cast<uintptr_t>(table_dev) % 64) != 0) {
+        set_last_error("group table: needs K %% 16 == 0 and a 64-byte aligned table");
+        return DSV3_ERR_UNSUPPORTED;
+    }
+    std::vector<uint8_t> host(group_table_bytes(n));
+    CUtensorMap* maps = reinterpret_cast<CUtensorMap*>(host.data());
+    const float** sp = reinterpret_cast<const float**>(host.data() + static_cast<size_t>(n) * sizeof(CUtensorMap));
+    for (int e = 0; e < n; ++e) {
+        if (!weights[e] || !scales[e] || (reinterpret_cast<uintptr_t>(weights[e]) % 16) != 0) {
+            set_last_error("group table: weight %d is null or not 16-byte aligned", e);
+            return DSV3_ERR_INVALID_ARGUMENT;
+        }
+        CUtensorMap m;
+        const int rc = make_tmap(&m, weights[e], N, K, kPRows);
+        if (rc != DSV3_OK) return rc;
+        memcpy(maps + e, &m, sizeof(m));
+        sp[e] = scales[e];
+    }
+    DSV3_CUDA_TRY(cudaMemcpyAsync(table_dev, host.data(), host.size(), cudaMemcpyHostToDevice, stream));
+    DSV3_CUDA_TRY(cudaStreamSynchronize(stream));   // `host` goes out of scope
+    return DSV3_OK;
+}
+
+}  // namespace dsv3

@@ -48,12 +48,36 @@ bool small_linear_supported(const void* act, const void* w, const void* c, int64
 int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, const void* w, const float* w_s, int64_t M,
                             int64_t N, int64_t K, int scale_fmt, void* c, cudaStream_t stream);
 
-// Grouped GEMM over per-group weights (MoE experts).
+// Weight-streaming GEMM (fp8_stream.cu): groups of rows against per-group weights, or one weight; optionally with
+// SwiGLU of two weights and quantisation of the product in the epilogue.
+struct StreamGemm {
+    const void* a;                     // e4m3 [rows, K]
+    const float* a_s;                  // token scales at a_s[row * as_row + chunk * as_chunk]
+    int64_t as_row, as_chunk;
+    int64_t rows, rows_expected, N, K;
+    int n_groups;                      // 0: one weight (w0, w0_s, w1, w1_s); otherwise tables and seg
+    const void *table0, *table1;       // group tables; table1 only with swiglu
+    const int* seg;                    // device memory
+    const void *w0, *w1;               // e4m3 [N, K]; w1 only with swiglu
+    const float *w0_s, *w1_s;
+    bool swiglu;
+    void* c;                           // bf16 [rows, N]                   -- plain
+    void* hq;                          // e4m3 [rows, N]                   -- swiglu
+    float* hs;                         // hs[row * hs_row + block * hs_blk] -- swiglu
+    int64_t hs_row, hs_blk;
+    int scale_fmt;
+    void* workspace;                   // stream_workspace_bytes(), or null: tiles are not split
+    size_t workspace_bytes;
+};
+int stream_tile(int64_t rows_per_group);
+size_t stream_workspace_bytes(int64_t rows_per_group);
+int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream);
+
+// Table of the weights of up to 256 groups: tensor maps followed by scale pointers, in device memory.
+constexpr int kMaxGroupsOfTable = 256;
 size_t group_table_bytes(int n);
 int build_group_table(void* table_dev, const void* const* weights, const float* const* scales, int n, int64_t N,
                       int64_t K, cudaStream_t stream);
-int launch_fp8_gemm_grouped(const void* table_dev, int n, const void* a, const float* a_s, const int* seg_dev,
-                            int64_t rows_total, int64_t rows_hint, int64_t N, int64_t K, void* c, cudaStream_t stream);
 
 // One thread waits for an mbarrier phase that never completes; the bounded wait gives up after limit_ns.
 int launch_bounded_wait_selftest(uint64_t limit_ns, cudaStream_t stream);

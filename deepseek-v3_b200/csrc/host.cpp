@@ -21,6 +21,7 @@
 
 #include <array>
 #include <exception>
+#include <memory>
 #include <vector>
 
 #include "dsv3_b200.h"
@@ -264,6 +265,16 @@ void count(PyObject* key) {
     Py_XDECREF(now);
 }
 
+void remember(const at::Tensor& x, int64_t block, int fmt, bool assume_no_inplace, const at::Tensor& q, const at::Tensor& s) {
+    const bool counted = !x.is_inference();
+    if (!counted && !assume_no_inplace) return;
+    if (g_memo.size() > 1) g_memo.pop_back();
+    g_memo.insert(g_memo.begin(),
+                  Remembered{decltype(Remembered::x)(x.getIntrusivePtr()), x.const_data_ptr(), {x.sizes().begin(), x.sizes().end()},
+                             counted ? static_cast<int64_t>(x._version()) : -1, block, fmt,
+                             c10::cuda::getCurrentCUDAStream(x.device().index()).stream(), q, s});
+}
+
 std::pair<at::Tensor, at::Tensor> quantise_remembered(const at::Tensor& x, int64_t block, int fmt, bool assume_no_inplace) {
     const bool counted = !x.is_inference();
     if ((!counted && !assume_no_inplace) || !x.is_cuda()) {
@@ -284,9 +295,142 @@ std::pair<at::Tensor, at::Tensor> quantise_remembered(const at::Tensor& x, int64
     }
     auto r = quantise(x, block, fmt);
     count(g_key_calls);
-    if (g_memo.size() > 1) g_memo.pop_back();
-    g_memo.insert(g_memo.begin(), Remembered{decltype(Remembered::x)(x.getIntrusivePtr()), x.const_data_ptr(), {x.sizes().begin(), x.sizes().end()},
-                                             version, block, fmt, stream, r.first, r.second});
+    remember(x, block, fmt, assume_no_inplace, r.first, r.second);
+    return r;
+}
+
+// ------------------------------------------------------------------ expert layer
+// Device tables of the local experts' projections and what they depend on.  The tables hold addresses, so before every
+// pass the host must know that the experts are still the ones they were built from.  Looking every weight up through
+// its module costs 0.3 us each (230 us for 256 experts); instead the dictionaries the look-ups went through are watched
+// for changes, and only the weights' storage addresses are compared (`param.data = ...` changes no dictionary).
+uint64_t g_dict_changes = 1;         // bumped whenever a watched dictionary changes
+int g_watcher = -1;
+
+#if PY_VERSION_HEX >= 0x030C0000
+int on_dict_change(PyDict_WatchEvent, PyObject*, PyObject*, PyObject*) {
+    ++g_dict_changes;
+    return 0;
+}
+#endif
+
+struct LookUp {
+    PyObject *dict, *key, *value;    // dict[key] is value (dict kept alive; value compared by identity)
+};
+
+struct Experts {
+    int n, start, fmt;
+    int64_t dim, inter;
+    at::Tensor table1, table3, table2;
+    PyObject* list;                  // the experts when they are a plain list, else null
+    std::vector<PyObject*> members;  // its members [start, start + n)
+    std::vector<LookUp> lookups;
+    uint64_t seen = 0;               // g_dict_changes when the look-ups were last verified
+    std::vector<std::pair<at::Tensor, const void*>> weights;
+    ~Experts() {
+        Py_XDECREF(list);
+        for (PyObject* m : members) Py_DECREF(m);
+        for (LookUp& l : lookups) {
+            Py_DECREF(l.dict);
+            Py_DECREF(l.key);
+            Py_DECREF(l.value);
+        }
+    }
+    bool current() {
+        if (list) {
+            for (int i = 0; i < n; ++i)
+                if (start + i >= PyList_GET_SIZE(list) || PyList_GET_ITEM(list, start + i) != members[i]) return false;
+        }
+        if (g_watcher < 0 || seen != g_dict_changes) {
+            for (const LookUp& l : lookups)
+                if (PyDict_GetItemWithError(l.dict, l.key) != l.value) return false;
+            seen = g_dict_changes;
+        }
+        for (const auto& w : weights)
+            if (w.first.const_data_ptr() != w.second) return false;
+        return true;
+    }
+};
+
+const char* kExpertsName = "dsv3_b200.experts";
+void free_experts(PyObject* c) { delete static_cast<Experts*>(PyCapsule_GetPointer(c, kExpertsName)); }
+Experts* experts_arg(PyObject* c) {
+    auto* e = static_cast<Experts*>(PyCapsule_GetPointer(c, kExpertsName));
+    if (!e) throw PythonError{};
+    return e;
+}
+
+// Result of the expert GEMMs of one pass, before the combination: one allocation, carved up.
+struct Routed {
+    at::Tensor arena, x;
+    int64_t T, dim;
+    int topk;
+    const void *o, *w;
+    const int32_t* pos;
+};
+const char* kRoutedName = "dsv3_b200.routed";
+void free_routed(PyObject* c) { delete static_cast<Routed*>(PyCapsule_GetPointer(c, kRoutedName)); }
+
+std::unique_ptr<Routed> run_experts(Experts& e, const at::Tensor& x_in, const at::Tensor& weights_in, const at::Tensor& indices_in,
+                                    int64_t n_routed, bool assume_no_inplace) {
+    if (indices_in.dim() != 2 || weights_in.sizes() != indices_in.sizes())
+        raise(PyExc_ValueError, "routing weights and indices must both be [tokens, top-k]");
+    const c10::Device dev = require_cuda(x_in, weights_in, indices_in, e.table1);
+    if (x_in.scalar_type() != at::kBFloat16) raise(PyExc_NotImplementedError, "the expert layer takes bfloat16 activations");
+    const at::Tensor x = x_in.is_contiguous() ? x_in : x_in.contiguous();
+    at::Tensor indices = indices_in.scalar_type() == at::kLong ? indices_in : indices_in.to(at::kLong);
+    at::Tensor weights = (weights_in.scalar_type() == at::kBFloat16 || weights_in.scalar_type() == at::kFloat) ? weights_in : weights_in.to(at::kFloat);
+    if (!indices.is_contiguous()) indices = indices.contiguous();
+    if (!weights.is_contiguous()) weights = weights.contiguous();
+    const int64_t T = indices.size(0), topk = indices.size(1), P = T * topk, dim = e.dim, inter = e.inter;
+    if (x.dim() != 2 || x.size(0) != T || x.size(1) != dim) raise(PyExc_ValueError, "activations must be [tokens, dim]");
+    auto r = std::make_unique<Routed>();
+    r->T = T;
+    r->dim = dim;
+    r->topk = static_cast<int>(topk);
+    r->x = x;
+    // this rank owns n of the layer's experts and, on average, that share of the pairs
+    const int64_t hint = n_routed > e.n ? std::max<int64_t>(1, (P * e.n + n_routed - 1) / n_routed) : 0;
+    int64_t at = 0;
+    auto take = [&](int64_t bytes) {
+        const int64_t here = at;
+        at += (bytes + 255) & ~int64_t(255);
+        return here;
+    };
+    const int64_t o_seg = take(4 * (e.n + 1)), o_pos = take(4 * P), o_w = take(2 * P), o_xq = take(P * dim), o_xs = take(4 * P * (dim / 128)),
+                  o_hq = take(P * inter), o_hs = take(4 * P * (inter / 128)), o_o = take(2 * P * dim);
+    r->arena = new_cuda({std::max<int64_t>(at, 1)}, at::kByte, dev);
+    uint8_t* base = static_cast<uint8_t*>(r->arena.data_ptr());
+    r->o = base + o_o;
+    r->w = base + o_w;
+    r->pos = reinterpret_cast<const int32_t*>(base + o_pos);
+    if (P == 0) return r;
+    at::Tensor xq = new_cuda(x.sizes(), at::kFloat8_e4m3fn, dev), xs = new_cuda_last(x, dim / 128, at::kFloat);
+    void* ws = nullptr;
+    size_t ws_bytes = 0;
+    if (const size_t need = dsv3_gemm_rows_workspace_bytes(e.n, P, hint)) {
+        const at::Tensor& w = workspace(dev, need);
+        ws = w.data_ptr();
+        ws_bytes = static_cast<size_t>(w.numel());
+    }
+    auto* seg = reinterpret_cast<int32_t*>(base + o_seg);
+    auto* xs_t = reinterpret_cast<float*>(base + o_xs);
+    auto* hs_t = reinterpret_cast<float*>(base + o_hs);
+    const void *t1 = e.table1.const_data_ptr(), *t3 = e.table3.const_data_ptr(), *t2 = e.table2.const_data_ptr();
+    const void *xp = x.const_data_ptr(), *wp = weights.const_data_ptr();
+    const int bf16 = weights.scalar_type() == at::kBFloat16;
+    const auto* ip = static_cast<const int64_t*>(indices.const_data_ptr());
+    void* xqp = xq.data_ptr();
+    float* xsp = static_cast<float*>(xs.data_ptr());
+    call_library(dev, [&](dsv3_stream_t st) {
+        int rc = dsv3_moe_dispatch(xp, T, dim, ip, wp, bf16, r->topk, e.start, e.n, e.fmt, seg, reinterpret_cast<int32_t*>(base + o_pos),
+                                   base + o_w, xqp, xsp, base + o_xq, xs_t, st);
+        if (rc == DSV3_OK)
+            rc = dsv3_swiglu_gemm_rows(t1, t3, e.n, base + o_xq, xs_t, seg, P, hint, inter, dim, e.fmt, base + o_hq, hs_t, ws, ws_bytes, st);
+        if (rc == DSV3_OK) rc = dsv3_fp8_gemm_rows(t2, e.n, base + o_hq, hs_t, seg, P, hint, dim, inter, base + o_o, ws, ws_bytes, st);
+        return rc;
+    });
+    if (x_in.is_contiguous()) remember(x_in, 128, e.fmt, assume_no_inplace, xq, xs);
     return r;
 }
 
@@ -419,6 +563,75 @@ PyObject* py_quantise_remembered(PyObject*, PyObject* const* args, Py_ssize_t n)
     });
 }
 
+// (n, start, dim, inter, scale_fmt, table1, table3, table2, list or None, members, look-ups [(dict, key, value)], weights)
+PyObject* py_experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        want_args(n, 12);
+        auto e = std::make_unique<Experts>();
+        e->list = nullptr;
+        e->n = static_cast<int>(int_arg(args[0]));
+        e->start = static_cast<int>(int_arg(args[1]));
+        e->dim = int_arg(args[2]);
+        e->inter = int_arg(args[3]);
+        e->fmt = scale_fmt_arg(args[4]);
+        e->table1 = tensor_arg(args[5]);
+        e->table3 = tensor_arg(args[6]);
+        e->table2 = tensor_arg(args[7]);
+        if (PyList_Check(args[8])) e->list = Py_NewRef(args[8]);
+        if (!PyList_Check(args[9]) || !PyList_Check(args[10]) || !PyList_Check(args[11]) || PyList_GET_SIZE(args[9]) != e->n)
+            raise(PyExc_TypeError, "members, look-ups and weights are lists");
+        for (Py_ssize_t i = 0; i < PyList_GET_SIZE(args[9]); ++i) e->members.push_back(Py_NewRef(PyList_GET_ITEM(args[9], i)));
+        for (Py_ssize_t i = 0; i < PyList_GET_SIZE(args[10]); ++i) {
+            PyObject *d, *k, *v;
+            if (!PyArg_ParseTuple(PyList_GET_ITEM(args[10], i), "O!OO", &PyDict_Type, &d, &k, &v)) throw PythonError{};
+            e->lookups.push_back({Py_NewRef(d), Py_NewRef(k), Py_NewRef(v)});
+#if PY_VERSION_HEX >= 0x030C0000
+            if (g_watcher >= 0 && PyDict_Watch(g_watcher, d) != 0) throw PythonError{};
+#endif
+        }
+        for (Py_ssize_t i = 0; i < PyList_GET_SIZE(args[11]); ++i) {
+            const at::Tensor& w = tensor_arg(PyList_GET_ITEM(args[11], i));
+            e->weights.emplace_back(w, w.const_data_ptr());
+        }
+        return PyCapsule_New(e.release(), kExpertsName, free_experts);
+    });
+}
+
+PyObject* py_experts_current(PyObject*, PyObject* capsule) {
+    return guarded([&]() -> PyObject* { return PyBool_FromLong(experts_arg(capsule)->current()); });
+}
+
+// (experts, x, weights, indices, n_routed, assume_no_inplace) -> result to hand to `combine`
+PyObject* py_run_experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        want_args(n, 6);
+        auto r = run_experts(*experts_arg(args[0]), tensor_arg(args[1]), tensor_arg(args[2]), tensor_arg(args[3]), int_arg(args[4]),
+                             PyObject_IsTrue(args[5]) == 1);
+        return PyCapsule_New(r.release(), kRoutedName, free_routed);
+    });
+}
+
+// (result of run_experts, z or None): the tokens' weighted sums, plus z
+PyObject* py_combine(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        want_args(n, 2);
+        auto* r = static_cast<Routed*>(PyCapsule_GetPointer(args[0], kRoutedName));
+        if (!r) throw PythonError{};
+        const c10::Device dev = r->arena.device();
+        const void* zp = nullptr;
+        if (args[1] != Py_None) {
+            const at::Tensor& z = tensor_arg(args[1]);
+            if (!z.is_contiguous() || z.scalar_type() != at::kBFloat16 || z.device() != dev || z.numel() != r->T * r->dim)
+                raise(PyExc_ValueError, "z must be a contiguous bfloat16 tensor of the layer's output size on the same device");
+            zp = z.const_data_ptr();
+        }
+        at::Tensor y = new_cuda({r->T, r->dim}, at::kBFloat16, dev);
+        void* yp = y.data_ptr();
+        call_library(dev, [&](dsv3_stream_t st) { return dsv3_moe_combine_add(r->o, r->pos, r->w, zp, r->T, r->topk, r->dim, yp, st); });
+        return wrap(std::move(y));
+    });
+}
+
 PyObject* py_set_stats(PyObject*, PyObject* dict) {
     Py_XSETREF(g_stats, Py_NewRef(dict));
     Py_RETURN_NONE;
@@ -452,6 +665,12 @@ PyMethodDef methods[] = {
      "(x, weight, block_size, scale_fmt, assume_no_inplace, fused_max_rows, fused_max_bytes)"},
     {"quantise_remembered", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_quantise_remembered)), METH_FASTCALL,
      "(x, block_size, scale_fmt, assume_no_inplace)"},
+    {"experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_experts)), METH_FASTCALL,
+     "(n, start, dim, inter, scale_fmt, table1, table3, table2, list, members, lookups, weights)"},
+    {"experts_current", py_experts_current, METH_O, "whether the experts are still those the tables were built from"},
+    {"run_experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_run_experts)), METH_FASTCALL,
+     "(experts, x, weights, indices, n_routed, assume_no_inplace)"},
+    {"combine", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_combine)), METH_FASTCALL, "(routed, z)"},
     {"set_stats", py_set_stats, METH_O, "dict whose counters linear() keeps"},
     {"forget", py_forget, METH_NOARGS, "drop the remembered quantisations"},
     {"clear_workspaces", py_clear_workspaces, METH_NOARGS, "zero the ticket headers of all split-K workspaces"},
@@ -468,6 +687,10 @@ PyMODINIT_FUNC PyInit__dsv3_host(void) {
     g_key_reused = PyUnicode_InternFromString("act_quant_reused");
     g_key_fused = PyUnicode_InternFromString("fused_linear_calls");
     g_attr_scale = PyUnicode_InternFromString("scale");
+#if PY_VERSION_HEX >= 0x030C0000
+    g_watcher = PyDict_AddWatcher(on_dict_change);
+    if (g_watcher < 0) PyErr_Clear();       // all watchers taken: look-ups are verified on every pass
+#endif
     PyObject* torch = PyImport_ImportModule("torch");
     g_oom_class = torch ? PyObject_GetAttrString(torch, "OutOfMemoryError") : nullptr;
     Py_XDECREF(torch);

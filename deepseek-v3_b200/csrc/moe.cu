@@ -4,6 +4,7 @@
 //   idx, top = where(indices == i) ; y[idx] += expert(x[idx]) * weights[idx, top, None]
 // with bf16 rounding after the product and after every accumulation, in ascending expert order.
 #include "gemm_plan.cuh"
+#include "quant_math.cuh"
 
 namespace dsv3 {
 
@@ -12,29 +13,43 @@ namespace {
 constexpr int kThreads = 256;
 
 // y[t, :] = sum over the token's experts, in ascending expert order, of bf16(o[pos, :] * w), each
-// partial sum rounded to bf16 (the arithmetic of `y[idx] += ...` on bf16 tensors).
+// partial sum rounded to bf16 (the arithmetic of `y[idx] += ...` on bf16 tensors); with z, y + z follows (model.py:693).
 //   pos [T, topk] int32: row of `o` holding expert output for the j-th smallest expert id of token t, or -1
 //   w   [T, topk] bf16 : routing weight of that pair
-__global__ void __launch_bounds__(kThreads) moe_combine_kernel(const __nv_bfloat16* __restrict__ o,
+// Bound by HBM: 2 dim (topk + 1 or 2) bytes per token.  The rows of up to eight experts are requested before the first
+// is used; with one load in flight per thread the same pass ran at 3.3 TB/s (79 us for 2048 tokens, top-8, dim 7168).
+constexpr int kCombineBatch = 8;
+
+__global__ void __launch_bounds__(kThreads, 4) moe_combine_kernel(const __nv_bfloat16* __restrict__ o,
                                                                 const int* __restrict__ pos,
                                                                 const __nv_bfloat16* __restrict__ w,
-                                                                __nv_bfloat16* __restrict__ y, int64_t T, int topk,
-                                                                int64_t dim) {
-    const int64_t groups_per_row = dim >> 3;                       // 8 bf16 = 16 bytes per thread
-    const int64_t total = T * groups_per_row;
-    const int64_t stride = static_cast<int64_t>(gridDim.x) * kThreads;
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x; i < total; i += stride) {
-        const int64_t t = i / groups_per_row;
-        const int64_t d = (i - t * groups_per_row) << 3;
-        float acc[8];
+                                                                const __nv_bfloat16* __restrict__ z,
+                                                                __nv_bfloat16* __restrict__ y, int topk, int64_t dim,
+                                                                FastDiv ctas_per_row) {
+    griddep_launch_dependents();
+    griddep_wait();
+    const uint32_t t = fast_div(blockIdx.x, ctas_per_row);
+    const int64_t d = (static_cast<int64_t>(blockIdx.x - t * ctas_per_row.d) * kThreads + threadIdx.x) << 3;   // 8 bf16 = 16 bytes per thread
+    if (d >= dim) return;
+    float acc[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] = 0.0f;
-        for (int j = 0; j < topk; ++j) {
-            const int r = __ldg(pos + t * topk + j);
-            if (r < 0) continue;
-            const float wf = __bfloat162float(w[t * topk + j]);
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(o + static_cast<int64_t>(r) * dim + d));
-            const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+    for (int e = 0; e < 8; ++e) acc[e] = 0.0f;
+    const uint4 zv = z ? __ldcs(reinterpret_cast<const uint4*>(z + t * dim + d)) : make_uint4(0u, 0u, 0u, 0u);
+    const int* tp = pos + static_cast<int64_t>(t) * topk;
+    const __nv_bfloat16* tw = w + static_cast<int64_t>(t) * topk;
+    for (int j0 = 0; j0 < topk; j0 += kCombineBatch) {
+        int r[kCombineBatch];
+        uint4 v[kCombineBatch];
+#pragma unroll
+        for (int j = 0; j < kCombineBatch; ++j) r[j] = j0 + j < topk ? __ldg(tp + j0 + j) : -1;
+#pragma unroll
+        for (int j = 0; j < kCombineBatch; ++j)
+            if (r[j] >= 0) v[j] = __ldcs(reinterpret_cast<const uint4*>(o + static_cast<int64_t>(r[j]) * dim + d));
+#pragma unroll
+        for (int j = 0; j < kCombineBatch; ++j) {
+            if (r[j] < 0) continue;
+            const float wf = __bfloat162float(tw[j0 + j]);
+            const uint32_t words[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float lo = __uint_as_float(words[e] << 16), hi = __uint_as_float(words[e] & 0xFFFF0000u);
@@ -44,9 +59,165 @@ __global__ void __launch_bounds__(kThreads) moe_combine_kernel(const __nv_bfloat
                 acc[2 * e + 1] = __bfloat162float(__float2bfloat16_rn(acc[2 * e + 1] + ph));
             }
         }
-        uint4 out = make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]), pack_bf16x2(acc[4], acc[5]),
-                               pack_bf16x2(acc[6], acc[7]));
-        *reinterpret_cast<uint4*>(y + t * dim + d) = out;
+    }
+    if (z) {
+        const uint32_t words[4] = {zv.x, zv.y, zv.z, zv.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            acc[2 * e] += __uint_as_float(words[e] << 16);
+            acc[2 * e + 1] += __uint_as_float(words[e] & 0xFFFF0000u);
+        }
+    }
+    *reinterpret_cast<uint4*>(y + t * dim + d) = make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]),
+                                                            pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
+}
+
+// Everything in front of the expert GEMMs in one launch: groups the (token, expert) pairs by local expert, orders every
+// token's pairs by expert id, quantises every token once (act_quant's arithmetic) and writes its FP8 row to the row of
+// each of its local pairs.  Replaces moe_route, act_quant and two gathers (and a conversion of the routing weights).
+//
+// A CTA owns `tpc` consecutive tokens and needs the rows of their pairs: the first row of every expert (all pairs) plus
+// how many pairs of the expert belong to earlier tokens.  Instead of a second launch or a grid barrier every CTA counts
+// all pairs itself, 8 bytes per pair from L2 into shared-memory histograms (one CTA doing all the bookkeeping took 59 us
+// for 16 K pairs); one large CTA per SM keeps that to 16 pairs per thread.  Several CTAs along y share a CTA's tokens when there are few tokens; they
+// derive the same rows, because a pair's place among the CTA's own pairs is counted in order there.
+constexpr int kDispMaxExperts = 256;
+constexpr int kDispPairs = 1024;          // own pairs of a CTA
+constexpr int kDispOrdered = 64;          // own pairs up to which rows are assigned in order
+constexpr int kDispUnroll = 4;
+constexpr int kDispThreads = 1024;
+
+struct DispatchParams {
+    const uint4* x;                       // bf16 [T, dim]
+    const int64_t* indices;               // [T, topk]
+    const void* weights;                  // [T, topk], bf16 or fp32
+    int weights_bf16;
+    int64_t T, P;
+    int topk, dim, start, n, tpc, scale_fmt;
+    int* seg;                             // [n + 1]
+    int* pos_sorted;                      // [T, topk]
+    __nv_bfloat16* w_sorted;              // [T, topk]
+    uint2* xq;                            // e4m3 [T, dim]
+    float* xs;                            // [T, dim / 128]
+    uint2* xq_rows;                       // e4m3 [P, dim]
+    float* xs_rows;                       // [dim / 128, P]
+};
+
+__global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const DispatchParams p) {
+    __shared__ int total[kDispMaxExperts], before[kDispMaxExperts], scan[kDispMaxExperts / 32];
+    __shared__ int own_e[kDispPairs], own_row[kDispPairs];
+    griddep_launch_dependents();
+    griddep_wait();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int topk = p.topk;
+    const int64_t t0 = static_cast<int64_t>(blockIdx.x) * p.tpc;
+    const int tokens = static_cast<int>(min(static_cast<int64_t>(p.tpc), p.T - t0));
+    const int own = tokens * topk;
+    const int64_t own0 = t0 * topk;
+    if (tid < kDispMaxExperts) {
+        total[tid] = 0;
+        before[tid] = 0;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int64_t pr = tid; pr < p.P; pr += kDispThreads) {
+        const int64_t e = __ldg(p.indices + pr) - p.start;
+        if (e >= 0 && e < p.n) {
+            atomicAdd(&total[e], 1);
+            if (pr < own0) atomicAdd(&before[e], 1);
+        }
+    }
+    for (int i = tid; i < own; i += kDispThreads) {
+        const int64_t e = __ldg(p.indices + own0 + i);
+        own_e[i] = static_cast<int>(max(min(e, static_cast<int64_t>(0x3fffffff)), static_cast<int64_t>(-1)));
+    }
+    __syncthreads();
+    // exclusive prefix sum over the experts; before[] becomes the first row of this CTA's pairs of each expert
+    {
+        const bool has = tid < kDispMaxExperts;                    // whole warps
+        int v = has ? total[tid] : 0, inc = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        if (has && lane == 31) scan[warp] = inc;
+        __syncthreads();
+        if (has) {
+            int base = inc - v;
+            for (int w = 0; w < warp; ++w) base += scan[w];
+            if (blockIdx.x == 0 && blockIdx.y == 0) {
+                if (tid < p.n) p.seg[tid] = base;
+                if (tid == p.n - 1) p.seg[p.n] = base + v;
+            }
+            before[tid] += base;
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < own; i += kDispThreads) {
+        const int e = own_e[i] - p.start;
+        int row = -1;
+        if (e >= 0 && e < p.n) {
+            if (own <= kDispOrdered) {
+                int k = 0;
+                for (int j = 0; j < i; ++j) k += own_e[j] == own_e[i];
+                row = before[e] + k;
+            } else {
+                row = atomicAdd(&before[e], 1);
+            }
+        }
+        own_row[i] = row;
+    }
+    __syncthreads();
+    if (blockIdx.y == 0) {
+        for (int i = tid; i < own; i += kDispThreads) {
+            const int t = i / topk, first = t * topk, e = own_e[i];
+            int rank = 0;                                          // place in ascending expert order
+            for (int j = first; j < first + topk; ++j) rank += own_e[j] < e || (own_e[j] == e && j < i);
+            const int64_t at = own0 + first + rank;
+            p.pos_sorted[at] = own_row[i];
+            p.w_sorted[at] = p.weights_bf16 ? static_cast<const __nv_bfloat16*>(p.weights)[own0 + i]
+                                            : __float2bfloat16_rn(static_cast<const float*>(p.weights)[own0 + i]);
+        }
+    }
+    // quantise: a half-warp per 128-value block, kDispUnroll blocks in flight
+    const int nb = p.dim / 128;
+    const int per_y = (nb + gridDim.y - 1) / gridDim.y;
+    const int b_lo = blockIdx.y * per_y, b_n = min(per_y, nb - b_lo);
+    if (b_n <= 0) return;
+    const int items = tokens * b_n;
+    const int lane16 = tid & 15;
+    constexpr int kHalfWarps = kDispThreads / 16;
+    for (int i0 = tid >> 4; i0 - (tid >> 4) < items; i0 += kHalfWarps * kDispUnroll) {       // uniform trip count
+        uint4 v[kDispUnroll];
+        int tl[kDispUnroll], bl[kDispUnroll];
+#pragma unroll
+        for (int u = 0; u < kDispUnroll; ++u) {
+            const int i = i0 + u * kHalfWarps;
+            tl[u] = i < items ? i / b_n : -1;
+            bl[u] = b_lo + i - tl[u] * b_n;
+            v[u] = tl[u] >= 0 ? __ldg(p.x + ((t0 + tl[u]) * nb + bl[u]) * 16 + lane16) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < kDispUnroll; ++u) {
+            float m = amax8(v[u]);
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            const float sc = scale_from_amax(m, p.scale_fmt);
+            if (tl[u] < 0) continue;
+            const uint2 q = (p.scale_fmt == DSV3_SCALE_FMT_FP32) ? quant8<true>(v[u], sc) : quant8<false>(v[u], sc);
+            const int64_t t = t0 + tl[u];
+            p.xq[(t * nb + bl[u]) * 16 + lane16] = q;
+            if (lane16 == 0) p.xs[t * nb + bl[u]] = sc;
+            for (int j = 0; j < topk; ++j) {
+                const int row = own_row[tl[u] * topk + j];
+                if (row < 0) continue;
+                p.xq_rows[(static_cast<int64_t>(row) * nb + bl[u]) * 16 + lane16] = q;
+                if (lane16 == 0) p.xs_rows[static_cast<int64_t>(bl[u]) * p.P + row] = sc;
+            }
+        }
     }
 }
 
@@ -117,6 +288,37 @@ __global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(const int64_t*
     }
 }
 
+int check_groups(int n, const void* a, int64_t K) {
+    if (n < 1 || n > kMaxGroupsOfTable || K < 16 || K % 16 != 0 || reinterpret_cast<uintptr_t>(a) % 16 != 0) {
+        set_last_error("grouped fp8_gemm: needs K %% 16 == 0, a 16-byte aligned a, and 1..%d groups", kMaxGroupsOfTable);
+        return DSV3_ERR_UNSUPPORTED;
+    }
+    return DSV3_OK;
+}
+
+int grouped_plain(const void* table, int n, const void* a, const float* a_s, int64_t as_row, int64_t as_chunk, const int32_t* seg,
+                  int64_t rows_total, int64_t rows_hint, int64_t N, int64_t K, void* c, void* workspace, size_t workspace_bytes,
+                  dsv3_stream_t stream) {
+    const int rc = check_groups(n, a, K);
+    if (rc != DSV3_OK) return rc;
+    StreamGemm q = {};
+    q.a = a;
+    q.a_s = a_s;
+    q.as_row = as_row;
+    q.as_chunk = as_chunk;
+    q.rows = rows_total;
+    q.rows_expected = rows_hint > 0 && rows_hint < rows_total ? rows_hint : rows_total;
+    q.N = N;
+    q.K = K;
+    q.n_groups = n;
+    q.table0 = table;
+    q.seg = seg;
+    q.c = c;
+    q.workspace = workspace;
+    q.workspace_bytes = workspace_bytes;
+    return launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
+}
+
 }  // namespace
 
 }  // namespace dsv3
@@ -147,8 +349,131 @@ int dsv3_fp8_gemm_grouped(const void* table, int n_groups, const void* a, const 
         set_last_error("fp8_gemm_grouped: null pointer");
         return DSV3_ERR_INVALID_ARGUMENT;
     }
-    return launch_fp8_gemm_grouped(table, n_groups, a, a_s, seg, rows_total, rows_hint, N, K, c,
-                                   static_cast<cudaStream_t>(stream));
+    return grouped_plain(table, n_groups, a, a_s, (K + 127) / 128, 1, seg, rows_total, rows_hint, N, K, c, nullptr, 0, stream);
+}
+
+int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total,
+                       int64_t rows_hint, int64_t N, int64_t K, void* c, void* workspace, size_t workspace_bytes,
+                       dsv3_stream_t stream) {
+    if (rows_total < 0 || rows_hint < 0 || N < 0 || K <= 0) {
+        set_last_error("fp8_gemm_rows: negative size");
+        return DSV3_ERR_INVALID_ARGUMENT;
+    }
+    if (rows_total == 0 || N == 0) return DSV3_OK;
+    if (!table || !a || !a_s_t || !seg || !c) {
+        set_last_error("fp8_gemm_rows: null pointer");
+        return DSV3_ERR_INVALID_ARGUMENT;
+    }
+    return grouped_plain(table, n_groups, a, a_s_t, 1, rows_total, seg, rows_total, rows_hint, N, K, c, workspace, workspace_bytes, stream);
+}
+
+int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, const void* a, const float* a_s_t, const int32_t* seg,
+                          int64_t rows_total, int64_t rows_hint, int64_t N, int64_t K, int scale_fmt, void* hq, float* hs_t,
+                          void* workspace, size_t workspace_bytes, dsv3_stream_t stream) {
+    if (rows_total < 0 || rows_hint < 0 || N < 0 || K <= 0) {
+        set_last_error("swiglu_gemm_rows: negative size");
+        return DSV3_ERR_INVALID_ARGUMENT;
+    }
+    if (scale_fmt != DSV3_SCALE_FMT_FP32 && scale_fmt != DSV3_SCALE_FMT_UE8M0) {
+        set_last_error("swiglu_gemm_rows: unknown scale_fmt %d", scale_fmt);
+        return DSV3_ERR_INVALID_ARGUMENT;
+    }
+    if (rows_total == 0 || N == 0) return DSV3_OK;
+    if (!table1 || !table3 || !a || !a_s_t || !seg || !hq || !hs_t) {
+        set_last_error("swiglu_gemm_rows: null pointer");
+        return DSV3_ERR_INVALID_ARGUMENT;
+    }
+    if (N % 128 != 0) {
+        set_last_error("swiglu_gemm_rows: N = %lld is not divisible by 128", static_cast<long long>(N));
+        return DSV3_ERR_UNSUPPORTED;
+    }
+    int rc = check_groups(n_groups, a, K);
+    if (rc != DSV3_OK) return rc;
+    StreamGemm q = {};
+    q.a = a;
+    q.a_s = a_s_t;
+    q.as_row = 1;
+    q.as_chunk = rows_total;
+    q.rows = rows_total;
+    q.rows_expected = rows_hint > 0 && rows_hint < rows_total ? rows_hint : rows_total;
+    q.N = N;
+    q.K = K;
+    q.n_groups = n_groups;
+    q.table0 = table1;
+    q.table1 = table3;
+    q.seg = seg;
+    q.swiglu = true;
+    q.hq = hq;
+    q.hs = hs_t;
+    q.hs_row = 1;
+    q.hs_blk = rows_total;
+    q.scale_fmt = scale_fmt;
+    q.workspace = workspace;
+    q.workspace_bytes = workspace_bytes;
+    return launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
+}
+
+size_t dsv3_gemm_rows_workspace_bytes(int n_groups, int64_t rows_total, int64_t rows_hint) {
+    if (n_groups <= 0 || rows_total <= 0) return 0;
+    const int64_t rows = rows_hint > 0 && rows_hint < rows_total ? rows_hint : rows_total;
+    return stream_workspace_bytes((rows + n_groups - 1) / n_groups);
+}
+
+int dsv3_moe_dispatch(const void* x, int64_t T, int64_t dim, const int64_t* indices, const void* weights, int weights_bf16, int topk,
+                      int start, int n_local, int scale_fmt, int32_t* seg, int32_t* pos_sorted, void* w_sorted, void* xq, float* xs,
+                      void* xq_rows, float* xs_rows_t, dsv3_stream_t stream) {
+    if (T < 0 || topk < 0 || n_local < 0 || dim < 0) {
+        set_last_error("moe_dispatch: negative size");
+        return DSV3_ERR_INVALID_ARGUMENT;
+    }
+    if (scale_fmt != DSV3_SCALE_FMT_FP32 && scale_fmt != DSV3_SCALE_FMT_UE8M0) {
+        set_last_error("moe_dispatch: unknown scale_fmt %d", scale_fmt);
+        return DSV3_ERR_INVALID_ARGUMENT;
+    }
+    if (T == 0 || topk == 0 || dim == 0) return DSV3_OK;
+    if (!x || !indices || !weights || !seg || !pos_sorted || !w_sorted || !xq || !xs || !xq_rows || !xs_rows_t) {
+        set_last_error("moe_dispatch: null pointer");
+        return DSV3_ERR_INVALID_ARGUMENT;
+    }
+    if (n_local < 1 || n_local > kDispMaxExperts || topk > kRouteMaxTopk || T * topk >= (1ll << 31) || dim % 128 != 0 || dim > (1 << 24)) {
+        set_last_error("moe_dispatch: 1..%d local experts, at most top-%d and 2^31 pairs, dim divisible by 128", kDispMaxExperts, kRouteMaxTopk);
+        return DSV3_ERR_UNSUPPORTED;
+    }
+    if (reinterpret_cast<uintptr_t>(x) % 16 != 0 || reinterpret_cast<uintptr_t>(xq) % 8 != 0 || reinterpret_cast<uintptr_t>(xq_rows) % 8 != 0) {
+        set_last_error("moe_dispatch: x must be 16-byte, xq and xq_rows 8-byte aligned");
+        return DSV3_ERR_UNSUPPORTED;
+    }
+    DispatchParams p;
+    p.x = static_cast<const uint4*>(x);
+    p.indices = indices;
+    p.weights = weights;
+    p.weights_bf16 = weights_bf16;
+    p.T = T;
+    p.P = T * topk;
+    p.topk = topk;
+    p.dim = static_cast<int>(dim);
+    p.start = start;
+    p.n = n_local;
+    p.scale_fmt = scale_fmt;
+    p.seg = seg;
+    p.pos_sorted = pos_sorted;
+    p.w_sorted = static_cast<__nv_bfloat16*>(w_sorted);
+    p.xq = static_cast<uint2*>(xq);
+    p.xs = xs;
+    p.xq_rows = static_cast<uint2*>(xq_rows);
+    p.xs_rows = xs_rows_t;
+    // one CTA per SM (every CTA counts all pairs), at most kDispPairs own pairs each
+    const int64_t wave = num_sms();
+    int64_t tpc = (T + wave - 1) / wave;
+    if (tpc > kDispPairs / topk) tpc = kDispPairs / topk;
+    p.tpc = static_cast<int>(tpc);
+    const int64_t gx = (T + tpc - 1) / tpc;
+    int gy = 1;                                                    // few tokens: share each token's blocks among CTAs
+    if (tpc * topk <= kDispOrdered)
+        while (gy < 8 && gx * gy * 2 <= wave && gy * 2 * 32 <= dim / 128) gy *= 2;
+    DSV3_CUDA_TRY(launch_dependent(moe_dispatch_kernel, dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), dim3(kDispThreads), 0,
+                                   static_cast<cudaStream_t>(stream), p));
+    return DSV3_OK;
 }
 
 int dsv3_moe_route(const int64_t* indices, const float* weights, int64_t T, int topk, int start, int n_local,
@@ -174,6 +499,11 @@ int dsv3_moe_route(const int64_t* indices, const float* weights, int64_t T, int 
 
 int dsv3_moe_combine(const void* o, const int32_t* pos, const void* w, int64_t T, int topk, int64_t dim, void* y,
                      dsv3_stream_t stream) {
+    return dsv3_moe_combine_add(o, pos, w, nullptr, T, topk, dim, y, stream);
+}
+
+int dsv3_moe_combine_add(const void* o, const int32_t* pos, const void* w, const void* z, int64_t T, int topk, int64_t dim, void* y,
+                         dsv3_stream_t stream) {
     if (T < 0 || topk < 0 || dim < 0) {
         set_last_error("moe_combine: negative size");
         return DSV3_ERR_INVALID_ARGUMENT;
@@ -183,18 +513,16 @@ int dsv3_moe_combine(const void* o, const int32_t* pos, const void* w, int64_t T
         set_last_error("moe_combine: null pointer");
         return DSV3_ERR_INVALID_ARGUMENT;
     }
-    if (dim % 8 != 0 || reinterpret_cast<uintptr_t>(o) % 16 != 0 || reinterpret_cast<uintptr_t>(y) % 16 != 0) {
-        set_last_error("moe_combine: dim must be a multiple of 8 and o, y 16-byte aligned");
+    const int64_t per_row = (dim / 8 + kThreads - 1) / kThreads;
+    if (dim % 8 != 0 || reinterpret_cast<uintptr_t>(o) % 16 != 0 || reinterpret_cast<uintptr_t>(y) % 16 != 0 ||
+        reinterpret_cast<uintptr_t>(z) % 16 != 0 || T * per_row >= (1ll << 31)) {
+        set_last_error("moe_combine: dim must be a multiple of 8 and o, y (and z) 16-byte aligned");
         return DSV3_ERR_UNSUPPORTED;
     }
-    const int64_t total = T * (dim >> 3);
-    int64_t grid = (total + kThreads - 1) / kThreads;
-    const int64_t cap = static_cast<int64_t>(num_sms()) * 8;
-    if (grid > cap) grid = cap;
-    moe_combine_kernel<<<static_cast<unsigned>(grid), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(o), pos, static_cast<const __nv_bfloat16*>(w),
-        static_cast<__nv_bfloat16*>(y), T, topk, dim);
-    DSV3_CUDA_TRY(cudaGetLastError());
+    DSV3_CUDA_TRY(launch_dependent(moe_combine_kernel, dim3(static_cast<unsigned>(T * per_row)), dim3(kThreads), 0,
+                                   static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(o), pos,
+                                   static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(z),
+                                   static_cast<__nv_bfloat16*>(y), topk, dim, make_fast_div(static_cast<uint32_t>(per_row))));
     return DSV3_OK;
 }
 

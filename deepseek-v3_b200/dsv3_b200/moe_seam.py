@@ -3,9 +3,10 @@
 ``MoE.forward`` of the reference (model.py:669-693) walks over the local experts in Python; every
 expert costs two host synchronisations (``bincount(...).tolist()``, ``torch.where``) and about six
 small launches.  ``grouped_moe_forward`` keeps inputs, outputs and arithmetic (same quantisation per
-token row, same bf16 rounding points, same ascending-expert accumulation order) but sorts the
-(token, expert) pairs on the device (one launch) and runs each of the three projections as one grouped GEMM
-over all local experts, followed by one combine kernel.  Nothing is read back to the host.
+token row, same bf16 rounding points, same ascending-expert accumulation order) but runs in
+four launches: routing bookkeeping with the quantisation of the tokens, w1 and w3 of all local experts with SwiGLU and
+the quantisation in front of w2, w2 of all local experts, and the weighted sum with the shared experts' output.
+Nothing is read back to the host.
 
     import model, dsv3_b200
     dsv3_b200.install_moe(model)        # model.MoE.forward = grouped_moe_forward
@@ -17,28 +18,51 @@ from typing import List
 
 import torch
 
-from . import _lib
-from . import linear_seam
+from . import _lib, linear_seam
 from ._lib import host, lib
-from .ops import swiglu_quant, _stream
+from .ops import _stream
+
+
+def _look_up(obj, name):
+    """The attribute and the dictionary it lives in (None where it lives elsewhere)."""
+    value = getattr(obj, name)
+    own = getattr(obj, "__dict__", None)
+    if own is not None:
+        for d in (own, own.get("_parameters"), own.get("_modules"), own.get("_buffers")):
+            if type(d) is dict and d.get(name) is value:
+                return value, (d, name, value)
+    return value, None
 
 
 class GroupedExperts:
     """Device tables (tensor maps + scale pointers) of the local experts' three projections."""
 
-    def __init__(self, experts: List, start: int):
+    def __init__(self, container, experts: List, start: int):
         self.start = start
         self.n = len(experts)
+        self.container = container
         e0 = experts[0]
         self.dim = e0.w1.weight.size(1)
         self.inter = e0.w1.weight.size(0)
         self.scale_fmt = getattr(e0.w1, "scale_fmt", None)
         self.device = e0.w1.weight.device
-        self._keep = experts                       # the tables point into these parameters
-        self.tables = {}
+        # every look-up from the container to a weight's storage that the tables depend on
+        found, weights, by_name = [], [], {"w1": [], "w3": [], "w2": []}
+        if not isinstance(container, list):
+            members = getattr(container, "_modules", None)
+            found += [(members, str(start + i), e) if type(members) is dict else None for i, e in enumerate(experts)]
+        for e in experts:
+            for name in by_name:
+                lin, step = _look_up(e, name)
+                w, step2 = _look_up(lin, "weight")
+                found += [step, step2]
+                weights.append(w)
+                by_name[name].append(w)
+        self.watched = all(f is not None for f in found)      # otherwise the weights are looked up on every pass
+        tables = {}
         for name, N, K in (("w1", self.inter, self.dim), ("w3", self.inter, self.dim), ("w2", self.dim, self.inter)):
-            ws = [getattr(e, name).weight for e in experts]
-            ss = [getattr(e, name).weight.scale for e in experts]
+            ws = by_name[name]
+            ss = [w.scale for w in ws]
             for w, s in zip(ws, ss):
                 assert w.element_size() == 1 and w.is_contiguous() and s.is_contiguous() and s.dtype == torch.float32
                 assert tuple(w.shape) == (N, K)
@@ -47,57 +71,38 @@ class GroupedExperts:
             sp = (ctypes.c_void_p * self.n)(*[s.data_ptr() for s in ss])
             with torch.cuda.device(self.device):
                 _lib.check(lib.dsv3_group_table_build(table.data_ptr(), wp, sp, self.n, N, K, _stream()))
-            self.tables[name] = (table, N, K)
-        self.signature = tuple(getattr(e, n).weight.data_ptr() for e in experts for n in ("w1", "w2", "w3"))
+            tables[name] = table
+        self._keep = (experts, [w.scale for w in weights])    # the tables point into these
+        self.signature = tuple(w.data_ptr() for w in weights)
+        self.handle = host.experts(self.n, start, self.dim, self.inter, self.scale_fmt, tables["w1"], tables["w3"], tables["w2"],
+                                   container if isinstance(container, list) else None, list(experts),
+                                   found if self.watched else [], weights)
 
-    def gemm(self, name: str, a: torch.Tensor, a_s: torch.Tensor, seg: torch.Tensor, rows_hint: int = 0) -> torch.Tensor:
-        table, N, K = self.tables[name]
-        rows = a.size(0)
-        c = torch.empty(rows, N, dtype=torch.bfloat16, device=a.device)
-        _lib.check(lib.dsv3_fp8_gemm_grouped(table.data_ptr(), self.n, a.data_ptr(), a_s.data_ptr(), seg.data_ptr(),
-                                             rows, rows_hint, N, K, c.data_ptr(), _stream()))
-        return c
+    def current(self, moe) -> bool:
+        """Whether ``moe``'s local experts are still the ones the tables were built from."""
+        if moe.experts is not self.container or moe.experts_start_idx != self.start or moe.experts_end_idx != self.start + self.n:
+            return False
+        if not self.watched and self.signature != tuple(getattr(moe.experts[i], n).weight.data_ptr()
+                                                        for i in range(self.start, self.start + self.n) for n in ("w1", "w3", "w2")):
+            return False
+        return host.experts_current(self.handle)
+
+    def run(self, x: torch.Tensor, weights: torch.Tensor, indices: torch.Tensor, n_routed: int = 0):
+        """The local experts' outputs for the routed tokens (model.py:683-688), to be handed to ``combine``: routing
+        bookkeeping and quantisation, w1 / w3 with SwiGLU and quantisation, w2, nothing read back.  ``n_routed``: experts
+        of the whole layer (this rank owns ``self.n`` of them and, on average, that share of the pairs)."""
+        return host.run_experts(self.handle, x, weights, indices, n_routed, linear_seam._assume_no_inplace)
 
     def routed(self, x: torch.Tensor, weights: torch.Tensor, indices: torch.Tensor, n_routed: int = 0) -> torch.Tensor:
-        """Sum over the local experts of ``expert(x[idx]) * weights`` (model.py:683-689).  ``n_routed``: experts of
-        the whole layer (this rank owns ``self.n`` of them and, on average, that share of the pairs)."""
-        T, topk = indices.shape
-        P = T * topk
-        n = self.n
-        hint = max(1, (P * n + n_routed - 1) // n_routed) if n_routed > n else 0
-        with torch.cuda.device(x.device):
-            # ---- group the (token, expert) pairs by local expert (pairs of other ranks' experts go last) and
-            # order every token's pairs by expert id: one launch, nothing read back
-            idx = indices if indices.dtype == torch.int64 else indices.long()
-            idx = idx if idx.is_contiguous() else idx.contiguous()
-            wf = (weights if weights.dtype == torch.float32 else weights.float()).contiguous()
-            seg = torch.empty(n + 1, dtype=torch.int32, device=x.device)
-            tok = torch.empty(P, dtype=torch.int32, device=x.device)
-            pair_row = torch.empty(P, dtype=torch.int32, device=x.device)
-            pos_s = torch.empty(T, topk, dtype=torch.int32, device=x.device)
-            w_s = torch.empty(T, topk, dtype=torch.bfloat16, device=x.device)
-            _lib.check(lib.dsv3_moe_route(idx.data_ptr(), wf.data_ptr(), T, topk, self.start, n, seg.data_ptr(),
-                                          tok.data_ptr(), pair_row.data_ptr(), pos_s.data_ptr(), w_s.data_ptr(), _stream()))
-            # ---- quantise every token once, gather the rows in expert order
-            xq, xs = host.quantise_remembered(x, 128, self.scale_fmt, linear_seam._assume_no_inplace)
-            xq_p = xq.view(torch.uint8).index_select(0, tok).view(torch.float8_e4m3fn)
-            xs_p = xs.index_select(0, tok)
-            # ---- w2(silu(w1 x) * w3 x), the bf16 rounding points of Expert.forward (model.py:633)
-            hq, hs = swiglu_quant(self.gemm("w1", xq_p, xs_p, seg, hint), self.gemm("w3", xq_p, xs_p, seg, hint), self.scale_fmt)
-            o = self.gemm("w2", hq, hs, seg, hint)
-            # ---- y[t] = sum over the token's local experts, ascending expert id, bf16 at every step
-            y = torch.empty(T, self.dim, dtype=torch.bfloat16, device=x.device)
-            _lib.check(lib.dsv3_moe_combine(o.data_ptr(), pos_s.data_ptr(), w_s.data_ptr(), T, topk, self.dim,
-                                            y.data_ptr(), _stream()))
-        return y
+        """Sum over the local experts of ``expert(x[idx]) * weights`` (model.py:683-689)."""
+        return host.combine(self.run(x, weights, indices, n_routed), None)
 
 
 def _grouped(moe) -> GroupedExperts:
-    local = [moe.experts[i] for i in range(moe.experts_start_idx, moe.experts_end_idx)]
-    sig = tuple(getattr(e, n).weight.data_ptr() for e in local for n in ("w1", "w2", "w3"))
     st = getattr(moe, "_dsv3_grouped", None)
-    if st is None or st.signature != sig:
-        st = GroupedExperts(local, moe.experts_start_idx)
+    if st is None or not st.current(moe):
+        local = [moe.experts[i] for i in range(moe.experts_start_idx, moe.experts_end_idx)]
+        st = GroupedExperts(moe.experts, local, moe.experts_start_idx)
         object.__setattr__(moe, "_dsv3_grouped", st)      # not a Module/Parameter: keep it out of the registry
     return st
 
@@ -112,12 +117,16 @@ def grouped_moe_forward(self, x: torch.Tensor, *, world_size: int = 1, fallback=
     shape = x.size()
     x = x.view(-1, self.dim)
     weights, indices = self.gate(x)
-    y = _grouped(self).routed(x, weights, indices, getattr(self, "n_routed_experts", 0))
+    routed = _grouped(self).run(x, weights, indices, getattr(self, "n_routed_experts", 0))
     z = self.shared_experts(x)
     if world_size > 1:
         import torch.distributed as dist
+        y = host.combine(routed, None)
         dist.all_reduce(y)
-    return (y + z).view(shape)
+        return (y + z).view(shape)
+    if z.dtype == torch.bfloat16 and z.is_contiguous() and z.size() == x.size():
+        return host.combine(routed, z).view(shape)
+    return (host.combine(routed, None) + z).view(shape)
 
 
 def install_moe(model_module) -> None:

@@ -171,7 +171,7 @@ int dsv3_set_num_sms(int n);
  *              if unknown (then rows_total).  Only a tuning input: it picks the token-tile width.  With tensor
  *              parallelism a rank owns n of the E experts and about rows_total * n / E of the rows.
  *   c        : bf16 [rows_total, N]; row r = a[r] @ weight[e(r)]^T with the block scales applied.
- * Limits: n <= 256, K <= 18432, K % 16 == 0.
+ * Limits: n <= 256, K % 16 == 0.
  */
 size_t dsv3_group_table_bytes(int n_groups);
 int dsv3_group_table_build(void* table, const void* const* weights, const float* const* scales, int n_groups,
@@ -206,6 +206,35 @@ int dsv3_moe_route(const int64_t* indices, const float* weights, int64_t T, int 
  */
 int dsv3_moe_combine(const void* o, const int32_t* pos, const void* w, int64_t T, int topk, int64_t dim, void* y,
                      dsv3_stream_t stream);
+
+int dsv3_moe_combine_add(const void* o, const int32_t* pos, const void* w, const void* z, int64_t T, int topk, int64_t dim, void* y,
+                         dsv3_stream_t stream);
+
+/*
+ * The expert layer in four launches -- MoE.forward, model.py:669-693, without the router and the shared experts:
+ *   dsv3_moe_dispatch       routing bookkeeping (as dsv3_moe_route), act_quant of every token, and a copy of its FP8 row
+ *                           for each of its local experts
+ *   dsv3_swiglu_gemm_rows   w1 and w3 of all local experts, silu(w1 x) * w3 x and the act_quant in front of w2
+ *   dsv3_fp8_gemm_rows      w2 of all local experts
+ *   dsv3_moe_combine_add    dsv3_moe_combine followed by the bf16 addition of z (model.py:693); z may be null
+ * Layouts: indices, weights, seg, pos_sorted, w_sorted as in dsv3_moe_route; weights bf16 or fp32 (weights_bf16);
+ * x bf16 [T, dim], dim % 128 == 0; xq e4m3 [T, dim], xs fp32 [T, dim/128] (what dsv3_act_quant writes for x);
+ * xq_rows e4m3 [T*topk, dim]; scales with the suffix _t are TRANSPOSED, fp32 [K/128, rows_total] (xs_rows_t, a_s_t,
+ * hs_t); hq e4m3 [rows_total, N].  Rows at and beyond seg[n] are not written.  The results equal those of the separate
+ * operators: FP8 bytes and scales bit for bit given equal GEMM results.
+ * workspace: dsv3_gemm_rows_workspace_bytes() bytes under the rules of dsv3_fp8_gemm's workspace (zeroed header, 256-byte
+ * aligned, not shared by overlapping calls); null: K is never split, which is slower for few rows.
+ */
+int dsv3_moe_dispatch(const void* x, int64_t T, int64_t dim, const int64_t* indices, const void* weights, int weights_bf16, int topk,
+                      int start, int n_local, int scale_fmt, int32_t* seg, int32_t* pos_sorted, void* w_sorted, void* xq, float* xs,
+                      void* xq_rows, float* xs_rows_t, dsv3_stream_t stream);
+size_t dsv3_gemm_rows_workspace_bytes(int n_groups, int64_t rows_total, int64_t rows_hint);
+int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, const void* a, const float* a_s_t, const int32_t* seg,
+                          int64_t rows_total, int64_t rows_hint, int64_t N, int64_t K, int scale_fmt, void* hq, float* hs_t,
+                          void* workspace, size_t workspace_bytes, dsv3_stream_t stream);
+int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total,
+                       int64_t rows_hint, int64_t N, int64_t K, void* c, void* workspace, size_t workspace_bytes,
+                       dsv3_stream_t stream);
 
 /*
  * One-shot all-reduce of a decode-sized bf16 tensor over peer-mapped buffers -- replaces `dist.all_reduce(y)` after
