@@ -58,6 +58,7 @@ constexpr int kRegsPromo = 232;
 static_assert(128 * kRegsControl + 256 * kRegsPromo <= 384 * 168, "register pool");
 
 constexpr int kTmemStages = 4;
+constexpr int kMaxClusterSplits = 8;      // portable cluster size
 constexpr int kMaxTickets = DSV3_WORKSPACE_HEADER_BYTES / 4;
 
 struct TcParams {
@@ -71,7 +72,8 @@ struct TcParams {
     int kc;                 // number of K chunks
     int tiles_p, tiles_q;
     int splits;
-    FastDiv div_splits, div_per_group, div_raster;   // for the work-item decoder
+    int cluster;            // the splits of a tile are the CTAs of one cluster and meet in shared memory (no partials, no tickets)
+    FastDiv div_splits, div_per_group, div_raster, div_rows;   // for the work-item decoder
     int raster;             // token-major tiles: P tiles (token tiles) that share consecutive Q tiles in the work order
     int tma_store;          // token-major tiles: results leave through shared memory and a TMA store (needs N % 8 == 0)
     int num_items;          // tiles_p * tiles_q * splits
@@ -97,8 +99,13 @@ struct Cfg {
     static constexpr int kScaleTabBytes = kSwap ? scale_tab_chunks(BN) * BN * 4 : 0;
     // token-major tiles: the 128 x 128 bf16 result tile is staged here (two 128-byte-swizzled 128 x 64 boxes)
     static constexpr int kStoreBytes = !kSwap ? kPRows * 128 * 2 : 0;
+    // Split-K inside a cluster: partial sums that the other CTAs send here.  16- and 32-token tiles have room of their own
+    // for them; the others re-use the operand stages once every CTA of the cluster is through with its own.
+    static constexpr bool kOwnExchange = kSwap && BN < 64;
+    static constexpr int kExchangePitch = kSwap ? BN + 4 : BN;               // floats per row (weight-major: + 16 bytes against bank conflicts)
+    static constexpr int kExchangeBytes = (kPRows + 8) * kExchangePitch * 4;    // splits * ceil(128 / splits) rows
     static constexpr int kStagesRaw =
-        (232448 - 2048 - kStoreBytes - kScaleTabBytes) / kStageBytes;
+        (232448 - 2048 - kStoreBytes - kScaleTabBytes - (kOwnExchange ? kExchangeBytes : 0)) / kStageBytes;
     static constexpr int kStagesCap = kStagesRaw > 10 ? 10 : kStagesRaw;
     // weight-major tiles: an even stage count, so that a stage always belongs to the same MMA issuer and
     // the issuer may probe its next full[] barrier (see the issuer loop)
@@ -106,7 +113,8 @@ struct Cfg {
     static constexpr int kTmemCols = kAccs * BN;  // 64..512, a power of two
     // tiles + result staging + tables + barriers + control words + slack for the 1024-byte alignment of the tiles
     static constexpr int kSmemBytes =
-        kStages * kStageBytes + kStoreBytes + kScaleTabBytes + 1024 + 1024;
+        kStages * kStageBytes + kStoreBytes + kScaleTabBytes + (kOwnExchange ? kExchangeBytes : 0) + 1024 + 1024;
+    static_assert(kOwnExchange || kExchangeBytes <= kStages * kStageBytes, "the exchange fits the operand stages");
     static_assert(kSmemBytes <= 232448, "shared memory per CTA");
     static_assert(kStages >= 3, "at least three smem stages");
     static_assert(kTmemCols >= 32 && kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "TMEM columns");
@@ -183,7 +191,8 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
     uint8_t* store_buf = gen_tiles + NS * C::kStageBytes;                       // 1024-byte aligned (swizzle atom)
     uint8_t* after_store = store_buf + C::kStoreBytes;
     float* sc_tab = reinterpret_cast<float*>(after_store);   // [chunk][token]
-    uint64_t* bars = reinterpret_cast<uint64_t*>(after_store + C::kScaleTabBytes);
+    float* exchange = reinterpret_cast<float*>(C::kOwnExchange ? after_store + C::kScaleTabBytes : gen_tiles);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(after_store + C::kScaleTabBytes + (C::kOwnExchange ? C::kExchangeBytes : 0));
     Control* ctl = reinterpret_cast<Control*>(bars + 2 * NS + 2 * NT + 2);
     const uint32_t bar0 = smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
@@ -233,7 +242,9 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
+    if (C::kOwnExchange && p.cluster) cluster_arrive();             // waited for in front of the exchange
 
+    bool exchanged = false;
     if constexpr (!kSwap) {
         if (warp < kFirstPromoWarp) {
             asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
@@ -552,7 +563,82 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
             // normal: thread = token row, CPT consecutive output columns
             // swap  : thread = output column (weight row), CPT tokens
             bool write_out = true;
-            if (p.splits > 1) {
+            if (p.cluster) {
+                // Split-K inside a cluster (one item per CTA).  CTA r of the cluster adds up and writes rows
+                // [r R, (r+1) R) of the tile, R = ceil(128 / splits): every CTA sends each peer its rows of the partial
+                // tile (st.shared::cluster), a cluster barrier later everybody adds what arrived, in split order.
+                // Against the ticket form below (partial tiles through L2, an atomic, the last arrival reads
+                // everything back) this takes about 1.5 us off a launch.
+                const int S = p.splits, R = (kPRows + S - 1) / S;
+                if constexpr (!C::kOwnExchange) cluster_arrive();   // through with the operand stages
+                cluster_wait();                                     // every CTA runs, and with shared stages is through with them
+                const int dest = static_cast<int>(fast_div(static_cast<uint32_t>(row), p.div_rows)), r_local = row - dest * R;
+                const uint32_t remote = mapa_shared(smem_u32(exchange), static_cast<uint32_t>(dest));
+                const int ntok = static_cast<int>(min(static_cast<int64_t>(BN), m_end - (q_base - col0)));   // weight-major tiles
+                if constexpr (kSwap) {              // [split][R rows][tokens]
+                    const uint32_t at = remote + 4u * ((it.split * R + r_local) * C::kExchangePitch + col0);
+#pragma unroll
+                    for (int j = 0; j < CPT; j += 4)
+                        if (col0 + j < ntok)
+                            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at + 4u * j), "f"(accf[j]), "f"(accf[j + 1]),
+                                         "f"(accf[j + 2]), "f"(accf[j + 3]) : "memory");
+                } else {                            // [split][R rows][32 16-byte slots], slot c of row r at c ^ (r & 31)
+#pragma unroll
+                    for (int j = 0; j < CPT / 4; ++j) {
+                        const uint32_t at = remote + 512u * (it.split * R + r_local) + 16u * ((col0 / 4 + j) ^ (row & 31));
+                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(accf[4 * j]), "f"(accf[4 * j + 1]),
+                                     "f"(accf[4 * j + 2]), "f"(accf[4 * j + 3]) : "memory");
+                    }
+                }
+                cluster_arrive();
+                cluster_wait();
+                const int me = static_cast<int>(cluster_ctarank()), rows_here = min(R, kPRows - me * R);
+                const int tid = threadIdx.x - kFirstPromoWarp * 32;
+                if constexpr (kSwap) {
+                    // a thread adds four tokens of one row; neighbouring threads take neighbouring rows (output columns)
+                    const int64_t n0 = static_cast<int64_t>(it.p_idx) * kPRows + me * R;
+                    for (int e = tid; e < (ntok + 3) / 4 * R; e += kPromoThreads) {
+                        const int t4 = static_cast<int>(fast_div(static_cast<uint32_t>(e), p.div_rows)), i = e - t4 * R;
+                        if (i >= rows_here || n0 + i >= N) continue;
+                        const float* src = exchange + i * C::kExchangePitch + 4 * t4;
+                        float4 sum = *reinterpret_cast<const float4*>(src);
+                        for (int sp = 1; sp < S; ++sp) {
+                            const float4 a = *reinterpret_cast<const float4*>(src + sp * R * C::kExchangePitch);
+                            sum.x += a.x; sum.y += a.y; sum.z += a.z; sum.w += a.w;
+                        }
+                        __nv_bfloat16* dst = p.c + (static_cast<int64_t>(it.row0) + 4 * t4) * N + n0 + i;
+                        const float v4[4] = {sum.x, sum.y, sum.z, sum.w};
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (4 * t4 + q < ntok) dst[q * N] = __float2bfloat16_rn(v4[q]);
+                    }
+                } else {
+                    const bool vec_ok = (N % 8) == 0;
+                    for (int e = tid; e < rows_here * 16; e += kPromoThreads) {      // eight columns each
+                        const int i = e >> 4, k8 = e & 15, r_tile = me * R + i;
+                        const int64_t m = static_cast<int64_t>(it.p_idx) * kPRows + r_tile, n = static_cast<int64_t>(it.q_idx) * BN + 8 * k8;
+                        if (m >= M || n >= N) continue;
+                        float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
+                        for (int sp = 0; sp < S; ++sp) {
+                            const float4* src = reinterpret_cast<const float4*>(exchange) + 32 * (sp * R + i);
+                            const float4 a = src[(2 * k8) ^ (r_tile & 31)], b = src[(2 * k8 + 1) ^ (r_tile & 31)];
+                            lo.x += a.x; lo.y += a.y; lo.z += a.z; lo.w += a.w;
+                            hi.x += b.x; hi.y += b.y; hi.z += b.z; hi.w += b.w;
+                        }
+                        __nv_bfloat16* dst = p.c + m * N + n;
+                        if (vec_ok && n + 8 <= N) {
+                            *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(lo.x, lo.y), pack_bf16x2(lo.z, lo.w), pack_bf16x2(hi.x, hi.y), pack_bf16x2(hi.z, hi.w));
+                        } else {
+                            const float v8[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+#pragma unroll
+                            for (int q = 0; q < 8; ++q)
+                                if (n + q < N) dst[q] = __float2bfloat16_rn(v8[q]);
+                        }
+                    }
+                }
+                write_out = false;
+                exchanged = true;
+            } else if (p.splits > 1) {
                 // Split-K: park the partial sums, take a ticket; the last arrival of the tile sums the
                 // partial tiles in split order (deterministic) and writes the result.  Partial tiles use a
                 // private layout chosen for coalescing, [split][tile][group of 4 columns][128 rows] float4:
@@ -668,6 +754,16 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
         }
     }
 
+    // The cluster barriers of the split-K exchange count every thread: the control warps pass through them here, and so
+    // does a promotion warp whose wait gave up.
+    if (p.cluster && (warp < kFirstPromoWarp || !exchanged)) {
+        __syncwarp();
+        if constexpr (!C::kOwnExchange) cluster_arrive();
+        cluster_wait();
+        cluster_arrive();
+        cluster_wait();
+    }
+
     // ---------------------------------------------------------------- teardown
     if (!kSwap && warp >= kFirstPromoWarp && (threadIdx.x & 127) == 0) bulk_wait_group0();   // result tiles have left shared memory
     __syncwarp();
@@ -765,6 +861,24 @@ int launch_variant(const CUtensorMap& tp, const CUtensorMap& tq, const CUtensorM
         DSV3_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
         configured[dev] = true;
     }
+    if (prm.cluster) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(prm.num_items));
+        cfg.blockDim = dim3(kNumThreads);
+        cfg.dynamicSmemBytes = C::kSmemBytes;
+        cfg.stream = stream;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(prm.splits);
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = pdl_enabled() ? 2 : 1;
+        DSV3_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, tp, tq, tc, prm));
+        return DSV3_OK;
+    }
     int grid = prm.num_items < num_sms() ? prm.num_items : num_sms();
     DSV3_CUDA_TRY(launch_dependent(kern, dim3(grid), dim3(kNumThreads), C::kSmemBytes, stream, tp, tq, tc, prm));
     return DSV3_OK;
@@ -777,6 +891,47 @@ bool tc_supported(const void* a, const void* b, const void* c, int64_t M, int64_
            (reinterpret_cast<uintptr_t>(b) % 16) == 0 && (reinterpret_cast<uintptr_t>(c) % 16) == 0 && M < (1ll << 31) && N < (1ll << 31) && K < (1ll << 31);
 }
 
+// How many clusters of `splits` CTAs of a variant the device holds at once (GPCs do not divide evenly by every size).
+namespace {
+template <int BN, bool kSwap>
+int clusters_of(int splits) {
+    using C = Cfg<BN, kSwap>;
+    static int cached[64][kMaxClusterSplits + 1] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = -1;
+    if (dev >= 0 && cached[dev][splits] > 0) return cached[dev][splits];
+    int n = 0;
+    if (dev >= 0) {
+        auto kern = fp8_gemm_tc_kernel<BN, kSwap>;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(static_cast<unsigned>(splits));
+        cfg.blockDim = dim3(kNumThreads);
+        cfg.dynamicSmemBytes = C::kSmemBytes;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+            (void)cudaGetLastError();
+            n = 0;
+        }
+        if (n > 0) cached[dev][splits] = n;
+    }
+    return n > 0 ? n : 128 / splits;      // no device (planning on a host without one): a cautious guess
+}
+}  // namespace
+
+static int64_t clusters_resident(bool swap, int bn, int splits) {
+    const int n = !swap ? clusters_of<128, false>(splits)
+                        : (bn == 16 ? clusters_of<16, true>(splits) : (bn == 32 ? clusters_of<32, true>(splits) : clusters_of<64, true>(splits)));
+    const int budget = num_sms() / splits;
+    return n < budget ? n : budget;
+}
+
 // Pinned values (dsv3_set_gemm_policy) are honoured or refused (pl.error), never rewritten; the automatic
 // plan adapts freely.
 TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split) {
@@ -785,6 +940,7 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
     pl.pair = false;
     pl.wide = false;
     pl.splits = 1;
+    pl.cluster = false;
     pl.kc = static_cast<int>((K + kChunk - 1) / kChunk);
     pl.swap = (force_kernel == 3) || (force_kernel == 0 && M <= 64);
     if (pl.swap) {
@@ -819,34 +975,41 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
         }
     } else if (force_kernel == 4 || force_kernel == 6) {
         splits = 1;
-    } else if (tiles <= kMaxTickets) {
-        // Splitting K fills idle SMs, but every split item pays for parking its partial tile, a fence and a
-        // ticket, and the last arrival of a tile sums the partial tiles.  Estimate, fitted to B200
-        // measurements (microseconds; the launch's fixed cost is the same for every factor and left out):
-        //   rounds(S) * (chunks_per_item(S) * c + (S > 1 ? e0 + e1 * S : 0)),   rounds = ceil(tiles * S / SMs)
-        // with c the time per K chunk of one CTA, never below the time the whole problem needs at HBM
-        // bandwidth.  The factor with the lowest estimate wins (ties: fewer splits).
+    } else {
+        // Splitting K over the CTAs of a cluster fills idle SMs; every split pays for the exchange of partial tiles.
+        // Estimate, fitted to B200 measurements (microseconds; a launch's fixed cost, 2.5-4 us, is left out):
+        //   S = 1: rounds * chunks * c1        S > 1 (all clusters resident at once): chunks / S * c + e
+        // c = time per K chunk of one CTA; c1 the same for the unsplit choice (above 128 tokens a pair kernel); neither
+        // below the time the whole problem needs at HBM bandwidth.  Measured, us, S = 1 / 2 / 4 / 8: 7168 -> 256 at
+        // M = 16 11.5 / 8.1 / 5.9 / 4.9, at M = 64 15.9 / 11.4 / 8.2 / 6.9; 7168 -> 576 at M = 256 16.3 / 15.2 / 12.1 / 11.1;
+        // a split that needs a second round of clusters loses badly (7168 -> 2048 at M = 16, S = 8: 11.7, S = 4: 6.8).
         const int sms = num_sms();
-        const double c = pl.swap ? (pl.bn == 64 ? 0.30 : 0.22) : 0.26;
-        const double e0 = pl.swap ? 2.2 : 2.3, e1 = pl.swap ? 0.2 * pl.bn / 64.0 : 0.5;
+        const double c = !pl.swap ? 0.29 : (pl.bn == 64 ? 0.23 : (pl.bn == 32 ? 0.19 : 0.18));
+        const double e = !pl.swap ? 3.4 : (pl.bn == 64 ? 1.9 : (pl.bn == 32 ? 1.3 : 1.0));
+        const double c1 = !pl.swap && M > kPRows ? 0.22 : c;
         const double hbm_floor = (static_cast<double>(N) * K + static_cast<double>(M) * K) / 6.0e6;
         double best = 1e30;
-        for (int sfac = 1; sfac <= 8 && sfac <= pl.kc; ++sfac) {
+        if (pl.kc <= tab) {
+            best = static_cast<double>((tiles + sms - 1) / sms) * pl.kc * c1;
+            if (best < hbm_floor) best = hbm_floor;
+        }
+        for (int sfac = 2; sfac <= kMaxClusterSplits && sfac <= pl.kc; ++sfac) {
             const int per_item = (pl.kc + sfac - 1) / sfac;
-            if (per_item > tab) continue;
-            const int64_t rounds = (tiles * sfac + sms - 1) / sms;
-            double t = static_cast<double>(rounds) * per_item * c;
+            if (per_item > tab || tiles > clusters_resident(pl.swap, pl.bn, sfac)) continue;
+            double t = per_item * c;
             if (t < hbm_floor) t = hbm_floor;
-            if (sfac > 1) t += static_cast<double>(rounds) * (e0 + e1 * sfac);
+            t += e;
             if (t < best - 1e-9) {
                 best = t;
                 splits = sfac;
+                pl.cluster = true;
             }
         }
     }
     if (force_split == 0 && (pl.kc + splits - 1) / splits > tab) {
         // the weight-major kernel keeps an item's scales in a shared-memory table: split K until an item fits
         splits = (pl.kc + tab - 1) / tab;
+        pl.cluster = false;
         if (splits > 32 || tiles > kMaxTickets) {
             if (force_kernel == 3) {
                 set_last_error("fp8_gemm: K=%lld is too long for the weight-major kernel's scale table", static_cast<long long>(K));
@@ -891,6 +1054,8 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
 }
 
 size_t tc_workspace_bytes(const TcPlan& pl, int64_t M, int64_t N) {
+    // (A split inside a cluster leaves the workspace untouched; the size is asked for all the same, so that a caller's
+    // buffer does not depend on which form a device or an SM budget makes the plan choose.)
     if (pl.splits <= 1) return 0;
     // one padded tile (128 x bn fp32) per (split, tile)
     (void)M;
@@ -902,7 +1067,7 @@ size_t tc_workspace_bytes(const TcPlan& pl, int64_t M, int64_t N) {
 int launch_fp8_gemm_tc(const void* a, const float* a_s, const void* b, const float* b_s, int64_t M, int64_t N,
                        int64_t K, void* c, void* workspace, size_t workspace_bytes, const TcPlan& pl,
                        cudaStream_t stream) {
-    if (pl.splits > 1) {
+    if (pl.splits > 1 && !pl.cluster) {
         const size_t need = tc_workspace_bytes(pl, M, N);
         if (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) % 256) != 0) {
             set_last_error("fp8_gemm: split-K needs a 256-byte aligned workspace of %zu bytes (got %zu)", need,
@@ -941,6 +1106,7 @@ int launch_fp8_gemm_tc(const void* a, const float* a_s, const void* b, const flo
     prm.tiles_p = pl.tiles_p;
     prm.tiles_q = pl.tiles_q;
     prm.splits = pl.splits;
+    prm.cluster = pl.cluster ? 1 : 0;
     prm.tma_store = tma_store ? 1 : 0;
     // Work order: `raster` token tiles share consecutive weight tiles.  For token-major tiles the group is
     // made as tall as keeps its activations (raster x 128 x K bytes) within about a quarter of L2, so that
@@ -950,6 +1116,7 @@ int launch_fp8_gemm_tc(const void* a, const float* a_s, const void* b, const flo
         const int64_t fit = (32ll << 20) / (static_cast<int64_t>(kPRows) * K);
         prm.raster = static_cast<int>(fit < 8 ? 8 : (fit > 64 ? 64 : fit));
     }
+    prm.div_rows = make_fast_div(static_cast<uint32_t>((kPRows + pl.splits - 1) / pl.splits));
     prm.div_splits = make_fast_div(static_cast<uint32_t>(prm.splits));
     prm.div_raster = make_fast_div(static_cast<uint32_t>(prm.raster));
     prm.div_per_group = make_fast_div(static_cast<uint32_t>(prm.raster) * static_cast<uint32_t>(prm.tiles_q));

@@ -13,6 +13,7 @@ struct TcPlan {
     bool swap;  // true: weights on the MMA M axis (small M)
     bool pair;  // token-major tiles on CTA pairs (fp8_gemm_tm.cu); never with split-K
     bool wide;  // with pair: 256 x 256 tiles (fp8_gemm_tw.cu)
+    bool cluster;   // the splits of a tile form a cluster and meet in shared memory
     int bn;     // rows of the second operand tile
     int tiles_p, tiles_q, splits, kc;
 };
