@@ -435,10 +435,20 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 if (!ok) break;
                 const int n = min(TC, s.c1 - k);
                 float* dst = tab + sl * TC * BN;
-                // columns beyond ntok keep what they held: they multiply products nobody reads
-                for (int i = tid; i < n * BN; i += kTabThreads) {
-                    const int ch = i / BN, col = i - ch * BN;
-                    if (col < s.ntok) dst[i] = __ldg(p.a_s + (s.row0 + col) * p.as_row + (k + ch) * p.as_chunk);
+                // All loads of a slot are in flight together: they queue behind the weights' (one after the other they held
+                // the first chunk back by 7 us).  Columns beyond ntok keep what they held: they multiply products nobody reads.
+                constexpr int kLoads = TC * BN / kTabThreads;
+                static_assert(kTabThreads % BN == 0 || BN % kTabThreads == 0, "a thread's columns do not depend on the trip");
+                float r[kLoads];
+#pragma unroll
+                for (int u = 0; u < kLoads; ++u) {
+                    const int i = tid + u * kTabThreads, ch = i / BN, col = i - ch * BN;
+                    if (ch < n && col < s.ntok) r[u] = __ldg(p.a_s + (s.row0 + col) * p.as_row + (k + ch) * p.as_chunk);
+                }
+#pragma unroll
+                for (int u = 0; u < kLoads; ++u) {
+                    const int i = tid + u * kTabThreads, ch = i / BN, col = i - ch * BN;
+                    if (ch < n && col < s.ntok) dst[i] = r[u];
                 }
                 mbar_arrive(sfull_bar(sl));
             }
