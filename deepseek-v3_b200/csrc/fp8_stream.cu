@@ -71,24 +71,30 @@ struct SCfg {
     static_assert(kTmemCols >= 32 && kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "TMEM columns");
 };
 
-struct StreamParams {
-    // weights: block b of a tile comes from map / scale set b
-    const CUtensorMap* g_map[2];        // grouped: per-group maps, in global memory
-    const float* const* g_scale[2];     // grouped: per-group scale pointers, in global memory
-    const float* scale[2];              // one group
-    const int* seg;                     // grouped: [n_groups + 1] row offsets, in global memory
-    int n_groups;                       // 0: one ordinary weight
-    int M;                              // rows of a
+// A launch works on up to two problems that share the shape of a tile: the groups (per-group weights, rows by group) and
+// one ordinary weight (the shared experts next to the routed ones).
+struct Side {
     int kc, nblk, tiles_p;              // K chunks, 128-row blocks of a weight, tiles per token tile
+    int rows;                           // rows of a (ordinary weight)
     const float* a_s;                   // token scales: a_s[row * as_row + chunk * as_chunk]
     int64_t as_row, as_chunk;
-    // results
     __nv_bfloat16* c;                   // plain: bf16 [rows, N]
     int64_t N;
     int vec_store;                      // rows of c are 16-byte aligned
     uint8_t* hq;                        // SwiGLU: e4m3 [rows, N]
     float* hs;                          // SwiGLU: hs[row * hs_row + block * hs_blk]
     int64_t hs_row, hs_blk;
+};
+constexpr int kGroups = 0, kOrdinary = 1;
+
+struct StreamParams {
+    Side side[2];
+    // groups: block b of a tile comes from map / scale set b, in global memory; row offsets seg[n_groups + 1] likewise
+    const CUtensorMap* g_map[2];
+    const float* const* g_scale[2];
+    const int* seg;
+    int n_groups;                       // 0: none
+    const float* scale[2];              // ordinary weight (its maps are kernel parameters); side[kOrdinary].rows == 0: none
     int scale_fmt;
     // split tiles
     float* partials;                    // [CTA][2][2 * BN / 4][128] float4, or null: whole tiles only
@@ -97,16 +103,19 @@ struct StreamParams {
 };
 
 struct Seg {          // a range of K chunks of one tile
-    int tile, c0, c1;
+    int side, kc, ut; // which problem, its K chunks, the tile's first unit
+    int c0, c1;
     int row0, ntok;   // token rows
     int group, p;     // weight, tile within the weight
 };
 
 // The CTA's share of the work and how tiles are split; every CTA derives the same plan from the same numbers.
-// 32-bit arithmetic throughout (the host checks that tiles * chunks fits): a 64-bit division takes about half a
-// microsecond here, and ranges computed as units * cta / ctas cost a small problem 15 us.
+// A unit is one K chunk of a tile; the groups' tiles come first.  32-bit arithmetic throughout (the host checks that the
+// units fit): a 64-bit division takes about half a microsecond here, and ranges computed as units * cta / ctas cost a
+// small problem 15 us.
 struct Plan {
-    int n_tiles, kc, G;      // G: CTAs that take part
+    int tiles0, tiles1, kc0, kc1;      // groups, ordinary weight
+    int G;                   // CTAs that take part
     bool split;
     int units, base, extra;  // split: the first `extra` CTAs take base + 1 units, the others base
     __device__ __forceinline__ int begin(int cta) const { return cta * base + min(cta, extra); }
@@ -117,16 +126,23 @@ struct Plan {
     }
 };
 
-__device__ __forceinline__ Plan make_plan(int n_tiles, int kc, int ctas, bool may_split) {
+// group_tiles: token tiles over all groups
+template <int BN>
+__device__ __forceinline__ Plan make_plan(const StreamParams& p, int group_tiles) {
     Plan pl;
-    pl.n_tiles = n_tiles;
-    pl.kc = kc;
+    pl.tiles0 = p.side[kGroups].tiles_p * group_tiles;
+    pl.tiles1 = p.side[kOrdinary].tiles_p * ((p.side[kOrdinary].rows + BN - 1) / BN);
+    pl.kc0 = p.side[kGroups].kc;
+    pl.kc1 = p.side[kOrdinary].kc;
+    const int n_tiles = pl.tiles0 + pl.tiles1, ctas = static_cast<int>(gridDim.x);
+    const int longest = max(pl.tiles0 > 0 ? pl.kc0 : 0, pl.tiles1 > 0 ? pl.kc1 : 0);
     pl.G = ctas;
-    pl.units = n_tiles * kc;
+    pl.units = pl.tiles0 * pl.kc0 + pl.tiles1 * pl.kc1;
     pl.base = pl.extra = 0;
     // whole tiles keep at least 15 of 16 CTA-rounds busy: splitting would only add the parked partial tiles
     const int left = n_tiles % ctas;
-    pl.split = may_split && n_tiles > 0 && left != 0 && static_cast<int64_t>(n_tiles) * 16 < static_cast<int64_t>(n_tiles - left + ctas) * 15;
+    const int64_t rounds = static_cast<int64_t>(n_tiles - left + (left ? ctas : 0)) * longest;
+    pl.split = p.partials != nullptr && n_tiles > 0 && static_cast<int64_t>(pl.units) * 16 < rounds * 15;
     if (pl.split) {
         const int g = pl.units / kMinUnits;
         if (g < pl.G) {
@@ -153,46 +169,55 @@ struct Walker {
             u1 = cta < pl.G ? pl.begin(cta + 1) : 0;
         } else {
             u = cta;
-            u1 = pl.n_tiles;
+            u1 = pl.tiles0 + pl.tiles1;
         }
     }
     __device__ __forceinline__ bool next(Seg& s) {
         if (u >= u1) return false;
+        int tile;                // within the side
         if (pl.split) {
-            s.tile = static_cast<int>(static_cast<unsigned>(u) / static_cast<unsigned>(pl.kc));
-            s.c0 = u - s.tile * pl.kc;
-            s.c1 = min(pl.kc, s.c0 + (u1 - u));
+            const int units0 = pl.tiles0 * pl.kc0;
+            s.side = u < units0 ? kGroups : kOrdinary;
+            s.kc = s.side == kGroups ? pl.kc0 : pl.kc1;
+            const int v = s.side == kGroups ? u : u - units0;
+            tile = static_cast<int>(static_cast<unsigned>(v) / static_cast<unsigned>(s.kc));
+            s.ut = u - v + tile * s.kc;
+            s.c0 = u - s.ut;
+            s.c1 = min(s.kc, s.c0 + (u1 - u));
             u += s.c1 - s.c0;
         } else {
-            s.tile = u;
+            s.side = u < pl.tiles0 ? kGroups : kOrdinary;
+            s.kc = s.side == kGroups ? pl.kc0 : pl.kc1;
+            tile = s.side == kGroups ? u : u - pl.tiles0;
+            s.ut = 0;
             s.c0 = 0;
-            s.c1 = pl.kc;
+            s.c1 = s.kc;
             u += pl.G;
         }
-        if (p.n_groups > 0) {
-            // group by binary search over prefix * tiles_p; inside a group the token tile runs fastest, so CTAs that
-            // work side by side share the weight blocks
+        // inside a weight the token tile runs fastest, so CTAs that work side by side share the weight blocks
+        int nq, first, rows;
+        if (s.side == kGroups) {
+            const int per = p.side[kGroups].tiles_p;
             int lo = 0, hi = p.n_groups;
             while (hi - lo > 1) {
                 const int mid = (lo + hi) >> 1;
-                if (prefix[mid] * p.tiles_p <= s.tile) lo = mid; else hi = mid;
+                if (prefix[mid] * per <= tile) lo = mid; else hi = mid;
             }
-            const int nq = prefix[lo + 1] - prefix[lo];
-            const int r = s.tile - prefix[lo] * p.tiles_p;
             s.group = lo;
-            s.p = nq == 1 ? r : r / nq;
-            const int q = r - s.p * nq;
-            const int e1 = __ldg(p.seg + lo + 1);
-            s.row0 = __ldg(p.seg + lo) + q * BN;
-            s.ntok = min(BN, e1 - s.row0);
+            nq = prefix[lo + 1] - prefix[lo];
+            tile -= prefix[lo] * per;
+            first = __ldg(p.seg + lo);
+            rows = __ldg(p.seg + lo + 1) - first;
         } else {
-            const int nq = (p.M + BN - 1) / BN;
             s.group = 0;
-            s.p = nq == 1 ? s.tile : s.tile / nq;
-            const int q = s.tile - s.p * nq;
-            s.row0 = q * BN;
-            s.ntok = min(BN, p.M - s.row0);
+            rows = p.side[kOrdinary].rows;
+            nq = (rows + BN - 1) / BN;
+            first = 0;
         }
+        s.p = nq == 1 ? tile : tile / nq;
+        const int q = tile - s.p * nq;
+        s.row0 = first + q * BN;
+        s.ntok = min(BN, rows - q * BN);
         return true;
     }
 };
@@ -231,14 +256,14 @@ __device__ __forceinline__ void prefix_groups(const StreamParams& p, int* prefix
 // its data all the same).  One thread.
 template <int BN, bool kSwiglu>
 __device__ __forceinline__ void prefetch_weights(const StreamParams& p, const void* w0, const void* w1, const int* prefix, int n) {
-    const Plan pl = make_plan(p.tiles_p * ((p.M + BN - 1) / BN), p.kc, static_cast<int>(gridDim.x), p.partials != nullptr);
+    const Plan pl = make_plan<BN>(p, 0);
     Walker<BN> wk(p, pl, prefix);
     Seg s;
     if (wk.next(s)) {
         const int r0 = (kSwiglu ? s.p : 2 * s.p) * kPRows;
         for (int k = s.c0; k < min(s.c1, s.c0 + n); ++k) {
             tma_prefetch_l2_2d(w0, k * kChunk, r0);
-            if (kSwiglu || 2 * s.p + 1 < p.nblk) tma_prefetch_l2_2d(w1, k * kChunk, kSwiglu ? r0 : r0 + kPRows);
+            if (kSwiglu || 2 * s.p + 1 < p.side[kOrdinary].nblk) tma_prefetch_l2_2d(w1, k * kChunk, kSwiglu ? r0 : r0 + kPRows);
         }
     }
 }
@@ -247,18 +272,19 @@ __device__ __forceinline__ void prefetch_weights(const StreamParams& p, const vo
 // the boxes that hold any of the tile's rows are fetched.
 template <class C, bool kSwiglu>
 __device__ __forceinline__ void produce(const StreamParams& p, const Plan& pl, const int* prefix, const void* w0, const void* w1,
-                                        const void* ta, uint32_t tiles, uint32_t bar0, Control* ctl) {
+                                        const void* ta0, const void* ta1, uint32_t tiles, uint32_t bar0, Control* ctl) {
     constexpr int NS = C::kStages, BN = C::BN;
     Walker<BN> wk(p, pl, prefix);
     Seg s;
     uint32_t g = 0;
     bool ok = true;
     while (ok && wk.next(s)) {
-        const void* m0 = p.n_groups > 0 ? static_cast<const void*>(p.g_map[0] + s.group) : w0;
-        const void* m1 = p.n_groups > 0 ? static_cast<const void*>(p.g_map[1] + s.group) : w1;
+        const void* m0 = s.side == kGroups ? static_cast<const void*>(p.g_map[0] + s.group) : w0;
+        const void* m1 = s.side == kGroups ? static_cast<const void*>(p.g_map[1] + s.group) : w1;
+        const void* ta = s.side == kGroups ? ta0 : ta1;
         const int r0 = (kSwiglu ? s.p : 2 * s.p) * kPRows;
         const int r1 = kSwiglu ? r0 : r0 + kPRows;
-        const bool two = kSwiglu || 2 * s.p + 1 < p.nblk;
+        const bool two = kSwiglu || 2 * s.p + 1 < p.side[s.side].nblk;
         const int boxes = (s.ntok + C::kBox - 1) / C::kBox;
         const uint32_t bytes = (two ? 2u : 1u) * kPRows * kChunk + static_cast<uint32_t>(boxes) * C::kBox * kChunk;
         for (int k = s.c0; k < s.c1; ++k, ++g) {
@@ -323,7 +349,8 @@ __device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_b
 template <int BN, bool kSwiglu>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
-                  const __grid_constant__ CUtensorMap tmap_a, const StreamParams p) {
+                  const __grid_constant__ CUtensorMap tmap_a0, const __grid_constant__ CUtensorMap tmap_a1,
+                  const __grid_constant__ StreamParams p) {
     using C = SCfg<BN, false>;
     constexpr int NS = C::kStages, NT = C::kSlots, TC = C::kTabChunks;
     constexpr int PW = BN == 16 ? 8 : 16;  // tokens per piece
@@ -365,8 +392,9 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         }
         ctl->abort_flag = 0;
         mbar_fence_init();
-        tma_prefetch_desc(&tmap_a);
-        if (p.n_groups == 0) {
+        if (p.n_groups > 0) tma_prefetch_desc(&tmap_a0);
+        if (p.side[kOrdinary].rows > 0) {
+            tma_prefetch_desc(&tmap_a1);
             tma_prefetch_desc(&tmap_w0);
             tma_prefetch_desc(&tmap_w1);
         }
@@ -380,13 +408,12 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
-    const int n_tiles = p.tiles_p * (p.n_groups > 0 ? prefix[kMaxGroups] : (p.M + BN - 1) / BN);
-    const Plan pl = make_plan(n_tiles, p.kc, static_cast<int>(gridDim.x), p.partials != nullptr);
+    const Plan pl = make_plan<BN>(p, p.n_groups > 0 ? prefix[kMaxGroups] : 0);
 
     if (warp < kFirstPromoWarp) {
       if constexpr (NP >= 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
       if (warp == 0) {
-        produce<C, kSwiglu>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a, tiles, bar0, ctl);
+        produce<C, kSwiglu>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
       } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         Walker<BN> wk(p, pl, prefix);
@@ -394,7 +421,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         uint32_t g = 0;
         bool ok = true;
         while (ok && wk.next(s)) {
-            const bool two = kSwiglu || 2 * s.p + 1 < p.nblk;
+            const bool two = kSwiglu || 2 * s.p + 1 < p.side[s.side].nblk;
             const uint32_t idesc = umma_idesc_e4m3_f32(kPRows, 16) + ((static_cast<uint32_t>(s.ntok + 15) / 16 - 1) << 18);   // N in units of 8 at bit 17
             for (int k = s.c0; k < s.c1; ++k, ++g) {
                 const int st = g % NS, ts = g % NT;
@@ -429,6 +456,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         bool ok = true;
         const int tid = threadIdx.x - 64;
         while (ok && wk.next(s)) {
+            const Side& d = p.side[s.side];
             for (int k = s.c0; k < s.c1; k += TC, ++t) {
                 const int sl = t & 1;
                 ok = __all_sync(0xffffffffu, bounded_wait(sempty_bar(sl), ((t >> 1) & 1u) ^ 1u, ctl, p.status, 7, t));
@@ -443,7 +471,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
 #pragma unroll
                 for (int u = 0; u < kLoads; ++u) {
                     const int i = tid + u * kTabThreads, ch = i / BN, col = i - ch * BN;
-                    if (ch < n && col < s.ntok) r[u] = __ldg(p.a_s + (s.row0 + col) * p.as_row + (k + ch) * p.as_chunk);
+                    if (ch < n && col < s.ntok) r[u] = __ldg(d.a_s + (s.row0 + col) * d.as_row + (k + ch) * d.as_chunk);
                 }
 #pragma unroll
                 for (int u = 0; u < kLoads; ++u) {
@@ -492,10 +520,11 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
             }
         };
         while (ok && wk.next(s)) {
-            const bool two = kSwiglu || 2 * s.p + 1 < p.nblk;
-            const float* b0 = (p.n_groups > 0 ? p.g_scale[0][s.group] : p.scale[0]) + static_cast<int64_t>(kSwiglu ? s.p : 2 * s.p) * p.kc;
-            const float* b1 = (p.n_groups > 0 ? p.g_scale[1][s.group] : p.scale[1]) +
-                              static_cast<int64_t>(kSwiglu ? s.p : (two ? 2 * s.p + 1 : 2 * s.p)) * p.kc;
+            const bool two = kSwiglu || 2 * s.p + 1 < p.side[s.side].nblk;
+            const Side& d = p.side[s.side];
+            const float* b0 = (s.side == kGroups ? p.g_scale[0][s.group] : p.scale[0]) + static_cast<int64_t>(kSwiglu ? s.p : 2 * s.p) * s.kc;
+            const float* b1 = (s.side == kGroups ? p.g_scale[1][s.group] : p.scale[1]) +
+                              static_cast<int64_t>(kSwiglu ? s.p : (two ? 2 * s.p + 1 : 2 * s.p)) * s.kc;
             // pieces of this thread that hold a token of the tile
             const int np = s.ntok <= col0 ? 0 : min(NP, (s.ntok - col0 + 2 * PW - 1) / (2 * PW));
 #pragma unroll
@@ -557,15 +586,14 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
             }
             if (!ok) break;
 
-            if (n_ch < p.kc) {
+            if (n_ch < s.kc) {
                 // part of a tile: park the pieces that hold tokens, take a ticket; the last part of the tile adds all
                 // parts in K order and goes on to write the result
                 const int cta = static_cast<int>(blockIdx.x);
-                const int ut = s.tile * pl.kc;
-                const int first = pl.owner(ut), last = pl.owner(ut + pl.kc - 1);
+                const int first = pl.owner(s.ut), last = pl.owner(s.ut + s.kc - 1);
                 constexpr int kTileVec = 2 * BN / 4 * kPRows;             // float4 per parked tile: [2 blocks][BN / 4][128 rows]
                 float4* base = reinterpret_cast<float4*>(p.partials) + (col0 / 4) * kPRows + row;
-                auto part = [&](int c) { return base + (static_cast<int64_t>(c) * 2 + (pl.begin(c) >= ut ? 0 : 1)) * kTileVec; };
+                auto part = [&](int c) { return base + (static_cast<int64_t>(c) * 2 + (pl.begin(c) >= s.ut ? 0 : 1)) * kTileVec; };
                 {
                     float4* dst = part(cta);
 #pragma unroll
@@ -616,15 +644,15 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     const int64_t n = static_cast<int64_t>(2 * s.p + b) * kPRows + row;
-                    if (n < p.N) {
-                        __nv_bfloat16* out = p.c + (static_cast<int64_t>(s.row0) + col0) * p.N + n;
+                    if (n < d.N) {
+                        __nv_bfloat16* out = d.c + (static_cast<int64_t>(s.row0) + col0) * d.N + n;
 #pragma unroll
                         for (int i = 0; i < NP; ++i) {
                             if (i >= np) continue;
 #pragma unroll
                             for (int j = 0; j < PW; ++j)
                                 if (col0 + 2 * PW * i + j < s.ntok)
-                                    out[(2 * PW * i + j) * p.N] = __float2bfloat16_rn(j & 1 ? acc[b][i][j / 2].y : acc[b][i][j / 2].x);
+                                    out[(2 * PW * i + j) * d.N] = __float2bfloat16_rn(j & 1 ? acc[b][i][j / 2].y : acc[b][i][j / 2].x);
                         }
                     }
                 }
@@ -681,11 +709,11 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                         const float m = fmaxf(fmaxf(red[tk], red[BN + tk]), fmaxf(red[2 * BN + tk], red[3 * BN + tk]));
                         const float sc = scale_from_amax(m, p.scale_fmt);
                         red[4 * BN + tk] = p.scale_fmt == DSV3_SCALE_FMT_FP32 ? rcp_approx(sc) : sc;
-                        p.hs[(static_cast<int64_t>(s.row0) + tk) * p.hs_row + s.p * p.hs_blk] = sc;
+                        d.hs[(static_cast<int64_t>(s.row0) + tk) * d.hs_row + s.p * d.hs_blk] = sc;
                     }
                 }
                 asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
-                uint8_t* out = p.hq + static_cast<int64_t>(s.row0) * p.N + static_cast<int64_t>(s.p) * kPRows + row;
+                uint8_t* out = d.hq + static_cast<int64_t>(s.row0) * d.N + static_cast<int64_t>(s.p) * kPRows + row;
 #pragma unroll 1
                 for (int q = 0; q < NG; ++q) {
                     const int tk = token(q), rem = s.ntok - tk;
@@ -697,8 +725,8 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                             const float s0 = sc[2 * e], s1 = sc[2 * e + 1];
                             const bool mul = p.scale_fmt == DSV3_SCALE_FMT_FP32;
                             const uint32_t two8 = cvt_e4m3x2(mul ? __fmul_rn(lo, s0) : div_full(lo, s0), mul ? __fmul_rn(hi, s1) : div_full(hi, s1));
-                            if (2 * e < rem) out[(tk + 2 * e) * p.N] = static_cast<uint8_t>(two8 & 0xFFu);
-                            if (2 * e + 1 < rem) out[(tk + 2 * e + 1) * p.N] = static_cast<uint8_t>(two8 >> 8);
+                            if (2 * e < rem) out[(tk + 2 * e) * d.N] = static_cast<uint8_t>(two8 & 0xFFu);
+                            if (2 * e + 1 < rem) out[(tk + 2 * e + 1) * d.N] = static_cast<uint8_t>(two8 >> 8);
                         }
                     }
 #pragma unroll
@@ -723,7 +751,8 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
 template <int BN, bool kSwiglu>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
-                const __grid_constant__ CUtensorMap tmap_a, const StreamParams p) {
+                const __grid_constant__ CUtensorMap tmap_a0, const __grid_constant__ CUtensorMap tmap_a1,
+                  const __grid_constant__ StreamParams p) {
     using C = SCfg<BN, true>;
     constexpr int NS = C::kStages, NT = C::kSlots;
     extern __shared__ uint8_t smem_raw[];
@@ -755,8 +784,9 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
         }
         ctl->abort_flag = 0;
         mbar_fence_init();
-        tma_prefetch_desc(&tmap_a);
-        if (p.n_groups == 0) {
+        if (p.n_groups > 0) tma_prefetch_desc(&tmap_a0);
+        if (p.side[kOrdinary].rows > 0) {
+            tma_prefetch_desc(&tmap_a1);
             tma_prefetch_desc(&tmap_w0);
             tma_prefetch_desc(&tmap_w1);
         }
@@ -770,13 +800,12 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
-    const int n_tiles = p.tiles_p * (p.n_groups > 0 ? prefix[kMaxGroups] : (p.M + BN - 1) / BN);
-    const Plan pl = make_plan(n_tiles, p.kc, static_cast<int>(gridDim.x), p.partials != nullptr);
+    const Plan pl = make_plan<BN>(p, p.n_groups > 0 ? prefix[kMaxGroups] : 0);
 
     if (warp < kFirstPromoWarp) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
         if (warp == 0) {
-            produce<C, kSwiglu>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a, tiles, bar0, ctl);
+            produce<C, kSwiglu>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
         } else if (warp == 1) {
             // -------------------------------------------------------- MMA issuer
             Walker<BN> wk(p, pl, prefix);
@@ -784,7 +813,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
             uint32_t g = 0;
             bool ok = true;
             while (ok && wk.next(s)) {
-                const bool two = kSwiglu || 2 * s.p + 1 < p.nblk;
+                const bool two = kSwiglu || 2 * s.p + 1 < p.side[s.side].nblk;
                 const uint32_t idesc = two ? umma_idesc_e4m3_f32(kPRows, 2 * kPRows) : umma_idesc_e4m3_f32(kPRows, kPRows);
                 for (int k = s.c0; k < s.c1; ++k, ++g) {
                     const int st = g % NS, ts = g % NT;
@@ -839,15 +868,18 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
         // 0.6 us, and with one chunk of look-ahead every chunk waited for it (1330 cycles instead of 700).  A tile's
         // first scales are requested before the result of the tile before it is written.
         const float *as = nullptr, *bs = nullptr;
+        int64_t as_chunk = 0;
         float ra[4], rb;         // rb: the weight block's scale of the next chunk (32 chunks to a cache line: L1)
         auto scales_of = [&](const Seg& q) {
             const int blk = kSwiglu ? q.p : 2 * q.p + grp;
-            as = p.a_s + (q.row0 + min(row, q.ntok - 1)) * p.as_row + q.c0 * p.as_chunk;
-            bs = (p.n_groups > 0 ? p.g_scale[grp][q.group] : p.scale[grp]) + static_cast<int64_t>(min(blk, p.nblk - 1)) * p.kc + q.c0;
+            const Side& d = p.side[q.side];
+            as_chunk = d.as_chunk;
+            as = d.a_s + (q.row0 + min(row, q.ntok - 1)) * d.as_row + q.c0 * as_chunk;
+            bs = (q.side == kGroups ? p.g_scale[grp][q.group] : p.scale[grp]) + static_cast<int64_t>(min(blk, d.nblk - 1)) * q.kc + q.c0;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int k = min(i, q.c1 - q.c0 - 1);
-                ra[i] = __ldg(as + k * p.as_chunk);
+                ra[i] = __ldg(as + k * as_chunk);
             }
             rb = __ldg(bs);
         };
@@ -855,8 +887,9 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
         if (more) scales_of(ahead);
         while (ok && more) {
             s = ahead;
+            const Side& d = p.side[s.side];
             const int blk = kSwiglu ? s.p : 2 * s.p + grp;
-            const bool active = quarter * 32 < s.ntok && blk < p.nblk;     // uniform in the warp
+            const bool active = quarter * 32 < s.ntok && blk < d.nblk;     // uniform in the warp
             const int n_ch = s.c1 - s.c0;
 #pragma unroll
             for (int j = 0; j < 64; ++j) acc[j] = make_float2(0.0f, 0.0f);
@@ -877,7 +910,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
                     const uint32_t taddr = t_lane + ts * 256;
                     tc_ld_x64(taddr, v);
                     const float sc = ra[i] * rb;
-                    ra[i] = __ldg(as + min(k + 4, n_ch - 1) * p.as_chunk);
+                    ra[i] = __ldg(as + min(k + 4, n_ch - 1) * as_chunk);
                     rb = __ldg(bs + min(k + 1, n_ch - 1));
                     tc_wait_ld();
                     fold(sc, 0);
@@ -891,15 +924,14 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
             more = wk.next(ahead);
             if (more) scales_of(ahead);
 
-            if (n_ch < p.kc) {
+            if (n_ch < s.kc) {
                 // part of a tile: park the valid rows, take a ticket; the last part of the tile adds all parts in K
                 // order and goes on to write the result
                 const int cta = static_cast<int>(blockIdx.x);
-                const int ut = s.tile * pl.kc;
-                const int first = pl.owner(ut), last = pl.owner(ut + pl.kc - 1);
+                const int first = pl.owner(s.ut), last = pl.owner(s.ut + s.kc - 1);
                 constexpr int kTileVec = 256 * BN / 4;                     // float4 per parked tile: [64 column groups][BN rows]
                 float4* base = reinterpret_cast<float4*>(p.partials) + grp * 32 * BN + row;
-                auto part = [&](int c) { return base + (static_cast<int64_t>(c) * 2 + (pl.begin(c) >= ut ? 0 : 1)) * kTileVec; };
+                auto part = [&](int c) { return base + (static_cast<int64_t>(c) * 2 + (pl.begin(c) >= s.ut ? 0 : 1)) * kTileVec; };
                 const bool mine_row = active && row < s.ntok;
                 if (mine_row) {
                     float4* dst = part(cta);
@@ -949,14 +981,14 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
                         const int r = r0 + (lane >> 3);
                         if (quarter * 32 + r >= s.ntok) continue;
                         const uint4 o = *reinterpret_cast<const uint4*>(wbuf + r * 128 + ((piece ^ (r & 7)) << 4));
-                        __nv_bfloat16* dst = p.c + (static_cast<int64_t>(s.row0) + quarter * 32 + r) * p.N + n;
-                        if (p.vec_store && n + 8 <= p.N) {
+                        __nv_bfloat16* dst = d.c + (static_cast<int64_t>(s.row0) + quarter * 32 + r) * d.N + n;
+                        if (d.vec_store && n + 8 <= d.N) {
                             *reinterpret_cast<uint4*>(dst) = o;
                         } else {
                             const uint32_t w4[4] = {o.x, o.y, o.z, o.w};
 #pragma unroll
                             for (int e = 0; e < 8; ++e)
-                                if (n + e < p.N) reinterpret_cast<uint16_t*>(dst)[e] = static_cast<uint16_t>(w4[e >> 1] >> (16 * (e & 1)));
+                                if (n + e < d.N) reinterpret_cast<uint16_t*>(dst)[e] = static_cast<uint16_t>(w4[e >> 1] >> (16 * (e & 1)));
                         }
                     }
                 }
@@ -1005,8 +1037,8 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
                 if (row < s.ntok) {
                     const float scale = scale_from_amax(m, p.scale_fmt);
                     const int64_t tok = static_cast<int64_t>(s.row0) + row;
-                    if (grp == 0) p.hs[tok * p.hs_row + s.p * p.hs_blk] = scale;
-                    uint4* out = reinterpret_cast<uint4*>(p.hq + tok * p.N + static_cast<int64_t>(s.p) * kPRows + grp * 64);
+                    if (grp == 0) d.hs[tok * d.hs_row + s.p * d.hs_blk] = scale;
+                    uint4* out = reinterpret_cast<uint4*>(d.hq + tok * d.N + static_cast<int64_t>(s.p) * kPRows + grp * 64);
 #pragma unroll 1
                     for (int c = 0; c < 4; ++c) {
                         const uint4 a = make_uint4(v[0], v[1], v[2], v[3]);
@@ -1031,8 +1063,8 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
 }
 
 template <int BN, bool kSwiglu, bool kRows>
-int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta, const StreamParams& prm, int64_t tiles_bound,
-                   cudaStream_t stream) {
+int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, const StreamParams& prm,
+                   int64_t tiles_bound, int64_t units_bound, cudaStream_t stream) {
     using C = SCfg<BN, kRows>;
     constexpr auto pick = [] {
         if constexpr (kRows) return fp8_rows_kernel<BN, kSwiglu>;
@@ -1051,9 +1083,9 @@ int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorM
         configured[dev] = true;
     }
     int64_t grid = num_sms();
-    const int64_t most = prm.partials ? tiles_bound * prm.kc : tiles_bound;      // no more CTAs than there can be work for
+    const int64_t most = prm.partials ? units_bound : tiles_bound;      // no more CTAs than there can be work for
     if (grid > most) grid = most;
-    DSV3_CUDA_TRY(launch_dependent(kern, dim3(static_cast<unsigned>(grid)), dim3(kNumThreads), C::kSmemBytes, stream, w0, w1, ta, prm));
+    DSV3_CUDA_TRY(launch_dependent(kern, dim3(static_cast<unsigned>(grid)), dim3(kNumThreads), C::kSmemBytes, stream, w0, w1, ta0, ta1, prm));
     return DSV3_OK;
 }
 
@@ -1073,64 +1105,77 @@ size_t stream_workspace_bytes(int64_t rows_per_group) {
     return DSV3_WORKSPACE_HEADER_BYTES + static_cast<size_t>(num_sms()) * 2 * (2 * bn) * kPRows * sizeof(float);
 }
 
+static int fill_side(Side& d, CUtensorMap* map, const StreamSide& q, bool swiglu, int bn) {
+    const int rc = make_tmap(map, q.a, q.rows, q.K, bn < 32 ? bn : 32);
+    if (rc != DSV3_OK) return rc;
+    d.kc = static_cast<int>((q.K + kChunk - 1) / kChunk);
+    d.nblk = static_cast<int>((q.N + kPRows - 1) / kPRows);
+    d.tiles_p = swiglu ? d.nblk : (d.nblk + 1) / 2;
+    d.rows = static_cast<int>(q.rows);
+    d.a_s = q.a_s;
+    d.as_row = q.as_row;
+    d.as_chunk = q.as_chunk;
+    d.c = static_cast<__nv_bfloat16*>(q.c);
+    d.N = q.N;
+    d.vec_store = (q.N % 8) == 0 && (reinterpret_cast<uintptr_t>(q.c) % 16) == 0;
+    d.hq = static_cast<uint8_t*>(q.hq);
+    d.hs = q.hs;
+    d.hs_row = q.hs_row;
+    d.hs_blk = q.hs_blk;
+    return DSV3_OK;
+}
+
 int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
     StreamParams prm;
     memset(&prm, 0, sizeof(prm));
-    CUtensorMap w0, w1, ta;
+    CUtensorMap w0, w1, ta0, ta1;
     memset(&w0, 0, sizeof(w0));
     memset(&w1, 0, sizeof(w1));
+    memset(&ta0, 0, sizeof(ta0));
+    memset(&ta1, 0, sizeof(ta1));
     int rc;
-    const int n = q.n_groups > 0 ? q.n_groups : 1;
-    const int bn = stream_tile((q.rows_expected + n - 1) / n);
-    const int box = bn < 32 ? bn : 32;
-    if ((rc = make_tmap(&ta, q.a, q.rows, q.K, box)) != DSV3_OK) return rc;
-    prm.kc = static_cast<int>((q.K + kChunk - 1) / kChunk);
-    prm.nblk = static_cast<int>((q.N + kPRows - 1) / kPRows);
-    prm.tiles_p = q.swiglu ? prm.nblk : (prm.nblk + 1) / 2;
+    const bool ordinary = q.ordinary.rows > 0;
+    const int64_t per_tile = q.n_groups > 0 ? (q.rows_expected + q.n_groups - 1) / q.n_groups : q.ordinary.rows;
+    const int bn = stream_tile(per_tile);
+    int64_t tiles[2] = {0, 0};
     if (q.n_groups > 0) {
+        if ((rc = fill_side(prm.side[kGroups], &ta0, q.groups, q.swiglu, bn)) != DSV3_OK) return rc;
         for (int b = 0; b < 2; ++b) {
             const void* tbl = (b == 1 && q.swiglu) ? q.table1 : q.table0;
             prm.g_map[b] = static_cast<const CUtensorMap*>(tbl);
             prm.g_scale[b] = reinterpret_cast<const float* const*>(static_cast<const uint8_t*>(tbl) + static_cast<size_t>(q.n_groups) * sizeof(CUtensorMap));
         }
         prm.seg = q.seg;
-    } else {
-        if ((rc = make_tmap(&w0, q.w0, q.N, q.K, kPRows)) != DSV3_OK) return rc;
-        if ((rc = make_tmap(&w1, q.swiglu ? q.w1 : q.w0, q.N, q.K, kPRows)) != DSV3_OK) return rc;
+        // token tiles: at most one partly filled tile per group on top of the full ones, and never more groups than rows
+        const int64_t rows = q.groups.rows;
+        tiles[0] = (rows / bn + (q.n_groups < rows ? q.n_groups : rows)) * prm.side[kGroups].tiles_p;
+    }
+    if (ordinary) {
+        const StreamSide& d = q.ordinary;
+        if ((rc = fill_side(prm.side[kOrdinary], &ta1, d, q.swiglu, bn)) != DSV3_OK) return rc;
+        if ((rc = make_tmap(&w0, q.w0, d.N, d.K, kPRows)) != DSV3_OK) return rc;
+        if ((rc = make_tmap(&w1, q.swiglu ? q.w1 : q.w0, d.N, d.K, kPRows)) != DSV3_OK) return rc;
         prm.scale[0] = q.w0_s;
         prm.scale[1] = q.swiglu ? q.w1_s : q.w0_s;
+        tiles[1] = (d.rows + bn - 1) / bn * prm.side[kOrdinary].tiles_p;
     }
     prm.n_groups = q.n_groups;
-    prm.M = static_cast<int>(q.rows);
-    prm.a_s = q.a_s;
-    prm.as_row = q.as_row;
-    prm.as_chunk = q.as_chunk;
-    prm.c = static_cast<__nv_bfloat16*>(q.c);
-    prm.N = q.N;
-    prm.vec_store = (q.N % 8) == 0 && (reinterpret_cast<uintptr_t>(q.c) % 16) == 0;
-    prm.hq = static_cast<uint8_t*>(q.hq);
-    prm.hs = q.hs;
-    prm.hs_row = q.hs_row;
-    prm.hs_blk = q.hs_blk;
     prm.scale_fmt = q.scale_fmt;
     prm.status = status_device_ptr();
     if (!prm.status) return DSV3_ERR_CUDA;
-    const size_t need = stream_workspace_bytes((q.rows_expected + n - 1) / n);
-    if (need > 0 && q.workspace && q.workspace_bytes >= need && (reinterpret_cast<uintptr_t>(q.workspace) % 256) == 0) {
+    const size_t need = stream_workspace_bytes(per_tile);
+    if (q.workspace && q.workspace_bytes >= need && (reinterpret_cast<uintptr_t>(q.workspace) % 256) == 0) {
         prm.tickets = static_cast<int*>(q.workspace);
         prm.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(q.workspace) + DSV3_WORKSPACE_HEADER_BYTES);
     }
-    // token tiles: at most one partly filled tile per group on top of the full ones, and never more groups than rows
-    const int64_t slots = q.n_groups > 0 ? q.rows / bn + (q.n_groups < q.rows ? q.n_groups : q.rows) : (q.rows + bn - 1) / bn;
-    const int64_t tiles_bound = slots * prm.tiles_p;
-    if (tiles_bound * prm.kc >= (1ll << 31)) {
-        set_last_error("fp8 stream GEMM: %lld tiles of %d K chunks are more than the work-item counter holds",
-                       static_cast<long long>(tiles_bound), prm.kc);
+    const int64_t units = tiles[0] * prm.side[kGroups].kc + tiles[1] * prm.side[kOrdinary].kc;
+    if (units >= (1ll << 31)) {
+        set_last_error("fp8 stream GEMM: %lld K chunks are more than the work-item counter holds", static_cast<long long>(units));
         return DSV3_ERR_UNSUPPORTED;
     }
-#define DSV3_STREAM_CASE(BN_, ROWS_)                                                                     \
-    return q.swiglu ? launch_variant<BN_, true, ROWS_>(w0, w1, ta, prm, tiles_bound, stream) \
-                    : launch_variant<BN_, false, ROWS_>(w0, w1, ta, prm, tiles_bound, stream)
+#define DSV3_STREAM_CASE(BN_, ROWS_)                                                                                            \
+    return q.swiglu ? launch_variant<BN_, true, ROWS_>(w0, w1, ta0, ta1, prm, tiles[0] + tiles[1], units, stream)  \
+                    : launch_variant<BN_, false, ROWS_>(w0, w1, ta0, ta1, prm, tiles[0] + tiles[1], units, stream)
     switch (bn) {
         case 16: DSV3_STREAM_CASE(16, false);
         case 32: DSV3_STREAM_CASE(32, false);

@@ -49,23 +49,28 @@ bool small_linear_supported(const void* act, const void* w, const void* c, int64
 int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, const void* w, const float* w_s, int64_t M,
                             int64_t N, int64_t K, int scale_fmt, void* c, cudaStream_t stream);
 
-// Weight-streaming GEMM (fp8_stream.cu): groups of rows against per-group weights, or one weight; optionally with
-// SwiGLU of two weights and quantisation of the product in the epilogue.
-struct StreamGemm {
+// Weight-streaming GEMM (fp8_stream.cu): groups of rows against per-group weights and, in the same launch, one ordinary
+// weight; optionally with SwiGLU of two weights and quantisation of the product in the epilogue.
+struct StreamSide {
     const void* a;                     // e4m3 [rows, K]
     const float* a_s;                  // token scales at a_s[row * as_row + chunk * as_chunk]
     int64_t as_row, as_chunk;
-    int64_t rows, rows_expected, N, K;
-    int n_groups;                      // 0: one weight (w0, w0_s, w1, w1_s); otherwise tables and seg
-    const void *table0, *table1;       // group tables; table1 only with swiglu
-    const int* seg;                    // device memory
-    const void *w0, *w1;               // e4m3 [N, K]; w1 only with swiglu
-    const float *w0_s, *w1_s;
-    bool swiglu;
+    int64_t rows, N, K;
     void* c;                           // bf16 [rows, N]                   -- plain
     void* hq;                          // e4m3 [rows, N]                   -- swiglu
     float* hs;                         // hs[row * hs_row + block * hs_blk] -- swiglu
     int64_t hs_row, hs_blk;
+};
+struct StreamGemm {
+    StreamSide groups;
+    int n_groups;                      // 0: no groups
+    int64_t rows_expected;             // rows the groups are expected to own together
+    const void *table0, *table1;       // group tables; table1 only with swiglu
+    const int* seg;                    // device memory
+    StreamSide ordinary;               // rows == 0: none
+    const void *w0, *w1;               // e4m3 [N, K]; w1 only with swiglu
+    const float *w0_s, *w1_s;
+    bool swiglu;
     int scale_fmt;
     void* workspace;                   // stream_workspace_bytes(), or null: tiles are not split
     size_t workspace_bytes;

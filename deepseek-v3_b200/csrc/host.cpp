@@ -365,14 +365,19 @@ struct Routed {
     at::Tensor arena, x;
     int64_t T, dim;
     int topk;
-    const void *o, *w;
+    const void *o, *w, *z = nullptr;      // z: the shared experts' output when the pass computed it
     const int32_t* pos;
 };
 const char* kRoutedName = "dsv3_b200.routed";
 void free_routed(PyObject* c) { delete static_cast<Routed*>(PyCapsule_GetPointer(c, kRoutedName)); }
 
+// Weights and scales of the shared experts, to be worked on in the same launches (w1, w3, w2).
+struct Shared {
+    at::Tensor w[3], s[3];
+};
+
 std::unique_ptr<Routed> run_experts(Experts& e, const at::Tensor& x_in, const at::Tensor& weights_in, const at::Tensor& indices_in,
-                                    int64_t n_routed, bool assume_no_inplace) {
+                                    int64_t n_routed, bool assume_no_inplace, const Shared* sh) {
     if (indices_in.dim() != 2 || weights_in.sizes() != indices_in.sizes())
         raise(PyExc_ValueError, "routing weights and indices must both be [tokens, top-k]");
     const c10::Device dev = require_cuda(x_in, weights_in, indices_in, e.table1);
@@ -399,6 +404,8 @@ std::unique_ptr<Routed> run_experts(Experts& e, const at::Tensor& x_in, const at
     };
     const int64_t o_seg = take(4 * (e.n + 1)), o_pos = take(4 * P), o_w = take(2 * P), o_xq = take(P * dim), o_xs = take(4 * P * (dim / 128)),
                   o_hq = take(P * inter), o_hs = take(4 * P * (inter / 128)), o_o = take(2 * P * dim);
+    const int64_t inter_s = sh ? sh->w[0].size(0) : 0;
+    const int64_t o_zh = take(T * inter_s), o_zs = take(4 * T * (inter_s / 128)), o_z = take(sh ? 2 * T * dim : 0);
     r->arena = new_cuda({std::max<int64_t>(at, 1)}, at::kByte, dev);
     uint8_t* base = static_cast<uint8_t*>(r->arena.data_ptr());
     r->o = base + o_o;
@@ -422,12 +429,21 @@ std::unique_ptr<Routed> run_experts(Experts& e, const at::Tensor& x_in, const at
     const auto* ip = static_cast<const int64_t*>(indices.const_data_ptr());
     void* xqp = xq.data_ptr();
     float* xsp = static_cast<float*>(xs.data_ptr());
+    dsv3_side_gemm_t up = {}, down = {};
+    if (sh) {
+        up = {xqp, xsp, 0, T, inter_s, dim, sh->w[0].const_data_ptr(), static_cast<const float*>(sh->s[0].const_data_ptr()),
+              sh->w[1].const_data_ptr(), static_cast<const float*>(sh->s[1].const_data_ptr()), base + o_zh, reinterpret_cast<float*>(base + o_zs)};
+        down = {base + o_zh, reinterpret_cast<const float*>(base + o_zs), 1, T, dim, inter_s, sh->w[2].const_data_ptr(),
+                static_cast<const float*>(sh->s[2].const_data_ptr()), nullptr, nullptr, base + o_z, nullptr};
+        r->z = base + o_z;
+    }
     call_library(dev, [&](dsv3_stream_t st) {
         int rc = dsv3_moe_dispatch(xp, T, dim, ip, wp, bf16, r->topk, e.start, e.n, e.fmt, seg, reinterpret_cast<int32_t*>(base + o_pos),
                                    base + o_w, xqp, xsp, base + o_xq, xs_t, st);
         if (rc == DSV3_OK)
-            rc = dsv3_swiglu_gemm_rows(t1, t3, e.n, base + o_xq, xs_t, seg, P, hint, inter, dim, e.fmt, base + o_hq, hs_t, ws, ws_bytes, st);
-        if (rc == DSV3_OK) rc = dsv3_fp8_gemm_rows(t2, e.n, base + o_hq, hs_t, seg, P, hint, dim, inter, base + o_o, ws, ws_bytes, st);
+            rc = dsv3_swiglu_gemm_rows(t1, t3, e.n, base + o_xq, xs_t, seg, P, hint, inter, dim, e.fmt, base + o_hq, hs_t, sh ? &up : nullptr, ws,
+                                       ws_bytes, st);
+        if (rc == DSV3_OK) rc = dsv3_fp8_gemm_rows(t2, e.n, base + o_hq, hs_t, seg, P, hint, dim, inter, base + o_o, sh ? &down : nullptr, ws, ws_bytes, st);
         return rc;
     });
     if (x_in.is_contiguous()) remember(x_in, 128, e.fmt, assume_no_inplace, xq, xs);
@@ -601,24 +617,45 @@ PyObject* py_experts_current(PyObject*, PyObject* capsule) {
     return guarded([&]() -> PyObject* { return PyBool_FromLong(experts_arg(capsule)->current()); });
 }
 
-// (experts, x, weights, indices, n_routed, assume_no_inplace) -> result to hand to `combine`
+// (experts, x, weights, indices, n_routed, assume_no_inplace, shared or None) -> result to hand to `combine`
+// shared: (w1, w3, w2) weights with their scales as attributes
 PyObject* py_run_experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
-        want_args(n, 6);
-        auto r = run_experts(*experts_arg(args[0]), tensor_arg(args[1]), tensor_arg(args[2]), tensor_arg(args[3]), int_arg(args[4]),
-                             PyObject_IsTrue(args[5]) == 1);
+        want_args(n, 7);
+        Experts& e = *experts_arg(args[0]);
+        Shared sh;
+        const bool with_shared = args[6] != Py_None;
+        if (with_shared) {
+            if (!PyTuple_Check(args[6]) || PyTuple_GET_SIZE(args[6]) != 3) raise(PyExc_TypeError, "shared is a tuple of three weights");
+            for (int i = 0; i < 3; ++i) {
+                PyObject* w = PyTuple_GET_ITEM(args[6], i);
+                sh.w[i] = tensor_arg(w);
+                PyObject* sc = PyObject_GetAttr(w, g_attr_scale);
+                if (!sc) throw PythonError{};
+                if (THPVariable_Check(sc)) sh.s[i] = THPVariable_Unpack(sc);
+                Py_DECREF(sc);
+                if (!sh.s[i].defined() || !sh.w[i].is_contiguous() || !sh.s[i].is_contiguous() || sh.s[i].scalar_type() != at::kFloat)
+                    raise(PyExc_ValueError, "shared weights and scales must be contiguous, scales float32");
+            }
+            require_cuda(e.table1, sh.w[0], sh.w[1], sh.w[2], sh.s[0], sh.s[1], sh.s[2]);
+            const int64_t f = sh.w[0].size(0);
+            if (sh.w[0].size(1) != e.dim || sh.w[1].sizes() != sh.w[0].sizes() || sh.w[2].size(0) != e.dim || sh.w[2].size(1) != f || f % 128 != 0)
+                raise(PyExc_ValueError, "shared weights do not fit the layer");
+        }
+        auto r = run_experts(e, tensor_arg(args[1]), tensor_arg(args[2]), tensor_arg(args[3]), int_arg(args[4]),
+                             PyObject_IsTrue(args[5]) == 1, with_shared ? &sh : nullptr);
         return PyCapsule_New(r.release(), kRoutedName, free_routed);
     });
 }
 
-// (result of run_experts, z or None): the tokens' weighted sums, plus z
+// (result of run_experts, z or None): the tokens' weighted sums, plus z (or the shared experts' output computed along)
 PyObject* py_combine(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         want_args(n, 2);
         auto* r = static_cast<Routed*>(PyCapsule_GetPointer(args[0], kRoutedName));
         if (!r) throw PythonError{};
         const c10::Device dev = r->arena.device();
-        const void* zp = nullptr;
+        const void* zp = r->z;
         if (args[1] != Py_None) {
             const at::Tensor& z = tensor_arg(args[1]);
             if (!z.is_contiguous() || z.scalar_type() != at::kBFloat16 || z.device() != dev || z.numel() != r->T * r->dim)
@@ -669,7 +706,7 @@ PyMethodDef methods[] = {
      "(n, start, dim, inter, scale_fmt, table1, table3, table2, list, members, lookups, weights)"},
     {"experts_current", py_experts_current, METH_O, "whether the experts are still those the tables were built from"},
     {"run_experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_run_experts)), METH_FASTCALL,
-     "(experts, x, weights, indices, n_routed, assume_no_inplace)"},
+     "(experts, x, weights, indices, n_routed, assume_no_inplace, shared)"},
     {"combine", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_combine)), METH_FASTCALL, "(routed, z)"},
     {"set_stats", py_set_stats, METH_O, "dict whose counters linear() keeps"},
     {"forget", py_forget, METH_NOARGS, "drop the remembered quantisations"},

@@ -296,26 +296,62 @@ int check_groups(int n, const void* a, int64_t K) {
     return DSV3_OK;
 }
 
-int grouped_plain(const void* table, int n, const void* a, const float* a_s, int64_t as_row, int64_t as_chunk, const int32_t* seg,
-                  int64_t rows_total, int64_t rows_hint, int64_t N, int64_t K, void* c, void* workspace, size_t workspace_bytes,
+StreamSide side_of(const void* a, const float* a_s, bool transposed, int64_t rows, int64_t N, int64_t K) {
+    StreamSide d = {};
+    d.a = a;
+    d.a_s = a_s;
+    d.as_row = transposed ? 1 : (K + 127) / 128;
+    d.as_chunk = transposed ? rows : 1;
+    d.rows = rows;
+    d.N = N;
+    d.K = K;
+    return d;
+}
+
+// The ordinary weight of dsv3_swiglu_gemm_rows / dsv3_fp8_gemm_rows.
+int add_ordinary(StreamGemm& q, const dsv3_side_gemm_t* s) {
+    if (!s || s->rows == 0 || s->N == 0) return DSV3_OK;
+    if (s->rows < 0 || s->N < 0 || s->K < 16 || s->K % 16 != 0 || s->rows >= (1ll << 31) || !s->a || !s->a_s || !s->w || !s->w_s || !s->out ||
+        (q.swiglu && (!s->w3 || !s->w3_s || !s->out_s_t || s->N % 128 != 0))) {
+        set_last_error("side gemm: null pointer, or sizes outside K %% 16 == 0 (and N %% 128 == 0 with SwiGLU)");
+        return DSV3_ERR_INVALID_ARGUMENT;
+    }
+    if (reinterpret_cast<uintptr_t>(s->a) % 16 || reinterpret_cast<uintptr_t>(s->w) % 16 || reinterpret_cast<uintptr_t>(s->w3) % 16 ||
+        reinterpret_cast<uintptr_t>(s->out) % 16) {
+        set_last_error("side gemm: a, w, w3 and out must be 16-byte aligned");
+        return DSV3_ERR_UNSUPPORTED;
+    }
+    q.ordinary = side_of(s->a, s->a_s, s->a_s_transposed != 0, s->rows, s->N, s->K);
+    q.w0 = s->w;
+    q.w0_s = s->w_s;
+    q.w1 = s->w3;
+    q.w1_s = s->w3_s;
+    if (q.swiglu) {
+        q.ordinary.hq = s->out;
+        q.ordinary.hs = s->out_s_t;
+        q.ordinary.hs_row = 1;
+        q.ordinary.hs_blk = s->rows;
+    } else {
+        q.ordinary.c = s->out;
+    }
+    return DSV3_OK;
+}
+
+int grouped_plain(const void* table, int n, const void* a, const float* a_s, bool transposed, const int32_t* seg, int64_t rows_total,
+                  int64_t rows_hint, int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace, size_t workspace_bytes,
                   dsv3_stream_t stream) {
-    const int rc = check_groups(n, a, K);
+    int rc = check_groups(n, a, K);
     if (rc != DSV3_OK) return rc;
     StreamGemm q = {};
-    q.a = a;
-    q.a_s = a_s;
-    q.as_row = as_row;
-    q.as_chunk = as_chunk;
-    q.rows = rows_total;
+    q.groups = side_of(a, a_s, transposed, rows_total, N, K);
+    q.groups.c = c;
     q.rows_expected = rows_hint > 0 && rows_hint < rows_total ? rows_hint : rows_total;
-    q.N = N;
-    q.K = K;
     q.n_groups = n;
     q.table0 = table;
     q.seg = seg;
-    q.c = c;
     q.workspace = workspace;
     q.workspace_bytes = workspace_bytes;
+    if ((rc = add_ordinary(q, side)) != DSV3_OK) return rc;
     return launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
 }
 
@@ -349,12 +385,12 @@ int dsv3_fp8_gemm_grouped(const void* table, int n_groups, const void* a, const 
         set_last_error("fp8_gemm_grouped: null pointer");
         return DSV3_ERR_INVALID_ARGUMENT;
     }
-    return grouped_plain(table, n_groups, a, a_s, (K + 127) / 128, 1, seg, rows_total, rows_hint, N, K, c, nullptr, 0, stream);
+    return grouped_plain(table, n_groups, a, a_s, false, seg, rows_total, rows_hint, N, K, c, nullptr, nullptr, 0, stream);
 }
 
 int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total,
-                       int64_t rows_hint, int64_t N, int64_t K, void* c, void* workspace, size_t workspace_bytes,
-                       dsv3_stream_t stream) {
+                       int64_t rows_hint, int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace,
+                       size_t workspace_bytes, dsv3_stream_t stream) {
     if (rows_total < 0 || rows_hint < 0 || N < 0 || K <= 0) {
         set_last_error("fp8_gemm_rows: negative size");
         return DSV3_ERR_INVALID_ARGUMENT;
@@ -364,12 +400,12 @@ int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const flo
         set_last_error("fp8_gemm_rows: null pointer");
         return DSV3_ERR_INVALID_ARGUMENT;
     }
-    return grouped_plain(table, n_groups, a, a_s_t, 1, rows_total, seg, rows_total, rows_hint, N, K, c, workspace, workspace_bytes, stream);
+    return grouped_plain(table, n_groups, a, a_s_t, true, seg, rows_total, rows_hint, N, K, c, side, workspace, workspace_bytes, stream);
 }
 
 int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, const void* a, const float* a_s_t, const int32_t* seg,
                           int64_t rows_total, int64_t rows_hint, int64_t N, int64_t K, int scale_fmt, void* hq, float* hs_t,
-                          void* workspace, size_t workspace_bytes, dsv3_stream_t stream) {
+                          const dsv3_side_gemm_t* side, void* workspace, size_t workspace_bytes, dsv3_stream_t stream) {
     if (rows_total < 0 || rows_hint < 0 || N < 0 || K <= 0) {
         set_last_error("swiglu_gemm_rows: negative size");
         return DSV3_ERR_INVALID_ARGUMENT;
@@ -390,26 +426,21 @@ int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, 
     int rc = check_groups(n_groups, a, K);
     if (rc != DSV3_OK) return rc;
     StreamGemm q = {};
-    q.a = a;
-    q.a_s = a_s_t;
-    q.as_row = 1;
-    q.as_chunk = rows_total;
-    q.rows = rows_total;
+    q.groups = side_of(a, a_s_t, true, rows_total, N, K);
+    q.groups.hq = hq;
+    q.groups.hs = hs_t;
+    q.groups.hs_row = 1;
+    q.groups.hs_blk = rows_total;
     q.rows_expected = rows_hint > 0 && rows_hint < rows_total ? rows_hint : rows_total;
-    q.N = N;
-    q.K = K;
     q.n_groups = n_groups;
     q.table0 = table1;
     q.table1 = table3;
     q.seg = seg;
     q.swiglu = true;
-    q.hq = hq;
-    q.hs = hs_t;
-    q.hs_row = 1;
-    q.hs_blk = rows_total;
     q.scale_fmt = scale_fmt;
     q.workspace = workspace;
     q.workspace_bytes = workspace_bytes;
+    if ((rc = add_ordinary(q, side)) != DSV3_OK) return rc;
     return launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
 }
 

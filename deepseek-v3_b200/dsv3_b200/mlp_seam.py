@@ -44,6 +44,27 @@ def mlp_forward(self, x: torch.Tensor, *, model_module, original) -> torch.Tenso
     return y
 
 
+def _scale_fmt_of(lin):
+    """The scale_fmt a Linear hands to linear(): only the plain one does (model.py:205; not :233, :262)."""
+    return getattr(lin, "scale_fmt", None) if type(lin).__name__ == "Linear" else None
+
+
+def plain_weights(mlp, x: torch.Tensor, scale_fmt):
+    """``(w1, w3, w2)`` weights of an MLP that ``mlp_forward`` serves and whose Linears do nothing but the GEMM in
+    ``scale_fmt`` (no bias, no hooks, the installed ``linear``), so that a caller may run them itself; otherwise None."""
+    model = getattr(getattr(type(mlp), "forward", None), "_dsv3_model", None)
+    if model is None or getattr(model, "world_size", 1) != 1 or not getattr(getattr(model, "linear", None), "_dsv3_linear", False):
+        return None
+    w1, w2, w3 = mlp.w1, mlp.w2, mlp.w3
+    for lin, names in ((w1, ("Linear", "ColumnParallelLinear")), (w3, ("Linear", "ColumnParallelLinear")), (w2, ("Linear", "RowParallelLinear"))):
+        if (type(lin).__name__ not in names or getattr(lin, "bias", None) is not None or _scale_fmt_of(lin) != scale_fmt
+                or getattr(lin, "_forward_hooks", None) or getattr(lin, "_forward_pre_hooks", None)):
+            return None
+    if getattr(mlp, "_forward_hooks", None) or getattr(mlp, "_forward_pre_hooks", None) or not _fusable(mlp, x, model):
+        return None
+    return w1.weight, w3.weight, w2.weight
+
+
 def install_mlp(model_module) -> None:
     """Replace ``model_module.MLP.forward`` and ``model_module.Expert.forward``; ``gemm_impl``, ``block_size``,
     ``world_size`` and ``dist`` of the module are read at call time."""
@@ -55,4 +76,5 @@ def install_mlp(model_module) -> None:
             return mlp_forward(self, x, model_module=model_module, original=_original)
 
         forward.__doc__ = mlp_forward.__doc__
+        forward._dsv3_model = model_module
         cls.forward = forward

@@ -222,19 +222,34 @@ int dsv3_moe_combine_add(const void* o, const int32_t* pos, const void* w, const
  * xq_rows e4m3 [T*topk, dim]; scales with the suffix _t are TRANSPOSED, fp32 [K/128, rows_total] (xs_rows_t, a_s_t,
  * hs_t); hq e4m3 [rows_total, N].  Rows at and beyond seg[n] are not written.  The results equal those of the separate
  * operators: FP8 bytes and scales bit for bit given equal GEMM results.
+ * side: an ordinary (ungrouped) weight to work on in the same launch, for few rows (the shared experts, model.py:656, 690),
+ * or null; w3, w3_s and out_s_t only in dsv3_swiglu_gemm_rows, where out is e4m3 [rows, N] with scales out_s_t
+ * [N/128, rows]; in dsv3_fp8_gemm_rows out is bf16 [rows, N].
  * workspace: dsv3_gemm_rows_workspace_bytes() bytes under the rules of dsv3_fp8_gemm's workspace (zeroed header, 256-byte
  * aligned, not shared by overlapping calls); null: K is never split, which is slower for few rows.
  */
 int dsv3_moe_dispatch(const void* x, int64_t T, int64_t dim, const int64_t* indices, const void* weights, int weights_bf16, int topk,
                       int start, int n_local, int scale_fmt, int32_t* seg, int32_t* pos_sorted, void* w_sorted, void* xq, float* xs,
                       void* xq_rows, float* xs_rows_t, dsv3_stream_t stream);
+typedef struct dsv3_side_gemm {
+    const void* a;        /* e4m3 [rows, K], K % 16 == 0 */
+    const float* a_s;     /* fp32 [rows, K/128], or [K/128, rows] when a_s_transposed */
+    int a_s_transposed;
+    int64_t rows, N, K;
+    const void* w;        /* e4m3 [N, K] */
+    const float* w_s;
+    const void* w3;
+    const float* w3_s;
+    void* out;
+    float* out_s_t;
+} dsv3_side_gemm_t;
 size_t dsv3_gemm_rows_workspace_bytes(int n_groups, int64_t rows_total, int64_t rows_hint);
 int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, const void* a, const float* a_s_t, const int32_t* seg,
                           int64_t rows_total, int64_t rows_hint, int64_t N, int64_t K, int scale_fmt, void* hq, float* hs_t,
-                          void* workspace, size_t workspace_bytes, dsv3_stream_t stream);
+                          const dsv3_side_gemm_t* side, void* workspace, size_t workspace_bytes, dsv3_stream_t stream);
 int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total,
-                       int64_t rows_hint, int64_t N, int64_t K, void* c, void* workspace, size_t workspace_bytes,
-                       dsv3_stream_t stream);
+                       int64_t rows_hint, int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace,
+                       size_t workspace_bytes, dsv3_stream_t stream);
 
 /*
  * One-shot all-reduce of a decode-sized bf16 tensor over peer-mapped buffers -- replaces `dist.all_reduce(y)` after
