@@ -432,12 +432,6 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
             auto unit_g = [&](int mu) -> uint32_t { return g + mu; };                        // pipeline counter
             auto unit_k = [&](int mu) -> int { return it.c0 + UC * mu; };                    // first K chunk of the unit
             auto unit_n = [&](int mu) -> int { return min(UC, it.c1 - unit_k(mu)); };        // chunks in the unit
-            // scale of K chunk c for this thread's row (token-major tiles); clamped so that the
-            // look-ahead never leaves the item
-            auto row_scale = [&](int c) -> float {
-                const int cc = min(c, it.c1 - 1);
-                return __ldg(as_ptr + cc) * __ldg(bs_ptr + cc);
-            };
             // acc[off ..] += v * (a_s * b_s) for K chunk ch; v holds HC columns starting at column 2*off
             auto fold = [&](int ch, const uint32_t* v, float sc, auto off_c) {
                 constexpr int off = decltype(off_c)::value;
@@ -480,7 +474,16 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                 // the FMAs; the other promotion warp of the scheduler overlaps with them.  Row scales (global
                 // memory) are fetched one unit ahead.
                 static_assert(CPT == 64, "token-major tiles: 64 columns per thread");
-                float sa0 = row_scale(unit_k(0)), sa1 = row_scale(unit_k(0) + 1);     // this unit's two chunks
+                // raw scales one unit ahead, multiplied when the unit begins (see fp8_gemm_tm.cu)
+                float ra0, ra1, rb0, rb1;
+                auto load_scales = [&](int k) {        // clamped so that the look-ahead never leaves the item
+                    const int c0 = min(k, it.c1 - 1), c1 = min(k + 1, it.c1 - 1);
+                    ra0 = __ldg(as_ptr + c0);
+                    ra1 = __ldg(as_ptr + c1);
+                    rb0 = __ldg(bs_ptr + c0);
+                    rb1 = __ldg(bs_ptr + c1);
+                };
+                load_scales(unit_k(0));
                 for (int mu = 0; ok && mu < n_mine; ++mu) {
                     const uint32_t gu = unit_g(mu);
                     const int ts = gu % NT;
@@ -494,11 +497,8 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                     const uint32_t taddr = t_lane + (ts * UC) * BN;
                     if (mu > 0) tc_ld_x64(taddr, va64);
                     if (nch > 1) tc_ld_x64(taddr + BN, vb64);
-                    float sb0 = 0.0f, sb1 = 0.0f;
-                    if (mu + 1 < n_mine) {
-                        sb0 = row_scale(unit_k(mu + 1));
-                        sb1 = row_scale(unit_k(mu + 1) + 1);
-                    }
+                    const float sa0 = ra0 * rb0, sa1 = ra1 * rb1;
+                    load_scales(unit_k(mu + 1));
                     tc_wait_ld();
                     tc_fence_before();
                     __syncwarp();
@@ -520,8 +520,6 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                             acc[j] = __ffma2_rn(make_float2(__uint_as_float(vb64[2 * j]), __uint_as_float(vb64[2 * j + 1])),
                                                 sc2, acc[j]);
                     }
-                    sa0 = sb0;
-                    sa1 = sb1;
                 }
             } else {
                 // ---- weight-major tiles: a unit is one chunk (16- and 32-token tiles) or two (64-token tiles);

@@ -110,6 +110,7 @@ __device__ __forceinline__ Tile decode_tile(int tile, const TwParams& p) {
     return t;
 }
 
+template <int kBlock>      // K chunks per scale load: 4 (K chunks a multiple of four, 16-byte aligned scales) or 1
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                    const __grid_constant__ CUtensorMap tmap_c, const TwParams p) {
@@ -269,10 +270,6 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 acc[pc * (kPiece / 2) + j] = __ffma2_rn(make_float2(__uint_as_float(vv[2 * j]), __uint_as_float(vv[2 * j + 1])), sc2,
                                                         acc[pc * (kPiece / 2) + j]);
         };
-        auto load_piece = [&](uint32_t taddr, uint32_t* vv) {
-            if constexpr (kPiece == 32) tc_ld_x32(taddr, vv);
-            else tc_ld_x16(taddr, vv);
-        };
         auto release = [&](int slot) {
             tc_fence_before();
             __syncwarp();
@@ -335,40 +332,60 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         };
         auto bs_row = [&](const Tile& t) { return p.b_s + static_cast<int64_t>(min(2 * t.q + half, p.nblk - 1)) * kc; };
 
+        // Scales, kBlock chunks at a time.  A thread's a_s row is a 32-byte sector of its own, and L1 (what the operand
+        // stages leave of it) does not hold 256 of them until the next chunk: one chunk at a time, the scales cost a quarter
+        // as much L2 traffic as the operands and a wait in every chunk (M 4096, N 7168, K 16384: 465 us, with no scale loads
+        // at all 419, as here 430).  One 16-byte load brings four chunks; it is issued as soon as the fourth
+        // product is formed and has that chunk's time to arrive.  Rows that 16-byte loads cannot read (K chunks not a
+        // multiple of four) take the scalar form, kBlock = 1.
+        float ra[kBlock], rb[kBlock];
+        auto next_scales = [&](const float* as, const float* bs, int k) {
+            if (k >= kc) return;
+            if constexpr (kBlock == 4) {
+                const float4 a4 = __ldg(reinterpret_cast<const float4*>(as + k)), b4 = __ldg(reinterpret_cast<const float4*>(bs + k));
+                ra[0] = a4.x; ra[1] = a4.y; ra[2] = a4.z; ra[3] = a4.w;
+                rb[0] = b4.x; rb[1] = b4.y; rb[2] = b4.z; rb[3] = b4.w;
+            } else {
+                ra[0] = __ldg(as + k);
+                rb[0] = __ldg(bs + k);
+            }
+        };
+        auto first_scales = [&](const Tile& t) { next_scales(as_row(t), bs_row(t), 0); };
         bool ok = true;
         uint32_t g = 0;            // chunk counter
         int tile = pair;
         if (tile < p.num_tiles) {
             Tile cur = decode_tile(tile, p);
-            float first = __ldg(as_row(cur)) * __ldg(bs_row(cur));     // product of the scales of the tile's first chunk
+            first_scales(cur);
             while (true) {
                 const float* as_ptr = as_row(cur);
                 const float* bs_ptr = bs_row(cur);
-                float sc = first;
 #pragma unroll
                 for (int j = 0; j < 64; ++j) acc[j] = make_float2(0.0f, 0.0f);
-                for (int k = 0; k < kc; ++k, ++g) {
-                    const int slot = static_cast<int>(g & 1u);
-                    const bool mine = bounded_wait_lean(tfull_bar(slot), (g >> 1) & 1u, ctl, p.status, 4, g);
-                    ok = __all_sync(0xffffffffu, mine);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t t_slot = t_lane + slot * kBN;
-                    // The left 64 columns are read back and folded, then the right 64 are read back and the slot
-                    // returns to the issuer: two read-back latencies per chunk; the last fold follows the release.
-                    tc_ld_x64(t_slot, &v[0][0]);
-                    // product of the scales of the tile's next chunk, one chunk ahead (clamped: the last re-reads its own)
-                    const int kn = min(k + 1, kc - 1);
-                    const float sc_next = __ldg(as_ptr + kn) * __ldg(bs_ptr + kn);
-                    tc_wait_ld();
-                    fold(v[0], sc, 0);
-                    fold(v[1], sc, 1);
-                    tc_ld_x64(t_slot + 2 * kPiece, &v[0][0]);
-                    tc_wait_ld();
-                    release(slot);
-                    fold(v[0], sc, 2);
-                    fold(v[1], sc, 3);
-                    sc = sc_next;
+                for (int k0 = 0; ok && k0 < kc; k0 += kBlock) {
+#pragma unroll
+                    for (int i = 0; i < kBlock; ++i) {
+                        const int slot = static_cast<int>(g & 1u);
+                        const bool mine = bounded_wait_lean(tfull_bar(slot), (g >> 1) & 1u, ctl, p.status, 4, g);
+                        ++g;
+                        ok = __all_sync(0xffffffffu, mine);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t t_slot = t_lane + slot * kBN;
+                        // The left 64 columns are read back and folded, then the right 64 are read back and the slot
+                        // returns to the issuer: two read-back latencies per chunk; the last fold follows the release.
+                        tc_ld_x64(t_slot, &v[0][0]);
+                        const float sc = ra[i] * rb[i];
+                        if (i == kBlock - 1) next_scales(as_ptr, bs_ptr, k0 + kBlock);
+                        tc_wait_ld();
+                        fold(v[0], sc, 0);
+                        fold(v[1], sc, 1);
+                        tc_ld_x64(t_slot + 2 * kPiece, &v[0][0]);
+                        tc_wait_ld();
+                        release(slot);
+                        fold(v[0], sc, 2);
+                        fold(v[1], sc, 3);
+                    }
                 }
                 if (!ok) break;
                 // the next tile's first scales are requested before this tile is written, so that their latency
@@ -378,7 +395,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 Tile nt = cur;
                 if (more) {
                     nt = decode_tile(next, p);
-                    first = __ldg(as_row(nt)) * __ldg(bs_row(nt));
+                    first_scales(nt);
                 }
                 write_tile(2 * cur.pp + static_cast<int>(rank), cur.q);
                 if (!more) break;
@@ -457,7 +474,8 @@ int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const flo
     prm.tma_store = tma_store ? 1 : 0;
     prm.num_tiles = static_cast<int>(tiles_pp * tiles_q);
 
-    auto kern = fp8_gemm_tw_kernel;
+    const bool vec = (prm.kc % 4) == 0 && ((reinterpret_cast<uintptr_t>(a_s) | reinterpret_cast<uintptr_t>(b_s)) % 16) == 0;
+    auto kern = vec ? fp8_gemm_tw_kernel<4> : fp8_gemm_tw_kernel<1>;
     static bool configured[64] = {};
     int dev = 0;
     DSV3_CUDA_TRY(cudaGetDevice(&dev));
@@ -466,7 +484,8 @@ int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const flo
         return DSV3_ERR_UNSUPPORTED;
     }
     if (!configured[dev]) {
-        DSV3_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+        DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+        DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
         configured[dev] = true;
     }
     const int max_pairs = num_sms() / 2;
