@@ -11,10 +11,10 @@
 //     both halves of a SwiGLU pair meet in the same thread's registers.
 //   * Up to 64 tokens per tile: weights are the M operand (128 TMEM lanes), tokens the N operand, and a tile of 16 tokens
 //     costs 16 columns (fp8_stream_kernel).  Up to 128 tokens: tokens are the M operand (fp8_rows_kernel).
-//   * Uneven split: where whole tiles would leave the last round of SMs mostly idle, the (tile, K chunk) space is cut
-//     into equal contiguous ranges, one per CTA.  A CTA then has at most two partial tiles (the head and the tail of
-//     its range); they are parked as fp32 (valid tokens only) and the CTA that takes a tile's last ticket adds them
-//     in K order, so the result does not depend on timing and nothing spins.
+//   * Uneven split: where whole tiles would leave the last round of SMs mostly idle, that round's (tile, K chunk) space
+//     is cut into equal contiguous ranges, one per CTA (struct Plan).  A CTA then has at most two partial tiles (the head
+//     and the tail of its range); they are parked as fp32 (valid tokens only) and the CTA that takes a tile's last ticket
+//     adds them in K order, so the result does not depend on timing and nothing spins.
 //
 // Roles: warp 0 TMA producer, warp 1 MMA issuer (both converged, one elected lane issues), warps 4..11 promotion: every
 // chunk product leaves TMEM and is folded into fp32 registers with its two scales (kernel.py:162).
@@ -44,6 +44,11 @@ constexpr int kRegsPromo = 232;
 static_assert(128 * kRegsControl + 256 * kRegsPromo <= 384 * 168, "register pool");
 constexpr int kMaxGroups = kMaxGroupsOfTable;
 constexpr int kMinUnits = 3;        // a split range is at least this many 32 KB chunks
+// What splitting the last round costs, in chunks of 0.75 us: behind whole tiles, or with nothing to overlap with; and the
+// time a CTA takes per chunk when it has HBM to itself, in sixteenths of that.
+constexpr int kSplitCost = 3, kSplitCostAlone = 3;
+template <int BN>
+constexpr int kAlone = BN <= 32 ? 7 : (BN == 64 ? 9 : 13);
 
 // kRows: tokens on the M side (fp8_rows_kernel); otherwise weights (fp8_stream_kernel).
 template <int BN_, bool kRows>
@@ -72,7 +77,7 @@ struct SCfg {
 };
 
 // A launch works on up to two problems that share the shape of a tile: the groups (per-group weights, rows by group) and
-// one ordinary weight (the shared experts next to the routed ones).
+// one ordinary weight (the shared experts next to the routed ones; kBoth).
 struct Side {
     int kc, nblk, tiles_p;              // K chunks, 128-row blocks of a weight, tiles per token tile
     int rows;                           // rows of a (ordinary weight)
@@ -93,8 +98,8 @@ struct StreamParams {
     const CUtensorMap* g_map[2];
     const float* const* g_scale[2];
     const int* seg;
-    int n_groups;                       // 0: none
-    const float* scale[2];              // ordinary weight (its maps are kernel parameters); side[kOrdinary].rows == 0: none
+    int n_groups;
+    const float* scale[2];              // ordinary weight (its maps are kernel parameters)
     int scale_fmt;
     // split tiles
     float* partials;                    // [CTA][2][2 * BN / 4][128] float4, or null: whole tiles only
@@ -109,15 +114,20 @@ struct Seg {          // a range of K chunks of one tile
     int group, p;     // weight, tile within the weight
 };
 
-// The CTA's share of the work and how tiles are split; every CTA derives the same plan from the same numbers.
-// A unit is one K chunk of a tile; the groups' tiles come first.  32-bit arithmetic throughout (the host checks that the
-// units fit): a 64-bit division takes about half a microsecond here, and ranges computed as units * cta / ctas cost a
-// small problem 15 us.
+// The CTA's share of the work; every CTA derives the same plan from the same numbers.  The tiles (the groups' first, then
+// the ordinary weight's) are worked on whole, one after the other per CTA, except where that would leave the machine
+// idle: then the (tile, K chunk) space of the last, partly filled round is cut into equal contiguous ranges, one per CTA.
+// A CTA begins with its range, so that parking partial tiles and adding them up overlaps with the loads of its whole
+// tiles.  With a single full round in front, that round is cut too: a tile then has two or three parts instead of ten,
+// which one CTA adds up while the others wait for it.
+// A unit is one K chunk of a split tile.  32-bit arithmetic throughout (the host checks that the units fit): a 64-bit
+// division takes about half a microsecond here, and ranges computed as units * cta / ctas cost a small problem 15 us.
 struct Plan {
-    int tiles0, tiles1, kc0, kc1;      // groups, ordinary weight
-    int G;                   // CTAs that take part
-    bool split;
-    int units, base, extra;  // split: the first `extra` CTAs take base + 1 units, the others base
+    int kc0, kc1;            // K chunks: groups, ordinary weight
+    int whole;               // whole tiles
+    int tiles0;              // the groups' tiles
+    int G;                   // CTAs that take a range
+    int units, base, extra;  // the first `extra` CTAs take base + 1 units, the others base
     __device__ __forceinline__ int begin(int cta) const { return cta * base + min(cta, extra); }
     __device__ __forceinline__ int owner(int u) const {
         const int head = extra * (base + 1);
@@ -127,85 +137,85 @@ struct Plan {
 };
 
 // group_tiles: token tiles over all groups
-template <int BN>
+template <int BN, bool kBoth>
 __device__ __forceinline__ Plan make_plan(const StreamParams& p, int group_tiles) {
     Plan pl;
     pl.tiles0 = p.side[kGroups].tiles_p * group_tiles;
-    pl.tiles1 = p.side[kOrdinary].tiles_p * ((p.side[kOrdinary].rows + BN - 1) / BN);
+    const int tiles1 = kBoth ? p.side[kOrdinary].tiles_p * ((p.side[kOrdinary].rows + BN - 1) / BN) : 0;
     pl.kc0 = p.side[kGroups].kc;
     pl.kc1 = p.side[kOrdinary].kc;
-    const int n_tiles = pl.tiles0 + pl.tiles1, ctas = static_cast<int>(gridDim.x);
-    const int longest = max(pl.tiles0 > 0 ? pl.kc0 : 0, pl.tiles1 > 0 ? pl.kc1 : 0);
-    pl.G = ctas;
-    pl.units = pl.tiles0 * pl.kc0 + pl.tiles1 * pl.kc1;
-    pl.base = pl.extra = 0;
-    // whole tiles keep at least 15 of 16 CTA-rounds busy: splitting would only add the parked partial tiles
-    const int left = n_tiles % ctas;
-    const int64_t rounds = static_cast<int64_t>(n_tiles - left + (left ? ctas : 0)) * longest;
-    pl.split = p.partials != nullptr && n_tiles > 0 && static_cast<int64_t>(pl.units) * 16 < rounds * 15;
-    if (pl.split) {
-        const int g = pl.units / kMinUnits;
-        if (g < pl.G) {
-            pl.G = g > n_tiles ? g : min(n_tiles, ctas);
-            pl.split = g > n_tiles;
+    const int ctas = static_cast<int>(gridDim.x);
+    const int rounds = static_cast<int>(static_cast<unsigned>(pl.tiles0) / static_cast<unsigned>(ctas));
+    const int rest0 = pl.tiles0 - rounds * ctas;
+    pl.whole = pl.tiles0 + tiles1;
+    pl.units = pl.G = pl.base = pl.extra = 0;
+    // Time of the last round, in sixteenths of the 0.75 us a chunk takes with every SM loading: whole tiles are bound by
+    // what one CTA folds (kAlone) or by HBM, an even cut by HBM, plus parking and adding up.
+    const int longest = max(rest0 > 0 ? pl.kc0 : 0, tiles1 > 0 ? pl.kc1 : 0);
+    const int first = rounds > 1 ? rounds * ctas : 0, split = pl.tiles0 - first;
+    const int rest = static_cast<int>(16u * static_cast<unsigned>(rest0 * pl.kc0 + tiles1 * pl.kc1) / static_cast<unsigned>(ctas));
+    if (p.partials != nullptr && longest * kAlone<BN> > rest + 16 * (rounds > 1 ? kSplitCost : kSplitCostAlone)) {
+        const int units = split * pl.kc0 + tiles1 * pl.kc1, G = min(ctas, max(1, units / kMinUnits));
+        if (G > split + tiles1 || G == ctas) {
+            pl.whole = first;
+            pl.G = G;
+            pl.units = units;
+            pl.base = static_cast<int>(static_cast<unsigned>(units) / static_cast<unsigned>(G));
+            pl.extra = units - pl.base * G;
         }
-        pl.base = static_cast<int>(static_cast<unsigned>(pl.units) / static_cast<unsigned>(pl.G));
-        pl.extra = pl.units - pl.base * pl.G;
     }
     return pl;
 }
 
 // Iterates over the segments of a CTA.
-template <int BN>
+template <int BN, bool kBoth>
 struct Walker {
     const StreamParams& p;
     const Plan& pl;
     const int* prefix;       // shared memory: token tiles of the groups before each group
-    int u, u1;               // split: next unit and end of the range; whole tiles: next tile
+    int u, u1;               // next unit and end of the CTA's range
+    int tile;                // next whole tile
     __device__ __forceinline__ Walker(const StreamParams& p_, const Plan& pl_, const int* prefix_) : p(p_), pl(pl_), prefix(prefix_) {
         const int cta = static_cast<int>(blockIdx.x);
-        if (pl.split) {
-            u = cta < pl.G ? pl.begin(cta) : 0;
-            u1 = cta < pl.G ? pl.begin(cta + 1) : 0;
-        } else {
-            u = cta;
-            u1 = pl.tiles0 + pl.tiles1;
-        }
+        u = cta < pl.G ? pl.begin(cta) : 0;
+        u1 = cta < pl.G ? pl.begin(cta + 1) : 0;
+        tile = cta;
     }
     __device__ __forceinline__ bool next(Seg& s) {
-        if (u >= u1) return false;
-        int tile;                // within the side
-        if (pl.split) {
-            const int units0 = pl.tiles0 * pl.kc0;
-            s.side = u < units0 ? kGroups : kOrdinary;
-            s.kc = s.side == kGroups ? pl.kc0 : pl.kc1;
-            const int v = s.side == kGroups ? u : u - units0;
-            tile = static_cast<int>(static_cast<unsigned>(v) / static_cast<unsigned>(s.kc));
-            s.ut = u - v + tile * s.kc;
+        int at;                  // tile within the side
+        if (u < u1) {
+            const int units0 = (pl.tiles0 - pl.whole) * pl.kc0;
+            s.side = !kBoth || u < units0 ? kGroups : kOrdinary;
+            s.kc = (!kBoth || s.side == kGroups) ? pl.kc0 : pl.kc1;
+            const int v = (!kBoth || s.side == kGroups) ? u : u - units0;
+            at = static_cast<int>(static_cast<unsigned>(v) / static_cast<unsigned>(s.kc));
+            s.ut = u - v + at * s.kc;
             s.c0 = u - s.ut;
             s.c1 = min(s.kc, s.c0 + (u1 - u));
             u += s.c1 - s.c0;
+            if (!kBoth || s.side == kGroups) at += pl.whole;
         } else {
-            s.side = u < pl.tiles0 ? kGroups : kOrdinary;
-            s.kc = s.side == kGroups ? pl.kc0 : pl.kc1;
-            tile = s.side == kGroups ? u : u - pl.tiles0;
+            if (tile >= pl.whole) return false;
+            s.side = !kBoth || tile < pl.tiles0 ? kGroups : kOrdinary;
+            s.kc = (!kBoth || s.side == kGroups) ? pl.kc0 : pl.kc1;
+            at = (!kBoth || s.side == kGroups) ? tile : tile - pl.tiles0;
             s.ut = 0;
             s.c0 = 0;
             s.c1 = s.kc;
-            u += pl.G;
+            tile += static_cast<int>(gridDim.x);
         }
         // inside a weight the token tile runs fastest, so CTAs that work side by side share the weight blocks
         int nq, first, rows;
-        if (s.side == kGroups) {
+        if (!kBoth || s.side == kGroups) {
             const int per = p.side[kGroups].tiles_p;
             int lo = 0, hi = p.n_groups;
             while (hi - lo > 1) {
                 const int mid = (lo + hi) >> 1;
-                if (prefix[mid] * per <= tile) lo = mid; else hi = mid;
+                if (prefix[mid] * per <= at) lo = mid; else hi = mid;
             }
             s.group = lo;
             nq = prefix[lo + 1] - prefix[lo];
-            tile -= prefix[lo] * per;
+            at -= prefix[lo] * per;
             first = __ldg(p.seg + lo);
             rows = __ldg(p.seg + lo + 1) - first;
         } else {
@@ -214,8 +224,8 @@ struct Walker {
             nq = (rows + BN - 1) / BN;
             first = 0;
         }
-        s.p = nq == 1 ? tile : tile / nq;
-        const int q = tile - s.p * nq;
+        s.p = nq == 1 ? at : at / nq;
+        const int q = at - s.p * nq;
         s.row0 = first + q * BN;
         s.ntok = min(BN, rows - q * BN);
         return true;
@@ -251,40 +261,23 @@ __device__ __forceinline__ void prefix_groups(const StreamParams& p, int* prefix
     }
 }
 
-// While the kernel before this one drains (programmatic dependent launch), the first weight boxes of an ordinary problem
-// come into L2 (the point of coherence: were the predecessor still writing them, the loads after the wait would see
-// its data all the same).  One thread.
-template <int BN, bool kSwiglu>
-__device__ __forceinline__ void prefetch_weights(const StreamParams& p, const void* w0, const void* w1, const int* prefix, int n) {
-    const Plan pl = make_plan<BN>(p, 0);
-    Walker<BN> wk(p, pl, prefix);
-    Seg s;
-    if (wk.next(s)) {
-        const int r0 = (kSwiglu ? s.p : 2 * s.p) * kPRows;
-        for (int k = s.c0; k < min(s.c1, s.c0 + n); ++k) {
-            tma_prefetch_l2_2d(w0, k * kChunk, r0);
-            if (kSwiglu || 2 * s.p + 1 < p.side[kOrdinary].nblk) tma_prefetch_l2_2d(w1, k * kChunk, kSwiglu ? r0 : r0 + kPRows);
-        }
-    }
-}
-
 // The TMA producer (one converged warp).  Stage: [BN token rows][block 0][block 1] of one K chunk; of the tokens only
 // the boxes that hold any of the tile's rows are fetched.
-template <class C, bool kSwiglu>
+template <class C, bool kSwiglu, bool kBoth>
 __device__ __forceinline__ void produce(const StreamParams& p, const Plan& pl, const int* prefix, const void* w0, const void* w1,
                                         const void* ta0, const void* ta1, uint32_t tiles, uint32_t bar0, Control* ctl) {
     constexpr int NS = C::kStages, BN = C::BN;
-    Walker<BN> wk(p, pl, prefix);
+    Walker<BN, kBoth> wk(p, pl, prefix);
     Seg s;
     uint32_t g = 0;
     bool ok = true;
     while (ok && wk.next(s)) {
-        const void* m0 = s.side == kGroups ? static_cast<const void*>(p.g_map[0] + s.group) : w0;
-        const void* m1 = s.side == kGroups ? static_cast<const void*>(p.g_map[1] + s.group) : w1;
-        const void* ta = s.side == kGroups ? ta0 : ta1;
+        const void* m0 = (!kBoth || s.side == kGroups) ? static_cast<const void*>(p.g_map[0] + s.group) : w0;
+        const void* m1 = (!kBoth || s.side == kGroups) ? static_cast<const void*>(p.g_map[1] + s.group) : w1;
+        const void* ta = (!kBoth || s.side == kGroups) ? ta0 : ta1;
         const int r0 = (kSwiglu ? s.p : 2 * s.p) * kPRows;
         const int r1 = kSwiglu ? r0 : r0 + kPRows;
-        const bool two = kSwiglu || 2 * s.p + 1 < p.side[s.side].nblk;
+        const bool two = kSwiglu || 2 * s.p + 1 < p.side[kBoth ? s.side : kGroups].nblk;
         const int boxes = (s.ntok + C::kBox - 1) / C::kBox;
         const uint32_t bytes = (two ? 2u : 1u) * kPRows * kChunk + static_cast<uint32_t>(boxes) * C::kBox * kChunk;
         for (int k = s.c0; k < s.c1; ++k, ++g) {
@@ -346,7 +339,7 @@ __device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_b
 // side the same expert layer, 57 tokens per tile, drew the board's whole power at 1380 MHz: half of the multiplications
 // were for nobody.)  Promotion group g owns every second piece of 16 tokens, of both blocks.
 // ---------------------------------------------------------------------------------------------------------------------
-template <int BN, bool kSwiglu>
+template <int BN, bool kSwiglu, bool kBoth>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
                   const __grid_constant__ CUtensorMap tmap_a0, const __grid_constant__ CUtensorMap tmap_a1,
@@ -392,36 +385,35 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         }
         ctl->abort_flag = 0;
         mbar_fence_init();
-        if (p.n_groups > 0) tma_prefetch_desc(&tmap_a0);
-        if (p.side[kOrdinary].rows > 0) {
+        tma_prefetch_desc(&tmap_a0);
+        if constexpr (kBoth) {
             tma_prefetch_desc(&tmap_a1);
             tma_prefetch_desc(&tmap_w0);
             tma_prefetch_desc(&tmap_w1);
         }
     }
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
-    if (threadIdx.x == 0 && p.n_groups == 0) prefetch_weights<BN, kSwiglu>(p, &tmap_w0, &tmap_w1, prefix, NS);
     griddep_launch_dependents();
     griddep_wait();
-    if (p.n_groups > 0) prefix_groups<BN>(p, prefix, scan, warp, lane);
+    prefix_groups<BN>(p, prefix, scan, warp, lane);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
-    const Plan pl = make_plan<BN>(p, p.n_groups > 0 ? prefix[kMaxGroups] : 0);
+    const Plan pl = make_plan<BN, kBoth>(p, prefix[kMaxGroups]);
 
     if (warp < kFirstPromoWarp) {
       if constexpr (NP >= 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
       if (warp == 0) {
-        produce<C, kSwiglu>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
+        produce<C, kSwiglu, kBoth>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
       } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        Walker<BN> wk(p, pl, prefix);
+        Walker<BN, kBoth> wk(p, pl, prefix);
         Seg s;
         uint32_t g = 0;
         bool ok = true;
         while (ok && wk.next(s)) {
-            const bool two = kSwiglu || 2 * s.p + 1 < p.side[s.side].nblk;
+            const bool two = kSwiglu || 2 * s.p + 1 < p.side[kBoth ? s.side : kGroups].nblk;
             const uint32_t idesc = umma_idesc_e4m3_f32(kPRows, 16) + ((static_cast<uint32_t>(s.ntok + 15) / 16 - 1) << 18);   // N in units of 8 at bit 17
             for (int k = s.c0; k < s.c1; ++k, ++g) {
                 const int st = g % NS, ts = g % NT;
@@ -450,13 +442,13 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         }
       } else {
         // ------------------------------------------------------------ token scales, TC chunks at a time
-        Walker<BN> wk(p, pl, prefix);
+        Walker<BN, kBoth> wk(p, pl, prefix);
         Seg s;
         uint32_t t = 0;          // ring counter
         bool ok = true;
         const int tid = threadIdx.x - 64;
         while (ok && wk.next(s)) {
-            const Side& d = p.side[s.side];
+            const Side& d = p.side[kBoth ? s.side : kGroups];
             for (int k = s.c0; k < s.c1; k += TC, ++t) {
                 const int sl = t & 1;
                 ok = __all_sync(0xffffffffu, bounded_wait(sempty_bar(sl), ((t >> 1) & 1u) ^ 1u, ctl, p.status, 7, t));
@@ -490,7 +482,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;                    // weight row within a block (TMEM lane)
         const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + col0;
-        Walker<BN> wk(p, pl, prefix);
+        Walker<BN, kBoth> wk(p, pl, prefix);
         Seg s;
         uint32_t g = 0, t = 0;
         bool ok = true;
@@ -520,10 +512,10 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
             }
         };
         while (ok && wk.next(s)) {
-            const bool two = kSwiglu || 2 * s.p + 1 < p.side[s.side].nblk;
-            const Side& d = p.side[s.side];
-            const float* b0 = (s.side == kGroups ? p.g_scale[0][s.group] : p.scale[0]) + static_cast<int64_t>(kSwiglu ? s.p : 2 * s.p) * s.kc;
-            const float* b1 = (s.side == kGroups ? p.g_scale[1][s.group] : p.scale[1]) +
+            const bool two = kSwiglu || 2 * s.p + 1 < p.side[kBoth ? s.side : kGroups].nblk;
+            const Side& d = p.side[kBoth ? s.side : kGroups];
+            const float* b0 = ((!kBoth || s.side == kGroups) ? p.g_scale[0][s.group] : p.scale[0]) + static_cast<int64_t>(kSwiglu ? s.p : 2 * s.p) * s.kc;
+            const float* b1 = ((!kBoth || s.side == kGroups) ? p.g_scale[1][s.group] : p.scale[1]) +
                               static_cast<int64_t>(kSwiglu ? s.p : (two ? 2 * s.p + 1 : 2 * s.p)) * s.kc;
             // pieces of this thread that hold a token of the tile
             const int np = s.ntok <= col0 ? 0 : min(NP, (s.ntok - col0 + 2 * PW - 1) / (2 * PW));
@@ -748,7 +740,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
 // columns of one block: one scale product per chunk and thread, and a row's maximum is two threads' business.  The MMA
 // costs 512 cycles per chunk whatever the number of tokens, which the weights' arrival (1300 cycles at 1.85 GHz) hides.
 // ---------------------------------------------------------------------------------------------------------------------
-template <int BN, bool kSwiglu>
+template <int BN, bool kSwiglu, bool kBoth>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
                 const __grid_constant__ CUtensorMap tmap_a0, const __grid_constant__ CUtensorMap tmap_a1,
@@ -784,36 +776,35 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
         }
         ctl->abort_flag = 0;
         mbar_fence_init();
-        if (p.n_groups > 0) tma_prefetch_desc(&tmap_a0);
-        if (p.side[kOrdinary].rows > 0) {
+        tma_prefetch_desc(&tmap_a0);
+        if constexpr (kBoth) {
             tma_prefetch_desc(&tmap_a1);
             tma_prefetch_desc(&tmap_w0);
             tma_prefetch_desc(&tmap_w1);
         }
     }
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
-    if (threadIdx.x == 0 && p.n_groups == 0) prefetch_weights<BN, kSwiglu>(p, &tmap_w0, &tmap_w1, prefix, NS);
     griddep_launch_dependents();
     griddep_wait();
-    if (p.n_groups > 0) prefix_groups<BN>(p, prefix, scan, warp, lane);
+    prefix_groups<BN>(p, prefix, scan, warp, lane);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
-    const Plan pl = make_plan<BN>(p, p.n_groups > 0 ? prefix[kMaxGroups] : 0);
+    const Plan pl = make_plan<BN, kBoth>(p, prefix[kMaxGroups]);
 
     if (warp < kFirstPromoWarp) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
         if (warp == 0) {
-            produce<C, kSwiglu>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
+            produce<C, kSwiglu, kBoth>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
         } else if (warp == 1) {
             // -------------------------------------------------------- MMA issuer
-            Walker<BN> wk(p, pl, prefix);
+            Walker<BN, kBoth> wk(p, pl, prefix);
             Seg s;
             uint32_t g = 0;
             bool ok = true;
             while (ok && wk.next(s)) {
-                const bool two = kSwiglu || 2 * s.p + 1 < p.side[s.side].nblk;
+                const bool two = kSwiglu || 2 * s.p + 1 < p.side[kBoth ? s.side : kGroups].nblk;
                 const uint32_t idesc = two ? umma_idesc_e4m3_f32(kPRows, 2 * kPRows) : umma_idesc_e4m3_f32(kPRows, kPRows);
                 for (int k = s.c0; k < s.c1; ++k, ++g) {
                     const int st = g % NS, ts = g % NT;
@@ -846,7 +837,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
         const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + grp * kPRows;
         uint8_t* my_x = xbuf + grp * (BN * 128);                // this group's half of the exchange buffer
         uint8_t* other_x = xbuf + (1 - grp) * (BN * 128);
-        Walker<BN> wk(p, pl, prefix);
+        Walker<BN, kBoth> wk(p, pl, prefix);
         Seg s, ahead;
         uint32_t g = 0;
         bool ok = true;
@@ -872,10 +863,10 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
         float ra[4], rb;         // rb: the weight block's scale of the next chunk (32 chunks to a cache line: L1)
         auto scales_of = [&](const Seg& q) {
             const int blk = kSwiglu ? q.p : 2 * q.p + grp;
-            const Side& d = p.side[q.side];
+            const Side& d = p.side[kBoth ? q.side : kGroups];
             as_chunk = d.as_chunk;
             as = d.a_s + (q.row0 + min(row, q.ntok - 1)) * d.as_row + q.c0 * as_chunk;
-            bs = (q.side == kGroups ? p.g_scale[grp][q.group] : p.scale[grp]) + static_cast<int64_t>(min(blk, d.nblk - 1)) * q.kc + q.c0;
+            bs = ((!kBoth || q.side == kGroups) ? p.g_scale[grp][q.group] : p.scale[grp]) + static_cast<int64_t>(min(blk, d.nblk - 1)) * q.kc + q.c0;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int k = min(i, q.c1 - q.c0 - 1);
@@ -887,7 +878,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
         if (more) scales_of(ahead);
         while (ok && more) {
             s = ahead;
-            const Side& d = p.side[s.side];
+            const Side& d = p.side[kBoth ? s.side : kGroups];
             const int blk = kSwiglu ? s.p : 2 * s.p + grp;
             const bool active = quarter * 32 < s.ntok && blk < d.nblk;     // uniform in the warp
             const int n_ch = s.c1 - s.c0;
@@ -1062,13 +1053,13 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
     teardown(ctl, warp, tmem_base, C::kTmemCols);
 }
 
-template <int BN, bool kSwiglu, bool kRows>
+template <int BN, bool kSwiglu, bool kRows, bool kBoth>
 int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, const StreamParams& prm,
                    int64_t tiles_bound, int64_t units_bound, cudaStream_t stream) {
     using C = SCfg<BN, kRows>;
     constexpr auto pick = [] {
-        if constexpr (kRows) return fp8_rows_kernel<BN, kSwiglu>;
-        else return fp8_stream_kernel<BN, kSwiglu>;
+        if constexpr (kRows) return fp8_rows_kernel<BN, kSwiglu, kBoth>;
+        else return fp8_stream_kernel<BN, kSwiglu, kBoth>;
     };
     auto kern = pick();
     static bool configured[64] = {};
@@ -1135,21 +1126,18 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
     memset(&ta1, 0, sizeof(ta1));
     int rc;
     const bool ordinary = q.ordinary.rows > 0;
-    const int64_t per_tile = q.n_groups > 0 ? (q.rows_expected + q.n_groups - 1) / q.n_groups : q.ordinary.rows;
+    const int64_t per_tile = (q.rows_expected + q.n_groups - 1) / q.n_groups;
     const int bn = stream_tile(per_tile);
     int64_t tiles[2] = {0, 0};
-    if (q.n_groups > 0) {
-        if ((rc = fill_side(prm.side[kGroups], &ta0, q.groups, q.swiglu, bn)) != DSV3_OK) return rc;
-        for (int b = 0; b < 2; ++b) {
-            const void* tbl = (b == 1 && q.swiglu) ? q.table1 : q.table0;
-            prm.g_map[b] = static_cast<const CUtensorMap*>(tbl);
-            prm.g_scale[b] = reinterpret_cast<const float* const*>(static_cast<const uint8_t*>(tbl) + static_cast<size_t>(q.n_groups) * sizeof(CUtensorMap));
-        }
-        prm.seg = q.seg;
-        // token tiles: at most one partly filled tile per group on top of the full ones, and never more groups than rows
-        const int64_t rows = q.groups.rows;
-        tiles[0] = (rows / bn + (q.n_groups < rows ? q.n_groups : rows)) * prm.side[kGroups].tiles_p;
+    if ((rc = fill_side(prm.side[kGroups], &ta0, q.groups, q.swiglu, bn)) != DSV3_OK) return rc;
+    for (int b = 0; b < 2; ++b) {
+        const void* tbl = (b == 1 && q.swiglu) ? q.table1 : q.table0;
+        prm.g_map[b] = static_cast<const CUtensorMap*>(tbl);
+        prm.g_scale[b] = reinterpret_cast<const float* const*>(static_cast<const uint8_t*>(tbl) + static_cast<size_t>(q.n_groups) * sizeof(CUtensorMap));
     }
+    prm.seg = q.seg;
+    // token tiles: at most one partly filled tile per group on top of the full ones, and never more groups than rows
+    tiles[0] = (q.groups.rows / bn + (q.n_groups < q.groups.rows ? q.n_groups : q.groups.rows)) * prm.side[kGroups].tiles_p;
     if (ordinary) {
         const StreamSide& d = q.ordinary;
         if ((rc = fill_side(prm.side[kOrdinary], &ta1, d, q.swiglu, bn)) != DSV3_OK) return rc;
@@ -1173,9 +1161,12 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
         set_last_error("fp8 stream GEMM: %lld K chunks are more than the work-item counter holds", static_cast<long long>(units));
         return DSV3_ERR_UNSUPPORTED;
     }
-#define DSV3_STREAM_CASE(BN_, ROWS_)                                                                                            \
-    return q.swiglu ? launch_variant<BN_, true, ROWS_>(w0, w1, ta0, ta1, prm, tiles[0] + tiles[1], units, stream)  \
-                    : launch_variant<BN_, false, ROWS_>(w0, w1, ta0, ta1, prm, tiles[0] + tiles[1], units, stream)
+    const int64_t bound = tiles[0] + tiles[1];
+#define DSV3_STREAM_CASE(BN_, ROWS_)                                                                                                  \
+    return q.swiglu ? (ordinary ? launch_variant<BN_, true, ROWS_, true>(w0, w1, ta0, ta1, prm, bound, units, stream)                 \
+                                : launch_variant<BN_, true, ROWS_, false>(w0, w1, ta0, ta1, prm, bound, units, stream))               \
+                    : (ordinary ? launch_variant<BN_, false, ROWS_, true>(w0, w1, ta0, ta1, prm, bound, units, stream)                \
+                                : launch_variant<BN_, false, ROWS_, false>(w0, w1, ta0, ta1, prm, bound, units, stream))
     switch (bn) {
         case 16: DSV3_STREAM_CASE(16, false);
         case 32: DSV3_STREAM_CASE(32, false);

@@ -63,7 +63,7 @@ struct StreamSide {
 };
 struct StreamGemm {
     StreamSide groups;
-    int n_groups;                      // 0: no groups
+    int n_groups;
     int64_t rows_expected;             // rows the groups are expected to own together
     const void *table0, *table1;       // group tables; table1 only with swiglu
     const int* seg;                    // device memory
