@@ -11,8 +11,8 @@
 //     both halves of a SwiGLU pair meet in the same thread's registers.
 //   * Up to 64 tokens per tile: weights are the M operand (128 TMEM lanes), tokens the N operand, and a tile of 16 tokens
 //     costs 16 columns (fp8_stream_kernel).  Up to 128 tokens: tokens are the M operand (fp8_rows_kernel).
-//   * Uneven split: where whole tiles would leave the last round of SMs mostly idle, that round's (tile, K chunk) space
-//     is cut into equal contiguous ranges, one per CTA (struct Plan).  A CTA then has at most two partial tiles (the head
+//   * Uneven split: where whole tiles would leave the last round of SMs mostly idle, the (tile, K chunk) space is cut into
+//     equal contiguous ranges, one per CTA (struct Plan).  A CTA then has at most two partial tiles (the head
 //     and the tail of its range); they are parked as fp32 (valid tokens only) and the CTA that takes a tile's last ticket
 //     adds them in K order, so the result does not depend on timing and nothing spins.
 //
@@ -42,13 +42,18 @@ constexpr int kTabThreads = 64;
 constexpr int kRegsControl = 40;
 constexpr int kRegsPromo = 232;
 static_assert(128 * kRegsControl + 256 * kRegsPromo <= 384 * 168, "register pool");
+// weights on the M side: fewer accumulators; the control warps' tile bookkeeping does not fit 40 registers (a spilled
+// variable goes through an L1 that the operand stages have squeezed out: 5 % of an expert layer)
+constexpr int kRegsControlM = 88;
+constexpr int kRegsPromoM = 208;
+static_assert(128 * kRegsControlM + 256 * kRegsPromoM <= 384 * 168, "register pool");
 constexpr int kMaxGroups = kMaxGroupsOfTable;
 constexpr int kMinUnits = 3;        // a split range is at least this many 32 KB chunks
-// What splitting the last round costs, in chunks of 0.75 us: behind whole tiles, or with nothing to overlap with; and the
-// time a CTA takes per chunk when it has HBM to itself, in sixteenths of that.
-constexpr int kSplitCost = 3, kSplitCostAlone = 3;
+// What cutting tiles costs, in chunks of 0.75 us, and the time a CTA takes per chunk when it has HBM to itself, in
+// sixteenths of that (B200: 64 tokens of a decode layer's 32 experts, one round, 464 us whole, 410 cut).
+constexpr int kSplitCost = 3;
 template <int BN>
-constexpr int kAlone = BN <= 32 ? 7 : (BN == 64 ? 9 : 13);
+constexpr int kAlone = BN <= 32 ? 7 : 9;
 
 // kRows: tokens on the M side (fp8_rows_kernel); otherwise weights (fp8_stream_kernel).
 template <int BN_, bool kRows>
@@ -115,17 +120,15 @@ struct Seg {          // a range of K chunks of one tile
 };
 
 // The CTA's share of the work; every CTA derives the same plan from the same numbers.  The tiles (the groups' first, then
-// the ordinary weight's) are worked on whole, one after the other per CTA, except where that would leave the machine
-// idle: then the (tile, K chunk) space of the last, partly filled round is cut into equal contiguous ranges, one per CTA.
-// A CTA begins with its range, so that parking partial tiles and adding them up overlaps with the loads of its whole
-// tiles.  With a single full round in front, that round is cut too: a tile then has two or three parts instead of ten,
-// which one CTA adds up while the others wait for it.
-// A unit is one K chunk of a split tile.  32-bit arithmetic throughout (the host checks that the units fit): a 64-bit
-// division takes about half a microsecond here, and ranges computed as units * cta / ctas cost a small problem 15 us.
+// the ordinary weight's) are worked on whole, one after the other per CTA, or (kSplit) where that would leave the machine
+// idle in the last of one or two rounds, the (tile, K chunk) space is cut into equal contiguous ranges, one per CTA.
+// (Cutting only the tiles of the last round was slower: each then has about ten parts, which one CTA adds up while the
+// others wait for it.  So was cutting a problem of more rounds: 14 rounds of 40 chunks took 380 us whole, 476 cut.)
+// A unit is one K chunk of a tile.  32-bit arithmetic throughout (the host checks that the units fit): a 64-bit division
+// takes about half a microsecond here, and ranges computed as units * cta / ctas cost a small problem 15 us.
 struct Plan {
     int kc0, kc1;            // K chunks: groups, ordinary weight
-    int whole;               // whole tiles
-    int tiles0;              // the groups' tiles
+    int tiles0, tiles1;      // groups, ordinary weight
     int G;                   // CTAs that take a range
     int units, base, extra;  // the first `extra` CTAs take base + 1 units, the others base
     __device__ __forceinline__ int begin(int cta) const { return cta * base + min(cta, extra); }
@@ -137,38 +140,36 @@ struct Plan {
 };
 
 // group_tiles: token tiles over all groups
-template <int BN, bool kBoth>
+template <int BN, bool kBoth, bool kSplit>
 __device__ __forceinline__ Plan make_plan(const StreamParams& p, int group_tiles) {
     Plan pl;
     pl.tiles0 = p.side[kGroups].tiles_p * group_tiles;
-    const int tiles1 = kBoth ? p.side[kOrdinary].tiles_p * ((p.side[kOrdinary].rows + BN - 1) / BN) : 0;
+    pl.tiles1 = kBoth ? p.side[kOrdinary].tiles_p * ((p.side[kOrdinary].rows + BN - 1) / BN) : 0;
     pl.kc0 = p.side[kGroups].kc;
     pl.kc1 = p.side[kOrdinary].kc;
+    pl.units = pl.tiles0 * pl.kc0 + pl.tiles1 * pl.kc1;
+    pl.G = pl.base = pl.extra = 0;
     const int ctas = static_cast<int>(gridDim.x);
     const int rounds = static_cast<int>(static_cast<unsigned>(pl.tiles0) / static_cast<unsigned>(ctas));
     const int rest0 = pl.tiles0 - rounds * ctas;
-    pl.whole = pl.tiles0 + tiles1;
-    pl.units = pl.G = pl.base = pl.extra = 0;
+    if constexpr (!kSplit) return pl;
     // Time of the last round, in sixteenths of the 0.75 us a chunk takes with every SM loading: whole tiles are bound by
-    // what one CTA folds (kAlone) or by HBM, an even cut by HBM, plus parking and adding up.
-    const int longest = max(rest0 > 0 ? pl.kc0 : 0, tiles1 > 0 ? pl.kc1 : 0);
-    const int first = rounds > 1 ? rounds * ctas : 0, split = pl.tiles0 - first;
-    const int rest = static_cast<int>(16u * static_cast<unsigned>(rest0 * pl.kc0 + tiles1 * pl.kc1) / static_cast<unsigned>(ctas));
-    if (p.partials != nullptr && longest * kAlone<BN> > rest + 16 * (rounds > 1 ? kSplitCost : kSplitCostAlone)) {
-        const int units = split * pl.kc0 + tiles1 * pl.kc1, G = min(ctas, max(1, units / kMinUnits));
-        if (G > split + tiles1 || G == ctas) {
-            pl.whole = first;
+    // what one CTA folds (kAlone), an even cut by HBM, plus parking and adding up.
+    const int longest = max(rest0 > 0 ? pl.kc0 : 0, pl.tiles1 > 0 ? pl.kc1 : 0);
+    const int rest = static_cast<int>(16u * static_cast<unsigned>(rest0 * pl.kc0 + pl.tiles1 * pl.kc1) / static_cast<unsigned>(ctas));
+    if (rounds < 2 && longest * kAlone<BN> > rest + 16 * kSplitCost) {
+        const int G = min(ctas, max(1, pl.units / kMinUnits));
+        if (G > pl.tiles0 + pl.tiles1 || G == ctas) {
             pl.G = G;
-            pl.units = units;
-            pl.base = static_cast<int>(static_cast<unsigned>(units) / static_cast<unsigned>(G));
-            pl.extra = units - pl.base * G;
+            pl.base = static_cast<int>(static_cast<unsigned>(pl.units) / static_cast<unsigned>(G));
+            pl.extra = pl.units - pl.base * G;
         }
     }
     return pl;
 }
 
 // Iterates over the segments of a CTA.
-template <int BN, bool kBoth>
+template <int BN, bool kBoth, bool kSplit>
 struct Walker {
     const StreamParams& p;
     const Plan& pl;
@@ -177,14 +178,14 @@ struct Walker {
     int tile;                // next whole tile
     __device__ __forceinline__ Walker(const StreamParams& p_, const Plan& pl_, const int* prefix_) : p(p_), pl(pl_), prefix(prefix_) {
         const int cta = static_cast<int>(blockIdx.x);
-        u = cta < pl.G ? pl.begin(cta) : 0;
-        u1 = cta < pl.G ? pl.begin(cta + 1) : 0;
+        u = kSplit && cta < pl.G ? pl.begin(cta) : 0;
+        u1 = kSplit && cta < pl.G ? pl.begin(cta + 1) : 0;
         tile = cta;
     }
     __device__ __forceinline__ bool next(Seg& s) {
         int at;                  // tile within the side
-        if (u < u1) {
-            const int units0 = (pl.tiles0 - pl.whole) * pl.kc0;
+        if (kSplit && u < u1) {
+            const int units0 = pl.tiles0 * pl.kc0;
             s.side = !kBoth || u < units0 ? kGroups : kOrdinary;
             s.kc = (!kBoth || s.side == kGroups) ? pl.kc0 : pl.kc1;
             const int v = (!kBoth || s.side == kGroups) ? u : u - units0;
@@ -193,9 +194,8 @@ struct Walker {
             s.c0 = u - s.ut;
             s.c1 = min(s.kc, s.c0 + (u1 - u));
             u += s.c1 - s.c0;
-            if (!kBoth || s.side == kGroups) at += pl.whole;
         } else {
-            if (tile >= pl.whole) return false;
+            if ((kSplit && pl.G > 0) || tile >= pl.tiles0 + pl.tiles1) return false;
             s.side = !kBoth || tile < pl.tiles0 ? kGroups : kOrdinary;
             s.kc = (!kBoth || s.side == kGroups) ? pl.kc0 : pl.kc1;
             at = (!kBoth || s.side == kGroups) ? tile : tile - pl.tiles0;
@@ -263,11 +263,11 @@ __device__ __forceinline__ void prefix_groups(const StreamParams& p, int* prefix
 
 // The TMA producer (one converged warp).  Stage: [BN token rows][block 0][block 1] of one K chunk; of the tokens only
 // the boxes that hold any of the tile's rows are fetched.
-template <class C, bool kSwiglu, bool kBoth>
+template <class C, bool kSwiglu, bool kBoth, bool kSplit>
 __device__ __forceinline__ void produce(const StreamParams& p, const Plan& pl, const int* prefix, const void* w0, const void* w1,
                                         const void* ta0, const void* ta1, uint32_t tiles, uint32_t bar0, Control* ctl) {
     constexpr int NS = C::kStages, BN = C::BN;
-    Walker<BN, kBoth> wk(p, pl, prefix);
+    Walker<BN, kBoth, kSplit> wk(p, pl, prefix);
     Seg s;
     uint32_t g = 0;
     bool ok = true;
@@ -339,7 +339,7 @@ __device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_b
 // side the same expert layer, 57 tokens per tile, drew the board's whole power at 1380 MHz: half of the multiplications
 // were for nobody.)  Promotion group g owns every second piece of 16 tokens, of both blocks.
 // ---------------------------------------------------------------------------------------------------------------------
-template <int BN, bool kSwiglu, bool kBoth>
+template <int BN, bool kSwiglu, bool kBoth, bool kSplit>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
                   const __grid_constant__ CUtensorMap tmap_a0, const __grid_constant__ CUtensorMap tmap_a1,
@@ -400,15 +400,15 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
-    const Plan pl = make_plan<BN, kBoth>(p, prefix[kMaxGroups]);
+    const Plan pl = make_plan<BN, kBoth, kSplit>(p, prefix[kMaxGroups]);
 
     if (warp < kFirstPromoWarp) {
-      if constexpr (NP >= 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
+      if constexpr (NP >= 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControlM));
       if (warp == 0) {
-        produce<C, kSwiglu, kBoth>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
+        produce<C, kSwiglu, kBoth, kSplit>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
       } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        Walker<BN, kBoth> wk(p, pl, prefix);
+        Walker<BN, kBoth, kSplit> wk(p, pl, prefix);
         Seg s;
         uint32_t g = 0;
         bool ok = true;
@@ -442,7 +442,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         }
       } else {
         // ------------------------------------------------------------ token scales, TC chunks at a time
-        Walker<BN, kBoth> wk(p, pl, prefix);
+        Walker<BN, kBoth, kSplit> wk(p, pl, prefix);
         Seg s;
         uint32_t t = 0;          // ring counter
         bool ok = true;
@@ -475,14 +475,15 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         }
       }
     } else {
-        if constexpr (NP >= 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsPromo));
+        if constexpr (NP >= 2) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsPromoM));
         // ------------------------------------------------------------ promotion + epilogue
         const int grp = (warp - kFirstPromoWarp) >> 2;
         const int col0 = grp * PW;
         const int quarter = warp & 3;
         const int row = quarter * 32 + lane;                    // weight row within a block (TMEM lane)
         const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + col0;
-        Walker<BN, kBoth> wk(p, pl, prefix);
+        auto kc_of = [&](const Seg& q) { return kBoth ? q.kc : p.side[kGroups].kc; };
+        Walker<BN, kBoth, kSplit> wk(p, pl, prefix);
         Seg s;
         uint32_t g = 0, t = 0;
         bool ok = true;
@@ -514,9 +515,9 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         while (ok && wk.next(s)) {
             const bool two = kSwiglu || 2 * s.p + 1 < p.side[kBoth ? s.side : kGroups].nblk;
             const Side& d = p.side[kBoth ? s.side : kGroups];
-            const float* b0 = ((!kBoth || s.side == kGroups) ? p.g_scale[0][s.group] : p.scale[0]) + static_cast<int64_t>(kSwiglu ? s.p : 2 * s.p) * s.kc;
+            const float* b0 = ((!kBoth || s.side == kGroups) ? p.g_scale[0][s.group] : p.scale[0]) + static_cast<int64_t>(kSwiglu ? s.p : 2 * s.p) * kc_of(s);
             const float* b1 = ((!kBoth || s.side == kGroups) ? p.g_scale[1][s.group] : p.scale[1]) +
-                              static_cast<int64_t>(kSwiglu ? s.p : (two ? 2 * s.p + 1 : 2 * s.p)) * s.kc;
+                              static_cast<int64_t>(kSwiglu ? s.p : (two ? 2 * s.p + 1 : 2 * s.p)) * kc_of(s);
             // pieces of this thread that hold a token of the tile
             const int np = s.ntok <= col0 ? 0 : min(NP, (s.ntok - col0 + 2 * PW - 1) / (2 * PW));
 #pragma unroll
@@ -578,11 +579,11 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
             }
             if (!ok) break;
 
-            if (n_ch < s.kc) {
+            if (kSplit && n_ch < kc_of(s)) {
                 // part of a tile: park the pieces that hold tokens, take a ticket; the last part of the tile adds all
                 // parts in K order and goes on to write the result
                 const int cta = static_cast<int>(blockIdx.x);
-                const int first = pl.owner(s.ut), last = pl.owner(s.ut + s.kc - 1);
+                const int first = pl.owner(s.ut), last = pl.owner(s.ut + kc_of(s) - 1);
                 constexpr int kTileVec = 2 * BN / 4 * kPRows;             // float4 per parked tile: [2 blocks][BN / 4][128 rows]
                 float4* base = reinterpret_cast<float4*>(p.partials) + (col0 / 4) * kPRows + row;
                 auto part = [&](int c) { return base + (static_cast<int64_t>(c) * 2 + (pl.begin(c) >= s.ut ? 0 : 1)) * kTileVec; };
@@ -746,6 +747,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
                 const __grid_constant__ CUtensorMap tmap_a0, const __grid_constant__ CUtensorMap tmap_a1,
                   const __grid_constant__ StreamParams p) {
     using C = SCfg<BN, true>;
+    constexpr bool kSplit = false;      // its partial tiles would be 128 KB each
     constexpr int NS = C::kStages, NT = C::kSlots;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -791,15 +793,15 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = ctl->tmem_base;
-    const Plan pl = make_plan<BN, kBoth>(p, prefix[kMaxGroups]);
+    const Plan pl = make_plan<BN, kBoth, kSplit>(p, prefix[kMaxGroups]);
 
     if (warp < kFirstPromoWarp) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
         if (warp == 0) {
-            produce<C, kSwiglu, kBoth>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
+            produce<C, kSwiglu, kBoth, kSplit>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
         } else if (warp == 1) {
             // -------------------------------------------------------- MMA issuer
-            Walker<BN, kBoth> wk(p, pl, prefix);
+            Walker<BN, kBoth, kSplit> wk(p, pl, prefix);
             Seg s;
             uint32_t g = 0;
             bool ok = true;
@@ -837,7 +839,8 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
         const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + grp * kPRows;
         uint8_t* my_x = xbuf + grp * (BN * 128);                // this group's half of the exchange buffer
         uint8_t* other_x = xbuf + (1 - grp) * (BN * 128);
-        Walker<BN, kBoth> wk(p, pl, prefix);
+        auto kc_of = [&](const Seg& q) { return kBoth ? q.kc : p.side[kGroups].kc; };
+        Walker<BN, kBoth, kSplit> wk(p, pl, prefix);
         Seg s, ahead;
         uint32_t g = 0;
         bool ok = true;
@@ -866,7 +869,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
             const Side& d = p.side[kBoth ? q.side : kGroups];
             as_chunk = d.as_chunk;
             as = d.a_s + (q.row0 + min(row, q.ntok - 1)) * d.as_row + q.c0 * as_chunk;
-            bs = ((!kBoth || q.side == kGroups) ? p.g_scale[grp][q.group] : p.scale[grp]) + static_cast<int64_t>(min(blk, d.nblk - 1)) * q.kc + q.c0;
+            bs = ((!kBoth || q.side == kGroups) ? p.g_scale[grp][q.group] : p.scale[grp]) + static_cast<int64_t>(min(blk, d.nblk - 1)) * kc_of(q) + q.c0;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const int k = min(i, q.c1 - q.c0 - 1);
@@ -915,40 +918,6 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
             more = wk.next(ahead);
             if (more) scales_of(ahead);
 
-            if (n_ch < s.kc) {
-                // part of a tile: park the valid rows, take a ticket; the last part of the tile adds all parts in K
-                // order and goes on to write the result
-                const int cta = static_cast<int>(blockIdx.x);
-                const int first = pl.owner(s.ut), last = pl.owner(s.ut + s.kc - 1);
-                constexpr int kTileVec = 256 * BN / 4;                     // float4 per parked tile: [64 column groups][BN rows]
-                float4* base = reinterpret_cast<float4*>(p.partials) + grp * 32 * BN + row;
-                auto part = [&](int c) { return base + (static_cast<int64_t>(c) * 2 + (pl.begin(c) >= s.ut ? 0 : 1)) * kTileVec; };
-                const bool mine_row = active && row < s.ntok;
-                if (mine_row) {
-                    float4* dst = part(cta);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j) __stcg(dst + j * BN, make_float4(acc[2 * j].x, acc[2 * j].y, acc[2 * j + 1].x, acc[2 * j + 1].y));
-                }
-                if (!last_part(p, ctl, first, last)) continue;
-#pragma unroll
-                for (int j = 0; j < 64; ++j) acc[j] = make_float2(0.0f, 0.0f);
-                if (mine_row) {
-                    for (int c = first; c <= last; ++c) {
-                        const float4* src = part(c);
-#pragma unroll
-                        for (int j0 = 0; j0 < 32; j0 += 16) {              // sixteen loads in flight
-                            float4 f[16];
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) f[j] = __ldcg(src + (j0 + j) * BN);
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) {
-                                acc[2 * (j0 + j)] = __fadd2_rn(acc[2 * (j0 + j)], make_float2(f[j].x, f[j].y));
-                                acc[2 * (j0 + j) + 1] = __fadd2_rn(acc[2 * (j0 + j) + 1], make_float2(f[j].z, f[j].w));
-                            }
-                        }
-                    }
-                }
-            }
             if (quarter * 32 >= s.ntok) continue;
             if constexpr (!kSwiglu) {
                 if (!active) continue;
@@ -1053,13 +1022,13 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
     teardown(ctl, warp, tmem_base, C::kTmemCols);
 }
 
-template <int BN, bool kSwiglu, bool kRows, bool kBoth>
+template <int BN, bool kSwiglu, bool kRows, bool kBoth, bool kSplit>
 int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, const StreamParams& prm,
                    int64_t tiles_bound, int64_t units_bound, cudaStream_t stream) {
     using C = SCfg<BN, kRows>;
     constexpr auto pick = [] {
         if constexpr (kRows) return fp8_rows_kernel<BN, kSwiglu, kBoth>;
-        else return fp8_stream_kernel<BN, kSwiglu, kBoth>;
+        else return fp8_stream_kernel<BN, kSwiglu, kBoth, kSplit>;
     };
     auto kern = pick();
     static bool configured[64] = {};
@@ -1074,7 +1043,7 @@ int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorM
         configured[dev] = true;
     }
     int64_t grid = num_sms();
-    const int64_t most = prm.partials ? units_bound : tiles_bound;      // no more CTAs than there can be work for
+    const int64_t most = kSplit ? units_bound : tiles_bound;      // no more CTAs than there can be work for
     if (grid > most) grid = most;
     DSV3_CUDA_TRY(launch_dependent(kern, dim3(static_cast<unsigned>(grid)), dim3(kNumThreads), C::kSmemBytes, stream, w0, w1, ta0, ta1, prm));
     return DSV3_OK;
@@ -1093,6 +1062,7 @@ int stream_tile(int64_t rows_per_group) {
 
 size_t stream_workspace_bytes(int64_t rows_per_group) {
     const int bn = stream_tile(rows_per_group);
+    if (bn > 64) return 0;            // 128-token tiles are never cut
     return DSV3_WORKSPACE_HEADER_BYTES + static_cast<size_t>(num_sms()) * 2 * (2 * bn) * kPRows * sizeof(float);
 }
 
@@ -1151,8 +1121,12 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
     prm.scale_fmt = q.scale_fmt;
     prm.status = status_device_ptr();
     if (!prm.status) return DSV3_ERR_CUDA;
+    // cutting tiles is worth considering when one or two rounds of whole tiles are expected (struct Plan)
     const size_t need = stream_workspace_bytes(per_tile);
-    if (q.workspace && q.workspace_bytes >= need && (reinterpret_cast<uintptr_t>(q.workspace) % 256) == 0) {
+    const int64_t groups_expected = q.n_groups < q.rows_expected ? q.n_groups : q.rows_expected;
+    const bool split = bn < 128 && groups_expected * prm.side[kGroups].tiles_p < 3 * num_sms() && q.workspace && q.workspace_bytes >= need &&
+                       (reinterpret_cast<uintptr_t>(q.workspace) % 256) == 0;
+    if (split) {
         prm.tickets = static_cast<int*>(q.workspace);
         prm.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(q.workspace) + DSV3_WORKSPACE_HEADER_BYTES);
     }
@@ -1162,17 +1136,23 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
         return DSV3_ERR_UNSUPPORTED;
     }
     const int64_t bound = tiles[0] + tiles[1];
-#define DSV3_STREAM_CASE(BN_, ROWS_)                                                                                                  \
-    return q.swiglu ? (ordinary ? launch_variant<BN_, true, ROWS_, true>(w0, w1, ta0, ta1, prm, bound, units, stream)                 \
-                                : launch_variant<BN_, true, ROWS_, false>(w0, w1, ta0, ta1, prm, bound, units, stream))               \
-                    : (ordinary ? launch_variant<BN_, false, ROWS_, true>(w0, w1, ta0, ta1, prm, bound, units, stream)                \
-                                : launch_variant<BN_, false, ROWS_, false>(w0, w1, ta0, ta1, prm, bound, units, stream))
+#define DSV3_STREAM_LAUNCH(BN_, SW_, ROWS_, SPLIT_)                                                                         \
+    return ordinary ? launch_variant<BN_, SW_, ROWS_, true, SPLIT_>(w0, w1, ta0, ta1, prm, bound, units, stream)           \
+                    : launch_variant<BN_, SW_, ROWS_, false, SPLIT_>(w0, w1, ta0, ta1, prm, bound, units, stream)
+#define DSV3_STREAM_CASE(BN_)                                                                                              \
+    case BN_:                                                                                                              \
+        if (q.swiglu) { if (split) DSV3_STREAM_LAUNCH(BN_, true, false, true); DSV3_STREAM_LAUNCH(BN_, true, false, false); } \
+        if (split) DSV3_STREAM_LAUNCH(BN_, false, false, true);                                                            \
+        DSV3_STREAM_LAUNCH(BN_, false, false, false)
     switch (bn) {
-        case 16: DSV3_STREAM_CASE(16, false);
-        case 32: DSV3_STREAM_CASE(32, false);
-        case 64: DSV3_STREAM_CASE(64, false);
-        case 128: DSV3_STREAM_CASE(128, true);
+        DSV3_STREAM_CASE(16);
+        DSV3_STREAM_CASE(32);
+        DSV3_STREAM_CASE(64);
+        case 128:
+            if (q.swiglu) DSV3_STREAM_LAUNCH(128, true, true, false);
+            DSV3_STREAM_LAUNCH(128, false, true, false);
     }
+#undef DSV3_STREAM_LAUNCH
 #undef DSV3_STREAM_CASE
     return DSV3_ERR_UNSUPPORTED;
 }
