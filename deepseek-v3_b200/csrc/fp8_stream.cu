@@ -66,15 +66,16 @@ struct SCfg {
     static constexpr int kSlotCols = kRows ? 2 * kPRows : 2 * BN;     // TMEM columns of one chunk product
     static constexpr int kSlots = kRows ? 2 : (BN <= 32 ? 8 : 512 / kSlotCols);
     static constexpr int kTmemCols = kSlots * kSlotCols;
-    // weights on the M side: ring of token scales, per-warp maxima and final scales
+    // weights on the M side: ring of scales, per-warp maxima and final scales
     static constexpr int kTabChunks = BN <= 32 ? 16 : 8;              // K chunks per slot of the scale ring
-    static constexpr int kTabBytes = kRows ? 0 : 2 * kTabChunks * BN * 4;
+    static constexpr int kTabBytes = kRows ? 0 : 2 * kTabChunks * (BN + 2) * 4;   // token scales, then the two blocks' scales
+    static constexpr int kSegBytes = kRows ? 0 : (kMaxGroups + 1) * 4;           // row offsets of the groups
     static constexpr int kRedBytes = kRows ? 0 : (4 + 1) * BN * 4;
     // tokens on the M side: exchange of SwiGLU halves / staging of results
     static constexpr int kXBytes = kRows ? 2 * BN * 128 : 0;
     // barriers, control words, group prefix and scan
     static constexpr int kCtlBytes = (2 * kStages + 2 * kSlots + 4) * 8 + static_cast<int>(sizeof(Control)) + (kMaxGroups + 1 + 8) * 4;
-    static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kTabBytes + kRedBytes + kXBytes + kCtlBytes;
+    static constexpr int kSmemBytes = 1024 + kStages * kStageBytes + kTabBytes + kRedBytes + kXBytes + kCtlBytes + kSegBytes;
     static_assert(kStageBytes >= kPRows * kChunk + kTokBytes || !kRows, "the MMA's 128 token rows stay inside the stage");
     static_assert(kSmemBytes <= 232448, "shared memory per CTA");
     static_assert(kSmemBytes > 116 * 1024, "one CTA per SM");
@@ -174,9 +175,10 @@ struct Walker {
     const StreamParams& p;
     const Plan& pl;
     const int* prefix;       // shared memory: token tiles of the groups before each group
+    const int* seg;          // row offsets of the groups, in shared memory, or where a tile is long enough in global
     int u, u1;               // next unit and end of the CTA's range
     int tile;                // next whole tile
-    __device__ __forceinline__ Walker(const StreamParams& p_, const Plan& pl_, const int* prefix_) : p(p_), pl(pl_), prefix(prefix_) {
+    __device__ __forceinline__ Walker(const StreamParams& p_, const Plan& pl_, const int* prefix_, const int* seg_) : p(p_), pl(pl_), prefix(prefix_), seg(seg_) {
         const int cta = static_cast<int>(blockIdx.x);
         u = kSplit && cta < pl.G ? pl.begin(cta) : 0;
         u1 = kSplit && cta < pl.G ? pl.begin(cta + 1) : 0;
@@ -216,8 +218,8 @@ struct Walker {
             s.group = lo;
             nq = prefix[lo + 1] - prefix[lo];
             at -= prefix[lo] * per;
-            first = __ldg(p.seg + lo);
-            rows = __ldg(p.seg + lo + 1) - first;
+            first = seg[lo];
+            rows = seg[lo + 1] - first;
         } else {
             s.group = 0;
             rows = p.side[kOrdinary].rows;
@@ -235,11 +237,18 @@ struct Walker {
 // Token tiles per group and their exclusive prefix sum over the groups, into shared memory (all threads of the CTA;
 // the caller synchronises before prefix[] is read).
 template <int BN>
-__device__ __forceinline__ void prefix_groups(const StreamParams& p, int* prefix, int* scan, int warp, int lane) {
+__device__ __forceinline__ void prefix_groups(const StreamParams& p, int* prefix, int* scan, int* seg, int warp, int lane) {
     int v = 0;
     if (threadIdx.x < kMaxGroups) {
         const int e = threadIdx.x;
-        if (e < p.n_groups) v = (__ldg(p.seg + e + 1) - __ldg(p.seg + e) + BN - 1) / BN;
+        if (e < p.n_groups) {
+            const int first = __ldg(p.seg + e), end = __ldg(p.seg + e + 1);
+            v = (end - first + BN - 1) / BN;
+            if (seg) {
+                seg[e] = first;
+                if (e == p.n_groups - 1) seg[e + 1] = end;
+            }
+        }
         int inc = v;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -264,10 +273,10 @@ __device__ __forceinline__ void prefix_groups(const StreamParams& p, int* prefix
 // The TMA producer (one converged warp).  Stage: [BN token rows][block 0][block 1] of one K chunk; of the tokens only
 // the boxes that hold any of the tile's rows are fetched.
 template <class C, bool kSwiglu, bool kBoth, bool kSplit>
-__device__ __forceinline__ void produce(const StreamParams& p, const Plan& pl, const int* prefix, const void* w0, const void* w1,
+__device__ __forceinline__ void produce(const StreamParams& p, const Plan& pl, const int* prefix, const int* seg, const void* w0, const void* w1,
                                         const void* ta0, const void* ta1, uint32_t tiles, uint32_t bar0, Control* ctl) {
     constexpr int NS = C::kStages, BN = C::BN;
-    Walker<BN, kBoth, kSplit> wk(p, pl, prefix);
+    Walker<BN, kBoth, kSplit> wk(p, pl, prefix, seg);
     Seg s;
     uint32_t g = 0;
     bool ok = true;
@@ -353,12 +362,14 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t tiles = (raw + 1023u) & ~1023u;
     uint8_t* gen = smem_raw + (tiles - raw);
-    float* tab = reinterpret_cast<float*>(gen + NS * C::kStageBytes);                 // [2][TC][BN]
+    float* tab = reinterpret_cast<float*>(gen + NS * C::kStageBytes);                 // [2][TC][BN] token scales
+    float* btab = tab + 2 * TC * BN;                                                  // [2][TC][2] scales of the two blocks
     float* red = reinterpret_cast<float*>(gen + NS * C::kStageBytes + C::kTabBytes);  // [4][BN] maxima, then [BN] scales
     uint64_t* bars = reinterpret_cast<uint64_t*>(gen + NS * C::kStageBytes + C::kTabBytes + C::kRedBytes);
     Control* ctl = reinterpret_cast<Control*>(bars + 2 * NS + 2 * NT + 4);
     int* prefix = reinterpret_cast<int*>(ctl + 1);
     int* scan = prefix + kMaxGroups + 1;                                              // [8] warp totals
+    int* seg = scan + 8;                                                              // [kMaxGroups + 1]
     const uint32_t bar0 = smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };
     auto empty_bar = [&](int s) { return bar0 + 8u * (NS + s); };
@@ -395,7 +406,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
     griddep_launch_dependents();
     griddep_wait();
-    prefix_groups<BN>(p, prefix, scan, warp, lane);
+    prefix_groups<BN>(p, prefix, scan, seg, warp, lane);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -405,10 +416,10 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
     if (warp < kFirstPromoWarp) {
       if constexpr (NP >= 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControlM));
       if (warp == 0) {
-        produce<C, kSwiglu, kBoth, kSplit>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
+        produce<C, kSwiglu, kBoth, kSplit>(p, pl, prefix, seg, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
       } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        Walker<BN, kBoth, kSplit> wk(p, pl, prefix);
+        Walker<BN, kBoth, kSplit> wk(p, pl, prefix, seg);
         Seg s;
         uint32_t g = 0;
         bool ok = true;
@@ -441,14 +452,17 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
             }
         }
       } else {
-        // ------------------------------------------------------------ token scales, TC chunks at a time
-        Walker<BN, kBoth, kSplit> wk(p, pl, prefix);
+        // ------------------------------------------------------------ scales, TC chunks at a time
+        Walker<BN, kBoth, kSplit> wk(p, pl, prefix, seg);
         Seg s;
         uint32_t t = 0;          // ring counter
         bool ok = true;
         const int tid = threadIdx.x - 64;
         while (ok && wk.next(s)) {
             const Side& d = p.side[kBoth ? s.side : kGroups];
+            // this thread's block and, below, chunk of the slot (threads below 2 TC)
+            const int blk = kSwiglu ? s.p : min(2 * s.p + (tid & 1), d.nblk - 1);
+            const float* bs = ((!kBoth || s.side == kGroups) ? p.g_scale[tid & 1][s.group] : p.scale[tid & 1]) + static_cast<int64_t>(blk) * s.kc;
             for (int k = s.c0; k < s.c1; k += TC, ++t) {
                 const int sl = t & 1;
                 ok = __all_sync(0xffffffffu, bounded_wait(sempty_bar(sl), ((t >> 1) & 1u) ^ 1u, ctl, p.status, 7, t));
@@ -459,7 +473,10 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 // the first chunk back by 7 us).  Columns beyond ntok keep what they held: they multiply products nobody reads.
                 constexpr int kLoads = TC * BN / kTabThreads;
                 static_assert(kTabThreads % BN == 0 || BN % kTabThreads == 0, "a thread's columns do not depend on the trip");
-                float r[kLoads];
+                static_assert(2 * TC <= kTabThreads, "one block scale per thread");
+                float r[kLoads], rb = 0.0f;
+                const bool has_b = (tid >> 1) < n;
+                if (has_b) rb = __ldg(bs + k + (tid >> 1));
 #pragma unroll
                 for (int u = 0; u < kLoads; ++u) {
                     const int i = tid + u * kTabThreads, ch = i / BN, col = i - ch * BN;
@@ -470,6 +487,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                     const int i = tid + u * kTabThreads, ch = i / BN, col = i - ch * BN;
                     if (ch < n && col < s.ntok) dst[i] = r[u];
                 }
+                if (has_b) btab[sl * TC * 2 + tid] = rb;
                 mbar_arrive(sfull_bar(sl));
             }
         }
@@ -483,7 +501,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         const int row = quarter * 32 + lane;                    // weight row within a block (TMEM lane)
         const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + col0;
         auto kc_of = [&](const Seg& q) { return kBoth ? q.kc : p.side[kGroups].kc; };
-        Walker<BN, kBoth, kSplit> wk(p, pl, prefix);
+        Walker<BN, kBoth, kSplit> wk(p, pl, prefix, seg);
         Seg s;
         uint32_t g = 0, t = 0;
         bool ok = true;
@@ -513,11 +531,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
             }
         };
         while (ok && wk.next(s)) {
-            const bool two = kSwiglu || 2 * s.p + 1 < p.side[kBoth ? s.side : kGroups].nblk;
             const Side& d = p.side[kBoth ? s.side : kGroups];
-            const float* b0 = ((!kBoth || s.side == kGroups) ? p.g_scale[0][s.group] : p.scale[0]) + static_cast<int64_t>(kSwiglu ? s.p : 2 * s.p) * kc_of(s);
-            const float* b1 = ((!kBoth || s.side == kGroups) ? p.g_scale[1][s.group] : p.scale[1]) +
-                              static_cast<int64_t>(kSwiglu ? s.p : (two ? 2 * s.p + 1 : 2 * s.p)) * kc_of(s);
             // pieces of this thread that hold a token of the tile
             const int np = s.ntok <= col0 ? 0 : min(NP, (s.ntok - col0 + 2 * PW - 1) / (2 * PW));
 #pragma unroll
@@ -526,7 +540,6 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 for (int i = 0; i < NP; ++i)
 #pragma unroll
                     for (int j = 0; j < PW / 2; ++j) acc[b][i][j] = make_float2(0.0f, 0.0f);
-            float bs0 = __ldg(b0 + s.c0), bs1 = __ldg(b1 + s.c0);
             int in_tab = 0;                         // chunk within the slot of the scale ring
             const int n_ch = s.c1 - s.c0;
             for (int k = 0; k < n_ch; ++k, ++g) {
@@ -536,6 +549,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                     if (!ok) break;
                 }
                 const float* as = tab + (sl * TC + in_tab) * BN + col0;
+                const float2 bs = *reinterpret_cast<const float2*>(btab + (sl * TC + in_tab) * 2);
                 const int ts = g % NT;
                 ok = __all_sync(0xffffffffu, bounded_wait_lean(tfull_bar(ts), (g / NT) & 1u, ctl, p.status, 4, g));
                 if (!ok) break;
@@ -550,13 +564,11 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 if constexpr (NP > 1) {
                     if (np > 1) load_piece(taddr, 1, v[1]);
                 }
-                const int kn = min(k + 1, n_ch - 1);                      // scales of the next chunk (the last re-reads its own)
-                const float nb0 = __ldg(b0 + s.c0 + kn), nb1 = __ldg(b1 + s.c0 + kn);
                 tc_wait_ld();
                 if (NP <= 2 || np <= 2) release();
-                if (np > 0) fold_piece(as, bs0, bs1, 0, v[0]);
+                if (np > 0) fold_piece(as, bs.x, bs.y, 0, v[0]);
                 if constexpr (NP > 1) {
-                    if (np > 1) fold_piece(as, bs0, bs1, 1, v[1]);
+                    if (np > 1) fold_piece(as, bs.x, bs.y, 1, v[1]);
                 }
                 if constexpr (NP > 2) {
                     if (np > 2) {
@@ -564,12 +576,10 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                         if (np > 3) load_piece(taddr, 3, v[1]);
                         tc_wait_ld();
                         release();
-                        fold_piece(as, bs0, bs1, 2, v[0]);
-                        if (np > 3) fold_piece(as, bs0, bs1, 3, v[1]);
+                        fold_piece(as, bs.x, bs.y, 2, v[0]);
+                        if (np > 3) fold_piece(as, bs.x, bs.y, 3, v[1]);
                     }
                 }
-                bs0 = nb0;
-                bs1 = nb1;
                 if (++in_tab == TC || k == n_ch - 1) {
                     __syncwarp();
                     if (lane == 0) mbar_arrive(sempty_bar(sl));
@@ -788,7 +798,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
     griddep_launch_dependents();
     griddep_wait();
-    prefix_groups<BN>(p, prefix, scan, warp, lane);
+    prefix_groups<BN>(p, prefix, scan, static_cast<int*>(nullptr), warp, lane);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -798,10 +808,10 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
     if (warp < kFirstPromoWarp) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
         if (warp == 0) {
-            produce<C, kSwiglu, kBoth, kSplit>(p, pl, prefix, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
+            produce<C, kSwiglu, kBoth, kSplit>(p, pl, prefix, p.seg, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
         } else if (warp == 1) {
             // -------------------------------------------------------- MMA issuer
-            Walker<BN, kBoth, kSplit> wk(p, pl, prefix);
+            Walker<BN, kBoth, kSplit> wk(p, pl, prefix, p.seg);
             Seg s;
             uint32_t g = 0;
             bool ok = true;
@@ -840,7 +850,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
         uint8_t* my_x = xbuf + grp * (BN * 128);                // this group's half of the exchange buffer
         uint8_t* other_x = xbuf + (1 - grp) * (BN * 128);
         auto kc_of = [&](const Seg& q) { return kBoth ? q.kc : p.side[kGroups].kc; };
-        Walker<BN, kBoth, kSplit> wk(p, pl, prefix);
+        Walker<BN, kBoth, kSplit> wk(p, pl, prefix, p.seg);
         Seg s, ahead;
         uint32_t g = 0;
         bool ok = true;
