@@ -976,19 +976,42 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
     } else {
         // Splitting K over the CTAs of a cluster fills idle SMs; every split pays for the exchange of partial tiles.
         // Estimate, fitted to B200 measurements (microseconds; a launch's fixed cost, 2.5-4 us, is left out):
-        //   S = 1: rounds * chunks * c1        S > 1 (all clusters resident at once): chunks / S * c + e
-        // c = time per K chunk of one CTA; c1 the same for the unsplit choice (above 128 tokens a pair kernel); neither
-        // below the time the whole problem needs at HBM bandwidth.  Measured, us, S = 1 / 2 / 4 / 8: 7168 -> 256 at
-        // M = 16 11.5 / 8.1 / 5.9 / 4.9, at M = 64 15.9 / 11.4 / 8.2 / 6.9; 7168 -> 576 at M = 256 16.3 / 15.2 / 12.1 / 11.1;
-        // a split that needs a second round of clusters loses badly (7168 -> 2048 at M = 16, S = 8: 11.7, S = 4: 6.8).
+        //   S = 1: rounds * (chunks * c + o)        S > 1 (all clusters resident at once): chunks / S * c + e
+        // c = time per K chunk of one CTA, never below the time the whole problem needs at HBM bandwidth.  Measured, us,
+        // S = 1 / 2 / 4 / 8: 7168 -> 256 at M = 16 11.5 / 8.1 / 5.9 / 4.9, at M = 64 15.9 / 11.4 / 8.2 / 6.9; 7168 -> 576 at M =
+        // 256 16.3 / 15.2 / 12.1 / 11.1; 2048 -> 1408 at M = 100 7.5 / 9.4 / 8.9 / 9.1; a split that needs a second round of
+        // clusters loses badly (7168 -> 2048 at M = 16, S = 8: 11.7, S = 4: 6.8).
         const int sms = num_sms();
-        const double c = !pl.swap ? 0.29 : (pl.bn == 64 ? 0.23 : (pl.bn == 32 ? 0.19 : 0.18));
-        const double e = !pl.swap ? 3.4 : (pl.bn == 64 ? 1.9 : (pl.bn == 32 ? 1.3 : 1.0));
-        const double c1 = !pl.swap && M > kPRows ? 0.22 : c;
+        const double c = !pl.swap ? 0.28 : (pl.bn == 64 ? 0.23 : (pl.bn == 32 ? 0.19 : 0.18));
+        const double e = !pl.swap ? 6.0 : (pl.bn == 64 ? 1.9 : (pl.bn == 32 ? 1.3 : 1.0));
         const double hbm_floor = (static_cast<double>(N) * K + static_cast<double>(M) * K) / 6.0e6;
         double best = 1e30;
         if (pl.kc <= tab) {
-            best = static_cast<double>((tiles + sms - 1) / sms) * pl.kc * c1;
+            best = static_cast<double>((tiles + sms - 1) / sms) * pl.kc * c;
+            if (!pl.swap) {
+                // Token-major tiles, three kernels: one CTA per 128 x 128 tile, or pairs on 256 x 128 and 256 x 256 tiles.
+                // The pairs fold a tile with fewer operand bytes, the small tiles fill the last round better; o = result
+                // tile and hand-over, and 0.4 to 1.2 for the cluster launch.  (Chunk times in a full machine; a single round runs at
+                // higher clocks.  Chosen so, 277 shapes of 72 to 4000 tokens are within a few per cent of the best of the
+                // three; with K below 1536 excluded from the 256 x 128 tiles and no estimate for the single CTA, thirty
+                // were 4-39 % away.)
+                const int pairs = sms / 2;
+                const int64_t pp = (static_cast<int64_t>(pl.tiles_p) + 1) / 2;
+                const auto unsplit = [&](int64_t n, int64_t units, double chunk, double chunk1, double o) {
+                    const int64_t rounds = (n + units - 1) / units;
+                    return static_cast<double>(rounds) * (pl.kc * (rounds == 1 ? chunk1 : chunk) + o);
+                };
+                best = unsplit(tiles, sms, 0.29, 0.29, 1.0);
+                if (force_kernel == 0) {
+                    const double full = pp * pl.tiles_q < pairs ? static_cast<double>(pp * pl.tiles_q) / pairs : 1.0;
+                    const double narrow = tm_pair_supported(M, N, K) ? 0.4 + 0.8 * full + unsplit(pp * pl.tiles_q, pairs, 0.265, 0.235, 0.8) : 1e30;
+                    const double wide = tw_pair_supported(M, N, K) ? 1.0 + unsplit(pp * ((N + 255) / 256), pairs, 0.41, 0.41, 1.3) : 1e30;
+                    pl.wide = wide < best && wide <= narrow;
+                    pl.pair = pl.wide || narrow < best;
+                    if (narrow < best) best = narrow;
+                    if (wide < best) best = wide;
+                }
+            }
             if (best < hbm_floor) best = hbm_floor;
         }
         for (int sfac = 2; sfac <= kMaxClusterSplits && sfac <= pl.kc; ++sfac) {
@@ -1001,6 +1024,7 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
                 best = t;
                 splits = sfac;
                 pl.cluster = true;
+                pl.pair = pl.wide = false;
             }
         }
     }
@@ -1018,35 +1042,20 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
         }
     }
     pl.splits = splits;
-    if (force_kernel == 4 && !tm_pair_supported(M, N, K, true)) {
+    if (force_kernel == 4 && !tm_pair_supported(M, N, K)) {
         set_last_error("fp8_gemm: the CTA-pair kernel needs more than 128 tokens (M=%lld)", static_cast<long long>(M));
         pl.error = DSV3_ERR_UNSUPPORTED;
         return pl;
     }
-    if (force_kernel == 6 && !tw_pair_supported(M, N, K, true)) {
+    if (force_kernel == 6 && !tw_pair_supported(M, N, K)) {
         set_last_error("fp8_gemm: the 256-wide CTA-pair kernel needs more than 128 tokens and more than 128 weight rows (M=%lld, N=%lld)",
                        static_cast<long long>(M), static_cast<long long>(N));
         pl.error = DSV3_ERR_UNSUPPORTED;
         return pl;
     }
-    if (!pl.swap && splits == 1) {
-        pl.pair = force_kernel == 4 || (force_kernel == 0 && tm_pair_supported(M, N, K, false));
+    if (force_kernel == 4 || force_kernel == 6) {
+        pl.pair = true;
         pl.wide = force_kernel == 6;
-        if (force_kernel == 0 && tw_pair_supported(M, N, K, false)) {
-            // 256-wide pair tiles against the best 128-wide alternative, in units of one SM working through one
-            // 128 x 128 tile: rounds over the machine times the tile's size, times the measured cost per flop of
-            // the wide kernel relative to the alternative (B200: 0.90-0.94 for K >= 1536 against the 128-wide
-            // pair kernel, 0.79-0.80 for shorter K against the single-CTA kernel).  Wide tiles lose where they
-            // fill the machine's last round badly (few token tiles, N a small multiple of 256).
-            const int sms = num_sms(), pairs = sms / 2;
-            const int64_t pp = (static_cast<int64_t>(pl.tiles_p) + 1) / 2;
-            const int64_t t_wide = pp * ((N + 255) / 256);
-            const double cost_wide = static_cast<double>((t_wide + pairs - 1) / pairs) * 2.0 * (pl.kc >= 12 ? 0.92 : 0.80);
-            const double cost_narrow = pl.pair ? static_cast<double>((pp * pl.tiles_q + pairs - 1) / pairs)
-                                               : static_cast<double>((tiles + sms - 1) / sms);
-            pl.wide = cost_wide <= cost_narrow;
-        }
-        pl.pair = pl.pair || pl.wide;
     }
     return pl;
 }

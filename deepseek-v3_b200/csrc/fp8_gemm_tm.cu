@@ -434,15 +434,12 @@ fp8_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 
 }  // namespace
 
-bool tm_pair_supported(int64_t M, int64_t N, int64_t K, bool forced) {
+bool tm_pair_supported(int64_t M, int64_t N, int64_t K) {
     (void)N;
-    // At least two token tiles (otherwise the second CTA of a pair would multiply zeros) and, when the choice is
-    // the library's, at least 12 K chunks: with short K the per-tile work of the promotion warps (first scale
-    // fetch, result tile) weighs more than the operand stream, and the single-CTA kernel with two-chunk hand-offs
-    // is faster (measured on B200, M = 4096: K = 512: 135 vs 111 us at N = 32768; K = 1536: 202 vs 205 us at
-    // N = 24576; K = 7168: 566 vs 617 us at N = 18432).
-    if (M <= kPRows) return false;
-    return forced || K >= 12 * kChunk;
+    (void)K;
+    // At least two token tiles: otherwise the second CTA of a pair would multiply zeros.  Whether it is the faster kernel for
+    // a problem is the plan's decision (tc_plan).
+    return M > kPRows;
 }
 
 int launch_fp8_gemm_tm(const void* a, const float* a_s, const void* b, const float* b_s, int64_t M, int64_t N,

@@ -428,9 +428,8 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 
 }  // namespace
 
-bool tw_pair_supported(int64_t M, int64_t N, int64_t K, bool forced) {
+bool tw_pair_supported(int64_t M, int64_t N, int64_t K) {
     (void)K;
-    (void)forced;
     // At least two token tiles (otherwise the second CTA of a pair would multiply zeros) and more than one weight
     // block (otherwise half of every accumulator would).  Whether it is the faster kernel for a problem is the
     // plan's decision (tc_plan).

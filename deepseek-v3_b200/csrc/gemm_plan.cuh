@@ -33,13 +33,12 @@ int make_tmap(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int b
 int make_tmap_out(CUtensorMap* map, void* base, int64_t M, int64_t N);
 
 // Token-major kernel on CTA pairs (256 x 128 tiles, tcgen05 cta_group::2, no split-K): fp8_gemm_tm.cu.
-// `forced`: the kernel was pinned, so only its hard limit applies, not the speed heuristic.
-bool tm_pair_supported(int64_t M, int64_t N, int64_t K, bool forced);
+bool tm_pair_supported(int64_t M, int64_t N, int64_t K);
 int launch_fp8_gemm_tm(const void* a, const float* a_s, const void* b, const float* b_s, int64_t M, int64_t N,
                        int64_t K, void* c, cudaStream_t stream);
 
 // Token-major kernel on CTA pairs with 256-wide accumulators (256 x 256 tiles, no split-K): fp8_gemm_tw.cu.
-bool tw_pair_supported(int64_t M, int64_t N, int64_t K, bool forced);
+bool tw_pair_supported(int64_t M, int64_t N, int64_t K);
 int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const float* b_s, int64_t M, int64_t N,
                        int64_t K, void* c, cudaStream_t stream);
 
