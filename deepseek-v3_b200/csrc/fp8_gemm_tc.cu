@@ -11,8 +11,8 @@
 //
 // The pipeline moves "units" of UC consecutive K chunks, numbered g = 0,1,2,... across all work
 // items of a CTA (UC = 2 for token-major tiles, 1 for weight-major tiles):
-//   warp 0 (1 lane)          TMA producer: waits empty[g % NS], loads the P and Q tiles of the unit's chunks
-//   warps 1,2 (1 lane each)  MMA issuers, unit g belongs to issuer g % 2: wait tempty[g % NT] and full[g % NS],
+//   warp 0                   TMA producer: waits empty[g % NS], loads the P and Q tiles of the unit's chunks
+//   warps 1,2                MMA issuers, unit g belongs to issuer g % 2: wait tempty[g % NT] and full[g % NS],
 //                            issue 4 MMAs per chunk, commit to empty[g % NS] and tfull[g % NT]
 //   warps 4..11              promotion: wait tfull[g % NT], read the unit back from TMEM (token-major: both
 //                            chunks behind a single tcgen05.wait::ld), release tempty, then do the FMAs; at
@@ -21,8 +21,11 @@
 // Operand roles: P is the 128-row MMA "A" operand, Q the BN-row MMA "B" operand.
 //   kSwap = false : P = 128 tokens of a,  Q = 128 rows of b  (M > 64: "token-major" tiles)
 //   kSwap = true  : P = 128 rows of b,    Q = BN tokens of a (M <= 64: "weight-major", weights stream once)
-// Split-K: a work item is (tile, split); partial tiles go to a workspace and the CTA that
-// takes the last ticket of a tile adds them in split order (deterministic, no spinning).
+// (producer and issuer warps stay converged; one elected lane issues)
+// Split-K, up to eight splits: the splits of a tile are the CTAs of one cluster, which exchange rows of the partial tile
+// through distributed shared memory and each add a share in split order.  Pinned factors, and more splits: a work item is
+// (tile, split), partial tiles go to a workspace and the CTA that takes the last ticket of a tile adds them in split order.
+// Both are deterministic; nothing spins.
 //
 // Hand-off costs set the structure: a dependent mbarrier.try_wait takes ~175 cycles even when the
 // phase is already complete and tcgen05.fence::after_thread_sync is of the same order, while a chunk

@@ -17,10 +17,10 @@
 // the promotion work per SM is unchanged.
 //
 // Roles, per CTA (r = rank in the pair; the even CTA is the leader):
-//   warp 0 (1 lane)          TMA producer: stage = two K chunks = 2 x (16 KB tokens + 8 KB weight half), four stages.
+//   warp 0                   TMA producer (converged, one elected lane issues): stage = two K chunks = 2 x (16 KB tokens + 8 KB weight half), four stages.
 //                            Both producers' loads complete on the LEADER's full[] barrier (ordinary, non-multicast
 //                            loads; only the completion signal crosses to the peer), each waits on its own empty[].
-//   warps 1,2 (1 lane each)  leader only: MMA issuers; the issuer of unit g (= chunks 2g, 2g+1) is g % 2 and owns
+//   warps 1,2                leader only: MMA issuers (the same); the issuer of unit g (= chunks 2g, 2g+1) is g % 2 and owns
 //                            TMEM slots 2*(g%2), 2*(g%2)+1 (in both CTAs).  Per chunk: wait tempty[slot] (16 arrivals:
 //                            the promotion warps of both CTAs), 4 x tcgen05.mma.cta_group::2 kind::f8f6f4 (M256 N128
 //                            K32), commit -> tfull[slot] of both CTAs; per unit: commit -> empty[stage] of both CTAs.

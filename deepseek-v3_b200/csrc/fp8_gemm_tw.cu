@@ -10,24 +10,23 @@
 // pipe's rate.  With N = 256 an instruction runs 128 cycles on 12 KB (4 KB of tokens, 8 KB of weights of which
 // half sit in the peer's shared memory), 96 B/clk, and a chunk needs 32 KB of loads per SM for 512 tensor-core
 // cycles instead of 24 KB for 256.  The price: the fp32 accumulator of one SM is 128 x 256 (128 registers in each
-// of 256 promotion threads), TMEM holds only two chunk products, and the read-back buffers shrink to 2 x 32
+// of 256 promotion threads), TMEM holds only two chunk products, and the read-back buffer shrinks to 64
 // registers per thread.
 //
 // Roles, per CTA (r = rank in the pair; the even CTA is the leader):
-//   warp 0 (1 lane)   TMA producer: stage = one K chunk = 16 KB tokens + 16 KB weights (this CTA's 128 of the
+//   warp 0            TMA producer (converged, one elected lane issues): stage = one K chunk = 16 KB tokens + 16 KB weights (this CTA's 128 of the
 //                     tile's 256 weight rows), five stages.  Both producers' loads complete on the LEADER's full[]
 //                     barrier (ordinary, non-multicast loads; only the completion signal crosses to the peer),
 //                     each waits on its own empty[].
-//   warps 1,2 (1 lane each)  leader only: MMA issuers; chunk g belongs to issuer g % 2, which owns TMEM slot g % 2.
+//   warps 1,2         leader only: MMA issuers (converged, one elected lane issues); chunk g belongs to issuer g % 2, which owns TMEM slot g % 2.
 //                     Per chunk: wait full[stage], wait tempty[slot] (16 arrivals: the promotion warps of both CTAs),
 //                     4 x tcgen05.mma.cta_group::2 kind::f8f6f4 (M256 N256 K32), commit -> tfull[slot] and
 //                     empty[stage] of both CTAs.  Stages alternate between the issuers, so full[] is waited for
 //                     without a probe.
 //   warps 4..11       promotion of this CTA's 128 x 256 half: warps 4..7 own columns 0..127 (one b_s block), warps
 //                     8..11 columns 128..255; a thread owns one accumulator row.  A chunk product is read back in
-//                     four pieces of 32 columns into two alternating buffers: while the tcgen05.ld of one piece is
-//                     in flight the FMAs of the piece before issue; the last piece of a chunk is folded under the
-//                     first load of the next chunk.  The slot goes back to the issuer when its last load has landed.
+//                     two halves of 64 columns through one buffer; the slot goes back to the issuer when the second
+//                     load has landed, and that half's FMAs follow the release.
 //                     Result tile: bf16 through shared memory and TMA stores.
 //
 // Every mbarrier wait is bounded: after about a second the waiting thread records what it was waiting for in
@@ -62,9 +61,7 @@ constexpr int kStorePasses = 1;                       // result tile staged whol
 constexpr int kStages = kStorePasses == 1 ? 5 : 6;    // of one chunk each
 constexpr int kSlots = 2;                             // TMEM slots of one chunk product (256 columns) each
 constexpr int kTmemCols = kSlots * kBN;
-constexpr int kPiece = 32;                            // columns per read-back
-constexpr int kPieces = 128 / kPiece;                 // read-backs per chunk product and thread
-static_assert(kPieces % 2 == 0, "a chunk's first piece goes to buffer 0 while buffer 1 holds the last piece of the chunk before");
+constexpr int kPiece = 32;                            // columns of an FMA batch; a read-back is two of them
 constexpr int kStoreBytes = kPRows * kBN * 2 / kStorePasses;   // bf16 result tile: 128-byte-swizzled 128 x 64 boxes
 constexpr int kSmemBytes = kStages * kChunkBytes + kStoreBytes + 1024 + 1024;
 static_assert(kSmemBytes <= 232448, "shared memory per CTA");

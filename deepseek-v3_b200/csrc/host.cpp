@@ -22,6 +22,7 @@
 #include <array>
 #include <exception>
 #include <memory>
+#include <algorithm>
 #include <vector>
 
 #include "dsv3_b200.h"
@@ -146,32 +147,48 @@ struct Workspace {
     int device;
     cudaStream_t stream;
     at::Tensor mem;
+    bool captured;          // a CUDA graph may refer to it: kept for good
 };
+// Ordered by last use.  Beyond kKeptWorkspaces the least recently used one goes back to torch's allocator, which
+// hands its memory out again in the order of the stream it was used on.
 // (never destroyed: at process exit the CUDA context may already be gone)
 std::vector<Workspace>& g_workspaces = *new std::vector<Workspace>;
-// Smaller predecessors of a grown workspace: a captured graph may still refer to them.  Sizes at least double, so
-// together they stay below the size of the live one.
+constexpr size_t kKeptWorkspaces = 16;
+// Predecessors of a grown workspace that a captured graph may still refer to.  Sizes at least double, so together they
+// stay below the size of the live one.
 std::vector<at::Tensor>& g_retired = *new std::vector<at::Tensor>;
 
 // The header of a workspace must be zero on first use; every call leaves it zero again.
 const at::Tensor& workspace(c10::Device dev, size_t bytes) {
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-    Workspace* slot = nullptr;
-    for (Workspace& w : g_workspaces)
-        if (w.device == dev.index() && w.stream == stream) slot = &w;
-    if (slot && static_cast<size_t>(slot->mem.numel()) >= bytes) return slot->mem;
-    int64_t size = std::max<int64_t>(static_cast<int64_t>(bytes), 16ll << 20);
-    if (slot) size = std::max<int64_t>(size, 2 * slot->mem.numel());
-    c10::cuda::OptionalCUDAGuard guard(dev);
-    at::Tensor mem = new_cuda({size}, at::kByte, dev);
-    if (cudaMemsetAsync(mem.data_ptr(), 0, DSV3_WORKSPACE_HEADER_BYTES, stream) != cudaSuccess)
-        raise(PyExc_RuntimeError, "could not clear the header of a new split-K workspace");
-    if (slot) {
-        g_retired.push_back(slot->mem);
-        slot->mem = mem;
-        return slot->mem;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    (void)cudaStreamIsCapturing(stream, &status);
+    const bool capturing = status != cudaStreamCaptureStatusNone;
+    auto it = std::find_if(g_workspaces.begin(), g_workspaces.end(),
+                           [&](const Workspace& w) { return w.device == dev.index() && w.stream == stream; });
+    const bool found = it != g_workspaces.end();
+    if (!found || static_cast<size_t>(it->mem.numel()) < bytes) {
+        int64_t size = std::max<int64_t>(static_cast<int64_t>(bytes), 16ll << 20);
+        if (found) size = std::max<int64_t>(size, 2 * it->mem.numel());
+        c10::cuda::OptionalCUDAGuard guard(dev);
+        at::Tensor mem = new_cuda({size}, at::kByte, dev);
+        if (cudaMemsetAsync(mem.data_ptr(), 0, DSV3_WORKSPACE_HEADER_BYTES, stream) != cudaSuccess)
+            raise(PyExc_RuntimeError, "could not clear the header of a new split-K workspace");
+        if (found) {
+            if (it->captured) g_retired.push_back(it->mem);
+            it->mem = std::move(mem);
+            it->captured = false;
+        } else {
+            if (g_workspaces.size() >= kKeptWorkspaces) {
+                auto old = std::find_if(g_workspaces.begin(), g_workspaces.end(), [](const Workspace& w) { return !w.captured; });
+                if (old != g_workspaces.end()) g_workspaces.erase(old);
+            }
+            g_workspaces.push_back({dev.index(), stream, std::move(mem), false});
+            it = g_workspaces.end() - 1;
+        }
     }
-    g_workspaces.push_back({dev.index(), stream, mem});
+    it->captured |= capturing;
+    if (it + 1 != g_workspaces.end()) std::rotate(it, it + 1, g_workspaces.end());
     return g_workspaces.back().mem;
 }
 
