@@ -105,8 +105,7 @@ struct Cfg {
     // Split-K inside a cluster: partial sums that the other CTAs send here.  16- and 32-token tiles have room of their own
     // for them; the others re-use the operand stages once every CTA of the cluster is through with its own.
     static constexpr bool kOwnExchange = kSwap && BN < 64;
-    static constexpr int kExchangePitch = kSwap ? BN + 4 : BN;               // floats per row (weight-major: + 16 bytes against bank conflicts)
-    static constexpr int kExchangeBytes = (kPRows + 8) * kExchangePitch * 4;    // splits * ceil(128 / splits) rows
+    static constexpr int kExchangeBytes = (kPRows + 10) * BN * 4;    // splits * (ceil(128 / splits) | 1) rows, at most 138
     static constexpr int kStagesRaw =
         (232448 - 2048 - kStoreBytes - kScaleTabBytes - (kOwnExchange ? kExchangeBytes : 0)) / kStageBytes;
     static constexpr int kStagesCap = kStagesRaw > 10 ? 10 : kStagesRaw;
@@ -570,27 +569,23 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                 // tile (st.shared::cluster), a cluster barrier later everybody adds what arrived, in split order.
                 // Against the ticket form below (partial tiles through L2, an atomic, the last arrival reads
                 // everything back) this takes about 1.5 us off a launch.
+                // A peer is reached in 512-byte runs: a store per row, 16 bytes at a time, made the same exchange 1.1 us
+                // slower for 128-token tiles and 0.6 us for 64 (7168 -> 576 at M = 256 10.5 -> 9.2, at M = 64 7.4 -> 6.7).
                 const int S = p.splits, R = (kPRows + S - 1) / S;
                 if constexpr (!C::kOwnExchange) cluster_arrive();   // through with the operand stages
                 cluster_wait();                                     // every CTA runs, and with shared stages is through with them
                 const int dest = static_cast<int>(fast_div(static_cast<uint32_t>(row), p.div_rows)), r_local = row - dest * R;
                 const uint32_t remote = mapa_shared(smem_u32(exchange), static_cast<uint32_t>(dest));
                 const int ntok = static_cast<int>(min(static_cast<int64_t>(BN), m_end - (q_base - col0)));   // weight-major tiles
-                if constexpr (kSwap) {              // [split][R rows][tokens]
-                    const uint32_t at = remote + 4u * ((it.split * R + r_local) * C::kExchangePitch + col0);
+                // [split][four columns][R | 1 rows] float4: the lanes of a store are consecutive rows, 512 contiguous bytes on
+                // their way to the peer
+                const int Rp = R | 1;
+                const uint32_t at = remote + 16u * ((it.split * (BN / 4) + col0 / 4) * Rp + r_local);
 #pragma unroll
-                    for (int j = 0; j < CPT; j += 4)
-                        if (col0 + j < ntok)
-                            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at + 4u * j), "f"(accf[j]), "f"(accf[j + 1]),
-                                         "f"(accf[j + 2]), "f"(accf[j + 3]) : "memory");
-                } else {                            // [split][R rows][32 16-byte slots], slot c of row r at c ^ (r & 31)
-#pragma unroll
-                    for (int j = 0; j < CPT / 4; ++j) {
-                        const uint32_t at = remote + 512u * (it.split * R + r_local) + 16u * ((col0 / 4 + j) ^ (row & 31));
-                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at), "f"(accf[4 * j]), "f"(accf[4 * j + 1]),
+                for (int j = 0; j < CPT / 4; ++j)
+                    if (!kSwap || col0 + 4 * j < ntok)
+                        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(at + 16u * j * Rp), "f"(accf[4 * j]), "f"(accf[4 * j + 1]),
                                      "f"(accf[4 * j + 2]), "f"(accf[4 * j + 3]) : "memory");
-                    }
-                }
                 cluster_arrive();
                 cluster_wait();
                 const int me = static_cast<int>(cluster_ctarank()), rows_here = min(R, kPRows - me * R);
@@ -601,10 +596,10 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                     for (int e = tid; e < (ntok + 3) / 4 * R; e += kPromoThreads) {
                         const int t4 = static_cast<int>(fast_div(static_cast<uint32_t>(e), p.div_rows)), i = e - t4 * R;
                         if (i >= rows_here || n0 + i >= N) continue;
-                        const float* src = exchange + i * C::kExchangePitch + 4 * t4;
-                        float4 sum = *reinterpret_cast<const float4*>(src);
+                        const float4* src = reinterpret_cast<const float4*>(exchange) + t4 * Rp + i;
+                        float4 sum = *src;
                         for (int sp = 1; sp < S; ++sp) {
-                            const float4 a = *reinterpret_cast<const float4*>(src + sp * R * C::kExchangePitch);
+                            const float4 a = src[sp * (BN / 4) * Rp];
                             sum.x += a.x; sum.y += a.y; sum.z += a.z; sum.w += a.w;
                         }
                         __nv_bfloat16* dst = p.c + (static_cast<int64_t>(it.row0) + 4 * t4) * N + n0 + i;
@@ -621,8 +616,8 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                         if (m >= M || n >= N) continue;
                         float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
                         for (int sp = 0; sp < S; ++sp) {
-                            const float4* src = reinterpret_cast<const float4*>(exchange) + 32 * (sp * R + i);
-                            const float4 a = src[(2 * k8) ^ (r_tile & 31)], b = src[(2 * k8 + 1) ^ (r_tile & 31)];
+                            const float4* src = reinterpret_cast<const float4*>(exchange) + (sp * (BN / 4) + 2 * k8) * Rp + i;
+                            const float4 a = src[0], b = src[Rp];
                             lo.x += a.x; lo.y += a.y; lo.z += a.z; lo.w += a.w;
                             hi.x += b.x; hi.y += b.y; hi.z += b.z; hi.w += b.w;
                         }
@@ -895,11 +890,9 @@ bool tc_supported(const void* a, const void* b, const void* c, int64_t M, int64_
 // How many clusters of `splits` CTAs of a variant the device holds at once (GPCs do not divide evenly by every size).
 namespace {
 template <int BN, bool kSwap>
-int clusters_of(int splits) {
+int clusters_of(int dev, int splits) {
     using C = Cfg<BN, kSwap>;
     static int cached[64][kMaxClusterSplits + 1] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = -1;
     if (dev >= 0 && cached[dev][splits] > 0) return cached[dev][splits];
     int n = 0;
     if (dev >= 0) {
@@ -926,10 +919,10 @@ int clusters_of(int splits) {
 }
 }  // namespace
 
-static int64_t clusters_resident(bool swap, int bn, int splits) {
-    const int n = !swap ? clusters_of<128, false>(splits)
-                        : (bn == 16 ? clusters_of<16, true>(splits) : (bn == 32 ? clusters_of<32, true>(splits) : clusters_of<64, true>(splits)));
-    const int budget = num_sms() / splits;
+static int64_t clusters_resident(int dev, int sms, bool swap, int bn, int splits) {
+    const int n = !swap ? clusters_of<128, false>(dev, splits)
+                        : (bn == 16 ? clusters_of<16, true>(dev, splits) : (bn == 32 ? clusters_of<32, true>(dev, splits) : clusters_of<64, true>(dev, splits)));
+    const int budget = sms / splits;
     return n < budget ? n : budget;
 }
 
@@ -979,15 +972,17 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
     } else {
         // Splitting K over the CTAs of a cluster fills idle SMs; every split pays for the exchange of partial tiles.
         // Estimate, fitted to B200 measurements (microseconds; a launch's fixed cost, 2.5-4 us, is left out):
-        //   S = 1: rounds * (chunks * c + o)        S > 1 (all clusters resident at once): chunks / S * c + e
-        // c = time per K chunk of one CTA, never below the time the whole problem needs at HBM bandwidth.  Measured, us,
-        // S = 1 / 2 / 4 / 8: 7168 -> 256 at M = 16 11.5 / 8.1 / 5.9 / 4.9, at M = 64 15.9 / 11.4 / 8.2 / 6.9; 7168 -> 576 at M =
-        // 256 16.3 / 15.2 / 12.1 / 11.1; 2048 -> 1408 at M = 100 7.5 / 9.4 / 8.9 / 9.1; a split that needs a second round of
-        // clusters loses badly (7168 -> 2048 at M = 16, S = 8: 11.7, S = 4: 6.8).
+        //   S = 1: rounds * (chunks * c + o)        S > 1 (all clusters resident at once): chunks / S * c + e(S)
+        // c = time per K chunk of one CTA; the chunks never take less than the operands need at 6 TB/s, or at 60 GB/s for
+        // each CTA there is (weight-major tiles; what a CTA's operand ring can keep in flight).  Measured, us, S = 2 / 3 /
+        // 4 / 6 / 8: 12288 -> 5120 at M = 1 15.4 / 13.2 / - / - / -; 7168 -> 2304 at M = 16 9.1 / 8.0 / 7.5 / 6.9 / -; 7168 -> 576
+        // at M = 64 11.4 / 9.5 / 8.3 / 7.8 / 7.1; 7168 -> 1536 at M = 200 13.5 / 12.3 / 11.0 / - / -, S = 5 11.3 (rows that do not
+        // divide evenly); a split that needs a second round of clusters loses badly (7168 -> 2048 at M = 16, S = 8: 12.9).
         const int sms = num_sms();
-        const double c = !pl.swap ? 0.28 : (pl.bn == 64 ? 0.23 : (pl.bn == 32 ? 0.19 : 0.18));
-        const double e = !pl.swap ? 6.0 : (pl.bn == 64 ? 1.9 : (pl.bn == 32 ? 1.3 : 1.0));
-        const double hbm_floor = (static_cast<double>(N) * K + static_cast<double>(M) * K) / 6.0e6;
+        const double c = !pl.swap ? 0.28 : (pl.bn == 64 ? 0.23 : 0.24);
+        const double e = !pl.swap ? 4.9 : (pl.bn == 64 ? 1.0 : 0.8), e_split = !pl.swap ? 0.0 : (pl.bn == 64 ? 0.05 : 0.1);
+        const double bytes = static_cast<double>(N) * K + static_cast<double>(M) * K;
+        const auto hbm_floor = [&](int64_t ctas) { return bytes / (pl.swap && ctas < 100 ? 6.0e4 * ctas : 6.0e6); };
         double best = 1e30;
         if (pl.kc <= tab) {
             best = static_cast<double>((tiles + sms - 1) / sms) * pl.kc * c;
@@ -1015,14 +1010,17 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
                     if (wide < best) best = wide;
                 }
             }
-            if (best < hbm_floor) best = hbm_floor;
+            if (const double floor = hbm_floor(tiles); best < floor) best = floor;
         }
+        // (the device is looked up once per plan: every look-up is 50 ns of a 4 us call)
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = -1;
         for (int sfac = 2; sfac <= kMaxClusterSplits && sfac <= pl.kc; ++sfac) {
             const int per_item = (pl.kc + sfac - 1) / sfac;
-            if (per_item > tab || tiles > clusters_resident(pl.swap, pl.bn, sfac)) continue;
+            if (per_item > tab || tiles > clusters_resident(dev, sms, pl.swap, pl.bn, sfac)) continue;
             double t = per_item * c;
-            if (t < hbm_floor) t = hbm_floor;
-            t += e;
+            if (const double floor = hbm_floor(tiles * sfac); t < floor) t = floor;
+            t += e + e_split * sfac + (!pl.swap && (sfac & (sfac - 1)) ? 0.6 : 0.0);
             if (t < best - 1e-9) {
                 best = t;
                 splits = sfac;
