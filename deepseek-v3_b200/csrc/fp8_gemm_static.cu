@@ -87,6 +87,9 @@ int dsv3_fp8_gemm_static(const void* a, const float* a_s, const void* b, const f
                        "call dsv3_fp8_gemm");
         return DSV3_ERR_UNSUPPORTED;
     }
+    // the same kernel as dsv3_fp8_gemm picks; this one needs no scratch
+    if (forced == 0 && gemm_policy_split() == 0 && decode_kernel_pays(M, N, K) && small_linear_supported(a, b, c, M, N, K, false))
+        return launch_fp8_linear_small(nullptr, a, a_s, b, b_s, M, N, K, DSV3_SCALE_FMT_FP32, c, st);
     TcPlan pl = tc_plan(M, N, K, forced, gemm_policy_split());
     if (pl.error != DSV3_OK) return pl.error;
     // The automatic plan may want more partial tiles than the array holds: fall back to the largest split factor

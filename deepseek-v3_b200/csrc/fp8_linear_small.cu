@@ -16,12 +16,14 @@
 //     copies already quantised activations there; the fragments are 16-byte shared-memory loads;
 //   * every chunk's product is scaled as the reference does, acc = fma(p * a_s, b_s, acc) (kernel.py:162);
 //   * K is split over the warps of a CTA and over the CTAs of a cluster (at most 8); partial sums meet in the
-//     shared memory of the cluster's first CTA (st.shared::cluster), which adds them in a fixed order, so the
-//     result is deterministic and no global scratch or atomics are involved.
+//     CTA's shared memory and then in that of the cluster's first CTA (st.shared::cluster), added in a fixed order,
+//     so the result is deterministic and no global scratch or atomics are involved.
 //
 // No wait in this kernel can hang: the only synchronisation is __syncthreads and the cluster barrier, which every
 // thread reaches unconditionally.
 #include <cuda.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "gemm_plan.cuh"
@@ -61,8 +63,8 @@ __device__ __forceinline__ void mma_e4m3(float (&d)[4], uint32_t a0, uint32_t a1
 
 __device__ __forceinline__ void prefetch_l2(const void* ptr) { asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr)); }
 
-__device__ __forceinline__ void st_cluster_f32(uint32_t addr_cluster, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr_cluster), "f"(v) : "memory");
+__device__ __forceinline__ void st_cluster_f32x4(uint32_t addr_cluster, float4 v) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr_cluster), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
 }
 
 constexpr size_t align16(size_t v) { return (v + 15) & ~static_cast<size_t>(15); }
@@ -93,7 +95,9 @@ __global__ void __launch_bounds__(kThreads) fp8_linear_small_kernel(const SmallP
     float* xs_s = reinterpret_cast<float*>(smem + align16(static_cast<size_t>(TOK) * row_bytes));   // [TOK][cpc]
     float* bs_s = xs_s + TOK * cpc;                                              // [WR][cpc]
     float* slots = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bs_s) + align16(static_cast<size_t>(WR) * cpc * 4));
-    // slots: [csize * WK][WR][16][TOK] partial sums, used in the cluster's first CTA
+    // partial sums: slots [WK][TOK][ROWS] of this CTA's warps, then [csize][TOK][ROWS] of the CTAs (the cluster's first one)
+    constexpr int ROWS = WR * 16;
+    float* gathered = slots + WK * TOK * ROWS;
 
     // rows of this lane (clamped at the edge: the loads stay inside the matrix, the results are masked)
     const uint8_t* wa = p.w + static_cast<int64_t>(min(r0 + g, N - 1)) * K + 16 * t;
@@ -102,6 +106,7 @@ __global__ void __launch_bounds__(kThreads) fp8_linear_small_kernel(const SmallP
     // into L2 may overlap the tail of the kernel that produces the activations (L2 is the point of coherence: if
     // that kernel were still writing the weights, the loads after the wait would see its data all the same).
     griddep_launch_dependents();
+    if (p.csize > 1) cluster_arrive();        // waited for before the first store into the first CTA's shared memory
     if (t == 0) {
         for (int s = 0; s < kRing && s < n_w; ++s) {
             prefetch_l2(wa + static_cast<int64_t>(w0 + s) * kChunkK);
@@ -127,31 +132,42 @@ __global__ void __launch_bounds__(kThreads) fp8_linear_small_kernel(const SmallP
 
     // ---- the CTA's K range of the activations: FP8 bytes and scales into shared memory
     if constexpr (kFused) {
-        // a half-warp per (token, chunk) block: 16 lanes x 8 bf16, as in the stand-alone act_quant kernel.  (Measured
-        // on B200: fetching several blocks per half-warp at once, or staging the bf16 rows with asynchronous copies
-        // first, helps at 8 tokens but costs registers or shared memory that the single-token case pays for; with
-        // more than a few tokens the per-CTA quantisation is the wrong trade anyway, see dsv3_fp8_linear's callers.)
+        // a half-warp per (token, chunk) block: 16 lanes x 8 bf16, as in the stand-alone act_quant kernel, kBlocks of them
+        // requested at once (each round is a trip to L2)
+        constexpr int kHalves = kThreads / 16;
         const int l16 = threadIdx.x & 15;
         const int nblk = p.M * n_cta;
-        for (int b0 = (threadIdx.x >> 5) * 2; b0 < nblk; b0 += kThreads / 16) {     // warp-uniform trip count
-            const int b = b0 + ((threadIdx.x >> 4) & 1);
-            const bool valid = b < nblk;
-            const int m = valid ? b / n_cta : 0;
-            const int cl = valid ? b - m * n_cta : 0;
-            const uint4 v = valid ? __ldg(p.x + (static_cast<int64_t>(m) * K + static_cast<int64_t>(c0 + cl) * kChunkK) / 8 + l16)
-                                  : zero4;
-            float mx = amax8(v);
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-            const float sc = scale_from_amax(mx, p.scale_fmt);
-            if (valid) {
-                const uint2 q = (p.scale_fmt == DSV3_SCALE_FMT_FP32) ? quant8<true>(v, sc) : quant8<false>(v, sc);
-                *reinterpret_cast<uint2*>(xq_s + m * row_bytes + cl * kChunkK + l16 * 8) = q;
-                if (l16 == 0) xs_s[m * cpc + cl] = sc;
+        auto quantise = [&](auto blocks) {
+            constexpr int kBlocks = decltype(blocks)::value;
+            for (int b0 = (threadIdx.x >> 5) * 2; b0 < nblk; b0 += kBlocks * kHalves) {     // warp-uniform trip count
+                uint4 v[kBlocks];
+                int m[kBlocks], cl[kBlocks];
+#pragma unroll
+                for (int i = 0; i < kBlocks; ++i) {
+                    const int b = b0 + i * kHalves + ((threadIdx.x >> 4) & 1);
+                    m[i] = b < nblk ? (p.M == 1 ? 0 : b / n_cta) : -1;
+                    cl[i] = m[i] >= 0 ? b - m[i] * n_cta : 0;
+                    v[i] = m[i] >= 0 ? __ldg(p.x + (static_cast<int64_t>(m[i]) * K + static_cast<int64_t>(c0 + cl[i]) * kChunkK) / 8 + l16) : zero4;
+                }
+#pragma unroll
+                for (int i = 0; i < kBlocks; ++i) {
+                    if (b0 + i * kHalves >= nblk) break;           // warp-uniform
+                    float mx = amax8(v[i]);
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+                    const float sc = scale_from_amax(mx, p.scale_fmt);
+                    if (m[i] >= 0) {
+                        const uint2 q = (p.scale_fmt == DSV3_SCALE_FMT_FP32) ? quant8<true>(v[i], sc) : quant8<false>(v[i], sc);
+                        *reinterpret_cast<uint2*>(xq_s + m[i] * row_bytes + cl[i] * kChunkK + l16 * 8) = q;
+                        if (l16 == 0) xs_s[m[i] * cpc + cl[i]] = sc;
+                    }
+                }
             }
-        }
+        };
+        if (nblk <= kHalves) quantise(std::integral_constant<int, 1>{});
+        else quantise(std::integral_constant<int, 4>{});
     } else {
         // already quantised activations: asynchronous 16-byte copies, all in flight at once
         const int pieces = n_cta * (kChunkK / 16);               // 16-byte pieces per token row
@@ -227,35 +243,42 @@ __global__ void __launch_bounds__(kThreads) fp8_linear_small_kernel(const SmallP
         }
     }
 
-    // ---- partial sums of all K splits meet in the first CTA of the cluster
-    {
-        const uint32_t base = mapa_shared(smem_u32(slots), 0);
-        const int slot = static_cast<int>(rank) * WK + wk;
+    // ---- partial sums: the warps' meet in the CTA's shared memory, the CTAs' in that of the cluster's first one.  (Every
+    // warp's 4-byte stores straight to the first CTA, tokens beyond M among them, made a launch up to 2.5 us slower: each is
+    // a packet of its own, and one SM receives them all.)
 #pragma unroll
-        for (int j = 0; j < MT; ++j)
+    for (int j = 0; j < MT; ++j)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int row = g + ((i & 2) ? 8 : 0), tok = 8 * j + 2 * t + (i & 1);
-                st_cluster_f32(base + 4u * static_cast<uint32_t>(((slot * WR + wr) * 16 + row) * TOK + tok), acc[j][i]);
-            }
-    }
+        for (int i = 0; i < 4; ++i) {
+            const int row = g + ((i & 2) ? 8 : 0), tok = 8 * j + 2 * t + (i & 1);
+            if (tok < p.M) slots[(wk * TOK + tok) * ROWS + wr * 16 + row] = acc[j][i];
+        }
+    __syncthreads();
     if (p.csize > 1) {
+        cluster_wait();       // every CTA of the cluster runs
+        const uint32_t first = mapa_shared(smem_u32(gathered), 0);
+        for (int idx = threadIdx.x; idx < ROWS / 4 * p.M; idx += kThreads) {
+            float4 sum = reinterpret_cast<const float4*>(slots)[idx];       // [token][rows]: idx runs over both
+#pragma unroll
+            for (int s = 1; s < WK; ++s) {
+                const float4 v = reinterpret_cast<const float4*>(slots + s * TOK * ROWS)[idx];
+                sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+            }
+            st_cluster_f32x4(first + 4u * (rank * TOK * ROWS + 4 * idx), sum);
+        }
         cluster_arrive();
         cluster_wait();
-    } else {
-        __syncthreads();      // launched without a cluster: the slots are this CTA's own
+        if (rank != 0) return;
     }
-    if (rank == 0) {
-        const int n_slots = p.csize * WK;
-        constexpr int ROWS = WR * 16;
-        for (int idx = threadIdx.x; idx < ROWS * p.M; idx += kThreads) {
-            const int tok = idx / ROWS, rw = idx - tok * ROWS;
-            const int n = rowgroup * ROWS + rw;
-            if (n >= N) continue;
-            float sum = 0.0f;
-            for (int s = 0; s < n_slots; ++s) sum += slots[(s * ROWS + rw) * TOK + tok];
-            p.c[static_cast<int64_t>(tok) * N + n] = __float2bfloat16_rn(sum);
-        }
+    const float* src = p.csize > 1 ? gathered : slots;
+    const int parts = p.csize > 1 ? p.csize : WK;
+    for (int idx = threadIdx.x; idx < ROWS * p.M; idx += kThreads) {
+        const int tok = idx / ROWS, rw = idx - tok * ROWS;
+        const int n = rowgroup * ROWS + rw;
+        if (n >= N) continue;
+        float sum = 0.0f;
+        for (int s = 0; s < parts; ++s) sum += src[s * TOK * ROWS + idx];
+        p.c[static_cast<int64_t>(tok) * N + n] = __float2bfloat16_rn(sum);
     }
 }
 
@@ -309,6 +332,13 @@ bool small_linear_supported(const void* act, const void* w, const void* c, int64
            (K % (fused ? 128 : 16)) == 0;
 }
 
+// Automatic choice of the register-streaming kernel: up to 8 rows, up to 8 MB of weights in at most 4096 rows (its layout
+// that splits K over the warps too).  It has less to set up than the tcgen05 pipeline; beyond 8 MB, or with more rows, the
+// tcgen05 kernel's TMA ring streams better.  B200, us, this kernel / tcgen05 at M = 1: 1024 -> 512 2.7 / 3.6; 7168 -> 576
+// 4.1 / 4.8; 2048 -> 1408 4.0 / 4.2; 5120 -> 1536 5.0 / 5.3; 16384 -> 512 6.0 / 6.8; 7168 -> 1536 6.3 / 5.8; 1024 -> 7168 4.3 /
+// 4.1; at M = 16 2048 -> 1408 4.7 / 4.4.  K is bounded by the activations that a CTA stages, 128 K chunks even unsplit.
+bool decode_kernel_pays(int64_t M, int64_t N, int64_t K) { return M <= 8 && N <= 4096 && K <= 16384 && N * K <= (8ll << 20); }
+
 // x != nullptr: fused (bf16 activations); otherwise (a, a_s) are the quantised activations.
 int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, const void* w, const float* w_s, int64_t M,
                             int64_t N, int64_t K, int scale_fmt, void* c, cudaStream_t stream) {
@@ -337,7 +367,7 @@ int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, cons
     const int mt = M <= 8 ? 1 : 2;
     const int tok = 8 * mt;
     const size_t smem = align16(static_cast<size_t>(tok) * (prm.cpc * kChunkK + kRowPad)) + static_cast<size_t>(tok) * prm.cpc * 4 +
-                        align16(static_cast<size_t>(wr) * prm.cpc * 4) + align16(static_cast<size_t>(csize) * wk * wr * 16 * tok * 4) + 16;
+                        align16(static_cast<size_t>(wr) * prm.cpc * 4) + static_cast<size_t>(csize + wk) * wr * 16 * tok * 4 + 16;
     if (smem > 200 * 1024) {
         set_last_error("fp8_linear: K=%lld is too long for the decode kernel's staging buffer", static_cast<long long>(K));
         return DSV3_ERR_UNSUPPORTED;

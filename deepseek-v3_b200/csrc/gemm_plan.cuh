@@ -45,6 +45,7 @@ int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const flo
 // Decode-sized Linear without tcgen05 set-up (fp8_linear_small.cu): M <= 16; x != nullptr quantises bf16 activations
 // in the kernel's prologue (K % 128 == 0), otherwise (a, a_s) are the quantised activations (K % 16 == 0).
 bool small_linear_supported(const void* act, const void* w, const void* c, int64_t M, int64_t N, int64_t K, bool fused);
+bool decode_kernel_pays(int64_t M, int64_t N, int64_t K);
 int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, const void* w, const float* w_s, int64_t M,
                             int64_t N, int64_t K, int scale_fmt, void* c, cudaStream_t stream);
 

@@ -577,7 +577,9 @@ PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_DECREF(scale_obj);
         if (!scale.defined()) raise(PyExc_TypeError, "weight.scale is not a tensor");
         const int64_t K = last_dim(x), rows = K ? x.numel() / K : 0;
-        if (rows > 0 && rows <= int_arg(args[5]) && w.numel() <= int_arg(args[6]) && block == 128 && K % 128 == 0 &&
+        // Every CTA quantises its K range of all rows: from three rows up two launches are faster for large weights (B200, us,
+        // fused / two at 4 rows: 7168 -> 1536 8.9 / 6.9, 5120 -> 1536 7.4 / 6.4, 2048 -> 2816 5.8 / 5.9, 7168 -> 576 5.3 / 6.3).
+        if (rows > 0 && rows <= int_arg(args[5]) && w.numel() <= int_arg(args[6]) && (rows <= 2 || w.numel() <= (6ll << 20)) && block == 128 && K % 128 == 0 &&
             x.scalar_type() == at::kBFloat16 && x.is_contiguous()) {
             count(g_key_fused);
             return wrap(linear_small(x, w, scale, fmt));

@@ -164,6 +164,14 @@ def test_cluster_split_k_against_the_cuda_core_kernel(M, N, K):
     assert_gemm_close(y.cpu(), kernel.fp8_gemm(a, a_s, b, b_s).cpu())
 
 
+# up to 8 rows and 8 MB of weights: the decode kernel's warps and CTAs each add a part of K -- one row group and one chunk, rows
+# that end inside a group, K tails, the largest N, the longest K
+@pytest.mark.parametrize("M", [1, 5, 8])
+@pytest.mark.parametrize("N,K", [(1, 16), (16, 128), (17, 16384), (512, 16384), (576, 7056), (4096, 2048), (4095, 1040)])
+def test_decode_kernel_against_the_cuda_core_kernel(M, N, K):
+    test_cluster_split_k_against_the_cuda_core_kernel(M, N, K)
+
+
 def test_swiglu_fast_form_equals_the_frameworks_silu_for_every_bf16():
     """swiglu8 rounds its fast silu a little below and above itself and falls back where the two differ: every finite bf16
     value of a, against act_quant(F.silu(a) * b) bit for bit."""
