@@ -122,24 +122,30 @@ def grouped_moe_forward(self, x: torch.Tensor, *, world_size: int = 1, fallback=
             raise NotImplementedError("grouped MoE needs FP8 expert weights, bf16 activations and <= 256 local experts")
         return fallback(self, x)
     shape = x.size()
-    x = x.view(-1, self.dim)
+    flat = len(shape) == 2 and shape[1] == self.dim       # (a view costs the host 2 us)
+    if not flat:
+        x = x.view(-1, self.dim)
     weights, indices = self.gate(x)
     st = _grouped(self)
     n_routed = getattr(self, "n_routed_experts", 0)
+    shared = None
     if world_size == 1 and x.size(0) <= SHARED_INLINE_MAX_ROWS:
         shared = plain_weights(self.shared_experts, x, st.scale_fmt)
-        if shared is not None:
-            return host.combine(st.run(x, weights, indices, n_routed, shared), None).view(shape)
-    routed = st.run(x, weights, indices, n_routed)
-    z = self.shared_experts(x)
-    if world_size > 1:
-        import torch.distributed as dist
+    routed = st.run(x, weights, indices, n_routed, shared)
+    if shared is not None:
         y = host.combine(routed, None)
-        dist.all_reduce(y)
-        return (y + z).view(shape)
-    if z.dtype == torch.bfloat16 and z.is_contiguous() and z.size() == x.size():
-        return host.combine(routed, z).view(shape)
-    return (host.combine(routed, None) + z).view(shape)
+    else:
+        z = self.shared_experts(x)
+        if world_size > 1:
+            import torch.distributed as dist
+            y = host.combine(routed, None)
+            dist.all_reduce(y)
+            y = y + z
+        elif z.dtype == torch.bfloat16 and z.is_contiguous() and z.size() == x.size():
+            y = host.combine(routed, z)
+        else:
+            y = host.combine(routed, None) + z
+    return y if flat else y.view(shape)
 
 
 def install_moe(model_module) -> None:
