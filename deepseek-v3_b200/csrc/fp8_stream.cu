@@ -514,7 +514,8 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 else tc_ld_x16(taddr + b * BN + 2 * PW * i, vv[b]);
             }
         };
-        // acc += (product * a_s) * b_s; one shared-memory load of the token scales serves both blocks
+        // acc += product * (a_s * b_s), the order of the other tcgen05 kernels, so that a tile that is not cut equals theirs bit
+        // for bit; one shared-memory load of the token scales serves both blocks
         auto fold_piece = [&](const float* as, float bs0, float bs1, int i, const uint32_t (&vv)[2][PW]) {
             const float4* as4 = reinterpret_cast<const float4*>(as + 2 * PW * i);
             const float2 b2[2] = {make_float2(bs0, bs0), make_float2(bs1, bs1)};
@@ -523,10 +524,9 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 const float4 a4 = as4[j];
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
-                    const float2 lo = __fmul2_rn(make_float2(__uint_as_float(vv[b][4 * j]), __uint_as_float(vv[b][4 * j + 1])), make_float2(a4.x, a4.y));
-                    const float2 hi = __fmul2_rn(make_float2(__uint_as_float(vv[b][4 * j + 2]), __uint_as_float(vv[b][4 * j + 3])), make_float2(a4.z, a4.w));
-                    acc[b][i][2 * j] = __ffma2_rn(lo, b2[b], acc[b][i][2 * j]);
-                    acc[b][i][2 * j + 1] = __ffma2_rn(hi, b2[b], acc[b][i][2 * j + 1]);
+                    const float2 lo = __fmul2_rn(make_float2(a4.x, a4.y), b2[b]), hi = __fmul2_rn(make_float2(a4.z, a4.w), b2[b]);
+                    acc[b][i][2 * j] = __ffma2_rn(make_float2(__uint_as_float(vv[b][4 * j]), __uint_as_float(vv[b][4 * j + 1])), lo, acc[b][i][2 * j]);
+                    acc[b][i][2 * j + 1] = __ffma2_rn(make_float2(__uint_as_float(vv[b][4 * j + 2]), __uint_as_float(vv[b][4 * j + 3])), hi, acc[b][i][2 * j + 1]);
                 }
             }
         };

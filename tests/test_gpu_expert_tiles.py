@@ -1,0 +1,92 @@
+"""Tiles of the expert GEMMs (w1/w3 with SwiGLU and quantisation, w2): whole and cut over K.
+
+References: the separate operators per group of rows.  Whole tiles fold every chunk as the other tcgen05 kernels do, so
+with the operators pinned to one split the results are equal bit for bit."""
+import ctypes
+
+import pytest
+import torch
+
+from test_gpu_stream import _Side, _bf16_default, _table, _weight  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+class _Layer:
+    """w1 / w3 / w2 of len(counts) groups, their rows, and an ordinary weight of side_rows rows next to them."""
+
+    def __init__(self, counts, inter, dim, side_rows, seed=0):
+        import kernel
+        from dsv3_b200 import _lib
+        self.counts, self.inter, self.dim, self.side_rows = counts, inter, dim, side_rows
+        g = torch.Generator(device="cuda").manual_seed(seed + sum(counts) * 7 + dim)
+        rows = lambda m, k: torch.randn(m, k, generator=g, device="cuda", dtype=torch.float32).bfloat16()
+        self.n, self.rows = len(counts), sum(counts)
+        self.w1, self.w3, self.w2 = ([_weight(a, b, g) for _ in counts] for a, b in ((inter, dim), (inter, dim), (dim, inter)))
+        self.tables = [_table(_lib.lib, _lib.check, w, *w[0].shape) for w in (self.w1, self.w3, self.w2)]
+        self.xq, self.xs = kernel.act_quant(rows(self.rows, dim))
+        self.xs_t = self.xs.t().contiguous()
+        self.seg = torch.tensor([sum(counts[:i]) for i in range(self.n + 1)], dtype=torch.int32, device="cuda")
+        if side_rows:
+            self.sq, self.ss = kernel.act_quant(rows(side_rows, dim))
+            self.s1, self.s3, self.s2 = _weight(256, dim, g), _weight(256, dim, g), _weight(dim, 256, g)
+        lib = _lib.lib
+        lib.dsv3_gemm_rows_workspace_bytes.restype = ctypes.c_size_t
+        self.need = lib.dsv3_gemm_rows_workspace_bytes(self.n, ctypes.c_int64(self.rows), ctypes.c_int64(0))
+
+    def run(self, workspace=None, between=lambda: None):
+        """(hq, hs_t, o) and, with side_rows, (zq, zs_t, z)."""
+        from dsv3_b200 import _lib
+        lib, i64, p = _lib.lib, ctypes.c_int64, lambda t: ctypes.c_void_p(t.data_ptr())
+        f8, f32 = dict(dtype=torch.uint8, device="cuda"), dict(dtype=torch.float32, device="cuda")
+        hq, hs, o = torch.zeros(self.rows, self.inter, **f8), torch.zeros(self.inter // 128, self.rows, **f32), torch.zeros(self.rows, self.dim, device="cuda")
+        out, up, down = [hq, hs, o], None, None
+        if self.side_rows:
+            m = self.side_rows
+            zq, zs, z = torch.zeros(m, 256, **f8), torch.zeros(2, m, **f32), torch.zeros(m, self.dim, device="cuda")
+            out += [zq, zs, z]
+            up = ctypes.byref(_Side(self.sq.data_ptr(), self.ss.data_ptr(), 0, m, 256, self.dim, self.s1.data_ptr(), self.s1.scale.data_ptr(),
+                                    self.s3.data_ptr(), self.s3.scale.data_ptr(), zq.data_ptr(), zs.data_ptr()))
+            down = ctypes.byref(_Side(zq.data_ptr(), zs.data_ptr(), 1, m, self.dim, 256, self.s2.data_ptr(), self.s2.scale.data_ptr(), None, None,
+                                      z.data_ptr(), None))
+        tail = (p(workspace) if workspace is not None else None, ctypes.c_size_t(workspace.numel() if workspace is not None else 0),
+                ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        t1, t3, t2 = self.tables
+        _lib.check(lib.dsv3_swiglu_gemm_rows(p(t1), p(t3), self.n, p(self.xq), p(self.xs_t), p(self.seg), i64(self.rows), i64(0), i64(self.inter),
+                                             i64(self.dim), 0, p(hq), p(hs), up, *tail))
+        between()
+        _lib.check(lib.dsv3_fp8_gemm_rows(p(t2), self.n, p(hq), p(hs), p(self.seg), i64(self.rows), i64(0), i64(self.dim), i64(self.inter), p(o), down,
+                                          *tail))
+        torch.cuda.synchronize()
+        return out
+
+    def operators(self, hq, hs, zq=None, zs=None):
+        """The operators' results per group; w2 works on the given hq / hs (and s2 on zq / zs)."""
+        import kernel
+        from dsv3_b200 import swiglu_quant
+        f8 = torch.float8_e4m3fn
+        parts = []
+        for e, c in enumerate(self.counts):
+            if c:
+                r = slice(sum(self.counts[:e]), sum(self.counts[:e + 1]))
+                a = (self.xq[r].contiguous(), self.xs[r].contiguous())
+                q, s = swiglu_quant(kernel.fp8_gemm(*a, self.w1[e], self.w1[e].scale), kernel.fp8_gemm(*a, self.w3[e], self.w3[e].scale))
+                parts.append((q, s.t(), kernel.fp8_gemm(hq[r].contiguous().view(f8), hs[:, r].t().contiguous(), self.w2[e], self.w2[e].scale)))
+        out = [torch.cat([p[0] for p in parts]), torch.cat([p[1] for p in parts], dim=1), torch.cat([p[2] for p in parts])]
+        if zq is not None:
+            q, s = swiglu_quant(kernel.fp8_gemm(self.sq, self.ss, self.s1, self.s1.scale), kernel.fp8_gemm(self.sq, self.ss, self.s3, self.s3.scale))
+            out += [q, s.t(), kernel.fp8_gemm(zq.view(f8), zs.t().contiguous(), self.s2, self.s2.scale)]
+        return out
+
+
+# every tile width (16, 32, 64 tokens with the weights on the M side, 128 with the tokens there), tiles with one row more
+@pytest.mark.parametrize("counts,policy", [([3, 0, 1, 17, 1, 0, 2, 5], 3), ([16, 33, 0, 7], 3), ([64, 5, 65, 30], 3), ([128, 60, 0, 7, 129], 2)],
+                         ids=["tile16", "tile32", "tile64", "tile128"])
+def test_whole_tiles_equal_the_operators_bit_for_bit(counts, policy):
+    import dsv3_b200
+    layer = _Layer(counts, 384, 1152, 9)
+    got = layer.run()
+    dsv3_b200.set_gemm_policy(policy, 1)             # one split, chunks in order
+    want = layer.operators(got[0], got[1], got[3], got[4])
+    for a, b in zip(got, want):
+        assert torch.equal(a.view(torch.uint8) if a.element_size() == 1 else a, b.view(torch.uint8) if b.element_size() == 1 else b)
