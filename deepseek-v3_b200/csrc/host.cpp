@@ -7,7 +7,7 @@
 // The extension adds nothing to the C ABI: it fills in the same arguments a C host would.
 //
 // Threads and streams: every entry point is called with the GIL held and releases it only around the library call;
-// the split-K workspaces are keyed on (device, stream), and calls that share one are ordered by their stream.
+// the split-K workspaces are keyed on (device, stream, capture), and calls that share one are ordered by their stream.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -142,30 +142,43 @@ void call_library(c10::Device dev, F&& f) {
     check(status);
 }
 
-// ------------------------------------------------------------------ split-K workspaces, one per (device, stream)
+// Which capture a stream takes part in: 0 for none, otherwise a number that no other capture of the process has.
+unsigned long long capture_of(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(stream, &status, &id) != cudaSuccess) {
+        (void)cudaGetLastError();          // the legacy stream next to a capture: not capturing itself
+        return 0;
+    }
+    return status == cudaStreamCaptureStatusNone ? 0 : id + 1;
+}
+
+// ------------------------------------------------------------------ split-K workspaces, one per (device, stream, capture)
 struct Workspace {
     int device;
     cudaStream_t stream;
+    unsigned long long capture;      // 0: eager calls
     at::Tensor mem;
-    bool captured;          // a CUDA graph may refer to it: kept for good
 };
-// Ordered by last use.  Beyond kKeptWorkspaces the least recently used one goes back to torch's allocator, which
-// hands its memory out again in the order of the stream it was used on.
+// Ordered by last use; beyond kKeptWorkspaces the one used longest ago goes back to torch's allocator, which hands its
+// memory out again in the order of the stream it was used on.
+// A graph has a workspace of its own: its header is cleared by a node of that graph, which nothing else may rely on (the
+// graph may be replayed late, never, or after another one), and a replay may run beside eager calls on the stream the graph
+// was captured on.  Its memory comes from the graph's pool, which stays reserved as long as the graph lives, so the
+// reference is given up when the stream is next seen in another capture or in none.
 // (never destroyed: at process exit the CUDA context may already be gone)
 std::vector<Workspace>& g_workspaces = *new std::vector<Workspace>;
 constexpr size_t kKeptWorkspaces = 16;
-// Predecessors of a grown workspace that a captured graph may still refer to.  Sizes at least double, so together they
-// stay below the size of the live one.
-std::vector<at::Tensor>& g_retired = *new std::vector<at::Tensor>;
 
 // The header of a workspace must be zero on first use; every call leaves it zero again.
 const at::Tensor& workspace(c10::Device dev, size_t bytes) {
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    (void)cudaStreamIsCapturing(stream, &status);
-    const bool capturing = status != cudaStreamCaptureStatusNone;
-    auto it = std::find_if(g_workspaces.begin(), g_workspaces.end(),
-                           [&](const Workspace& w) { return w.device == dev.index() && w.stream == stream; });
+    const unsigned long long capture = capture_of(stream);
+    const auto here = [&](const Workspace& w) { return w.device == dev.index() && w.stream == stream; };
+    g_workspaces.erase(std::remove_if(g_workspaces.begin(), g_workspaces.end(),
+                                      [&](const Workspace& w) { return here(w) && w.capture != 0 && w.capture != capture; }),
+                       g_workspaces.end());
+    auto it = std::find_if(g_workspaces.begin(), g_workspaces.end(), [&](const Workspace& w) { return here(w) && w.capture == capture; });
     const bool found = it != g_workspaces.end();
     if (!found || static_cast<size_t>(it->mem.numel()) < bytes) {
         int64_t size = std::max<int64_t>(static_cast<int64_t>(bytes), 16ll << 20);
@@ -175,19 +188,13 @@ const at::Tensor& workspace(c10::Device dev, size_t bytes) {
         if (cudaMemsetAsync(mem.data_ptr(), 0, DSV3_WORKSPACE_HEADER_BYTES, stream) != cudaSuccess)
             raise(PyExc_RuntimeError, "could not clear the header of a new split-K workspace");
         if (found) {
-            if (it->captured) g_retired.push_back(it->mem);
             it->mem = std::move(mem);
-            it->captured = false;
         } else {
-            if (g_workspaces.size() >= kKeptWorkspaces) {
-                auto old = std::find_if(g_workspaces.begin(), g_workspaces.end(), [](const Workspace& w) { return !w.captured; });
-                if (old != g_workspaces.end()) g_workspaces.erase(old);
-            }
-            g_workspaces.push_back({dev.index(), stream, std::move(mem), false});
+            if (g_workspaces.size() >= kKeptWorkspaces) g_workspaces.erase(g_workspaces.begin());
+            g_workspaces.push_back({dev.index(), stream, capture, std::move(mem)});
             it = g_workspaces.end() - 1;
         }
     }
-    it->captured |= capturing;
     if (it + 1 != g_workspaces.end()) std::rotate(it, it + 1, g_workspaces.end());
     return g_workspaces.back().mem;
 }
