@@ -275,6 +275,7 @@ struct Remembered {
     int64_t block;
     int fmt;
     cudaStream_t stream;
+    unsigned long long capture;   // a graph's quantisation is computed at its replays: for that capture only; and the other way round
     at::Tensor q, s;
 };
 std::vector<Remembered>& g_memo = *new std::vector<Remembered>;     // at most two, most recent first
@@ -293,10 +294,10 @@ void remember(const at::Tensor& x, int64_t block, int fmt, bool assume_no_inplac
     const bool counted = !x.is_inference();
     if (!counted && !assume_no_inplace) return;
     if (g_memo.size() > 1) g_memo.pop_back();
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(x.device().index()).stream();
     g_memo.insert(g_memo.begin(),
                   Remembered{decltype(Remembered::x)(x.getIntrusivePtr()), x.const_data_ptr(), {x.sizes().begin(), x.sizes().end()},
-                             counted ? static_cast<int64_t>(x._version()) : -1, block, fmt,
-                             c10::cuda::getCurrentCUDAStream(x.device().index()).stream(), q, s});
+                             counted ? static_cast<int64_t>(x._version()) : -1, block, fmt, stream, capture_of(stream), q, s});
 }
 
 std::pair<at::Tensor, at::Tensor> quantise_remembered(const at::Tensor& x, int64_t block, int fmt, bool assume_no_inplace) {
@@ -311,7 +312,7 @@ std::pair<at::Tensor, at::Tensor> quantise_remembered(const at::Tensor& x, int64
         Remembered& e = g_memo[i];
         // a weak reference keeps the TensorImpl's address from being reused, so equal addresses mean the same tensor
         if (e.x._unsafe_get_target() == x.unsafeGetTensorImpl() && e.version == version && e.data == x.const_data_ptr() &&
-            e.block == block && e.fmt == fmt && e.stream == stream && x.sizes() == at::IntArrayRef(e.sizes)) {
+            e.block == block && e.fmt == fmt && e.stream == stream && x.sizes() == at::IntArrayRef(e.sizes) && e.capture == capture_of(stream)) {
             count(g_key_reused);
             if (i) std::swap(g_memo[0], g_memo[i]);
             return {g_memo[0].q, g_memo[0].s};

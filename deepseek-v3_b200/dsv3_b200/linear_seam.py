@@ -19,7 +19,8 @@ branches and changes how the FP8 branch is launched:
 
 The memo holds the two most recent inputs (``wq_a(x)``, ``wq_b(q_norm(..))``, ``wkv_a(x)`` of model.py:464-468
 touch two tensors alternately).  An entry is reused only for the same tensor object, on the same CUDA stream,
-with an unchanged in-place modification counter.  Tensors created under ``torch.inference_mode()`` have no such
+with an unchanged in-place modification counter, and inside a graph capture only for that capture (the quantisation is
+then part of the graph).  Tensors created under ``torch.inference_mode()`` have no such
 counter: for them the memo is off unless ``assume_no_inplace=True`` is passed to ``install_linear`` -- the host
 then promises not to modify a projection's input in place between two Linears (the reference's model.py never
 does).

@@ -1,4 +1,5 @@
-"""State that the host extension keeps between calls, across the boundary of a CUDA graph: workspaces.
+"""State that the host extension keeps between calls, across the boundary of a CUDA graph: workspaces and
+remembered quantisations.
 
 A pass through a graph must not depend on which other graph, or which eager call, came before it."""
 import pytest
@@ -65,3 +66,51 @@ def test_ticket_header_of_a_workspace_that_a_capture_made(order, make):
         graphs[i].replay()
         torch.cuda.synchronize()
         assert torch.equal(outs[i], want)
+
+
+def _inputs():
+    g = torch.Generator(device="cuda").manual_seed(8)
+    x = torch.randn(2, 40, 1024, generator=g, device="cuda", dtype=torch.float32).bfloat16()
+    return x[0].clone(), x[1].clone(), _weight(256, 1024, g), _weight(384, 1024, g)
+
+
+def test_a_graph_does_not_use_the_quantisation_of_an_eager_call():
+    """The usual order of a host: a warm pass and the capture on one stream, then replays with new contents."""
+    from dsv3_b200 import linear_seam as L
+    x, new, w, w3 = _inputs()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        L.linear(x, w)
+    stream.synchronize()
+    L.stats.update(act_quant_calls=0, act_quant_reused=0)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        y, y3 = L.linear(x, w), L.linear(x, w3)
+    assert (L.stats["act_quant_calls"], L.stats["act_quant_reused"]) == (1, 1), "shared inside the capture"
+    want, want3 = L.linear(new, w), L.linear(new, w3)
+    x.copy_(new)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and torch.equal(y3, want3)
+
+
+def test_an_eager_call_does_not_use_the_quantisation_of_a_graph():
+    """A quantisation recorded in a capture has not been computed; another capture does not own it either."""
+    from dsv3_b200 import linear_seam as L
+    x, _, w, w3 = _inputs()
+    want, want3 = L.linear(x.clone(), w), L.linear(x.clone(), w3)
+    stream = torch.cuda.Stream()
+    keep = _polluted_pool(stream)
+    graphs, outs = [], []
+    for _ in range(2):
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1], pool=keep.pool(), stream=stream):
+            outs.append(L.linear(x, w3))
+    with torch.cuda.stream(stream):
+        got = L.linear(x, w)
+    stream.synchronize()
+    assert torch.equal(got, want)
+    for i in (1, 0):
+        graphs[i].replay()
+        torch.cuda.synchronize()
+        assert torch.equal(outs[i], want3)
