@@ -170,8 +170,10 @@ struct Workspace {
 std::vector<Workspace>& g_workspaces = *new std::vector<Workspace>;
 constexpr size_t kKeptWorkspaces = 16;
 
-// The header of a workspace must be zero on first use; every call leaves it zero again.
-const at::Tensor& workspace(c10::Device dev, size_t bytes) {
+// The header of a workspace must be zero on first use; every call leaves it zero again.  The caller holds the returned tensor
+// until its launches have been issued: while it has released the GIL for them, another thread may replace or drop the
+// entry, and only memory given up after the launches is handed out behind them in the stream's order.
+at::Tensor workspace(c10::Device dev, size_t bytes) {
     const cudaStream_t stream = c10::cuda::getCurrentCUDAStream(dev.index()).stream();
     const unsigned long long capture = capture_of(stream);
     const auto here = [&](const Workspace& w) { return w.device == dev.index() && w.stream == stream; };
@@ -235,13 +237,9 @@ at::Tensor gemm(const at::Tensor& a, const at::Tensor& a_s, const at::Tensor& b,
     require_bf16_default();
     at::Tensor c = new_cuda_last(a, N, at::kBFloat16);
     const size_t need = dsv3_fp8_gemm_workspace_bytes(M, N, K);
-    void* ws = nullptr;
-    size_t ws_bytes = 0;
-    if (need) {
-        const at::Tensor& w = workspace(dev, need);
-        ws = w.data_ptr();
-        ws_bytes = static_cast<size_t>(w.numel());
-    }
+    const at::Tensor held = need ? workspace(dev, need) : at::Tensor();
+    void* ws = need ? held.data_ptr() : nullptr;
+    const size_t ws_bytes = need ? static_cast<size_t>(held.numel()) : 0;
     const void *ap = a.const_data_ptr(), *bp = b.const_data_ptr();
     const float *asp = static_cast<const float*>(a_s.const_data_ptr()), *bsp = static_cast<const float*>(b_s.const_data_ptr());
     void* cp = c.data_ptr();
@@ -438,13 +436,10 @@ std::unique_ptr<Routed> run_experts(Experts& e, const at::Tensor& x_in, const at
     r->pos = reinterpret_cast<const int32_t*>(base + o_pos);
     if (P == 0) return r;
     at::Tensor xq = new_cuda(x.sizes(), at::kFloat8_e4m3fn, dev), xs = new_cuda_last(x, dim / 128, at::kFloat);
-    void* ws = nullptr;
-    size_t ws_bytes = 0;
-    if (const size_t need = dsv3_gemm_rows_workspace_bytes(e.n, P, hint)) {
-        const at::Tensor& w = workspace(dev, need);
-        ws = w.data_ptr();
-        ws_bytes = static_cast<size_t>(w.numel());
-    }
+    const size_t need = dsv3_gemm_rows_workspace_bytes(e.n, P, hint);
+    const at::Tensor held = need ? workspace(dev, need) : at::Tensor();
+    void* ws = need ? held.data_ptr() : nullptr;
+    const size_t ws_bytes = need ? static_cast<size_t>(held.numel()) : 0;
     auto* seg = reinterpret_cast<int32_t*>(base + o_seg);
     auto* xs_t = reinterpret_cast<float*>(base + o_xs);
     auto* hs_t = reinterpret_cast<float*>(base + o_hs);
