@@ -79,13 +79,13 @@ __global__ void __launch_bounds__(kThreads, 4) moe_combine_kernel(const __nv_bfl
 // A CTA owns `tpc` consecutive tokens and needs the rows of their pairs: the first row of every expert (all pairs) plus
 // how many pairs of the expert belong to earlier tokens.  Instead of a second launch or a grid barrier every CTA counts
 // all pairs itself, 8 bytes per pair from L2 into shared-memory histograms (one CTA doing all the bookkeeping took 59 us
-// for 16 K pairs); one large CTA per SM keeps that to 16 pairs per thread.  Several CTAs along y share a CTA's tokens when there are few tokens; they
-// derive the same rows, because a pair's place among the CTA's own pairs is counted in order there.
+// for 16 K pairs); one large CTA per SM keeps that to 16 pairs per thread.  An expert's rows are in the order of the pairs,
+// counted and never drawn from an atomic: where the expert GEMMs cut a tile over K, its place decides the order of its sums,
+// so a row's place must not depend on timing.  It also lets several CTAs along y share a CTA's tokens when there are few.
 constexpr int kDispMaxExperts = 256;
-constexpr int kDispPairs = 1024;          // own pairs of a CTA
-constexpr int kDispOrdered = 64;          // own pairs up to which rows are assigned in order
 constexpr int kDispUnroll = 4;
 constexpr int kDispThreads = 1024;
+constexpr int kDispPairs = kDispThreads;  // own pairs of a CTA: one per thread
 
 struct DispatchParams {
     const uint4* x;                       // bf16 [T, dim]
@@ -106,6 +106,7 @@ struct DispatchParams {
 __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const DispatchParams p) {
     __shared__ int total[kDispMaxExperts], before[kDispMaxExperts], scan[kDispMaxExperts / 32];
     __shared__ int own_e[kDispPairs], own_row[kDispPairs];
+    __shared__ __align__(8) uint8_t in_warp[kDispThreads / 32][kDispMaxExperts];      // a warp's own pairs of each expert
     griddep_launch_dependents();
     griddep_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -118,6 +119,8 @@ __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const Dispat
         total[tid] = 0;
         before[tid] = 0;
     }
+    static_assert(sizeof(in_warp) == 8 * kDispThreads, "eight bytes per thread");
+    reinterpret_cast<uint2*>(&in_warp[0][0])[tid] = make_uint2(0u, 0u);
     __syncthreads();
 #pragma unroll 4
     for (int64_t pr = tid; pr < p.P; pr += kDispThreads) {
@@ -127,9 +130,16 @@ __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const Dispat
             if (pr < own0) atomicAdd(&before[e], 1);
         }
     }
-    for (int i = tid; i < own; i += kDispThreads) {
-        const int64_t e = __ldg(p.indices + own0 + i);
-        own_e[i] = static_cast<int>(max(min(e, static_cast<int64_t>(0x3fffffff)), static_cast<int64_t>(-1)));
+    int mine = -1, rank_in_warp;              // this thread's pair: local expert and its place among the warp's pairs of that expert
+    {
+        if (tid < own) {
+            const int64_t e = __ldg(p.indices + own0 + tid);
+            own_e[tid] = static_cast<int>(max(min(e, static_cast<int64_t>(0x3fffffff)), static_cast<int64_t>(-1)));
+            if (e >= p.start && e - p.start < p.n) mine = static_cast<int>(e - p.start);
+        }
+        const unsigned same = __match_any_sync(0xffffffffu, mine);
+        rank_in_warp = __popc(same & ((1u << lane) - 1u));
+        if (mine >= 0 && rank_in_warp == 0) in_warp[warp][mine] = static_cast<uint8_t>(__popc(same));
     }
     __syncthreads();
     // exclusive prefix sum over the experts; before[] becomes the first row of this CTA's pairs of each expert
@@ -154,23 +164,18 @@ __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const Dispat
         }
     }
     __syncthreads();
-    for (int i = tid; i < own; i += kDispThreads) {
-        const int e = own_e[i] - p.start;
+    if (tid < own) {
         int row = -1;
-        if (e >= 0 && e < p.n) {
-            if (own <= kDispOrdered) {
-                int k = 0;
-                for (int j = 0; j < i; ++j) k += own_e[j] == own_e[i];
-                row = before[e] + k;
-            } else {
-                row = atomicAdd(&before[e], 1);
-            }
+        if (mine >= 0) {
+            row = before[mine] + rank_in_warp;
+            for (int w = 0; w < warp; ++w) row += in_warp[w][mine];
         }
-        own_row[i] = row;
+        own_row[tid] = row;
     }
     __syncthreads();
     if (blockIdx.y == 0) {
-        for (int i = tid; i < own; i += kDispThreads) {
+        if (tid < own) {
+            const int i = tid;
             const int t = i / topk, first = t * topk, e = own_e[i];
             int rank = 0;                                          // place in ascending expert order
             for (int j = first; j < first + topk; ++j) rank += own_e[j] < e || (own_e[j] == e && j < i);
@@ -228,8 +233,8 @@ __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const Dispat
 //   tok [P]            : token of the pair placed at each row (pairs of other ranks' experts follow seg[n])
 //   pair_row [P]       : scratch; row given to pair p, or -1 when its expert is not local
 //   pos_sorted, w_sorted [T, topk]: per token, rows and routing weights in ascending expert order
-// The order of an expert's rows is whatever the atomics give; every row's result depends on that row alone, so
-// the outputs do not depend on it.
+// The order of an expert's rows is whatever the atomics give; with whole tiles (dsv3_fp8_gemm_grouped) every row's result
+// depends on that row alone, so the outputs do not depend on it.
 constexpr int kRouteThreads = 1024;
 constexpr int kRouteMaxExperts = 256;
 constexpr int kRouteMaxTopk = 32;
@@ -500,8 +505,7 @@ int dsv3_moe_dispatch(const void* x, int64_t T, int64_t dim, const int64_t* indi
     p.tpc = static_cast<int>(tpc);
     const int64_t gx = (T + tpc - 1) / tpc;
     int gy = 1;                                                    // few tokens: share each token's blocks among CTAs
-    if (tpc * topk <= kDispOrdered)
-        while (gy < 8 && gx * gy * 2 <= wave && gy * 2 * 32 <= dim / 128) gy *= 2;
+    while (gy < 8 && gx * gy * 2 <= wave && gy * 2 * 32 <= dim / 128) gy *= 2;
     DSV3_CUDA_TRY(launch_dependent(moe_dispatch_kernel, dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), dim3(kDispThreads), 0,
                                    static_cast<cudaStream_t>(stream), p));
     return DSV3_OK;

@@ -90,3 +90,33 @@ def test_whole_tiles_equal_the_operators_bit_for_bit(counts, policy):
     want = layer.operators(got[0], got[1], got[3], got[4])
     for a, b in zip(got, want):
         assert torch.equal(a.view(torch.uint8) if a.element_size() == 1 else a, b.view(torch.uint8) if b.element_size() == 1 else b)
+
+
+# fewer and more than one pair per thread of a warp, one CTA's limit of pairs, more tokens than CTAs, few SMs; repeated experts
+@pytest.mark.parametrize("T,topk,E,start,n,sms", [(1, 8, 256, 0, 256, 0), (40, 8, 16, 4, 8, 0), (1400, 8, 64, 0, 64, 0), (300, 32, 40, 8, 32, 2),
+                                                   (4099, 6, 256, 128, 128, 0), (513, 2, 4, 0, 4, 4)])
+def test_rows_of_an_expert_are_in_the_order_of_the_pairs(T, topk, E, start, n, sms):
+    import dsv3_b200
+    from dsv3_b200 import _lib
+    lib, dim = _lib.lib, 128
+    g = torch.Generator(device="cuda").manual_seed(T)
+    x = torch.randn(T, dim, generator=g, device="cuda", dtype=torch.float32).bfloat16()
+    idx = torch.randint(0, E, (T, topk), generator=g, device="cuda")
+    w = torch.rand(T, topk, generator=g, device="cuda", dtype=torch.float32)
+    P, i32, p, i64 = T * topk, dict(dtype=torch.int32, device="cuda"), (lambda t: ctypes.c_void_p(t.data_ptr())), ctypes.c_int64
+    seg, pos, ws = torch.empty(n + 1, **i32), torch.empty(T, topk, **i32), torch.empty(T, topk, device="cuda")
+    xq, xs = torch.empty(T, dim, dtype=torch.uint8, device="cuda"), torch.empty(T, 1, dtype=torch.float32, device="cuda")
+    xr, xst = torch.empty(P, dim, dtype=torch.uint8, device="cuda"), torch.empty(1, P, dtype=torch.float32, device="cuda")
+    dsv3_b200.set_num_sms(sms)
+    try:
+        _lib.check(lib.dsv3_moe_dispatch(p(x), i64(T), i64(dim), p(idx), p(w), 0, topk, start, n, 0, p(seg), p(pos), p(ws), p(xq), p(xs), p(xr),
+                                         p(xst), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    finally:
+        dsv3_b200.set_num_sms(0)
+    key = (idx - start).flatten()
+    local = (key >= 0) & (key < n)
+    order = torch.where(local, key, n).sort(stable=True).indices           # pairs by expert, then as they come
+    row = torch.empty_like(order)
+    row[order] = torch.arange(P, device="cuda")
+    row = torch.where(local, row, -1).view(T, topk)
+    assert torch.equal(pos.long(), row.gather(1, idx.sort(dim=1, stable=True).indices))
