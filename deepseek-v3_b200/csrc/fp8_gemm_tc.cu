@@ -1145,9 +1145,11 @@ int launch_fp8_gemm_tc(const void* a, const float* a_s, const void* b, const flo
 }
 
 // ---------------------------------------------------------------------------------------------
-// Self-test of the bounded wait the tcgen05 kernels are built on: one thread waits, with the given limit, for
-// an mbarrier phase that nothing will ever complete.  The wait runs out, records (kind 9, counter, CTA) in the
-// status words and the kernel returns normally: nothing traps, faults or spins without a bound.
+// Self-test of what the tcgen05 kernels do when a wait gives up: one warp waits, with the given limit, for an mbarrier
+// phase that nothing will ever complete, while seven others already stand in the barrier that the eight share.  The wait
+// runs out, records (kind 9, counter, CTA) in the status words, and the warp takes part in the barrier with what it knows;
+// every warp turns away and the kernel returns normally: nothing traps, faults or spins without a bound.  (A warp that
+// the barrier told otherwise records kind 10.)
 // ---------------------------------------------------------------------------------------------
 namespace {
 
@@ -1158,8 +1160,11 @@ __global__ void bounded_wait_selftest_kernel(unsigned int* status, uint64_t limi
         ctl.abort_flag = 0;
         mbar_init(smem_u32(&bar), 1);
         mbar_fence_init();
-        (void)bounded_wait_ns(smem_u32(&bar), 0, &ctl, status, 9, 0, limit_ns);
     }
+    __syncthreads();
+    bool ok = true;
+    if (threadIdx.x < 32) ok = __all_sync(0xffffffffu, bounded_wait_ns(smem_u32(&bar), 0, &ctl, status, 9, 0, limit_ns));
+    if (barrier_all<256>(1, ok)) status[1] = 10;
 }
 
 }  // namespace
@@ -1167,7 +1172,7 @@ __global__ void bounded_wait_selftest_kernel(unsigned int* status, uint64_t limi
 int launch_bounded_wait_selftest(uint64_t limit_ns, cudaStream_t stream) {
     unsigned int* status = status_device_ptr();
     if (!status) return DSV3_ERR_CUDA;
-    bounded_wait_selftest_kernel<<<1, 32, 0, stream>>>(status, limit_ns);
+    bounded_wait_selftest_kernel<<<1, 256, 0, stream>>>(status, limit_ns);
     DSV3_CUDA_TRY(cudaGetLastError());
     return DSV3_OK;
 }

@@ -20,7 +20,8 @@
 // chunk product leaves TMEM and is folded into fp32 registers with its two scales (kernel.py:162).
 //
 // Every mbarrier wait is bounded (tc_wait.cuh); producers wait for the last commits onto their barriers before the
-// CTA leaves.
+// CTA leaves.  A promotion warp whose wait gave up goes on through the tiles without working on them, to take part in the
+// barriers where other warps may be waiting for it (barrier_all).
 #include <cuda.h>
 
 #include <cstring>
@@ -310,9 +311,11 @@ __device__ __forceinline__ void produce(const StreamParams& p, const Plan& pl, c
         ok = __all_sync(0xffffffffu, bounded_wait(bar0 + 8u * (NS + d % NS), (d / NS) & 1u, ctl, p.status, 1, d));
 }
 
-// Ticket of a partial tile: parks are done; returns whether this CTA holds the tile's last ticket (promotion threads).
-__device__ __forceinline__ bool last_part(const StreamParams& p, Control* ctl, int first, int last) {
-    asm volatile("bar.sync 1, 256;" ::: "memory");
+// Ticket of a partial tile whose parts are parked (promotion threads): whether this CTA holds the tile's last ticket.
+// ok comes in as "this warp's waits have succeeded" and goes out as "every warp's have"; without that no ticket is taken.
+__device__ __forceinline__ bool last_part(const StreamParams& p, Control* ctl, int first, int last, bool& ok) {
+    ok = barrier_all<256>(1, ok);
+    if (!ok) return false;
     if (threadIdx.x == kFirstPromoWarp * 32) {
         int tk;
         // releases the parked tile (cumulative over the barrier) and acquires the other parts
@@ -530,7 +533,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 }
             }
         };
-        while (ok && wk.next(s)) {
+        while (wk.next(s)) {
             const Side& d = p.side[kBoth ? s.side : kGroups];
             // pieces of this thread that hold a token of the tile
             const int np = s.ntok <= col0 ? 0 : min(NP, (s.ntok - col0 + 2 * PW - 1) / (2 * PW));
@@ -542,7 +545,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                     for (int j = 0; j < PW / 2; ++j) acc[b][i][j] = make_float2(0.0f, 0.0f);
             int in_tab = 0;                         // chunk within the slot of the scale ring
             const int n_ch = s.c1 - s.c0;
-            for (int k = 0; k < n_ch; ++k, ++g) {
+            for (int k = 0; ok && k < n_ch; ++k, ++g) {
                 const int sl = t & 1;
                 if (in_tab == 0) {
                     ok = __all_sync(0xffffffffu, bounded_wait_lean(sfull_bar(sl), (t >> 1) & 1u, ctl, p.status, 8, t));
@@ -587,7 +590,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                     ++t;
                 }
             }
-            if (!ok) break;
+            if (!kSplit && !kSwiglu && !ok) break; // (no barrier ahead)
 
             if (kSplit && n_ch < kc_of(s)) {
                 // part of a tile: park the pieces that hold tokens, take a ticket; the last part of the tile adds all
@@ -597,7 +600,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 constexpr int kTileVec = 2 * BN / 4 * kPRows;             // float4 per parked tile: [2 blocks][BN / 4][128 rows]
                 float4* base = reinterpret_cast<float4*>(p.partials) + (col0 / 4) * kPRows + row;
                 auto part = [&](int c) { return base + (static_cast<int64_t>(c) * 2 + (pl.begin(c) >= s.ut ? 0 : 1)) * kTileVec; };
-                {
+                if (ok) {
                     float4* dst = part(cta);
 #pragma unroll
                     for (int i = 0; i < NP; ++i)
@@ -609,7 +612,9 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                                     __stcg(dst + (b * (BN / 4) + i * (PW / 2) + j) * kPRows,
                                            make_float4(acc[b][i][2 * j].x, acc[b][i][2 * j].y, acc[b][i][2 * j + 1].x, acc[b][i][2 * j + 1].y));
                 }
-                if (!last_part(p, ctl, first, last)) continue;
+                const bool mine = last_part(p, ctl, first, last, ok);
+                if (!ok) break;                    // all eight warps
+                if (!mine) continue;
 #pragma unroll
                 for (int i = 0; i < NP; ++i) {
                     if (i >= np) continue;
@@ -644,6 +649,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 }
             }
             if constexpr (!kSwiglu) {
+                if (!ok) continue;
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     const int64_t n = static_cast<int64_t>(2 * s.p + b) * kPRows + row;
@@ -677,7 +683,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 // first token of group q
                 auto token = [&](int q) { return PW == 8 ? col0 : col0 + 2 * PW * (q >> 1) + 8 * (q & 1); };
 #pragma unroll 1
-                for (int q = 0; q < NG; ++q) {
+                for (int q = 0; ok && q < NG; ++q) {
                     const int tk = token(q), rem = s.ntok - tk;
                     uint32_t h[4] = {0u, 0u, 0u, 0u};
                     if (rem > 0) {
@@ -704,7 +710,11 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
 #pragma unroll
                     for (int e = 0; e < 4; ++e) h1[4 * NG - 4 + e] = h[e];
                 }
-                asm volatile("bar.sync %0, 128;" ::"r"(2 + grp) : "memory");
+                ok = barrier_all<128>(2 + grp, ok);
+                if (!ok) {                         // this group's four warps; the barrier of a partial tile counts them too
+                    if constexpr (kSplit) continue;
+                    else break;
+                }
                 {
                     const int gt = threadIdx.x & 127;
                     const int tk = col0 + 2 * PW * (gt / PW) + gt % PW;
@@ -889,7 +899,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
         };
         bool more = wk.next(ahead);
         if (more) scales_of(ahead);
-        while (ok && more) {
+        while (more) {
             s = ahead;
             const Side& d = p.side[kBoth ? s.side : kGroups];
             const int blk = kSwiglu ? s.p : 2 * s.p + grp;
@@ -924,7 +934,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
                     fold(sc, 32);
                 }
             }
-            if (!ok) break;
+            if (!kSwiglu && !ok) break;            // (no barrier ahead)
             more = wk.next(ahead);
             if (more) scales_of(ahead);
 
@@ -980,7 +990,8 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
                     v[4 * c + 2] = give ? lo.z : hi.z;
                     v[4 * c + 3] = give ? lo.w : hi.w;
                 }
-                asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
+                ok = barrier_all<64>(2 + quarter, ok);
+                if (!ok) break;                    // both warps of these rows
                 float m = 0.0f;
                 // Rolled loops over a register file that turns by one group per trip: unrolled, this epilogue was longer
                 // than the instruction cache holds and cost 8000-14000 cycles per tile.  (Rows beyond the tile's hold

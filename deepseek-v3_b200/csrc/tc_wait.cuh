@@ -69,6 +69,26 @@ __device__ __forceinline__ bool bounded_wait_lean(uint32_t bar, uint32_t parity,
     return false;
 }
 
+// A named barrier of kThreads threads (whole warps) that also tells whether `ok` held in all of them.  The promotion warps
+// meet at such a barrier first wherever they are about to rely on one another: a warp whose bounded wait gave up takes part
+// with ok = false and everybody turns away together, so that no warp is left behind in a barrier that another will not
+// reach.  Between it and the last barrier of the same hand-over there is no wait that could give up.
+template <int kThreads>
+__device__ __forceinline__ bool barrier_all(uint32_t id, bool ok) {
+    uint32_t all;
+    asm volatile(
+        "{\n"
+        ".reg .pred mine, every;\n"
+        "setp.ne.u32 mine, %1, 0;\n"
+        "barrier.cta.red.and.aligned.pred every, %2, %3, mine;\n"
+        "selp.u32 %0, 1, 0, every;\n"
+        "}\n"
+        : "=r"(all)
+        : "r"(ok ? 1u : 0u), "r"(id), "n"(kThreads)
+        : "memory");
+    return all != 0u;
+}
+
 // bounded_wait preceded by the result of an earlier probe of the same barrier and parity.
 //
 // A parity probe (mbarrier.test_wait.parity P) answers "has the phase with parity P completed?", which is

@@ -296,8 +296,9 @@ int dsv3_weight_quant(const void* w, int64_t N, int64_t K, void* q, float* s, ds
 int dsv3_check_device_status(dsv3_stream_t stream, uint32_t detail[4]);
 
 /*
- * Self-test of the bounded device-side wait: enqueues a one-thread kernel that waits for an mbarrier phase nothing
- * completes; after limit_ns (1 ns .. 1 s) the wait gives up and records kind 9 in the status words, so the next
+ * Self-test of the bounded device-side wait: enqueues a one-block kernel in which one warp waits for an mbarrier phase
+ * nothing completes while seven others stand in a barrier with it; after limit_ns (1 ns .. 1 s) the wait gives up and
+ * records kind 9 in the status words, all warps leave the barrier knowing of it, and the next
  * dsv3_check_device_status returns DSV3_ERR_DEVICE_TIMEOUT.  The kernel returns normally; nothing faults or traps.
  * Callers of the GEMM entry points should poll dsv3_check_device_status at step boundaries: after a give-up the
  * affected result is incomplete.
