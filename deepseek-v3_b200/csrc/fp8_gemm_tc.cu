@@ -387,7 +387,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
             }
         };
 
-        for (int item = blockIdx.x; ok && item < p.num_items; item += gridDim.x) {
+        for (int item = blockIdx.x; item < p.num_items; item += gridDim.x) {
             const Item it = decode_item<BN, kSwap>(item, p);
             const uint32_t item_cur = item_no++;
             float2 acc[CPT / 2];
@@ -413,10 +413,11 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
             // chunk loop reads them with a few broadcast vector loads.  (The host plan splits K so that an
             // item never has more chunks than the table holds.)
             if constexpr (kSwap) {
-                {
-                    bool mine = bounded_wait(tab_free_bar, (item_cur & 1u) ^ 1u, ctl, p.status, 7, item_cur);
+                if (ok) {
+                    const bool mine = bounded_wait(tab_free_bar, (item_cur & 1u) ^ 1u, ctl, p.status, 7, item_cur);
                     ok = __all_sync(0xffffffffu, mine);
-                    if (!ok) break;
+                }
+                if (ok) {
                     const int tid = threadIdx.x - kFirstPromoWarp * 32;
                     for (int idx = tid; idx < n_ch * BN; idx += kPromoThreads) {
                         const int chl = idx / BN, col = idx - chl * BN;
@@ -424,9 +425,8 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                         sc_tab[idx] = __ldg(as_ptr + m * kc + it.c0 + chl) * __ldg(bs_ptr + it.c0 + chl);
                     }
                     mbar_arrive(tab_ready_bar);
-                    mine = bounded_wait(tab_ready_bar, item_cur & 1u, ctl, p.status, 8, item_cur);
+                    const bool mine = bounded_wait(tab_ready_bar, item_cur & 1u, ctl, p.status, 8, item_cur);
                     ok = __all_sync(0xffffffffu, mine);
-                    if (!ok) break;
                 }
             }
             const int n_units = (n_ch + UC - 1) / UC;
@@ -456,7 +456,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
             // the TMEM load of the next step is in flight.
             uint32_t va[kBatched ? 1 : HC], vb[kBatched ? 1 : HC];
             if constexpr (kBatched) {
-                if (n_mine > 0) {   // first unit of the item: wait and start its first load here
+                if (ok && n_mine > 0) {   // first unit of the item: wait and start its first load here
                     const uint32_t gu = unit_g(0);
                     const bool mine = wait_probed(probe, tfull_bar(gu % NT), (gu / NT) & 1u, ctl, p.status, 4, gu);
                     ok = __all_sync(0xffffffffu, mine);
@@ -466,7 +466,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                     }
                 }
             } else {
-                if (n_mine > 0) ok = issue_load(unit_g(0), 0, 0, va);
+                if (ok && n_mine > 0) ok = issue_load(unit_g(0), 0, 0, va);
             }
             if constexpr (!kSwap) {
                 static_assert(UC == 2, "token-major tiles pair two chunks per unit");
@@ -552,9 +552,11 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                 }
             }
             g += n_units;
-            if (!ok) break;
+            // A warp whose wait gave up goes on through the items without working on them, to take part in the barriers
+            // where other warps may be waiting for it (barrier_all); the cluster's barriers come behind the loop.
+            if (!ok && (p.cluster || (p.splits == 1 && (kSwap || !p.tma_store)))) break;
             if constexpr (kSwap) {
-                mbar_arrive(tab_free_bar);   // this thread is done reading the scale table
+                if (ok) mbar_arrive(tab_free_bar);   // this thread is done reading the scale table
             }
 
             float* accf = reinterpret_cast<float*>(acc);
@@ -645,7 +647,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                 const int64_t split_stride = static_cast<int64_t>(p.tiles_p) * p.tiles_q * kTileVec;
                 float4* tile_part = reinterpret_cast<float4*>(p.partials) + static_cast<int64_t>(it.tile) * kTileVec +
                                     (col0 / 4) * kPRows + row;
-                {
+                if (ok) {
                     float4* dst = tile_part + it.split * split_stride;
 #pragma unroll
                     for (int j = 0; j < CPT / 4; ++j)
@@ -655,7 +657,8 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                 // is cumulative.  The ticket slot alternates between items, so the next item's ticket cannot
                 // overwrite this one before every thread has read it (a barrier of the next item lies between).
                 const int slot = static_cast<int>(item_cur & 1u);
-                promo_barrier<kWriters>();
+                ok = barrier_all<kWriters>(1, ok);
+                if (!ok) break;                  // all eight warps
                 if (threadIdx.x == kFirstPromoWarp * 32) {
                     // one acquire-release atomic: releases the partial tiles (cumulative over the barrier above) and
                     // acquires the other splits' tiles for the reads below
@@ -706,7 +709,8 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                         uint8_t* sbuf = store_buf + half * (kPRows * 128);
                         const bool issuer = ((threadIdx.x & 127) == 0);
                         if (issuer) bulk_wait_group_read0();
-                        asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
+                        ok = barrier_all<128>(2 + half, ok);
+                        if (!ok) break;          // this half's four warps (unsplit: no barrier counts all eight)
 #pragma unroll
                         for (int cidx = 0; cidx < CPT / 8; ++cidx) {
                             const int j = cidx * 8;

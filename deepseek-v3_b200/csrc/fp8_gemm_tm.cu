@@ -292,15 +292,19 @@ fp8_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         // swizzle: 16-byte slot c of row r sits at slot c ^ (r & 7), which also keeps the vector stores free of
         // bank conflicts) and one thread hands it to the TMA, which clips rows beyond M and columns beyond N.
         // The store of the previous tile is only known to have read the buffer once its issuer has waited for
-        // it, hence the first barrier.  tp = token tile of this CTA.
-        auto write_tile = [&](int tp, int tq) {
-            if (static_cast<int64_t>(tp) * kPRows >= p.M) return;     // the odd half of the last pair: nothing to store
+        // it, hence the first barrier, which every tile passes and which also says whether a wait of any of the four
+        // warps gave up (false: they all turn away).  tp = token tile of this CTA.
+        const bool issuer = ((threadIdx.x & 127) == 0);
+        auto write_tile = [&](int tp, int tq, bool well) -> bool {
+            if (p.tma_store) {
+                if (issuer) bulk_wait_group_read0();
+                well = barrier_all<128>(2 + half, well);
+            }
+            if (!well) return false;
+            if (static_cast<int64_t>(tp) * kPRows >= p.M) return true;     // the odd half of the last pair: nothing to store
             const float* accf = reinterpret_cast<const float*>(acc);
             if (p.tma_store) {
                 uint8_t* sbuf = store_buf + half * (kPRows * 128);
-                const bool issuer = ((threadIdx.x & 127) == 0);
-                if (issuer) bulk_wait_group_read0();
-                asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
 #pragma unroll
                 for (int cidx = 0; cidx < 8; ++cidx) {
                     const int j = cidx * 8;
@@ -325,6 +329,7 @@ fp8_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                         if (n0 + j < N) crow[n0 + j] = __float2bfloat16_rn(accf[j]);
                 }
             }
+            return true;
         };
 
         bool ok = true;
@@ -332,6 +337,7 @@ fp8_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         uint32_t probe = 0;        // result of test_wait on the tfull[] barrier that is waited for next
         bool pend = false;         // vb holds a chunk product that is not folded into acc yet
         float pend_sc = 0.0f;
+        bool gone = false;         // turned away in a barrier, because a wait of another warp gave up
         bool epi = false;          // acc (after the pending fold) is the finished previous tile, not written yet
 
         int tile = pair;
@@ -363,7 +369,7 @@ fp8_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                         if (pend) fold(vb, pend_sc);
                         pend = false;
                         const Tile prev = decode_tile(tile - n_pairs, p);
-                        write_tile(2 * prev.pp + static_cast<int>(rank), prev.q);
+                        if (!write_tile(2 * prev.pp + static_cast<int>(rank), prev.q, true)) { gone = true; break; }
 #pragma unroll
                         for (int j = 0; j < 32; ++j) acc[j] = make_float2(0.0f, 0.0f);
                         epi = false;
@@ -396,17 +402,15 @@ fp8_gemm_tm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                     pend = (u * kUC + 1 < kc);
                     pend_sc = sa1;
                 }
-                if (!ok) break;
+                if (!ok || gone) break;
                 epi = true;
                 if (tile + n_pairs >= p.num_tiles) break;
                 tile += n_pairs;
             }
-            if (ok) {     // `tile` is the last tile of this pair
+            if (!gone) {     // `tile` is the last tile of this pair, or the one in which a wait gave up
                 if (pend) fold(vb, pend_sc);
-                if (epi) {
-                    const Tile last = decode_tile(tile, p);
-                    write_tile(2 * last.pp + static_cast<int>(rank), last.q);
-                }
+                const Tile last = decode_tile(tile, p);
+                write_tile(2 * last.pp + static_cast<int>(rank), last.q, ok);
             }
         }
     }

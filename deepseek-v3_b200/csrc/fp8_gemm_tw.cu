@@ -276,19 +276,26 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         // swizzle: 16-byte slot c of row r sits at slot c ^ (r & 7), which also keeps the vector stores free of
         // bank conflicts) and one thread hands them to the TMA, which clips rows beyond M and columns beyond N.
         // The stores of the previous tile are only known to have read the buffer once their issuer has waited for
-        // them, hence the first barrier.  tp = token tile of this CTA.
-        auto write_tile = [&](int tp, int tq) {
-            if (static_cast<int64_t>(tp) * kPRows >= p.M) return;     // the odd half of the last pair: nothing to store
+        // them, hence the first barrier, which every tile passes and which also says whether a wait of any of the four
+        // warps gave up (false: they all turn away).  tp = token tile of this CTA.
+        const bool issuer = (((threadIdx.x - kFirstPromoWarp * 32) & 127) == 0);
+        auto write_tile = [&](int tp, int tq) -> bool {
+            if (p.tma_store) {
+                if (issuer) bulk_wait_group_read0();
+                if (!barrier_all<128>(2 + half, true)) return false;
+            }
+            if (static_cast<int64_t>(tp) * kPRows >= p.M) return true;     // the odd half of the last pair: nothing to store
             const int64_t n0 = static_cast<int64_t>(tq) * kBN + col0;
-            if (n0 >= p.N) return;                                    // the tile's right half lies beyond N
+            if (n0 >= p.N) return true;                                    // the tile's right half lies beyond N
             if (p.tma_store) {
                 constexpr int kBoxes = 2 / kStorePasses;               // boxes per warp group and pass
                 uint8_t* sbuf = store_buf + half * (kBoxes * kPRows * 128);
-                const bool issuer = (((threadIdx.x - kFirstPromoWarp * 32) & 127) == 0);
 #pragma unroll
                 for (int pass = 0; pass < kStorePasses; ++pass) {
-                    if (issuer) bulk_wait_group_read0();
-                    asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
+                    if (pass > 0) {
+                        if (issuer) bulk_wait_group_read0();
+                        asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
+                    }
 #pragma unroll
                     for (int c8 = 0; c8 < 8 * kBoxes; ++c8) {      // 16-byte slot of the thread's columns: box cc / 8, slot cc % 8
                         const int cc = pass * 8 * kBoxes + c8;
@@ -319,6 +326,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                     }
                 }
             }
+            return true;
         };
 
         // Scale rows of a tile for this thread, as element offsets: a_s of its token (clamped at the edge), b_s of
@@ -384,7 +392,10 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                         fold(v[1], sc, 3);
                     }
                 }
-                if (!ok) break;
+                if (!ok) {
+                    if (p.tma_store) barrier_all<128>(2 + half, false);
+                    break;
+                }
                 // the next tile's first scales are requested before this tile is written, so that their latency
                 // (and the tile decode) hides under the epilogue while the issuer already fills both TMEM slots
                 const int next = tile + n_pairs;
@@ -394,8 +405,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                     nt = decode_tile(next, p);
                     first_scales(nt);
                 }
-                write_tile(2 * cur.pp + static_cast<int>(rank), cur.q);
-                if (!more) break;
+                if (!write_tile(2 * cur.pp + static_cast<int>(rank), cur.q) || !more) break;
                 tile = next;
                 cur = nt;
             }
