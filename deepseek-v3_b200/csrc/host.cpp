@@ -326,7 +326,8 @@ std::pair<at::Tensor, at::Tensor> quantise_remembered(const at::Tensor& x, int64
 // Device tables of the local experts' projections and what they depend on.  The tables hold addresses, so before every
 // pass the host must know that the experts are still the ones they were built from.  Looking every weight up through
 // its module costs 0.3 us each (230 us for 256 experts); instead the dictionaries the look-ups went through are watched
-// for changes, and only the weights' storage addresses are compared (`param.data = ...` changes no dictionary).
+// for changes, and only the storage addresses of the weights and scales are compared (`param.data = ...` changes no
+// dictionary).  They are kept as Python objects: an object's tensor may be exchanged (torch.utils.swap_tensors).
 uint64_t g_dict_changes = 1;         // bumped whenever a watched dictionary changes
 int g_watcher = -1;
 
@@ -349,9 +350,10 @@ struct Experts {
     std::vector<PyObject*> members;  // its members [start, start + n)
     std::vector<LookUp> lookups;
     uint64_t seen = 0;               // g_dict_changes when the look-ups were last verified
-    std::vector<std::pair<at::Tensor, const void*>> weights;
+    std::vector<std::pair<PyObject*, const void*>> tensors;     // weights and scales with the addresses in the tables
     ~Experts() {
         Py_XDECREF(list);
+        for (auto& t : tensors) Py_DECREF(t.first);
         for (PyObject* m : members) Py_DECREF(m);
         for (LookUp& l : lookups) {
             Py_DECREF(l.dict);
@@ -369,8 +371,8 @@ struct Experts {
                 if (PyDict_GetItemWithError(l.dict, l.key) != l.value) return false;
             seen = g_dict_changes;
         }
-        for (const auto& w : weights)
-            if (w.first.const_data_ptr() != w.second) return false;
+        for (const auto& t : tensors)
+            if (THPVariable_Unpack(t.first).const_data_ptr() != t.second) return false;
         return true;
     }
 };
@@ -601,7 +603,8 @@ PyObject* py_quantise_remembered(PyObject*, PyObject* const* args, Py_ssize_t n)
     });
 }
 
-// (n, start, dim, inter, scale_fmt, table1, table3, table2, list or None, members, look-ups [(dict, key, value)], weights)
+// (n, start, dim, inter, scale_fmt, table1, table3, table2, list or None, members, look-ups [(dict, key, value)], weights and
+// scales)
 PyObject* py_experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         want_args(n, 12);
@@ -617,7 +620,7 @@ PyObject* py_experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
         e->table2 = tensor_arg(args[7]);
         if (PyList_Check(args[8])) e->list = Py_NewRef(args[8]);
         if (!PyList_Check(args[9]) || !PyList_Check(args[10]) || !PyList_Check(args[11]) || PyList_GET_SIZE(args[9]) != e->n)
-            raise(PyExc_TypeError, "members, look-ups and weights are lists");
+            raise(PyExc_TypeError, "members, look-ups and tensors are lists");
         for (Py_ssize_t i = 0; i < PyList_GET_SIZE(args[9]); ++i) e->members.push_back(Py_NewRef(PyList_GET_ITEM(args[9], i)));
         for (Py_ssize_t i = 0; i < PyList_GET_SIZE(args[10]); ++i) {
             PyObject *d, *k, *v;
@@ -628,8 +631,9 @@ PyObject* py_experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
 #endif
         }
         for (Py_ssize_t i = 0; i < PyList_GET_SIZE(args[11]); ++i) {
-            const at::Tensor& w = tensor_arg(PyList_GET_ITEM(args[11], i));
-            e->weights.emplace_back(w, w.const_data_ptr());
+            PyObject* t = PyList_GET_ITEM(args[11], i);
+            const void* at = tensor_arg(t).const_data_ptr();
+            e->tensors.emplace_back(Py_NewRef(t), at);
         }
         return PyCapsule_New(e.release(), kExpertsName, free_experts);
     });
@@ -725,7 +729,7 @@ PyMethodDef methods[] = {
     {"quantise_remembered", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_quantise_remembered)), METH_FASTCALL,
      "(x, block_size, scale_fmt, assume_no_inplace)"},
     {"experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_experts)), METH_FASTCALL,
-     "(n, start, dim, inter, scale_fmt, table1, table3, table2, list, members, lookups, weights)"},
+     "(n, start, dim, inter, scale_fmt, table1, table3, table2, list, members, lookups, tensors)"},
     {"experts_current", py_experts_current, METH_O, "whether the experts are still those the tables were built from"},
     {"run_experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_run_experts)), METH_FASTCALL,
      "(experts, x, weights, indices, n_routed, assume_no_inplace, shared)"},

@@ -30,14 +30,17 @@ SHARED_INLINE_MAX_ROWS = 512
 
 
 def _look_up(obj, name):
-    """The attribute and the dictionary it lives in (None where it lives elsewhere)."""
+    """The attribute and the dictionary entries it was found through (one None where it lives elsewhere)."""
     value = getattr(obj, name)
     own = getattr(obj, "__dict__", None)
-    if own is not None:
-        for d in (own, own.get("_parameters"), own.get("_modules"), own.get("_buffers")):
+    if type(own) is dict:
+        if own.get(name) is value:
+            return value, [(own, name, value)]
+        for kind in ("_parameters", "_modules", "_buffers"):
+            d = own.get(kind)
             if type(d) is dict and d.get(name) is value:
-                return value, (d, name, value)
-    return value, None
+                return value, [(own, kind, d), (d, name, value)]
+    return value, [None]
 
 
 class GroupedExperts:
@@ -52,19 +55,23 @@ class GroupedExperts:
         self.inter = e0.w1.weight.size(0)
         self.scale_fmt = getattr(e0.w1, "scale_fmt", None)
         self.device = e0.w1.weight.device
-        # every look-up from the container to a weight's storage that the tables depend on
-        found, weights, by_name = [], [], {"w1": [], "w3": [], "w2": []}
+        # every look-up from the container to a weight's and its scales' storage that the tables depend on
+        found, weights, scales, by_name = [], [], [], {"w1": [], "w3": [], "w2": []}
         if not isinstance(container, list):
             members = getattr(container, "_modules", None)
+            if type(members) is dict:
+                found.append((container.__dict__, "_modules", members))
             found += [(members, str(start + i), e) if type(members) is dict else None for i, e in enumerate(experts)]
         for e in experts:
             for name in by_name:
                 lin, step = _look_up(e, name)
                 w, step2 = _look_up(lin, "weight")
-                found += [step, step2]
+                s, step3 = _look_up(w, "scale")
+                found += step + step2 + step3
                 weights.append(w)
+                scales.append(s)
                 by_name[name].append(w)
-        self.watched = all(f is not None for f in found)      # otherwise the weights are looked up on every pass
+        self.watched = all(f is not None for f in found)      # otherwise they are looked up on every pass
         tables = {}
         for name, N, K in (("w1", self.inter, self.dim), ("w3", self.inter, self.dim), ("w2", self.dim, self.inter)):
             ws = by_name[name]
@@ -78,18 +85,26 @@ class GroupedExperts:
             with torch.cuda.device(self.device):
                 _lib.check(lib.dsv3_group_table_build(table.data_ptr(), wp, sp, self.n, N, K, _stream()))
             tables[name] = table
-        self._keep = (experts, [w.scale for w in weights])    # the tables point into these
-        self.signature = tuple(w.data_ptr() for w in weights)
+        self._keep = (experts, scales)                        # the tables point into these
+        self.signature = self._addresses(container)
         self.handle = host.experts(self.n, start, self.dim, self.inter, self.scale_fmt, tables["w1"], tables["w3"], tables["w2"],
                                    container if isinstance(container, list) else None, list(experts),
-                                   found if self.watched else [], weights)
+                                   found if self.watched else [], weights + scales)
+
+    def _addresses(self, container):
+        """Storage of every weight and its scales, looked up from the container."""
+        found = []
+        for i in range(self.start, self.start + self.n):
+            for name in ("w1", "w3", "w2"):
+                w = getattr(container[i], name).weight
+                found += [w.data_ptr(), w.scale.data_ptr()]
+        return found
 
     def current(self, moe) -> bool:
         """Whether ``moe``'s local experts are still the ones the tables were built from."""
         if moe.experts is not self.container or moe.experts_start_idx != self.start or moe.experts_end_idx != self.start + self.n:
             return False
-        if not self.watched and self.signature != tuple(getattr(moe.experts[i], n).weight.data_ptr()
-                                                        for i in range(self.start, self.start + self.n) for n in ("w1", "w3", "w2")):
+        if not self.watched and self.signature != self._addresses(self.container):
             return False
         return host.experts_current(self.handle)
 
