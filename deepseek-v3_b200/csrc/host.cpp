@@ -401,13 +401,13 @@ struct Shared {
     at::Tensor w[3], s[3];
 };
 
-std::unique_ptr<Routed> run_experts(Experts& e, const at::Tensor& x_in, const at::Tensor& weights_in, const at::Tensor& indices_in,
+std::unique_ptr<Routed> run_experts(Experts& e, const at::Tensor& x, const at::Tensor& weights_in, const at::Tensor& indices_in,
                                     int64_t n_routed, bool assume_no_inplace, const Shared* sh) {
     if (indices_in.dim() != 2 || weights_in.sizes() != indices_in.sizes())
         raise(PyExc_ValueError, "routing weights and indices must both be [tokens, top-k]");
-    const c10::Device dev = require_cuda(x_in, weights_in, indices_in, e.table1);
-    if (x_in.scalar_type() != at::kBFloat16) raise(PyExc_NotImplementedError, "the expert layer takes bfloat16 activations");
-    const at::Tensor x = x_in.is_contiguous() ? x_in : x_in.contiguous();
+    const c10::Device dev = require_cuda(x, weights_in, indices_in, e.table1);
+    require(x.is_contiguous(), "Input tensor must be contiguous");     // as act_quant
+    if (x.scalar_type() != at::kBFloat16) raise(PyExc_NotImplementedError, "the expert layer takes bfloat16 activations");
     at::Tensor indices = indices_in.scalar_type() == at::kLong ? indices_in : indices_in.to(at::kLong);
     at::Tensor weights = (weights_in.scalar_type() == at::kBFloat16 || weights_in.scalar_type() == at::kFloat) ? weights_in : weights_in.to(at::kFloat);
     if (!indices.is_contiguous()) indices = indices.contiguous();
@@ -468,7 +468,7 @@ std::unique_ptr<Routed> run_experts(Experts& e, const at::Tensor& x_in, const at
         if (rc == DSV3_OK) rc = dsv3_fp8_gemm_rows(t2, e.n, base + o_hq, hs_t, seg, P, hint, dim, inter, base + o_o, sh ? &down : nullptr, ws, ws_bytes, st);
         return rc;
     });
-    if (x_in.is_contiguous()) remember(x_in, 128, e.fmt, assume_no_inplace, xq, xs);
+    remember(x, 128, e.fmt, assume_no_inplace, xq, xs);
     return r;
 }
 
