@@ -156,10 +156,11 @@ def grouped_moe_forward(self, x: torch.Tensor, *, world_size: int = 1, fallback=
             y = host.combine(routed, None)
             dist.all_reduce(y)
             y = y + z
-        elif z.dtype == torch.bfloat16 and z.is_contiguous() and z.size() == x.size():
+        elif (z.dtype == torch.bfloat16 and z.is_contiguous() and z.size() == x.size() and z.data_ptr() % 16 == 0
+              and not z.requires_grad):
             y = host.combine(routed, z)
         else:
-            y = host.combine(routed, None) + z
+            y = host.combine(routed, None) + z          # any tensor that can be added, with its gradient
     return y if flat else y.view(shape)
 
 
