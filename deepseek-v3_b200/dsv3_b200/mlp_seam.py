@@ -13,6 +13,7 @@ all-reduce of a ``RowParallelLinear`` (model.py:263-264) and the bias.
 from __future__ import annotations
 
 import torch
+from torch.nn.modules import module as _nn_module
 
 from .ops import fp8_gemm, swiglu_quant
 
@@ -49,18 +50,26 @@ def _scale_fmt_of(lin):
     return getattr(lin, "scale_fmt", None) if type(lin).__name__ == "Linear" else None
 
 
+def _intercepted(module) -> bool:
+    """Whether a call of the module does more than its class's forward: hooks, or a forward of its own."""
+    return bool(getattr(module, "_forward_hooks", None) or getattr(module, "_forward_pre_hooks", None)
+                or "forward" in getattr(module, "__dict__", ()))
+
+
 def plain_weights(mlp, x: torch.Tensor, scale_fmt):
     """``(w1, w3, w2)`` weights of an MLP that ``mlp_forward`` serves and whose Linears do nothing but the GEMM in
-    ``scale_fmt`` (no bias, no hooks, the installed ``linear``), so that a caller may run them itself; otherwise None."""
+    ``scale_fmt`` (no bias, no hooks, no forward of their own, the installed ``linear``), so that a caller may run them itself; otherwise None."""
     model = getattr(getattr(type(mlp), "forward", None), "_dsv3_model", None)
     if model is None or getattr(model, "world_size", 1) != 1 or not getattr(getattr(model, "linear", None), "_dsv3_linear", False):
+        return None
+    if _intercepted(mlp) or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:
         return None
     w1, w2, w3 = mlp.w1, mlp.w2, mlp.w3
     for lin, names in ((w1, ("Linear", "ColumnParallelLinear")), (w3, ("Linear", "ColumnParallelLinear")), (w2, ("Linear", "RowParallelLinear"))):
         if (type(lin).__name__ not in names or getattr(lin, "bias", None) is not None or _scale_fmt_of(lin) != scale_fmt
-                or getattr(lin, "_forward_hooks", None) or getattr(lin, "_forward_pre_hooks", None)):
+                or _intercepted(lin)):
             return None
-    if getattr(mlp, "_forward_hooks", None) or getattr(mlp, "_forward_pre_hooks", None) or not _fusable(mlp, x, model):
+    if not _fusable(mlp, x, model):
         return None
     return w1.weight, w3.weight, w2.weight
 

@@ -1,6 +1,9 @@
 """Forms of a call of the expert layer at the edge of what it takes."""
+import types
+
 import pytest
 import torch
+import torch.nn.functional as F
 
 from test_gpu_moe import _MoE
 from test_gpu_stream import _bf16_default  # noqa: F401
@@ -38,3 +41,69 @@ def test_any_shared_result_that_can_be_added(form):
     if form == "needs_grad":
         got.sum().backward()
         assert torch.equal(z.grad, torch.ones_like(z))
+
+
+class Linear(torch.nn.Module):
+    """model.py's Linear by name, calling the model's linear()."""
+    scale_fmt = bias = None
+
+    def __init__(self, n, k, seed, model):
+        super().__init__()
+        import dsv3_b200
+        g = torch.Generator(device="cuda").manual_seed(seed)
+        w, s = dsv3_b200.weight_quant((torch.randn(n, k, generator=g, device="cuda", dtype=torch.float32) * 0.02).bfloat16())
+        self.weight = torch.nn.Parameter(w, requires_grad=False)
+        self.weight.scale = s
+        self.model = [model]
+
+    def forward(self, x):
+        return self.model[0].linear(x, self.weight, self.bias, self.scale_fmt)
+
+
+def _host():
+    """A model whose three seams are installed, its expert layer with shared experts, and an input."""
+    import dsv3_b200
+    model = types.SimpleNamespace(gemm_impl="fp8", block_size=128, world_size=1, dist=None)
+
+    class MLP(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.w1, self.w2, self.w3 = Linear(128, 256, 1, model), Linear(256, 128, 2, model), Linear(128, 256, 3, model)
+
+        def forward(self, x):
+            return self.w2(F.silu(self.w1(x)) * self.w3(x))
+
+    model.MLP, model.Expert = MLP, type("Expert", (MLP,), {"forward": MLP.forward})
+    dsv3_b200.install_linear(model)
+    dsv3_b200.install_mlp(model)
+    moe, x = _layer_and_input()
+    moe.shared_experts = MLP()
+    return moe, x
+
+
+def _own_forward(moe, part, seen):
+    module = moe.shared_experts if part == "mlp" else getattr(moe.shared_experts, part)
+    inner = module.forward
+    module.forward = lambda x: (seen.append(1), inner(x))[1]
+
+
+def _global_hook(moe, part, seen):
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda m, i, o: seen.append(1))
+    return handle.remove
+
+
+@pytest.mark.parametrize("intercept,part", [(_own_forward, "mlp"), (_own_forward, "w1"), (_own_forward, "w3"), (_global_hook, None)])
+def test_shared_experts_that_are_intercepted_are_called(intercept, part):
+    import dsv3_b200
+    moe, x = _host()
+    want = dsv3_b200.grouped_moe_forward(moe, x)
+    seen = []
+    undo = intercept(moe, part, seen)
+    try:
+        got = dsv3_b200.grouped_moe_forward(moe, x)
+    finally:
+        if undo:
+            undo()
+    assert seen
+    err, rms = (got.float() - want.float()).abs(), want.float().pow(2).mean().sqrt()
+    assert bool((err <= 2e-2 * (want.float().abs() + rms)).all())         # the bound of test_gpu_moe.py
