@@ -144,7 +144,7 @@ def grouped_moe_forward(self, x: torch.Tensor, *, world_size: int = 1, fallback=
     st = _grouped(self)
     n_routed = getattr(self, "n_routed_experts", 0)
     shared = None
-    if world_size == 1 and x.size(0) <= SHARED_INLINE_MAX_ROWS:
+    if world_size == 1 and 0 < indices.numel() and x.size(0) <= SHARED_INLINE_MAX_ROWS:     # (no pairs: no launch to join)
         shared = plain_weights(self.shared_experts, x, st.scale_fmt)
     routed = st.run(x, weights, indices, n_routed, shared)
     if shared is not None:

@@ -107,3 +107,11 @@ def test_shared_experts_that_are_intercepted_are_called(intercept, part):
     assert seen
     err, rms = (got.float() - want.float()).abs(), want.float().pow(2).mean().sqrt()
     assert bool((err <= 2e-2 * (want.float().abs() + rms)).all())         # the bound of test_gpu_moe.py
+
+
+@pytest.mark.parametrize("rows,topk", [(24, 0), (0, 2)])
+def test_no_pairs_leave_the_shared_result(rows, topk):
+    import dsv3_b200
+    moe, x = _host()
+    moe.gate = lambda x: (torch.empty(x.size(0), topk, device="cuda"), torch.zeros(x.size(0), topk, dtype=torch.int64, device="cuda"))
+    assert torch.equal(dsv3_b200.grouped_moe_forward(moe, x[:rows]), moe.shared_experts(x[:rows]))
