@@ -58,7 +58,8 @@ def _intercepted(module) -> bool:
 
 def plain_weights(mlp, x: torch.Tensor, scale_fmt):
     """``(w1, w3, w2)`` weights of an MLP that ``mlp_forward`` serves and whose Linears do nothing but the GEMM in
-    ``scale_fmt`` (no bias, no hooks, no forward of their own, the installed ``linear``), so that a caller may run them itself; otherwise None."""
+    ``scale_fmt`` (no bias, no hooks, no forward of their own, the installed ``linear``), so that a caller may run them
+    itself; otherwise None."""
     model = getattr(getattr(type(mlp), "forward", None), "_dsv3_model", None)
     if model is None or getattr(model, "world_size", 1) != 1 or not getattr(getattr(model, "linear", None), "_dsv3_linear", False):
         return None

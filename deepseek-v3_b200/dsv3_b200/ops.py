@@ -97,7 +97,7 @@ def weight_dequant(x: torch.Tensor, s: torch.Tensor, block_size: int = 128) -> t
                 return hit[1]
     y = host.weight_dequant(x, s, block_size)
     dequant_stats["launches"] += 1
-    if key is not None:
+    if key is not None and not torch.cuda.is_current_stream_capturing():      # (a recorded launch has computed nothing yet)
         import weakref
         try:
             _dequant_cache[key] = (weakref.ref(x), y)

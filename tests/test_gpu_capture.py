@@ -1,5 +1,5 @@
-"""State that the host extension keeps between calls, across the boundary of a CUDA graph: workspaces and
-remembered quantisations.
+"""State that the host extension keeps between calls, across the boundary of a CUDA graph: workspaces,
+remembered quantisations and de-quantised weights.
 
 A pass through a graph must not depend on which other graph, or which eager call, came before it."""
 import pytest
@@ -114,3 +114,25 @@ def test_an_eager_call_does_not_use_the_quantisation_of_a_graph():
         graphs[i].replay()
         torch.cuda.synchronize()
         assert torch.equal(outs[i], want3)
+
+
+def test_a_de_quantised_weight_of_a_graph_is_not_remembered():
+    """weight_dequant's cache: what a capture recorded is computed at its replays, an eager call before them computes its own."""
+    import dsv3_b200
+    import kernel
+    w = _weight(512, 512, torch.Generator(device="cuda").manual_seed(2))
+    want = kernel.weight_dequant(w, w.scale)
+    stream = torch.cuda.Stream()
+    keep = _polluted_pool(stream)
+    graph = torch.cuda.CUDAGraph()
+    dsv3_b200.enable_weight_dequant_cache()
+    try:
+        with torch.cuda.graph(graph, pool=keep.pool(), stream=stream):
+            y = kernel.weight_dequant(w, w.scale)
+        got = kernel.weight_dequant(w, w.scale)
+        assert torch.equal(got, want)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, want) and kernel.weight_dequant(w, w.scale) is got
+    finally:
+        dsv3_b200.disable_weight_dequant_cache()
