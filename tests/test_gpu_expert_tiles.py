@@ -1,13 +1,15 @@
 """Tiles of the expert GEMMs (w1/w3 with SwiGLU and quantisation, w2): whole and cut over K.
 
 References: the separate operators per group of rows.  Whole tiles fold every chunk as the other tcgen05 kernels do, so
-with the operators pinned to one split the results are equal bit for bit."""
+with the operators pinned to one split the results are equal bit for bit; a cut tile adds the same terms in another
+order and is held to the bounds of test_gpu_stream.py."""
 import ctypes
 
 import pytest
 import torch
 
-from test_gpu_stream import _Side, _bf16_default, _table, _weight  # noqa: F401
+from gpu_util import assert_gemm_close
+from test_gpu_stream import _Side, _bf16_default, _h_close, _table, _weight  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -90,6 +92,39 @@ def test_whole_tiles_equal_the_operators_bit_for_bit(counts, policy):
     want = layer.operators(got[0], got[1], got[3], got[4])
     for a, b in zip(got, want):
         assert torch.equal(a.view(torch.uint8) if a.element_size() == 1 else a, b.view(torch.uint8) if b.element_size() == 1 else b)
+
+
+# Both launches are cut (33 and 16 K chunks; 33 weight blocks, so that w2's last tile holds one): two token tiles of one group,
+# the second with one row, each in about five parts; and one round and a bit, where a range holds a head, a whole tile and a tail
+_ONE = {16: [17, 0, 0, 0, 0, 0, 0], 32: [33, 0, 0], 64: [65, 0]}
+_TEN = {16: [1, 2, 3, 4, 1, 2, 3, 4, 5, 2], 32: [9, 20, 3, 14, 11, 12, 23, 4, 15, 32], 64: [29, 40, 33, 64, 31, 32, 23, 44, 35, 32]}
+
+
+@pytest.mark.parametrize("side_rows", [0, 9])
+@pytest.mark.parametrize("tile", [16, 32, 64])
+@pytest.mark.parametrize("groups", [_ONE, _TEN], ids=["parts", "ranges"])
+def test_cut_tiles(groups, tile, side_rows):
+    from dsv3_b200 import _lib
+    header = _lib.WORKSPACE_HEADER_BYTES
+    layer = _Layer(groups[tile], 2048, 4224, side_rows)
+    ws = torch.zeros(layer.need, dtype=torch.uint8, device="cuda")
+    ws[header:] = 0x55
+    cut = []
+
+    def parked():
+        cut.append(bool((ws[header:] != 0x55).any()))
+        assert not bool(ws[:header].any()), "tickets are left clean"
+        ws[header:] = 0x55
+
+    got = layer.run(ws, parked)
+    parked()
+    assert cut == [True, True], "partial tiles were parked by both launches"
+    for a, b in zip(got, layer.run(ws)):
+        assert torch.equal(a, b), "parts are added in K order, whoever comes last"
+    want = layer.operators(got[0], got[1], *got[3:5])
+    for i in range(0, len(got), 3):
+        _h_close(got[i].view(torch.float8_e4m3fn), got[i + 1], want[i], want[i + 1].t())
+        assert_gemm_close(got[i + 2].cpu(), want[i + 2].cpu())
 
 
 # fewer and more than one pair per thread of a warp, one CTA's limit of pairs, more tokens than CTAs, few SMs; repeated experts
