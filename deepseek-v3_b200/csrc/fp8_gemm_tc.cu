@@ -1140,8 +1140,6 @@ int launch_fp8_gemm_tc(const void* a, const float* a_s, const void* b, const flo
             case 64: return launch_variant<64, true>(tp, tq, tc, prm, stream);
         }
     } else if (pl.bn == 128) {
-        // long K: two promotion groups on alternate chunks; short K: the end-of-tile combine would
-        // cost more than it saves
         return launch_variant<128, false>(tp, tq, tc, prm, stream);
     }
     set_last_error("fp8_gemm: no tcgen05 variant for tile width %d", pl.bn);

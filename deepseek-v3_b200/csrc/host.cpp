@@ -568,10 +568,11 @@ PyObject* py_fp8_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     });
 }
 
-// (x, weight, block_size, scale_fmt, assume_no_inplace, fused_max_rows, fused_max_bytes): linear()'s FP8 branch.
+// (x, weight, block_size, scale_fmt, assume_no_inplace, fused_max_rows, fused_max_bytes, fused_max_bytes_3_rows): linear()'s FP8
+// branch.  The limits of the fused launch, with their reasons, are in ops.py.
 PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
-        want_args(n, 7);
+        want_args(n, 8);
         const at::Tensor &x = tensor_arg(args[0]), &w = tensor_arg(args[1]);
         const int64_t block = int_arg(args[2]);
         const int fmt = scale_fmt_arg(args[3]);
@@ -582,9 +583,7 @@ PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_DECREF(scale_obj);
         if (!scale.defined()) raise(PyExc_TypeError, "weight.scale is not a tensor");
         const int64_t K = last_dim(x), rows = K ? x.numel() / K : 0;
-        // Every CTA quantises its K range of all rows: from three rows up two launches are faster for large weights (B200, us,
-        // fused / two at 4 rows: 7168 -> 1536 8.9 / 6.9, 5120 -> 1536 7.4 / 6.4, 2048 -> 2816 5.8 / 5.9, 7168 -> 576 5.3 / 6.3).
-        if (rows > 0 && rows <= int_arg(args[5]) && w.numel() <= int_arg(args[6]) && (rows <= 2 || w.numel() <= (6ll << 20)) && block == 128 && K % 128 == 0 &&
+        if (rows > 0 && rows <= int_arg(args[5]) && w.numel() <= int_arg(args[rows <= 2 ? 6 : 7]) && block == 128 && K % 128 == 0 &&
             x.scalar_type() == at::kBFloat16 && x.is_contiguous()) {
             count(g_key_fused);
             return wrap(linear_small(x, w, scale, fmt));
@@ -725,7 +724,7 @@ PyMethodDef methods[] = {
     {"fp8_gemm", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_fp8_gemm)), METH_FASTCALL, "(a, a_s, b, b_s)"},
     {"fp8_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_fp8_linear)), METH_FASTCALL, "(x, weight, scale, scale_fmt)"},
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_linear)), METH_FASTCALL,
-     "(x, weight, block_size, scale_fmt, assume_no_inplace, fused_max_rows, fused_max_bytes)"},
+     "(x, weight, block_size, scale_fmt, assume_no_inplace, fused_max_rows, fused_max_bytes, fused_max_bytes_3_rows)"},
     {"quantise_remembered", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_quantise_remembered)), METH_FASTCALL,
      "(x, block_size, scale_fmt, assume_no_inplace)"},
     {"experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_experts)), METH_FASTCALL,

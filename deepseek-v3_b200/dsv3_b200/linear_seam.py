@@ -10,8 +10,8 @@
 redirects all of them without touching the file.  The replacement keeps the reference's three
 branches and changes how the FP8 branch is launched:
 
-* at most 4 rows (a decode step at small batch) and at most 16 MB of weights: one launch, the activations are
-  quantised in the GEMM's prologue (``fp8_linear``) instead of ``act_quant`` followed by ``fp8_gemm`` and an FP8
+* 1 or 2 rows (a decode step at small batch) and at most 16 MB of weights, or 3 or 4 rows and at most 6 MB: one
+  launch, the activations are quantised in the GEMM's prologue (``fp8_linear``) instead of ``act_quant`` followed by ``fp8_gemm`` and an FP8
   round trip through HBM;
 * more rows: the quantisation of an activation tensor is remembered while that tensor is alive and unmodified,
   so that Linears fed the same input (``wq_a``/``wkv_a`` in MLA, ``w1``/``w3`` in MLP and Expert) quantise it
@@ -33,7 +33,7 @@ import torch
 import torch.nn.functional as F
 
 from ._lib import host
-from .ops import weight_dequant, FUSED_LINEAR_MAX_ROWS, FUSED_LINEAR_MAX_WEIGHT_BYTES
+from .ops import weight_dequant, FUSED_LINEAR_MAX_ROWS, FUSED_LINEAR_MAX_WEIGHT_BYTES, FUSED_LINEAR_MAX_WEIGHT_BYTES_3_ROWS
 
 stats = {"act_quant_calls": 0, "act_quant_reused": 0, "fused_linear_calls": 0}
 _assume_no_inplace = False
@@ -47,7 +47,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         return F.linear(x, weight, bias)
     if gemm_impl == "bf16":
         return F.linear(x, weight_dequant(weight, weight.scale), bias)
-    y = host.linear(x, weight, block_size, scale_fmt, _assume_no_inplace, FUSED_LINEAR_MAX_ROWS, FUSED_LINEAR_MAX_WEIGHT_BYTES)
+    y = host.linear(x, weight, block_size, scale_fmt, _assume_no_inplace, FUSED_LINEAR_MAX_ROWS, FUSED_LINEAR_MAX_WEIGHT_BYTES,
+                    FUSED_LINEAR_MAX_WEIGHT_BYTES_3_ROWS)
     if bias is not None:
         y += bias
     return y

@@ -24,8 +24,10 @@ from .mlp_seam import plain_weights
 from .ops import _stream
 
 # Up to this many tokens the shared experts are worked on in the routed experts' launches, which saves three to four
-# launches of 3-8 us; beyond it their own GEMMs use the machine better (B200, us, inline / separate: 40 tokens 114 / 127,
-# 150 tokens 136 / 158, 333 tokens 171 / 186; 700 tokens 842 / 755).
+# launches of 3-8 us; their tiles take the routed experts' token width, so with many tokens their own GEMMs use the machine
+# better.  B200, us, inline / separate, at 16, 64, 150, 333, 512 and 700 tokens: 64 experts of 2048 x 1408 92 / 107, 110 / 127,
+# 122 / 141, 144 / 159, 162 / 185, 181 / 194; 160 of 5120 x 1536 249 / 259, 424 / 433, 543 / 560, 605 / 603, 676 / 661, 658 / 645; 256 of
+# 7168 x 2048 623 / 643, 1088 / 1114, 1440 / 1453, 1668 / 1660, 1817 / 1809, 1958 / 1979.
 SHARED_INLINE_MAX_ROWS = 512
 
 
