@@ -88,7 +88,7 @@ class GroupedExperts:
                 _lib.check(lib.dsv3_group_table_build(table.data_ptr(), wp, sp, self.n, N, K, _stream()))
             tables[name] = table
         self._keep = (experts, scales)                        # the tables point into these
-        self.signature = self._addresses(container)
+        self.signature = None if self.watched else self._addresses(container)
         self.handle = host.experts(self.n, start, self.dim, self.inter, self.scale_fmt, tables["w1"], tables["w3"], tables["w2"],
                                    container if isinstance(container, list) else None, list(experts),
                                    found if self.watched else [], weights + scales)
