@@ -72,18 +72,17 @@ class GroupedExperts:
                 found += step + step2 + step3
                 weights.append(w)
                 scales.append(s)
-                by_name[name].append(w)
+                by_name[name].append((w, s))
         self.watched = all(f is not None for f in found)      # otherwise they are looked up on every pass
         tables = {}
         for name, N, K in (("w1", self.inter, self.dim), ("w3", self.inter, self.dim), ("w2", self.dim, self.inter)):
-            ws = by_name[name]
-            ss = [w.scale for w in ws]
-            for w, s in zip(ws, ss):
+            pairs, shape = by_name[name], torch.Size((N, K))
+            for w, s in pairs:
                 assert w.element_size() == 1 and w.is_contiguous() and s.is_contiguous() and s.dtype == torch.float32
-                assert tuple(w.shape) == (N, K)
+                assert w.shape == shape
             table = torch.empty(lib.dsv3_group_table_bytes(self.n), dtype=torch.uint8, device=self.device)
-            wp = (ctypes.c_void_p * self.n)(*[w.data_ptr() for w in ws])
-            sp = (ctypes.c_void_p * self.n)(*[s.data_ptr() for s in ss])
+            wp = (ctypes.c_void_p * self.n)(*[w.data_ptr() for w, _ in pairs])
+            sp = (ctypes.c_void_p * self.n)(*[s.data_ptr() for _, s in pairs])
             with torch.cuda.device(self.device):
                 _lib.check(lib.dsv3_group_table_build(table.data_ptr(), wp, sp, self.n, N, K, _stream()))
             tables[name] = table
