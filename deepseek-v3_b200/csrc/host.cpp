@@ -706,16 +706,11 @@ PyObject* py_forget(PyObject*, PyObject*) {
     Py_RETURN_NONE;
 }
 
-// After a bounded wait gave up, tickets may be left non-zero.
-PyObject* py_clear_workspaces(PyObject*, PyObject*) {
-    return guarded([&]() -> PyObject* {
-        for (Workspace& w : g_workspaces) {
-            c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(w.device));
-            if (cudaMemsetAsync(w.mem.data_ptr(), 0, DSV3_WORKSPACE_HEADER_BYTES, w.stream) != cudaSuccess)
-                raise(PyExc_RuntimeError, "could not clear the header of a split-K workspace");
-        }
-        Py_RETURN_NONE;
-    });
+// After a bounded wait gave up, tickets may be left non-zero: the next call gets a new workspace with a clear header.  (A
+// workspace is not cleared in place: its stream may be in a capture, or gone.  A graph clears its own at every replay.)
+PyObject* py_drop_workspaces(PyObject*, PyObject*) {
+    g_workspaces.clear();
+    Py_RETURN_NONE;
 }
 
 PyMethodDef methods[] = {
@@ -737,7 +732,7 @@ PyMethodDef methods[] = {
     {"combine", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_combine)), METH_FASTCALL, "(routed, z)"},
     {"set_stats", py_set_stats, METH_O, "dict whose counters linear() keeps"},
     {"forget", py_forget, METH_NOARGS, "drop the remembered quantisations"},
-    {"clear_workspaces", py_clear_workspaces, METH_NOARGS, "zero the ticket headers of all split-K workspaces"},
+    {"drop_workspaces", py_drop_workspaces, METH_NOARGS, "give the split-K workspaces back"},
     {nullptr, nullptr, 0, nullptr},
 };
 

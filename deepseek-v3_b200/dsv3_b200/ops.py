@@ -163,5 +163,5 @@ def check_device_status() -> None:
     detail = (ctypes.c_uint32 * 4)()
     rc = lib.dsv3_check_device_status(_stream(), ctypes.byref(detail))
     if rc != _lib.OK:
-        host.clear_workspaces()           # tickets may be left non-zero by an aborted launch
+        host.drop_workspaces()            # tickets may be left non-zero by an aborted launch
         _lib.check(rc)

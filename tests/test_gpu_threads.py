@@ -41,3 +41,22 @@ def test_workspace_that_another_thread_drops(make):
         t.join()
     torch.cuda.synchronize()
     assert not bool(torch.stack(wrong).any())
+
+
+def test_after_a_wait_gave_up_workspaces_of_streams_that_are_gone_do_not_matter():
+    """check_device_status makes the next calls start with clear tickets, whatever has become of the streams so far."""
+    import ctypes
+    import dsv3_b200
+    from dsv3_b200 import _lib
+    call = _split_linear()
+    want = call()
+    rt, handle = torch.cuda.cudart(), ctypes.c_void_p()
+    assert int(rt.cudaStreamCreate(ctypes.addressof(handle))) == 0
+    with torch.cuda.stream(torch.cuda.ExternalStream(handle.value)):
+        assert torch.equal(call(), want)
+        torch.cuda.current_stream().synchronize()
+    assert int(rt.cudaStreamDestroy(handle.value)) == 0
+    _lib.check(_lib.lib.dsv3_selftest_bounded_wait(2_000_000, torch.cuda.current_stream().cuda_stream))
+    with pytest.raises(_lib.Dsv3Error):
+        dsv3_b200.check_device_status()
+    assert torch.equal(call(), want)
