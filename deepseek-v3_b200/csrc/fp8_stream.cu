@@ -1124,7 +1124,7 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
     for (int b = 0; b < 2; ++b) {
         const void* tbl = (b == 1 && q.swiglu) ? q.table1 : q.table0;
         prm.g_map[b] = static_cast<const CUtensorMap*>(tbl);
-        prm.g_scale[b] = reinterpret_cast<const float* const*>(static_cast<const uint8_t*>(tbl) + static_cast<size_t>(q.n_groups) * sizeof(CUtensorMap));
+        prm.g_scale[b] = table_scales(tbl, q.n_groups);
     }
     prm.seg = q.seg;
     // token tiles: at most one partly filled tile per group on top of the full ones, and never more groups than rows
@@ -1178,8 +1178,8 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
     return DSV3_ERR_UNSUPPORTED;
 }
 
-// The table holds, in device memory, n tensor maps followed by n scale pointers.
-size_t group_table_bytes(int n) { return static_cast<size_t>(n) * (sizeof(CUtensorMap) + sizeof(const float*)); }
+// The table holds, in device memory, n tensor maps, n scale pointers and n weight pointers.
+size_t group_table_bytes(int n) { return static_cast<size_t>(n) * (sizeof(CUtensorMap) + sizeof(const float*) + sizeof(const uint8_t*)); }
 
 int build_group_table(void* table_dev, const void* const* weights, const float* const* scales, int n, int64_t N,
                       int64_t K, cudaStream_t stream) {
@@ -1194,6 +1194,7 @@ int build_group_table(void* table_dev, const void* const* weights, const float* 
     std::vector<uint8_t> host(group_table_bytes(n));
     CUtensorMap* maps = reinterpret_cast<CUtensorMap*>(host.data());
     const float** sp = reinterpret_cast<const float**>(host.data() + static_cast<size_t>(n) * sizeof(CUtensorMap));
+    const void** wp = reinterpret_cast<const void**>(sp + n);
     for (int e = 0; e < n; ++e) {
         if (!weights[e] || !scales[e] || (reinterpret_cast<uintptr_t>(weights[e]) % 16) != 0) {
             set_last_error("group table: weight %d is null or not 16-byte aligned", e);
@@ -1204,6 +1205,7 @@ int build_group_table(void* table_dev, const void* const* weights, const float* 
         if (rc != DSV3_OK) return rc;
         memcpy(maps + e, &m, sizeof(m));
         sp[e] = scales[e];
+        wp[e] = weights[e];
     }
     DSV3_CUDA_TRY(cudaMemcpyAsync(table_dev, host.data(), host.size(), cudaMemcpyHostToDevice, stream));
     DSV3_CUDA_TRY(cudaStreamSynchronize(stream));   // `host` goes out of scope

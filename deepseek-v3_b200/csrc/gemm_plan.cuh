@@ -79,9 +79,13 @@ int stream_tile(int64_t rows_per_group);
 size_t stream_workspace_bytes(int64_t rows_per_group);
 int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream);
 
-// Table of the weights of up to 256 groups: tensor maps followed by scale pointers, in device memory.
+// Table of the weights of up to 256 groups: tensor maps, scale pointers and weight pointers, in device memory.
 constexpr int kMaxGroupsOfTable = 256;
 size_t group_table_bytes(int n);
+inline const float* const* table_scales(const void* table, int n) {
+    return reinterpret_cast<const float* const*>(static_cast<const uint8_t*>(table) + static_cast<size_t>(n) * sizeof(CUtensorMap));
+}
+inline const uint8_t* const* table_weights(const void* table, int n) { return reinterpret_cast<const uint8_t* const*>(table_scales(table, n) + n); }
 int build_group_table(void* table_dev, const void* const* weights, const float* const* scales, int n, int64_t N,
                       int64_t K, cudaStream_t stream);
 

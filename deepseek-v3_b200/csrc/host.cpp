@@ -387,6 +387,11 @@ Experts* experts_arg(PyObject* c) {
     return e;
 }
 
+// Weights and scales of the shared experts, to be worked on in the same launches (w1, w3, w2).
+struct Shared {
+    at::Tensor w[3], s[3];
+};
+
 // Result of the expert GEMMs of one pass, before the combination: one allocation, carved up.
 struct Routed {
     at::Tensor arena, x;
@@ -394,16 +399,19 @@ struct Routed {
     int topk;
     const void *o, *w, *z = nullptr;      // z: the shared experts' output when the pass computed it
     const int32_t* pos;
+    // a handful of tokens: w2 and the combination are one launch, still to come
+    PyObject* experts = nullptr;          // the capsule, which keeps table and weights
+    Shared sh;
+    dsv3_few_shared_t few_sh = {};
+    const void *route = nullptr, *h = nullptr;
+    Routed() = default;
+    Routed(const Routed&) = delete;
+    ~Routed() { Py_XDECREF(experts); }
 };
 const char* kRoutedName = "dsv3_b200.routed";
 void free_routed(PyObject* c) { delete static_cast<Routed*>(PyCapsule_GetPointer(c, kRoutedName)); }
 
-// Weights and scales of the shared experts, to be worked on in the same launches (w1, w3, w2).
-struct Shared {
-    at::Tensor w[3], s[3];
-};
-
-std::unique_ptr<Routed> run_experts(Experts& e, const at::Tensor& x, const at::Tensor& weights_in, const at::Tensor& indices_in,
+std::unique_ptr<Routed> run_experts(PyObject* capsule, Experts& e, const at::Tensor& x, const at::Tensor& weights_in, const at::Tensor& indices_in,
                                     int64_t n_routed, bool assume_no_inplace, const Shared* sh) {
     if (indices_in.dim() != 2 || weights_in.sizes() != indices_in.sizes())
         raise(PyExc_ValueError, "routing weights and indices must both be [tokens, top-k]");
@@ -429,6 +437,29 @@ std::unique_ptr<Routed> run_experts(Experts& e, const at::Tensor& x, const at::T
         at += (bytes + 255) & ~int64_t(255);
         return here;
     };
+    if (P > 0 && dsv3_few_experts_pay(T, r->topk, e.n, n_routed, dim, inter, sh ? sh->w[0].size(0) : 0)) {
+        const int64_t inter_s = sh ? sh->w[0].size(0) : 0;
+        const int64_t o_route = take(static_cast<int64_t>(dsv3_few_route_bytes())), o_h = take(2 * P * inter), o_hz = take(2 * T * inter_s);
+        r->arena = new_cuda({at}, at::kByte, dev);
+        uint8_t* base = static_cast<uint8_t*>(r->arena.data_ptr());
+        r->route = base + o_route;
+        r->h = base + o_h;
+        r->experts = Py_NewRef(capsule);
+        if (sh) {
+            r->sh = *sh;
+            auto scale = [&](int i) { return static_cast<const float*>(sh->s[i].const_data_ptr()); };
+            r->few_sh = {sh->w[0].const_data_ptr(), scale(0), sh->w[1].const_data_ptr(), scale(1), sh->w[2].const_data_ptr(), scale(2), inter_s, base + o_hz};
+        }
+        const void *t1 = e.table1.const_data_ptr(), *t3 = e.table3.const_data_ptr(), *t2 = e.table2.const_data_ptr();
+        const void *xp = x.const_data_ptr(), *wp = weights.const_data_ptr();
+        const int bf16 = weights.scalar_type() == at::kBFloat16;
+        const auto* ip = static_cast<const int64_t*>(indices.const_data_ptr());
+        call_library(dev, [&](dsv3_stream_t st) {
+            return dsv3_few_up(t1, t3, t2, e.n, xp, T, dim, ip, wp, bf16, r->topk, e.start, inter, e.fmt, base + o_route, base + o_h,
+                               sh ? &r->few_sh : nullptr, st);
+        });
+        return r;
+    }
     const int64_t o_seg = take(4 * (e.n + 1)), o_pos = take(4 * P), o_w = take(2 * P), o_xq = take(P * dim), o_xs = take(4 * P * (dim / 128)),
                   o_hq = take(P * inter), o_hs = take(4 * P * (inter / 128)), o_o = take(2 * P * dim);
     const int64_t inter_s = sh ? sh->w[0].size(0) : 0;
@@ -669,7 +700,7 @@ PyObject* py_run_experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
             if (sh.w[0].size(1) != e.dim || sh.w[1].sizes() != sh.w[0].sizes() || sh.w[2].size(0) != e.dim || sh.w[2].size(1) != f || f % 128 != 0)
                 raise(PyExc_ValueError, "shared weights do not fit the layer");
         }
-        auto r = run_experts(e, tensor_arg(args[1]), tensor_arg(args[2]), tensor_arg(args[3]), int_arg(args[4]),
+        auto r = run_experts(args[0], e, tensor_arg(args[1]), tensor_arg(args[2]), tensor_arg(args[3]), int_arg(args[4]),
                              PyObject_IsTrue(args[5]) == 1, with_shared ? &sh : nullptr);
         return PyCapsule_New(r.release(), kRoutedName, free_routed);
     });
@@ -691,6 +722,15 @@ PyObject* py_combine(PyObject*, PyObject* const* args, Py_ssize_t n) {
         }
         at::Tensor y = new_cuda({r->T, r->dim}, at::kBFloat16, dev);
         void* yp = y.data_ptr();
+        if (r->route) {
+            const bool own = r->sh.w[0].defined() && args[1] == Py_None;       // z takes the place of what was computed along
+            const Experts& e = *experts_arg(r->experts);
+            const void* t2 = e.table2.const_data_ptr();
+            call_library(dev, [&](dsv3_stream_t st) {
+                return dsv3_few_down(t2, e.n, r->route, r->h, r->T, r->topk, r->dim, e.inter, e.fmt, own ? &r->few_sh : nullptr, zp, yp, st);
+            });
+            return wrap(std::move(y));
+        }
         call_library(dev, [&](dsv3_stream_t st) { return dsv3_moe_combine_add(r->o, r->pos, r->w, zp, r->T, r->topk, r->dim, yp, st); });
         return wrap(std::move(y));
     });

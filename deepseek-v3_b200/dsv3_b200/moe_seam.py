@@ -5,8 +5,8 @@ expert costs two host synchronisations (``bincount(...).tolist()``, ``torch.wher
 small launches.  ``grouped_moe_forward`` keeps inputs, outputs and arithmetic (same quantisation per
 token row, same bf16 rounding points, same ascending-expert accumulation order) but runs in
 four launches: routing bookkeeping with the quantisation of the tokens, w1 and w3 of all local experts with SwiGLU and
-the quantisation in front of w2, w2 of all local experts, and the weighted sum with the shared experts' output.
-Nothing is read back to the host.
+the quantisation in front of w2, w2 of all local experts, and the weighted sum with the shared experts' output; or, where few pairs are expected, two (w1 and
+w3 with everything in front of them, w2 with the weighted sum).  Nothing is read back to the host.
 
     import model, dsv3_b200
     dsv3_b200.install_moe(model)        # model.MoE.forward = grouped_moe_forward

@@ -252,6 +252,35 @@ int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const flo
                        size_t workspace_bytes, dsv3_stream_t stream);
 
 /*
+ * The same layer for a handful of tokens (at most 8, and 64 pairs) in two launches: dsv3_few_up is w1 and w3 of the touched
+ * experts with SwiGLU (the pairs are sorted and the tokens quantised inside), dsv3_few_down is w2, the weighted sum and the
+ * addition of the shared experts' output.  dsv3_few_experts_pay: 1 where the pair of them is the faster form (n_routed: experts
+ * of the whole layer, 0 if only the n_local ones), 0 otherwise, or where the sizes are not supported: dim, inter and
+ * inter_shared divisible by 128.
+ *   route  : dsv3_few_route_bytes() bytes, 16-byte aligned, written by few_up for few_down
+ *   h      : bf16 [T*topk, inter] scratch between the two
+ *   shared : weights of the shared experts and scratch h, bf16 [T, inter]; or null.  Then z, bf16 [T, dim], is added if not null.
+ *   y      : bf16 [T, dim]
+ */
+typedef struct dsv3_few_shared {
+    const void* w1;
+    const float* w1_s;
+    const void* w3;
+    const float* w3_s;
+    const void* w2;
+    const float* w2_s;
+    int64_t inter;
+    void* h;
+} dsv3_few_shared_t;
+int dsv3_few_experts_pay(int64_t T, int topk, int n_local, int64_t n_routed, int64_t dim, int64_t inter, int64_t inter_shared);
+size_t dsv3_few_route_bytes(void);
+int dsv3_few_up(const void* table1, const void* table3, const void* table2, int n, const void* x, int64_t T, int64_t dim, const int64_t* indices,
+                const void* weights, int weights_bf16, int topk, int start, int64_t inter, int scale_fmt, void* route, void* h,
+                const dsv3_few_shared_t* shared, dsv3_stream_t stream);
+int dsv3_few_down(const void* table2, int n, const void* route, const void* h, int64_t T, int topk, int64_t dim, int64_t inter, int scale_fmt,
+                  const dsv3_few_shared_t* shared, const void* z, void* y, dsv3_stream_t stream);
+
+/*
  * One-shot all-reduce of a decode-sized bf16 tensor over peer-mapped buffers -- replaces `dist.all_reduce(y)` after
  * a row-parallel Linear and after the MoE expert loop (model.py:263-264, 691-692) for small y, where a ring or tree
  * collective is bound by latency.  One process per GPU; every rank
