@@ -10,7 +10,8 @@
 //     against up to BN tokens: the token tile crosses from L2 once per 256 weight rows instead of once per 128, and
 //     both halves of a SwiGLU pair meet in the same thread's registers.
 //   * Up to 64 tokens per tile: weights are the M operand (128 TMEM lanes), tokens the N operand, and a tile of 16 tokens
-//     costs 16 columns (fp8_stream_kernel).  Up to 128 tokens: tokens are the M operand (fp8_rows_kernel).
+//     costs 16 columns (fp8_stream_kernel).  Up to 128 tokens: tokens are the M operand (fp8_rows_kernel).  With many tokens
+//     the two work side by side, each on the groups that suit it (stream_tile).
 //   * Uneven split: where whole tiles would leave the last round of SMs mostly idle, the (tile, K chunk) space is cut into
 //     equal contiguous ranges, one per CTA (struct Plan).  A CTA then has at most two partial tiles (the head
 //     and the tail of its range); they are parked as fp32 (valid tokens only) and the CTA that takes a tile's last ticket
@@ -68,8 +69,8 @@ struct SCfg {
     static constexpr int kSlots = kRows ? 2 : (BN <= 32 ? 8 : 512 / kSlotCols);
     static constexpr int kTmemCols = kSlots * kSlotCols;
     // weights on the M side: ring of scales, per-warp maxima and final scales
-    static constexpr int kTabChunks = BN <= 32 ? 16 : 8;              // K chunks per slot of the scale ring
-    static constexpr int kTabBytes = kRows ? 0 : 2 * kTabChunks * (BN + 2) * 4;   // token scales, then the two blocks' scales
+    static constexpr int kTabChunks = BN <= 16 ? 16 : (BN <= 32 ? 12 : 8);              // K chunks per slot of the scale ring
+    static constexpr int kTabBytes = kRows ? 0 : 2 * kTabChunks * 2 * BN * 4;         // token scale x block scale, of both blocks
     static constexpr int kSegBytes = kRows ? 0 : (kMaxGroups + 1) * 4;           // row offsets of the groups
     static constexpr int kRedBytes = kRows ? 0 : (4 + 1) * BN * 4;
     // tokens on the M side: exchange of SwiGLU halves / staging of results
@@ -98,6 +99,15 @@ struct Side {
     int64_t hs_row, hs_blk;
 };
 constexpr int kGroups = 0, kOrdinary = 1;
+// Two launches that work on different groups of one problem (launch_fp8_stream) run side by side: the second's CTAs start as
+// the first's leave.  It does not wait for the first before it begins (what both read was complete when the first let
+// its dependents go), but for its end before it ends, so that whatever waits for the second has waited for both.
+constexpr int kFirstOfTwo = 1, kSecondOfTwo = 2;
+__device__ __forceinline__ void wait_for_inputs(int overlap) {
+    if (overlap != kFirstOfTwo) griddep_launch_dependents();
+    if (overlap != kSecondOfTwo) griddep_wait();
+    if (overlap == kFirstOfTwo) griddep_launch_dependents();
+}
 
 struct StreamParams {
     Side side[2];
@@ -106,6 +116,8 @@ struct StreamParams {
     const float* const* g_scale[2];
     const int* seg;
     int n_groups;
+    int min_rows, max_rows;             // groups with fewer or more rows are another launch's
+    int overlap;                        // kFirstOfTwo, kSecondOfTwo or 0: this launch and another work on the same problem
     const float* scale[2];              // ordinary weight (its maps are kernel parameters)
     int scale_fmt;
     // split tiles
@@ -244,7 +256,8 @@ __device__ __forceinline__ void prefix_groups(const StreamParams& p, int* prefix
         const int e = threadIdx.x;
         if (e < p.n_groups) {
             const int first = __ldg(p.seg + e), end = __ldg(p.seg + e + 1);
-            v = (end - first + BN - 1) / BN;
+            const int rows = end - first;
+            v = rows >= p.min_rows && rows <= p.max_rows ? (rows + BN - 1) / BN : 0;
             if (seg) {
                 seg[e] = first;
                 if (e == p.n_groups - 1) seg[e + 1] = end;
@@ -329,7 +342,7 @@ __device__ __forceinline__ bool last_part(const StreamParams& p, Control* ctl, i
     return mine;
 }
 
-__device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_base, uint32_t cols) {
+__device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_base, uint32_t cols, int overlap) {
     __syncwarp();
     tc_fence_before();
     __syncthreads();
@@ -343,6 +356,7 @@ __device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_b
         tc_fence_after();
         tc_dealloc(tmem_base, cols);
     }
+    if (overlap == kSecondOfTwo) griddep_wait();
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -365,8 +379,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t tiles = (raw + 1023u) & ~1023u;
     uint8_t* gen = smem_raw + (tiles - raw);
-    float* tab = reinterpret_cast<float*>(gen + NS * C::kStageBytes);                 // [2][TC][BN] token scales
-    float* btab = tab + 2 * TC * BN;                                                  // [2][TC][2] scales of the two blocks
+    float* tab = reinterpret_cast<float*>(gen + NS * C::kStageBytes);                 // [2][TC][2][BN] token scale x scale of block 0, 1
     float* red = reinterpret_cast<float*>(gen + NS * C::kStageBytes + C::kTabBytes);  // [4][BN] maxima, then [BN] scales
     uint64_t* bars = reinterpret_cast<uint64_t*>(gen + NS * C::kStageBytes + C::kTabBytes + C::kRedBytes);
     Control* ctl = reinterpret_cast<Control*>(bars + 2 * NS + 2 * NT + 4);
@@ -407,8 +420,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         }
     }
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
-    griddep_launch_dependents();
-    griddep_wait();
+    wait_for_inputs(p.overlap);
     prefix_groups<BN>(p, prefix, scan, seg, warp, lane);
     tc_fence_before();
     __syncthreads();
@@ -463,34 +475,37 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         const int tid = threadIdx.x - 64;
         while (ok && wk.next(s)) {
             const Side& d = p.side[kBoth ? s.side : kGroups];
-            // this thread's block and, below, chunk of the slot (threads below 2 TC)
-            const int blk = kSwiglu ? s.p : min(2 * s.p + (tid & 1), d.nblk - 1);
-            const float* bs = ((!kBoth || s.side == kGroups) ? p.g_scale[tid & 1][s.group] : p.scale[tid & 1]) + static_cast<int64_t>(blk) * s.kc;
+            const int blk1 = kSwiglu ? s.p : min(2 * s.p + 1, d.nblk - 1), blk0 = kSwiglu ? s.p : 2 * s.p;
+            const float* bs0 = ((!kBoth || s.side == kGroups) ? p.g_scale[0][s.group] : p.scale[0]) + static_cast<int64_t>(blk0) * s.kc;
+            const float* bs1 = ((!kBoth || s.side == kGroups) ? p.g_scale[1][s.group] : p.scale[1]) + static_cast<int64_t>(blk1) * s.kc;
             for (int k = s.c0; k < s.c1; k += TC, ++t) {
                 const int sl = t & 1;
                 ok = __all_sync(0xffffffffu, bounded_wait(sempty_bar(sl), ((t >> 1) & 1u) ^ 1u, ctl, p.status, 7, t));
                 if (!ok) break;
                 const int n = min(TC, s.c1 - k);
-                float* dst = tab + sl * TC * BN;
+                float* dst = tab + sl * TC * 2 * BN;
                 // All loads of a slot are in flight together: they queue behind the weights' (one after the other they held
                 // the first chunk back by 7 us).  Columns beyond ntok keep what they held: they multiply products nobody reads.
                 constexpr int kLoads = TC * BN / kTabThreads;
                 static_assert(kTabThreads % BN == 0 || BN % kTabThreads == 0, "a thread's columns do not depend on the trip");
-                static_assert(2 * TC <= kTabThreads, "one block scale per thread");
-                float r[kLoads], rb = 0.0f;
-                const bool has_b = (tid >> 1) < n;
-                if (has_b) rb = __ldg(bs + k + (tid >> 1));
+                float r[kLoads], r0[kLoads], r1[kLoads];
 #pragma unroll
                 for (int u = 0; u < kLoads; ++u) {
                     const int i = tid + u * kTabThreads, ch = i / BN, col = i - ch * BN;
-                    if (ch < n && col < s.ntok) r[u] = __ldg(d.a_s + (s.row0 + col) * d.as_row + (k + ch) * d.as_chunk);
+                    if (ch < n && col < s.ntok) {
+                        r[u] = __ldg(d.a_s + (s.row0 + col) * d.as_row + (k + ch) * d.as_chunk);
+                        r0[u] = __ldg(bs0 + k + ch);
+                        r1[u] = __ldg(bs1 + k + ch);
+                    }
                 }
 #pragma unroll
                 for (int u = 0; u < kLoads; ++u) {
                     const int i = tid + u * kTabThreads, ch = i / BN, col = i - ch * BN;
-                    if (ch < n && col < s.ntok) dst[i] = r[u];
+                    if (ch < n && col < s.ntok) {
+                        dst[ch * 2 * BN + col] = r[u] * r0[u];
+                        dst[ch * 2 * BN + BN + col] = r[u] * r1[u];
+                    }
                 }
-                if (has_b) btab[sl * TC * 2 + tid] = rb;
                 mbar_arrive(sfull_bar(sl));
             }
         }
@@ -518,18 +533,18 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
             }
         };
         // acc += product * (a_s * b_s), the order of the other tcgen05 kernels, so that a tile that is not cut equals theirs bit
-        // for bit; one shared-memory load of the token scales serves both blocks
-        auto fold_piece = [&](const float* as, float bs0, float bs1, int i, const uint32_t (&vv)[2][PW]) {
-            const float4* as4 = reinterpret_cast<const float4*>(as + 2 * PW * i);
-            const float2 b2[2] = {make_float2(bs0, bs0), make_float2(bs1, bs1)};
+        // for bit.  The scale warps form a_s * b_s once per CTA: formed here, by every thread for all of its rows, the
+        // multiplications took as much of the FP32 pipes as the sums (64-token tiles, 256 experts of 7168 x 2048 with 64 tokens
+        // each: 2936 -> 2724 us).
+        auto fold_piece = [&](const float* as, int i, const uint32_t (&vv)[2][PW]) {
 #pragma unroll
-            for (int j = 0; j < PW / 4; ++j) {
-                const float4 a4 = as4[j];
+            for (int b = 0; b < 2; ++b) {
+                const float4* as4 = reinterpret_cast<const float4*>(as + b * BN + 2 * PW * i);
 #pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    const float2 lo = __fmul2_rn(make_float2(a4.x, a4.y), b2[b]), hi = __fmul2_rn(make_float2(a4.z, a4.w), b2[b]);
-                    acc[b][i][2 * j] = __ffma2_rn(make_float2(__uint_as_float(vv[b][4 * j]), __uint_as_float(vv[b][4 * j + 1])), lo, acc[b][i][2 * j]);
-                    acc[b][i][2 * j + 1] = __ffma2_rn(make_float2(__uint_as_float(vv[b][4 * j + 2]), __uint_as_float(vv[b][4 * j + 3])), hi, acc[b][i][2 * j + 1]);
+                for (int j = 0; j < PW / 4; ++j) {
+                    const float4 a4 = as4[j];
+                    acc[b][i][2 * j] = __ffma2_rn(make_float2(__uint_as_float(vv[b][4 * j]), __uint_as_float(vv[b][4 * j + 1])), make_float2(a4.x, a4.y), acc[b][i][2 * j]);
+                    acc[b][i][2 * j + 1] = __ffma2_rn(make_float2(__uint_as_float(vv[b][4 * j + 2]), __uint_as_float(vv[b][4 * j + 3])), make_float2(a4.z, a4.w), acc[b][i][2 * j + 1]);
                 }
             }
         };
@@ -551,8 +566,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                     ok = __all_sync(0xffffffffu, bounded_wait_lean(sfull_bar(sl), (t >> 1) & 1u, ctl, p.status, 8, t));
                     if (!ok) break;
                 }
-                const float* as = tab + (sl * TC + in_tab) * BN + col0;
-                const float2 bs = *reinterpret_cast<const float2*>(btab + (sl * TC + in_tab) * 2);
+                const float* as = tab + (sl * TC + in_tab) * 2 * BN + col0;
                 const int ts = g % NT;
                 ok = __all_sync(0xffffffffu, bounded_wait_lean(tfull_bar(ts), (g / NT) & 1u, ctl, p.status, 4, g));
                 if (!ok) break;
@@ -569,9 +583,9 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                 }
                 tc_wait_ld();
                 if (NP <= 2 || np <= 2) release();
-                if (np > 0) fold_piece(as, bs.x, bs.y, 0, v[0]);
+                if (np > 0) fold_piece(as, 0, v[0]);
                 if constexpr (NP > 1) {
-                    if (np > 1) fold_piece(as, bs.x, bs.y, 1, v[1]);
+                    if (np > 1) fold_piece(as, 1, v[1]);
                 }
                 if constexpr (NP > 2) {
                     if (np > 2) {
@@ -579,8 +593,8 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
                         if (np > 3) load_piece(taddr, 3, v[1]);
                         tc_wait_ld();
                         release();
-                        fold_piece(as, bs.x, bs.y, 2, v[0]);
-                        if (np > 3) fold_piece(as, bs.x, bs.y, 3, v[1]);
+                        fold_piece(as, 2, v[0]);
+                        if (np > 3) fold_piece(as, 3, v[1]);
                     }
                 }
                 if (++in_tab == TC || k == n_ch - 1) {
@@ -750,14 +764,14 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
             }
         }
     }
-    teardown(ctl, warp, tmem_base, C::kTmemCols);
+    teardown(ctl, warp, tmem_base, C::kTmemCols, p.overlap);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Up to 128 tokens per tile: tokens on the M side (128 TMEM lanes), the two weight blocks side by side on the N side.
 //
-// With weights on the M side a token's scale varies along a thread's registers (a shared-memory load and four packed
-// operations per two tokens and block) and a token's maximum spans 128 threads.  Here a thread owns one token row and 128
+// With weights on the M side a token's scale varies along a thread's registers (a shared-memory load per four tokens and
+// block) and a token's maximum spans 128 threads.  Here a thread owns one token row and 128
 // columns of one block: one scale product per chunk and thread, and a row's maximum is two threads' business.  The MMA
 // costs 512 cycles per chunk whatever the number of tokens, which the weights' arrival (1300 cycles at 1.85 GHz) hides.
 // ---------------------------------------------------------------------------------------------------------------------
@@ -806,8 +820,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
         }
     }
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
-    griddep_launch_dependents();
-    griddep_wait();
+    wait_for_inputs(p.overlap);
     prefix_groups<BN>(p, prefix, scan, static_cast<int*>(nullptr), warp, lane);
     tc_fence_before();
     __syncthreads();
@@ -1040,7 +1053,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
             }
         }
     }
-    teardown(ctl, warp, tmem_base, C::kTmemCols);
+    teardown(ctl, warp, tmem_base, C::kTmemCols, p.overlap);
 }
 
 template <int BN, bool kSwiglu, bool kRows, bool kBoth, bool kSplit>
@@ -1075,15 +1088,21 @@ int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorM
 // Token tile for an expected load per group.  Uneven routing puts some groups above the expectation; a group that needs
 // a second tile reads its weights a second time (from L2).  Weights on the M side cost only the tokens that are there, so
 // 16 to 64 differ by a few per cent (B200, us, tile 16 / 32 / 64: 2.5 tokens per expert 137 / 139 / 142, 26 tokens
-// 964 / 792 / 784, 31 tokens of a small layer 198 / 184 / 191); from about 44 tokens the 128-token tile with tokens on
-// the M side is ahead (64 tokens: 3291 with tile 64, 2815 with 128).
+// 964 / 792 / 784, 31 tokens of a small layer 198 / 184 / 191).  Above 40 tokens the groups are divided between two launches:
+// those of more than 64 rows in tiles of 128 with tokens on the M side, which read the weights once for 128 tokens, the others in
+// tiles of 64 with the weights there, which multiply no empty rows: an expert layer at these sizes runs at the board's power
+// limit, and half of the experts of an unevenly routed layer have fewer than half of the mean.  us, one kind of tile for all groups
+// (128; 64 from 24 to 44 tokens) / divided: 256 experts of 7168 x 2048, 25 tokens each 2055 / 2010, 32 2126 / 2117, 44 2430 / 2275,
+// 64 2555 / 2339, 128 3586 / 3426; 160 of 5120 x 1536, 26 tokens 744 / 760, 41 873 / 854, 75 1085 / 1005; 64 of 2048 x 1408,
+// 31 tokens 142 / 142, 42 156 / 158, 66 199 / 195, 94 226 / 220.
+constexpr int kDivide = 64;
 int stream_tile(int64_t rows_per_group) {
-    return rows_per_group <= 4 ? 16 : (rows_per_group <= 24 ? 32 : (rows_per_group <= 44 ? 64 : 128));
+    return rows_per_group <= 4 ? 16 : (rows_per_group <= 24 ? 32 : (rows_per_group <= 40 ? 64 : 128));
 }
 
 size_t stream_workspace_bytes(int64_t rows_per_group) {
     const int bn = stream_tile(rows_per_group);
-    if (bn > 64) return 0;            // 128-token tiles are never cut
+    if (bn > 64) return 0;            // of 128 tokens or divided: never cut
     return DSV3_WORKSPACE_HEADER_BYTES + static_cast<size_t>(num_sms()) * 2 * (2 * bn) * kPRows * sizeof(float);
 }
 
@@ -1139,6 +1158,7 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
         tiles[1] = (d.rows + bn - 1) / bn * prm.side[kOrdinary].tiles_p;
     }
     prm.n_groups = q.n_groups;
+    prm.max_rows = INT32_MAX;
     prm.scale_fmt = q.scale_fmt;
     prm.status = status_device_ptr();
     if (!prm.status) return DSV3_ERR_CUDA;
@@ -1169,9 +1189,21 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
         DSV3_STREAM_CASE(16);
         DSV3_STREAM_CASE(32);
         DSV3_STREAM_CASE(64);
-        case 128:
-            if (q.swiglu) DSV3_STREAM_LAUNCH(128, true, true, false);
-            DSV3_STREAM_LAUNCH(128, false, true, false);
+        case 128: {
+            prm.min_rows = kDivide + 1;
+            prm.overlap = kFirstOfTwo;
+            auto large = [&]() -> int {
+                if (q.swiglu) DSV3_STREAM_LAUNCH(128, true, true, false);
+                DSV3_STREAM_LAUNCH(128, false, true, false);
+            };
+            if ((rc = large()) != DSV3_OK) return rc;
+            prm.min_rows = 0;
+            prm.max_rows = kDivide;
+            prm.overlap = kSecondOfTwo;
+            if ((rc = make_tmap(&ta0, q.groups.a, q.groups.rows, q.groups.K, 32)) != DSV3_OK) return rc;
+            return q.swiglu ? launch_variant<64, true, false, false, false>(w0, w1, ta0, ta1, prm, bound, units, stream)
+                            : launch_variant<64, false, false, false, false>(w0, w1, ta0, ta1, prm, bound, units, stream);
+        }
     }
 #undef DSV3_STREAM_LAUNCH
 #undef DSV3_STREAM_CASE
