@@ -34,8 +34,6 @@ namespace dsv3 {
 namespace {
 
 constexpr int kChunkK = 128;    // K elements (= bytes) per scale block
-constexpr int kWarps = 4;
-constexpr int kThreads = kWarps * 32;
 constexpr int kRing = 4;        // weight chunks in flight per warp (16 x 16-byte loads per lane)
 constexpr int kRowPad = 64;     // bytes between the staged token rows beyond the K range: the 8 lanes of one
                                 // shared-memory phase (two token rows x four 16-byte pieces) then hit 8 different bank groups
@@ -69,11 +67,11 @@ __device__ __forceinline__ void st_cluster_f32x4(uint32_t addr_cluster, float4 v
 
 constexpr size_t align16(size_t v) { return (v + 15) & ~static_cast<size_t>(15); }
 
-// WR x WK = kWarps: WR row tiles of 16 weight rows per CTA, WK warps share a row tile and split the CTA's K range.
+// WR x WK warps: WR row tiles of 16 weight rows per CTA, WK warps share a row tile and split the CTA's K range.
 // MT: token groups of 8 (1 or 2).  kFused: activations arrive as bf16 and are quantised here.
 template <int WR, int WK, int MT, bool kFused>
-__global__ void __launch_bounds__(kThreads) fp8_linear_small_kernel(const SmallParams p) {
-    static_assert(WR * WK == kWarps, "warp layout");
+__global__ void __launch_bounds__(WR * WK * 32) fp8_linear_small_kernel(const SmallParams p) {
+    constexpr int kThreads = WR * WK * 32;
     constexpr int TOK = 8 * MT;
     extern __shared__ __align__(16) uint8_t smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -133,7 +131,9 @@ __global__ void __launch_bounds__(kThreads) fp8_linear_small_kernel(const SmallP
     // ---- the CTA's K range of the activations: FP8 bytes and scales into shared memory
     if constexpr (kFused) {
         // a half-warp per (token, chunk) block: 16 lanes x 8 bf16, as in the stand-alone act_quant kernel, kBlocks of them
-        // requested at once (each round is a trip to L2)
+        // requested at once (each round is a trip to L2) and worked on side by side: blocks beyond the last go along as zeros,
+        // since a branch between the blocks would put their chains of shuffles one behind the other (7168 -> 1536 at 2 and 4
+        // tokens 7.5 / 8.8 us with it, 7.0 / 8.2 without)
         constexpr int kHalves = kThreads / 16;
         const int l16 = threadIdx.x & 15;
         const int nblk = p.M * n_cta;
@@ -151,7 +151,6 @@ __global__ void __launch_bounds__(kThreads) fp8_linear_small_kernel(const SmallP
                 }
 #pragma unroll
                 for (int i = 0; i < kBlocks; ++i) {
-                    if (b0 + i * kHalves >= nblk) break;           // warp-uniform
                     float mx = amax8(v[i]);
                     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
                     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
@@ -298,7 +297,7 @@ int launch_variant(const SmallParams& prm, int rowgroups, size_t smem_bytes, cud
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(rowgroups * prm.csize));
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(WR * WK * 32);
     cfg.dynamicSmemBytes = smem_bytes;
     cfg.stream = stream;
     // attributes: dependent launch first, the cluster dimension only when K is split over more than one CTA (a
@@ -354,14 +353,24 @@ int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, cons
     prm.K = static_cast<int>(K);
     prm.kc = static_cast<int>((K + kChunkK - 1) / kChunkK);
     prm.scale_fmt = scale_fmt;
-    // Layout: few weight rows -> a CTA takes one 16-row tile and its four warps split K (more CTAs, and every CTA
+    // Layout: few weight rows -> a CTA takes one 16-row tile and its four (or eight) warps split K (more CTAs, and every CTA
     // quantises only its own K range); many rows -> a CTA takes four row tiles that share the staged activations.
     const bool narrow = N <= 4096;
-    const int wr = narrow ? 1 : 4, wk = narrow ? 4 : 1;
+    const int wr = narrow ? 1 : 4;
+    int wk = narrow ? 4 : 1;
     const int rowgroups = static_cast<int>((N + 16 * wr - 1) / (16 * wr));
     // K splits across the CTAs of a cluster: enough CTAs for two per SM, at least 1.5 chunks per warp
     int csize = 1;
     while (csize < 8 && rowgroups * csize < 2 * num_sms() && prm.kc >= 3 * csize * wk) csize *= 2;
+    // Up to 8 rows, half as many CTAs of eight warps instead, where that leaves no cluster to exchange sums in, or where the
+    // CTAs of four would not all be resident (three per SM; a second round costs as much as the first).  us at 1 / 2 / 4 rows, four
+    // warps / eight: 1536 -> 3072 4.1 / 4.6 / 4.7, 3.8 / 4.5 / 4.6; 2048 -> 2816 4.4 / 5.0 / 5.2, 4.1 / 4.8 / 5.0; 7168 -> 2304 10.5 /
+    // 11.0 / 13.2, 7.4 / 7.6 / 9.0; but, at 1 / 2 rows, 5120 -> 1536 (clusters of four) 5.7 / 6.0, 5.9 / 6.2 and 7168 -> 2048 7.2 / 7.8,
+    // 7.4 / 8.0; and at 16 rows, with twice the accumulators, 1536 -> 3072 8.2, 12.6.
+    if (narrow && M <= 8 && (csize == 2 || (csize > 2 && rowgroups * csize > 7 * num_sms() / 2))) {
+        wk = 8;
+        csize /= 2;
+    }
     prm.csize = csize;
     prm.cpc = (prm.kc + csize - 1) / csize;
     const int mt = M <= 8 ? 1 : 2;
@@ -374,6 +383,9 @@ int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, cons
     }
     const bool fused = x != nullptr;
 #define DSV3_SMALL_CASE(WR_, WK_, MT_, F_) return launch_variant<WR_, WK_, MT_, F_>(prm, rowgroups, smem, stream)
+    if (wk == 8) {
+        if (fused) DSV3_SMALL_CASE(1, 8, 1, true); else DSV3_SMALL_CASE(1, 8, 1, false);
+    }
     if (narrow) {
         if (mt == 1) { if (fused) DSV3_SMALL_CASE(1, 4, 1, true); else DSV3_SMALL_CASE(1, 4, 1, false); }
         else         { if (fused) DSV3_SMALL_CASE(1, 4, 2, true); else DSV3_SMALL_CASE(1, 4, 2, false); }

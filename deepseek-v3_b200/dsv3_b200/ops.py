@@ -123,10 +123,10 @@ def fp8_linear(x: torch.Tensor, weight: torch.Tensor, scale: torch.Tensor, scale
 
 # The kernel takes up to 16 rows; the seam uses it where quantising the activations inside every CTA is cheaper than a launch of
 # its own: up to 2 rows for weights of at most 16 MB, 3 and 4 rows for at most 6 MB.  B200, us, one launch / two, replayed from
-# a graph with the weights in HBM, at 1, 2 and 4 rows: 7168 -> 576 4.3 / 5.6, 4.8 / 5.6, 5.3 / 5.7; 2048 -> 2816 4.6 / 5.5, 5.4 / 6.1,
-# 5.8 / 6.2; 5120 -> 1536 (7.5 MB) 5.6 / 6.4, 6.0 / 6.5, 7.4 / 6.7; 7168 -> 1536 (10.5 MB) 6.9 / 6.7, 7.4 / 6.9, 8.8 / 7.0.  Launched one
+# a graph with the weights in HBM, at 1, 2 and 4 rows: 7168 -> 576 4.2 / 5.6, 4.6 / 5.6, 4.8 / 5.7; 2048 -> 2816 4.1 / 5.5, 4.8 / 6.1,
+# 5.0 / 6.2; 5120 -> 1536 (7.5 MB) 5.6 / 6.4, 5.6 / 6.5, 7.0 / 6.7; 7168 -> 1536 (10.5 MB) 6.8 / 6.7, 7.0 / 6.9, 8.2 / 7.0.  Launched one
 # by one the host needs about 4 us for each, so that one launch is ahead up to 8 us: the line for 1 and 2 rows is drawn for
-# that.  (Near 16 MB it depends on the shape: 2304 -> 7168 at 1 row 7.3 / 7.4, 7168 -> 2304 11.0 / 7.8.)
+# that.  (Near 16 MB, at 1 row: 2304 -> 7168 7.5 / 7.4, 7168 -> 2304 7.4 / 7.8.)
 FUSED_LINEAR_MAX_ROWS = 4
 FUSED_LINEAR_MAX_WEIGHT_BYTES = 16 << 20
 FUSED_LINEAR_MAX_WEIGHT_BYTES_3_ROWS = 6 << 20
