@@ -1007,7 +1007,13 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
                 if (force_kernel == 0) {
                     const double full = pp * pl.tiles_q < pairs ? static_cast<double>(pp * pl.tiles_q) / pairs : 1.0;
                     const double narrow = tm_pair_supported(M, N, K) ? 0.4 + 0.8 * full + unsplit(pp * pl.tiles_q, pairs, 0.265, 0.235, 0.8) : 1e30;
-                    const double wide = tw_pair_supported(M, N, K) ? 1.0 + unsplit(pp * ((N + 255) / 256), pairs, 0.41, 0.41, 1.3) : 1e30;
+                    double wide = 1e30;
+                    if (tw_pair_supported(M, N, K)) {          // (the last round of the wide tiles may be cut into strips)
+                        const int64_t n = pp * ((N + 255) / 256), tail = n % pairs;
+                        const int strip = tw_strip_width(tail, pairs, pl.kc);
+                        wide = 1.0 + (strip ? static_cast<double>(n / pairs) * (pl.kc * 0.41 + 1.3) + pl.kc * (strip == 64 ? 0.27 : 0.37) + 2.0
+                                            : unsplit(n, pairs, 0.41, 0.41, 1.3));
+                    }
                     pl.wide = wide < best && wide <= narrow;
                     pl.pair = pl.wide || narrow < best;
                     if (narrow < best) best = narrow;

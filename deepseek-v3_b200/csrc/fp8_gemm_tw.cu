@@ -87,7 +87,8 @@ struct TwParams {
     int raster;             // token-tile pairs that share consecutive weight tiles in the work order
     FastDiv div_per_group, div_raster;
     int tma_store;          // results leave through shared memory and a TMA store (needs N % 8 == 0)
-    int num_tiles;          // tiles_pp * tiles_q
+    int num_tiles;          // whole tiles: all, or all but those of the last round
+    int tail_tiles, tail_w; // tiles shared out in strips of tail_w columns (128 or 64) instead, one strip per pair; 0: none
 };
 
 struct Tile {
@@ -107,10 +108,32 @@ __device__ __forceinline__ Tile decode_tile(int tile, const TwParams& p) {
     return t;
 }
 
+// The last round.  A machine of 74 pairs works on 448 tiles in six rounds and a seventh of four tiles, which takes as long as the
+// others while 70 pairs have nothing to do.  Where at most half of the pairs would have a tile in the last round, its
+// tiles are cut into strips of 128 or 64 columns, one per pair: a strip loads its tokens like a tile but multiplies a half or a
+// quarter of it, and needs no exchange with the others (every column is summed in the same order: the result is the same bit
+// for bit).  A chunk then takes 0.37 or 0.27 us (the loads in flight) instead of 0.41.  B200, us, whole tiles / strips: M 4096,
+// N 7168, K 16384 (448 tiles) 476 / 460; M 8192, N 7168, K 18432 (896) 1048 / 1024; M 8192, N 18432, K 7168 (2304) 988 / 979;
+// M 1003, N 576, K 7168 (12) 25.1 / 18.8.
+struct Strip {
+    Tile t;
+    int n0;                 // first column
+    bool any;
+};
+__device__ __forceinline__ Strip decode_strip(int pair, const TwParams& p) {
+    Strip s = {};
+    const int shift = p.tail_w == 64 ? 2 : 1;
+    if (p.tail_w == 0 || (pair >> shift) >= p.tail_tiles) return s;
+    s.t = decode_tile(p.num_tiles + (pair >> shift), p);
+    s.n0 = s.t.q * kBN + (pair & ((1 << shift) - 1)) * p.tail_w;
+    s.any = s.n0 < p.N;
+    return s;
+}
+
 template <int kBlock>      // K chunks per scale load: 4 (K chunks a multiple of four, 16-byte aligned scales) or 1
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                   const __grid_constant__ CUtensorMap tmap_c, const TwParams p) {
+                   const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_s, const TwParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t tiles = (raw + 1023u) & ~1023u;     // the same offset in both CTAs of the pair
@@ -151,10 +174,14 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     // the kernel before this one in the stream.  While waiting for that kernel, the producer thread pulls
     // the first weight boxes of this CTA's first tile into L2 (L2 is the point of coherence: should the
     // predecessor still be writing those weights, the later TMA loads see its data all the same).
-    if (threadIdx.x == 0 && pair < p.num_tiles) {
-        const Tile t = decode_tile(pair, p);
+    if (threadIdx.x == 0) {
         const int n_pre = min(kc, kStages);
-        for (int j = 0; j < n_pre; ++j) tma_prefetch_l2_2d(&tmap_b, j * kChunk, t.q * kBN + static_cast<int>(rank) * kBHalf);
+        if (pair < p.num_tiles) {
+            const Tile t = decode_tile(pair, p);
+            for (int j = 0; j < n_pre; ++j) tma_prefetch_l2_2d(&tmap_b, j * kChunk, t.q * kBN + static_cast<int>(rank) * kBHalf);
+        } else if (const Strip s = decode_strip(pair, p); s.any) {
+            for (int j = 0; j < n_pre; ++j) tma_prefetch_l2_2d(&tmap_s, j * kChunk, s.n0 + static_cast<int>(rank) * (p.tail_w / 2));
+        }
     }
     griddep_launch_dependents();
     // the peer's barriers must be initialised before anything is signalled across the pair
@@ -175,10 +202,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 uint32_t g = 0;
                 uint32_t probe = 0;   // result of test_wait on empty[] for chunk g, issued one chunk earlier
                 bool ok = true;
-                for (int tile = pair; ok && tile < p.num_tiles; tile += n_pairs) {
-                    const Tile t = decode_tile(tile, p);
-                    const int a_row = (2 * t.pp + static_cast<int>(rank)) * kPRows;
-                    const int b_row = t.q * kBN + static_cast<int>(rank) * kBHalf;
+                auto load_tile = [&](const void* tmap, int a_row, int b_row, uint32_t bytes) {
                     for (int k = 0; k < kc; ++k, ++g) {
                         const int s = g % kStages;
                         ok = __all_sync(0xffffffffu, wait_probed(probe, empty_bar(s), ((g / kStages) & 1u) ^ 1u, ctl, p.status, 1, g));
@@ -189,13 +213,20 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                         // before this arrive has been made (the phase cannot complete without it)
                         const uint32_t dst = tiles + s * kChunkBytes;
                         if (elect_one()) {
-                            if (rank == 0) mbar_arrive_expect_tx(full_bar(s), 2 * kChunkBytes);
+                            if (rank == 0) mbar_arrive_expect_tx(full_bar(s), bytes);
                             tma_load_2d_pair(dst, &tmap_a, k * kChunk, a_row, lead_full);
-                            tma_load_2d_pair(dst + kPRows * kChunk, &tmap_b, k * kChunk, b_row, lead_full);
+                            tma_load_2d_pair(dst + kPRows * kChunk, tmap, k * kChunk, b_row, lead_full);
                         }
                         __syncwarp();
                     }
+                };
+                for (int tile = pair; ok && tile < p.num_tiles; tile += n_pairs) {
+                    const Tile t = decode_tile(tile, p);
+                    load_tile(&tmap_b, (2 * t.pp + static_cast<int>(rank)) * kPRows, t.q * kBN + static_cast<int>(rank) * kBHalf, 2 * kChunkBytes);
                 }
+                if (const Strip st = decode_strip(pair, p); ok && st.any)
+                    load_tile(&tmap_s, (2 * st.t.pp + static_cast<int>(rank)) * kPRows, st.n0 + static_cast<int>(rank) * (p.tail_w / 2),
+                              2u * (kPRows + p.tail_w / 2) * kChunk);
                 // Nothing waits for the commits onto the empty[] barriers of the last chunks; wait for them here so
                 // that none is in flight when the CTA leaves (it would land in whatever CTA gets this shared memory next).
                 for (uint32_t d = (g > kStages ? g - kStages : 0u); ok && d < g; ++d)
@@ -208,7 +239,6 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             // The whole warp walks the loop (waits included) and one elected lane issues: control flow, addresses
             // and descriptors then stay warp-uniform, which is what makes a tcgen05 instruction cheap to issue.
             if (rank == 0) {
-                constexpr uint32_t idesc = umma_idesc_e4m3_f32(2 * kPRows, kBN);
                 const uint32_t me = static_cast<uint32_t>(warp - 1);
                 const int slot = static_cast<int>(me);
                 const uint32_t peer_tfull = mapa_shared(tfull_bar(slot), 1);
@@ -216,7 +246,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 const uint32_t d_tmem = tmem_base + slot * kBN;
                 bool ok = true;
                 uint32_t g = 0;
-                for (int tile = pair; ok && tile < p.num_tiles; tile += n_pairs) {
+                auto multiply_tile = [&](uint32_t idesc) {
                     for (int k = 0; k < kc; ++k, ++g) {
                         if ((g & 1u) != me) continue;
                         const int s = g % kStages;
@@ -242,7 +272,9 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                         }
                         __syncwarp();
                     }
-                }
+                };
+                for (int tile = pair; ok && tile < p.num_tiles; tile += n_pairs) multiply_tile(umma_idesc_e4m3_f32(2 * kPRows, kBN));
+                if (ok && decode_strip(pair, p).any) multiply_tile(umma_idesc_e4m3_f32(2 * kPRows, static_cast<uint32_t>(p.tail_w)));
             }
         }
     } else {
@@ -405,9 +437,63 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                     nt = decode_tile(next, p);
                     first_scales(nt);
                 }
-                if (!write_tile(2 * cur.pp + static_cast<int>(rank), cur.q) || !more) break;
+                ok = write_tile(2 * cur.pp + static_cast<int>(rank), cur.q);
+                if (!ok || !more) break;
                 tile = next;
                 cur = nt;
+            }
+        }
+        // ---- a strip of the last round: the two warp groups take half of its columns each, and store them directly
+        if (const Strip st = decode_strip(pair, p); ok && st.any) {
+            const int cw = p.tail_w / 2, n0 = st.n0 + half * cw;
+            const float* as_ptr = as_row(st.t);
+            const float* bs_ptr = p.b_s + static_cast<int64_t>(st.n0 / 128) * kc;
+            // scales are requested four chunks ahead: a chunk takes half as long as a load that misses L1
+            float sa[4], sb[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                sa[i] = __ldg(as_ptr + min(i, kc - 1));
+                sb[i] = __ldg(bs_ptr + min(i, kc - 1));
+            }
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[j] = make_float2(0.0f, 0.0f);
+            const uint32_t t_strip = t_lane - col0 + half * cw;
+            for (int k0 = 0; ok && k0 < kc; k0 += 4) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    if (k0 + i >= kc) break;
+                    const int slot = static_cast<int>(g & 1u);
+                    ok = __all_sync(0xffffffffu, bounded_wait_lean(tfull_bar(slot), (g >> 1) & 1u, ctl, p.status, 4, g));
+                    ++g;
+                    if (!ok) break;
+                    tc_fence_after();
+                    const float sc = sa[i] * sb[i];
+                    if (cw == 64) tc_ld_x64(t_strip + slot * kBN, &v[0][0]);
+                    else tc_ld_x32(t_strip + slot * kBN, &v[0][0]);
+                    sa[i] = __ldg(as_ptr + min(k0 + i + 4, kc - 1));
+                    sb[i] = __ldg(bs_ptr + min(k0 + i + 4, kc - 1));
+                    tc_wait_ld();
+                    release(slot);
+                    fold(v[0], sc, 0);
+                    if (cw == 64) fold(v[1], sc, 1);
+                }
+            }
+            const int64_t m = static_cast<int64_t>(2 * st.t.pp + static_cast<int>(rank)) * kPRows + row;
+            if (ok && m < p.M) {
+                __nv_bfloat16* crow = p.c + m * p.N;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const int n = n0 + 8 * j;
+                    if (8 * j >= cw || n >= p.N) break;
+                    if (p.tma_store) {                              // (N % 8 == 0)
+                        *reinterpret_cast<uint4*>(crow + n) = make_uint4(pack_bf16x2(acc[4 * j].x, acc[4 * j].y), pack_bf16x2(acc[4 * j + 1].x, acc[4 * j + 1].y),
+                                                                         pack_bf16x2(acc[4 * j + 2].x, acc[4 * j + 2].y), pack_bf16x2(acc[4 * j + 3].x, acc[4 * j + 3].y));
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            if (n + e < p.N) crow[n + e] = __float2bfloat16_rn(e & 1 ? acc[4 * j + e / 2].y : acc[4 * j + e / 2].x);
+                    }
+                }
             }
         }
     }
@@ -441,6 +527,12 @@ bool tw_pair_supported(int64_t M, int64_t N, int64_t K) {
     // block (otherwise half of every accumulator would).  Whether it is the faster kernel for a problem is the
     // plan's decision (tc_plan).
     return M > kPRows && N > 128;
+}
+
+// (128-wide strips of a short K gain nothing: M 2063, N 7168, K 2304, 30 of 252 tiles, 37.9 us whole, 38.5 in strips)
+int tw_strip_width(int64_t tiles, int64_t pairs, int kc) {
+    if (tiles == 0 || 2 * tiles > pairs) return 0;
+    return 4 * tiles <= pairs ? 64 : (kc >= 24 ? 128 : 0);
 }
 
 int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const float* b_s, int64_t M, int64_t N,
@@ -478,7 +570,14 @@ int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const flo
     prm.div_raster = make_fast_div(static_cast<uint32_t>(prm.raster));
     prm.div_per_group = make_fast_div(static_cast<uint32_t>(prm.raster) * static_cast<uint32_t>(prm.tiles_q));
     prm.tma_store = tma_store ? 1 : 0;
+    const int max_pairs = num_sms() / 2;
     prm.num_tiles = static_cast<int>(tiles_pp * tiles_q);
+    prm.tail_tiles = prm.num_tiles % max_pairs;
+    prm.tail_w = tw_strip_width(prm.tail_tiles, max_pairs, prm.kc);
+    if (prm.tail_w == 0) prm.tail_tiles = 0;
+    prm.num_tiles -= prm.tail_tiles;
+    CUtensorMap ts = tb;
+    if (prm.tail_w && (rc = make_tmap(&ts, b, N, K, prm.tail_w / 2)) != DSV3_OK) return rc;
 
     const bool vec = (prm.kc % 4) == 0 && ((reinterpret_cast<uintptr_t>(a_s) | reinterpret_cast<uintptr_t>(b_s)) % 16) == 0;
     auto kern = vec ? fp8_gemm_tw_kernel<4> : fp8_gemm_tw_kernel<1>;
@@ -494,8 +593,8 @@ int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const flo
         DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
         configured[dev] = true;
     }
-    const int max_pairs = num_sms() / 2;
-    const int pairs = prm.num_tiles < max_pairs ? prm.num_tiles : max_pairs;
+    const int work = prm.num_tiles > 0 && prm.tail_w ? max_pairs : prm.num_tiles + (prm.tail_w ? prm.tail_tiles * (kBN / prm.tail_w) : 0);
+    const int pairs = work < max_pairs ? work : max_pairs;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
     cfg.blockDim = dim3(kNumThreads);
@@ -510,7 +609,7 @@ int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const flo
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    DSV3_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, prm));
+    DSV3_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, ts, prm));
     return DSV3_OK;
 }
 

@@ -39,6 +39,8 @@ int launch_fp8_gemm_tm(const void* a, const float* a_s, const void* b, const flo
 
 // Token-major kernel on CTA pairs with 256-wide accumulators (256 x 256 tiles, no split-K): fp8_gemm_tw.cu.
 bool tw_pair_supported(int64_t M, int64_t N, int64_t K);
+// Width of the strips that the tiles of a last round of `tiles` are cut into on a machine of `pairs` (0: not cut).
+int tw_strip_width(int64_t tiles, int64_t pairs, int kc);
 int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const float* b_s, int64_t M, int64_t N,
                        int64_t K, void* c, cudaStream_t stream);
 
