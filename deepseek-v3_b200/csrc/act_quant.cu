@@ -30,20 +30,26 @@ constexpr int kUnroll = 4;  // blocks in flight per half-warp per loop trip
 // accesses, with every CTA touching addresses megabytes apart, ran 20-30 % slower on B200.)
 constexpr int kBlocksPerCta = (kThreads / 16) * kUnroll;
 
+// kU: blocks per half-warp.  Up to ten CTAs of one block each per SM (eight are resident) it is one: few rows then have all SMs to
+// themselves, and their blocks do not queue behind one another in a thread.  B200, us, 4 / 1 blocks: 100 x 7168 1.86 / 1.73, 300 x 7168
+// 3.40 / 2.55; 1003 x 7168 5.16 / 5.76, 4096 x 7168 15.3 / 18.4; with the GEMM behind it, 7168 -> 1536 at M = 1 7.46 / 7.05, 300 17.2 /
+// 15.3, 400 18.5 / 17.4, 16384 -> 512 at M = 200 (25600 blocks) 15.3 / 15.6.
+constexpr int kFewCtas = 10;
+template <int kU>
 __global__ void __launch_bounds__(kThreads, 4) act_quant128_kernel(const uint4* __restrict__ x, uint2* __restrict__ y,
                                                                  float* __restrict__ s, int64_t nblk, int scale_fmt) {
     griddep_launch_dependents();   // a dependent launch (the GEMM) may set itself up while this kernel runs
     griddep_wait();
     const int lane16 = threadIdx.x & 15;
-    const int64_t b0 = static_cast<int64_t>(blockIdx.x) * kBlocksPerCta + (threadIdx.x >> 4);
-    uint4 v[kUnroll];
+    const int64_t b0 = static_cast<int64_t>(blockIdx.x) * ((kThreads / 16) * kU) + (threadIdx.x >> 4);
+    uint4 v[kU];
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < kU; ++u) {
         const int64_t b = b0 + u * (kThreads / 16);
         v[u] = (b < nblk) ? __ldcs(x + b * 16 + lane16) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
-    for (int u = 0; u < kUnroll; ++u) {
+    for (int u = 0; u < kU; ++u) {
         const int64_t b = b0 + u * (kThreads / 16);
         float m = amax8(v[u]);
         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
@@ -137,13 +143,15 @@ int launch_act_quant(const void* x, int64_t rows, int64_t K, int block_size, int
     if (nblk == 0) return DSV3_OK;
     const int64_t cap = static_cast<int64_t>(num_sms()) * 8;  // 8 resident CTAs of 256 threads per SM
     if (block_size == 128) {
-        const int64_t grid = (nblk + kBlocksPerCta - 1) / kBlocksPerCta;
+        const bool few = nblk <= static_cast<int64_t>(num_sms()) * (kThreads / 16) * kFewCtas;
+        const int64_t per_cta = few ? kThreads / 16 : kBlocksPerCta;
+        const int64_t grid = (nblk + per_cta - 1) / per_cta;
         if (grid >= (1ll << 31)) {
             set_last_error("act_quant: too many blocks (%lld)", static_cast<long long>(nblk));
             return DSV3_ERR_UNSUPPORTED;
         }
-        DSV3_CUDA_TRY(launch_dependent(act_quant128_kernel, dim3(static_cast<unsigned>(grid)), dim3(kThreads), 0, stream,
-                                       static_cast<const uint4*>(x), static_cast<uint2*>(y), s, nblk, scale_fmt));
+        DSV3_CUDA_TRY(launch_dependent(few ? act_quant128_kernel<1> : act_quant128_kernel<kUnroll>, dim3(static_cast<unsigned>(grid)), dim3(kThreads), 0,
+                                       stream, static_cast<const uint4*>(x), static_cast<uint2*>(y), s, nblk, scale_fmt));
     } else {
         const int64_t per_cta = kThreads / 32;
         int64_t grid = (nblk + per_cta - 1) / per_cta;
