@@ -67,6 +67,8 @@ __device__ __forceinline__ void st_cluster_f32x4(uint32_t addr_cluster, float4 v
 
 constexpr size_t align16(size_t v) { return (v + 15) & ~static_cast<size_t>(15); }
 
+constexpr size_t kMaxSmem = 200 * 1024;      // of a CTA: the staged activations, scales and partial sums
+
 // WR x WK warps: WR row tiles of 16 weight rows per CTA, WK warps share a row tile and split the CTA's K range.
 // MT: token groups of 8 (1 or 2).  kFused: activations arrive as bf16 and are quantised here.
 template <int WR, int WK, int MT, bool kFused>
@@ -366,18 +368,23 @@ int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, cons
     // CTAs of four would not all be resident (three per SM; a second round costs as much as the first).  us at 1 / 2 / 4 rows, four
     // warps / eight: 1536 -> 3072 4.1 / 4.6 / 4.7, 3.8 / 4.5 / 4.6; 2048 -> 2816 4.4 / 5.0 / 5.2, 4.1 / 4.8 / 5.0; 7168 -> 2304 10.5 /
     // 11.0 / 13.2, 7.4 / 7.6 / 9.0; but, at 1 / 2 rows, 5120 -> 1536 (clusters of four) 5.7 / 6.0, 5.9 / 6.2 and 7168 -> 2048 7.2 / 7.8,
-    // 7.4 / 8.0; and at 16 rows, with twice the accumulators, 1536 -> 3072 8.2, 12.6.
-    if (narrow && M <= 8 && (csize == 2 || (csize > 2 && rowgroups * csize > 7 * num_sms() / 2))) {
+    // 7.4 / 8.0; and at 16 rows, with twice the accumulators, 1536 -> 3072 8.2, 12.6.  Each CTA then stages twice the K range: a K
+    // too long for that (beyond 24064 without a cluster) stays with four warps.
+    const int mt = M <= 8 ? 1 : 2;
+    const int tok = 8 * mt;
+    auto smem_of = [&](int warps, int ctas) {
+        const size_t cpc = static_cast<size_t>((prm.kc + ctas - 1) / ctas);
+        return align16(static_cast<size_t>(tok) * (cpc * kChunkK + kRowPad)) + static_cast<size_t>(tok) * cpc * 4 +
+               align16(static_cast<size_t>(wr) * cpc * 4) + static_cast<size_t>(ctas + warps) * wr * 16 * tok * 4 + 16;
+    };
+    if (narrow && M <= 8 && (csize == 2 || (csize > 2 && rowgroups * csize > 7 * num_sms() / 2)) && smem_of(8, csize / 2) <= kMaxSmem) {
         wk = 8;
         csize /= 2;
     }
     prm.csize = csize;
     prm.cpc = (prm.kc + csize - 1) / csize;
-    const int mt = M <= 8 ? 1 : 2;
-    const int tok = 8 * mt;
-    const size_t smem = align16(static_cast<size_t>(tok) * (prm.cpc * kChunkK + kRowPad)) + static_cast<size_t>(tok) * prm.cpc * 4 +
-                        align16(static_cast<size_t>(wr) * prm.cpc * 4) + static_cast<size_t>(csize + wk) * wr * 16 * tok * 4 + 16;
-    if (smem > 200 * 1024) {
+    const size_t smem = smem_of(wk, csize);
+    if (smem > kMaxSmem) {
         set_last_error("fp8_linear: K=%lld is too long for the decode kernel's staging buffer", static_cast<long long>(K));
         return DSV3_ERR_UNSUPPORTED;
     }

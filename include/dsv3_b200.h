@@ -103,7 +103,8 @@ int dsv3_fp8_gemm(const void* a, const float* a_s, const void* b, const float* b
  * product is scaled as the reference does (acc += (dot * a_s) * b_s, kernel.py:162), K is split across warps and
  * CTA clusters and summed in a fixed order: the result is deterministic and lies within the fp8_gemm tolerance
  * of dsv3_act_quant followed by dsv3_fp8_gemm (the order of the fp32 partial sums differs).  No workspace.
- * Other shapes return DSV3_ERR_UNSUPPORTED: call the two operators instead.
+ * Other shapes return DSV3_ERR_UNSUPPORTED: call the two operators instead.  So does a K whose share per CTA outgrows the
+ * staging buffer: any K up to 23168 (11008 with more than 8 rows) fits, and up to eight times that the fewer weight rows there are.
  */
 int dsv3_fp8_linear(const void* x, int64_t M, int64_t K, const void* w, const float* w_s, int64_t N,
                     int scale_fmt, void* c, dsv3_stream_t stream);
