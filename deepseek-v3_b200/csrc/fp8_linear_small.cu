@@ -286,16 +286,17 @@ __global__ void __launch_bounds__(WR * WK * 32) fp8_linear_small_kernel(const Sm
 template <int WR, int WK, int MT, bool kFused>
 int launch_variant(const SmallParams& prm, int rowgroups, size_t smem_bytes, cudaStream_t stream) {
     auto kern = fp8_linear_small_kernel<WR, WK, MT, kFused>;
-    static size_t configured[64] = {};
+    // the largest size there is, whatever this call needs: threads whose first calls differ set the same
+    static bool configured[64] = {};
     int dev = 0;
     DSV3_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) {
         set_last_error("fp8_linear: device ordinal %d is outside the supported range", dev);
         return DSV3_ERR_UNSUPPORTED;
     }
-    if (smem_bytes > 48 * 1024 && configured[dev] < smem_bytes) {
-        DSV3_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_bytes)));
-        configured[dev] = smem_bytes;
+    if (!configured[dev]) {
+        DSV3_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxSmem)));
+        configured[dev] = true;
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(rowgroups * prm.csize));

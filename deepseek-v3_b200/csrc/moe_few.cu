@@ -492,17 +492,20 @@ int up_smem(int64_t T, int64_t dim) {
 }
 int down_smem(int64_t widest) { return static_cast<int>(kMaxTokens * (widest + kRowPad) + kMaxTokens * (widest / kChunkK) * 4); }
 
+constexpr int kMaxUpSmem = 160 * 1024, kMaxDownSmem = 96 * 1024;
+
+// The kernel is given the largest size there is, whatever this call needs: threads whose first calls differ set the same.
 template <typename P>
-int launch(void (*kern)(P), int grid, int threads, int smem, const P& prm, cudaStream_t stream, int (&configured)[64]) {
+int launch(void (*kern)(P), int grid, int threads, int smem, int max_smem, const P& prm, cudaStream_t stream, bool (&configured)[64]) {
     int dev = 0;
     DSV3_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) {
         set_last_error("expert layer: device ordinal %d is outside the supported range", dev);
         return DSV3_ERR_UNSUPPORTED;
     }
-    if (smem > 24 * 1024 && configured[dev] < smem) {
-        DSV3_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        configured[dev] = smem;
+    if (!configured[dev]) {
+        DSV3_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+        configured[dev] = true;
     }
     DSV3_CUDA_TRY(launch_dependent(kern, dim3(static_cast<unsigned>(grid)), dim3(threads), static_cast<size_t>(smem), stream, prm));
     return DSV3_OK;
@@ -512,7 +515,7 @@ int launch(void (*kern)(P), int grid, int threads, int smem, const P& prm, cudaS
 bool supported(int64_t T, int topk, int n, int64_t dim, int64_t inter, int64_t inter_s) {
     return T >= 1 && T <= kMaxTokens && topk >= 1 && T * topk <= kMaxPairs && n >= 1 && n <= kMaxExperts && dim >= 128 && dim % 128 == 0 && inter >= 128 &&
            inter % 128 == 0 && inter_s >= 0 && inter_s % 128 == 0 && dim < (1 << 20) && inter < (1 << 20) && inter_s < (1 << 20) &&
-           up_smem(T, dim) <= 160 * 1024 && down_smem(inter > inter_s ? inter : inter_s) <= 96 * 1024;
+           up_smem(T, dim) <= kMaxUpSmem && down_smem(inter > inter_s ? inter : inter_s) <= kMaxDownSmem;
 }
 
 bool aligned16(const void* q) { return reinterpret_cast<uintptr_t>(q) % 16 == 0; }
@@ -583,11 +586,11 @@ int dsv3_few_up(const void* table1, const void* table3, const void* table2, int 
     p.inter = static_cast<int>(inter);
     p.inter_s = static_cast<int>(inter_s);
     p.scale_fmt = scale_fmt;
-    static int configured[64] = {};
+    static bool configured[64] = {};
     // one CTA per SM, and no more than there can be items
     const int64_t most = (inter_s + (T * topk < n ? T * topk : n + topk) * inter) / 16;
     const int grid = static_cast<int>(most < num_sms() ? most : num_sms());
-    return launch(expert_up_few_kernel, grid, kUpThreads, up_smem(T, dim), p, static_cast<cudaStream_t>(stream), configured);
+    return launch(expert_up_few_kernel, grid, kUpThreads, up_smem(T, dim), kMaxUpSmem, p, static_cast<cudaStream_t>(stream), configured);
 }
 
 int dsv3_few_down(const void* table2, int n, const void* route, const void* h, int64_t T, int topk, int64_t dim, int64_t inter, int scale_fmt,
@@ -623,8 +626,8 @@ int dsv3_few_down(const void* table2, int n, const void* route, const void* h, i
     p.inter = static_cast<int>(inter);
     p.inter_s = static_cast<int>(inter_s);
     p.scale_fmt = scale_fmt;
-    static int configured[64] = {};
-    return launch(expert_down_few_kernel, static_cast<int>(dim / 16), kDownThreads, down_smem(inter > inter_s ? inter : inter_s), p,
+    static bool configured[64] = {};
+    return launch(expert_down_few_kernel, static_cast<int>(dim / 16), kDownThreads, down_smem(inter > inter_s ? inter : inter_s), kMaxDownSmem, p,
                   static_cast<cudaStream_t>(stream), configured);
 }
 
