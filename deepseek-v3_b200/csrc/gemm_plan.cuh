@@ -83,6 +83,7 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream);
 
 // Table of the weights of up to 256 groups: tensor maps, scale pointers and weight pointers, in device memory.
 constexpr int kMaxGroupsOfTable = 256;
+constexpr int kMaxTopk = 32;       // experts per token, whichever form of the expert layer takes the call
 size_t group_table_bytes(int n);
 inline const float* const* table_scales(const void* table, int n) {
     return reinterpret_cast<const float* const*>(static_cast<const uint8_t*>(table) + static_cast<size_t>(n) * sizeof(CUtensorMap));

@@ -237,7 +237,6 @@ __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const Dispat
 // depends on that row alone, so the outputs do not depend on it.
 constexpr int kRouteThreads = 1024;
 constexpr int kRouteMaxExperts = 256;
-constexpr int kRouteMaxTopk = 32;
 
 __global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(const int64_t* __restrict__ indices,
                                                                   const float* __restrict__ weights, int64_t T, int topk,
@@ -273,8 +272,8 @@ __global__ void __launch_bounds__(kRouteThreads) moe_route_kernel(const int64_t*
     }
     __syncthreads();   // pair_row is read below by other threads of this CTA
     for (int64_t t = threadIdx.x; t < T; t += kRouteThreads) {
-        int64_t e[kRouteMaxTopk];
-        int order[kRouteMaxTopk];
+        int64_t e[kMaxTopk];
+        int order[kMaxTopk];
         for (int j = 0; j < topk; ++j) {          // insertion sort of the token's experts, ascending
             const int64_t ej = indices[t * topk + j];
             int k = j;
@@ -471,8 +470,8 @@ int dsv3_moe_dispatch(const void* x, int64_t T, int64_t dim, const int64_t* indi
         set_last_error("moe_dispatch: null pointer");
         return DSV3_ERR_INVALID_ARGUMENT;
     }
-    if (n_local < 1 || n_local > kDispMaxExperts || topk > kRouteMaxTopk || T * topk >= (1ll << 31) || dim % 128 != 0 || dim > (1 << 24)) {
-        set_last_error("moe_dispatch: 1..%d local experts, at most top-%d and 2^31 pairs, dim divisible by 128", kDispMaxExperts, kRouteMaxTopk);
+    if (n_local < 1 || n_local > kDispMaxExperts || topk > kMaxTopk || T * topk >= (1ll << 31) || dim % 128 != 0 || dim > (1 << 24)) {
+        set_last_error("moe_dispatch: 1..%d local experts, at most top-%d and 2^31 pairs, dim divisible by 128", kDispMaxExperts, kMaxTopk);
         return DSV3_ERR_UNSUPPORTED;
     }
     if (reinterpret_cast<uintptr_t>(x) % 16 != 0 || reinterpret_cast<uintptr_t>(xq) % 8 != 0 || reinterpret_cast<uintptr_t>(xq_rows) % 8 != 0) {
@@ -518,8 +517,8 @@ int dsv3_moe_route(const int64_t* indices, const float* weights, int64_t T, int 
         set_last_error("moe_route: negative size");
         return DSV3_ERR_INVALID_ARGUMENT;
     }
-    if (n_local > kRouteMaxExperts || topk > kRouteMaxTopk || T * topk >= (1ll << 31)) {
-        set_last_error("moe_route: at most %d local experts, top-%d and 2^31 pairs", kRouteMaxExperts, kRouteMaxTopk);
+    if (n_local > kRouteMaxExperts || topk > kMaxTopk || T * topk >= (1ll << 31)) {
+        set_last_error("moe_route: at most %d local experts, top-%d and 2^31 pairs", kRouteMaxExperts, kMaxTopk);
         return DSV3_ERR_UNSUPPORTED;
     }
     if (!seg || (T * topk > 0 && (!indices || !weights || !tok || !pair_row || !pos_sorted || !w_sorted))) {

@@ -513,8 +513,8 @@ int launch(void (*kern)(P), int grid, int threads, int smem, int max_smem, const
 
 // What the two kernels can do; whether they pay is few_experts_pay's business.
 bool supported(int64_t T, int topk, int n, int64_t dim, int64_t inter, int64_t inter_s) {
-    return T >= 1 && T <= kMaxTokens && topk >= 1 && T * topk <= kMaxPairs && n >= 1 && n <= kMaxExperts && dim >= 128 && dim % 128 == 0 && inter >= 128 &&
-           inter % 128 == 0 && inter_s >= 0 && inter_s % 128 == 0 && dim < (1 << 20) && inter < (1 << 20) && inter_s < (1 << 20) &&
+    return T >= 1 && T <= kMaxTokens && topk >= 1 && topk <= kMaxTopk && T * topk <= kMaxPairs && n >= 1 && n <= kMaxExperts &&
+           dim >= 128 && dim % 128 == 0 && inter >= 128 && inter % 128 == 0 && inter_s >= 0 && inter_s % 128 == 0 && dim < (1 << 20) && inter < (1 << 20) && inter_s < (1 << 20) &&
            up_smem(T, dim) <= kMaxUpSmem && down_smem(inter > inter_s ? inter : inter_s) <= kMaxDownSmem;
 }
 
@@ -555,7 +555,8 @@ int dsv3_few_up(const void* table1, const void* table3, const void* table2, int 
     }
     if (!supported(T, topk, n, dim, inter, inter_s) || !aligned16(x) || !aligned16(h) ||
         (shared && (!aligned16(shared->w1) || !aligned16(shared->w3) || !aligned16(shared->w2) || !aligned16(shared->h)))) {
-        set_last_error("few_up: 1..%d tokens, at most %d pairs and %d experts, sizes divisible by 128, 16-byte alignment", kMaxTokens, kMaxPairs, kMaxExperts);
+        set_last_error("few_up: 1..%d tokens, at most top-%d, %d pairs and %d experts, sizes divisible by 128, 16-byte alignment", kMaxTokens, kMaxTopk,
+                       kMaxPairs, kMaxExperts);
         return DSV3_ERR_UNSUPPORTED;
     }
     UpParams p = {};
@@ -605,7 +606,8 @@ int dsv3_few_down(const void* table2, int n, const void* route, const void* h, i
         return DSV3_ERR_INVALID_ARGUMENT;
     }
     if (!supported(T, topk, n, dim, inter, inter_s) || !aligned16(h) || !aligned16(z) || (shared && (!aligned16(shared->w2) || !aligned16(shared->h)))) {
-        set_last_error("few_down: 1..%d tokens, at most %d pairs and %d experts, sizes divisible by 128, 16-byte alignment", kMaxTokens, kMaxPairs, kMaxExperts);
+        set_last_error("few_down: 1..%d tokens, at most top-%d, %d pairs and %d experts, sizes divisible by 128, 16-byte alignment", kMaxTokens, kMaxTopk,
+                       kMaxPairs, kMaxExperts);
         return DSV3_ERR_UNSUPPORTED;
     }
     DownParams p = {};

@@ -253,7 +253,7 @@ int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const flo
                        size_t workspace_bytes, dsv3_stream_t stream);
 
 /*
- * The same layer for a handful of tokens (at most 8, and 64 pairs) in two launches: dsv3_few_up is w1 and w3 of the touched
+ * The same layer for a handful of tokens (at most 8, top-32 and 64 pairs) in two launches: dsv3_few_up is w1 and w3 of the touched
  * experts with SwiGLU (the pairs are sorted and the tokens quantised inside), dsv3_few_down is w2, the weighted sum and the
  * addition of the shared experts' output.  dsv3_few_experts_pay: 1 where the pair of them is the faster form (n_routed: experts
  * of the whole layer, 0 if only the n_local ones), 0 otherwise, or where the sizes are not supported: dim, inter and
