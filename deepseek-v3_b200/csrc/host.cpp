@@ -706,6 +706,15 @@ PyObject* py_run_experts(PyObject*, PyObject* const* args, Py_ssize_t n) {
     });
 }
 
+// Whether w2 of this pass is still to come (with the combination): until then its weights must stay what they were.
+PyObject* py_weights_pending(PyObject*, PyObject* routed) {
+    return guarded([&]() -> PyObject* {
+        auto* r = static_cast<Routed*>(PyCapsule_GetPointer(routed, kRoutedName));
+        if (!r) throw PythonError{};
+        return PyBool_FromLong(r->route != nullptr);
+    });
+}
+
 // (result of run_experts, z or None): the tokens' weighted sums, plus z (or the shared experts' output computed along)
 PyObject* py_combine(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
@@ -769,6 +778,7 @@ PyMethodDef methods[] = {
     {"experts_current", py_experts_current, METH_O, "whether the experts are still those the tables were built from"},
     {"run_experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_run_experts)), METH_FASTCALL,
      "(experts, x, weights, indices, n_routed, assume_no_inplace, shared)"},
+    {"weights_pending", py_weights_pending, METH_O, "whether `combine` of this result still reads the experts' weights"},
     {"combine", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_combine)), METH_FASTCALL, "(routed, z)"},
     {"set_stats", py_set_stats, METH_O, "dict whose counters linear() keeps"},
     {"forget", py_forget, METH_NOARGS, "drop the remembered quantisations"},

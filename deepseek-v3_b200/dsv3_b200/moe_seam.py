@@ -46,7 +46,7 @@ def _look_up(obj, name):
 
 
 class GroupedExperts:
-    """Device tables (tensor maps + scale pointers) of the local experts' three projections."""
+    """Device tables (tensor maps, pointers of scales and weights) of the local experts' three projections."""
 
     def __init__(self, container, experts: List, start: int):
         self.start = start
@@ -111,9 +111,11 @@ class GroupedExperts:
 
     def run(self, x: torch.Tensor, weights: torch.Tensor, indices: torch.Tensor, n_routed: int = 0, shared=None):
         """The local experts' outputs for the routed tokens (model.py:683-688), to be handed to ``combine``: routing
-        bookkeeping and quantisation, w1 / w3 with SwiGLU and quantisation, w2, nothing read back.  ``n_routed``: experts
-        of the whole layer (this rank owns ``self.n`` of them and, on average, that share of the pairs).  ``shared``: the
-        shared experts' (w1, w3, w2), to be worked on in the same launches; ``combine`` then adds their output."""
+        bookkeeping and quantisation, w1 / w3 with SwiGLU and quantisation, w2, nothing read back.  With few pairs w2 is
+        left to ``combine`` (``host.weights_pending``): until then, and on the same stream, the weights must stay what they
+        were.  ``n_routed``: experts of the whole layer (this rank owns ``self.n`` of them and, on average, that share of the
+        pairs).  ``shared``: the shared experts' (w1, w3, w2), to be worked on in the same launches; ``combine`` then adds
+        their output."""
         return host.run_experts(self.handle, x, weights, indices, n_routed, linear_seam._assume_no_inplace, shared)
 
     def routed(self, x: torch.Tensor, weights: torch.Tensor, indices: torch.Tensor, n_routed: int = 0) -> torch.Tensor:
@@ -151,11 +153,13 @@ def grouped_moe_forward(self, x: torch.Tensor, *, world_size: int = 1, fallback=
     if shared is not None:
         y = host.combine(routed, None)
     else:
+        # the shared experts may be any code of the host's: what still reads the routed experts' weights is launched before it
+        y = host.combine(routed, None) if world_size > 1 or host.weights_pending(routed) else None
         z = self.shared_experts(x)
-        if world_size > 1:
-            import torch.distributed as dist
-            y = host.combine(routed, None)
-            dist.all_reduce(y)
+        if y is not None:
+            if world_size > 1:
+                import torch.distributed as dist
+                dist.all_reduce(y)
             y = y + z
         elif (z.dtype == torch.bfloat16 and z.is_contiguous() and z.size() == x.size() and z.data_ptr() % 16 == 0
               and not z.requires_grad):

@@ -26,3 +26,24 @@ def test_more_experts_per_token_than_the_dispatch_takes_are_refused():
             with pytest.raises(dsv3_b200.Dsv3Error) as e:
                 dsv3_b200.grouped_moe_forward(moe, x)
             assert e.value.status == -2
+
+
+@pytest.mark.parametrize("world_size", [1, 2])
+def test_weights_are_read_before_the_shared_experts_are_called(world_size, monkeypatch):
+    """A host may give the routed experts' weights other contents (the next layer's, say) from there on."""
+    import dsv3_b200
+    monkeypatch.setattr(torch.distributed, "all_reduce", lambda y: y.mul_(2))
+    moe, x = _layer()
+    moe.gate = lambda x: (torch.ones(2, 2, device="cuda"), torch.tensor([[0, 1], [3, 60]], device="cuda"))
+    z = torch.randn(2, 512, device="cuda")
+    moe.shared_experts = lambda x: z
+    want = dsv3_b200.grouped_moe_forward(moe, x, world_size=world_size)
+
+    def overwrite(x):
+        for e in moe.experts[:4]:
+            e.w2.weight.view(torch.uint8).zero_()
+        return z
+
+    moe.shared_experts = overwrite
+    assert torch.equal(dsv3_b200.grouped_moe_forward(moe, x, world_size=world_size), want)
+    assert not torch.equal(want, z)
