@@ -37,7 +37,7 @@ int cuda_fail(cudaError_t e, const char* what) {
 
 static int g_sm_budget = 0;   // dsv3_set_num_sms: SMs the persistent GEMM kernels may occupy (0 = all)
 
-int num_sms() {
+static int all_sms() {
     static int cached[64] = {};
     int dev = 0;
     int n = 148;
@@ -49,8 +49,11 @@ int num_sms() {
         }
         n = cached[dev];
     }
-    return (g_sm_budget > 0 && g_sm_budget < n) ? g_sm_budget : n;
+    return n;
 }
+
+bool sm_budget_set() { return g_sm_budget > 0 && g_sm_budget < all_sms(); }
+int num_sms() { return sm_budget_set() ? g_sm_budget : all_sms(); }
 
 bool pdl_enabled() {
     static const bool on = (getenv("DSV3_DISABLE_PDL") == nullptr);

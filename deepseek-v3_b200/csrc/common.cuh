@@ -16,7 +16,8 @@ namespace dsv3 {
 // ---------------------------------------------------------------- host side
 void set_last_error(const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);  // records detail, returns DSV3_ERR_CUDA
-int num_sms();                                   // SM count of the current device (cached)
+int num_sms();                                   // SM count of the current device (cached), or the budget set for it
+bool sm_budget_set();                            // dsv3_set_num_sms leaves fewer than there are
 bool pdl_enabled();                              // programmatic dependent launch (off when DSV3_DISABLE_PDL is set)
 
 // Launches `kern` so that it may be scheduled while the kernel before it in the stream is still draining

@@ -534,7 +534,8 @@ int dsv3_few_experts_pay(int64_t T, int topk, int n_local, int64_t n_routed, int
     // copy rate but cost 25 us around that.  B200, us, one layer replayed from a graph with cold weights, here / in four
     // launches, by expected pairs: 7168 x 2048, 32 of 256 experts: 1 16.4 / 29.6, 2 35 / 43, 4 43 / 45, 6 50 / 48; all 256: 8 87 / 84.
     // 5120 x 1536, 20 of 160: 0.75 24 / 35, 1.5 30 / 37, 3 50 / 45.  2048 x 1408, 16 of 64: 1.5 21 / 31, 3 24 / 31, 6 42 / 35.
-    if (!supported(T, topk, n_local, dim, inter, inter_shared)) return 0;
+    // Not under an SM budget: `down` is one small CTA per 16 columns, which spread over all SMs.
+    if (!supported(T, topk, n_local, dim, inter, inter_shared) || sm_budget_set()) return 0;
     return T * topk * n_local <= 2 * (n_routed > n_local ? n_routed : n_local);
 }
 

@@ -152,7 +152,8 @@ int dsv3_set_gemm_policy(int kernel, int split_k);
  * (default).  No counterpart in the reference.  For hosts that run a collective next to the GEMMs: a persistent
  * kernel that fills every SM keeps the collective's CTAs waiting until it ends, and the GEMM launched after that
  * finds SMs taken and runs a straggling round; leaving the collective its SMs (about as many as it has
- * channels) avoids both.  Process-wide like the policy above: read when a GEMM is launched (or captured), so it can
+ * channels) avoids both.  The two-launch form of the expert layer (dsv3_few_*) does not keep to it, and
+ * dsv3_few_experts_pay says so.  Process-wide like the policy above: read when a GEMM is launched (or captured), so it can
  * be changed between the launches of one captured graph; change it only while no other thread is inside the library.
  */
 int dsv3_set_num_sms(int n);
