@@ -1231,13 +1231,15 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
         DSV3_STREAM_CASE(32);
         DSV3_STREAM_CASE(64);
         case 128: {
-            prm.min_rows = kDivide + 1;
-            prm.overlap = kFirstOfTwo;
+            // (not under an SM budget: side by side the two launches occupy twice the SMs of either)
+            const bool divide = !sm_budget_set();
+            prm.min_rows = divide ? kDivide + 1 : 0;
+            prm.overlap = divide ? kFirstOfTwo : 0;
             auto large = [&]() -> int {
                 if (q.swiglu) DSV3_STREAM_LAUNCH(128, true, true, false);
                 DSV3_STREAM_LAUNCH(128, false, true, false);
             };
-            if ((rc = large()) != DSV3_OK) return rc;
+            if ((rc = large()) != DSV3_OK || !divide) return rc;
             prm.min_rows = 0;
             prm.max_rows = kDivide;
             prm.overlap = kSecondOfTwo;
