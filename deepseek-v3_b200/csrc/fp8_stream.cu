@@ -10,8 +10,8 @@
 //     against up to BN tokens: the token tile crosses from L2 once per 256 weight rows instead of once per 128, and
 //     both halves of a SwiGLU pair meet in the same thread's registers.
 //   * Up to 64 tokens per tile: weights are the M operand (128 TMEM lanes), tokens the N operand, and a tile of 16 tokens
-//     costs 16 columns (fp8_stream_kernel).  Up to 128 tokens: tokens are the M operand (fp8_rows_kernel).  With many tokens
-//     the two work side by side, each on the groups that suit it (stream_tile).
+//     costs 16 columns (stream_tiles).  Up to 128 tokens: tokens are the M operand (rows_tiles).  With many tokens
+//     one launch has CTAs of both, each for the groups that suit it (stream_tile).
 //   * Uneven split: where whole tiles would leave the last round of SMs mostly idle, the (tile, K chunk) space is cut into
 //     equal contiguous ranges, one per CTA (struct Plan).  A CTA then has at most two partial tiles (the head
 //     and the tail of its range); they are parked as fp32 (valid tokens only) and the CTA that takes a tile's last ticket
@@ -57,7 +57,7 @@ constexpr int kSplitCost = 3;
 template <int BN>
 constexpr int kAlone = BN <= 32 ? 7 : 9;
 
-// kRows: tokens on the M side (fp8_rows_kernel); otherwise weights (fp8_stream_kernel).  kProducts: what its scale ring holds.
+// kRows: tokens on the M side (rows_tiles); otherwise weights (stream_tiles).  kProducts: what its scale ring holds.
 template <int BN_, bool kRows, bool kProducts>
 struct SCfg {
     static constexpr int BN = BN_;
@@ -109,16 +109,6 @@ struct Side {
     int64_t hs_row, hs_blk;
 };
 constexpr int kGroups = 0, kOrdinary = 1;
-// Two launches that work on different groups of one problem (launch_fp8_stream) run side by side: the second's CTAs start as
-// the first's leave.  It does not wait for the first before it begins (what both read was complete when the first let
-// its dependents go), but for its end before it ends, so that whatever waits for the second has waited for both.
-constexpr int kFirstOfTwo = 1, kSecondOfTwo = 2;
-__device__ __forceinline__ void wait_for_inputs(int overlap) {
-    if (overlap != kFirstOfTwo) griddep_launch_dependents();
-    if (overlap != kSecondOfTwo) griddep_wait();
-    if (overlap == kFirstOfTwo) griddep_launch_dependents();
-}
-
 struct StreamParams {
     Side side[2];
     // groups: block b of a tile comes from map / scale set b, in global memory; row offsets seg[n_groups + 1] likewise
@@ -126,8 +116,8 @@ struct StreamParams {
     const float* const* g_scale[2];
     const int* seg;
     int n_groups;
-    int min_rows, max_rows;             // groups with fewer or more rows are another launch's
-    int overlap;                        // kFirstOfTwo, kSecondOfTwo or 0: this launch and another work on the same problem
+    int min_rows, max_rows;             // groups with fewer or more rows are not this problem's
+    int first_cta, ctas;                // the CTAs of the grid that work on it
     const float* scale[2];              // ordinary weight (its maps are kernel parameters)
     int scale_fmt;
     // split tiles
@@ -173,7 +163,7 @@ __device__ __forceinline__ Plan make_plan(const StreamParams& p, int group_tiles
     pl.kc1 = p.side[kOrdinary].kc;
     pl.units = pl.tiles0 * pl.kc0 + pl.tiles1 * pl.kc1;
     pl.G = pl.base = pl.extra = 0;
-    const int ctas = static_cast<int>(gridDim.x);
+    const int ctas = p.ctas;
     const int rounds = static_cast<int>(static_cast<unsigned>(pl.tiles0) / static_cast<unsigned>(ctas));
     const int rest0 = pl.tiles0 - rounds * ctas;
     if constexpr (!kSplit) return pl;
@@ -202,7 +192,7 @@ struct Walker {
     int u, u1;               // next unit and end of the CTA's range
     int tile;                // next whole tile
     __device__ __forceinline__ Walker(const StreamParams& p_, const Plan& pl_, const int* prefix_, const int* seg_) : p(p_), pl(pl_), prefix(prefix_), seg(seg_) {
-        const int cta = static_cast<int>(blockIdx.x);
+        const int cta = static_cast<int>(blockIdx.x) - p.first_cta;
         u = kSplit && cta < pl.G ? pl.begin(cta) : 0;
         u1 = kSplit && cta < pl.G ? pl.begin(cta + 1) : 0;
         tile = cta;
@@ -227,7 +217,7 @@ struct Walker {
             s.ut = 0;
             s.c0 = 0;
             s.c1 = s.kc;
-            tile += static_cast<int>(gridDim.x);
+            tile += p.ctas;
         }
         // inside a weight the token tile runs fastest, so CTAs that work side by side share the weight blocks
         int nq, first, rows;
@@ -352,7 +342,7 @@ __device__ __forceinline__ bool last_part(const StreamParams& p, Control* ctl, i
     return mine;
 }
 
-__device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_base, uint32_t cols, int overlap) {
+__device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_base, uint32_t cols) {
     __syncwarp();
     tc_fence_before();
     __syncthreads();
@@ -366,7 +356,6 @@ __device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_b
         tc_fence_after();
         tc_dealloc(tmem_base, cols);
     }
-    if (overlap == kSecondOfTwo) griddep_wait();
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -376,10 +365,8 @@ __device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_b
 // were for nobody.)  Promotion group g owns every second piece of 16 tokens, of both blocks.
 // ---------------------------------------------------------------------------------------------------------------------
 template <int BN, bool kSwiglu, bool kBoth, bool kSplit>
-__global__ void __launch_bounds__(kNumThreads, 1)
-fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
-                  const __grid_constant__ CUtensorMap tmap_a0, const __grid_constant__ CUtensorMap tmap_a1,
-                  const __grid_constant__ StreamParams p) {
+__device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const CUtensorMap* tmap_w1, const CUtensorMap* tmap_a0, const CUtensorMap* tmap_a1,
+                                             const StreamParams& p) {
     constexpr bool kProducts = scale_products<BN, kSplit>;
     using C = SCfg<BN, false, kProducts>;
     constexpr int NS = C::kStages, NT = C::kSlots, TC = C::kTabChunks;
@@ -425,15 +412,16 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
         }
         ctl->abort_flag = 0;
         mbar_fence_init();
-        tma_prefetch_desc(&tmap_a0);
+        tma_prefetch_desc(tmap_a0);
         if constexpr (kBoth) {
-            tma_prefetch_desc(&tmap_a1);
-            tma_prefetch_desc(&tmap_w0);
-            tma_prefetch_desc(&tmap_w1);
+            tma_prefetch_desc(tmap_a1);
+            tma_prefetch_desc(tmap_w0);
+            tma_prefetch_desc(tmap_w1);
         }
     }
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
-    wait_for_inputs(p.overlap);
+    griddep_launch_dependents();
+    griddep_wait();
     prefix_groups<BN>(p, prefix, scan, seg, warp, lane);
     tc_fence_before();
     __syncthreads();
@@ -444,7 +432,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
     if (warp < kFirstPromoWarp) {
       if constexpr (NP >= 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControlM));
       if (warp == 0) {
-        produce<C, kSwiglu, kBoth, kSplit>(p, pl, prefix, seg, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
+        produce<C, kSwiglu, kBoth, kSplit>(p, pl, prefix, seg, tmap_w0, tmap_w1, tmap_a0, tmap_a1, tiles, bar0, ctl);
       } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
         Walker<BN, kBoth, kSplit> wk(p, pl, prefix, seg);
@@ -650,7 +638,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
             if (kSplit && n_ch < kc_of(s)) {
                 // part of a tile: park the pieces that hold tokens, take a ticket; the last part of the tile adds all
                 // parts in K order and goes on to write the result
-                const int cta = static_cast<int>(blockIdx.x);
+                const int cta = static_cast<int>(blockIdx.x) - p.first_cta;
                 const int first = pl.owner(s.ut), last = pl.owner(s.ut + kc_of(s) - 1);
                 constexpr int kTileVec = 2 * BN / 4 * kPRows;             // float4 per parked tile: [2 blocks][BN / 4][128 rows]
                 float4* base = reinterpret_cast<float4*>(p.partials) + (col0 / 4) * kPRows + row;
@@ -805,7 +793,7 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
             }
         }
     }
-    teardown(ctl, warp, tmem_base, C::kTmemCols, p.overlap);
+    teardown(ctl, warp, tmem_base, C::kTmemCols);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -817,10 +805,8 @@ fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_cons
 // costs 512 cycles per chunk whatever the number of tokens, which the weights' arrival (1300 cycles at 1.85 GHz) hides.
 // ---------------------------------------------------------------------------------------------------------------------
 template <int BN, bool kSwiglu, bool kBoth>
-__global__ void __launch_bounds__(kNumThreads, 1)
-fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
-                const __grid_constant__ CUtensorMap tmap_a0, const __grid_constant__ CUtensorMap tmap_a1,
-                  const __grid_constant__ StreamParams p) {
+__device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUtensorMap* tmap_w1, const CUtensorMap* tmap_a0, const CUtensorMap* tmap_a1,
+                                           const StreamParams& p) {
     using C = SCfg<BN, true, false>;
     constexpr bool kSplit = false;      // its partial tiles would be 128 KB each
     constexpr int NS = C::kStages, NT = C::kSlots;
@@ -853,15 +839,16 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
         }
         ctl->abort_flag = 0;
         mbar_fence_init();
-        tma_prefetch_desc(&tmap_a0);
+        tma_prefetch_desc(tmap_a0);
         if constexpr (kBoth) {
-            tma_prefetch_desc(&tmap_a1);
-            tma_prefetch_desc(&tmap_w0);
-            tma_prefetch_desc(&tmap_w1);
+            tma_prefetch_desc(tmap_a1);
+            tma_prefetch_desc(tmap_w0);
+            tma_prefetch_desc(tmap_w1);
         }
     }
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
-    wait_for_inputs(p.overlap);
+    griddep_launch_dependents();
+    griddep_wait();
     prefix_groups<BN>(p, prefix, scan, static_cast<int*>(nullptr), warp, lane);
     tc_fence_before();
     __syncthreads();
@@ -872,7 +859,7 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
     if (warp < kFirstPromoWarp) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
         if (warp == 0) {
-            produce<C, kSwiglu, kBoth, kSplit>(p, pl, prefix, p.seg, &tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, tiles, bar0, ctl);
+            produce<C, kSwiglu, kBoth, kSplit>(p, pl, prefix, p.seg, tmap_w0, tmap_w1, tmap_a0, tmap_a1, tiles, bar0, ctl);
         } else if (warp == 1) {
             // -------------------------------------------------------- MMA issuer
             Walker<BN, kBoth, kSplit> wk(p, pl, prefix, p.seg);
@@ -1094,19 +1081,30 @@ fp8_rows_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_consta
             }
         }
     }
-    teardown(ctl, warp, tmem_base, C::kTmemCols, p.overlap);
+    teardown(ctl, warp, tmem_base, C::kTmemCols);
 }
 
-template <int BN, bool kSwiglu, bool kRows, bool kBoth, bool kSplit>
-int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, const StreamParams& prm,
-                   int64_t tiles_bound, int64_t units_bound, cudaStream_t stream) {
-    using C = SCfg<BN, kRows, !kRows && scale_products<BN, kSplit>>;
-    constexpr auto pick = [] {
-        if constexpr (kRows) return fp8_rows_kernel<BN, kSwiglu, kBoth>;
-        else return fp8_stream_kernel<BN, kSwiglu, kBoth, kSplit>;
-    };
-    auto kern = pick();
-    static bool configured[64] = {};
+template <int BN, bool kSwiglu, bool kBoth, bool kSplit>
+__global__ void __launch_bounds__(kNumThreads, 1)
+fp8_stream_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
+                  const __grid_constant__ CUtensorMap tmap_a0, const __grid_constant__ CUtensorMap tmap_a1,
+                  const __grid_constant__ StreamParams p) {
+    stream_tiles<BN, kSwiglu, kBoth, kSplit>(&tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, p);
+}
+
+// The groups divided between both kinds of tiles (launch_fp8_stream says when), one CTA per SM at a time: the CTAs of `small`
+// start as those of `large`, which come first, leave.
+template <bool kSwiglu, bool kBoth>
+__global__ void __launch_bounds__(kNumThreads, 1)
+fp8_divided_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
+                   const __grid_constant__ CUtensorMap tmap_a0, const __grid_constant__ CUtensorMap tmap_a1,
+                   const __grid_constant__ StreamParams large, const __grid_constant__ StreamParams small) {
+    if (static_cast<int>(blockIdx.x) < large.ctas) rows_tiles<128, kSwiglu, kBoth>(&tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, large);
+    else stream_tiles<64, kSwiglu, false, false>(&tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, small);
+}
+
+template <typename... KArgs, typename... Args>
+int launch(void (*kern)(KArgs...), int64_t grid, int smem, bool (&configured)[64], cudaStream_t stream, const Args&... args) {
     int dev = 0;
     DSV3_CUDA_TRY(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) {
@@ -1114,14 +1112,36 @@ int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorM
         return DSV3_ERR_UNSUPPORTED;
     }
     if (!configured[dev]) {
-        DSV3_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes));
+        DSV3_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         configured[dev] = true;
     }
-    int64_t grid = num_sms();
-    const int64_t most = kSplit ? units_bound : tiles_bound;      // no more CTAs than there can be work for
-    if (grid > most) grid = most;
-    DSV3_CUDA_TRY(launch_dependent(kern, dim3(static_cast<unsigned>(grid)), dim3(kNumThreads), C::kSmemBytes, stream, w0, w1, ta0, ta1, prm));
+    DSV3_CUDA_TRY(launch_dependent(kern, dim3(static_cast<unsigned>(grid)), dim3(kNumThreads), smem, stream, args...));
     return DSV3_OK;
+}
+
+// most: no more CTAs than there can be work for
+template <int BN, bool kSwiglu, bool kBoth, bool kSplit>
+int launch_stream(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, StreamParams prm, int64_t most,
+                  cudaStream_t stream) {
+    using C = SCfg<BN, false, scale_products<BN, kSplit>>;
+    static bool configured[64] = {};
+    prm.ctas = static_cast<int>(most < num_sms() ? most : num_sms());
+    return launch(fp8_stream_kernel<BN, kSwiglu, kBoth, kSplit>, prm.ctas, C::kSmemBytes, configured, stream, w0, w1, ta0, ta1, prm);
+}
+
+template <bool kSwiglu, bool kBoth>
+int launch_divided(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, StreamParams prm, int64_t most_large,
+                   int64_t most_small, int divide, cudaStream_t stream) {
+    constexpr int kLarge = SCfg<128, true, false>::kSmemBytes, kSmall = SCfg<64, false, true>::kSmemBytes;
+    static bool configured[64] = {};
+    StreamParams small = prm;
+    prm.min_rows = divide + 1;
+    prm.ctas = static_cast<int>(most_large < num_sms() ? most_large : num_sms());
+    small.max_rows = divide;
+    small.first_cta = prm.ctas;
+    small.ctas = divide ? static_cast<int>(most_small < num_sms() ? most_small : num_sms()) : 0;
+    return launch(fp8_divided_kernel<kSwiglu, kBoth>, prm.ctas + small.ctas, kLarge > kSmall ? kLarge : kSmall, configured, stream, w0, w1, ta0, ta1,
+                  prm, small);
 }
 
 }  // namespace
@@ -1129,7 +1149,7 @@ int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorM
 // Token tile for an expected load per group.  Uneven routing puts some groups above the expectation; a group that needs
 // a second tile reads its weights a second time (from L2).  Weights on the M side cost only the tokens that are there, so
 // 16 to 64 differ by a few per cent (B200, us, tile 16 / 32 / 64: 2.5 tokens per expert 137 / 139 / 142, 26 tokens
-// 964 / 792 / 784, 31 tokens of a small layer 198 / 184 / 191).  Above 40 tokens the groups are divided between two launches:
+// 964 / 792 / 784, 31 tokens of a small layer 198 / 184 / 191).  Above 40 tokens the groups are divided between two kinds:
 // those of more than 64 rows in tiles of 128 with tokens on the M side, which read the weights once for 128 tokens, the others in
 // tiles of 64 with the weights there, which multiply no empty rows: an expert layer at these sizes runs at the board's power
 // limit, and half of the experts of an unevenly routed layer have fewer than half of the mean.  us, one kind of tile for all groups
@@ -1137,6 +1157,7 @@ int launch_variant(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorM
 // 64 2555 / 2339, 128 3586 / 3426; 160 of 5120 x 1536, 26 tokens 744 / 760, 41 873 / 854, 75 1085 / 1005; 64 of 2048 x 1408,
 // 31 tokens 142 / 142, 42 156 / 158, 66 199 / 195, 94 226 / 220.
 constexpr int kDivide = 64;
+static_assert(kDivide <= 64, "one tile of stream_tiles<64>");
 int stream_tile(int64_t rows_per_group) {
     return rows_per_group <= 4 ? 16 : (rows_per_group <= 24 ? 32 : (rows_per_group <= 40 ? 64 : 128));
 }
@@ -1217,35 +1238,28 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
         set_last_error("fp8 stream GEMM: %lld K chunks are more than the work-item counter holds", static_cast<long long>(units));
         return DSV3_ERR_UNSUPPORTED;
     }
-    const int64_t bound = tiles[0] + tiles[1];
-#define DSV3_STREAM_LAUNCH(BN_, SW_, ROWS_, SPLIT_)                                                                         \
-    return ordinary ? launch_variant<BN_, SW_, ROWS_, true, SPLIT_>(w0, w1, ta0, ta1, prm, bound, units, stream)           \
-                    : launch_variant<BN_, SW_, ROWS_, false, SPLIT_>(w0, w1, ta0, ta1, prm, bound, units, stream)
+    const int64_t bound = split ? units : tiles[0] + tiles[1];
+#define DSV3_STREAM_LAUNCH(BN_, SW_, SPLIT_)                                                                               \
+    return ordinary ? launch_stream<BN_, SW_, true, SPLIT_>(w0, w1, ta0, ta1, prm, bound, stream)                          \
+                    : launch_stream<BN_, SW_, false, SPLIT_>(w0, w1, ta0, ta1, prm, bound, stream)
 #define DSV3_STREAM_CASE(BN_)                                                                                              \
     case BN_:                                                                                                              \
-        if (q.swiglu) { if (split) DSV3_STREAM_LAUNCH(BN_, true, false, true); DSV3_STREAM_LAUNCH(BN_, true, false, false); } \
-        if (split) DSV3_STREAM_LAUNCH(BN_, false, false, true);                                                            \
-        DSV3_STREAM_LAUNCH(BN_, false, false, false)
+        if (q.swiglu) { if (split) DSV3_STREAM_LAUNCH(BN_, true, true); DSV3_STREAM_LAUNCH(BN_, true, false); }            \
+        if (split) DSV3_STREAM_LAUNCH(BN_, false, true);                                                                   \
+        DSV3_STREAM_LAUNCH(BN_, false, false)
     switch (bn) {
         DSV3_STREAM_CASE(16);
         DSV3_STREAM_CASE(32);
         DSV3_STREAM_CASE(64);
         case 128: {
-            // (not under an SM budget: side by side the two launches occupy twice the SMs of either)
-            const bool divide = !sm_budget_set();
-            prm.min_rows = divide ? kDivide + 1 : 0;
-            prm.overlap = divide ? kFirstOfTwo : 0;
-            auto large = [&]() -> int {
-                if (q.swiglu) DSV3_STREAM_LAUNCH(128, true, true, false);
-                DSV3_STREAM_LAUNCH(128, false, true, false);
-            };
-            if ((rc = large()) != DSV3_OK || !divide) return rc;
-            prm.min_rows = 0;
-            prm.max_rows = kDivide;
-            prm.overlap = kSecondOfTwo;
-            if ((rc = make_tmap(&ta0, q.groups.a, q.groups.rows, q.groups.K, 32)) != DSV3_OK) return rc;
-            return q.swiglu ? launch_variant<64, true, false, false, false>(w0, w1, ta0, ta1, prm, bound, units, stream)
-                            : launch_variant<64, false, false, false, false>(w0, w1, ta0, ta1, prm, bound, units, stream);
+            // a group of at most kDivide rows is one token tile
+            const int64_t small = (q.n_groups < q.groups.rows ? q.n_groups : q.groups.rows) * prm.side[kGroups].tiles_p;
+            const int divide = sm_budget_set() ? 0 : kDivide;       // under a budget both kinds' CTAs could be resident side by side
+            if (q.swiglu)
+                return ordinary ? launch_divided<true, true>(w0, w1, ta0, ta1, prm, bound, small, divide, stream)
+                                : launch_divided<true, false>(w0, w1, ta0, ta1, prm, bound, small, divide, stream);
+            return ordinary ? launch_divided<false, true>(w0, w1, ta0, ta1, prm, bound, small, divide, stream)
+                            : launch_divided<false, false>(w0, w1, ta0, ta1, prm, bound, small, divide, stream);
         }
     }
 #undef DSV3_STREAM_LAUNCH

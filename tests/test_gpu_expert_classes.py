@@ -1,5 +1,5 @@
-"""Expert GEMMs whose groups are divided between two launches (more than 64 rows, and the others): either class empty, both, and
-the edge between them, with a side problem in the first launch."""
+"""Expert GEMMs whose groups are divided between two kinds of tiles (more than 64 rows, and the others): either class empty, both, and
+the edge between them, with a side problem among the first CTAs'."""
 import pytest
 
 from test_gpu_stream import _bf16_default, test_expert_gemms_match_the_operators_per_group as _check_groups  # noqa: F401

@@ -36,7 +36,8 @@ def _layer(tokens):
     import dsv3_b200
     moe = _MoE(512, 512, 4, 2, 0, 4, seed=23)
     x = torch.randn(tokens, 512, generator=torch.Generator(device="cuda").manual_seed(tokens), device="cuda", dtype=torch.float32).bfloat16()
-    moe.shared_experts = lambda x: x
+    routing = moe.gate(x)
+    moe.gate, moe.shared_experts = lambda x: routing, lambda x: x
     return lambda: dsv3_b200.grouped_moe_forward(moe, x)
 
 
@@ -51,3 +52,9 @@ def test_the_gemms_keep_to_an_sm_budget(tokens):
     finally:
         dsv3_b200.set_num_sms(0)
     assert len(gemms) == 2 and max(gemms) <= 8
+
+
+@pytest.mark.parametrize("tokens", [40, 200])
+def test_four_launches_whatever_the_tiles(tokens):
+    """Groups that are divided between two kinds of tiles are worked on in one launch: all of its CTAs wait for what came before."""
+    assert len(_kernels(_layer(tokens))) == 4
