@@ -57,8 +57,8 @@ constexpr int kSplitCost = 3;
 template <int BN>
 constexpr int kAlone = BN <= 32 ? 7 : 9;
 
-// kRows: tokens on the M side (rows_tiles); otherwise weights (stream_tiles).  kProducts: what its scale ring holds.
-template <int BN_, bool kRows, bool kProducts>
+// kRows: tokens on the M side (rows_tiles); otherwise weights (stream_tiles).
+template <int BN_, bool kRows>
 struct SCfg {
     static constexpr int BN = BN_;
     static constexpr int kBox = BN < 32 ? BN : 32;                    // token rows per TMA box
@@ -69,8 +69,8 @@ struct SCfg {
     static constexpr int kSlots = kRows ? 2 : (BN <= 32 ? 8 : 512 / kSlotCols);
     static constexpr int kTmemCols = kSlots * kSlotCols;
     // weights on the M side: ring of scales, per-warp maxima and final scales
-    static constexpr int kTabChunks = BN <= 16 ? 16 : (BN <= 32 ? (kProducts ? 12 : 16) : 8);      // K chunks per slot of the scale ring
-    static constexpr int kTabBytes = kRows ? 0 : 2 * kTabChunks * (kProducts ? 2 * BN : BN + 2) * 4;
+    static constexpr int kTabChunks = BN <= 16 ? 16 : (BN <= 32 ? 12 : 8);              // K chunks per slot of the scale ring
+    static constexpr int kTabBytes = kRows ? 0 : 2 * kTabChunks * 2 * BN * 4;         // token scale x block scale, of both blocks
     static constexpr int kSegBytes = kRows ? 0 : (kMaxGroups + 1) * 4;           // row offsets of the groups
     static constexpr int kRedBytes = kRows ? 0 : (4 + 1) * BN * 4;
     // tokens on the M side: exchange of SwiGLU halves / staging of results
@@ -83,16 +83,6 @@ struct SCfg {
     static_assert(kSmemBytes > 116 * 1024, "one CTA per SM");
     static_assert(kTmemCols >= 32 && kTmemCols <= 512 && (kTmemCols & (kTmemCols - 1)) == 0, "TMEM columns");
 };
-
-// Who multiplies a token's scale by a block's (weights on the M side).  The scale warps, once per CTA: with tiles of 64 tokens the
-// promotion threads, each doing it for all of its rows, spent as much of the FP32 pipes on it as on the sums (256 experts of
-// 7168 x 2048 with 64 tokens each: 2936 -> 2724 us).  The promotion threads, with the narrower tiles of a problem that is cut: it
-// has few chunks per CTA and waits for the first scales, and a scale warp would make three loads per chunk and token for one.  us,
-// promotion threads / scale warps, one layer: cut, 20 of 160 experts of 5120 x 1536 at 4, 8 and 12 tokens 42.8 / 43.6, 43.9 /
-// 44.8, 49.4 / 50.6, 16 of 64 of 2048 x 1408 at 24 and 64 47.0 / 48.0, 53.8 / 54.6; whole tiles, all 64 at 8, 96 and 150 67.6 / 66.7,
-// 112.5 / 111.4, 120.3 / 119.0.
-template <int BN, bool kSplit>
-constexpr bool scale_products = BN > 32 || !kSplit;
 
 // A launch works on up to two problems that share the shape of a tile: the groups (per-group weights, rows by group) and
 // one ordinary weight (the shared experts next to the routed ones; kBoth).
@@ -367,8 +357,7 @@ __device__ __forceinline__ void teardown(Control* ctl, int warp, uint32_t tmem_b
 template <int BN, bool kSwiglu, bool kBoth, bool kSplit>
 __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const CUtensorMap* tmap_w1, const CUtensorMap* tmap_a0, const CUtensorMap* tmap_a1,
                                              const StreamParams& p) {
-    constexpr bool kProducts = scale_products<BN, kSplit>;
-    using C = SCfg<BN, false, kProducts>;
+    using C = SCfg<BN, false>;
     constexpr int NS = C::kStages, NT = C::kSlots, TC = C::kTabChunks;
     constexpr int PW = BN == 16 ? 8 : 16;  // tokens per piece
     constexpr int NP = BN / 2 / PW;        // pieces per promotion thread: piece i covers tokens (2 i + group) PW ...
@@ -377,9 +366,7 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t tiles = (raw + 1023u) & ~1023u;
     uint8_t* gen = smem_raw + (tiles - raw);
-    // the scale ring: [2][TC][2][BN] token scale x scale of block 0, 1; or [2][TC][BN] token scales, then [2][TC][2] block scales
-    float* tab = reinterpret_cast<float*>(gen + NS * C::kStageBytes);
-    [[maybe_unused]] float* btab = tab + 2 * TC * BN;
+    float* tab = reinterpret_cast<float*>(gen + NS * C::kStageBytes);                 // [2][TC][2][BN] token scale x scale of block 0, 1
     float* red = reinterpret_cast<float*>(gen + NS * C::kStageBytes + C::kTabBytes);  // [4][BN] maxima, then [BN] scales
     uint64_t* bars = reinterpret_cast<uint64_t*>(gen + NS * C::kStageBytes + C::kTabBytes + C::kRedBytes);
     Control* ctl = reinterpret_cast<Control*>(bars + 2 * NS + 2 * NT + 4);
@@ -474,35 +461,40 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
         uint32_t t = 0;          // ring counter
         bool ok = true;
         const int tid = threadIdx.x - 64;
+        // Block scales: a lane loads that of block lane % 2 of chunk lane / 2 and the warp's lanes hand them round (with a load of
+        // its own for each of a thread's products, three for one, 64-token tiles took up to 6 % longer, cut ones of 16 and 32 up
+        // to 2 %).  Whole tiles of 16 and 32 are ahead by up to 1 % with loads of their own.  us, own loads / handed round, one
+        // layer: 64-token tiles, 256 experts of 7168 x 2048 at 1003 tokens 1937 / 1823, 160 of 5120 x 1536 at 700 680 / 644;
+        // divided, 1600 tokens 870 / 829; cut, 20 of 160 of 5120 x 1536 at 12 tokens 50.6 / 49.5; whole 32-token
+        // tiles, 32 of 256 of 7168 x 2048 at 280 tokens 251.8 / 253.7.
+        constexpr bool kOwn = BN > 32 || kSplit;
         while (ok && wk.next(s)) {
             const Side& d = p.side[kBoth ? s.side : kGroups];
             auto block_scales = [&](int b) {
                 const int blk = kSwiglu ? s.p : min(2 * s.p + b, d.nblk - 1);
                 return ((!kBoth || s.side == kGroups) ? p.g_scale[b][s.group] : p.scale[b]) + static_cast<int64_t>(blk) * s.kc;
             };
-            // products: the scales of both blocks; otherwise those of this thread's block
-            const float* bs0 = block_scales(kProducts ? 0 : tid & 1);
-            [[maybe_unused]] const float* bs1 = kProducts ? block_scales(1) : nullptr;
+            const float* bs0 = block_scales(kOwn ? lane & 1 : 0);
+            [[maybe_unused]] const float* bs1 = kOwn ? nullptr : block_scales(1);
             for (int k = s.c0; k < s.c1; k += TC, ++t) {
                 const int sl = t & 1;
                 ok = __all_sync(0xffffffffu, bounded_wait(sempty_bar(sl), ((t >> 1) & 1u) ^ 1u, ctl, p.status, 7, t));
                 if (!ok) break;
                 const int n = min(TC, s.c1 - k);
-                float* dst = tab + sl * TC * (kProducts ? 2 * BN : BN);
+                float* dst = tab + sl * TC * 2 * BN;
                 // All loads of a slot are in flight together: they queue behind the weights' (one after the other they held
                 // the first chunk back by 7 us).  Columns beyond ntok keep what they held: they multiply products nobody reads.
                 constexpr int kLoads = TC * BN / kTabThreads;
                 static_assert(kTabThreads % BN == 0 || BN % kTabThreads == 0, "a thread's columns do not depend on the trip");
-                static_assert(2 * TC <= kTabThreads, "one block scale per thread");
+                static_assert(2 * TC <= 32, "one block scale per lane");
                 float r[kLoads], rb[kLoads][2], own = 0.0f;
-                const bool has_own = !kProducts && (tid >> 1) < n;
-                if (has_own) own = __ldg(bs0 + k + (tid >> 1));
+                if (kOwn && (lane >> 1) < n) own = __ldg(bs0 + k + (lane >> 1));
 #pragma unroll
                 for (int u = 0; u < kLoads; ++u) {
                     const int i = tid + u * kTabThreads, ch = i / BN, col = i - ch * BN;
                     if (ch < n && col < s.ntok) {
                         r[u] = __ldg(d.a_s + (s.row0 + col) * d.as_row + (k + ch) * d.as_chunk);
-                        if constexpr (kProducts) {
+                        if constexpr (!kOwn) {
                             rb[u][0] = __ldg(bs0 + k + ch);
                             rb[u][1] = __ldg(bs1 + k + ch);
                         }
@@ -511,16 +503,15 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
 #pragma unroll
                 for (int u = 0; u < kLoads; ++u) {
                     const int i = tid + u * kTabThreads, ch = i / BN, col = i - ch * BN;
+                    if constexpr (kOwn) {
+                        rb[u][0] = __shfl_sync(0xffffffffu, own, 2 * ch);
+                        rb[u][1] = __shfl_sync(0xffffffffu, own, 2 * ch + 1);
+                    }
                     if (ch < n && col < s.ntok) {
-                        if constexpr (kProducts) {
-                            dst[ch * 2 * BN + col] = r[u] * rb[u][0];
-                            dst[ch * 2 * BN + BN + col] = r[u] * rb[u][1];
-                        } else {
-                            dst[i] = r[u];
-                        }
+                        dst[ch * 2 * BN + col] = r[u] * rb[u][0];
+                        dst[ch * 2 * BN + BN + col] = r[u] * rb[u][1];
                     }
                 }
-                if (has_own) btab[sl * TC * 2 + tid] = own;
                 mbar_arrive(sfull_bar(sl));
             }
         }
@@ -548,30 +539,18 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
             }
         };
         // acc += product * (a_s * b_s), the order of the other tcgen05 kernels, so that a tile that is not cut equals theirs bit
-        // for bit.  Where the token scales come as they are, one shared-memory load of them serves both blocks.
-        auto fold_piece = [&](const float* as, float2 bs, int i, const uint32_t (&vv)[2][PW]) {
-            auto add = [&](int b, int j, float2 lo, float2 hi) {
-                acc[b][i][2 * j] = __ffma2_rn(make_float2(__uint_as_float(vv[b][4 * j]), __uint_as_float(vv[b][4 * j + 1])), lo, acc[b][i][2 * j]);
-                acc[b][i][2 * j + 1] = __ffma2_rn(make_float2(__uint_as_float(vv[b][4 * j + 2]), __uint_as_float(vv[b][4 * j + 3])), hi, acc[b][i][2 * j + 1]);
-            };
-            if constexpr (kProducts) {
+        // for bit.  The scale warps form a_s * b_s once per CTA: formed here, by every thread for all of its rows, the
+        // multiplications took as much of the FP32 pipes as the sums (64-token tiles, 256 experts of 7168 x 2048 with 64 tokens
+        // each: 2936 -> 2724 us).
+        auto fold_piece = [&](const float* as, int i, const uint32_t (&vv)[2][PW]) {
 #pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    const float4* as4 = reinterpret_cast<const float4*>(as + b * BN + 2 * PW * i);
-#pragma unroll
-                    for (int j = 0; j < PW / 4; ++j) {
-                        const float4 a4 = as4[j];
-                        add(b, j, make_float2(a4.x, a4.y), make_float2(a4.z, a4.w));
-                    }
-                }
-            } else {
-                const float4* as4 = reinterpret_cast<const float4*>(as + 2 * PW * i);
-                const float2 b2[2] = {make_float2(bs.x, bs.x), make_float2(bs.y, bs.y)};
+            for (int b = 0; b < 2; ++b) {
+                const float4* as4 = reinterpret_cast<const float4*>(as + b * BN + 2 * PW * i);
 #pragma unroll
                 for (int j = 0; j < PW / 4; ++j) {
                     const float4 a4 = as4[j];
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) add(b, j, __fmul2_rn(make_float2(a4.x, a4.y), b2[b]), __fmul2_rn(make_float2(a4.z, a4.w), b2[b]));
+                    acc[b][i][2 * j] = __ffma2_rn(make_float2(__uint_as_float(vv[b][4 * j]), __uint_as_float(vv[b][4 * j + 1])), make_float2(a4.x, a4.y), acc[b][i][2 * j]);
+                    acc[b][i][2 * j + 1] = __ffma2_rn(make_float2(__uint_as_float(vv[b][4 * j + 2]), __uint_as_float(vv[b][4 * j + 3])), make_float2(a4.z, a4.w), acc[b][i][2 * j + 1]);
                 }
             }
         };
@@ -593,9 +572,7 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
                     ok = __all_sync(0xffffffffu, bounded_wait_lean(sfull_bar(sl), (t >> 1) & 1u, ctl, p.status, 8, t));
                     if (!ok) break;
                 }
-                const float* as = tab + (sl * TC + in_tab) * (kProducts ? 2 * BN : BN) + col0;
-                float2 bs = make_float2(0.0f, 0.0f);
-                if constexpr (!kProducts) bs = *reinterpret_cast<const float2*>(btab + (sl * TC + in_tab) * 2);
+                const float* as = tab + (sl * TC + in_tab) * 2 * BN + col0;
                 const int ts = g % NT;
                 ok = __all_sync(0xffffffffu, bounded_wait_lean(tfull_bar(ts), (g / NT) & 1u, ctl, p.status, 4, g));
                 if (!ok) break;
@@ -612,9 +589,9 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
                 }
                 tc_wait_ld();
                 if (NP <= 2 || np <= 2) release();
-                if (np > 0) fold_piece(as, bs, 0, v[0]);
+                if (np > 0) fold_piece(as, 0, v[0]);
                 if constexpr (NP > 1) {
-                    if (np > 1) fold_piece(as, bs, 1, v[1]);
+                    if (np > 1) fold_piece(as, 1, v[1]);
                 }
                 if constexpr (NP > 2) {
                     if (np > 2) {
@@ -622,8 +599,8 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
                         if (np > 3) load_piece(taddr, 3, v[1]);
                         tc_wait_ld();
                         release();
-                        fold_piece(as, bs, 2, v[0]);
-                        if (np > 3) fold_piece(as, bs, 3, v[1]);
+                        fold_piece(as, 2, v[0]);
+                        if (np > 3) fold_piece(as, 3, v[1]);
                     }
                 }
                 if (++in_tab == TC || k == n_ch - 1) {
@@ -807,7 +784,7 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
 template <int BN, bool kSwiglu, bool kBoth>
 __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUtensorMap* tmap_w1, const CUtensorMap* tmap_a0, const CUtensorMap* tmap_a1,
                                            const StreamParams& p) {
-    using C = SCfg<BN, true, false>;
+    using C = SCfg<BN, true>;
     constexpr bool kSplit = false;      // its partial tiles would be 128 KB each
     constexpr int NS = C::kStages, NT = C::kSlots;
     extern __shared__ uint8_t smem_raw[];
@@ -1123,7 +1100,7 @@ int launch(void (*kern)(KArgs...), int64_t grid, int smem, bool (&configured)[64
 template <int BN, bool kSwiglu, bool kBoth, bool kSplit>
 int launch_stream(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, StreamParams prm, int64_t most,
                   cudaStream_t stream) {
-    using C = SCfg<BN, false, scale_products<BN, kSplit>>;
+    using C = SCfg<BN, false>;
     static bool configured[64] = {};
     prm.ctas = static_cast<int>(most < num_sms() ? most : num_sms());
     return launch(fp8_stream_kernel<BN, kSwiglu, kBoth, kSplit>, prm.ctas, C::kSmemBytes, configured, stream, w0, w1, ta0, ta1, prm);
@@ -1132,7 +1109,7 @@ int launch_stream(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMa
 template <bool kSwiglu, bool kBoth>
 int launch_divided(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, StreamParams prm, int64_t most_large,
                    int64_t most_small, int divide, cudaStream_t stream) {
-    constexpr int kLarge = SCfg<128, true, false>::kSmemBytes, kSmall = SCfg<64, false, true>::kSmemBytes;
+    constexpr int kLarge = SCfg<128, true>::kSmemBytes, kSmall = SCfg<64, false>::kSmemBytes;
     static bool configured[64] = {};
     StreamParams small = prm;
     prm.min_rows = divide + 1;
