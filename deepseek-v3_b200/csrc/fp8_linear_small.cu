@@ -365,12 +365,16 @@ int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, cons
     // K splits across the CTAs of a cluster: enough CTAs for two per SM, at least 1.5 chunks per warp
     int csize = 1;
     while (csize < 8 && rowgroups * csize < 2 * num_sms() && prm.kc >= 3 * csize * wk) csize *= 2;
-    // Up to 8 rows, half as many CTAs of eight warps instead, where that leaves no cluster to exchange sums in, or where the
-    // CTAs of four would not all be resident (three per SM; a second round costs as much as the first).  us at 1 / 2 / 4 rows, four
-    // warps / eight: 1536 -> 3072 4.1 / 4.6 / 4.7, 3.8 / 4.5 / 4.6; 2048 -> 2816 4.4 / 5.0 / 5.2, 4.1 / 4.8 / 5.0; 7168 -> 2304 10.5 /
-    // 11.0 / 13.2, 7.4 / 7.6 / 9.0; but, at 1 / 2 rows, 5120 -> 1536 (clusters of four) 5.7 / 6.0, 5.9 / 6.2 and 7168 -> 2048 7.2 / 7.8,
-    // 7.4 / 8.0; and at 16 rows, with twice the accumulators, 1536 -> 3072 8.2, 12.6.  Each CTA then stages twice the K range: a K
-    // too long for that (beyond 24064 without a cluster) stays with four warps.
+    // Up to 8 rows, half as many CTAs of eight warps instead, where that leaves no cluster to exchange sums in, or where clusters of
+    // four-warp CTAs come near to filling the machine: registers admit four such CTAs per SM, 592, of which clusters of four and
+    // eight find room for 568 (cudaOccupancyMaxActiveClusters); beyond, a second round costs as much as the first, and already
+    // from 520 on the last clusters wait for room.  The line, three and a half per SM, is drawn by measurement.  us at 1 / 2 / 4
+    // rows, four warps / eight: no cluster, 1536 -> 3072 4.1 / 4.6 / 4.7, 3.8 / 4.5 / 4.6, 2048 -> 2816 4.4 / 5.0 / 5.2, 4.1 / 4.8 / 5.0;
+    // 7168 -> 2304 (576 CTAs) 10.5 / 10.9 / 13.0, 7.4 / 7.6 / 8.9; 7168 -> 2272 (568) 8.1 / 8.3 / 9.9, 7.4 / 7.5 / 8.8; 7168 -> 1040 (520 in
+    // clusters of eight) 4.9 / 5.2 / 6.4, 4.8 / 5.2 / 5.4; but 5120 -> 2176 (544) 5.97 / 6.00 / 7.38, 6.00 / 6.05 / 7.53, 7168 -> 2048 (512)
+    // 7.0 / 7.2 / 8.6, 7.15 / 7.3 / 8.7, 5120 -> 1536 (384) 5.5 / 5.6 / 6.9, 5.6 / 5.7 / 7.2; and at 16 rows, with twice the
+    // accumulators, 1536 -> 3072 8.2, 12.6.  Each CTA then stages twice the K range: a K too long for that (beyond 24064
+    // without a cluster) stays with four warps.
     const int mt = M <= 8 ? 1 : 2;
     const int tok = 8 * mt;
     auto smem_of = [&](int warps, int ctas) {
