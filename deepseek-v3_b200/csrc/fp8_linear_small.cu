@@ -26,17 +26,14 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "decode_math.cuh"
 #include "gemm_plan.cuh"
-#include "quant_math.cuh"
 
 namespace dsv3 {
 
 namespace {
 
-constexpr int kChunkK = 128;    // K elements (= bytes) per scale block
 constexpr int kRing = 4;        // weight chunks in flight per warp (16 x 16-byte loads per lane)
-constexpr int kRowPad = 64;     // bytes between the staged token rows beyond the K range: the 8 lanes of one
-                                // shared-memory phase (two token rows x four 16-byte pieces) then hit 8 different bank groups
 
 struct SmallParams {
     const uint4* x;          // bf16 [M, K], 8 values per uint4 (quantised here)       -- or nullptr
@@ -50,14 +47,6 @@ struct SmallParams {
     int csize;               // CTAs per cluster (K splits across CTAs)
     int scale_fmt;
 };
-
-__device__ __forceinline__ void mma_e4m3(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 __device__ __forceinline__ void prefetch_l2(const void* ptr) { asm volatile("prefetch.global.L2 [%0];" ::"l"(ptr)); }
 
@@ -153,15 +142,9 @@ __global__ void __launch_bounds__(WR * WK * 32) fp8_linear_small_kernel(const Sm
                 }
 #pragma unroll
                 for (int i = 0; i < kBlocks; ++i) {
-                    float mx = amax8(v[i]);
-                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-                    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-                    const float sc = scale_from_amax(mx, p.scale_fmt);
+                    const float sc = half_warp_scale(v[i], p.scale_fmt);
                     if (m[i] >= 0) {
-                        const uint2 q = (p.scale_fmt == DSV3_SCALE_FMT_FP32) ? quant8<true>(v[i], sc) : quant8<false>(v[i], sc);
-                        *reinterpret_cast<uint2*>(xq_s + m[i] * row_bytes + cl[i] * kChunkK + l16 * 8) = q;
+                        *reinterpret_cast<uint2*>(xq_s + m[i] * row_bytes + cl[i] * kChunkK + l16 * 8) = quantised8(v[i], sc, p.scale_fmt);
                         if (l16 == 0) xs_s[m[i] * cpc + cl[i]] = sc;
                     }
                 }
@@ -227,11 +210,8 @@ __global__ void __launch_bounds__(WR * WK * 32) fp8_linear_small_kernel(const Sm
                     const uint8_t* xr = xq_s + (8 * j + g) * row_bytes + cl * kChunkK + 16 * t;
                     const uint4 f0 = *reinterpret_cast<const uint4*>(xr);
                     const uint4 f1 = *reinterpret_cast<const uint4*>(xr + 64);
-                    float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                    mma_e4m3(part, ring[s][0].x, ring[s][1].x, ring[s][0].y, ring[s][1].y, f0.x, f0.y);
-                    mma_e4m3(part, ring[s][0].z, ring[s][1].z, ring[s][0].w, ring[s][1].w, f0.z, f0.w);
-                    mma_e4m3(part, ring[s][2].x, ring[s][3].x, ring[s][2].y, ring[s][3].y, f1.x, f1.y);
-                    mma_e4m3(part, ring[s][2].z, ring[s][3].z, ring[s][2].w, ring[s][3].w, f1.z, f1.w);
+                    float part[4];
+                    chunk_product(part, ring[s], f0, f1);
                     // part[0..1]: weight row g, tokens 8j+2t, 8j+2t+1; part[2..3]: weight row g+8, same tokens
                     const float as0 = xs_s[(8 * j + 2 * t) * cpc + cl], as1 = xs_s[(8 * j + 2 * t + 1) * cpc + cl];
                     acc[j][0] = fmaf(part[0] * as0, bs, acc[j][0]);

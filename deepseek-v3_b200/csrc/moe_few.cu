@@ -27,18 +27,16 @@
 #include <cuda.h>
 
 #include "common.cuh"
+#include "decode_math.cuh"
 #include "gemm_plan.cuh"
-#include "quant_math.cuh"
 
 namespace dsv3 {
 
 namespace {
 
-constexpr int kChunkK = 128;
 constexpr int kMaxTokens = 8;               // the N side of one mma
 constexpr int kMaxPairs = 64;
 constexpr int kRing = 4;                    // chunks in flight per warp (of each weight)
-constexpr int kRowPad = 64;                 // a shared-memory phase is two token rows of four lanes, 64 bytes each: 8 different bank groups
 constexpr int kUpWarps = 8, kUpThreads = kUpWarps * 32;
 constexpr int kDownWarps = 4, kDownThreads = kDownWarps * 32;
 constexpr int kMaxExperts = kMaxGroupsOfTable;
@@ -83,13 +81,6 @@ struct DownParams {
     int T, n, dim, inter, inter_s, scale_fmt;
 };
 
-__device__ __forceinline__ void mma_e4m3(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile(
-        "mma.sync.aligned.m16n8k32.row.col.f32.e4m3.e4m3.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-
 // One chunk of 16 weight rows: rows g and g + 8 of the lane's quad, bytes 16 t .. of both 64-byte halves.
 struct Frag {
     uint4 v[4];
@@ -105,11 +96,8 @@ struct Frag {
     }
     // acc[0..1]: weight row g, tokens 2t and 2t + 1; acc[2..3]: weight row g + 8
     __device__ __forceinline__ void fold(float (&acc)[4], const uint4& f0, const uint4& f1, float as0, float as1) const {
-        float part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        mma_e4m3(part, v[0].x, v[1].x, v[0].y, v[1].y, f0.x, f0.y);
-        mma_e4m3(part, v[0].z, v[1].z, v[0].w, v[1].w, f0.z, f0.w);
-        mma_e4m3(part, v[2].x, v[3].x, v[2].y, v[3].y, f1.x, f1.y);
-        mma_e4m3(part, v[2].z, v[3].z, v[2].w, v[3].w, f1.z, f1.w);
+        float part[4];
+        chunk_product(part, v, f0, f1);
         acc[0] = fmaf(part[0] * as0, s, acc[0]);
         acc[1] = fmaf(part[1] * as1, s, acc[1]);
         acc[2] = fmaf(part[2] * as0, s, acc[2]);
@@ -144,13 +132,8 @@ __device__ __forceinline__ void quantise_blocks(int blocks, int scale_fmt, Src&&
         for (int u = 0; u < kUnroll; ++u) {
             const int b = b0 + u * kHalves + ((threadIdx.x >> 4) & 1);
             if (b0 + u * kHalves >= blocks) break;                                       // uniform in the warp
-            float m = amax8(v[u]);
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-            const float sc = scale_from_amax(m, scale_fmt);
-            if (b < blocks) dst(b, l16, scale_fmt == DSV3_SCALE_FMT_FP32 ? quant8<true>(v[u], sc) : quant8<false>(v[u], sc), sc);
+            const float sc = half_warp_scale(v[u], scale_fmt);
+            if (b < blocks) dst(b, l16, quantised8(v[u], sc, scale_fmt), sc);
         }
     }
 }
