@@ -47,3 +47,78 @@ def test_weights_are_read_before_the_shared_experts_are_called(world_size, monke
     moe.shared_experts = overwrite
     assert torch.equal(dsv3_b200.grouped_moe_forward(moe, x, world_size=world_size), want)
     assert not torch.equal(want, z)
+
+
+def _close(got, want):
+    err, rms = (got.float() - want.float()).abs(), want.float().pow(2).mean().sqrt()
+    return bool((err <= 2e-2 * (want.float().abs() + rms)).all())               # the bound of test_gpu_moe.py
+
+
+ROUTINGS = [[[0, 1], [2, 3]], [[3, 3], [3, 3]], [[9, 60], [17, 2]], [[10, 11], [12, 13]]]      # all, one, one pair, none of them local
+
+
+def test_replays_of_a_graph_follow_the_routing():
+    import dsv3_b200
+    from test_gpu_few_experts import _pairs_one_by_one
+    moe, x = _layer()
+    weights, indices = torch.ones(2, 2, device="cuda"), torch.tensor(ROUTINGS[0], device="cuda")
+    moe.gate, moe.shared_experts = lambda x: (weights, indices), lambda x: torch.zeros_like(x)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        dsv3_b200.grouped_moe_forward(moe, x)
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        y = dsv3_b200.grouped_moe_forward(moe, x)
+    for step, routing in enumerate(ROUTINGS[1:] + ROUTINGS):
+        indices.copy_(torch.tensor(routing))
+        weights.uniform_(0.2, 1.0)
+        x.normal_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, dsv3_b200.grouped_moe_forward(moe, x)), step
+        assert _close(y, _pairs_one_by_one(moe, x, weights, indices)), step
+    dsv3_b200.check_device_status()
+
+
+@pytest.mark.parametrize("world_size", [1, 2])
+def test_shared_experts_beside_the_two_launches(world_size, monkeypatch):
+    """In the same launches, and behind them where there are several ranks."""
+    import dsv3_b200
+    from test_gpu_few_experts import _pairs_one_by_one
+    from test_gpu_moe_calls import _host
+    monkeypatch.setattr(torch.distributed, "all_reduce", lambda y: y.mul_(2))
+    moe, x = _host()
+    x = x[:1]
+    weights, indices = torch.tensor([[0.3, 0.7]], device="cuda"), torch.tensor([[3, 1]], device="cuda")
+    moe.gate = lambda x: (weights, indices)
+    want = _pairs_one_by_one(moe, x, weights, indices) * world_size + moe.shared_experts(x)
+    for _ in range(2):
+        assert _close(dsv3_b200.grouped_moe_forward(moe, x, world_size=world_size), want)
+
+
+def test_two_threads():
+    """Layers of different sizes, each thread on a stream of its own."""
+    import threading
+    import dsv3_b200
+    calls, wrong = [], []
+    for tokens, dim, inter in ((2, 512, 256), (1, 2048, 384)):
+        moe, x = _layer(tokens=tokens, dim=dim, inter=inter)
+        moe.shared_experts = lambda x: torch.zeros_like(x)
+        routing = torch.rand(tokens, 2, device="cuda"), torch.tensor(ROUTINGS[0][:tokens], device="cuda")
+        moe.gate = lambda x, routing=routing: routing
+        calls.append((moe, x, dsv3_b200.grouped_moe_forward(moe, x)))
+    torch.cuda.synchronize()
+
+    def repeat(moe, x, want):
+        torch.set_default_dtype(torch.bfloat16)
+        with torch.cuda.stream(torch.cuda.Stream()):
+            wrong.append(torch.stack([(dsv3_b200.grouped_moe_forward(moe, x) != want).any() for _ in range(200)]).any())
+            torch.cuda.current_stream().synchronize()
+
+    threads = [threading.Thread(target=repeat, args=c) for c in calls]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert len(wrong) == 2 and not any(bool(w) for w in wrong)
