@@ -1124,15 +1124,18 @@ int launch_divided(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorM
 }  // namespace
 
 // Token tile for an expected load per group.  Uneven routing puts some groups above the expectation; a group that needs
-// a second tile reads its weights a second time (from L2).  Weights on the M side cost only the tokens that are there, so
-// 16 to 64 differ by a few per cent (B200, us, tile 16 / 32 / 64: 2.5 tokens per expert 137 / 139 / 142, 26 tokens
-// 964 / 792 / 784, 31 tokens of a small layer 198 / 184 / 191).  Above 40 tokens the groups are divided between two kinds:
-// those of more than 64 rows in tiles of 128 with tokens on the M side, which read the weights once for 128 tokens, the others in
-// tiles of 64 with the weights there, which multiply no empty rows: an expert layer at these sizes runs at the board's power
-// limit, and half of the experts of an unevenly routed layer have fewer than half of the mean.  us, one kind of tile for all groups
-// (128; 64 from 24 to 44 tokens) / divided: 256 experts of 7168 x 2048, 25 tokens each 2055 / 2010, 32 2126 / 2117, 44 2430 / 2275,
-// 64 2555 / 2339, 128 3586 / 3426; 160 of 5120 x 1536, 26 tokens 744 / 760, 41 873 / 854, 75 1085 / 1005; 64 of 2048 x 1408,
-// 31 tokens 142 / 142, 42 156 / 158, 66 199 / 195, 94 226 / 220.
+// a second tile reads its weights a second time (from L2).  Weights on the M side cost only the tokens that are there.  B200, us,
+// tile 16 / 32 / 64, one layer: 256 experts of 7168 x 2048 at 2.5 tokens per expert 1253 / 1252 / 1228, 16 1838 / 1813 / 1712, 26
+// 2172 / 1912 / 1819; 160 of 5120 x 1536 at 19 733 / 667 / 620, 26 747 / 662 / 649; 64 of 2048 x 1408 at 21 134 / 127 / 129, 31 169 /
+// 141 / 143.  Where tiles are cut, narrow ones park and add less: 20 of 160 experts of 5120 x 1536 at 0.3, 0.9 and
+// 4.5 tokens 41 / 43 / 45, 52 / 54 / 58, 86 / 88 / 97, 16 of 64 of 2048 x 1408 at 5.6 and 11 46 / 49 / 53, 47 / 50 / 56.  The lines at 4 and 24
+// are drawn between the two: with many large experts 64 is ahead below them, with few cut ones 16 above.  Above 40 tokens the groups are divided between two
+// kinds: those of more than 64 rows in tiles of 128 with tokens on the M side, which read the weights once for 128 tokens, the
+// others in tiles of 64 with the weights there, which multiply no empty rows: an expert layer at these sizes runs at the
+// board's power limit, and half of the experts of an unevenly routed layer have fewer than half of the mean.  us, tiles of 64
+// for all groups / divided: 256 experts of 7168 x 2048, 25 tokens each 1822 / 1826, 32 1858 / 1873, 38 1898 / 1924, 44 2034 / 1974, 64
+// 2456 / 2263; 160 of 5120 x 1536, 34 tokens 699 / 721, 41 722 / 743, 75 962 / 916; 64 of 2048 x 1408, 31 tokens 141 / 144, 38 140 /
+// 139, 42 146 / 143, 66 183 / 181.  Tiles of 128 for all groups, 64 tokens of 7168 x 2048: 2555.
 constexpr int kDivide = 64;
 static_assert(kDivide <= 64, "one tile of stream_tiles<64>");
 int stream_tile(int64_t rows_per_group) {

@@ -13,8 +13,8 @@
 //     item's loads are issued while the present one is summed up.  Every CTA sorts the (token, expert) pairs and
 //     quantises the tokens itself, under its first weight loads.
 //   * down: a CTA owns 16 columns of the result and walks over the experts in ascending order, so the weighted bf16 sums
-//     of a token (model.py:689) stay in a register; it quantises the rows of h it needs.  dim / 16 CTAs of four warps, all
-//     resident at once.
+//     of a token (model.py:689) stay in a register; it quantises the rows of h it needs.  dim / 16 CTAs of four warps, four to an SM:
+//     resident at once up to 9472 columns and experts 5900 wide, in several rounds beyond.
 //   * while `up` sums its last item and `down` is being started HBM would be idle; each CTA asks the L2 for its share of the
 //     touched w2 instead.
 // B200, one token, one layer of 7168 x 2048 with 32 of 256 experts local, top-8, and an eighth of the shared expert, replayed from
@@ -514,9 +514,11 @@ extern "C" {
 int dsv3_few_experts_pay(int64_t T, int topk, int n_local, int64_t n_routed, int64_t dim, int64_t inter, int64_t inter_shared) {
     // Up to two local pairs on average.  Both launches walk over the experts one after the other and lose time at every one of
     // them, and the rows of more tokens take L1 from the weight streams; the tiles of fp8_stream.cu stream many experts at the
-    // copy rate but cost 25 us around that.  B200, us, one layer replayed from a graph with cold weights, here / in four
-    // launches, by expected pairs: 7168 x 2048, 32 of 256 experts: 1 16.4 / 29.6, 2 35 / 43, 4 43 / 45, 6 50 / 48; all 256: 8 87 / 84.
-    // 5120 x 1536, 20 of 160: 0.75 24 / 35, 1.5 30 / 37, 3 50 / 45.  2048 x 1408, 16 of 64: 1.5 21 / 31, 3 24 / 31, 6 42 / 35.
+    // copy rate but cost 25 us around that.  B200, us, layers with cold weights and unlike routing replayed from a graph (mean), here
+    // / in four launches, by expected pairs: 7168 x 2048, 32 of 256 experts: 1 18.5 / 29.6, 2 21.9 / 33.7, 3 26.0 / 37.3, 4 30.6 / 39.3, 6
+    // 49.0 / 48.7; all 256: 8 82 / 80.  5120 x 1536, 20 of 160: 0.75 15.0 / 28.3, 1.5 22.2 / 32.1, 3 30.7 / 35.0.  2048 x 1408, 16 of 64:
+    // 1.5 15.1 / 28.7, 3 21.6 / 28.5, 6 32.2 / 29.0.  On average the two launches are ahead up to four pairs; a step with more
+    // touched experts than that loses, and with two expected such steps are rare.
     // Not under an SM budget: `down` is one small CTA per 16 columns, which spread over all SMs.
     if (!supported(T, topk, n_local, dim, inter, inter_shared) || sm_budget_set()) return 0;
     return T * topk * n_local <= 2 * (n_routed > n_local ? n_routed : n_local);

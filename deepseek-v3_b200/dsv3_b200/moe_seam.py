@@ -5,8 +5,9 @@ expert costs two host synchronisations (``bincount(...).tolist()``, ``torch.wher
 small launches.  ``grouped_moe_forward`` keeps inputs, outputs and arithmetic (same quantisation per
 token row, same bf16 rounding points, same ascending-expert accumulation order) but runs in
 four launches: routing bookkeeping with the quantisation of the tokens, w1 and w3 of all local experts with SwiGLU and
-the quantisation in front of w2, w2 of all local experts, and the weighted sum with the shared experts' output; or, where few pairs are expected, two (w1 and
-w3 with everything in front of them, w2 with the weighted sum).  Nothing is read back to the host.
+the quantisation in front of w2, w2 of all local experts, and the weighted sum with the shared experts' output; or, where
+few pairs are expected, two (w1 and w3 with everything in front of them, w2 with the weighted sum).  Nothing is read back
+to the host.
 
     import model, dsv3_b200
     dsv3_b200.install_moe(model)        # model.MoE.forward = grouped_moe_forward
@@ -25,9 +26,9 @@ from .ops import _stream
 
 # Up to this many tokens the shared experts are worked on in the routed experts' launches, which saves three to four
 # launches of 3-8 us; their tiles take the routed experts' token width, so with many tokens their own GEMMs use the machine
-# better.  B200, us, inline / separate, at 16, 64, 150, 333, 512 and 700 tokens: 64 experts of 2048 x 1408 92 / 107, 110 / 127,
-# 122 / 141, 144 / 159, 162 / 185, 181 / 194; 160 of 5120 x 1536 249 / 259, 424 / 433, 543 / 560, 605 / 603, 676 / 661, 658 / 645; 256 of
-# 7168 x 2048 623 / 643, 1088 / 1114, 1440 / 1453, 1668 / 1660, 1817 / 1809, 1958 / 1979.
+# better.  B200, us, inline / separate, at 16, 64, 150, 333, 512 and 700 tokens: 64 experts of 2048 x 1408 82 / 95, 106 / 123,
+# 119 / 138, 140 / 155, 153 / 174, 171 / 182; 160 of 5120 x 1536 226 / 240, 440 / 460, 543 / 558, 616 / 609, 657 / 649, 649 / 654; 256 of
+# 7168 x 2048 561 / 580, 1188 / 1210, 1460 / 1477, 1633 / 1636, 1812 / 1791, 1930 / 1897.
 SHARED_INLINE_MAX_ROWS = 512
 
 
