@@ -126,6 +126,13 @@ struct Seg {          // a range of K chunks of one tile
 // The CTA's share of the work; every CTA derives the same plan from the same numbers.  The tiles (the groups' first, then
 // the ordinary weight's) are worked on whole, one after the other per CTA, or (kSplit) where that would leave the machine
 // idle in the last of one or two rounds, the (tile, K chunk) space is cut into equal contiguous ranges, one per CTA.
+// Whole tiles of the ordinary weight are spread evenly among the groups': the ordinary weight is read once and multiplied by
+// many tokens, so its tiles keep the tensor core busy and HBM idle while the groups' do the opposite, and side by side on
+// different SMs they share the machine.  Their distance has no factor in common with the number of CTAs, or they would all be
+// the same few CTAs'.  us, ordinary weight last / spread: 32 of 256 experts of 7168 x 2048 with the shared one, 200 tokens
+// 227.7 / 212.4, 333 253.4 / 231.5, 512 307 / 279; 64 of 2048 x 1408 with two, 333 tokens 140.2 / 133.5; 160 of 5120 x 1536 with two, 512
+// 672 / 629.  Where the ordinary weight has more tiles than the groups they stay last (8 of 64 experts of 2048 x 1408, 512
+// tokens: 59.8 last, 62.2 first): the groups' tiles wait for HBM and are better begun early.
 // (Cutting only the tiles of the last round was slower: each then has about ten parts, which one CTA adds up while the
 // others wait for it.  So was cutting a problem of more rounds: 14 rounds of 40 chunks took 380 us whole, 476 cut.)
 // A unit is one K chunk of a tile.  32-bit arithmetic throughout (the host checks that the units fit): a 64-bit division
@@ -133,6 +140,7 @@ struct Seg {          // a range of K chunks of one tile
 struct Plan {
     int kc0, kc1;            // K chunks: groups, ordinary weight
     int tiles0, tiles1;      // groups, ordinary weight
+    int every;               // whole tiles: every so-manieth is one of the ordinary weight while there are any (0: they come last)
     int G;                   // CTAs that take a range
     int units, base, extra;  // the first `extra` CTAs take base + 1 units, the others base
     __device__ __forceinline__ int begin(int cta) const { return cta * base + min(cta, extra); }
@@ -142,6 +150,15 @@ struct Plan {
                         : extra + static_cast<int>(static_cast<unsigned>(u - head) / static_cast<unsigned>(base));
     }
 };
+
+__device__ __forceinline__ bool coprime(int a, int b) {
+    while (b != 0) {
+        const int r = static_cast<int>(static_cast<unsigned>(a) % static_cast<unsigned>(b));
+        a = b;
+        b = r;
+    }
+    return a == 1;
+}
 
 // group_tiles: token tiles over all groups
 template <int BN, bool kBoth, bool kSplit>
@@ -153,7 +170,14 @@ __device__ __forceinline__ Plan make_plan(const StreamParams& p, int group_tiles
     pl.kc1 = p.side[kOrdinary].kc;
     pl.units = pl.tiles0 * pl.kc0 + pl.tiles1 * pl.kc1;
     pl.G = pl.base = pl.extra = 0;
+    pl.every = 0;
     const int ctas = p.ctas;
+    if constexpr (kBoth && !kSplit) {
+        if (pl.tiles1 > 0 && pl.tiles0 >= pl.tiles1) {
+            pl.every = static_cast<int>(static_cast<unsigned>(pl.tiles0 + pl.tiles1) / static_cast<unsigned>(pl.tiles1));
+            while (!coprime(pl.every, ctas)) --pl.every;
+        }
+    }
     const int rounds = static_cast<int>(static_cast<unsigned>(pl.tiles0) / static_cast<unsigned>(ctas));
     const int rest0 = pl.tiles0 - rounds * ctas;
     if constexpr (!kSplit) return pl;
@@ -201,9 +225,15 @@ struct Walker {
             u += s.c1 - s.c0;
         } else {
             if ((kSplit && pl.G > 0) || tile >= pl.tiles0 + pl.tiles1) return false;
-            s.side = !kBoth || tile < pl.tiles0 ? kGroups : kOrdinary;
+            if (kBoth && !kSplit && pl.every > 0) {
+                const int j = static_cast<int>(static_cast<unsigned>(tile) / static_cast<unsigned>(pl.every));
+                s.side = j < pl.tiles1 && j * pl.every == tile ? kOrdinary : kGroups;
+                at = s.side == kOrdinary ? j : tile - min(pl.tiles1, j + 1);
+            } else {
+                s.side = !kBoth || tile < pl.tiles0 ? kGroups : kOrdinary;
+                at = (!kBoth || s.side == kGroups) ? tile : tile - pl.tiles0;
+            }
             s.kc = (!kBoth || s.side == kGroups) ? pl.kc0 : pl.kc1;
-            at = (!kBoth || s.side == kGroups) ? tile : tile - pl.tiles0;
             s.ut = 0;
             s.c0 = 0;
             s.c1 = s.kc;

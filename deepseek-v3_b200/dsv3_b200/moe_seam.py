@@ -30,6 +30,21 @@ from .ops import _stream
 # 119 / 138, 140 / 155, 153 / 174, 171 / 182; 160 of 5120 x 1536 226 / 240, 440 / 460, 543 / 558, 616 / 609, 657 / 649, 649 / 654; 256 of
 # 7168 x 2048 561 / 580, 1188 / 1210, 1460 / 1477, 1633 / 1636, 1812 / 1791, 1930 / 1897.
 SHARED_INLINE_MAX_ROWS = 512
+# With more tokens they still are where the routed experts' launches have tiles of 128 tokens (more than 40 pairs per expert on
+# average) and little enough to read that launches, last rounds and the SwiGLU pass of a separate MLP weigh.  At 1024, 1500 and
+# 2048 tokens, inline / separate: 64 experts of 2048 x 1408 198 / 214, 255 / 262, 306 / 319; 8 of those 64 72 / 92, 97 / 115, 102 / 128; 20 of 160 of
+# 5120 x 1536 (64-token tiles) 232 / 202, 217 / 222, 261 / 274; 32 of 256 of 7168 x 2048 (64-token tiles) 357 / 350, 410 / 427, 474 / 478; but
+# 160 of 5120 x 1536 (64-token tiles) 751 / 734, 838 / 839, 983 / 978, 256 of 7168 x 2048 2326 / 2295 at 2048, and at 4096 32 of those
+# 256 765 / 747: those draw the board's full power either way, and pairs of SMs multiply with fewer operand bytes.
+SHARED_INLINE_MAX_ROWS_SMALL = 2048
+SHARED_INLINE_MAX_BYTES_SMALL = 1500 << 20      # of the local experts' weights
+
+
+def _shared_inline(st, rows: int, topk: int, n_routed: int) -> bool:
+    if rows <= SHARED_INLINE_MAX_ROWS:
+        return True
+    return (rows <= SHARED_INLINE_MAX_ROWS_SMALL and rows * topk > 40 * max(n_routed, st.n)
+            and 3 * st.n * st.inter * st.dim <= SHARED_INLINE_MAX_BYTES_SMALL)
 
 
 def _look_up(obj, name):
@@ -148,7 +163,7 @@ def grouped_moe_forward(self, x: torch.Tensor, *, world_size: int = 1, fallback=
     st = _grouped(self)
     n_routed = getattr(self, "n_routed_experts", 0)
     shared = None
-    if world_size == 1 and 0 < indices.numel() and x.size(0) <= SHARED_INLINE_MAX_ROWS:     # (no pairs: no launch to join)
+    if world_size == 1 and 0 < indices.numel() and _shared_inline(st, x.size(0), indices.size(-1), n_routed):     # (no pairs: no launch to join)
         shared = plain_weights(self.shared_experts, x, st.scale_fmt)
     routed = st.run(x, weights, indices, n_routed, shared)
     if shared is not None:
