@@ -16,11 +16,31 @@ constexpr int kThreads = 256;
 // partial sum rounded to bf16 (the arithmetic of `y[idx] += ...` on bf16 tensors); with z, y + z follows (model.py:693).
 //   pos [T, topk] int32: row of `o` holding expert output for the j-th smallest expert id of token t, or -1
 //   w   [T, topk] bf16 : routing weight of that pair
-// Bound by HBM: 2 dim (topk + 1 or 2) bytes per token.  The rows of up to eight experts are requested before the first
-// is used; with one load in flight per thread the same pass ran at 3.3 TB/s (79 us for 2048 tokens, top-8, dim 7168).
-constexpr int kCombineBatch = 8;
+// Bound by HBM: 2 dim (local pairs + 1 or 2 per token) bytes, and by what a CTA spends besides: its look-up of the token's rows and the
+// wait for them behind it, where a rank owns a few of the experts for one or two rows, and two roundings per value.  So the
+// arithmetic is packed, two values to an instruction (in fp32 with conversions it bound full rows: 4096 tokens, 128 of 256 experts of
+// dim 7168, 89.8 us, so 69.7), and with many tokens a thread takes four 16-byte pieces of a row, two rows at a time: a quarter of the
+// CTAs, and eight loads in flight again where both are there (57.4).  us, before / <1, 6> / <4, 2>: 32 of 256 experts of dim 7168,
+// 4 tokens 3.3 / 2.8 / 3.8, 333 8.1 / 7.4 / 6.3, 4096 66.0 / 61.1 / 35.8; 128 of them, 333 10.8 / 8.4 / 8.8; 20 of 160 of dim 5120, 333
+// 6.1 / 4.7 / 4.8, 4096 43.9 / 32.2 / 20.7; rows of 2048, 64 of 64 experts, make CTAs of 64 threads: 2048 tokens 18.0 / 10.8 / 11.6.  Two
+// pieces and four rows lie in between; a list of the rows of several tokens, worked on side by side, did too.
+constexpr int kCombineManyTokens = 400, kCombineManyDim = 4096;
 
-__global__ void __launch_bounds__(kThreads, 4) moe_combine_kernel(const __nv_bfloat16* __restrict__ o,
+// Two bf16 values to a word, each result rounded once to bf16: what a product or sum formed in fp32 and then rounded gives (a
+// product of two bf16 values is exact in fp32, and a sum that is not lies too far from a tie of bf16 to be rounded twice).
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("add.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
+template <int kPieces, int kCombineBatch>
+__global__ void __launch_bounds__(kThreads, kPieces == 1 ? 5 : 4) moe_combine_kernel(const __nv_bfloat16* __restrict__ o,
                                                                 const int* __restrict__ pos,
                                                                 const __nv_bfloat16* __restrict__ w,
                                                                 const __nv_bfloat16* __restrict__ z,
@@ -29,47 +49,59 @@ __global__ void __launch_bounds__(kThreads, 4) moe_combine_kernel(const __nv_bfl
     griddep_launch_dependents();
     griddep_wait();
     const uint32_t t = fast_div(blockIdx.x, ctas_per_row);
-    const int64_t d = (static_cast<int64_t>(blockIdx.x - t * ctas_per_row.d) * kThreads + threadIdx.x) << 3;   // 8 bf16 = 16 bytes per thread
-    if (d >= dim) return;
-    float acc[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] = 0.0f;
-    const uint4 zv = z ? __ldcs(reinterpret_cast<const uint4*>(z + t * dim + d)) : make_uint4(0u, 0u, 0u, 0u);
     const int* tp = pos + static_cast<int64_t>(t) * topk;
-    const __nv_bfloat16* tw = w + static_cast<int64_t>(t) * topk;
+    const unsigned short* tw = reinterpret_cast<const unsigned short*>(w) + static_cast<int64_t>(t) * topk;
+    // 8 bf16 = 16 bytes per thread and piece
+    const int64_t d = (static_cast<int64_t>(blockIdx.x - t * ctas_per_row.d) * (kPieces * blockDim.x) + threadIdx.x) << 3, step = static_cast<int64_t>(blockDim.x) << 3;
+    bool in[kPieces];
+    uint4 zv[kPieces];
+    uint32_t acc[kPieces][4];
+#pragma unroll
+    for (int q = 0; q < kPieces; ++q) {
+        in[q] = d + q * step < dim;
+        zv[q] = z && in[q] ? __ldcs(reinterpret_cast<const uint4*>(z + t * dim + d + q * step)) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[q][e] = 0u;
+    }
     for (int j0 = 0; j0 < topk; j0 += kCombineBatch) {
         int r[kCombineBatch];
-        uint4 v[kCombineBatch];
+        uint32_t wf[kCombineBatch];
+        uint4 v[kCombineBatch][kPieces];
 #pragma unroll
-        for (int j = 0; j < kCombineBatch; ++j) r[j] = j0 + j < topk ? __ldg(tp + j0 + j) : -1;
-#pragma unroll
-        for (int j = 0; j < kCombineBatch; ++j)
-            if (r[j] >= 0) v[j] = __ldcs(reinterpret_cast<const uint4*>(o + static_cast<int64_t>(r[j]) * dim + d));
+        for (int j = 0; j < kCombineBatch; ++j) {
+            r[j] = j0 + j < topk ? __ldg(tp + j0 + j) : -1;
+            wf[j] = 0x10001u * __ldg(tw + min(j0 + j, topk - 1));
+        }
 #pragma unroll
         for (int j = 0; j < kCombineBatch; ++j) {
             if (r[j] < 0) continue;
-            const float wf = __bfloat162float(tw[j0 + j]);
-            const uint32_t words[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+            const __nv_bfloat16* src = o + static_cast<int64_t>(r[j]) * dim + d;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const float lo = __uint_as_float(words[e] << 16), hi = __uint_as_float(words[e] & 0xFFFF0000u);
-                const float pl = __bfloat162float(__float2bfloat16_rn(lo * wf));       // bf16 product
-                const float ph = __bfloat162float(__float2bfloat16_rn(hi * wf));
-                acc[2 * e] = __bfloat162float(__float2bfloat16_rn(acc[2 * e] + pl));    // bf16 accumulate
-                acc[2 * e + 1] = __bfloat162float(__float2bfloat16_rn(acc[2 * e + 1] + ph));
+            for (int q = 0; q < kPieces; ++q)
+                if (in[q]) v[j][q] = __ldcs(reinterpret_cast<const uint4*>(src + q * step));
+        }
+#pragma unroll
+        for (int j = 0; j < kCombineBatch; ++j) {
+            if (r[j] < 0) continue;
+#pragma unroll
+            for (int q = 0; q < kPieces; ++q) {
+                const uint32_t words[4] = {v[j][q].x, v[j][q].y, v[j][q].z, v[j][q].w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[q][e] = add_bf16x2(acc[q][e], mul_bf16x2(words[e], wf[j]));
             }
         }
     }
-    if (z) {
-        const uint32_t words[4] = {zv.x, zv.y, zv.z, zv.w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            acc[2 * e] += __uint_as_float(words[e] << 16);
-            acc[2 * e + 1] += __uint_as_float(words[e] & 0xFFFF0000u);
+    for (int q = 0; q < kPieces; ++q) {
+        if (!in[q]) continue;
+        if (z) {
+            acc[q][0] = add_bf16x2(acc[q][0], zv[q].x);
+            acc[q][1] = add_bf16x2(acc[q][1], zv[q].y);
+            acc[q][2] = add_bf16x2(acc[q][2], zv[q].z);
+            acc[q][3] = add_bf16x2(acc[q][3], zv[q].w);
         }
+        *reinterpret_cast<uint4*>(y + t * dim + d + q * step) = make_uint4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
     }
-    *reinterpret_cast<uint4*>(y + t * dim + d) = make_uint4(pack_bf16x2(acc[0], acc[1]), pack_bf16x2(acc[2], acc[3]),
-                                                            pack_bf16x2(acc[4], acc[5]), pack_bf16x2(acc[6], acc[7]));
 }
 
 // Everything in front of the expert GEMMs in one launch: groups the (token, expert) pairs by local expert, orders every
@@ -547,13 +579,15 @@ int dsv3_moe_combine_add(const void* o, const int32_t* pos, const void* w, const
         set_last_error("moe_combine: null pointer");
         return DSV3_ERR_INVALID_ARGUMENT;
     }
-    const int64_t per_row = (dim / 8 + kThreads - 1) / kThreads;
+    const bool many = T >= kCombineManyTokens && dim > kCombineManyDim;
+    const int64_t cols = dim / 8, pieces = many ? 4 : 1, per_row = (cols + pieces * kThreads - 1) / (pieces * kThreads);
+    const int threads = static_cast<int>(((cols + pieces * per_row - 1) / (pieces * per_row) + 31) / 32 * 32);
     if (dim % 8 != 0 || reinterpret_cast<uintptr_t>(o) % 16 != 0 || reinterpret_cast<uintptr_t>(y) % 16 != 0 ||
         reinterpret_cast<uintptr_t>(z) % 16 != 0 || T * per_row >= (1ll << 31)) {
         set_last_error("moe_combine: dim must be a multiple of 8 and o, y (and z) 16-byte aligned");
         return DSV3_ERR_UNSUPPORTED;
     }
-    DSV3_CUDA_TRY(launch_dependent(moe_combine_kernel, dim3(static_cast<unsigned>(T * per_row)), dim3(kThreads), 0,
+    DSV3_CUDA_TRY(launch_dependent(many ? moe_combine_kernel<4, 2> : moe_combine_kernel<1, 6>, dim3(static_cast<unsigned>(T * per_row)), dim3(static_cast<unsigned>(threads)), 0,
                                    static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(o), pos,
                                    static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(z),
                                    static_cast<__nv_bfloat16*>(y), topk, dim, make_fast_div(static_cast<uint32_t>(per_row))));
