@@ -108,6 +108,7 @@ struct StreamParams {
     int n_groups;
     int min_rows, max_rows;             // groups with fewer or more rows are not this problem's
     int first_cta, ctas;                // the CTAs of the grid that work on it
+    uint64_t coprime;                   // bit i: i has no factor in common with ctas
     const float* scale[2];              // ordinary weight (its maps are kernel parameters)
     int scale_fmt;
     // split tiles
@@ -151,15 +152,6 @@ struct Plan {
     }
 };
 
-__device__ __forceinline__ bool coprime(int a, int b) {
-    while (b != 0) {
-        const int r = static_cast<int>(static_cast<unsigned>(a) % static_cast<unsigned>(b));
-        a = b;
-        b = r;
-    }
-    return a == 1;
-}
-
 // group_tiles: token tiles over all groups
 template <int BN, bool kBoth, bool kSplit>
 __device__ __forceinline__ Plan make_plan(const StreamParams& p, int group_tiles) {
@@ -174,8 +166,9 @@ __device__ __forceinline__ Plan make_plan(const StreamParams& p, int group_tiles
     const int ctas = p.ctas;
     if constexpr (kBoth && !kSplit) {
         if (pl.tiles1 > 0 && pl.tiles0 >= pl.tiles1) {
-            pl.every = static_cast<int>(static_cast<unsigned>(pl.tiles0 + pl.tiles1) / static_cast<unsigned>(pl.tiles1));
-            while (!coprime(pl.every, ctas)) --pl.every;
+            // (the distances that will do come from the host: looking for one here, by division, cost 0.6 us)
+            const int most = min(63, static_cast<int>(static_cast<unsigned>(pl.tiles0 + pl.tiles1) / static_cast<unsigned>(pl.tiles1)));
+            pl.every = 63 - __clzll(static_cast<long long>(p.coprime & (~0ull >> (63 - most))));
         }
     }
     const int rounds = static_cast<int>(static_cast<unsigned>(pl.tiles0) / static_cast<unsigned>(ctas));
@@ -302,6 +295,17 @@ __device__ __forceinline__ void prefix_groups(const StreamParams& p, int* prefix
         for (int w = 0; w < kMaxGroups / 32; ++w) tot += scan[w];
         prefix[kMaxGroups] = tot;        // groups beyond n_groups hold no tiles
     }
+}
+
+// The groups' tensor maps and scale pointers on their way from HBM into the L2, where a CTA's first loads would otherwise wait for
+// them: the weights of the layers in between have long displaced them.  Each CTA asks for a few lines, while what comes before
+// this kernel is still running (the tables do not change; the L2 is the point of coherence).
+__device__ __forceinline__ void prefetch_tables(const StreamParams& p, int lane, int warp) {
+    if (warp != 3) return;
+    const int lines = p.n_groups + (p.n_groups * 8 + 127) / 128;
+    for (int i = static_cast<int>(blockIdx.x) - p.first_cta + lane * p.ctas; i < lines; i += 32 * p.ctas)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t*>(p.g_map[b]) + i * 128));
 }
 
 // The TMA producer (one converged warp).  Stage: [BN token rows][block 0][block 1] of one K chunk; of the tokens only
@@ -438,6 +442,7 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
     }
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
     griddep_launch_dependents();
+    prefetch_tables(p, lane, warp);
     griddep_wait();
     prefix_groups<BN>(p, prefix, scan, seg, warp, lane);
     tc_fence_before();
@@ -855,6 +860,7 @@ __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUt
     }
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
     griddep_launch_dependents();
+    prefetch_tables(p, lane, warp);
     griddep_wait();
     prefix_groups<BN>(p, prefix, scan, static_cast<int*>(nullptr), warp, lane);
     tc_fence_before();
@@ -1126,6 +1132,14 @@ int launch(void (*kern)(KArgs...), int64_t grid, int smem, bool (&configured)[64
     return DSV3_OK;
 }
 
+uint64_t coprime_with(int n) {
+    uint64_t mask = ~1ull;
+    for (int p : {2, 3, 5, 7, 11, 13, 17, 19, 23, 29, 31, 37, 41, 43, 47, 53, 59, 61})
+        if (n % p == 0)
+            for (int i = p; i < 64; i += p) mask &= ~(1ull << i);
+    return mask;
+}
+
 // most: no more CTAs than there can be work for
 template <int BN, bool kSwiglu, bool kBoth, bool kSplit>
 int launch_stream(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, StreamParams prm, int64_t most,
@@ -1133,6 +1147,7 @@ int launch_stream(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMa
     using C = SCfg<BN, false>;
     static bool configured[64] = {};
     prm.ctas = static_cast<int>(most < num_sms() ? most : num_sms());
+    if (kBoth && !kSplit) prm.coprime = coprime_with(prm.ctas);
     return launch(fp8_stream_kernel<BN, kSwiglu, kBoth, kSplit>, prm.ctas, C::kSmemBytes, configured, stream, w0, w1, ta0, ta1, prm);
 }
 
@@ -1144,6 +1159,7 @@ int launch_divided(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorM
     StreamParams small = prm;
     prm.min_rows = divide + 1;
     prm.ctas = static_cast<int>(most_large < num_sms() ? most_large : num_sms());
+    if (kBoth) prm.coprime = coprime_with(prm.ctas);
     small.max_rows = divide;
     small.first_cta = prm.ctas;
     small.ctas = divide ? static_cast<int>(most_small < num_sms() ? most_small : num_sms()) : 0;
