@@ -8,11 +8,7 @@
 // Bit-exactness contract (what the reference's kernel computes when compiled for a GPU):
 //   amax = max|x| (NaN operands dropped) ; amax = max(amax, 1e-4f)
 //   s = div.full.f32(amax, 448) ; [ue8m0: s = exp2(ceil(log2(s)))]
-//   y = cvt.rn.satfinite.e4m3(div.full.f32(x, s))
-// For the fp32 scale format the quotient is formed as x * rcp.approx.f32(s): on sm_100 this is
-// bit-identical to div.full.f32(x, s) for every bf16 x and every scale a bf16 block maximum can
-// produce (checked exhaustively on a B200: 5.3e8 (amax, x) pairs, no mismatch), and it needs one
-// reciprocal per block instead of one division per element.
+//   y = cvt.rn.satfinite.e4m3(div.full.f32(x, s)), the quotient formed as a product (quant_math.cuh)
 #include "common.cuh"
 #include "quant_math.cuh"
 
@@ -48,20 +44,17 @@ __global__ void __launch_bounds__(kThreads, 4) act_quant128_kernel(const uint4* 
         const int64_t b = b0 + u * (kThreads / 16);
         v[u] = (b < nblk) ? __ldcs(x + b * 16 + lane16) : make_uint4(0, 0, 0, 0);
     }
+    float m[kU], r[kU];
+#pragma unroll
+    for (int u = 0; u < kU; ++u) m[u] = amax8(v[u]);
+    const float sc = block_scales<kU>(m, scale_fmt, r);
 #pragma unroll
     for (int u = 0; u < kU; ++u) {
         const int64_t b = b0 + u * (kThreads / 16);
-        float m = amax8(v[u]);
-        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
-        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
-        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-        const float sc = scale_from_amax(m, scale_fmt);
-        if (b < nblk) {
-            y[b * 16 + lane16] = (scale_fmt == DSV3_SCALE_FMT_FP32) ? quant8<true>(v[u], sc) : quant8<false>(v[u], sc);
-            if (lane16 == 0) s[b] = sc;
-        }
+        if (b < nblk) y[b * 16 + lane16] = quant8(v[u], r[u]);
     }
+    const int64_t b = b0 + own_block<kU>() * (kThreads / 16);
+    if (own_block_writer<kU>() && b < nblk) s[b] = sc;
 }
 
 // Any block size that is a multiple of 8 and at most 1024: one warp per block.
@@ -84,11 +77,11 @@ __global__ void __launch_bounds__(kThreads) act_quant_generic_kernel(const uint4
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        const float sc = scale_from_amax(m, scale_fmt);
+        const float sc = scale_from_amax(m, scale_fmt), r = rcp_approx(sc);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const int g = lane + 32 * i;
-            if (g < groups) y[b * groups + g] = quant8<false>(v[i], sc);
+            if (g < groups) y[b * groups + g] = quant8(v[i], r);
         }
         if (lane == 0) s[b] = sc;
     }
@@ -118,21 +111,20 @@ __global__ void __launch_bounds__(kThreads, 6) swiglu_quant128_kernel(const uint
         va[u] = (blk < nblk) ? __ldcs(a + blk * 16 + lane16) : make_uint4(0, 0, 0, 0);
         vb[u] = (blk < nblk) ? __ldcs(b + blk * 16 + lane16) : make_uint4(0, 0, 0, 0);
     }
+    float m[kSwigluUnroll], r[kSwigluUnroll];
+#pragma unroll
+    for (int u = 0; u < kSwigluUnroll; ++u) {
+        va[u] = swiglu8(va[u], vb[u]);
+        m[u] = amax8(va[u]);
+    }
+    const float sc = block_scales<kSwigluUnroll>(m, scale_fmt, r);
 #pragma unroll
     for (int u = 0; u < kSwigluUnroll; ++u) {
         const int64_t blk = b0 + u * (kThreads / 16);
-        const uint4 h = swiglu8(va[u], vb[u]);
-        float m = amax8(h);
-        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
-        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
-        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-        const float sc = scale_from_amax(m, scale_fmt);
-        if (blk < nblk) {
-            y[blk * 16 + lane16] = (scale_fmt == DSV3_SCALE_FMT_FP32) ? quant8<true>(h, sc) : quant8<false>(h, sc);
-            if (lane16 == 0) s[blk] = sc;
-        }
+        if (blk < nblk) y[blk * 16 + lane16] = quant8(va[u], r[u]);
     }
+    const int64_t blk = b0 + own_block<kSwigluUnroll>() * (kThreads / 16);
+    if (own_block_writer<kSwigluUnroll>() && blk < nblk) s[blk] = sc;
 }
 
 }  // namespace

@@ -37,8 +37,5 @@ __device__ __forceinline__ float half_warp_scale(const uint4& v, int scale_fmt) 
     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
     return scale_from_amax(m, scale_fmt);
 }
-__device__ __forceinline__ uint2 quantised8(const uint4& v, float scale, int scale_fmt) {
-    return scale_fmt == DSV3_SCALE_FMT_FP32 ? quant8<true>(v, scale) : quant8<false>(v, scale);
-}
 
 }  // namespace dsv3

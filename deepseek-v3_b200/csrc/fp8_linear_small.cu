@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(WR * WK * 32) fp8_linear_small_kernel(const Sm
                 for (int i = 0; i < kBlocks; ++i) {
                     const float sc = half_warp_scale(v[i], p.scale_fmt);
                     if (m[i] >= 0) {
-                        *reinterpret_cast<uint2*>(xq_s + m[i] * row_bytes + cl[i] * kChunkK + l16 * 8) = quantised8(v[i], sc, p.scale_fmt);
+                        *reinterpret_cast<uint2*>(xq_s + m[i] * row_bytes + cl[i] * kChunkK + l16 * 8) = quant8(v[i], rcp_approx(sc));
                         if (l16 == 0) xs_s[m[i] * cpc + cl[i]] = sc;
                     }
                 }

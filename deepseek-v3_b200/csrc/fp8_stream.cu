@@ -776,7 +776,7 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
                     if (gt < NP * PW && tk < s.ntok) {
                         const float m = fmaxf(fmaxf(red[tk], red[BN + tk]), fmaxf(red[2 * BN + tk], red[3 * BN + tk]));
                         const float sc = scale_from_amax(m, p.scale_fmt);
-                        red[4 * BN + tk] = p.scale_fmt == DSV3_SCALE_FMT_FP32 ? rcp_approx(sc) : sc;
+                        red[4 * BN + tk] = rcp_approx(sc);
                         d.hs[(static_cast<int64_t>(s.row0) + tk) * d.hs_row + s.p * d.hs_blk] = sc;
                     }
                 }
@@ -791,8 +791,7 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
                         for (int e = 0; e < 4; ++e) {
                             const float lo = bf16_bits_to_float(h1[e] & 0xFFFFu), hi = __uint_as_float(h1[e] & 0xFFFF0000u);
                             const float s0 = sc[2 * e], s1 = sc[2 * e + 1];
-                            const bool mul = p.scale_fmt == DSV3_SCALE_FMT_FP32;
-                            const uint32_t two8 = cvt_e4m3x2(mul ? __fmul_rn(lo, s0) : div_full(lo, s0), mul ? __fmul_rn(hi, s1) : div_full(hi, s1));
+                            const uint32_t two8 = cvt_e4m3x2(__fmul_rn(lo, s0), __fmul_rn(hi, s1));
                             if (2 * e < rem) out[(tk + 2 * e) * d.N] = static_cast<uint8_t>(two8 & 0xFFu);
                             if (2 * e + 1 < rem) out[(tk + 2 * e + 1) * d.N] = static_cast<uint8_t>(two8 >> 8);
                         }
@@ -1070,7 +1069,7 @@ __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUt
                 asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
                 m = fmaxf(m, *reinterpret_cast<const float*>(my_x + slot));
                 if (row < s.ntok) {
-                    const float scale = scale_from_amax(m, p.scale_fmt);
+                    const float scale = scale_from_amax(m, p.scale_fmt), r = rcp_approx(scale);
                     const int64_t tok = static_cast<int64_t>(s.row0) + row;
                     if (grp == 0) d.hs[tok * d.hs_row + s.p * d.hs_blk] = scale;
                     uint4* out = reinterpret_cast<uint4*>(d.hq + tok * d.N + static_cast<int64_t>(s.p) * kPRows + grp * 64);
@@ -1080,14 +1079,7 @@ __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUt
                         const uint4 b = make_uint4(v[4], v[5], v[6], v[7]);
 #pragma unroll
                         for (int e = 0; e < 24; ++e) v[e] = v[e + 8];
-                        uint2 qa, qb;
-                        if (p.scale_fmt == DSV3_SCALE_FMT_FP32) {
-                            qa = quant8<true>(a, scale);
-                            qb = quant8<true>(b, scale);
-                        } else {
-                            qa = quant8<false>(a, scale);
-                            qb = quant8<false>(b, scale);
-                        }
+                        const uint2 qa = quant8(a, r), qb = quant8(b, r);
                         out[c] = make_uint4(qa.x, qa.y, qb.x, qb.y);
                     }
                 }

@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const Dispat
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
             const float sc = scale_from_amax(m, p.scale_fmt);
             if (tl[u] < 0) continue;
-            const uint2 q = (p.scale_fmt == DSV3_SCALE_FMT_FP32) ? quant8<true>(v[u], sc) : quant8<false>(v[u], sc);
+            const uint2 q = quant8(v[u], rcp_approx(sc));
             const int64_t t = t0 + tl[u];
             p.xq[(t * nb + bl[u]) * 16 + lane16] = q;
             if (lane16 == 0) p.xs[t * nb + bl[u]] = sc;

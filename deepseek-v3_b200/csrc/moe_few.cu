@@ -133,7 +133,7 @@ __device__ __forceinline__ void quantise_blocks(int blocks, int scale_fmt, Src&&
             const int b = b0 + u * kHalves + ((threadIdx.x >> 4) & 1);
             if (b0 + u * kHalves >= blocks) break;                                       // uniform in the warp
             const float sc = half_warp_scale(v[u], scale_fmt);
-            if (b < blocks) dst(b, l16, quantised8(v[u], sc, scale_fmt), sc);
+            if (b < blocks) dst(b, l16, quant8(v[u], rcp_approx(sc)), sc);
         }
     }
 }

@@ -4,10 +4,10 @@
 //   amax = max|x| (NaN operands dropped) ; amax = max(amax, 1e-4f)
 //   s = div.full.f32(amax, 448) ; [ue8m0: s = exp2(ceil(log2(s)))]
 //   y = cvt.rn.satfinite.e4m3(div.full.f32(x, s))
-// For the fp32 scale format the quotient is formed as x * rcp.approx.f32(s): on sm_100 this is
-// bit-identical to div.full.f32(x, s) for every bf16 x and every scale a bf16 block maximum can
-// produce (checked exhaustively on a B200: 5.3e8 (amax, x) pairs, no mismatch), and it needs one
-// reciprocal per block instead of one division per element.
+// The quotient is formed as x * rcp.approx.f32(s), one reciprocal per block instead of one division per element.  For the fp32
+// scale format this is bit-identical to div.full.f32(x, s) on sm_100 for every bf16 x and every scale a bf16 block maximum
+// can produce (checked exhaustively on a B200: 5.3e8 (amax, x) pairs, no mismatch).  For ue8m0 both are exact: a scale is a power of
+// two from 2^-22 to 2^120, whose reciprocal rcp.approx gives exactly (every one of them checked on a B200), or infinite.
 #pragma once
 
 #include "common.cuh"
@@ -21,15 +21,17 @@ __device__ __forceinline__ float scale_from_amax(float amax, int scale_fmt) {
     return s;
 }
 
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
+// max|x| of eight bf16 values
 __device__ __forceinline__ float amax8(const uint4& v) {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-    float m = 0.0f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        m = fmaxf(m, fabsf(bf16_bits_to_float(w[i] & 0xFFFFu)));
-        m = fmaxf(m, fabsf(__uint_as_float(w[i] & 0xFFFF0000u)));
-    }
-    return m;
+    // two values to a word; a NaN gives way to the other operand, and a lane of nothing but NaN returns one, which fmaxf drops
+    const uint32_t m = max_bf16x2(max_bf16x2(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu), max_bf16x2(v.z & 0x7FFF7FFFu, v.w & 0x7FFF7FFFu));
+    return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xFFFF0000u));
 }
 
 __device__ __forceinline__ float rcp_approx(float s) {
@@ -38,18 +40,58 @@ __device__ __forceinline__ float rcp_approx(float s) {
     return r;
 }
 
-// kRcp: quotient as x * rcp.approx(s) (fp32 scale format) instead of div.full(x, s).
-template <bool kRcp>
-__device__ __forceinline__ uint2 quant8(const uint4& v, float s) {
+// The scales of a half-warp's kU blocks, whose values lie eight to a lane (m: a lane's maxima).  The lanes share the work out: in the
+// first exchanges each gives away the blocks that it will not finish, so that a lane ends up with one block's maximum (five
+// exchanges for four blocks instead of sixteen) and forms one scale and one reciprocal instead of four (for ue8m0 a logarithm and an
+// exponential each): with a block at a time the passes that are not at the HBM rate were bound by instructions.  B200, us, a block at
+// a time and, for ue8m0, divisions / so: 512 x 7168 3.20 / 2.72, ue8m0 4.36 / 2.84; 1003 x 7168 3.48 / 3.10, 4.70 / 3.25; 4096 x 2048 4.07 / 3.61, 5.31 /
+// 3.77; 16384 x 7168 52.9 / 52.8, 58.4 / 52.8; swiglu_quant 8192 x 18432 133.5 / 126.9, 153.5 / 132.7.  (Where a CTA quantises a few blocks
+// for itself, under the loads of its weights, the exchanges only lengthen the chain: 7168 -> 1536 at one row 5.97 / 6.29; the
+// dispatch of the expert layer, whose rounds of blocks are few, 64 experts and 2048 tokens 12.9 / 13.6.)  Returns the scale of block own_block<kU>(), which the quarter (kU = 4) or half of the lanes hold; r: every
+// block's reciprocal, in all lanes.  All 32 lanes take part.
+template <int kU>
+__device__ __forceinline__ int own_block() {
+    const int lane = threadIdx.x & 31;
+    return kU == 4 ? (lane >> 2) & 3 : (kU == 2 ? (lane >> 3) & 1 : 0);
+}
+template <int kU>
+__device__ __forceinline__ bool own_block_writer() { return (threadIdx.x & (16 / kU - 1)) == 0; }
+template <int kU>
+__device__ __forceinline__ float block_scales(const float (&m)[kU], int scale_fmt, float (&r)[kU]) {
+    static_assert(kU == 1 || kU == 2 || kU == 4, "blocks of a half-warp");
+    const int lane = threadIdx.x & 31;
+    float keep;
+    if constexpr (kU == 4) {
+        const bool hi = lane & 8;
+        const float a = fmaxf(hi ? m[2] : m[0], __shfl_xor_sync(0xffffffffu, hi ? m[0] : m[2], 8));
+        const float b = fmaxf(hi ? m[3] : m[1], __shfl_xor_sync(0xffffffffu, hi ? m[1] : m[3], 8));
+        const bool odd = lane & 4;
+        keep = fmaxf(odd ? b : a, __shfl_xor_sync(0xffffffffu, odd ? a : b, 4));
+    } else if constexpr (kU == 2) {
+        const bool hi = lane & 8;
+        keep = fmaxf(hi ? m[1] : m[0], __shfl_xor_sync(0xffffffffu, hi ? m[0] : m[1], 8));
+        keep = fmaxf(keep, __shfl_xor_sync(0xffffffffu, keep, 4));
+    } else {
+        keep = fmaxf(m[0], __shfl_xor_sync(0xffffffffu, m[0], 8));
+        keep = fmaxf(keep, __shfl_xor_sync(0xffffffffu, keep, 4));
+    }
+    keep = fmaxf(keep, __shfl_xor_sync(0xffffffffu, keep, 2));
+    keep = fmaxf(keep, __shfl_xor_sync(0xffffffffu, keep, 1));
+    const float s = scale_from_amax(keep, scale_fmt);
+    const float mine = rcp_approx(s);
+#pragma unroll
+    for (int u = 0; u < kU; ++u) r[u] = kU == 1 ? mine : __shfl_sync(0xffffffffu, mine, (lane & 16) | (u * (16 / kU)));
+    return s;
+}
+
+// Eight values times the reciprocal of their block's scale.
+__device__ __forceinline__ uint2 quant8(const uint4& v, float r) {
     const uint32_t w[4] = {v.x, v.y, v.z, v.w};
     uint16_t p[4];
-    const float r = kRcp ? rcp_approx(s) : 0.0f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const float xl = bf16_bits_to_float(w[i] & 0xFFFFu), xh = __uint_as_float(w[i] & 0xFFFF0000u);
-        const float lo = kRcp ? __fmul_rn(xl, r) : div_full(xl, s);
-        const float hi = kRcp ? __fmul_rn(xh, r) : div_full(xh, s);
-        p[i] = cvt_e4m3x2(lo, hi);
+        const float2 q = __fmul2_rn(make_float2(bf16_bits_to_float(w[i] & 0xFFFFu), __uint_as_float(w[i] & 0xFFFF0000u)), make_float2(r, r));
+        p[i] = cvt_e4m3x2(q.x, q.y);
     }
     return make_uint2(static_cast<uint32_t>(p[0]) | (static_cast<uint32_t>(p[1]) << 16),
                       static_cast<uint32_t>(p[2]) | (static_cast<uint32_t>(p[3]) << 16));
