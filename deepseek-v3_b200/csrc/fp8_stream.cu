@@ -133,7 +133,9 @@ struct Seg {          // a range of K chunks of one tile
 // the same few CTAs'.  us, ordinary weight last / spread: 32 of 256 experts of 7168 x 2048 with the shared one, 200 tokens
 // 227.7 / 212.4, 333 253.4 / 231.5, 512 307 / 279; 64 of 2048 x 1408 with two, 333 tokens 140.2 / 133.5; 160 of 5120 x 1536 with two, 512
 // 672 / 629.  Where the ordinary weight has more tiles than the groups they stay last (8 of 64 experts of 2048 x 1408, 512
-// tokens: 59.8 last, 62.2 first): the groups' tiles wait for HBM and are better begun early.
+// tokens: 59.8 last, 62.2 first): the groups' tiles wait for HBM and are better begun early.  Short ones (less than half the groups' K:
+// w2 of a tensor-parallel shard of the shared expert) stay last as well, where they fill up the last round: two layers of a decode
+// step, one rank of eight, at 16, 32 and 64 tokens 236.2 / 308.1 / 404.7 spread, 234.1 / 305.9 / 401.1 last.
 // (Cutting only the tiles of the last round was slower: each then has about ten parts, which one CTA adds up while the
 // others wait for it.  So was cutting a problem of more rounds: 14 rounds of 40 chunks took 380 us whole, 476 cut.)
 // A unit is one K chunk of a tile.  32-bit arithmetic throughout (the host checks that the units fit): a 64-bit division
@@ -165,7 +167,7 @@ __device__ __forceinline__ Plan make_plan(const StreamParams& p, int group_tiles
     pl.every = 0;
     const int ctas = p.ctas;
     if constexpr (kBoth && !kSplit) {
-        if (pl.tiles1 > 0 && pl.tiles0 >= pl.tiles1) {
+        if (pl.tiles1 > 0 && pl.tiles0 >= pl.tiles1 && 2 * pl.kc1 >= pl.kc0) {
             // (the distances that will do come from the host: looking for one here, by division, cost 0.6 us)
             const int most = min(63, static_cast<int>(static_cast<unsigned>(pl.tiles0 + pl.tiles1) / static_cast<unsigned>(pl.tiles1)));
             pl.every = 63 - __clzll(static_cast<long long>(p.coprime & (~0ull >> (63 - most))));
