@@ -1038,6 +1038,32 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
                 pl.pair = pl.wide = false;
             }
         }
+        // Up to 256 tokens the weight-major tiles are an alternative, 64 tokens at a time: the weights come from L2 once per token
+        // tile, but a part of a tile is half as large, and so is its exchange: 3.3 + 0.29 per chunk on the scale above.
+        // us, token-major / so: 7168 -> 576 at M = 65, 128, 192, 256 8.8 / 7.4, 9.1 / 7.5, 9.3 / 8.0, 9.6 / 8.8; 7168 -> 1536 at 65, 128, 192 9.4 / 8.75,
+        // 9.9 / 9.2, 10.9 / 10.7, but at 256 11.3 / 13.1; 5120 -> 2304 at 128 10.2 / 9.25; 16384 -> 512 at 128 11.25 / 9.4; 4096 -> 768 at 256 9.1 /
+        // 8.0; 7168 -> 2304 at 96 and 192 10.7 / 10.5, 12.7 / 13.1; unsplit, 2048 -> 7168 at 128 8.4 / 8.7, 16384 -> 7168 at 65 28.8 / 44.6.
+        if (!pl.swap && force_kernel == 0 && M <= 256) {
+            const int64_t swapped = (N + kPRows - 1) / kPRows * ((M + 63) / 64);
+            int taken = 0;
+            for (int sfac = 2; sfac <= kMaxClusterSplits && sfac <= pl.kc; ++sfac) {
+                const int per_item = (pl.kc + sfac - 1) / sfac;
+                if (per_item > scale_tab_chunks(64) || swapped > clusters_resident(dev, sms, true, 64, sfac)) continue;
+                const double t = 3.3 + per_item * 0.29;
+                if (t < best - 1e-9) {
+                    best = t;
+                    taken = sfac;
+                }
+            }
+            if (taken) {
+                pl.swap = pl.cluster = true;
+                pl.pair = pl.wide = false;
+                pl.bn = 64;
+                pl.tiles_p = static_cast<int>((N + kPRows - 1) / kPRows);
+                pl.tiles_q = static_cast<int>((M + 63) / 64);
+                splits = taken;
+            }
+        }
     }
     if (force_split == 0 && (pl.kc + splits - 1) / splits > tab) {
         // the weight-major kernel keeps an item's scales in a shared-memory table: split K until an item fits
