@@ -930,6 +930,18 @@ static int64_t clusters_resident(int dev, int sms, bool swap, int bn, int splits
     return n < budget ? n : budget;
 }
 
+// Microseconds of a launch of weight-major tiles of bn tokens, `chunks` K chunks to each of `ctas` CTAs, that HBM does not bound
+// (B200, a replayed graph; within 0.4 of 60 shapes of 17 to 256 tokens): set-up, chunks, and for tiles cut over a cluster the exchange,
+// which grows with the CTAs that load side by side and, for tiles of 64, with the tokens in them.
+static double small_estimate(int bn, int64_t M, int chunks, int splits, int64_t ctas) {
+    const double n = static_cast<double>(ctas);
+    if (bn == 16) return 2.82 + 0.1875 * chunks + (splits > 1 ? 0.8 + 0.012 * n : 0.0);
+    if (bn == 32) return 3.25 + 0.195 * chunks + (splits > 1 ? 0.2 + 0.0155 * n : 0.0);
+    if (splits == 1) return 4.1 + 0.28 * chunks;
+    const double per_tile = static_cast<double>(M) / static_cast<double>((M + 63) / 64);
+    return 3.6 + 0.26 * chunks + 0.6 + 0.0125 * n + (per_tile > 33.0 ? 0.7 * (per_tile - 33.0) / 31.0 : 0.0);
+}
+
 // Pinned values (dsv3_set_gemm_policy) are honoured or refused (pl.error), never rewritten; the automatic
 // plan adapts freely.
 TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split) {
@@ -950,6 +962,7 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
         pl.tiles_p = static_cast<int>((M + kPRows - 1) / kPRows);
         pl.tiles_q = static_cast<int>((N + 127) / 128);
     }
+    struct { int bn, tiles_q, splits; } chosen = {0, 0, 0};      // narrower token tiles than these
     const int64_t tiles = static_cast<int64_t>(pl.tiles_p) * pl.tiles_q;
     if (tiles * 64 >= (1ll << 31)) {     // the work-item counters are 32-bit (at most 64 splits)
         set_last_error("fp8_gemm: %lld output tiles are more than the work-item counter holds", static_cast<long long>(tiles));
@@ -1038,32 +1051,43 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
                 pl.pair = pl.wide = false;
             }
         }
-        // Up to 256 tokens the weight-major tiles are an alternative, 64 tokens at a time: the weights come from L2 once per token
-        // tile, but a part of a tile is half as large, and so is its exchange: 3.3 + 0.29 per chunk on the scale above.
-        // us, token-major / so: 7168 -> 576 at M = 65, 128, 192, 256 8.8 / 7.4, 9.1 / 7.5, 9.3 / 8.0, 9.6 / 8.8; 7168 -> 1536 at 65, 128, 192 9.4 / 8.75,
-        // 9.9 / 9.2, 10.9 / 10.7, but at 256 11.3 / 13.1; 5120 -> 2304 at 128 10.2 / 9.25; 16384 -> 512 at 128 11.25 / 9.4; 4096 -> 768 at 256 9.1 /
-        // 8.0; 7168 -> 2304 at 96 and 192 10.7 / 10.5, 12.7 / 13.1; unsplit, 2048 -> 7168 at 128 8.4 / 8.7, 16384 -> 7168 at 65 28.8 / 44.6.
-        if (!pl.swap && force_kernel == 0 && M <= 256) {
-            const int64_t swapped = (N + kPRows - 1) / kPRows * ((M + 63) / 64);
-            int taken = 0;
-            for (int sfac = 2; sfac <= kMaxClusterSplits && sfac <= pl.kc; ++sfac) {
-                const int per_item = (pl.kc + sfac - 1) / sfac;
-                if (per_item > scale_tab_chunks(64) || swapped > clusters_resident(dev, sms, true, 64, sfac)) continue;
-                const double t = 3.3 + per_item * 0.29;
-                if (t < best - 1e-9) {
-                    best = t;
-                    taken = sfac;
+        // Narrower token tiles.  Up to 256 tokens and 24 MB of weights a launch is set-up, exchange and a few chunks, and tiles of 16, 32
+        // or 64 tokens with the weights on the M side (the weights then come from L2 once per token tile) have less of each: a narrow
+        // tile's parts are small, and with enough tiles none is cut.  small_estimate() in absolute microseconds, fitted like the above; the
+        // token-major tiles' 2.4 us of launch are added here, and what a cluster loses when many load side by side.
+        // us, one tile as wide as M or token-major tiles / so: 7168 -> 576 at M = 33, 64, 128, 256 6.5 / 6.0, 7.2 / 6.3, 9.1 / 7.1, 9.6 / 8.8; 7168 -> 1536 at
+        // 64, 96, 192 7.7 / 7.35, 9.8 / 8.7, 10.9 / 10.7; 16384 -> 512 at 64, 128 9.2 / 7.8, 11.25 / 9.0; uncut, 2048 -> 7168 at 32, 64 6.5 / 5.8, 8.0 / 6.4,
+        // 512 -> 4096 at 64, 128 5.3 / 3.7, 5.1 / 4.1, 1536 -> 3072 at 128 7.0 / 5.6, 2048 -> 1408 at 256 7.45 / 6.3.  No gain: 7168 -> 2304 at 33
+        // 7.9 / 8.5, 7168 -> 1536 at 256 11.3 / 13.1; with more weights, 16384 -> 7168 at 64 28.5 / 31.7.
+        if (force_kernel == 0 && M > 16 && M <= 256 && N * K <= (24ll << 20)) {
+            const int64_t rows = (N + kPRows - 1) / kPRows;
+            double now = best + 2.4 + (pl.cluster ? 0.017 * (static_cast<double>(tiles * splits) - 72.0) : 0.0);
+            const double margin = pl.swap ? 0.15 : 0.5;     // (what the estimates are apart, of one kernel and of two)
+            if (pl.swap) now = tiles * splits <= sms ? small_estimate(pl.bn, M, (pl.kc + splits - 1) / splits, splits, tiles * splits) : 1e30;
+            for (int bn = 16; bn <= 64; bn *= 2) {
+                const int64_t q = (M + bn - 1) / bn, narrow = rows * q;
+                if (pl.swap && bn >= pl.bn) break;
+                for (int sfac = 1; sfac <= kMaxClusterSplits && sfac <= pl.kc && narrow * sfac <= sms; ++sfac) {
+                    const int per_item = (pl.kc + sfac - 1) / sfac;
+                    if (per_item > scale_tab_chunks(bn) || (sfac > 1 && narrow > clusters_resident(dev, sms, true, bn, sfac))) continue;
+                    const double t = small_estimate(bn, M, per_item, sfac, narrow * sfac);
+                    if (t < now - margin) {
+                        now = t + margin;                   // (once, not against one another)
+                        chosen = {bn, static_cast<int>(q), sfac};
+                    }
                 }
             }
-            if (taken) {
-                pl.swap = pl.cluster = true;
-                pl.pair = pl.wide = false;
-                pl.bn = 64;
-                pl.tiles_p = static_cast<int>((N + kPRows - 1) / kPRows);
-                pl.tiles_q = static_cast<int>((M + 63) / 64);
-                splits = taken;
-            }
         }
+    }
+    if (chosen.bn) {
+        pl.swap = true;
+        pl.pair = pl.wide = false;
+        pl.bn = chosen.bn;
+        pl.tiles_p = static_cast<int>((N + kPRows - 1) / kPRows);
+        pl.tiles_q = chosen.tiles_q;
+        pl.splits = chosen.splits;
+        pl.cluster = chosen.splits > 1;
+        return pl;
     }
     if (force_split == 0 && (pl.kc + splits - 1) / splits > tab) {
         // the weight-major kernel keeps an item's scales in a shared-memory table: split K until an item fits

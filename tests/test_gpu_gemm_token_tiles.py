@@ -1,5 +1,6 @@
-"""65 to 256 tokens on few weight rows, where the automatic plan takes weight-major tiles of 64 tokens split inside clusters: edges of the
-token tiles and of the range, weight tiles cut by N, a K tail, against the CUDA-core kernel; and what the plan asks for stays within reason."""
+"""17 to 256 tokens on few weights, where the automatic plan takes several token tiles of 16, 32 or 64 with the weights on the M side, whole
+or split inside clusters: edges of the token tiles and of the range, weight tiles cut by N, K tails, a K longer than a tile's scale
+table, against the CUDA-core kernel."""
 import pytest
 import torch
 
@@ -9,8 +10,8 @@ from test_gpu_stream import _bf16_default  # noqa: F401
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("M", [65, 127, 128, 129, 193, 256, 257])
-@pytest.mark.parametrize("N,K", [(576, 7168), (1, 8192), (250, 4096 + 48), (1101, 5120)])
+@pytest.mark.parametrize("M", [17, 31, 33, 64, 65, 96, 129, 193, 256, 257])
+@pytest.mark.parametrize("N,K", [(576, 7168), (1, 8192), (250, 4096 + 48), (1101, 5120), (7168, 2048), (4096, 512), (2000, 656), (70, 131072), (300, 24576)])
 def test_token_tiles_against_the_cuda_core_kernel(M, N, K):
     import dsv3_b200
     import kernel
