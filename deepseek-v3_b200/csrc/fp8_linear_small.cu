@@ -336,7 +336,7 @@ int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, cons
     prm.K = static_cast<int>(K);
     prm.kc = static_cast<int>((K + kChunkK - 1) / kChunkK);
     prm.scale_fmt = scale_fmt;
-    // Layout: few weight rows -> a CTA takes one 16-row tile and its four (or eight) warps split K (more CTAs, and every CTA
+    // Layout: few weight rows -> a CTA takes one 16-row tile and its four (eight, sixteen) warps split K (more CTAs, and every CTA
     // quantises only its own K range); many rows -> a CTA takes four row tiles that share the staged activations.
     const bool narrow = N <= 4096;
     const int wr = narrow ? 1 : 4;
@@ -362,7 +362,21 @@ int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, cons
         return align16(static_cast<size_t>(tok) * (cpc * kChunkK + kRowPad)) + static_cast<size_t>(tok) * cpc * 4 +
                align16(static_cast<size_t>(wr) * cpc * 4) + static_cast<size_t>(ctas + warps) * wr * 16 * tok * 4 + 16;
     };
-    if (narrow && M <= 8 && (csize == 2 || (csize > 2 && rowgroups * csize > 7 * num_sms() / 2)) && smem_of(8, csize / 2) <= kMaxSmem) {
+    // Where the row tiles are no more than the SMs and clusters would be of at most four, or no more than twice the SMs and no clusters
+    // are needed, one CTA of sixteen or eight warps per row tile does without the exchange, and quantises the activations
+    // with all of them (registers admit one such CTA per SM, or two).  us at 1 / 2 / 4 rows, before / so: 2048 -> 1408 3.48 / 4.21 / 4.24, 3.18 / 3.34 /
+    // 4.16; 1408 -> 2048 4.21 / 4.13 / 5.47, 2.94 / 3.08 / 3.77; eight warps, 512 -> 4096 3.12 / 3.18 / 3.88, 2.74 / 2.82 / 2.84; 7168 -> 2304 6.61 / 6.84, 6.20 / 6.45; level:
+    // 7168 -> 1536 5.99 / 6.28, 6.06 / 6.34, 5120 -> 1536 5.11 / 5.21, 5.06 / 5.21.  Sixteen warps in clusters of two instead of four in
+    // eight: 7168 -> 576 4.18 / 4.48 / 4.68, 4.32 / 4.99 / 5.25.  With activations that are quantised already only the exchange is gained,
+    // which few chunks, or few CTAs with many, do not pay for: 1408 -> 2048 3.52, 3.09; but 256 -> 2048 2.63, 2.84; 1024 -> 1024 2.85, 3.00; 4096 -> 768 at
+    // eight rows 3.75, 4.05.  (Both kinds of activations take the same layout: their results are the same bit for bit.)
+    const bool pays = prm.kc >= 10 && (prm.kc <= 24 || rowgroups >= 80);
+    if (narrow && M <= 8 && rowgroups <= num_sms() && csize <= 4 && pays && smem_of(16, 1) <= kMaxSmem) {
+        wk = 16;
+        csize = 1;
+    } else if (narrow && M <= 8 && rowgroups <= 2 * num_sms() && rowgroups > num_sms() && csize == 1 && smem_of(8, 1) <= kMaxSmem) {
+        wk = 8;
+    } else if (narrow && M <= 8 && (csize == 2 || (csize > 2 && rowgroups * csize > 7 * num_sms() / 2)) && smem_of(8, csize / 2) <= kMaxSmem) {
         wk = 8;
         csize /= 2;
     }
@@ -375,6 +389,9 @@ int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, cons
     }
     const bool fused = x != nullptr;
 #define DSV3_SMALL_CASE(WR_, WK_, MT_, F_) return launch_variant<WR_, WK_, MT_, F_>(prm, rowgroups, smem, stream)
+    if (wk == 16) {
+        if (fused) DSV3_SMALL_CASE(1, 16, 1, true); else DSV3_SMALL_CASE(1, 16, 1, false);
+    }
     if (wk == 8) {
         if (fused) DSV3_SMALL_CASE(1, 8, 1, true); else DSV3_SMALL_CASE(1, 8, 1, false);
     }
