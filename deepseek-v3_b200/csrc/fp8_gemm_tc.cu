@@ -1051,15 +1051,16 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
                 pl.pair = pl.wide = false;
             }
         }
-        // Narrower token tiles.  Up to 256 tokens and 24 MB of weights a launch is set-up, exchange and a few chunks, and tiles of 16, 32
+        // Narrower token tiles.  From 33 to 256 tokens and up to 24 MB of weights a launch is set-up, exchange and a few chunks, and tiles of 16, 32
         // or 64 tokens with the weights on the M side (the weights then come from L2 once per token tile) have less of each: a narrow
         // tile's parts are small, and with enough tiles none is cut.  small_estimate() in absolute microseconds, fitted like the above; the
         // token-major tiles' 2.4 us of launch are added here, and what a cluster loses when many load side by side.
         // us, one tile as wide as M or token-major tiles / so: 7168 -> 576 at M = 33, 64, 128, 256 6.5 / 6.0, 7.2 / 6.3, 9.1 / 7.1, 9.6 / 8.8; 7168 -> 1536 at
-        // 64, 96, 192 7.7 / 7.35, 9.8 / 8.7, 10.9 / 10.7; 16384 -> 512 at 64, 128 9.2 / 7.8, 11.25 / 9.0; uncut, 2048 -> 7168 at 32, 64 6.5 / 5.8, 8.0 / 6.4,
+        // 64, 96, 192 7.7 / 7.35, 9.8 / 8.7, 10.9 / 10.7; 16384 -> 512 at 64, 128 9.2 / 7.8, 11.25 / 9.0; uncut, 2048 -> 7168 at 64 8.0 / 6.4,
         // 512 -> 4096 at 64, 128 5.3 / 3.7, 5.1 / 4.1, 1536 -> 3072 at 128 7.0 / 5.6, 2048 -> 1408 at 256 7.45 / 6.3.  No gain: 7168 -> 2304 at 33
-        // 7.9 / 8.5, 7168 -> 1536 at 256 11.3 / 13.1; with more weights, 16384 -> 7168 at 64 28.5 / 31.7.
-        if (force_kernel == 0 && M > 16 && M <= 256 && N * K <= (24ll << 20)) {
+        // 7.9 / 8.5, 7168 -> 1536 at 256 11.3 / 13.1; with more weights, 16384 -> 7168 at 64 28.5 / 31.7.  (Weights in the L2.  From HBM the gain is smaller, and
+        // up to 32 tokens it is a loss: two layers of a decode step, one rank of eight, 32 tokens 303.0 / 307.2, 48 356.3 / 353.2, 64 398.3 / 389.4.)
+        if (force_kernel == 0 && M > 32 && M <= 256 && N * K <= (24ll << 20)) {
             const int64_t rows = (N + kPRows - 1) / kPRows;
             double now = best + 2.4 + (pl.cluster ? 0.017 * (static_cast<double>(tiles * splits) - 72.0) : 0.0);
             const double margin = pl.swap ? 0.15 : 0.5;     // (what the estimates are apart, of one kernel and of two)
