@@ -1182,8 +1182,8 @@ int stream_tile(int64_t rows_per_group) {
     return rows_per_group <= 4 ? 16 : (rows_per_group <= 24 ? 32 : (rows_per_group <= 40 ? 64 : 128));
 }
 
-size_t stream_workspace_bytes(int64_t rows_per_group) {
-    const int bn = stream_tile(rows_per_group);
+size_t stream_workspace_bytes(int64_t rows_per_group) { return stream_tile_workspace_bytes(stream_tile(rows_per_group)); }
+size_t stream_tile_workspace_bytes(int bn) {
     if (bn > 64) return 0;            // of 128 tokens or divided: never cut
     return DSV3_WORKSPACE_HEADER_BYTES + static_cast<size_t>(num_sms()) * 2 * (2 * bn) * kPRows * sizeof(float);
 }
@@ -1218,18 +1218,21 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
     memset(&ta1, 0, sizeof(ta1));
     int rc;
     const bool ordinary = q.ordinary.rows > 0;
-    const int64_t per_tile = (q.rows_expected + q.n_groups - 1) / q.n_groups;
-    const int bn = stream_tile(per_tile);
+    const int64_t per_tile = q.n_groups > 0 ? (q.rows_expected + q.n_groups - 1) / q.n_groups : q.ordinary.rows;
+    const int bn = q.tile ? q.tile : stream_tile(per_tile);
     int64_t tiles[2] = {0, 0};
-    if ((rc = fill_side(prm.side[kGroups], &ta0, q.groups, q.swiglu, bn)) != DSV3_OK) return rc;
-    for (int b = 0; b < 2; ++b) {
-        const void* tbl = (b == 1 && q.swiglu) ? q.table1 : q.table0;
-        prm.g_map[b] = static_cast<const CUtensorMap*>(tbl);
-        prm.g_scale[b] = table_scales(tbl, q.n_groups);
+    if (q.n_groups > 0) {
+        if ((rc = fill_side(prm.side[kGroups], &ta0, q.groups, q.swiglu, bn)) != DSV3_OK) return rc;
+        for (int b = 0; b < 2; ++b) {
+            const void* tbl = (b == 1 && q.swiglu) ? q.table1 : q.table0;
+            prm.g_map[b] = static_cast<const CUtensorMap*>(tbl);
+            prm.g_scale[b] = table_scales(tbl, q.n_groups);
+        }
+        prm.seg = q.seg;
     }
-    prm.seg = q.seg;
     // token tiles: at most one partly filled tile per group on top of the full ones, and never more groups than rows
-    tiles[0] = (q.groups.rows / bn + (q.n_groups < q.groups.rows ? q.n_groups : q.groups.rows)) * prm.side[kGroups].tiles_p;
+    if (q.n_groups > 0)
+        tiles[0] = (q.groups.rows / bn + (q.n_groups < q.groups.rows ? q.n_groups : q.groups.rows)) * prm.side[kGroups].tiles_p;
     if (ordinary) {
         const StreamSide& d = q.ordinary;
         if ((rc = fill_side(prm.side[kOrdinary], &ta1, d, q.swiglu, bn)) != DSV3_OK) return rc;
@@ -1238,6 +1241,7 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
         prm.scale[0] = q.w0_s;
         prm.scale[1] = q.swiglu ? q.w1_s : q.w0_s;
         tiles[1] = (d.rows + bn - 1) / bn * prm.side[kOrdinary].tiles_p;
+        if (q.n_groups == 0) ta0 = ta1;                       // (a kernel prefetches both)
     }
     prm.n_groups = q.n_groups;
     prm.max_rows = INT32_MAX;
@@ -1245,9 +1249,10 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
     prm.status = status_device_ptr();
     if (!prm.status) return DSV3_ERR_CUDA;
     // cutting tiles is worth considering when one or two rounds of whole tiles are expected (struct Plan)
-    const size_t need = stream_workspace_bytes(per_tile);
+    const size_t need = stream_tile_workspace_bytes(bn);
     const int64_t groups_expected = q.n_groups < q.rows_expected ? q.n_groups : q.rows_expected;
-    const bool split = bn < 128 && groups_expected * prm.side[kGroups].tiles_p < 3 * num_sms() && q.workspace && q.workspace_bytes >= need &&
+    const int64_t tiles_expected = q.n_groups > 0 ? groups_expected * prm.side[kGroups].tiles_p : tiles[1];
+    const bool split = bn < 128 && tiles_expected < 3 * num_sms() && q.workspace && q.workspace_bytes >= need &&
                        (reinterpret_cast<uintptr_t>(q.workspace) % 256) == 0;
     if (split) {
         prm.tickets = static_cast<int*>(q.workspace);

@@ -74,11 +74,13 @@ struct StreamGemm {
     const float *w0_s, *w1_s;
     bool swiglu;
     int scale_fmt;
+    int tile;                          // tokens per tile (16, 32, 64, 128), or 0: by rows_expected
     void* workspace;                   // stream_workspace_bytes(), or null: tiles are not split
     size_t workspace_bytes;
 };
 int stream_tile(int64_t rows_per_group);
 size_t stream_workspace_bytes(int64_t rows_per_group);
+size_t stream_tile_workspace_bytes(int bn);
 int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream);
 
 // Table of the weights of up to 256 groups: tensor maps, scale pointers and weight pointers, in device memory.

@@ -324,6 +324,35 @@ std::pair<at::Tensor, at::Tensor> quantise_remembered(const at::Tensor& x, int64
     return r;
 }
 
+// ------------------------------------------------------------------ an MLP whose Linears are plain
+// w2(swiglu_quant(w1(x), w3(x))) in three launches: the quantisation of x, w1 and w3 with everything in front of w2, w2.
+// Undefined where the separate launches are faster.
+at::Tensor mlp(const at::Tensor& x, const at::Tensor (&w)[3], const at::Tensor (&s)[3], int x_fmt, int h_fmt, bool assume_no_inplace) {
+    const int64_t K = last_dim(x), M = K ? x.numel() / K : 0, N = w[0].size(0);
+    if (w[0].dim() != 2 || w[0].sizes() != w[1].sizes() || w[0].size(1) != K || !dsv3_swiglu_linear_pays(M, N, K)) return {};
+    for (int i = 0; i < 2; ++i) {
+        require(w[i].is_contiguous(), "Input tensors must be contiguous");
+        require(s[i].is_contiguous(), "Scaling factor tensors must be contiguous");
+        if (w[i].element_size() != 1 || s[i].scalar_type() != at::kFloat) raise(PyExc_NotImplementedError, "fp8_gemm takes 1-byte FP8 operands and float32 scales");
+        if (reinterpret_cast<uintptr_t>(w[i].const_data_ptr()) % 16 != 0) return {};        // (the tcgen05 kernels' limit)
+    }
+    require_bf16_default();
+    auto q = quantise_remembered(x, 128, x_fmt, assume_no_inplace);
+    const c10::Device dev = require_cuda(q.first, w[0], s[0], w[1], s[1]);
+    at::Tensor h = new_cuda_last(x, N, at::kFloat8_e4m3fn), hs = new_cuda_last(x, N / 128, at::kFloat);
+    const size_t need = dsv3_swiglu_linear_workspace_bytes(M, N, K);
+    const at::Tensor held = need ? workspace(dev, need) : at::Tensor();
+    void* ws = need ? held.data_ptr() : nullptr;
+    const size_t ws_bytes = need ? static_cast<size_t>(held.numel()) : 0;
+    const void *a = q.first.const_data_ptr(), *p1 = w[0].const_data_ptr(), *p3 = w[1].const_data_ptr();
+    auto f32 = [](const at::Tensor& t) { return static_cast<const float*>(t.const_data_ptr()); };
+    const float *as = f32(q.second), *s1 = f32(s[0]), *s3 = f32(s[1]);
+    void* hp = h.data_ptr();
+    float* hsp = static_cast<float*>(hs.data_ptr());
+    call_library(dev, [&](dsv3_stream_t st) { return dsv3_swiglu_linear(a, as, p1, s1, p3, s3, M, N, K, h_fmt, hp, hsp, ws, ws_bytes, st); });
+    return gemm(h, hs, w[2], s[2]);
+}
+
 // ------------------------------------------------------------------ expert layer
 // Device tables of the local experts' projections and what they depend on.  The tables hold addresses, so before every
 // pass the host must know that the experts are still the ones they were built from.  Looking every weight up through
@@ -626,6 +655,25 @@ PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
     });
 }
 
+// (x, w1, w3, w2, scale_fmt of x, scale_fmt in front of w2, assume_no_inplace) -> y, or None where the separate launches are faster
+PyObject* py_mlp(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    return guarded([&]() -> PyObject* {
+        want_args(n, 7);
+        at::Tensor w[3], s[3];
+        for (int i = 0; i < 3; ++i) {
+            w[i] = tensor_arg(args[1 + i]);
+            PyObject* scale_obj = PyObject_GetAttr(args[1 + i], g_attr_scale);
+            if (!scale_obj) throw PythonError{};
+            if (THPVariable_Check(scale_obj)) s[i] = THPVariable_Unpack(scale_obj);
+            Py_DECREF(scale_obj);
+            if (!s[i].defined()) raise(PyExc_TypeError, "weight.scale is not a tensor");
+        }
+        at::Tensor y = mlp(tensor_arg(args[0]), w, s, scale_fmt_arg(args[4]), scale_fmt_arg(args[5]), PyObject_IsTrue(args[6]) == 1);
+        if (!y.defined()) Py_RETURN_NONE;
+        return wrap(std::move(y));
+    });
+}
+
 // (x, block_size, scale_fmt, assume_no_inplace) -> (y, s), remembered
 PyObject* py_quantise_remembered(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
@@ -771,6 +819,7 @@ PyMethodDef methods[] = {
     {"fp8_linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_fp8_linear)), METH_FASTCALL, "(x, weight, scale, scale_fmt)"},
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_linear)), METH_FASTCALL,
      "(x, weight, block_size, scale_fmt, assume_no_inplace, fused_max_rows, fused_max_bytes, fused_max_bytes_3_rows)"},
+    {"mlp", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_mlp)), METH_FASTCALL, "(x, w1, w3, w2, x_fmt, h_fmt, assume_no_inplace)"},
     {"quantise_remembered", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_quantise_remembered)), METH_FASTCALL,
      "(x, block_size, scale_fmt, assume_no_inplace)"},
     {"experts", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_experts)), METH_FASTCALL,

@@ -367,6 +367,34 @@ StreamSide side_of(const void* a, const float* a_s, bool transposed, int64_t row
     return d;
 }
 
+// Tokens per tile for w1 and w3 of an ordinary MLP with SwiGLU and quantisation in one launch, or 0 where two GEMMs and
+// swiglu_quant are as fast.  With enough weight to keep half of the SMs on whole tiles the launch is a stream of weights up to 128
+// tokens; beyond, the pair tiles of the GEMMs multiply better.  With less it is set-up, epilogue and the chunks of a tile, whole
+// (base + chunk * K chunks) or cut over K as the kernel's own plan decides (cut + unit * units), until whole tiles of 128 no longer fit
+// one round.  B200, us in a replayed graph, three launches / one: 7168 -> 18432 at M = 1, 16, 64, 128 47 / 44, 51 / 45, 61 / 48, 61 / 51, 192
+// 72 / 75; 5120 -> 12288 at 64, 128 37 / 29, 40 / 30; 7168 -> 2304 at 1, 16, 64, 256, 1024 15.4 / 12.9, 16.8 / 14.1, 21.0 / 18.0, 30.5 / 25.8,
+// 42.0 / 34.7; 2048 -> 2816 at 64, 192, 512 14.0 / 10.1, 17.6 / 11.8, 21.9 / 16.1; 2048 -> 1408 at 8, 64, 256 8.8 / 9.5, 13.1 / 9.6, 15.3 / 11.6 (and
+// two launches fewer from the host).
+int swiglu_linear_tile(int64_t M, int64_t N, int64_t K) {
+    const int64_t blocks = N / 128, kc = (K + 127) / 128, sms = num_sms();
+    if (2 * blocks >= sms) return M <= 16 ? 16 : (M <= 64 ? 64 : (M <= 128 ? 128 : 0));
+    struct Cost { int tile, alone; double base, chunk, cut, unit; };
+    constexpr Cost kCosts[] = {{16, 7, 4.6, 0.33, 8.9, 0.0030}, {32, 7, 5.8, 0.36, 11.3, 0.0036}, {64, 9, 7.2, 0.46, 17.0, 0.0036}, {128, 0, 7.5, 0.42, 0.0, 0.0}};
+    int best = 0;
+    double least = 1e30;
+    for (const Cost& c : kCosts) {
+        const int64_t tiles = blocks * ((M + c.tile - 1) / c.tile);
+        if (tiles > sms) continue;
+        const bool is_cut = kc * c.alone > 16 * tiles * kc / sms + 48;            // (make_plan in fp8_stream.cu)
+        const double t = is_cut ? c.cut + c.unit * static_cast<double>(tiles * kc) : c.base + c.chunk * static_cast<double>(kc);
+        if (t < least) {
+            least = t;
+            best = c.tile;
+        }
+    }
+    return best;
+}
+
 // The ordinary weight of dsv3_swiglu_gemm_rows / dsv3_fp8_gemm_rows.
 int add_ordinary(StreamGemm& q, const dsv3_side_gemm_t* s) {
     if (!s || s->rows == 0 || s->N == 0) return DSV3_OK;
@@ -500,6 +528,41 @@ int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, 
     q.workspace = workspace;
     q.workspace_bytes = workspace_bytes;
     if ((rc = add_ordinary(q, side)) != DSV3_OK) return rc;
+    return launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
+}
+
+int dsv3_swiglu_linear_pays(int64_t M, int64_t N, int64_t K) {
+    return M > 0 && N > 0 && N % 128 == 0 && K >= 128 && K % 128 == 0 && M < (1ll << 31) && swiglu_linear_tile(M, N, K) > 0;
+}
+
+size_t dsv3_swiglu_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+    const int tile = M > 0 && N > 0 && K > 0 ? swiglu_linear_tile(M, N, K) : 0;
+    return tile ? stream_tile_workspace_bytes(tile) : 0;
+}
+
+int dsv3_swiglu_linear(const void* a, const float* a_s, const void* w1, const float* w1_s, const void* w3, const float* w3_s, int64_t M, int64_t N,
+                       int64_t K, int scale_fmt, void* h, float* h_s, void* workspace, size_t workspace_bytes, dsv3_stream_t stream) {
+    if (M < 0 || N < 0 || K <= 0) {
+        set_last_error("swiglu_linear: negative size");
+        return DSV3_ERR_INVALID_ARGUMENT;
+    }
+    if (scale_fmt != DSV3_SCALE_FMT_FP32 && scale_fmt != DSV3_SCALE_FMT_UE8M0) {
+        set_last_error("swiglu_linear: unknown scale_fmt %d", scale_fmt);
+        return DSV3_ERR_INVALID_ARGUMENT;
+    }
+    if (M == 0 || N == 0) return DSV3_OK;
+    const dsv3_side_gemm_t side = {a, a_s, 0, M, N, K, w1, w1_s, w3, w3_s, h, h_s};
+    StreamGemm q = {};
+    q.swiglu = true;
+    const int rc = add_ordinary(q, &side);
+    if (rc != DSV3_OK) return rc;
+    q.ordinary.hs_row = N / 128;                     // as swiglu_quant writes them
+    q.ordinary.hs_blk = 1;
+    q.scale_fmt = scale_fmt;
+    q.tile = swiglu_linear_tile(M, N, K);
+    if (q.tile == 0) q.tile = 128;
+    q.workspace = workspace;
+    q.workspace_bytes = workspace_bytes;
     return launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
 }
 

@@ -15,6 +15,8 @@ from __future__ import annotations
 import torch
 from torch.nn.modules import module as _nn_module
 
+from . import linear_seam
+from ._lib import host
 from .ops import fp8_gemm, swiglu_quant
 
 
@@ -33,8 +35,11 @@ def mlp_forward(self, x: torch.Tensor, *, model_module, original) -> torch.Tenso
     row_parallel = type(w2).__name__ == "RowParallelLinear"
     # only plain Linear hands its scale_fmt to linear() (model.py:205); the parallel Linears do not (model.py:233, 262)
     scale_fmt = None if (row_parallel or type(w2).__name__ == "ColumnParallelLinear") else getattr(w2, "scale_fmt", None)
-    hq, hs = swiglu_quant(self.w1(x), self.w3(x), scale_fmt)
-    y = fp8_gemm(hq, hs, w2.weight, w2.weight.scale)
+    up = _plain_up(self, model_module)
+    y = host.mlp(x, up[0], up[1], w2.weight, up[2], scale_fmt, linear_seam._assume_no_inplace) if up else None
+    if y is None:
+        hq, hs = swiglu_quant(self.w1(x), self.w3(x), scale_fmt)
+        y = fp8_gemm(hq, hs, w2.weight, w2.weight.scale)
     if row_parallel:
         if model_module.world_size > 1:
             model_module.dist.all_reduce(y)
@@ -43,6 +48,22 @@ def mlp_forward(self, x: torch.Tensor, *, model_module, original) -> torch.Tenso
     elif getattr(w2, "bias", None) is not None:
         y += w2.bias
     return y
+
+
+def _plain_up(mlp, model):
+    """``(w1, w3, scale_fmt)`` where both do nothing but the GEMM, through the installed ``linear``, on equally quantised
+    activations; otherwise None.  The three launches of ``host.mlp`` (the quantisation, w1 and w3 with everything up to w2's
+    quantisation, w2) are then as good as theirs."""
+    if getattr(model, "world_size", 1) != 1 or not getattr(getattr(model, "linear", None), "_dsv3_linear", False):
+        return None
+    if _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:
+        return None
+    w1, w3 = mlp.w1, mlp.w3
+    for lin in (w1, w3):
+        if type(lin).__name__ not in ("Linear", "ColumnParallelLinear") or getattr(lin, "bias", None) is not None or _intercepted(lin):
+            return None
+    fmt = _scale_fmt_of(w1)
+    return (w1.weight, w3.weight, fmt) if _scale_fmt_of(w3) == fmt else None
 
 
 def _scale_fmt_of(lin):

@@ -37,7 +37,7 @@ def test_shared_experts_of_many_tokens(tokens, inline):
     launches = len(_kernels(lambda: dsv3_b200.grouped_moe_forward(moe, x)))
     routing = moe.gate(x)
     gate = len(_kernels(lambda: moe.gate(x)))
-    assert launches - gate == (4 if inline else 8)
+    assert (launches - gate == 4) == inline and launches - gate >= 4
     moe.gate = lambda x: routing
     got = dsv3_b200.grouped_moe_forward(moe, x)
     want, _ = moe.reference_forward(x)
