@@ -944,7 +944,7 @@ static double small_estimate(int bn, int64_t M, int chunks, int splits, int64_t 
 
 // Pinned values (dsv3_set_gemm_policy) are honoured or refused (pl.error), never rewritten; the automatic
 // plan adapts freely.
-TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split) {
+static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split) {
     TcPlan pl;
     pl.error = DSV3_OK;
     pl.pair = false;
@@ -1100,7 +1100,7 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
                 pl.error = DSV3_ERR_UNSUPPORTED;
                 return pl;
             }
-            return tc_plan(M, N, K, 2, 0);   // automatic choice, absurdly long K: token-major tiles instead
+            return work_out_plan(M, N, K, 2, 0);   // automatic choice, absurdly long K: token-major tiles instead
         }
     }
     pl.splits = splits;
@@ -1120,6 +1120,26 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
         pl.wide = force_kernel == 6;
     }
     return pl;
+}
+
+// A plan is asked for twice per call, for the workspace and for the launch, and takes 0.1 to 0.2 us to work out, of calls that keep the
+// host busy for 4.5: a thread remembers the last few by what they depend on, the problem's size and the SMs there are.
+TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split) {
+    if (force_kernel != 0 || force_split != 0) return work_out_plan(M, N, K, force_kernel, force_split);
+    struct Remembered {
+        int64_t M, N, K;
+        int sms;
+        TcPlan plan;
+    };
+    static thread_local Remembered remembered[16] = {};
+    const int sms = num_sms();
+    Remembered& r = remembered[static_cast<uint64_t>(M * 5 + N / 16 * 7 + K / 128 * 3) & 15u];
+    if (r.M != M || r.N != N || r.K != K || r.sms != sms) {
+        const TcPlan plan = work_out_plan(M, N, K, 0, 0);
+        if (plan.error != DSV3_OK) return plan;          // (the message is the call's own)
+        r = {M, N, K, sms, plan};
+    }
+    return r.plan;
 }
 
 size_t tc_workspace_bytes(const TcPlan& pl, int64_t M, int64_t N) {
