@@ -24,27 +24,36 @@ from ._lib import host, lib
 from .mlp_seam import plain_weights
 from .ops import _stream
 
-# Up to this many tokens the shared experts are worked on in the routed experts' launches, which saves three to four
-# launches of 3-8 us; their tiles take the routed experts' token width, so with many tokens their own GEMMs use the machine
-# better.  B200, us, inline / separate, at 16, 64, 150, 333, 512 and 700 tokens: 64 experts of 2048 x 1408 82 / 95, 106 / 123,
-# 119 / 138, 140 / 155, 153 / 174, 171 / 182; 160 of 5120 x 1536 226 / 240, 440 / 460, 543 / 558, 616 / 609, 657 / 649, 649 / 654; 256 of
-# 7168 x 2048 561 / 580, 1188 / 1210, 1460 / 1477, 1633 / 1636, 1812 / 1791, 1930 / 1897.
+# Up to this many tokens the shared experts are worked on in the routed experts' launches, which saves two launches of
+# 3-8 us and their fill and drain; their tiles take the routed experts' token width, so with many tokens their own GEMMs use
+# the machine better.  B200, us, inline / separate, at 64, 150, 333, 512 and 700 tokens: 64 experts of 2048 x 1408 105 / 118,
+# 114 / 129, 135 / 148, 149 / 169, 171 / 178; 160 of 5120 x 1536 427 / 440, 532 / 557, 598 / 620, 650 / 660, 670 / 675; 256 of
+# 7168 x 2048 1136 / 1160, 1418 / 1438, 1640 / 1650, 1765 / 1800, 1930 / 1889; 32 of those 256 186 / 208, 210 / 234, 246 / 275, 296 / 305,
+# 352 / 340.
 SHARED_INLINE_MAX_ROWS = 512
+# On a rank with few of the experts, their narrow tiles read the shared experts' weights from L2 once per 32 tokens or so: when
+# that is more than the local experts' own weights (and than what launches cost, hence the floor) it is what the launch
+# waits for.  Inline / separate at 256, 333 and 512 tokens: 20 of 160 experts of 5120 x 1536 120 / 134, 140 / 134, 169 / 146; 10 of those
+# 105 / 106, 107 / 105, 133 / 118; 8 of 256 of 7168 x 2048 112 / 119, 137 / 135, 146 / 146; 16 of those 152 / 160, 163 / 178,
+# 197 / 193; but 16 of 64 of 2048 x 1408, whose weights are small, 64 / 82, 81 / 91, 68 / 87.
+SHARED_INLINE_REREAD_FLOOR = 400 << 20
 # With more tokens they still are where the routed experts' launches have tiles of 128 tokens (more than 40 pairs per expert on
 # average) and little enough to read that launches, last rounds and the SwiGLU pass of a separate MLP weigh.  At 1024, 1500 and
-# 2048 tokens, inline / separate: 64 experts of 2048 x 1408 198 / 214, 255 / 262, 306 / 319; 8 of those 64 72 / 92, 97 / 115, 102 / 128; 20 of 160 of
-# 5120 x 1536 (64-token tiles) 232 / 202, 217 / 222, 261 / 274; 32 of 256 of 7168 x 2048 (64-token tiles) 357 / 350, 410 / 427, 474 / 478; but
-# 160 of 5120 x 1536 (64-token tiles) 751 / 734, 838 / 839, 983 / 978, 256 of 7168 x 2048 2326 / 2295 at 2048, and at 4096 32 of those
-# 256 765 / 747: those draw the board's full power either way, and pairs of SMs multiply with fewer operand bytes.
+# 2048 tokens, inline / separate: 64 experts of 2048 x 1408 200 / 216, 255 / 258, 308 / 317; 8 of those 64 68 / 90, 89 / 111,
+# 100 / 123; 20 of 160 of 5120 x 1536 (64-token tiles at 1024) 229 / 199, 216 / 224, 261 / 272; 32 of 256 of 7168 x 2048 (64-token
+# tiles at 1024) 370 / 357, 411 / 426, 483 / 483; but 160 of 5120 x 1536 (64-token tiles at 1024) 790 / 768, 876 / 862, 1000 / 1024,
+# 256 of 7168 x 2048 2326 / 2295 at 2048, and at 4096 32 of those 256 765 / 747: those draw the board's full power either way, and
+# pairs of SMs multiply with fewer operand bytes.
 SHARED_INLINE_MAX_ROWS_SMALL = 2048
 SHARED_INLINE_MAX_BYTES_SMALL = 1500 << 20      # of the local experts' weights
 
 
-def _shared_inline(st, rows: int, topk: int, n_routed: int) -> bool:
-    if rows <= SHARED_INLINE_MAX_ROWS:
-        return True
-    return (rows <= SHARED_INLINE_MAX_ROWS_SMALL and rows * topk > 40 * max(n_routed, st.n)
-            and 3 * st.n * st.inter * st.dim <= SHARED_INLINE_MAX_BYTES_SMALL)
+def _shared_inline(st, rows: int, topk: int, n_routed: int, shared_width: int) -> bool:
+    local_bytes = 3 * st.n * st.inter * st.dim
+    if rows * topk <= 40 * max(n_routed, st.n):
+        reread = 3 * shared_width * st.dim * rows // 32
+        return rows <= SHARED_INLINE_MAX_ROWS and reread <= max(local_bytes, SHARED_INLINE_REREAD_FLOOR)
+    return rows <= SHARED_INLINE_MAX_ROWS or rows <= SHARED_INLINE_MAX_ROWS_SMALL and local_bytes <= SHARED_INLINE_MAX_BYTES_SMALL
 
 
 def _look_up(obj, name):
@@ -163,8 +172,10 @@ def grouped_moe_forward(self, x: torch.Tensor, *, world_size: int = 1, fallback=
     st = _grouped(self)
     n_routed = getattr(self, "n_routed_experts", 0)
     shared = None
-    if world_size == 1 and 0 < indices.numel() and _shared_inline(st, x.size(0), indices.size(-1), n_routed):     # (no pairs: no launch to join)
+    if world_size == 1 and 0 < indices.numel() and x.size(0) <= SHARED_INLINE_MAX_ROWS_SMALL:     # (no pairs: no launch to join)
         shared = plain_weights(self.shared_experts, x, st.scale_fmt)
+        if shared is not None and not _shared_inline(st, x.size(0), indices.size(-1), n_routed, shared[0].size(0)):
+            shared = None
     routed = st.run(x, weights, indices, n_routed, shared)
     if shared is not None:
         y = host.combine(routed, None)
