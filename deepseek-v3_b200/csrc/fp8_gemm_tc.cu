@@ -20,7 +20,8 @@
 //                            a TMA store) or park a split-K partial tile
 // Operand roles: P is the 128-row MMA "A" operand, Q the BN-row MMA "B" operand.
 //   kSwap = false : P = 128 tokens of a,  Q = 128 rows of b  (M > 64: "token-major" tiles)
-//   kSwap = true  : P = 128 rows of b,    Q = BN tokens of a (M <= 64: "weight-major", weights stream once)
+//   kSwap = true  : P = 128 rows of b,    Q = BN tokens of a ("weight-major": M <= 64, where weights stream once; up to 256 tokens on
+//                   few weights, in several token tiles, whose smaller parts are exchanged sooner: small_estimate)
 // (producer and issuer warps stay converged; one elected lane issues)
 // Split-K, up to eight splits: the splits of a tile are the CTAs of one cluster, which exchange rows of the partial tile
 // through distributed shared memory and each add a share in split order.  Pinned factors, and more splits: a work item is

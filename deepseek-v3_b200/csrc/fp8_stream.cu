@@ -1,6 +1,7 @@
 // Weight-streaming FP8 GEMM for sm_100a: few tokens per weight, every weight byte read once.  Used for the expert
-// loop of an expert layer (all local experts, and for few rows the shared experts, in one launch per projection); w1 and
-// w3 carry SwiGLU and the quantisation in front of w2 in their epilogue.
+// loop of an expert layer (all local experts, and for few rows the shared experts, in one launch per projection) and, without
+// groups, for w1 and w3 of an MLP whose tiles fit one round (swiglu_linear_tile); w1 and w3 carry SwiGLU and the quantisation in
+// front of w2 in their epilogue.
 //
 // Replaces the per-expert act_quant + fp8_gemm calls of MoE.forward, inference/model.py:683-689 and :633, and
 // `F.silu(w1(x)) * w3(x)` followed by w2's act_quant, model.py:532 and :158-159.
