@@ -172,9 +172,11 @@ def grouped_moe_forward(self, x: torch.Tensor, *, world_size: int = 1, fallback=
     st = _grouped(self)
     n_routed = getattr(self, "n_routed_experts", 0)
     shared = None
-    if world_size == 1 and 0 < indices.numel() and x.size(0) <= SHARED_INLINE_MAX_ROWS_SMALL:     # (no pairs: no launch to join)
+    rows = x.size(0)
+    if world_size == 1 and rows <= SHARED_INLINE_MAX_ROWS_SMALL and 0 < indices.numel():     # (no pairs: no launch to join)
         shared = plain_weights(self.shared_experts, x, st.scale_fmt)
-        if shared is not None and not _shared_inline(st, x.size(0), indices.size(-1), n_routed, shared[0].size(0)):
+        # (up to 64 rows the weights are read twice at most, and the rule costs the host 1 us)
+        if rows > 64 and shared is not None and not _shared_inline(st, rows, indices.size(-1), n_routed, shared[0].size(0)):
             shared = None
     routed = st.run(x, weights, indices, n_routed, shared)
     if shared is not None:
