@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Benchmark of the FP8 GEMM path: the DeepSeek-V3 Linear shape sweep (BASELINE config 2).
+"""Benchmark of the FP8 GEMM path: the DeepSeek-V3 Linear shape sweep.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
@@ -60,7 +60,7 @@ def shard(shape, tp):
 def sweep_rows(world: int, rank: int = 0):
     """Rows of the sweep this rank executes: (name, K, N, kind, needs_all_reduce, counted).
 
-    The global problem set is the same for every world size (BASELINE configs[1]: the 9 full Linear shapes
+    The global problem set is the same for every world size (the 9 full Linear shapes
     and 7 shapes that are already the TP=8 per-rank slice).  With more than one rank it is spread the way the
     reference's tensor parallelism spreads it (model.py:208-267, 636-666):
       * column-parallel: every rank N/ws rows of W; row-parallel: every rank K/ws columns of W, partial
@@ -252,7 +252,7 @@ def run_reference(args):
     val = fl / t / 1e12
     sample = f"M={M} column of the sweep ({len(rows)} shapes), act_quant+fp8_gemm per shape"
     cfg = workload_config(1)
-    cfg["workload"] = (f"bounded sample of BASELINE configs[1]: the M={M} column only ({len(rows)} (K->N) rows), act_quant + fp8_gemm "
+    cfg["workload"] = (f"bounded sample of the sweep: the M={M} column only ({len(rows)} (K->N) rows), act_quant + fp8_gemm "
                        "per shape on the host; the GPU arm reports the same column as `same_sample_as_reference`")
     cfg["m_values"] = [M]
     line = {
@@ -265,7 +265,7 @@ def run_reference(args):
         "e2e": {"value": val, "unit": "TFLOP/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0},
         "gpu_launches": 0,
         "note": "reference = CPU restatement of inference/kernel.py (oracle/dsv3_oracle.c, OpenMP); the Python/Triton "
-                "reference itself cannot travel to the GPU box",
+                "reference is not part of this repository",
     }
     print(json.dumps(line), flush=True)
 
@@ -273,7 +273,7 @@ def run_reference(args):
 def workload_config(world):
     rows = sweep_rows(1)
     return {
-        "workload": "BASELINE configs[1]: fp8_gemm sweep over DeepSeek-V3 Linear shapes (dim 7168), "
+        "workload": "fp8_gemm sweep over DeepSeek-V3 Linear shapes (dim 7168), "
                     f"{len(rows)} (K->N) rows x M in {MS}; activations N(0,1) bf16 -> act_quant, weights N(0,0.02) "
                     "quantised per 128x128 block",
         "shapes": [f"{n}:{k}->{o}" for n, k, o, *_ in rows],
@@ -797,7 +797,7 @@ def run_detail(args):
 
 
 def run_moe_layer(args):
-    """one DeepSeekMoE layer at V3 dims (dim 7168, 256 routed experts of moe_inter 2048,
+    """One DeepSeekMoE layer at V3 dims (dim 7168, 256 routed experts of moe_inter 2048,
     sigmoid gate with bias, 8 groups / 4 kept, top-8, route_scale 2.5, one shared expert), T tokens.
     Routed experts are sharded E/ws per rank and the routed output is all_reduced (model.py:658-666, 691-692).
     Times the reference's expert loop (model.py:683-689, restated on the drop-in operators, with its host
@@ -933,7 +933,7 @@ def run_moe_layer(args):
             "metric": "moe_layer_tokens_per_s", "value": T / (ms_grp * 1e-3), "unit": "tokens/s", "n_gpus": world,
             "steps": args.steps, "warmup": max(2, args.warmup), "ms_per_step": ms_grp, "higher_is_better": True,
             "scaling": "strong", "vs_baseline": None, "dtype": "fp8_e4m3 x fp8_e4m3 -> fp32", "data": "synthetic",
-            "config": {"workload": f"BASELINE configs[2]: DeepSeekMoE layer, dim {dim}, {E} routed experts (inter {inter}) "
+            "config": {"workload": f"DeepSeekMoE layer, dim {dim}, {E} routed experts (inter {inter}) "
                                    f"+ 1 shared, top-{topk}, T={T} tokens, experts sharded {n_local} per rank"},
             "grouped_ms": ms_grp, "expert_loop_ms": ms_loop, "speedup_vs_expert_loop": ms_loop / ms_grp,
             "grouped_tflops": flops / (ms_grp * 1e-3) / 1e12, "agrees_with_expert_loop": ok,
@@ -948,7 +948,7 @@ def run_moe_layer(args):
 
 
 def run_decode_step(args):
-    """BASELINE configs[4] on the GEMM path: one decode step of the 671B-shaped model at tensor parallelism = world.
+    """One decode step of the 671B-shaped model at tensor parallelism = world.
 
     Per layer the Linear sequence of model.py at M = batch rows: MLA wq_a, wq_b, wkv_a, weight_dequant(wkv_b), wo
     (+ all_reduce) (model.py:461-496); layers 0-2 the dense MLP w1, w3, w2 (+ all_reduce) (model.py:500-532); layers
@@ -1193,7 +1193,7 @@ def run_decode_step(args):
             "metric": "decode_tokens_per_s_671B_shapes_gemm_path", "value": first["tokens_per_s"], "unit": "tokens/s",
             "n_gpus": world, "steps": max(3, args.steps), "warmup": 1, "ms_per_step": first["graph_ms"], "higher_is_better": True,
             "scaling": "strong", "vs_baseline": None, "dtype": "fp8_e4m3 x fp8_e4m3 -> fp32", "data": "synthetic",
-            "config": {"workload": f"BASELINE configs[4] on the GEMM path: 61 layers of DeepSeek-V3 671B Linear shapes at TP={tp}"
+            "config": {"workload": f"GEMM path of 61 layers of DeepSeek-V3 671B Linear shapes at TP={tp}"
                                    + (" (one rank's shards on one GPU, no collectives)" if tp != world else "") + ", "
                                    f"one decode step (M = batch rows), {n_inst} distinct instances per layer kind visited in rotation; "
                                    "attention scores, RoPE, norms, embedding and head are not executed",
@@ -1228,10 +1228,10 @@ def main():
                     help="run one problem instead of the sweep (the case ncu captures are taken on)")
     ap.add_argument("--detail", action="store_true", help="per-(shape, M) table instead of the aggregate sweep")
     ap.add_argument("--detail-m", default=None, metavar="M1,M2,...", help="restrict --detail to these M values")
-    ap.add_argument("--moe-layer", action="store_true", help="BASELINE configs[2]: one MoE layer, expert loop vs grouped")
+    ap.add_argument("--moe-layer", action="store_true", help="one MoE layer, expert loop vs grouped")
     ap.add_argument("--moe-tokens", type=int, default=2048)
     ap.add_argument("--moe-experts", type=int, default=256)
-    ap.add_argument("--decode-step", action="store_true", help="BASELINE configs[4] on the GEMM path: one 671B-shaped decode step")
+    ap.add_argument("--decode-step", action="store_true", help="one 671B-shaped decode step")
     ap.add_argument("--decode-batch", default="1,16,64")
     ap.add_argument("--decode-instances", type=int, default=2, help="distinct weight instances per layer kind")
     ap.add_argument("--decode-tp-shapes", type=int, default=0,

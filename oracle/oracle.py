@@ -1,6 +1,6 @@
 """CPU oracle for the FP8 GEMM path of DeepSeek-V3's inference code.
 
-TEST INFRASTRUCTURE ONLY: the checker for the CUDA kernels and the timed CPU
+TEST INFRASTRUCTURE ONLY: what the CUDA kernels are compared with and the timed CPU
 baseline.  Product code must never import this module.
 
 Two independent restatements live here so that they can check each other:
