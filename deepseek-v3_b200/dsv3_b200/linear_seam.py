@@ -64,7 +64,7 @@ def install_linear(model_module, assume_no_inplace: bool = False) -> None:
         return linear(x, weight, bias, scale_fmt, gemm_impl=model_module.gemm_impl,
                       block_size=model_module.block_size)
     _linear.__doc__ = linear.__doc__
-    _linear._dsv3_linear = True
+    _linear._dsv3_linear = _linear        # itself: a wrapper that copies attributes is told from it
     model_module.linear = _linear
 
 

@@ -21,13 +21,12 @@ from torch.nn.modules import module as _nn_module
 from . import linear_seam
 from ._lib import host
 from .ops import fp8_gemm, swiglu_quant
+from .plain import calls_forward, installed_linear, linear_takes_fmt
 
 
 def _fusable(self, x, model_module) -> bool:
-    w2 = self.w2
     return (getattr(model_module, "gemm_impl", "fp8") == "fp8" and getattr(model_module, "block_size", 128) == 128
-            and w2.weight.element_size() == 1 and self.w1.weight.element_size() == 1 and self.w3.weight.element_size() == 1
-            and w2.weight.size(1) % 128 == 0 and x.dtype == torch.bfloat16)
+            and host.fp8_weights(self.w1.weight, self.w3.weight, self.w2.weight) and x.dtype is torch.bfloat16)
 
 
 def mlp_forward(self, x: torch.Tensor, *, model_module, original) -> torch.Tensor:
@@ -53,48 +52,56 @@ def mlp_forward(self, x: torch.Tensor, *, model_module, original) -> torch.Tenso
     return y
 
 
+_UP, _DOWN = ("Linear", "ColumnParallelLinear"), ("Linear", "RowParallelLinear")
+
+
+def _plain_format(model, w1, w3, w2=None):
+    """The scale_fmt that the Linears all hand to the installed ``linear``, where they do nothing but that (classes of the names
+    above, no bias, no hooks, no code of their own); otherwise False."""
+    if (getattr(model, "world_size", 1) != 1 or not installed_linear(model) or _nn_module._global_forward_hooks
+            or _nn_module._global_forward_pre_hooks):
+        return False
+    up, intercepted = type(w1), host.intercepted
+    if (up.__name__ not in _UP or intercepted(w1) or intercepted(w3) or getattr(w1, "bias", None) is not None
+            or getattr(w3, "bias", None) is not None):
+        return False
+    takes_fmt = linear_takes_fmt(w1, model, w3 if type(w3) is up else None)
+    if takes_fmt is None:
+        return False
+    fmt = w1.scale_fmt if takes_fmt else None
+    if type(w3) is not up:
+        takes_fmt = linear_takes_fmt(w3, model) if type(w3).__name__ in _UP else None
+        if takes_fmt is None:
+            return False
+    if (w3.scale_fmt if takes_fmt else None) != fmt:
+        return False
+    if w2 is not None:
+        if type(w2).__name__ not in _DOWN or intercepted(w2) or getattr(w2, "bias", None) is not None:
+            return False
+        takes_fmt = linear_takes_fmt(w2, model)
+        if takes_fmt is None or (w2.scale_fmt if takes_fmt else None) != fmt:
+            return False
+    return fmt
+
+
 def _plain_up(mlp, model):
     """``(w1, w3, scale_fmt)`` where both do nothing but the GEMM, through the installed ``linear``, on equally quantised
     activations; otherwise None.  The three launches of ``host.mlp`` (the quantisation, w1 and w3 with everything up to w2's
     quantisation, w2) are then as good as theirs."""
-    if getattr(model, "world_size", 1) != 1 or not getattr(getattr(model, "linear", None), "_dsv3_linear", False):
-        return None
-    if _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:
-        return None
     w1, w3 = mlp.w1, mlp.w3
-    for lin in (w1, w3):
-        if type(lin).__name__ not in ("Linear", "ColumnParallelLinear") or getattr(lin, "bias", None) is not None or _intercepted(lin):
-            return None
-    fmt = _scale_fmt_of(w1)
-    return (w1.weight, w3.weight, fmt) if _scale_fmt_of(w3) == fmt else None
-
-
-def _scale_fmt_of(lin):
-    """The scale_fmt a Linear hands to linear(): only the plain one does (model.py:205; not :233, :262)."""
-    return getattr(lin, "scale_fmt", None) if type(lin).__name__ == "Linear" else None
-
-
-def _intercepted(module) -> bool:
-    """Whether a call of the module does more than its class's forward: hooks, or a forward of its own."""
-    return bool(getattr(module, "_forward_hooks", None) or getattr(module, "_forward_pre_hooks", None)
-                or "forward" in getattr(module, "__dict__", ()))
+    fmt = _plain_format(model, w1, w3)
+    return None if fmt is False else (w1.weight, w3.weight, fmt)
 
 
 def plain_weights(mlp, x: torch.Tensor, scale_fmt):
     """``(w1, w3, w2)`` weights of an MLP that ``mlp_forward`` serves and whose Linears do nothing but the GEMM in
-    ``scale_fmt`` (no bias, no hooks, no forward of their own, the installed ``linear``), so that a caller may run them
-    itself; otherwise None."""
-    model = getattr(getattr(type(mlp), "forward", None), "_dsv3_model", None)
-    if model is None or getattr(model, "world_size", 1) != 1 or not getattr(getattr(model, "linear", None), "_dsv3_linear", False):
-        return None
-    if _intercepted(mlp) or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:
+    ``scale_fmt``, so that a caller may run them itself; otherwise None."""
+    forward = getattr(type(mlp), "forward", None)
+    installed, model = getattr(forward, "_dsv3_mlp", (None, None))
+    if installed is None or installed is not forward or host.intercepted(mlp) or not calls_forward(mlp, model):
         return None
     w1, w2, w3 = mlp.w1, mlp.w2, mlp.w3
-    for lin, names in ((w1, ("Linear", "ColumnParallelLinear")), (w3, ("Linear", "ColumnParallelLinear")), (w2, ("Linear", "RowParallelLinear"))):
-        if (type(lin).__name__ not in names or getattr(lin, "bias", None) is not None or _scale_fmt_of(lin) != scale_fmt
-                or _intercepted(lin)):
-            return None
-    if not _fusable(mlp, x, model):
+    if _plain_format(model, w1, w3, w2) != scale_fmt or not _fusable(mlp, x, model):
         return None
     return w1.weight, w3.weight, w2.weight
 
@@ -110,5 +117,5 @@ def install_mlp(model_module) -> None:
             return mlp_forward(self, x, model_module=model_module, original=_original)
 
         forward.__doc__ = mlp_forward.__doc__
-        forward._dsv3_model = model_module
+        forward._dsv3_mlp = forward, model_module        # itself: a wrapper that copies attributes is told from it
         cls.forward = forward
