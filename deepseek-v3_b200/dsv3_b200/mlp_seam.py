@@ -34,6 +34,8 @@ def mlp_forward(self, x: torch.Tensor, *, model_module, original) -> torch.Tenso
     if not _fusable(self, x, model_module):
         return original(self, x)
     w2 = self.w2
+    if host.intercepted(w2) or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:
+        return original(self, x)                          # w2 is not called below
     row_parallel = type(w2).__name__ == "RowParallelLinear"
     # only plain Linear hands its scale_fmt to linear() (model.py:205); the parallel Linears do not (model.py:233, 262)
     scale_fmt = None if (row_parallel or type(w2).__name__ == "ColumnParallelLinear") else getattr(w2, "scale_fmt", None)

@@ -183,3 +183,30 @@ def test_an_mlp_of_the_hosts_is_called():
     for cls in (MLP, Called):
         assert mlp_seam.plain_weights(cls(), X, None) is None
     assert mlp_seam.plain_weights(type("Own", (model.MLP,), {})(), X, None) is not None
+
+
+def _hook(model, mlp, seen):
+    mlp.w2.register_forward_hook(lambda m, i, o: seen.append(1))
+
+
+def _own_forward(model, mlp, seen):
+    inner = mlp.w2.forward
+    mlp.w2.forward = lambda x: (seen.append(1), inner(x))[1]
+
+
+def _global_hook(model, mlp, seen):
+    return torch.nn.modules.module.register_module_forward_pre_hook(lambda m, i: seen.append(1) if m is mlp.w2 else None).remove
+
+
+@pytest.mark.parametrize("change", [_hook, _own_forward, _global_hook])
+def test_w2_that_is_intercepted_is_called(change):
+    model = _model()
+    mlp, seen = model.MLP(), []
+    model.linear = lambda x, weight, bias=None, scale_fmt=None: x + 1
+    undo = change(model, mlp, seen)
+    try:
+        y = mlp(X)
+    finally:
+        if undo:
+            undo()
+    assert seen == [1] and torch.equal(y, torch.nn.functional.silu(X + 1) * (X + 1) + 1)
