@@ -1166,6 +1166,11 @@ int launch_fp8_gemm_tc(const void* a, const float* a_s, const void* b, const flo
         }
     }
     if (pl.error != DSV3_OK) return pl.error;
+    // (a plan that overlooks this makes the kernel write past its shared memory; whatever made the plan, it is not launched)
+    if (pl.swap && (pl.splits < 1 || (pl.kc + pl.splits - 1) / pl.splits > scale_tab_chunks(pl.bn))) {
+        set_last_error("fp8_gemm: %d K chunks in %d parts are more than the weight-major kernel's scale table holds", pl.kc, pl.splits);
+        return DSV3_ERR_UNSUPPORTED;
+    }
     if (pl.wide) return launch_fp8_gemm_tw(a, a_s, b, b_s, M, N, K, c, stream);
     if (pl.pair) return launch_fp8_gemm_tm(a, a_s, b, b_s, M, N, K, c, stream);
     CUtensorMap tp, tq, tc;
