@@ -1,4 +1,5 @@
 // extern "C" surface of libdsv3_b200.so: argument checks, kernel selection, status plumbing.
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -35,7 +36,7 @@ int cuda_fail(cudaError_t e, const char* what) {
     return DSV3_ERR_CUDA;
 }
 
-static int g_sm_budget = 0;   // dsv3_set_num_sms: SMs the persistent GEMM kernels may occupy (0 = all)
+static std::atomic<int> g_sm_budget{0};   // dsv3_set_num_sms: SMs the persistent GEMM kernels may occupy (0 = all)
 
 static int all_sms() {
     static int cached[64] = {};
@@ -52,8 +53,15 @@ static int all_sms() {
     return n;
 }
 
-bool sm_budget_set() { return g_sm_budget > 0 && g_sm_budget < all_sms(); }
-int num_sms() { return sm_budget_set() ? g_sm_budget : all_sms(); }
+// (the budget is read once: another thread may set it in between)
+int num_sms() {
+    const int budget = g_sm_budget.load(std::memory_order_relaxed), all = all_sms();
+    return budget > 0 && budget < all ? budget : all;
+}
+bool sm_budget_set() {
+    const int budget = g_sm_budget.load(std::memory_order_relaxed);
+    return budget > 0 && budget < all_sms();
+}
 
 bool pdl_enabled() {
     static const bool on = (getenv("DSV3_DISABLE_PDL") == nullptr);
@@ -209,7 +217,7 @@ int dsv3_set_num_sms(int n) {
         set_last_error("set_num_sms: 0 (all SMs) or at least 2");
         return DSV3_ERR_INVALID_ARGUMENT;
     }
-    g_sm_budget = n;
+    g_sm_budget.store(n, std::memory_order_relaxed);
     return DSV3_OK;
 }
 
