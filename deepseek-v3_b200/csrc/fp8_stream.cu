@@ -1138,26 +1138,26 @@ uint64_t coprime_with(int n) {
 // most: no more CTAs than there can be work for
 template <int BN, bool kSwiglu, bool kBoth, bool kSplit>
 int launch_stream(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, StreamParams prm, int64_t most,
-                  cudaStream_t stream) {
+                  int sms, cudaStream_t stream) {
     using C = SCfg<BN, false>;
     static bool configured[64] = {};
-    prm.ctas = static_cast<int>(most < num_sms() ? most : num_sms());
+    prm.ctas = static_cast<int>(most < sms ? most : sms);
     if (kBoth && !kSplit) prm.coprime = coprime_with(prm.ctas);
     return launch(fp8_stream_kernel<BN, kSwiglu, kBoth, kSplit>, prm.ctas, C::kSmemBytes, configured, stream, w0, w1, ta0, ta1, prm);
 }
 
 template <bool kSwiglu, bool kBoth>
 int launch_divided(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, StreamParams prm, int64_t most_large,
-                   int64_t most_small, int divide, cudaStream_t stream) {
+                   int64_t most_small, int divide, int sms, cudaStream_t stream) {
     constexpr int kLarge = SCfg<128, true>::kSmemBytes, kSmall = SCfg<64, false>::kSmemBytes;
     static bool configured[64] = {};
     StreamParams small = prm;
     prm.min_rows = divide + 1;
-    prm.ctas = static_cast<int>(most_large < num_sms() ? most_large : num_sms());
+    prm.ctas = static_cast<int>(most_large < sms ? most_large : sms);
     if (kBoth) prm.coprime = coprime_with(prm.ctas);
     small.max_rows = divide;
     small.first_cta = prm.ctas;
-    small.ctas = divide ? static_cast<int>(most_small < num_sms() ? most_small : num_sms()) : 0;
+    small.ctas = divide ? static_cast<int>(most_small < sms ? most_small : sms) : 0;
     return launch(fp8_divided_kernel<kSwiglu, kBoth>, prm.ctas + small.ctas, kLarge > kSmall ? kLarge : kSmall, configured, stream, w0, w1, ta0, ta1,
                   prm, small);
 }
@@ -1183,10 +1183,12 @@ int stream_tile(int64_t rows_per_group) {
     return rows_per_group <= 4 ? 16 : (rows_per_group <= 24 ? 32 : (rows_per_group <= 40 ? 64 : 128));
 }
 
+static size_t tile_workspace_bytes(int bn, int sms);
 size_t stream_workspace_bytes(int64_t rows_per_group) { return stream_tile_workspace_bytes(stream_tile(rows_per_group)); }
-size_t stream_tile_workspace_bytes(int bn) {
+size_t stream_tile_workspace_bytes(int bn) { return tile_workspace_bytes(bn, num_sms()); }
+static size_t tile_workspace_bytes(int bn, int sms) {
     if (bn > 64) return 0;            // of 128 tokens or divided: never cut
-    return DSV3_WORKSPACE_HEADER_BYTES + static_cast<size_t>(num_sms()) * 2 * (2 * bn) * kPRows * sizeof(float);
+    return DSV3_WORKSPACE_HEADER_BYTES + static_cast<size_t>(sms) * 2 * (2 * bn) * kPRows * sizeof(float);
 }
 
 static int fill_side(Side& d, CUtensorMap* map, const StreamSide& q, bool swiglu, int bn) {
@@ -1250,10 +1252,11 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
     prm.status = status_device_ptr();
     if (!prm.status) return DSV3_ERR_CUDA;
     // cutting tiles is worth considering when one or two rounds of whole tiles are expected (struct Plan)
-    const size_t need = stream_tile_workspace_bytes(bn);
+    const int sms = num_sms();                                // once: the grid must fit the workspace, whatever budget is set meanwhile
+    const size_t need = tile_workspace_bytes(bn, sms);
     const int64_t groups_expected = q.n_groups < q.rows_expected ? q.n_groups : q.rows_expected;
     const int64_t tiles_expected = q.n_groups > 0 ? groups_expected * prm.side[kGroups].tiles_p : tiles[1];
-    const bool split = bn < 128 && tiles_expected < 3 * num_sms() && q.workspace && q.workspace_bytes >= need &&
+    const bool split = bn < 128 && tiles_expected < 3 * sms && q.workspace && q.workspace_bytes >= need &&
                        (reinterpret_cast<uintptr_t>(q.workspace) % 256) == 0;
     if (split) {
         prm.tickets = static_cast<int*>(q.workspace);
@@ -1266,8 +1269,8 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
     }
     const int64_t bound = split ? units : tiles[0] + tiles[1];
 #define DSV3_STREAM_LAUNCH(BN_, SW_, SPLIT_)                                                                               \
-    return ordinary ? launch_stream<BN_, SW_, true, SPLIT_>(w0, w1, ta0, ta1, prm, bound, stream)                          \
-                    : launch_stream<BN_, SW_, false, SPLIT_>(w0, w1, ta0, ta1, prm, bound, stream)
+    return ordinary ? launch_stream<BN_, SW_, true, SPLIT_>(w0, w1, ta0, ta1, prm, bound, sms, stream)                          \
+                    : launch_stream<BN_, SW_, false, SPLIT_>(w0, w1, ta0, ta1, prm, bound, sms, stream)
 #define DSV3_STREAM_CASE(BN_)                                                                                              \
     case BN_:                                                                                                              \
         if (q.swiglu) { if (split) DSV3_STREAM_LAUNCH(BN_, true, true); DSV3_STREAM_LAUNCH(BN_, true, false); }            \
@@ -1282,10 +1285,10 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
             const int64_t small = (q.n_groups < q.groups.rows ? q.n_groups : q.groups.rows) * prm.side[kGroups].tiles_p;
             const int divide = sm_budget_set() ? 0 : kDivide;       // under a budget both kinds' CTAs could be resident side by side
             if (q.swiglu)
-                return ordinary ? launch_divided<true, true>(w0, w1, ta0, ta1, prm, bound, small, divide, stream)
-                                : launch_divided<true, false>(w0, w1, ta0, ta1, prm, bound, small, divide, stream);
-            return ordinary ? launch_divided<false, true>(w0, w1, ta0, ta1, prm, bound, small, divide, stream)
-                            : launch_divided<false, false>(w0, w1, ta0, ta1, prm, bound, small, divide, stream);
+                return ordinary ? launch_divided<true, true>(w0, w1, ta0, ta1, prm, bound, small, divide, sms, stream)
+                                : launch_divided<true, false>(w0, w1, ta0, ta1, prm, bound, small, divide, sms, stream);
+            return ordinary ? launch_divided<false, true>(w0, w1, ta0, ta1, prm, bound, small, divide, sms, stream)
+                            : launch_divided<false, false>(w0, w1, ta0, ta1, prm, bound, small, divide, sms, stream);
         }
     }
 #undef DSV3_STREAM_LAUNCH
