@@ -38,11 +38,13 @@ int cuda_fail(cudaError_t e, const char* what) {
 
 static std::atomic<int> g_sm_budget{0};   // dsv3_set_num_sms: SMs the persistent GEMM kernels may occupy (0 = all)
 
-static int all_sms() {
+static int all_sms(int* device = nullptr) {
     static int cached[64] = {};
     int dev = 0;
     int n = 148;
+    if (device) *device = -1;
     if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64) {
+        if (device) *device = dev;
         if (cached[dev] == 0) {
             int q = 0;
             if (cudaDeviceGetAttribute(&q, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || q <= 0) q = 148;
@@ -54,10 +56,11 @@ static int all_sms() {
 }
 
 // (the budget is read once: another thread may set it in between)
-int num_sms() {
-    const int budget = g_sm_budget.load(std::memory_order_relaxed), all = all_sms();
+int num_sms_of_device(int* device) {
+    const int budget = g_sm_budget.load(std::memory_order_relaxed), all = all_sms(device);
     return budget > 0 && budget < all ? budget : all;
 }
+int num_sms() { return num_sms_of_device(nullptr); }
 bool sm_budget_set() {
     const int budget = g_sm_budget.load(std::memory_order_relaxed);
     return budget > 0 && budget < all_sms();

@@ -17,6 +17,7 @@ namespace dsv3 {
 void set_last_error(const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);  // records detail, returns DSV3_ERR_CUDA
 int num_sms();                                   // SM count of the current device (cached), or the budget set for it
+int num_sms_of_device(int* device);              // the same, and which device that is (-1: none, or beyond the 64 that are cached)
 bool sm_budget_set();                            // dsv3_set_num_sms leaves fewer than there are
 bool pdl_enabled();                              // programmatic dependent launch (off when DSV3_DISABLE_PDL is set)
 

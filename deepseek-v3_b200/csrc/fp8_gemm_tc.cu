@@ -894,6 +894,7 @@ bool tc_supported(const void* a, const void* b, const void* c, int64_t M, int64_
 
 // How many clusters of `splits` CTAs of a variant the device holds at once (GPCs do not divide evenly by every size).
 namespace {
+thread_local bool t_guessed = false;      // set where the device did not tell
 template <int BN, bool kSwap>
 int clusters_of(int dev, int splits) {
     using C = Cfg<BN, kSwap>;
@@ -920,7 +921,9 @@ int clusters_of(int dev, int splits) {
         }
         if (n > 0) cached[dev][splits] = n;
     }
-    return n > 0 ? n : 128 / splits;      // no device (planning on a host without one): a cautious guess
+    if (n > 0) return n;
+    t_guessed = true;
+    return 128 / splits;      // no device (planning on a host without one): a cautious guess
 }
 }  // namespace
 
@@ -944,8 +947,8 @@ static double small_estimate(int bn, int64_t M, int chunks, int splits, int64_t 
 }
 
 // Pinned values (dsv3_set_gemm_policy) are honoured or refused (pl.error), never rewritten; the automatic
-// plan adapts freely.
-static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split) {
+// plan adapts freely.  dev, sms: the device (-1: none) and the SMs there are on it, or the budget for them.
+static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split, int dev, int sms) {
     TcPlan pl;
     pl.error = DSV3_OK;
     pl.pair = false;
@@ -996,7 +999,6 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
         // 4 / 6 / 8: 12288 -> 5120 at M = 1 15.4 / 13.2 / - / - / -; 7168 -> 2304 at M = 16 9.1 / 8.0 / 7.5 / 6.9 / -; 7168 -> 576
         // at M = 64 11.4 / 9.5 / 8.3 / 7.8 / 7.1; 7168 -> 1536 at M = 200 13.5 / 12.3 / 11.0 / - / -, S = 5 11.3 (rows that do not
         // divide evenly); a split that needs a second round of clusters loses badly (7168 -> 2048 at M = 16, S = 8: 12.9).
-        const int sms = num_sms();
         const double c = !pl.swap ? 0.28 : (pl.bn == 64 ? 0.23 : 0.24);
         const double e = !pl.swap ? 4.9 : (pl.bn == 64 ? 1.0 : 0.8), e_split = !pl.swap ? 0.0 : (pl.bn == 64 ? 0.05 : 0.1);
         const double bytes = static_cast<double>(N) * K + static_cast<double>(M) * K;
@@ -1036,9 +1038,6 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
             }
             if (const double floor = hbm_floor(tiles); best < floor) best = floor;
         }
-        // (the device is looked up once per plan: every look-up is 50 ns of a 4 us call)
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) dev = -1;
         for (int sfac = 2; sfac <= kMaxClusterSplits && sfac <= pl.kc; ++sfac) {
             const int per_item = (pl.kc + sfac - 1) / sfac;
             if (per_item > tab || tiles > clusters_resident(dev, sms, pl.swap, pl.bn, sfac)) continue;
@@ -1101,7 +1100,7 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
                 pl.error = DSV3_ERR_UNSUPPORTED;
                 return pl;
             }
-            return work_out_plan(M, N, K, 2, 0);   // automatic choice, absurdly long K: token-major tiles instead
+            return work_out_plan(M, N, K, 2, 0, dev, sms);   // automatic choice, absurdly long K: token-major tiles instead
         }
     }
     pl.splits = splits;
@@ -1124,23 +1123,29 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
 }
 
 // A plan is asked for twice per call, for the workspace and for the launch, and takes 0.1 to 0.2 us to work out, of calls that keep the
-// host busy for 4.5: a thread remembers the last few by what they depend on, the problem's size and the SMs there are.
+// host busy for 4.5: a thread remembers the last sixteen by all that they depend on.  (Looked through in turn, 4 to 15 ns; a slot
+// for each by its sizes made the Linears of one layer displace one another.)
 TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split) {
-    if (force_kernel != 0 || force_split != 0) return work_out_plan(M, N, K, force_kernel, force_split);
+    int dev = 0;
+    const int sms = num_sms_of_device(&dev);
+    if (force_kernel != 0 || force_split != 0 || dev < 0) return work_out_plan(M, N, K, force_kernel, force_split, dev, sms);
     struct Remembered {
         int64_t M, N, K;
-        int sms;
+        int sms, dev;
         TcPlan plan;
     };
-    static thread_local Remembered remembered[16] = {};
-    const int sms = num_sms();
-    Remembered& r = remembered[static_cast<uint64_t>(M * 5 + N / 16 * 7 + K / 128 * 3) & 15u];
-    if (r.M != M || r.N != N || r.K != K || r.sms != sms) {
-        const TcPlan plan = work_out_plan(M, N, K, 0, 0);
-        if (plan.error != DSV3_OK) return plan;          // (the message is the call's own)
-        r = {M, N, K, sms, plan};
+    constexpr unsigned kRemembered = 16;
+    static thread_local Remembered remembered[kRemembered] = {};
+    static thread_local unsigned oldest = 0;
+    for (const Remembered& r : remembered)
+        if (r.M == M && r.N == N && r.K == K && r.sms == sms && r.dev == dev) return r.plan;
+    t_guessed = false;
+    const TcPlan plan = work_out_plan(M, N, K, 0, 0, dev, sms);
+    if (plan.error == DSV3_OK && !t_guessed) {           // (the message of an error is the call's own)
+        remembered[oldest] = {M, N, K, sms, dev, plan};
+        oldest = (oldest + 1) % kRemembered;
     }
-    return r.plan;
+    return plan;
 }
 
 size_t tc_workspace_bytes(const TcPlan& pl, int64_t M, int64_t N) {
