@@ -51,12 +51,6 @@ constexpr int kRegsControlM = 88;
 constexpr int kRegsPromoM = 208;
 static_assert(128 * kRegsControlM + 256 * kRegsPromoM <= 384 * 168, "register pool");
 constexpr int kMaxGroups = kMaxGroupsOfTable;
-constexpr int kMinUnits = 3;        // a split range is at least this many 32 KB chunks
-// What cutting tiles costs, in chunks of 0.75 us, and the time a CTA takes per chunk when it has HBM to itself, in
-// sixteenths of that (B200: 64 tokens of a decode layer's 32 experts, one round, 464 us whole, 410 cut).
-constexpr int kSplitCost = 3;
-template <int BN>
-constexpr int kAlone = BN <= 32 ? 7 : 9;
 
 // kRows: tokens on the M side (rows_tiles); otherwise weights (stream_tiles).
 template <int BN_, bool kRows>
@@ -177,13 +171,10 @@ __device__ __forceinline__ Plan make_plan(const StreamParams& p, int group_tiles
     const int rounds = static_cast<int>(static_cast<unsigned>(pl.tiles0) / static_cast<unsigned>(ctas));
     const int rest0 = pl.tiles0 - rounds * ctas;
     if constexpr (!kSplit) return pl;
-    // Time of the last round, in sixteenths of the 0.75 us a chunk takes with every SM loading: whole tiles are bound by
-    // what one CTA folds (kAlone), an even cut by HBM, plus parking and adding up.
-    const int longest = max(rest0 > 0 ? pl.kc0 : 0, pl.tiles1 > 0 ? pl.kc1 : 0);
-    const int rest = static_cast<int>(16u * static_cast<unsigned>(rest0 * pl.kc0 + pl.tiles1 * pl.kc1) / static_cast<unsigned>(ctas));
-    if (rounds < 2 && longest * kAlone<BN> > rest + 16 * kSplitCost) {
-        const int G = min(ctas, max(1, pl.units / kMinUnits));
-        if (G > pl.tiles0 + pl.tiles1 || G == ctas) {
+    if (rounds < 2) {
+        const int G = cut_ranges(BN, pl.tiles0 + pl.tiles1, pl.units, rest0 * pl.kc0 + pl.tiles1 * pl.kc1,
+                                 max(rest0 > 0 ? pl.kc0 : 0, pl.tiles1 > 0 ? pl.kc1 : 0), ctas);
+        if (G > 0) {
             pl.G = G;
             pl.base = static_cast<int>(static_cast<unsigned>(pl.units) / static_cast<unsigned>(G));
             pl.extra = pl.units - pl.base * G;

@@ -78,6 +78,17 @@ struct StreamGemm {
     void* workspace;                   // stream_workspace_bytes(), or null: tiles are not split
     size_t workspace_bytes;
 };
+// Whether a last round is cut over K, and into how many ranges (0: tiles are worked on whole).  tiles, units: of the whole problem, a
+// unit being one K chunk of a tile; last: units of the last round; longest: chunks of its longest tile.  Time of that round, in
+// sixteenths of the 0.75 us a chunk takes with every SM loading: whole tiles are bound by what one CTA folds when it has HBM to
+// itself, an even cut by HBM, plus parking and adding up, three chunks (B200: 64 tokens of a decode layer's 32 experts, one round,
+// 464 us whole, 410 cut).  A range is at least three 32 KB chunks.
+__host__ __device__ inline int cut_ranges(int bn, int tiles, int units, int last, int longest, int ctas) {
+    const int alone = bn <= 32 ? 7 : 9;
+    if (bn > 64 || longest * alone <= static_cast<int>(16u * static_cast<unsigned>(last) / static_cast<unsigned>(ctas)) + 16 * 3) return 0;
+    const int by_size = units / 3 > 1 ? units / 3 : 1, ranges = ctas < by_size ? ctas : by_size;
+    return ranges > tiles || ranges == ctas ? ranges : 0;
+}
 int stream_tile(int64_t rows_per_group);
 size_t stream_workspace_bytes(int64_t rows_per_group);
 size_t stream_tile_workspace_bytes(int bn);

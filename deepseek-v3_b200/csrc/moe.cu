@@ -378,14 +378,15 @@ StreamSide side_of(const void* a, const float* a_s, bool transposed, int64_t row
 int swiglu_linear_tile(int64_t M, int64_t N, int64_t K) {
     const int64_t blocks = N / 128, kc = (K + 127) / 128, sms = num_sms();
     if (2 * blocks >= sms) return M <= 16 ? 16 : (M <= 64 ? 64 : (M <= 128 ? 128 : 0));
-    struct Cost { int tile, alone; double base, chunk, cut, unit; };
-    constexpr Cost kCosts[] = {{16, 7, 4.6, 0.33, 8.9, 0.0030}, {32, 7, 5.8, 0.36, 11.3, 0.0036}, {64, 9, 7.2, 0.46, 17.0, 0.0036}, {128, 0, 7.5, 0.42, 0.0, 0.0}};
+    struct Cost { int tile; double base, chunk, cut, unit; };
+    constexpr Cost kCosts[] = {{16, 4.6, 0.33, 8.9, 0.0030}, {32, 5.8, 0.36, 11.3, 0.0036}, {64, 7.2, 0.46, 17.0, 0.0036}, {128, 7.5, 0.42, 0.0, 0.0}};
     int best = 0;
     double least = 1e30;
     for (const Cost& c : kCosts) {
         const int64_t tiles = blocks * ((M + c.tile - 1) / c.tile);
-        if (tiles > sms) continue;
-        const bool is_cut = kc * c.alone > 16 * tiles * kc / sms + 48;            // (make_plan in fp8_stream.cu)
+        if (tiles > sms || tiles * kc >= (1ll << 27)) continue;
+        const int units = static_cast<int>(tiles * kc);
+        const bool is_cut = cut_ranges(c.tile, static_cast<int>(tiles), units, units, static_cast<int>(kc), units < sms ? units : static_cast<int>(sms)) > 0;
         const double t = is_cut ? c.cut + c.unit * static_cast<double>(tiles * kc) : c.base + c.chunk * static_cast<double>(kc);
         if (t < least) {
             least = t;
