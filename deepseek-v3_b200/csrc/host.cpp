@@ -327,10 +327,13 @@ std::pair<at::Tensor, at::Tensor> quantise_remembered(const at::Tensor& x, int64
 
 // ------------------------------------------------------------------ an MLP whose Linears are plain
 // w2(swiglu_quant(w1(x), w3(x))) in three launches: the quantisation of x, w1 and w3 with everything in front of w2, w2.
-// Undefined where the separate launches are faster.
+// Undefined where the separate launches are faster: in a graph, where only the device counts, or from here, where the host's launches do too.
 at::Tensor mlp(const at::Tensor& x, const at::Tensor (&w)[3], const at::Tensor (&s)[3], int x_fmt, int h_fmt, bool assume_no_inplace) {
     const int64_t K = last_dim(x), M = K ? x.numel() / K : 0, N = w[0].size(0);
-    if (w[0].dim() != 2 || w[0].sizes() != w[1].sizes() || w[0].size(1) != K || !dsv3_swiglu_linear_pays(M, N, K)) return {};
+    if (w[0].dim() != 2 || w[0].sizes() != w[1].sizes() || w[0].size(1) != K) return {};
+    if (!dsv3_swiglu_linear_pays(M, N, K) &&
+        (!dsv3_swiglu_linear_saves_launches(M, N, K) || !x.is_cuda() || capture_of(c10::cuda::getCurrentCUDAStream(x.device().index()).stream()) != 0))
+        return {};
     for (int i = 0; i < 2; ++i) {
         require(w[i].is_contiguous(), "Input tensors must be contiguous");
         require(s[i].is_contiguous(), "Scaling factor tensors must be contiguous");

@@ -367,14 +367,10 @@ StreamSide side_of(const void* a, const float* a_s, bool transposed, int64_t row
     return d;
 }
 
-// Tokens per tile for w1 and w3 of an ordinary MLP with SwiGLU and quantisation in one launch, or 0 where two GEMMs and
-// swiglu_quant are as fast.  With enough weight to keep half of the SMs on whole tiles the launch is a stream of weights up to 128
-// tokens; beyond, the pair tiles of the GEMMs multiply better.  With less it is set-up, epilogue and the chunks of a tile, whole
-// (base + chunk * K chunks) or cut over K as the kernel's own plan decides (cut + unit * units), until whole tiles of 128 no longer fit
-// one round.  B200, us in a replayed graph, three launches / one: 7168 -> 18432 at M = 1, 16, 64, 128 47 / 44, 51 / 45, 61 / 48, 61 / 51, 192
-// 72 / 75; 5120 -> 12288 at 64, 128 37 / 29, 40 / 30; 7168 -> 2304 at 1, 16, 64, 256, 1024 15.4 / 12.9, 16.8 / 14.1, 21.0 / 18.0, 30.5 / 25.8,
-// 42.0 / 34.7; 2048 -> 2816 at 64, 192, 512 14.0 / 10.1, 17.6 / 11.8, 21.9 / 16.1; 2048 -> 1408 at 8, 64, 256 8.8 / 9.5, 13.1 / 9.6, 15.3 / 11.6 (and
-// two launches fewer from the host).
+// Tokens per tile for w1 and w3 of an ordinary MLP with SwiGLU and quantisation in one launch, or 0 where no width does: with enough
+// weight to keep half of the SMs on whole tiles the launch is a stream of weights up to 128 tokens; beyond, the pair tiles of the
+// GEMMs multiply better.  With less it is set-up, epilogue and the chunks of a tile, whole (base + chunk * K chunks) or cut over K as
+// the kernel's own plan decides (cut + unit * units), until whole tiles of 128 no longer fit one round.
 int swiglu_linear_tile(int64_t M, int64_t N, int64_t K) {
     const int64_t blocks = N / 128, kc = (K + 127) / 128, sms = num_sms();
     if (2 * blocks >= sms) return M <= 16 ? 16 : (M <= 64 ? 64 : (M <= 128 ? 128 : 0));
@@ -394,6 +390,25 @@ int swiglu_linear_tile(int64_t M, int64_t N, int64_t K) {
         }
     }
     return best;
+}
+
+// Whether that is faster on the device than two GEMMs and swiglu_quant.  Cut tiles are not where the separate launches are at their
+// best: up to 8 rows on weights that the decode kernel takes (but for few K chunks, which nothing cuts), up to 16 and 32 rows on few
+// or long rows of weights, whose GEMMs split K inside clusters.  B200, us per MLP in a graph of as many as displace the L2, five
+// launches / three: 2048 -> 1408 at 1, 8, 16, 48, 256, 1024 rows 12.0 / 15.0, 13.1 / 15.0, 16.3 / 16.5, 19.3 / 17.3, 22.5 / 19.7, 32.1 /
+// 25.6; 1408 -> 2048 at 1, 9, 17 11.8 / 14.6, 16.9 / 16.4, 17.4 / 14.5; 1024 -> 1024 at 1, 8 11.4 / 10.9, 12.6 / 11.0; 4096 -> 1408 at 8,
+// 16, 33 16.4 / 18.7, 19.1 / 20.1, 21.6 / 20.1; 7168 -> 1024 at 16, 24, 33 19.4 / 22.6, 20.3 / 20.6, 23.2 / 22.0; 7168 -> 1536 at 1, 8, 33
+// 22.1 / 21.1, 21.0 / 21.6, 25.3 / 23.0; 7168 -> 2304 at 1, 16, 24, 48, 256 24.3 / 21.9, 24.3 / 23.0, 25.1 / 26.1, 30.2 / 27.8, 42.0 / 38.1;
+// 7168 -> 4608 at 16, 17, 48 32.9 / 31.2, 33.4 / 34.6, 39.7 / 38.3; 7168 -> 512 at 16, 64, 80 17.3 / 19.8, 20.0 / 20.3, 22.2 / 19.0; 5120 ->
+// 12288 at 1, 128 44.6 / 41.2, 62.3 / 51.6; 7168 -> 18432 at 1, 16, 128 73.9 / 69.9, 77.9 / 71.7, 102.3 / 90.3.
+bool swiglu_linear_faster(int64_t M, int64_t N, int64_t K) {
+    const int64_t blocks = N / 128, kc = (K + 127) / 128;
+    if (2 * blocks >= num_sms()) return true;
+    if (M <= 8 && decode_kernel_pays(M, N, K)) return kc <= 8;
+    if (M <= 2) return true;                       // (larger weights at one or two rows: the fused Linear)
+    if (M <= 16) return kc <= 24 || blocks >= 16;
+    if (M <= 32) return kc <= 40;
+    return M > 64 || kc <= 40 || blocks > 6;
 }
 
 // The ordinary weight of dsv3_swiglu_gemm_rows / dsv3_fp8_gemm_rows.
@@ -532,9 +547,18 @@ int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, 
     return launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
 }
 
-int dsv3_swiglu_linear_pays(int64_t M, int64_t N, int64_t K) {
-    return M > 0 && N > 0 && N % 128 == 0 && K >= 128 && K % 128 == 0 && M < (1ll << 31) && swiglu_linear_tile(M, N, K) > 0;
+// (a kernel or split that the host pinned is one of fp8_gemm's: the separate launches honour or refuse it)
+static bool swiglu_linear_serves(int64_t M, int64_t N, int64_t K) {
+    return M > 0 && N > 0 && N % 128 == 0 && K >= 128 && K % 128 == 0 && M < (1ll << 31) && gemm_policy_kernel() == 0 && gemm_policy_split() == 0 &&
+           swiglu_linear_tile(M, N, K) > 0;
 }
+
+int dsv3_swiglu_linear_pays(int64_t M, int64_t N, int64_t K) { return swiglu_linear_serves(M, N, K) && swiglu_linear_faster(M, N, K); }
+
+// Launching three kernels instead of five saves a host 4 to 10 us, of 23 to 30 that it needs for an MLP; up to 24 MB of weights the
+// device needs no more than that.  us from Python, five launches / three: 2048 -> 1408 at 1 row 23.5 / 19.6, at 16 30.3 / 20.0; 7168 -> 2304 at
+// 24 30.3 / 27.1, 7168 -> 3072 at 17 31.1 / 29.9; but 7168 -> 4608 34.7 / 35.5.
+int dsv3_swiglu_linear_saves_launches(int64_t M, int64_t N, int64_t K) { return swiglu_linear_serves(M, N, K) && N * K <= (24ll << 20); }
 
 size_t dsv3_swiglu_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
     const int tile = M > 0 && N > 0 && K > 0 ? swiglu_linear_tile(M, N, K) : 0;

@@ -3,7 +3,8 @@
 Both compute ``w2(F.silu(w1(x)) * w3(x))`` (model.py:532, 633).  In FP8 mode the product is quantised straight away by
 the ``linear()`` call of ``w2`` (model.py:158-159), so silu, multiply and act_quant are three launches and two bf16
 round trips through HBM for what is one pass over the data.  Where ``w1`` and ``w3`` are plain Linears of the installed
-``linear`` and the library's rule on sizes says that it pays (few rows, or tiles that fit one round of the SMs),
+``linear`` and the library's rules on sizes say that it pays (few rows, or tiles that fit one round of the SMs; on the
+device, or outside of a graph capture for the host that launches),
 ``mlp_forward`` is three launches behind one host call: the quantisation of ``x``, ``w1`` and ``w3`` with SwiGLU and the
 quantisation in front of ``w2``, and ``w2``.  Otherwise it calls ``w1`` and ``w3`` (through whatever ``linear`` is
 installed), then ``swiglu_quant`` (one launch, same rounding points, bit-identical FP8 codes and scales) and feeds

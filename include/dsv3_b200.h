@@ -250,9 +250,11 @@ size_t dsv3_gemm_rows_workspace_bytes(int n_groups, int64_t rows_total, int64_t 
  * w1 and w3 of an ordinary MLP in one launch -- act_quant(silu(fp8_gemm(a, w1)) * fp8_gemm(a, w3)), model.py:532, 633 up to w2's GEMM:
  * a e4m3 [M, K] with scales fp32 [M, K/128], weights e4m3 [N, K] with theirs, N % 128 == 0; h e4m3 [M, N], h_s fp32 [M, N/128], what
  * dsv3_swiglu_quant writes given equal GEMM results.  workspace: under the rules of dsv3_fp8_gemm's (null: K is never split).
- * _pays: whether it is faster than the separate launches (any M is taken all the same).
+ * _pays: whether it is faster on the device than the separate launches (any M is taken all the same); _saves_launches: whether it is
+ * faster where the host's launches, and not the device, are what bounds.  Both 0 while dsv3_set_gemm_policy pins a kernel or split.
  */
 int dsv3_swiglu_linear_pays(int64_t M, int64_t N, int64_t K);
+int dsv3_swiglu_linear_saves_launches(int64_t M, int64_t N, int64_t K);
 size_t dsv3_swiglu_linear_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int dsv3_swiglu_linear(const void* a, const float* a_s, const void* w1, const float* w1_s, const void* w3, const float* w3_s,
                        int64_t M, int64_t N, int64_t K, int scale_fmt, void* h, float* h_s, void* workspace, size_t workspace_bytes,
