@@ -316,9 +316,12 @@ bool small_linear_supported(const void* act, const void* w, const void* c, int64
 
 // Automatic choice of the register-streaming kernel: up to 8 rows, up to 8 MB of weights in at most 4096 rows (its layout
 // that splits K over the warps too).  It has less to set up than the tcgen05 pipeline; beyond 8 MB, or with more rows, the
-// tcgen05 kernel's TMA ring streams better.  B200, us, this kernel / tcgen05 at M = 1: 1024 -> 512 2.7 / 3.6; 7168 -> 576
-// 4.1 / 4.8; 2048 -> 1408 4.0 / 4.2; 5120 -> 1536 5.0 / 5.3; 16384 -> 512 6.0 / 6.8; 7168 -> 1536 6.3 / 5.8; 1024 -> 7168 4.3 /
-// 4.1; at M = 16 2048 -> 1408 4.7 / 4.4.  K is bounded by the activations that a CTA stages, 128 K chunks even unsplit.
+// tcgen05 kernel's TMA ring streams as well or better.  B200, us, this kernel / tcgen05 at one row with weights from HBM: 1024 -> 2048 3.00 /
+// 3.79; 7168 -> 576 4.00 / 4.89; 2048 -> 1408 3.07 / 4.11; 5120 -> 1536 4.88 / 5.36; 4096 -> 2048 4.21 / 5.31; 16384 -> 512 5.85 / 6.65; at eight
+// rows 2048 -> 1408 3.07 / 4.31, 5120 -> 1536 4.89 / 5.52; beyond the line 7168 -> 1280 5.79 / 5.53, 7168 -> 1536 6.12 / 5.85, 4096 -> 3072 6.05 /
+// 5.89, 5120 -> 3072 7.26 / 6.65; but 5120 -> 2048 4.96 / 5.66, 7168 -> 2048 6.18 / 6.45.  Within it, 71 to 73 row tiles of many chunks are more
+// CTAs in clusters than there is room for: 7168 -> 1152 7.88 / 5.48.  K is bounded by the activations that a CTA stages, 128 K chunks even
+// unsplit.
 bool decode_kernel_pays(int64_t M, int64_t N, int64_t K) { return M <= 8 && N <= 4096 && K <= 16384 && N * K <= (8ll << 20); }
 
 // x != nullptr: fused (bf16 activations); otherwise (a, a_s) are the quantised activations.
@@ -364,13 +367,17 @@ int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, cons
     };
     // Where the row tiles are no more than the SMs and clusters would be of at most four, or no more than twice the SMs and no clusters
     // are needed, one CTA of sixteen or eight warps per row tile does without the exchange, and quantises the activations
-    // with all of them (registers admit one such CTA per SM, or two).  us at 1 / 2 / 4 rows, before / so: 2048 -> 1408 3.48 / 4.21 / 4.24, 3.18 / 3.34 /
-    // 4.16; 1408 -> 2048 4.21 / 4.13 / 5.47, 2.94 / 3.08 / 3.77; eight warps, 512 -> 4096 3.12 / 3.18 / 3.88, 2.74 / 2.82 / 2.84; 7168 -> 2304 6.61 / 6.84, 6.20 / 6.45; level:
-    // 7168 -> 1536 5.99 / 6.28, 6.06 / 6.34, 5120 -> 1536 5.11 / 5.21, 5.06 / 5.21.  Sixteen warps in clusters of two instead of four in
-    // eight: 7168 -> 576 4.18 / 4.48 / 4.68, 4.32 / 4.99 / 5.25.  With activations that are quantised already only the exchange is gained,
-    // which few chunks, or few CTAs with many, do not pay for: 1408 -> 2048 3.52, 3.09; but 256 -> 2048 2.63, 2.84; 1024 -> 1024 2.85, 3.00; 4096 -> 768 at
-    // eight rows 3.75, 4.05.  (Both kinds of activations take the same layout: their results are the same bit for bit.)
-    const bool pays = prm.kc >= 10 && (prm.kc <= 24 || rowgroups >= 80);
+    // with all of them (registers admit one such CTA per SM, or two).  us at 1 / 2 / 4 / 8 rows with weights from HBM, before / so: 2048 -> 1408
+    // 3.69 / 4.07 / 4.21 / 5.33, 3.18 / 3.27 / 3.94 / 3.90; 1408 -> 2048 4.30 / 4.37 / 5.68 / 6.64, 2.97 / 3.02 / 3.59 / 3.46; 4096 -> 1536 4.40 /
+    // 4.95 / 5.10 / 6.29, 4.18 / 4.75 / 4.98 / 6.17; 7168 -> 2048 6.78 / 6.93 / 8.08 / 10.67, 6.62 / 6.77 / 8.06 / 10.48; 7168 -> 2304 7.15 / 7.29 /
+    // 8.47 / 10.82, 6.87 / 6.99 / 8.22 / 10.69; eight warps, 512 -> 4096 3.07 / 3.18 / 3.79 / 3.60, 2.66 / 2.72 / 2.77 / 3.13.  With more than 24
+    // chunks that the sixteen warps do not share evenly the cluster stays ahead until it is 512 CTAs: 7168 -> 1280 6.21 / 6.34 / 7.52,
+    // 6.34 / 6.52 / 7.73; 7168 -> 1536 6.46 / 6.63 / 7.75, 6.62 / 6.69 / 7.95; 5120 -> 1536 5.34 / 5.45 / 6.74, 5.40 / 5.46 / 6.87; but 6144 -> 1280
+    // 5.72 / 5.79 / 7.11, 5.64 / 5.72 / 7.14.  Sixteen warps in clusters of two instead of four in eight: 7168 -> 576 4.18 / 4.48 / 4.68, 4.32 /
+    // 4.99 / 5.25.  With activations that are quantised already only the exchange is gained, which few chunks, or few CTAs with many, do
+    // not pay for: 1408 -> 2048 at one row 3.67, 2.92; but 256 -> 2048 2.47, 2.72; 1024 -> 1024 2.70, 2.82; 4096 -> 768 at eight rows 3.67,
+    // 3.89.  (Both kinds of activations take the same layout: their results are the same bit for bit.)
+    const bool pays = prm.kc >= 10 && (prm.kc <= 24 || (rowgroups >= 80 && (prm.kc % 16 == 0 || rowgroups >= 128)));
     if (narrow && M <= 8 && rowgroups <= num_sms() && csize <= 4 && pays && smem_of(16, 1) <= kMaxSmem) {
         wk = 16;
         csize = 1;

@@ -1,0 +1,27 @@
+"""Which layout the decode-sized Linear takes at both sides of the lines, read from a captured graph: a CTA of sixteen or eight warps to
+a row tile, or four-warp CTAs in clusters."""
+import pytest
+import torch
+
+from test_gpu_expert_launches import _kernels
+from test_gpu_stream import _bf16_default, _weight  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N,K,ctas,warps", [
+    (1408, 2048, 88, 16),
+    (1280, 3072, 80, 16),           # 24 chunks: any number of row tiles
+    (1280, 3200, 320, 4),           # 25 that sixteen warps do not share evenly: clusters of four
+    (1280, 4096, 80, 16),           # 32 that they do
+    (1264, 4096, 316, 4),           # 79 row tiles
+    (1536, 7168, 384, 4),           # 56 chunks
+    (2032, 7168, 508, 4),           # 127 row tiles
+    (2048, 7168, 128, 16),
+    (2376, 1280, 149, 8),
+])
+def test_layout(N, K, ctas, warps):
+    import dsv3_b200
+    g = torch.Generator(device="cuda").manual_seed(N)
+    w, x = _weight(N, K, g), torch.randn(1, K, generator=g, device="cuda", dtype=torch.float32).bfloat16()
+    assert _kernels(lambda: dsv3_b200.fp8_linear(x, w, w.scale)) == [(ctas, 32 * warps)]
