@@ -31,12 +31,15 @@ from .ops import _stream
 # 7168 x 2048 1136 / 1160, 1418 / 1438, 1640 / 1650, 1765 / 1800, 1930 / 1889; 32 of those 256 186 / 208, 210 / 234, 246 / 275, 296 / 305,
 # 352 / 340.
 SHARED_INLINE_MAX_ROWS = 512
-# On a rank with few of the experts, their narrow tiles read the shared experts' weights from L2 once per 32 tokens or so: when
-# that is more than the local experts' own weights (and than what launches cost, hence the floor) it is what the launch
-# waits for.  Inline / separate at 256, 333 and 512 tokens: 20 of 160 experts of 5120 x 1536 120 / 134, 140 / 134, 169 / 146; 10 of those
-# 105 / 106, 107 / 105, 133 / 118; 8 of 256 of 7168 x 2048 112 / 119, 137 / 135, 146 / 146; 16 of those 152 / 160, 163 / 178,
-# 197 / 193; but 16 of 64 of 2048 x 1408, whose weights are small, 64 / 82, 81 / 91, 68 / 87.
+# On a rank with few of the experts, their narrow tiles read the shared experts' weights from L2 once per tile of 16, 32 or 64
+# tokens: when that is more than the local experts' own weights (and than what launches cost, hence the floor) it is what the
+# launch waits for.  Inline / separate at 128, 256, 333 and 512 tokens: 20 of 160 experts of 5120 x 1536 101 / 120, 121 / 133, 140 / 132,
+# 167 / 144; 10 of those 80 / 91, 105 / 101, 107 / 102, 133 / 115; 8 of 256 of 7168 x 2048 (at 128 tiles of 16) 100 / 104, 111 / 115,
+# 137 / 132, 145 / 144; 16 of those 134 / 141, 149 / 156, 161 / 175, 191 / 187; but 16 of 64 of 2048 x 1408, whose weights are small,
+# 57 / 67, 65 / 79, at 512 (tiles of 64) 69 / 85.
 SHARED_INLINE_REREAD_FLOOR = 400 << 20
+# Up to 64 rows are at most four tiles: four times these weights are below the floor, and the rule costs the host 1 us.
+SHARED_INLINE_FEW_ROWS, SHARED_INLINE_FEW_ROWS_MAX_WEIGHT = 64, 32 << 20
 # With more tokens they still are where the routed experts' launches have tiles of 128 tokens (more than 40 pairs per expert on
 # average) and little enough to read that launches, last rounds and the SwiGLU pass of a separate MLP weigh.  At 1024, 1500 and
 # 2048 tokens, inline / separate: 64 experts of 2048 x 1408 200 / 216, 255 / 258, 308 / 317; 8 of those 64 68 / 90, 89 / 111,
@@ -50,8 +53,9 @@ SHARED_INLINE_MAX_BYTES_SMALL = 1500 << 20      # of the local experts' weights
 
 def _shared_inline(st, rows: int, topk: int, n_routed: int, shared_width: int) -> bool:
     local_bytes = 3 * st.n * st.inter * st.dim
-    if rows * topk <= 40 * max(n_routed, st.n):
-        reread = 3 * shared_width * st.dim * rows // 32
+    pairs = -(-rows * topk // max(n_routed, st.n))                    # of an expert: what the tiles' width is chosen by (stream_tile)
+    if pairs <= 40:
+        reread = 3 * shared_width * st.dim * rows // (16 if pairs <= 4 else 32 if pairs <= 24 else 64)
         return rows <= SHARED_INLINE_MAX_ROWS and reread <= max(local_bytes, SHARED_INLINE_REREAD_FLOOR)
     return rows <= SHARED_INLINE_MAX_ROWS or rows <= SHARED_INLINE_MAX_ROWS_SMALL and local_bytes <= SHARED_INLINE_MAX_BYTES_SMALL
 
@@ -175,8 +179,8 @@ def grouped_moe_forward(self, x: torch.Tensor, *, world_size: int = 1, fallback=
     rows = x.size(0)
     if world_size == 1 and rows <= SHARED_INLINE_MAX_ROWS_SMALL and 0 < indices.numel():     # (no pairs: no launch to join)
         shared = plain_weights(self.shared_experts, x, st.scale_fmt)
-        # (up to 64 rows the weights are read twice at most, and the rule costs the host 1 us)
-        if rows > 64 and shared is not None and not _shared_inline(st, rows, indices.size(-1), n_routed, shared[0].size(0)):
+        if (shared is not None and (rows > SHARED_INLINE_FEW_ROWS or shared[0].numel() > SHARED_INLINE_FEW_ROWS_MAX_WEIGHT)
+                and not _shared_inline(st, rows, indices.size(-1), n_routed, shared[0].size(0))):
             shared = None
     routed = st.run(x, weights, indices, n_routed, shared)
     if shared is not None:
