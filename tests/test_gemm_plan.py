@@ -1,24 +1,44 @@
-"""Sizes that the automatic plan asks a workspace for, over the range where it chooses between token tiles: a plan of many small tiles
-never asks for more than a ticket header and the padded parts of tiles that the machine holds at once."""
+"""The automatic plan over the range where it chooses between token tiles, and plans that are refused."""
 import ctypes
 
 import pytest
 import torch
 
 
-def test_workspace_of_narrow_token_tiles():
-    from dsv3_b200 import _lib
-    ws = _lib.lib.dsv3_fp8_gemm_workspace_bytes
-    for M in (33, 48, 64, 65, 100, 256):
-        for N, K in ((576, 7168), (7168, 2048), (1408, 2048), (512, 16384), (4096, 512)):
-            assert ws(M, N, K) <= _lib.WORKSPACE_HEADER_BYTES + 148 * 128 * 128 * 4
-    assert ws(64, 4096, 512) == 0 and ws(128, 3072, 1536) == 0          # enough narrow tiles: none is split
-
-
 class Plan(ctypes.Structure):
     """TcPlan of csrc/gemm_plan.cuh"""
     _fields_ = [("error", ctypes.c_int), ("swap", ctypes.c_bool), ("pair", ctypes.c_bool), ("wide", ctypes.c_bool), ("cluster", ctypes.c_bool),
                 ("bn", ctypes.c_int), ("tiles_p", ctypes.c_int), ("tiles_q", ctypes.c_int), ("splits", ctypes.c_int), ("kc", ctypes.c_int)]
+
+
+def _plan(M, N, K):
+    from dsv3_b200 import _lib
+    tc_plan = getattr(_lib.lib, "_ZN4dsv37tc_planElllii")
+    tc_plan.argtypes, tc_plan.restype = [ctypes.c_int64] * 3 + [ctypes.c_int] * 2, Plan
+    p = tc_plan(M, N, K, 0, 0)
+    return (p.bn, p.tiles_p, p.tiles_q, p.splits) if p.swap else None
+
+
+@pytest.mark.parametrize("M,N,K,plan", [
+    (32, 7168, 2048, (32, 56, 1, 2)),       # one tile as wide as M, cut
+    (33, 7168, 2048, (32, 56, 2, 1)),       # several, whole
+    (64, 4096, 512, (16, 32, 4, 1)),
+    (128, 3072, 1536, (32, 24, 4, 1)),
+    (256, 1408, 2048, (32, 11, 8, 1)),
+    (257, 1408, 2048, None),                # token-major tiles
+    (33, 576, 7168, (32, 5, 2, 8)),         # several, cut over clusters
+    (128, 512, 16384, (32, 4, 4, 8)),
+    (200, 512, 49152, (64, 4, 4, 8)),       # 24 MB of weights
+    (200, 512, 49168, None),
+    (64, 16384, 1552, (64, 128, 1, 1)),     # beyond: one tile as wide as M
+])
+def test_narrow_token_tiles(M, N, K, plan):
+    """Token tiles, weight tiles and splits at both sides of the lines; the workspace is a padded part of a tile for every split."""
+    from dsv3_b200 import _lib
+    assert _plan(M, N, K) == plan
+    if plan:
+        bn, p, q, splits = plan
+        assert _lib.lib.dsv3_fp8_gemm_workspace_bytes(M, N, K) == (_lib.WORKSPACE_HEADER_BYTES + splits * p * q * 128 * bn * 4 if splits > 1 else 0)
 
 
 @pytest.mark.parametrize("bn,splits,chunks,fits", [(64, 1, 73, False), (64, 2, 145, False), (32, 1, 145, False), (16, 1, 145, False),

@@ -30,14 +30,14 @@ def test_tiles_of_the_ordinary_weight_among_the_groups(counts, inter, dim, side_
 
 @pytest.mark.parametrize("tokens,inline", [(100, True), (2048, True), (2049, False)])
 def test_shared_experts_of_many_tokens(tokens, inline):
-    """In the routed experts' launches or in their own."""
+    """In the routed experts' four launches or in two of their own: their activations are quantised already."""
     import dsv3_b200
     moe, _ = _host()
     x = torch.randn(tokens, 256, generator=torch.Generator(device="cuda").manual_seed(tokens), device="cuda", dtype=torch.float32).bfloat16()
     launches = len(_kernels(lambda: dsv3_b200.grouped_moe_forward(moe, x)))
     routing = moe.gate(x)
     gate = len(_kernels(lambda: moe.gate(x)))
-    assert (launches - gate == 4) == inline and launches - gate >= 4
+    assert launches - gate == (4 if inline else 6)
     moe.gate = lambda x: routing
     got = dsv3_b200.grouped_moe_forward(moe, x)
     want, _ = moe.reference_forward(x)

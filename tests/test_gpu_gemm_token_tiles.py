@@ -1,5 +1,5 @@
-"""17 to 256 tokens on few weights, where the automatic plan takes several token tiles of 16, 32 or 64 with the weights on the M side, whole
-or split inside clusters: edges of the token tiles and of the range, weight tiles cut by N, K tails, a K longer than a tile's scale
+"""33 to 256 tokens on few weights, where the automatic plan takes several token tiles of 16, 32 or 64 with the weights on the M side, whole
+or split inside clusters (test_gemm_plan.py holds which), and sizes beside that range: edges of the token tiles and of the range, weight tiles cut by N, K tails, a K longer than a tile's scale
 table, against the CUDA-core kernel."""
 import pytest
 import torch

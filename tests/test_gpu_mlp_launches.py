@@ -83,11 +83,14 @@ def test_codes_and_scales_in_front_of_w2(M, N, K, fmt):
         _h_close(h[:M].view(torch.float8_e4m3fn), hs[:M].t(), want, want_s)
 
 
-@pytest.mark.parametrize("change", ["hook", "forward", "world", "format", "bias"])
-def test_what_keeps_the_separate_launches(change):
-    mlp, model = _host(256, 128)
-    x = _rows(20, 256)
-    want = mlp(x)
+@pytest.mark.parametrize("change,launches", [(None, 3), ("hook", 5), ("forward", 5), ("world", 5), ("format", 6), ("bias", 6)])
+def test_what_keeps_the_separate_launches(change, launches):
+    """Against the operators, each with the bias and the format of its Linear; five launches, one more where the activations are
+    quantised twice or the bias is added."""
+    import kernel
+    from dsv3_b200 import swiglu_quant
+    mlp, model = _host(1024, 512)
+    x = _rows(20, 1024)
     seen = []
     if change == "hook":
         mlp.w1.register_forward_hook(lambda m, i, o: seen.append(1))
@@ -98,9 +101,16 @@ def test_what_keeps_the_separate_launches(change):
         model.world_size = 2
     elif change == "format":
         mlp.w3.scale_fmt = "ue8m0"
-    else:
-        mlp.w1.bias = torch.zeros(128, device="cuda")
-    got = mlp(x)
+    elif change == "bias":
+        mlp.w1.bias = torch.linspace(-2, 2, 512, device="cuda")
+    got = mlp(x.view(x.shape))
     assert bool(seen) == (change in ("hook", "forward"))
+
+    def up(lin):
+        y = kernel.fp8_gemm(*kernel.act_quant(x, 128, lin.scale_fmt), lin.weight, lin.weight.scale)
+        return y if lin.bias is None else y + lin.bias
+    want = kernel.fp8_gemm(*swiglu_quant(up(mlp.w1), up(mlp.w3), mlp.w2.scale_fmt), mlp.w2.weight, mlp.w2.weight.scale)
     err, rms = (got.float() - want.float()).abs(), want.float().pow(2).mean().sqrt()
-    assert change == "format" or bool((err <= 2e-2 * (want.float().abs() + rms)).all())
+    assert bool((err <= 2e-2 * (want.float().abs() + rms)).all())
+    assert change is None or torch.equal(got, want), "the same operators"
+    assert len(_kernels(lambda: mlp(x.view(x.shape)))) == launches
