@@ -678,27 +678,30 @@ PyObject* py_mlp(PyObject*, PyObject* const* args, Py_ssize_t n) {
     });
 }
 
-// Whether a call of this object does more than its class's forward: hooks, a forward of its own, a compiled call.  (Here, as it is
-// asked four times per call of an expert layer: 0.05 us instead of 0.15.)
-PyObject* py_intercepted(PyObject*, PyObject* module) {
+// Whether a call of any of these objects does more than its class's forward: hooks, a forward of its own, a compiled call.  (Here, as
+// four are asked about per call of an expert layer: 0.2 us together instead of 0.15 each.)
+PyObject* py_intercepted(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
-        PyObject* own = PyObject_GetAttr(module, g_attr_dict);
-        if (!own) {
-            if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw PythonError{};
-            PyErr_Clear();
-            Py_RETURN_FALSE;
-        }
-        int found = 1;
-        if (PyDict_Check(own)) {
-            const auto at = [&](PyObject* key) { return PyDict_GetItemWithError(own, key); };
-            PyObject* compiled = at(g_key_compiled);
-            found = at(g_key_forward) != nullptr || (compiled && compiled != Py_None);
-            for (PyObject* key : {g_key_hooks, g_key_pre_hooks}) {
-                PyObject* hooks = found ? nullptr : at(key);
-                if (hooks) found = PyObject_IsTrue(hooks);
+        int found = 0;
+        for (Py_ssize_t i = 0; i < n && found == 0; ++i) {
+            PyObject* own = PyObject_GetAttr(args[i], g_attr_dict);
+            if (!own) {
+                if (!PyErr_ExceptionMatches(PyExc_AttributeError)) throw PythonError{};
+                PyErr_Clear();
+                continue;
             }
+            found = 1;
+            if (PyDict_Check(own)) {
+                const auto at = [&](PyObject* key) { return PyDict_GetItemWithError(own, key); };
+                PyObject* compiled = at(g_key_compiled);
+                found = at(g_key_forward) != nullptr || (compiled && compiled != Py_None);
+                for (PyObject* key : {g_key_hooks, g_key_pre_hooks}) {
+                    PyObject* hooks = found ? nullptr : at(key);
+                    if (hooks) found = PyObject_IsTrue(hooks);
+                }
+            }
+            Py_DECREF(own);
         }
-        Py_DECREF(own);
         if (found < 0 || PyErr_Occurred()) throw PythonError{};
         return PyBool_FromLong(found);
     });
@@ -861,7 +864,8 @@ PyMethodDef methods[] = {
     {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_linear)), METH_FASTCALL,
      "(x, weight, block_size, scale_fmt, assume_no_inplace, fused_max_rows, fused_max_bytes, fused_max_bytes_3_rows)"},
     {"mlp", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_mlp)), METH_FASTCALL, "(x, w1, w3, w2, x_fmt, h_fmt, assume_no_inplace)"},
-    {"intercepted", py_intercepted, METH_O, "whether a call of this object does more than its class's forward"},
+    {"intercepted", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_intercepted)), METH_FASTCALL,
+     "whether a call of any of these objects does more than its class's forward"},
     {"fp8_weights", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_fp8_weights)), METH_FASTCALL, "(w1, w3, w2)"},
     {"quantise_remembered", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)(void)>(py_quantise_remembered)), METH_FASTCALL,
      "(x, block_size, scale_fmt, assume_no_inplace)"},

@@ -59,14 +59,13 @@ _UP, _DOWN = ("Linear", "ColumnParallelLinear"), ("Linear", "RowParallelLinear")
 
 
 def _plain_format(model, w1, w3, w2=None):
-    """The scale_fmt that the Linears all hand to the installed ``linear``, where they do nothing but that (classes of the names
-    above, no bias, no hooks, no code of their own); otherwise False."""
+    """The scale_fmt that the Linears, which nothing intercepts, all hand to the installed ``linear``, where they do nothing but that
+    (classes of the names above, no bias, no code of their own); otherwise False."""
     if (getattr(model, "world_size", 1) != 1 or not installed_linear(model) or _nn_module._global_forward_hooks
             or _nn_module._global_forward_pre_hooks):
         return False
-    up, intercepted = type(w1), host.intercepted
-    if (up.__name__ not in _UP or intercepted(w1) or intercepted(w3) or getattr(w1, "bias", None) is not None
-            or getattr(w3, "bias", None) is not None):
+    up = type(w1)
+    if up.__name__ not in _UP or getattr(w1, "bias", None) is not None or getattr(w3, "bias", None) is not None:
         return False
     takes_fmt = linear_takes_fmt(w1, model, w3 if type(w3) is up else None)
     if takes_fmt is None:
@@ -79,7 +78,7 @@ def _plain_format(model, w1, w3, w2=None):
     if (w3.scale_fmt if takes_fmt else None) != fmt:
         return False
     if w2 is not None:
-        if type(w2).__name__ not in _DOWN or intercepted(w2) or getattr(w2, "bias", None) is not None:
+        if type(w2).__name__ not in _DOWN or getattr(w2, "bias", None) is not None:
             return False
         takes_fmt = linear_takes_fmt(w2, model)
         if takes_fmt is None or (w2.scale_fmt if takes_fmt else None) != fmt:
@@ -92,6 +91,8 @@ def _plain_up(mlp, model):
     activations; otherwise None.  The three launches of ``host.mlp`` (the quantisation, w1 and w3 with everything up to w2's
     quantisation, w2) are then as good as theirs."""
     w1, w3 = mlp.w1, mlp.w3
+    if host.intercepted(w1, w3):
+        return None
     fmt = _plain_format(model, w1, w3)
     return None if fmt is False else (w1.weight, w3.weight, fmt)
 
@@ -99,12 +100,13 @@ def _plain_up(mlp, model):
 def plain_weights(mlp, x: torch.Tensor, scale_fmt):
     """``(w1, w3, w2)`` weights of an MLP that ``mlp_forward`` serves and whose Linears do nothing but the GEMM in
     ``scale_fmt``, so that a caller may run them itself; otherwise None."""
-    forward = getattr(type(mlp), "forward", None)
-    installed, model = getattr(forward, "_dsv3_mlp", (None, None))
-    if installed is None or installed is not forward or host.intercepted(mlp) or not calls_forward(mlp, model):
+    installed = getattr(type(mlp), "forward", None)
+    seen, model = getattr(installed, "_dsv3_mlp", (None, None))
+    if seen is None or seen is not installed:
         return None
     w1, w2, w3 = mlp.w1, mlp.w2, mlp.w3
-    if _plain_format(model, w1, w3, w2) != scale_fmt or not _fusable(mlp, x, model):
+    if (host.intercepted(mlp, w1, w2, w3) or not calls_forward(mlp, model) or _plain_format(model, w1, w3, w2) != scale_fmt
+            or not _fusable(mlp, x, model)):
         return None
     return w1.weight, w3.weight, w2.weight
 
