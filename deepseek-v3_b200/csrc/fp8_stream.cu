@@ -122,12 +122,16 @@ struct Seg {          // a range of K chunks of one tile
 // The CTA's share of the work; every CTA derives the same plan from the same numbers.  The tiles (the groups' first, then
 // the ordinary weight's) are worked on whole, one after the other per CTA, or (kSplit) where that would leave the machine
 // idle in the last of one or two rounds, the (tile, K chunk) space is cut into equal contiguous ranges, one per CTA.
-// Whole tiles of the ordinary weight are spread evenly among the groups': the ordinary weight is read once and multiplied by
+// Whole tiles of the ordinary weight are spread among the groups': the ordinary weight is read once and multiplied by
 // many tokens, so its tiles keep the tensor core busy and HBM idle while the groups' do the opposite, and side by side on
 // different SMs they share the machine.  Their distance has no factor in common with the number of CTAs, or they would all be
-// the same few CTAs'.  us, ordinary weight last / spread: 32 of 256 experts of 7168 x 2048 with the shared one, 200 tokens
-// 227.7 / 212.4, 333 253.4 / 231.5, 512 307 / 279; 64 of 2048 x 1408 with two, 333 tokens 140.2 / 133.5; 160 of 5120 x 1536 with two, 512
-// 672 / 629.  Where the ordinary weight has more tiles than the groups they stay last (8 of 64 experts of 2048 x 1408, 512
+// the same few CTAs'.  us per layer in a replayed graph, ordinary weight last / spread: 32 of 256 experts of 7168 x 2048 with the shared
+// one, 200 tokens 228.7 / 213.2, 333 256.9 / 228.1, 512 299.5 / 263.5; 160 of 5120 x 1536 with two, 512 658 / 626; 64 of 2048 x 1408 with
+// two, 333 tokens 133.2 / 128.7, 1024 188 / 186.  Where the groups have fewer than twice as many tiles, and the CTAs are even in number,
+// the only such distance is 1: the ordinary weight comes first.  So 16 of 64 experts of 2048 x 1408, 2048 tokens (352 and 352 tiles) 125.5
+// last, 123.8 first, 126.4 at a distance of 3 with the rest at the end; 32 of 256 of 7168 x 2048, 1800 and 2048 398.6, 394.4, 401.2 and
+// 420.2, 411.4, 422.2; 64 of 2048 x 1408, 512 (231 and 88) 143.9, 143.6, 143.7; 32 of those, 600 (143 and 110) 97.4, 97.5, 96.5.
+// Where the ordinary weight has more tiles than the groups they stay last (8 of 64 experts of 2048 x 1408, 512
 // tokens: 59.8 last, 62.2 first): the groups' tiles wait for HBM and are better begun early.  Short ones (less than half the groups' K:
 // w2 of a tensor-parallel shard of the shared expert) stay last as well, where they fill up the last round: two layers of a decode
 // step, one rank of eight, at 16, 32 and 64 tokens 236.2 / 308.1 / 404.7 spread, 234.1 / 305.9 / 401.1 last.
@@ -138,7 +142,7 @@ struct Seg {          // a range of K chunks of one tile
 struct Plan {
     int kc0, kc1;            // K chunks: groups, ordinary weight
     int tiles0, tiles1;      // groups, ordinary weight
-    int every;               // whole tiles: every so-manieth is one of the ordinary weight while there are any (0: they come last)
+    int every;               // whole tiles: every so-manieth is one of the ordinary weight while there are any (1: they come first; 0: last)
     int G;                   // CTAs that take a range
     int units, base, extra;  // the first `extra` CTAs take base + 1 units, the others base
     __device__ __forceinline__ int begin(int cta) const { return cta * base + min(cta, extra); }

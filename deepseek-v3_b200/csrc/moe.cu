@@ -29,7 +29,8 @@ constexpr int kThreads = 256;
 constexpr int kCombineManyTokens = 400, kCombineManyDim = 4096;
 
 // Two bf16 values to a word, each result rounded once to bf16: what a product or sum formed in fp32 and then rounded gives (a
-// product of two bf16 values is exact in fp32, and a sum that is not lies too far from a tie of bf16 to be rounded twice).
+// product of two bf16 values is exact in fp32, and a sum that is not lies too far from a tie of bf16 to be rounded twice; below
+// 2^-126 a product need not be exact in fp32, and is rounded once here where the other form rounds it twice).
 __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -392,9 +393,9 @@ int swiglu_linear_tile(int64_t M, int64_t N, int64_t K) {
     return best;
 }
 
-// Whether that is faster on the device than two GEMMs and swiglu_quant.  Cut tiles are not where the separate launches are at their
-// best: up to 8 rows on weights that the decode kernel takes (but for few K chunks, which nothing cuts), up to 16 and 32 rows on few
-// or long rows of weights, whose GEMMs split K inside clusters.  B200, us per MLP in a graph of as many as displace the L2, five
+// Whether that is faster on the device than two GEMMs and swiglu_quant.  It is not where its tiles are cut and the GEMMs are at their
+// best: up to 8 rows on weights that the decode kernel takes (with few K chunks nothing is cut), and up to 16, 32 and 64 rows on few, or
+// on long, rows of weights, which the GEMMs cut inside clusters.  B200, us per MLP in a graph of as many as displace the L2, five
 // launches / three: 2048 -> 1408 at 1, 8, 16, 48, 256, 1024 rows 12.0 / 15.0, 13.1 / 15.0, 16.3 / 16.5, 19.3 / 17.3, 22.5 / 19.7, 32.1 /
 // 25.6; 1408 -> 2048 at 1, 9, 17 11.8 / 14.6, 16.9 / 16.4, 17.4 / 14.5; 1024 -> 1024 at 1, 8 11.4 / 10.9, 12.6 / 11.0; 4096 -> 1408 at 8,
 // 16, 33 16.4 / 18.7, 19.1 / 20.1, 21.6 / 20.1; 7168 -> 1024 at 16, 24, 33 19.4 / 22.6, 20.3 / 20.6, 23.2 / 22.0; 7168 -> 1536 at 1, 8, 33
