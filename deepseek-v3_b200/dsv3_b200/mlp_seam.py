@@ -37,10 +37,12 @@ def mlp_forward(self, x: torch.Tensor, *, model_module, original) -> torch.Tenso
     w2 = self.w2
     if host.intercepted(w2) or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks:
         return original(self, x)                          # w2 is not called below
-    row_parallel = type(w2).__name__ == "RowParallelLinear"
+    up, down = _plain_up(self, model_module), type(w2).__name__
+    if down == "Linear" and not (up and type(w2) is type(self.w1)) and linear_takes_fmt(w2, model_module) is None:
+        return original(self, x)                          # an adapter of that name, say
+    row_parallel = down == "RowParallelLinear"
     # only plain Linear hands its scale_fmt to linear() (model.py:205); the parallel Linears do not (model.py:233, 262)
-    scale_fmt = None if (row_parallel or type(w2).__name__ == "ColumnParallelLinear") else getattr(w2, "scale_fmt", None)
-    up = _plain_up(self, model_module)
+    scale_fmt = None if (row_parallel or down == "ColumnParallelLinear") else getattr(w2, "scale_fmt", None)
     y = host.mlp(x, up[0], up[1], w2.weight, up[2], scale_fmt, linear_seam._assume_no_inplace) if up else None
     if y is None:
         hq, hs = swiglu_quant(self.w1(x), self.w3(x), scale_fmt)

@@ -198,7 +198,20 @@ def _global_hook(model, mlp, seen):
     return torch.nn.modules.module.register_module_forward_pre_hook(lambda m, i: seen.append(1) if m is mlp.w2 else None).remove
 
 
-@pytest.mark.parametrize("change", [_hook, _own_forward, _global_hook])
+def _adapter(model, mlp, seen):
+    def forward(self, x):
+        seen.append(1)
+        return model.linear(x, self.weight)
+    mlp.w2 = type("Linear", (model.Linear,), {"forward": forward})()
+
+
+def _patched_class(model, mlp, seen):
+    mlp.w1, mlp.w3 = model.ColumnParallelLinear(), model.ColumnParallelLinear()
+    inner = model.Linear.forward
+    model.Linear.forward = lambda self, x: (seen.append(1), inner(self, x))[1]
+
+
+@pytest.mark.parametrize("change", [_hook, _own_forward, _global_hook, _adapter, _patched_class])
 def test_w2_that_is_intercepted_is_called(change):
     model = _model()
     mlp, seen = model.MLP(), []
