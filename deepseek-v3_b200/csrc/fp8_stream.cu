@@ -297,7 +297,8 @@ __device__ __forceinline__ void prefix_groups(const StreamParams& p, int* prefix
 
 // The groups' tensor maps and scale pointers on their way from HBM into the L2, where a CTA's first loads would otherwise wait for
 // them: the weights of the layers in between have long displaced them.  Each CTA asks for a few lines, while what comes before
-// this kernel is still running (the tables do not change; the L2 is the point of coherence).
+// this kernel is still running (the tables do not change; the L2 is the point of coherence).  us per layer in a replayed graph, without /
+// with: 64 experts of 2048 x 1408, 16 and 333 tokens 78.2 / 78.0, 125.7 / 125.4; 32 of 256 of 7168 x 2048, 16 112.3 / 112.1.
 __device__ __forceinline__ void prefetch_tables(const StreamParams& p, int lane, int warp) {
     if (warp != 3) return;
     const int lines = p.n_groups + (p.n_groups * 8 + 127) / 128;
