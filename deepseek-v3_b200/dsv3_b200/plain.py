@@ -18,11 +18,20 @@ from torch.nn.modules import module as _nn_module
 _Module = _nn_module.Module
 
 
-class _Operand:
+class _Fixed(type):
+    """A class whose attributes cannot be set, by way of an object's ``__class__``."""
+
+    def __setattr__(cls, name, value):
+        raise AttributeError(name)
+
+    __delattr__ = __setattr__
+
+
+class _Operand(metaclass=_Fixed):
     __slots__ = ()
 
 
-class _Sealed:
+class _Sealed(metaclass=_Fixed):
     """Attributes as given; none can be set."""
 
     def __init__(self, **attributes):
@@ -34,7 +43,7 @@ class _Sealed:
     __delattr__ = __setattr__
 
 
-class _Call:
+class _Call(metaclass=_Fixed):
     """Keeps the arguments of its calls and returns an operand."""
     __slots__ = ("calls", "result")
 
@@ -100,10 +109,13 @@ def _run(module, model, target, **attributes):
         if run_forward:
             attributes["forward"] = lambda x: run_forward(me, x)
     me = _Sealed(**attributes)
+    before = dict(me.__dict__), dict(stand_in.__dict__)
     if cls.__call__ is _Module._wrapped_call_impl and cls._call_impl is _Module._call_impl:
-        return me.forward(x), x
-    run_call = _sandboxed(cls.__call__, model, stand_in)
-    return (run_call(me, x), x) if run_call else (None, x)
+        y = me.forward(x)
+    else:
+        run_call = _sandboxed(cls.__call__, model, stand_in)
+        y = run_call(me, x) if run_call else None
+    return (y, x) if before == (me.__dict__, stand_in.__dict__) else (None, x)
 
 
 def _judge_linear(lin, model):

@@ -114,12 +114,21 @@ def _new_code(model, mlp, seen):
 
 
 def _subclass(body):
+    """w1 and w3 of a class that is called Linear too, its forward written in the model's own module."""
     def change(model, mlp, seen):
         names = {}
-        exec(body, dict(model.__dict__, seen=seen, torch=torch), names)
+        model.seen = seen
+        exec(body, model.__dict__, names)
         cls = type("Linear", (model.Linear,), {"forward": names["forward"]})
         mlp.w1, mlp.w3 = cls(), cls()
     return change
+
+
+def test_a_class_of_that_name_with_the_same_code_is_plain():
+    model = _model()
+    mlp = model.MLP()
+    _subclass("def forward(self, x):\n y = linear(x, self.weight, self.bias, scale_fmt=self.scale_fmt)\n return y")(model, mlp, [])
+    assert _plain(mlp, model) == (True, True)
 
 
 def _class_call(model, mlp, seen):
@@ -150,6 +159,9 @@ CHANGES = {
     "caught": _subclass("def forward(self, x):\n try:\n  seen.append(1)\n except Exception:\n  pass\n return linear(x, self.weight, self.bias)"),
     "stored": _subclass("def forward(self, x):\n self.x = x\n return linear(x, self.weight, self.bias, self.scale_fmt)"),
     "global": _subclass("def forward(self, x):\n global last\n last = x\n return linear(x, self.weight, self.bias, self.scale_fmt)"),
+    "class attribute": _subclass("def forward(self, x):\n self.__class__.last = x\n return linear(x, self.weight, self.bias, self.scale_fmt)"),
+    "operand's class": _subclass("def forward(self, x):\n x.__class__.last = x\n return linear(x, self.weight, self.bias, self.scale_fmt)"),
+    "dictionary": _subclass("def forward(self, x):\n self.__dict__['last'] = x\n return linear(x, self.weight, self.bias, self.scale_fmt)"),
     "training": _subclass("def forward(self, x):\n if self.training: x = x + 1\n return linear(x, self.weight, self.bias, self.scale_fmt)"),
     "other weight": _subclass("def forward(self, x):\n return linear(x, self.weight_b, self.bias, self.scale_fmt)"),
 }
