@@ -711,10 +711,10 @@ PyObject* py_intercepted(PyObject*, PyObject* const* args, Py_ssize_t n) {
 PyObject* py_fp8_weights(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return guarded([&]() -> PyObject* {
         want_args(n, 3);
-        bool ok = true;
-        for (int i = 0; i < 3; ++i) ok = ok && tensor_arg(args[i]).element_size() == 1;
-        const at::Tensor& w2 = tensor_arg(args[2]);
-        return PyBool_FromLong(ok && w2.dim() > 1 && w2.size(1) % 128 == 0);
+        for (int i = 0; i < 3; ++i)
+            if (!THPVariable_Check(args[i]) || THPVariable_Unpack(args[i]).element_size() != 1) Py_RETURN_FALSE;
+        const at::Tensor& w2 = THPVariable_Unpack(args[2]);
+        return PyBool_FromLong(w2.dim() > 1 && w2.size(1) % 128 == 0);
     });
 }
 

@@ -235,3 +235,13 @@ def test_w2_that_is_intercepted_is_called(change):
         if undo:
             undo()
     assert seen == [1] and torch.equal(y, torch.nn.functional.silu(X + 1) * (X + 1) + 1)
+
+
+def test_weights_that_are_no_fp8_tensors_are_the_hosts():
+    model = _model()
+    for weight in (torch.zeros(128, 128), object()):
+        mlp = model.MLP()
+        model.linear = lambda x, w, bias=None, scale_fmt=None: x + 1
+        del mlp.w3.weight
+        mlp.w3.weight = weight
+        assert torch.equal(mlp(X), torch.nn.functional.silu(X + 1) * (X + 1) + 1)
