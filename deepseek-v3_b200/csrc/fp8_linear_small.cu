@@ -367,17 +367,18 @@ int launch_fp8_linear_small(const void* x, const void* a, const float* a_s, cons
     };
     // Where the row tiles are no more than the SMs and clusters would be of at most four, or no more than twice the SMs and no clusters
     // are needed, one CTA of sixteen or eight warps per row tile does without the exchange, and quantises the activations
-    // with all of them (registers admit one such CTA per SM, or two).  us at 1 / 2 / 4 / 8 rows with weights from HBM, before / so: 2048 -> 1408
+    // with all of them (registers admit one such CTA per SM, or two).  us at 1 / 2 / 4 / 8 rows in a graph with weights from HBM, before / so: 2048 -> 1408
     // 3.69 / 4.07 / 4.21 / 5.33, 3.18 / 3.27 / 3.94 / 3.90; 1408 -> 2048 4.30 / 4.37 / 5.68 / 6.64, 2.97 / 3.02 / 3.59 / 3.46; 4096 -> 1536 4.40 /
     // 4.95 / 5.10 / 6.29, 4.18 / 4.75 / 4.98 / 6.17; 7168 -> 2048 6.78 / 6.93 / 8.08 / 10.67, 6.62 / 6.77 / 8.06 / 10.48; 7168 -> 2304 7.15 / 7.29 /
     // 8.47 / 10.82, 6.87 / 6.99 / 8.22 / 10.69; eight warps, 512 -> 4096 3.07 / 3.18 / 3.79 / 3.60, 2.66 / 2.72 / 2.77 / 3.13.  With more than 24
-    // chunks that the sixteen warps do not share evenly the cluster stays ahead until it is 512 CTAs: 7168 -> 1280 6.21 / 6.34 / 7.52,
-    // 6.34 / 6.52 / 7.73; 7168 -> 1536 6.46 / 6.63 / 7.75, 6.62 / 6.69 / 7.95; 5120 -> 1536 5.34 / 5.45 / 6.74, 5.40 / 5.46 / 6.87; but 6144 -> 1280
-    // 5.72 / 5.79 / 7.11, 5.64 / 5.72 / 7.14.  Sixteen warps in clusters of two instead of four in eight: 7168 -> 576 4.18 / 4.48 / 4.68, 4.32 /
-    // 4.99 / 5.25.  With activations that are quantised already only the exchange is gained, which few chunks, or few CTAs with many, do
+    // chunks to 80 to 127 row tiles the cluster is up to 3 % ahead in a graph, 7168 -> 1536 6.46 / 6.63 / 7.75, 6.62 / 6.69 / 7.95, 5120 -> 1536 5.34 /
+    // 5.45 / 6.74, 5.40 / 5.46 / 6.87, 6144 -> 1280 5.72 / 5.79 / 7.11, 5.64 / 5.72 / 7.14, but behind where the launches come one by one, as a
+    // cluster's launch takes longer: at 1 / 2 rows 6.95 / 7.10, 6.89 / 7.01; 6.05 / 6.11, 5.80 / 5.79; 6.38 / 6.47, 6.10 / 6.21 (weights in the
+    // L2 6.38 / 6.57, 6.08 / 6.34; 5.53 / 5.62, 5.20 / 5.34; 5.82 / 5.91, 5.40 / 5.56).  Sixteen warps in
+    // clusters of two instead of four in eight: 7168 -> 576 4.18 / 4.48 / 4.68, 4.32 / 4.99 / 5.25.  With activations that are quantised already only the exchange is gained, which few chunks, or few CTAs with many, do
     // not pay for: 1408 -> 2048 at one row 3.67, 2.92; but 256 -> 2048 2.47, 2.72; 1024 -> 1024 2.70, 2.82; 4096 -> 768 at eight rows 3.67,
     // 3.89.  (Both kinds of activations take the same layout: their results are the same bit for bit.)
-    const bool pays = prm.kc >= 10 && (prm.kc <= 24 || (rowgroups >= 80 && (prm.kc % 16 == 0 || rowgroups >= 128)));
+    const bool pays = prm.kc >= 10 && (prm.kc <= 24 || rowgroups >= 80);
     if (narrow && M <= 8 && rowgroups <= num_sms() && csize <= 4 && pays && smem_of(16, 1) <= kMaxSmem) {
         wk = 16;
         csize = 1;

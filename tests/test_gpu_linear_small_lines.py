@@ -12,12 +12,10 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("N,K,ctas,warps", [
     (1408, 2048, 88, 16),
     (1280, 3072, 80, 16),           # 24 chunks: any number of row tiles
-    (1280, 3200, 320, 4),           # 25 that sixteen warps do not share evenly: clusters of four
-    (1280, 4096, 80, 16),           # 32 that they do
-    (1264, 4096, 316, 4),           # 79 row tiles
-    (1536, 7168, 384, 4),           # 56 chunks
-    (2032, 7168, 508, 4),           # 127 row tiles
-    (2048, 7168, 128, 16),
+    (1280, 3200, 80, 16),           # 25 chunks, 80 row tiles
+    (1264, 3200, 316, 4),           # 79: clusters of four
+    (1536, 7168, 96, 16),
+    (576, 7168, 288, 4),            # clusters of eight
     (2376, 1280, 149, 8),
 ])
 def test_layout(N, K, ctas, warps):
