@@ -106,6 +106,7 @@ struct StreamParams {
     uint64_t coprime;                   // bit i: i has no factor in common with ctas
     const float* scale[2];              // ordinary weight (its maps are kernel parameters)
     int scale_fmt;
+    int early;                          // StreamGemm::early
     // split tiles
     float* partials;                    // [CTA][2][2 * BN / 4][128] float4, or null: whole tiles only
     int* tickets;                       // one per CTA, zero on entry and on exit
@@ -242,8 +243,8 @@ struct Walker {
             s.group = lo;
             nq = prefix[lo + 1] - prefix[lo];
             at -= prefix[lo] * per;
-            first = seg[lo];
-            rows = seg[lo + 1] - first;
+            first = BN == 128 ? __ldcg(seg + lo) : seg[lo];
+            rows = (BN == 128 ? __ldcg(seg + lo + 1) : seg[lo + 1]) - first;
         } else {
             s.group = 0;
             rows = p.side[kOrdinary].rows;
@@ -266,7 +267,7 @@ __device__ __forceinline__ void prefix_groups(const StreamParams& p, int* prefix
     if (threadIdx.x < kMaxGroups) {
         const int e = threadIdx.x;
         if (e < p.n_groups) {
-            const int first = __ldg(p.seg + e), end = __ldg(p.seg + e + 1);
+            const int first = __ldcg(p.seg + e), end = __ldcg(p.seg + e + 1);
             const int rows = end - first;
             v = rows >= p.min_rows && rows <= p.max_rows ? (rows + BN - 1) / BN : 0;
             if (seg) {
@@ -308,7 +309,8 @@ __device__ __forceinline__ void prefetch_tables(const StreamParams& p, int lane,
 }
 
 // The TMA producer (one converged warp).  Stage: [BN token rows][block 0][block 1] of one K chunk; of the tokens only
-// the boxes that hold any of the tile's rows are fetched.
+// the boxes that hold any of the tile's rows are fetched.  With `early` the kernel before this one may still be running: the first
+// weights are fetched all the same, the tokens, which it writes, behind the wait for it.
 template <class C, bool kSwiglu, bool kBoth, bool kSplit>
 __device__ __forceinline__ void produce(const StreamParams& p, const Plan& pl, const int* prefix, const int* seg, const void* w0, const void* w1,
                                         const void* ta0, const void* ta1, uint32_t tiles, uint32_t bar0, Control* ctl) {
@@ -316,7 +318,7 @@ __device__ __forceinline__ void produce(const StreamParams& p, const Plan& pl, c
     Walker<BN, kBoth, kSplit> wk(p, pl, prefix, seg);
     Seg s;
     uint32_t g = 0;
-    bool ok = true;
+    bool ok = true, early = p.early != 0;
     while (ok && wk.next(s)) {
         const void* m0 = (!kBoth || s.side == kGroups) ? static_cast<const void*>(p.g_map[0] + s.group) : w0;
         const void* m1 = (!kBoth || s.side == kGroups) ? static_cast<const void*>(p.g_map[1] + s.group) : w1;
@@ -326,7 +328,30 @@ __device__ __forceinline__ void produce(const StreamParams& p, const Plan& pl, c
         const bool two = kSwiglu || 2 * s.p + 1 < p.side[kBoth ? s.side : kGroups].nblk;
         const int boxes = (s.ntok + C::kBox - 1) / C::kBox;
         const uint32_t bytes = (two ? 2u : 1u) * kPRows * kChunk + static_cast<uint32_t>(boxes) * C::kBox * kChunk;
-        for (int k = s.c0; k < s.c1; ++k, ++g) {
+        int k = s.c0;
+        if (early) {
+            early = false;
+            const int n = min(NS, s.c1 - s.c0);
+            if (elect_one()) {
+                for (int i = 0; i < n; ++i) {
+                    const uint32_t full = bar0 + 8u * i, dst = tiles + i * C::kStageBytes;
+                    mbar_arrive_expect_tx(full, bytes);
+                    tma_load_2d(dst + C::kTokBytes, m0, (k + i) * kChunk, r0, full);
+                    if (two) tma_load_2d(dst + C::kTokBytes + kPRows * kChunk, m1, (k + i) * kChunk, r1, full);
+                }
+            }
+            __syncwarp();
+            griddep_wait();
+            if (elect_one()) {
+                for (int i = 0; i < n; ++i)
+                    for (int b = 0; b < boxes; ++b)
+                        tma_load_2d(tiles + i * C::kStageBytes + b * C::kBox * kChunk, ta, (k + i) * kChunk, s.row0 + b * C::kBox, bar0 + 8u * i);
+            }
+            __syncwarp();
+            k += n;
+            g = n;
+        }
+        for (; k < s.c1; ++k, ++g) {
             const int st = g % NS;
             const uint32_t full = bar0 + 8u * st, empty = bar0 + 8u * (NS + st);
             ok = __all_sync(0xffffffffu, bounded_wait(empty, ((g / NS) & 1u) ^ 1u, ctl, p.status, 1, g));
@@ -341,6 +366,7 @@ __device__ __forceinline__ void produce(const StreamParams& p, const Plan& pl, c
             __syncwarp();
         }
     }
+    if (early) griddep_wait();                 // (no work)
     // nothing else waits for the commits onto the empty[] barriers of the last chunks: none may be in flight
     // when the CTA leaves (it would land in whatever CTA gets this shared memory next)
     for (uint32_t d = (g > static_cast<uint32_t>(NS) ? g - NS : 0u); ok && d < g; ++d)
@@ -440,9 +466,9 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
         }
     }
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
-    griddep_launch_dependents();
     prefetch_tables(p, lane, warp);
-    griddep_wait();
+    if (!p.early) griddep_wait();
+    griddep_launch_dependents();               // behind the wait: what an early dependent relies on
     prefix_groups<BN>(p, prefix, scan, seg, warp, lane);
     tc_fence_before();
     __syncthreads();
@@ -450,6 +476,7 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
     const uint32_t tmem_base = ctl->tmem_base;
     const Plan pl = make_plan<BN, kBoth, kSplit>(p, prefix[kMaxGroups]);
 
+    if (p.early && warp != 0) griddep_wait();  // (the producer: behind its first weights)
     if (warp < kFirstPromoWarp) {
       if constexpr (NP >= 2) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControlM));
       if (warp == 0) {
@@ -857,9 +884,9 @@ __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUt
         }
     }
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
-    griddep_launch_dependents();
     prefetch_tables(p, lane, warp);
-    griddep_wait();
+    if (!p.early) griddep_wait();
+    griddep_launch_dependents();               // behind the wait: what an early dependent relies on
     prefix_groups<BN>(p, prefix, scan, static_cast<int*>(nullptr), warp, lane);
     tc_fence_before();
     __syncthreads();
@@ -867,6 +894,7 @@ __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUt
     const uint32_t tmem_base = ctl->tmem_base;
     const Plan pl = make_plan<BN, kBoth, kSplit>(p, prefix[kMaxGroups]);
 
+    if (p.early && warp != 0) griddep_wait();  // (the producer: behind its first weights)
     if (warp < kFirstPromoWarp) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsControl));
         if (warp == 0) {
@@ -1245,6 +1273,7 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
     prm.n_groups = q.n_groups;
     prm.max_rows = INT32_MAX;
     prm.scale_fmt = q.scale_fmt;
+    prm.early = q.early ? 1 : 0;
     prm.status = status_device_ptr();
     if (!prm.status) return DSV3_ERR_CUDA;
     // cutting tiles is worth considering when one or two rounds of whole tiles are expected (struct Plan)

@@ -529,9 +529,8 @@ std::unique_ptr<Routed> run_experts(PyObject* capsule, Experts& e, const at::Ten
         int rc = dsv3_moe_dispatch(xp, T, dim, ip, wp, bf16, r->topk, e.start, e.n, e.fmt, seg, reinterpret_cast<int32_t*>(base + o_pos),
                                    base + o_w, xqp, xsp, base + o_xq, xs_t, st);
         if (rc == DSV3_OK)
-            rc = dsv3_swiglu_gemm_rows(t1, t3, e.n, base + o_xq, xs_t, seg, P, hint, inter, dim, e.fmt, base + o_hq, hs_t, sh ? &up : nullptr, ws,
-                                       ws_bytes, st);
-        if (rc == DSV3_OK) rc = dsv3_fp8_gemm_rows(t2, e.n, base + o_hq, hs_t, seg, P, hint, dim, inter, base + o_o, sh ? &down : nullptr, ws, ws_bytes, st);
+            rc = dsv3_expert_gemms(t1, t3, t2, e.n, base + o_xq, xs_t, seg, P, hint, inter, dim, e.fmt, base + o_hq, hs_t, base + o_o,
+                                   sh ? &up : nullptr, sh ? &down : nullptr, ws, ws_bytes, st);
         return rc;
     });
     remember(x, 128, e.fmt, assume_no_inplace, xq, xs);

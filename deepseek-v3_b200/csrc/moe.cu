@@ -443,7 +443,7 @@ int add_ordinary(StreamGemm& q, const dsv3_side_gemm_t* s) {
 
 int grouped_plain(const void* table, int n, const void* a, const float* a_s, bool transposed, const int32_t* seg, int64_t rows_total,
                   int64_t rows_hint, int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace, size_t workspace_bytes,
-                  dsv3_stream_t stream) {
+                  bool early, dsv3_stream_t stream) {
     int rc = check_groups(n, a, K);
     if (rc != DSV3_OK) return rc;
     StreamGemm q = {};
@@ -453,6 +453,7 @@ int grouped_plain(const void* table, int n, const void* a, const float* a_s, boo
     q.n_groups = n;
     q.table0 = table;
     q.seg = seg;
+    q.early = early;
     q.workspace = workspace;
     q.workspace_bytes = workspace_bytes;
     if ((rc = add_ordinary(q, side)) != DSV3_OK) return rc;
@@ -489,12 +490,12 @@ int dsv3_fp8_gemm_grouped(const void* table, int n_groups, const void* a, const 
         set_last_error("fp8_gemm_grouped: null pointer");
         return DSV3_ERR_INVALID_ARGUMENT;
     }
-    return grouped_plain(table, n_groups, a, a_s, false, seg, rows_total, rows_hint, N, K, c, nullptr, nullptr, 0, stream);
+    return grouped_plain(table, n_groups, a, a_s, false, seg, rows_total, rows_hint, N, K, c, nullptr, nullptr, 0, false, stream);
 }
 
-int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total,
-                       int64_t rows_hint, int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace,
-                       size_t workspace_bytes, dsv3_stream_t stream) {
+static int gemm_rows(const void* table, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total, int64_t rows_hint,
+                     int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace, size_t workspace_bytes, bool early,
+                     dsv3_stream_t stream) {
     if (rows_total < 0 || rows_hint < 0 || N < 0 || K <= 0) {
         set_last_error("fp8_gemm_rows: negative size");
         return DSV3_ERR_INVALID_ARGUMENT;
@@ -504,7 +505,13 @@ int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const flo
         set_last_error("fp8_gemm_rows: null pointer");
         return DSV3_ERR_INVALID_ARGUMENT;
     }
-    return grouped_plain(table, n_groups, a, a_s_t, true, seg, rows_total, rows_hint, N, K, c, side, workspace, workspace_bytes, stream);
+    return grouped_plain(table, n_groups, a, a_s_t, true, seg, rows_total, rows_hint, N, K, c, side, workspace, workspace_bytes, early, stream);
+}
+
+int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total,
+                       int64_t rows_hint, int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace,
+                       size_t workspace_bytes, dsv3_stream_t stream) {
+    return gemm_rows(table, n_groups, a, a_s_t, seg, rows_total, rows_hint, N, K, c, side, workspace, workspace_bytes, false, stream);
 }
 
 int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, const void* a, const float* a_s_t, const int32_t* seg,
@@ -546,6 +553,17 @@ int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, 
     q.workspace_bytes = workspace_bytes;
     if ((rc = add_ordinary(q, side)) != DSV3_OK) return rc;
     return launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
+}
+
+// The second launch begins to read its weights while the CTAs of the first leave (StreamGemm::early).
+int dsv3_expert_gemms(const void* table1, const void* table3, const void* table2, int n_groups, const void* a, const float* a_s_t, const int32_t* seg,
+                      int64_t rows_total, int64_t rows_hint, int64_t inter, int64_t dim, int scale_fmt, void* hq, float* hs_t, void* o,
+                      const dsv3_side_gemm_t* up, const dsv3_side_gemm_t* down, void* workspace, size_t workspace_bytes, dsv3_stream_t stream) {
+    const int rc = dsv3_swiglu_gemm_rows(table1, table3, n_groups, a, a_s_t, seg, rows_total, rows_hint, inter, dim, scale_fmt, hq, hs_t, up, workspace,
+                                         workspace_bytes, stream);
+    if (rc != DSV3_OK) return rc;
+    return gemm_rows(table2, n_groups, hq, hs_t, seg, rows_total, rows_hint, dim, inter, o, down, workspace, workspace_bytes,
+                     rows_total > 0 && inter > 0, stream);
 }
 
 // (a kernel or split that the host pinned is one of fp8_gemm's: the separate launches honour or refuse it)
