@@ -21,18 +21,21 @@ __device__ __forceinline__ float scale_from_amax(float amax, int scale_fmt) {
     return s;
 }
 
-__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+// The larger magnitudes of two pairs of bf16 values, with signs that say nothing; a NaN gives way to the other operand.
+__device__ __forceinline__ uint32_t max_abs_bf16x2(uint32_t a, uint32_t b) {
     uint32_t d;
-    asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
-
-// max|x| of eight bf16 values
-__device__ __forceinline__ float amax8(const uint4& v) {
-    // two values to a word; a NaN gives way to the other operand, and a lane of nothing but NaN returns one, which fmaxf drops
-    const uint32_t m = max_bf16x2(max_bf16x2(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu), max_bf16x2(v.z & 0x7FFF7FFFu, v.w & 0x7FFF7FFFu));
+__device__ __forceinline__ uint32_t max_abs8(const uint4& v) { return max_abs_bf16x2(max_abs_bf16x2(v.x, v.y), max_abs_bf16x2(v.z, v.w)); }
+// The larger of a pair's magnitudes; a NaN is dropped.
+__device__ __forceinline__ float amax_of_pair(uint32_t m) {
+    m &= 0x7FFF7FFFu;
     return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xFFFF0000u));
 }
+
+// max|x| of eight bf16 values (two values to a word; a lane of nothing but NaN is one, which fmaxf drops)
+__device__ __forceinline__ float amax8(const uint4& v) { return amax_of_pair(max_abs8(v)); }
 
 __device__ __forceinline__ float rcp_approx(float s) {
     float r;
@@ -103,24 +106,18 @@ static __device__ __noinline__ float silu_exact(float a) {
     return __bfloat162float(__float2bfloat16_rn(a / (1.0f + expf(-a))));
 }
 
-__device__ __forceinline__ uint32_t swiglu2_exact(uint32_t a2, uint32_t b2) {
-    const float lo = silu_exact(bf16_bits_to_float(a2 & 0xFFFFu)), hi = silu_exact(__uint_as_float(a2 & 0xFFFF0000u));
-    return pack_bf16x2(lo * bf16_bits_to_float(b2 & 0xFFFFu), hi * __uint_as_float(b2 & 0xFFFF0000u));
-}
-
 // h = bf16(bf16(silu(a)) * b) for eight bf16 pairs.
-// The fast form a * rcp(1 + ex2(-a log2 e)) is within 2^-19.5 of the exact form for |a| <= 15 (ex2: 2 ulp, its rounded
-// argument 1.2 |a| ulp, rcp 1 ulp, two roundings, and 2 ulp for the exact form's own expf).  It is rounded to bf16 once a
-// little below and once a little above itself: where the two agree they are the exact form's value, where they
-// disagree (0.05 % of values) or a value lies outside that range the exact form is evaluated.  16 instructions per
-// value instead of 40; the exact form is a call, since inlined into an unrolled epilogue it outgrew the instruction cache
-// (20000 cycles per tile).
+// silu's fast form, a * rcp(1 + ex2(-a log2 e)), is within 13 ulp of fp32 of the exact one, and rounds to the same bf16 value for every
+// bf16 a but -87.5, -88 and -88.5, whose reciprocals are flushed (all 65536 checked on a B200): those are a * exp(a / 2) * exp(a / 2).
+// The product of two bf16 values is rounded once, as by way of fp32, which holds it exactly unless it is below 2^-126.
+// The exact form by a call where the fast one lay near a rounding boundary (0.05 % of values, 13 % of a warp's trips) cost the epilogue of a
+// 128-token tile 2300 of 9700 cycles, the check, the separate product and the maximum per word another 600.  us, with them / without: w1 and w3 of 64
+// experts of 2048 x 1408, 512 rows each 256 / 225, of 32 of 7168 x 2048 485 / 451; swiglu_quant 8192 x 18432 127 / 111, ue8m0 138 / 112,
+// 2048 x 2048 6.8 / 5.0; MLP 2048 -> 2816 at 500 rows 28.1 / 26.6.
 __device__ __forceinline__ uint4 swiglu8(const uint4& a, const uint4& b) {
     const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
     constexpr float kLog2e = 1.44269504088896340736f;
-    constexpr float kEps = 1.34e-6f;       // 2^-19.5
-    uint32_t h[4], diff[4];
-    __nv_bfloat162 top = __float2bfloat162_rn(0.0f);
+    uint32_t h[4], top = 0u;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         // two values to an FP32 instruction: with one each, swiglu_quant was bound by issue (8192 x 18432 142.9 us, 134.0 so)
@@ -133,20 +130,23 @@ __device__ __forceinline__ uint4 swiglu8(const uint4& a, const uint4& b) {
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r2.x) : "f"(e2.x));
         asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r2.y) : "f"(e2.y));
         const float2 s2 = __fmul2_rn(a2, r2);
-        const float2 lo2 = __fmul2_rn(s2, make_float2(1.0f - kEps, 1.0f - kEps)), hi2 = __fmul2_rn(s2, make_float2(1.0f + kEps, 1.0f + kEps));
-        const uint32_t below = pack_bf16x2(lo2.x, lo2.y);
-        const uint32_t above = pack_bf16x2(hi2.x, hi2.y);
-        diff[i] = below ^ above;
-        top = __hmax2_nan(top, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&aw[i])));
-        const float2 h2 = __fmul2_rn(make_float2(bf16_bits_to_float(above & 0xFFFFu), __uint_as_float(above & 0xFFFF0000u)),
-                                     make_float2(bf16_bits_to_float(bw[i] & 0xFFFFu), __uint_as_float(bw[i] & 0xFFFF0000u)));
-        h[i] = pack_bf16x2(h2.x, h2.y);
+        const __nv_bfloat162 silu = __floats2bfloat162_rn(s2.x, s2.y), h2 = __hmul2(silu, *reinterpret_cast<const __nv_bfloat162*>(&bw[i]));
+        h[i] = *reinterpret_cast<const uint32_t*>(&h2);
+        asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(top) : "r"(top), "r"(aw[i]));
     }
-    const bool far = !__hble2(top, __float2bfloat162_rn(15.0f));
-    if (far || (diff[0] | diff[1] | diff[2] | diff[3]) != 0u) {
+    top &= 0x7FFF7FFFu;
+    if (!__hble2(*reinterpret_cast<const __nv_bfloat162*>(&top), __float2bfloat162_rn(87.0f))) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (far || diff[i] != 0u) h[i] = swiglu2_exact(aw[i], bw[i]);
+        for (int i = 0; i < 8; ++i) {
+            const int up = i & 1 ? 0 : 16;              // shifts the value to the upper half of the word
+            const float v = __uint_as_float((aw[i / 2] << up) & 0xFFFF0000u), w = __uint_as_float((bw[i / 2] << up) & 0xFFFF0000u);
+            if (v > -88.7f && v < -87.0f) {
+                float root;
+                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(root) : "f"(v * (0.5f * kLog2e)));
+                const uint32_t r = __bfloat16_as_ushort(__float2bfloat16_rn(__bfloat162float(__float2bfloat16_rn(v * root * root)) * w));
+                h[i / 2] = up ? (h[i / 2] & 0xFFFF0000u) | r : (h[i / 2] & 0xFFFFu) | (r << 16);
+            }
+        }
     }
     return make_uint4(h[0], h[1], h[2], h[3]);
 }
