@@ -106,7 +106,7 @@ struct StreamParams {
     uint64_t coprime;                   // bit i: i has no factor in common with ctas
     const float* scale[2];              // ordinary weight (its maps are kernel parameters)
     int scale_fmt;
-    int early;                          // StreamGemm::early
+    int leads, early;                   // StreamGemm::leads, early
     // split tiles
     float* partials;                    // [CTA][2][2 * BN / 4][128] float4, or null: whole tiles only
     int* tickets;                       // one per CTA, zero on entry and on exit
@@ -466,9 +466,10 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
         }
     }
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
+    if (!p.leads) griddep_launch_dependents();
     prefetch_tables(p, lane, warp);
     if (!p.early) griddep_wait();
-    griddep_launch_dependents();               // behind the wait: what an early dependent relies on
+    if (p.leads) griddep_launch_dependents();  // behind the wait: what an early dependent relies on
     prefix_groups<BN>(p, prefix, scan, seg, warp, lane);
     tc_fence_before();
     __syncthreads();
@@ -884,9 +885,10 @@ __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUt
         }
     }
     if (warp == 1) tc_alloc(smem_u32(&ctl->tmem_base), C::kTmemCols);
+    if (!p.leads) griddep_launch_dependents();
     prefetch_tables(p, lane, warp);
     if (!p.early) griddep_wait();
-    griddep_launch_dependents();               // behind the wait: what an early dependent relies on
+    if (p.leads) griddep_launch_dependents();  // behind the wait: what an early dependent relies on
     prefix_groups<BN>(p, prefix, scan, static_cast<int*>(nullptr), warp, lane);
     tc_fence_before();
     __syncthreads();
@@ -1274,6 +1276,7 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
     prm.n_groups = q.n_groups;
     prm.max_rows = INT32_MAX;
     prm.scale_fmt = q.scale_fmt;
+    prm.leads = q.leads ? 1 : 0;
     prm.early = q.early ? 1 : 0;
     prm.status = status_device_ptr();
     if (!prm.status) return DSV3_ERR_CUDA;

@@ -73,13 +73,13 @@ struct StreamGemm {
     const void *w0, *w1;               // e4m3 [N, K]; w1 only with swiglu
     const float *w0_s, *w1_s;
     bool swiglu;
-    // The launch before this one on the stream is another of these, and only its results (a, a_s, and c's memory) have to be waited
+    // early: the launch before this one on the stream is another of these, with `leads`, and only its results (a, a_s, and c's memory) have to be waited
     // for: row offsets, tables and weights are read while it still runs.  They are complete by then, since it lets its dependents
     // start only once what came before it has finished.  w2's CTAs plan their tiles and fill their rings with weights on the SMs that
     // w1's and w3's have left; us per layer, without / with: 64 experts of 2048 x 1408, 7 and 333 tokens 61.7 / 57.3, 135.0 / 132.6, 8 of them
     // and 62 39.9 / 37.6; 20 of 160 of 5120 x 1536, 442 145.4 / 138.8, all 160 and 40 356.5 / 353.0; two layers of a decode step, one rank of
     // eight, 16 sequences 230.2 / 223.3; 256 experts of 7168 x 2048, 2048 tokens 2373 / 2379 (their runs differ by 1 %).
-    bool early;
+    bool leads, early;
     int scale_fmt;
     int tile;                          // tokens per tile (16, 32, 64, 128), or 0: by rows_expected
     void* workspace;                   // stream_workspace_bytes(), or null: tiles are not split

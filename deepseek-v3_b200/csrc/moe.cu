@@ -514,9 +514,9 @@ int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const flo
     return gemm_rows(table, n_groups, a, a_s_t, seg, rows_total, rows_hint, N, K, c, side, workspace, workspace_bytes, false, stream);
 }
 
-int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, const void* a, const float* a_s_t, const int32_t* seg,
-                          int64_t rows_total, int64_t rows_hint, int64_t N, int64_t K, int scale_fmt, void* hq, float* hs_t,
-                          const dsv3_side_gemm_t* side, void* workspace, size_t workspace_bytes, dsv3_stream_t stream) {
+static int swiglu_rows(const void* table1, const void* table3, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total,
+                       int64_t rows_hint, int64_t N, int64_t K, int scale_fmt, void* hq, float* hs_t, const dsv3_side_gemm_t* side, void* workspace,
+                       size_t workspace_bytes, bool leads, dsv3_stream_t stream) {
     if (rows_total < 0 || rows_hint < 0 || N < 0 || K <= 0) {
         set_last_error("swiglu_gemm_rows: negative size");
         return DSV3_ERR_INVALID_ARGUMENT;
@@ -548,6 +548,7 @@ int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, 
     q.table1 = table3;
     q.seg = seg;
     q.swiglu = true;
+    q.leads = leads;
     q.scale_fmt = scale_fmt;
     q.workspace = workspace;
     q.workspace_bytes = workspace_bytes;
@@ -555,12 +556,19 @@ int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, 
     return launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
 }
 
+int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, const void* a, const float* a_s_t, const int32_t* seg,
+                          int64_t rows_total, int64_t rows_hint, int64_t N, int64_t K, int scale_fmt, void* hq, float* hs_t,
+                          const dsv3_side_gemm_t* side, void* workspace, size_t workspace_bytes, dsv3_stream_t stream) {
+    return swiglu_rows(table1, table3, n_groups, a, a_s_t, seg, rows_total, rows_hint, N, K, scale_fmt, hq, hs_t, side, workspace, workspace_bytes, false,
+                       stream);
+}
+
 // The second launch begins to read its weights while the CTAs of the first leave (StreamGemm::early).
 int dsv3_expert_gemms(const void* table1, const void* table3, const void* table2, int n_groups, const void* a, const float* a_s_t, const int32_t* seg,
                       int64_t rows_total, int64_t rows_hint, int64_t inter, int64_t dim, int scale_fmt, void* hq, float* hs_t, void* o,
                       const dsv3_side_gemm_t* up, const dsv3_side_gemm_t* down, void* workspace, size_t workspace_bytes, dsv3_stream_t stream) {
-    const int rc = dsv3_swiglu_gemm_rows(table1, table3, n_groups, a, a_s_t, seg, rows_total, rows_hint, inter, dim, scale_fmt, hq, hs_t, up, workspace,
-                                         workspace_bytes, stream);
+    const int rc = swiglu_rows(table1, table3, n_groups, a, a_s_t, seg, rows_total, rows_hint, inter, dim, scale_fmt, hq, hs_t, up, workspace,
+                               workspace_bytes, true, stream);
     if (rc != DSV3_OK) return rc;
     return gemm_rows(table2, n_groups, hq, hs_t, seg, rows_total, rows_hint, dim, inter, o, down, workspace, workspace_bytes,
                      rows_total > 0 && inter > 0, stream);
