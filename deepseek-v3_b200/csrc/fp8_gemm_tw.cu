@@ -130,7 +130,7 @@ __device__ __forceinline__ Strip decode_strip(int pair, const TwParams& p) {
     return s;
 }
 
-template <int kBlock>      // K chunks per scale load: 4 (K chunks a multiple of four, 16-byte aligned scales) or 1
+template <int kBlock>      // K chunks per scale load: 4 (K chunks a multiple of four, 16-byte aligned scales), 2 (of two, 8-byte) or 1
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                    const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_s, const TwParams p) {
@@ -374,7 +374,8 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         // as much L2 traffic as the operands and a wait in every chunk (M 4096, N 7168, K 16384: 465 us, with no scale loads
         // at all 419, as here 430).  One 16-byte load brings four chunks; it is issued as soon as the fourth
         // product is formed and has that chunk's time to arrive.  Rows that 16-byte loads cannot read (K chunks not a
-        // multiple of four) take the scalar form, kBlock = 1.
+        // multiple of four) take 8-byte loads, kBlock = 2, or the scalar form; scalar / 8-byte, M 4096, N 7168, K 2304 64.2 / 62.6 us, M 8862,
+        // N 2608, K 8960 195.4 / 190.7, M 2000, N 2048, K 2816 15.9 / 15.5.
         float ra[kBlock], rb[kBlock];
         auto next_scales = [&](const float* as, const float* bs, int k) {
             if (k >= kc) return;
@@ -382,6 +383,10 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 const float4 a4 = __ldg(reinterpret_cast<const float4*>(as + k)), b4 = __ldg(reinterpret_cast<const float4*>(bs + k));
                 ra[0] = a4.x; ra[1] = a4.y; ra[2] = a4.z; ra[3] = a4.w;
                 rb[0] = b4.x; rb[1] = b4.y; rb[2] = b4.z; rb[3] = b4.w;
+            } else if constexpr (kBlock == 2) {
+                const float2 a2 = __ldg(reinterpret_cast<const float2*>(as + k)), b2 = __ldg(reinterpret_cast<const float2*>(bs + k));
+                ra[0] = a2.x; ra[1] = a2.y;
+                rb[0] = b2.x; rb[1] = b2.y;
             } else {
                 ra[0] = __ldg(as + k);
                 rb[0] = __ldg(bs + k);
@@ -579,8 +584,8 @@ int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const flo
     CUtensorMap ts = tb;
     if (prm.tail_w && (rc = make_tmap(&ts, b, N, K, prm.tail_w / 2)) != DSV3_OK) return rc;
 
-    const bool vec = (prm.kc % 4) == 0 && ((reinterpret_cast<uintptr_t>(a_s) | reinterpret_cast<uintptr_t>(b_s)) % 16) == 0;
-    auto kern = vec ? fp8_gemm_tw_kernel<4> : fp8_gemm_tw_kernel<1>;
+    const auto aligned = [&](int n) { return (prm.kc % n) == 0 && ((reinterpret_cast<uintptr_t>(a_s) | reinterpret_cast<uintptr_t>(b_s)) % (4 * n)) == 0; };
+    auto kern = aligned(4) ? fp8_gemm_tw_kernel<4> : aligned(2) ? fp8_gemm_tw_kernel<2> : fp8_gemm_tw_kernel<1>;
     static bool configured[64] = {};
     int dev = 0;
     DSV3_CUDA_TRY(cudaGetDevice(&dev));
@@ -590,6 +595,7 @@ int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const flo
     }
     if (!configured[dev]) {
         DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+        DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
         DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
         configured[dev] = true;
     }
