@@ -4,29 +4,31 @@
 //
 // Replaces inference/kernel.py:118-172 (fp8_gemm_kernel) and its launch at :194-195 for prefill-sized M.
 //
-// Why 256 columns.  A tcgen05.mma reads its operands from shared memory every time it is issued: M128 N128 K32
-// (per SM) takes 8 KB for 64 tensor-core cycles, 128 B/clk, which is all shared memory delivers, and the TMA
-// writes of the next operands compete for the same bandwidth; measured, such tiles stop at half of the tensor
-// pipe's rate.  With N = 256 an instruction runs 128 cycles on 12 KB (4 KB of tokens, 8 KB of weights of which
-// half sit in the peer's shared memory), 96 B/clk, and a chunk needs 32 KB of loads per SM for 512 tensor-core
-// cycles instead of 24 KB for 256.  The price: the fp32 accumulator of one SM is 128 x 256 (128 registers in each
-// of 256 promotion threads), TMEM holds only two chunk products, and the read-back buffer shrinks to 64
-// registers per thread.
+// Why 256 columns.  An SM takes about 60 bytes per clock from the L2: a chunk of 256 columns needs 32 KB of loads per SM for 512
+// tensor-core cycles, one of 128 columns 24 KB for 256.  The price: the fp32 accumulator of one SM is 128 x 256 (128 registers in each
+// of 256 promotion threads), TMEM holds only two chunk products, and the read-back buffer shrinks to 64 registers per thread.
+//
+// Why each product in two halves (N128).  A slot handed back as a whole was away for 1100 cycles besides its own 512 (commit, wake-up,
+// two read-backs with the FMAs between them, arrivals from both CTAs, issue), so that two slots gave a product every 810 cycles.
+// As halves, one for either warp group, the next product's left half is computed while the right one is still being read: 675.  The tokens
+// are read from shared memory twice for that, 96 instead of 64 bytes per clock.  In a loop of launches the clock falls with the
+// work it does (1 kW): us, whole slots / halves, act_quant included, M 500, N 7168, K 7168 35.6 / 34.2; M 867, N 18432, K 7168 126.8 / 123.4; M 4096, N 7168,
+// K 16384 495 / 490; MLP 5120 -> 12288 at 2693 rows 538 / 521, 7168 -> 18432 at 8192 3098 / 3038.
 //
 // Roles, per CTA (r = rank in the pair; the even CTA is the leader):
-//   warp 0            TMA producer (converged, one elected lane issues): stage = one K chunk = 16 KB tokens + 16 KB weights (this CTA's 128 of the
-//                     tile's 256 weight rows), five stages.  Both producers' loads complete on the LEADER's full[]
+//   warp 0            TMA producer (converged, one elected lane issues): stage = one K chunk = 16 KB tokens + 16 KB weights (64 rows
+//                     of either 128-row block of the tile), five stages.  Both producers' loads complete on the LEADER's full[]
 //                     barrier (ordinary, non-multicast loads; only the completion signal crosses to the peer),
 //                     each waits on its own empty[].
 //   warps 1,2         leader only: MMA issuers (converged, one elected lane issues); chunk g belongs to issuer g % 2, which owns TMEM slot g % 2.
-//                     Per chunk: wait full[stage], wait tempty[slot] (16 arrivals: the promotion warps of both CTAs),
-//                     4 x tcgen05.mma.cta_group::2 kind::f8f6f4 (M256 N256 K32), commit -> tfull[slot] and
-//                     empty[stage] of both CTAs.  Stages alternate between the issuers, so full[] is waited for
+//                     Per chunk: wait full[stage]; per half: wait tempty[half][slot] (8 arrivals: the half's promotion warps of both
+//                     CTAs), 4 x tcgen05.mma.cta_group::2 kind::f8f6f4 (M256 N128 K32), commit -> tfull[half][slot] of both CTAs,
+//                     behind the second half also empty[stage].  Stages alternate between the issuers, so full[] is waited for
 //                     without a probe.
 //   warps 4..11       promotion of this CTA's 128 x 256 half: warps 4..7 own columns 0..127 (one b_s block), warps
-//                     8..11 columns 128..255; a thread owns one accumulator row.  A chunk product is read back in
-//                     two halves of 64 columns through one buffer; the slot goes back to the issuer when the second
-//                     load has landed, and that half's FMAs follow the release.
+//                     8..11 columns 128..255; a thread owns one accumulator row.  A half product is read back in
+//                     two pieces of 64 columns through one buffer; the half slot goes back to the issuer when the second
+//                     load has landed, and that piece's FMAs follow the release.
 //                     Result tile: bf16 through shared memory and TMA stores.
 //
 // Every mbarrier wait is bounded: after about a second the waiting thread records what it was waiting for in
@@ -55,11 +57,11 @@ constexpr int kRegsPromo = 232;
 static_assert(128 * kRegsControl + 256 * kRegsPromo <= 384 * 168, "register pool");
 
 constexpr int kBN = 256;                              // tile width: two b_s blocks, one per promotion warp group
-constexpr int kBHalf = kBN / 2;                       // weight rows each CTA of the pair loads
+constexpr int kBHalf = kBN / 2;                       // weight rows each CTA of the pair loads: half of either 128-row block
 constexpr int kChunkBytes = (kPRows + kBHalf) * kChunk;   // per CTA: token tile + half weight tile of one chunk
 constexpr int kStorePasses = 1;                       // result tile staged whole (1) or one 64-column box per warp group at a time (2)
 constexpr int kStages = kStorePasses == 1 ? 5 : 6;    // of one chunk each
-constexpr int kSlots = 2;                             // TMEM slots of one chunk product (256 columns) each
+constexpr int kSlots = 2;                             // TMEM slots of one chunk product (two halves of 128 columns) each; barriers: [half][slot]
 constexpr int kTmemCols = kSlots * kBN;
 constexpr int kPiece = 32;                            // columns of an FMA batch; a read-back is two of them
 constexpr int kStoreBytes = kPRows * kBN * 2 / kStorePasses;   // bf16 result tile: 128-byte-swizzled 128 x 64 boxes
@@ -69,7 +71,7 @@ static_assert(kSmemBytes > 116 * 1024, "one CTA per SM (it allocates all of TMEM
 static_assert(kTmemCols == 512, "all of TMEM");
 // The issuers alternate, so a stage's full[] barrier is waited for by one issuer at one use and by the other at the
 // next.  A parity wait is only exact for a barrier that is at most one phase behind.  That holds here: an issuer
-// reaches chunk g after it was given its TMEM slot for chunk g - 2, i.e. after the promotion warps have read chunk
+// reaches chunk g after it was given both halves of its TMEM slot for chunk g - 2, i.e. after the promotion warps have read chunk
 // g - 4 and, in order, every chunk before it -- among them chunk g - kStages, the stage's previous use, whose
 // product could only exist after the other issuer had waited for that use's loads.
 static_assert(kStages >= 4 && kSlots == 2, "phase argument for the full[] waits of alternating issuers");
@@ -140,12 +142,12 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     uint8_t* gen_tiles = smem_raw + (tiles - raw);
     uint8_t* store_buf = gen_tiles + kStages * kChunkBytes;                       // 1024-byte aligned (swizzle atom)
     uint64_t* bars = reinterpret_cast<uint64_t*>(store_buf + kStoreBytes);
-    Control* ctl = reinterpret_cast<Control*>(bars + 2 * kStages + 2 * kSlots);
+    Control* ctl = reinterpret_cast<Control*>(bars + 2 * kStages + 4 * kSlots);
     const uint32_t bar0 = smem_u32(bars);
     auto full_bar = [&](int s) { return bar0 + 8u * s; };                        // used in the leader only
     auto empty_bar = [&](int s) { return bar0 + 8u * (kStages + s); };
     auto tfull_bar = [&](int s) { return bar0 + 8u * (2 * kStages + s); };
-    auto tempty_bar = [&](int s) { return bar0 + 8u * (2 * kStages + kSlots + s); };   // used in the leader only
+    auto tempty_bar = [&](int s) { return bar0 + 8u * (2 * kStages + 2 * kSlots + s); };   // used in the leader only
 
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);   // uniform, and known to be
     const int lane = threadIdx.x & 31;
@@ -159,9 +161,9 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
         }
-        for (int s = 0; s < kSlots; ++s) {
+        for (int s = 0; s < 2 * kSlots; ++s) {
             mbar_init(tfull_bar(s), 1);
-            mbar_init(tempty_bar(s), 2 * kPromoThreads / 32);   // every promotion warp of both CTAs reads its half of every slot
+            mbar_init(tempty_bar(s), kPromoThreads / 32);       // one warp group of each CTA reads a half
         }
         ctl->abort_flag = 0;
         mbar_fence_init();
@@ -178,7 +180,8 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         const int n_pre = min(kc, kStages);
         if (pair < p.num_tiles) {
             const Tile t = decode_tile(pair, p);
-            for (int j = 0; j < n_pre; ++j) tma_prefetch_l2_2d(&tmap_b, j * kChunk, t.q * kBN + static_cast<int>(rank) * kBHalf);
+            for (int j = 0; j < n_pre; ++j)
+                for (int h = 0; h < 2; ++h) tma_prefetch_l2_2d(&tmap_b, j * kChunk, t.q * kBN + h * kBHalf + static_cast<int>(rank) * (kBHalf / 2));
         } else if (const Strip s = decode_strip(pair, p); s.any) {
             for (int j = 0; j < n_pre; ++j) tma_prefetch_l2_2d(&tmap_s, j * kChunk, s.n0 + static_cast<int>(rank) * (p.tail_w / 2));
         }
@@ -202,7 +205,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 uint32_t g = 0;
                 uint32_t probe = 0;   // result of test_wait on empty[] for chunk g, issued one chunk earlier
                 bool ok = true;
-                auto load_tile = [&](const void* tmap, int a_row, int b_row, uint32_t bytes) {
+                auto load_tile = [&](const void* tmap, int boxes, int a_row, int b_row, uint32_t bytes) {
                     for (int k = 0; k < kc; ++k, ++g) {
                         const int s = g % kStages;
                         ok = __all_sync(0xffffffffu, wait_probed(probe, empty_bar(s), ((g / kStages) & 1u) ^ 1u, ctl, p.status, 1, g));
@@ -216,16 +219,17 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                             if (rank == 0) mbar_arrive_expect_tx(full_bar(s), bytes);
                             tma_load_2d_pair(dst, &tmap_a, k * kChunk, a_row, lead_full);
                             tma_load_2d_pair(dst + kPRows * kChunk, tmap, k * kChunk, b_row, lead_full);
+                            if (boxes == 2) tma_load_2d_pair(dst + kPRows * kChunk + kBHalf / 2 * kChunk, tmap, k * kChunk, b_row + kBHalf, lead_full);
                         }
                         __syncwarp();
                     }
                 };
                 for (int tile = pair; ok && tile < p.num_tiles; tile += n_pairs) {
                     const Tile t = decode_tile(tile, p);
-                    load_tile(&tmap_b, (2 * t.pp + static_cast<int>(rank)) * kPRows, t.q * kBN + static_cast<int>(rank) * kBHalf, 2 * kChunkBytes);
+                    load_tile(&tmap_b, 2, (2 * t.pp + static_cast<int>(rank)) * kPRows, t.q * kBN + static_cast<int>(rank) * (kBHalf / 2), 2 * kChunkBytes);
                 }
                 if (const Strip st = decode_strip(pair, p); ok && st.any)
-                    load_tile(&tmap_s, (2 * st.t.pp + static_cast<int>(rank)) * kPRows, st.n0 + static_cast<int>(rank) * (p.tail_w / 2),
+                    load_tile(&tmap_s, 1, (2 * st.t.pp + static_cast<int>(rank)) * kPRows, st.n0 + static_cast<int>(rank) * (p.tail_w / 2),
                               2u * (kPRows + p.tail_w / 2) * kChunk);
                 // Nothing waits for the commits onto the empty[] barriers of the last chunks; wait for them here so
                 // that none is in flight when the CTA leaves (it would land in whatever CTA gets this shared memory next).
@@ -234,47 +238,58 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             }
         } else if (warp <= 2) {
             // ------------------------------------------------------------ MMA issuers (leader CTA; chunk g -> issuer g % 2)
-            // One thread issues about one tcgen05 instruction per hundred cycles, and a chunk costs eight (four MMAs,
-            // four commits) for 512 tensor-core cycles: two threads share the chunks, each owning one TMEM slot.
+            // One thread issues about one tcgen05 instruction per hundred cycles, and a chunk costs fourteen (eight MMAs,
+            // six commits) for 512 tensor-core cycles: two threads share the chunks, each owning one TMEM slot.
             // The whole warp walks the loop (waits included) and one elected lane issues: control flow, addresses
             // and descriptors then stay warp-uniform, which is what makes a tcgen05 instruction cheap to issue.
             if (rank == 0) {
                 const uint32_t me = static_cast<uint32_t>(warp - 1);
                 const int slot = static_cast<int>(me);
-                const uint32_t peer_tfull = mapa_shared(tfull_bar(slot), 1);
+                const uint32_t peer_tfull0 = mapa_shared(tfull_bar(0), 1);
                 const uint32_t peer_empty0 = mapa_shared(empty_bar(0), 1);
                 const uint32_t d_tmem = tmem_base + slot * kBN;
                 bool ok = true;
                 uint32_t g = 0;
-                auto multiply_tile = [&](uint32_t idesc) {
+                // parts == 2: the halves of a tile, one after the other; 1: a strip, which both warp groups read
+                auto multiply_tile = [&](uint32_t idesc, int parts) {
                     for (int k = 0; k < kc; ++k, ++g) {
                         if ((g & 1u) != me) continue;
                         const int s = g % kStages;
                         ok = __all_sync(0xffffffffu, bounded_wait(full_bar(s), (g / kStages) & 1u, ctl, p.status, 2, g));
                         if (!ok) break;
-                        ok = __all_sync(0xffffffffu, bounded_wait(tempty_bar(slot), ((g >> 1) & 1u) ^ 1u, ctl, p.status, 3, g));
-                        if (!ok) break;
-                        tc_fence_after();
                         const uint32_t sp = tiles + s * kChunkBytes;
                         const uint64_t da = umma_desc_k_major_sw128(sp);
-                        const uint64_t db = umma_desc_k_major_sw128(sp + kPRows * kChunk);
-                        if (elect_one()) {
+                        for (int h = 0; h < parts; ++h) {
+                            ok = __all_sync(0xffffffffu, bounded_wait(tempty_bar(h * kSlots + slot), ((g >> 1) & 1u) ^ 1u, ctl, p.status, 3, g) &&
+                                                         (parts == 2 || bounded_wait(tempty_bar(kSlots + slot), ((g >> 1) & 1u) ^ 1u, ctl, p.status, 3, g)));
+                            if (!ok) break;
+                            tc_fence_after();
+                            const uint64_t db = umma_desc_k_major_sw128(sp + kPRows * kChunk + h * (kBHalf / 2) * kChunk);
+                            if (elect_one()) {
 #pragma unroll
-                            for (int kk = 0; kk < kChunk / 32; ++kk) {
-                                // 32 bytes further along K inside the 128-byte swizzle atom: +2 in address units of 16 B
-                                tc_mma_f8_pair(d_tmem, da + 2u * kk, db + 2u * kk, idesc, kk > 0 ? 1u : 0u);
+                                for (int kk = 0; kk < kChunk / 32; ++kk) {
+                                    // 32 bytes further along K inside the 128-byte swizzle atom: +2 in address units of 16 B
+                                    tc_mma_f8_pair(d_tmem + h * kBHalf, da + 2u * kk, db + 2u * kk, idesc, kk > 0 ? 1u : 0u);
+                                }
+                                // this product is complete in the TMEM of both CTAs; behind the last one the stage is reusable in both
+                                tc_commit_pair(tfull_bar(h * kSlots + slot));
+                                tc_commit_pair(peer_tfull0 + 8u * (h * kSlots + slot));
+                                if (parts == 1) {
+                                    tc_commit_pair(tfull_bar(kSlots + slot));
+                                    tc_commit_pair(peer_tfull0 + 8u * (kSlots + slot));
+                                }
+                                if (h == parts - 1) {
+                                    tc_commit_pair(empty_bar(s));
+                                    tc_commit_pair(peer_empty0 + 8u * s);
+                                }
                             }
-                            // this chunk's product is complete in the TMEM of both CTAs; the stage is reusable in both
-                            tc_commit_pair(tfull_bar(slot));
-                            tc_commit_pair(peer_tfull);
-                            tc_commit_pair(empty_bar(s));
-                            tc_commit_pair(peer_empty0 + 8u * s);
+                            __syncwarp();
                         }
-                        __syncwarp();
+                        if (!ok) break;
                     }
                 };
-                for (int tile = pair; ok && tile < p.num_tiles; tile += n_pairs) multiply_tile(umma_idesc_e4m3_f32(2 * kPRows, kBN));
-                if (ok && decode_strip(pair, p).any) multiply_tile(umma_idesc_e4m3_f32(2 * kPRows, static_cast<uint32_t>(p.tail_w)));
+                for (int tile = pair; ok && tile < p.num_tiles; tile += n_pairs) multiply_tile(umma_idesc_e4m3_f32(2 * kPRows, kBHalf), 2);
+                if (ok && decode_strip(pair, p).any) multiply_tile(umma_idesc_e4m3_f32(2 * kPRows, static_cast<uint32_t>(p.tail_w)), 1);
             }
         }
     } else {
@@ -287,7 +302,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         const int quarter = warp & 3;                       // TMEM lane quarter this warp may access
         const int row = quarter * 32 + lane;                // accumulator row (TMEM lane)
         const uint32_t t_lane = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + col0;
-        const uint32_t lead_tempty0 = mapa_shared(tempty_bar(0), 0);   // the leader's tempty[0], as seen from this CTA
+        const uint32_t lead_tempty0 = mapa_shared(tempty_bar(half * kSlots), 0);   // this group's first, in the leader
 
         uint32_t v[2][kPiece];
         float2 acc[64];
@@ -408,13 +423,13 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 #pragma unroll
                     for (int i = 0; i < kBlock; ++i) {
                         const int slot = static_cast<int>(g & 1u);
-                        const bool mine = bounded_wait_lean(tfull_bar(slot), (g >> 1) & 1u, ctl, p.status, 4, g);
+                        const bool mine = bounded_wait_lean(tfull_bar(half * kSlots + slot), (g >> 1) & 1u, ctl, p.status, 4, g);
                         ++g;
                         ok = __all_sync(0xffffffffu, mine);
                         if (!ok) break;
                         tc_fence_after();
                         const uint32_t t_slot = t_lane + slot * kBN;
-                        // The left 64 columns are read back and folded, then the right 64 are read back and the slot
+                        // The first 64 columns are read back and folded, then the other 64 are read back and the half slot
                         // returns to the issuer: two read-back latencies per chunk; the last fold follows the release.
                         tc_ld_x64(t_slot, &v[0][0]);
                         const float sc = ra[i] * rb[i];
@@ -468,7 +483,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 for (int i = 0; i < 4; ++i) {
                     if (k0 + i >= kc) break;
                     const int slot = static_cast<int>(g & 1u);
-                    ok = __all_sync(0xffffffffu, bounded_wait_lean(tfull_bar(slot), (g >> 1) & 1u, ctl, p.status, 4, g));
+                    ok = __all_sync(0xffffffffu, bounded_wait_lean(tfull_bar(half * kSlots + slot), (g >> 1) & 1u, ctl, p.status, 4, g));
                     ++g;
                     if (!ok) break;
                     tc_fence_after();
@@ -553,7 +568,7 @@ int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const flo
     memset(&tc, 0, sizeof(tc));
     int rc;
     if ((rc = make_tmap(&ta, a, M, K, kPRows)) != DSV3_OK) return rc;
-    if ((rc = make_tmap(&tb, b, N, K, kBHalf)) != DSV3_OK) return rc;
+    if ((rc = make_tmap(&tb, b, N, K, kBHalf / 2)) != DSV3_OK) return rc;
     const bool tma_store = (N % 8) == 0;   // row pitch of the result must be a multiple of 16 bytes for a tensor map
     if (tma_store && (rc = make_tmap_out(&tc, c, M, N)) != DSV3_OK) return rc;
     TwParams prm;
