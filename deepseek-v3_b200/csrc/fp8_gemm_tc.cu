@@ -1012,7 +1012,9 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
                 // tile and hand-over, and 0.4 to 1.2 for the cluster launch.  (Chunk times in a full machine; a single round runs at
                 // higher clocks.  Chosen so, 277 shapes of 72 to 4000 tokens are within a few per cent of the best of the
                 // three; with K below 1536 excluded from the 256 x 128 tiles and no estimate for the single CTA, thirty
-                // were 4-39 % away.)
+                // were 4-39 % away.  The wide tiles' figures are those of products in halves: 198 shapes of 140 to 3000 tokens are 0.3 % from
+                // the best on average, with the figures from before, 0.41 and 1.3, 0.5 %: M 200, N 24576, K 1536 15.9 / 14.6 us, M 1500, N 4096,
+                // K 512 10.7 / 9.5, M 2048, N 3072, K 1536 18.5 / 17.5.)
                 const int pairs = sms / 2;
                 const int64_t pp = (static_cast<int64_t>(pl.tiles_p) + 1) / 2;
                 const auto unsplit = [&](int64_t n, int64_t units, double chunk, double chunk1, double o) {
@@ -1027,8 +1029,8 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
                     if (tw_pair_supported(M, N, K)) {          // (the last round of the wide tiles may be cut into strips)
                         const int64_t n = pp * ((N + 255) / 256), tail = n % pairs;
                         const int strip = tw_strip_width(tail, pairs, pl.kc);
-                        wide = 1.0 + (strip ? static_cast<double>(n / pairs) * (pl.kc * 0.41 + 1.3) + pl.kc * (strip == 64 ? 0.27 : 0.37) + 2.0
-                                            : unsplit(n, pairs, 0.41, 0.41, 1.3));
+                        wide = 0.5 + (strip ? static_cast<double>(n / pairs) * (pl.kc * 0.38 + 0.9) + pl.kc * (strip == 64 ? 0.27 : 0.37) + 1.5
+                                            : unsplit(n, pairs, 0.38, 0.38, 0.9));
                     }
                     pl.wide = wide < best && wide <= narrow;
                     pl.pair = pl.wide || narrow < best;
