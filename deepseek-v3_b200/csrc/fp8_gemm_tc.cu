@@ -826,8 +826,8 @@ int make_tmap(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int b
     return DSV3_OK;
 }
 
-// Result matrix [M, N] bf16, row-major; box = 64 columns (128 bytes) x 128 rows, 128-byte swizzle.
-int make_tmap_out(CUtensorMap* map, void* base, int64_t M, int64_t N) {
+// Result matrix [M, N] bf16, row-major; box = 64 columns (128 bytes) x box_rows rows, 128-byte swizzle.
+int make_tmap_out(CUtensorMap* map, void* base, int64_t M, int64_t N, int box_rows) {
     EncodeTiledFn fn = encode_fn();
     if (!fn) {
         set_last_error("cuTensorMapEncodeTiled is not available from the driver");
@@ -835,7 +835,7 @@ int make_tmap_out(CUtensorMap* map, void* base, int64_t M, int64_t N) {
     }
     const cuuint64_t dims[2] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(M)};
     const cuuint64_t strides[1] = {static_cast<cuuint64_t>(N) * 2};
-    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(kPRows)};
+    const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(box_rows)};
     const cuuint32_t estr[2] = {1, 1};
     const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides, box, estr,
                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,

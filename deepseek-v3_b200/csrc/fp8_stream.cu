@@ -844,7 +844,7 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
 // ---------------------------------------------------------------------------------------------------------------------
 template <int BN, bool kSwiglu, bool kBoth>
 __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUtensorMap* tmap_w1, const CUtensorMap* tmap_a0, const CUtensorMap* tmap_a1,
-                                           const StreamParams& p) {
+                                           const CUtensorMap* tmap_c0, const CUtensorMap* tmap_c1, const StreamParams& p) {
     using C = SCfg<BN, true>;
     constexpr bool kSplit = false;      // its partial tiles would be 128 KB each
     constexpr int NS = C::kStages, NT = C::kSlots;
@@ -1023,17 +1023,30 @@ __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUt
             if (quarter * 32 >= s.ntok) continue;
             if constexpr (!kSwiglu) {
                 if (!active) continue;
-                // 32 rows x 64 columns at a time through the warp's own 4 KB, so that global stores cover whole lines
+                // 32 rows x 64 columns at a time through the warp's own 4 KB; where all of the rows are the tile's, from there by a TMA
+                // store (an SM's stores go out at 25 bytes per clock, 2600 cycles for a tile, which nobody then waits for).  us, w2 of 32 experts of
+                // 7168 x 2048 with 512 rows each 332 / 316, 64 of 2048 x 1408 with 128 and 512 44.1 / 41.9, 128 / 119.
                 uint8_t* wbuf = my_x + quarter * (32 * 128);
                 const int64_t n0 = static_cast<int64_t>(blk) * kPRows;
+                const bool whole = d.vec_store && quarter * 32 + 32 <= s.ntok;
 #pragma unroll
                 for (int half = 0; half < 2; ++half) {
+                    if (lane == 0) bulk_wait_group_read0();        // the store before has read the buffer
                     __syncwarp();
 #pragma unroll
                     for (int c = 0; c < 8; ++c) {
                         const float2* a = acc + half * 32 + c * 4;
                         *reinterpret_cast<uint4*>(wbuf + lane * 128 + ((c ^ (lane & 7)) << 4)) =
                             make_uint4(pack_bf16x2(a[0].x, a[0].y), pack_bf16x2(a[1].x, a[1].y), pack_bf16x2(a[2].x, a[2].y), pack_bf16x2(a[3].x, a[3].y));
+                    }
+                    if (whole) {
+                        fence_proxy_async_shared();
+                        __syncwarp();
+                        if (lane == 0) {
+                            tma_store_2d(!kBoth || s.side == kGroups ? tmap_c0 : tmap_c1, smem_u32(wbuf), static_cast<int>(n0) + half * 64, s.row0 + quarter * 32);
+                            bulk_commit_group();
+                        }
+                        continue;
                     }
                     __syncwarp();
                     const int piece = lane & 7;
@@ -1116,6 +1129,7 @@ __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUt
             }
         }
     }
+    if (!kSwiglu && warp >= kFirstPromoWarp && lane == 0) bulk_wait_group0();      // results have left shared memory
     teardown(ctl, warp, tmem_base, C::kTmemCols);
 }
 
@@ -1133,8 +1147,8 @@ template <bool kSwiglu, bool kBoth>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_divided_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
                    const __grid_constant__ CUtensorMap tmap_a0, const __grid_constant__ CUtensorMap tmap_a1,
-                   const __grid_constant__ StreamParams large, const __grid_constant__ StreamParams small) {
-    if (static_cast<int>(blockIdx.x) < large.ctas) rows_tiles<128, kSwiglu, kBoth>(&tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, large);
+                   const __grid_constant__ CUtensorMap tmap_c0, const __grid_constant__ CUtensorMap tmap_c1, const __grid_constant__ StreamParams large, const __grid_constant__ StreamParams small) {
+    if (static_cast<int>(blockIdx.x) < large.ctas) rows_tiles<128, kSwiglu, kBoth>(&tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, &tmap_c0, &tmap_c1, large);
     else stream_tiles<64, kSwiglu, false, false>(&tmap_w0, &tmap_w1, &tmap_a0, &tmap_a1, small);
 }
 
@@ -1176,6 +1190,15 @@ int launch_stream(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMa
 template <bool kSwiglu, bool kBoth>
 int launch_divided(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, StreamParams prm, int64_t most_large,
                    int64_t most_small, int divide, int sms, cudaStream_t stream) {
+    CUtensorMap c0, c1;
+    memset(&c0, 0, sizeof(c0));
+    memset(&c1, 0, sizeof(c1));
+    if (!kSwiglu)
+        for (int i = 0; i < 2; ++i) {
+            const Side& d = prm.side[i];
+            int rc;
+            if (d.c && d.vec_store && (rc = make_tmap_out(i == kGroups ? &c0 : &c1, d.c, d.rows, d.N, 32)) != DSV3_OK) return rc;
+        }
     constexpr int kLarge = SCfg<128, true>::kSmemBytes, kSmall = SCfg<64, false>::kSmemBytes;
     static bool configured[64] = {};
     StreamParams small = prm;
@@ -1186,7 +1209,7 @@ int launch_divided(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorM
     small.first_cta = prm.ctas;
     small.ctas = divide ? static_cast<int>(most_small < sms ? most_small : sms) : 0;
     return launch(fp8_divided_kernel<kSwiglu, kBoth>, prm.ctas + small.ctas, kLarge > kSmall ? kLarge : kSmall, configured, stream, w0, w1, ta0, ta1,
-                  prm, small);
+                  c0, c1, prm, small);
 }
 
 }  // namespace

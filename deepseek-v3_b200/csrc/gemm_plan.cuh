@@ -27,10 +27,10 @@ int launch_fp8_gemm_tc(const void* a, const float* a_s, const void* b, const flo
                        cudaStream_t stream);
 
 // Tensor maps over the operands as they lie in memory.  Operand: [rows, K] bytes, row-major; box = 128 bytes x
-// box_rows, 128-byte swizzle, zero fill outside.  Result: [M, N] bf16, row-major; box = 64 columns x 128 rows,
+// box_rows, 128-byte swizzle, zero fill outside.  Result: [M, N] bf16, row-major; box = 64 columns x 128 (or box_rows) rows,
 // 128-byte swizzle (N % 8 == 0).
 int make_tmap(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int box_rows);
-int make_tmap_out(CUtensorMap* map, void* base, int64_t M, int64_t N);
+int make_tmap_out(CUtensorMap* map, void* base, int64_t M, int64_t N, int box_rows = 128);
 
 // Token-major kernel on CTA pairs (256 x 128 tiles, tcgen05 cta_group::2, no split-K): fp8_gemm_tm.cu.
 bool tm_pair_supported(int64_t M, int64_t N, int64_t K);
