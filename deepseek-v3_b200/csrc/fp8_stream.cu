@@ -732,6 +732,36 @@ __device__ __forceinline__ void stream_tiles(const CUtensorMap* tmap_w0, const C
             }
             if constexpr (!kSwiglu) {
                 if (!ok) continue;
+                if (BN == 64 && d.vec_store) {
+                    // A thread holds one column; four neighbours exchange four tokens so that each stores four columns of one, and a warp
+                    // four tokens' 64 bytes at a time.  A store takes the SM 8 cycles with one token's and 13 with four: a tile of 64 tokens 3800
+                    // / 2500 cycles of 21000 (us, w2 of 64 experts of 7168 x 2048, 64 rows each 178 / 167, 2048 x 1408 48.8 / 45.2; layers of 32
+                    // of 256 experts at 2206 tokens 469.5 / 462.1, 16 of 64 small ones at 600 70.8 / 70.0).  With few tokens the exchange only
+                    // lengthens the chain: 16 tokens 800 / 950, 8 of 64 small experts at 62 tokens (tiles of 32) 37.2 / 38.1.
+                    const int odd = lane & 1, up = (lane >> 1) & 1;
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        const int64_t n = static_cast<int64_t>(2 * s.p + b) * kPRows + (row & ~3);
+                        if ((2 * s.p + b) * kPRows + quarter * 32 >= d.N) continue;        // uniform in the warp
+                        __nv_bfloat16* out = d.c + (static_cast<int64_t>(s.row0) + col0 + odd + 2 * up) * d.N + n;
+#pragma unroll
+                        for (int i = 0; i < NP; ++i) {
+                            if (i >= np) continue;
+#pragma unroll
+                            for (int j = 0; j < PW; j += 4) {
+                                const uint32_t w0 = pack_bf16x2(acc[b][i][j / 2].x, acc[b][i][j / 2].y), w1 = pack_bf16x2(acc[b][i][j / 2 + 1].x, acc[b][i][j / 2 + 1].y);
+                                const uint32_t p0 = __shfl_xor_sync(0xffffffffu, w0, 1), p1 = __shfl_xor_sync(0xffffffffu, w1, 1);
+                                // tokens j + odd and j + 2 + odd of two columns
+                                const uint32_t a0 = odd ? __byte_perm(p0, w0, 0x7632) : __byte_perm(w0, p0, 0x5410);
+                                const uint32_t a1 = odd ? __byte_perm(p1, w1, 0x7632) : __byte_perm(w1, p1, 0x5410);
+                                const uint32_t r = __shfl_xor_sync(0xffffffffu, up ? a0 : a1, 2);
+                                if (col0 + 2 * PW * i + j + odd + 2 * up < s.ntok && n < d.N)
+                                    *reinterpret_cast<uint2*>(out + (2 * PW * i + j) * d.N) = up ? make_uint2(r, a1) : make_uint2(a0, r);
+                            }
+                        }
+                    }
+                    continue;
+                }
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
                     const int64_t n = static_cast<int64_t>(2 * s.p + b) * kPRows + row;

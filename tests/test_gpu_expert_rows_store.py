@@ -28,7 +28,7 @@ def test_only_the_groups_rows_are_written(counts, N):
     i64, p = ctypes.c_int64, lambda t: ctypes.c_void_p(t.data_ptr())
     _lib.check(_lib.lib.dsv3_fp8_gemm_rows(p(_table(_lib.lib, _lib.check, w, N, K)), n, p(xq), p(xs_t), p(seg), i64(rows), i64(0), i64(N), i64(K), p(out),
                                            None, None, ctypes.c_size_t(0), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
-    dsv3_b200.set_gemm_policy(2, 1)
+    dsv3_b200.set_gemm_policy(2 if sum(counts) > 40 * n else 3, 1)             # tiles of 128 tokens, or weight-major ones
     at = 0
     for c, e in zip(counts, w):
         if c:
