@@ -1117,7 +1117,7 @@ __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUt
                 }
                 ok = barrier_all<64>(2 + quarter, ok);
                 if (!ok) break;                    // both warps of these rows
-                uint32_t m2 = 0u;
+                float m = 0.0f;
                 // Rolled loops over a register file that turns by one group per trip: unrolled, this epilogue was longer
                 // than the instruction cache holds and cost 8000-14000 cycles per tile.  (Rows beyond the tile's hold
                 // products of weights with weights: not worth silu's exact path.)
@@ -1133,10 +1133,9 @@ __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUt
                         v[29] = h.y;
                         v[30] = h.z;
                         v[31] = h.w;
-                        m2 = max_abs_bf16x2(m2, max_abs8(h));
+                        m = fmaxf(m, amax8(h));
                     }
                 }
-                float m = amax_of_pair(m2);
                 // only this thread reads slot `row` of the other group's half
                 *reinterpret_cast<float*>(other_x + slot) = m;
                 asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");

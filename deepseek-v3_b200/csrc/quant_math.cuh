@@ -21,21 +21,18 @@ __device__ __forceinline__ float scale_from_amax(float amax, int scale_fmt) {
     return s;
 }
 
-// The larger magnitudes of two pairs of bf16 values, with signs that say nothing; a NaN gives way to the other operand.
-__device__ __forceinline__ uint32_t max_abs_bf16x2(uint32_t a, uint32_t b) {
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
     uint32_t d;
-    asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
     return d;
 }
-__device__ __forceinline__ uint32_t max_abs8(const uint4& v) { return max_abs_bf16x2(max_abs_bf16x2(v.x, v.y), max_abs_bf16x2(v.z, v.w)); }
-// The larger of a pair's magnitudes; a NaN is dropped.
-__device__ __forceinline__ float amax_of_pair(uint32_t m) {
-    m &= 0x7FFF7FFFu;
+
+// max|x| of eight bf16 values
+__device__ __forceinline__ float amax8(const uint4& v) {
+    // two values to a word; a NaN gives way to the other operand, and a lane of nothing but NaN returns one, which fmaxf drops
+    const uint32_t m = max_bf16x2(max_bf16x2(v.x & 0x7FFF7FFFu, v.y & 0x7FFF7FFFu), max_bf16x2(v.z & 0x7FFF7FFFu, v.w & 0x7FFF7FFFu));
     return fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xFFFF0000u));
 }
-
-// max|x| of eight bf16 values (two values to a word; a lane of nothing but NaN is one, which fmaxf drops)
-__device__ __forceinline__ float amax8(const uint4& v) { return amax_of_pair(max_abs8(v)); }
 
 __device__ __forceinline__ float rcp_approx(float s) {
     float r;
@@ -117,7 +114,8 @@ static __device__ __noinline__ float silu_exact(float a) {
 __device__ __forceinline__ uint4 swiglu8(const uint4& a, const uint4& b) {
     const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
     constexpr float kLog2e = 1.44269504088896340736f;
-    uint32_t h[4], top = 0u;
+    uint32_t h[4];
+    __nv_bfloat162 top = __float2bfloat162_rn(0.0f);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         // two values to an FP32 instruction: with one each, swiglu_quant was bound by issue (8192 x 18432 142.9 us, 134.0 so)
@@ -132,10 +130,9 @@ __device__ __forceinline__ uint4 swiglu8(const uint4& a, const uint4& b) {
         const float2 s2 = __fmul2_rn(a2, r2);
         const __nv_bfloat162 silu = __floats2bfloat162_rn(s2.x, s2.y), h2 = __hmul2(silu, *reinterpret_cast<const __nv_bfloat162*>(&bw[i]));
         h[i] = *reinterpret_cast<const uint32_t*>(&h2);
-        asm("max.NaN.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(top) : "r"(top), "r"(aw[i]));
+        top = __hmax2_nan(top, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&aw[i])));
     }
-    top &= 0x7FFF7FFFu;
-    if (!__hble2(*reinterpret_cast<const __nv_bfloat162*>(&top), __float2bfloat162_rn(87.0f))) {
+    if (!__hble2(top, __float2bfloat162_rn(87.0f))) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int up = i & 1 ? 0 : 16;              // shifts the value to the upper half of the word
