@@ -19,7 +19,7 @@
 //                            the end of a work item write the result (token-major: through shared memory and
 //                            a TMA store) or park a split-K partial tile
 // Operand roles: P is the 128-row MMA "A" operand, Q the BN-row MMA "B" operand.
-//   kSwap = false : P = 128 tokens of a,  Q = 128 rows of b  (M > 64: "token-major" tiles)
+//   kSwap = false : P = 128 tokens of a,  Q = 128 or 64 rows of b  (M > 64: "token-major" tiles)
 //   kSwap = true  : P = 128 rows of b,    Q = BN tokens of a ("weight-major": M <= 64, where weights stream once; up to 256 tokens on
 //                   few weights, in several token tiles, whose smaller parts are exchanged sooner: small_estimate)
 // (producer and issuer warps stay converged; one elected lane issues)
@@ -97,12 +97,12 @@ struct Cfg {
     static constexpr int kChunkBytes = kPRows * kChunk + BN * kChunk;      // P and Q tile of one chunk
     static constexpr int kStageBytes = kUC * kChunkBytes;
     // chunk products resident in TMEM: four 128-column accumulators, or eight of 64 columns
-    static constexpr int kAccs = (kSwap && BN == 64) ? 8 : kTmemStages;
+    static constexpr int kAccs = BN == 64 ? 8 : kTmemStages;
     static constexpr int kTmemUnits = kAccs / kUC;                          // unit products resident in TMEM
     // weight-major tiles: a_s * b_s of the item's chunks for the tile's BN tokens, [chunk][token]
     static constexpr int kScaleTabBytes = kSwap ? scale_tab_chunks(BN) * BN * 4 : 0;
     // token-major tiles: the 128 x 128 bf16 result tile is staged here (two 128-byte-swizzled 128 x 64 boxes)
-    static constexpr int kStoreBytes = !kSwap ? kPRows * 128 * 2 : 0;
+    static constexpr int kStoreBytes = !kSwap && BN == 128 ? kPRows * 128 * 2 : 0;
     // Split-K inside a cluster: partial sums that the other CTAs send here.  16- and 32-token tiles have room of their own
     // for them; the others re-use the operand stages once every CTA of the cluster is through with its own.
     static constexpr bool kOwnExchange = kSwap && BN < 64;
@@ -185,7 +185,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
     constexpr int NT = C::kTmemUnits;    // TMEM stages, in units
     constexpr int CPT = BN / 2;       // accumulator columns per promotion thread (a thread owns half a row)
     constexpr int kWriters = kPromoThreads;
-    static_assert(kSwap || BN == 128, "token-major tiles are 128 x 128 (one b_s value per tile and chunk)");
+    static_assert(kSwap || BN == 128 || BN == 64, "token-major tiles are 128 x 128 or 128 x 64: one b_s value per tile and chunk");
 
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
@@ -363,7 +363,11 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
         uint32_t probe = 0;   // result of test_wait on tfull[] for the next unit
         // token-major tiles: two read-back buffers of one chunk (64 columns) each
         constexpr bool kBatched = !kSwap;
-        uint32_t va64[kBatched ? 64 : 1], vb64[kBatched ? 64 : 1];
+        uint32_t va64[kBatched ? CPT : 1], vb64[kBatched ? CPT : 1];
+        auto load_chunk = [](uint32_t taddr, uint32_t* v) {
+            if constexpr (CPT == 64) tc_ld_x64(taddr, v);
+            else if constexpr (CPT == 32) tc_ld_x32(taddr, v);
+        };
         // Issues (does not wait for) the load of step `st` of chunk `j` of unit `gu`; the first step of a
         // unit first waits for the unit's products to be complete in TMEM.
         auto issue_load = [&](uint32_t gu, int j, int st, uint32_t* v) -> bool {
@@ -403,7 +407,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
             const float* bs_ptr;
             if constexpr (!kSwap) {
                 as_ptr = p.a_s + min(p_row, M - 1) * kc;
-                bs_ptr = p.b_s + static_cast<int64_t>(it.q_idx) * kc;          // BN == 128
+                bs_ptr = p.b_s + static_cast<int64_t>(it.q_idx) * BN / 128 * kc;
             } else {
                 as_ptr = p.a_s;
                 bs_ptr = p.b_s + static_cast<int64_t>(it.p_idx) * kc;        // 128 weight rows = one scale row
@@ -463,7 +467,7 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                     ok = __all_sync(0xffffffffu, mine);
                     if (ok) {
                         tc_fence_after();
-                        tc_ld_x64(t_lane + ((gu % NT) * UC) * BN, va64);
+                        load_chunk(t_lane + ((gu % NT) * UC) * BN, va64);
                     }
                 }
             } else {
@@ -476,7 +480,6 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                 // per unit exposes the TMEM latency once), returns the TMEM stage at once and only then does
                 // the FMAs; the other promotion warp of the scheduler overlaps with them.  Row scales (global
                 // memory) are fetched one unit ahead.
-                static_assert(CPT == 64, "token-major tiles: 64 columns per thread");
                 // raw scales one unit ahead, multiplied when the unit begins (see fp8_gemm_tm.cu)
                 float ra0, ra1, rb0, rb1;
                 auto load_scales = [&](int k) {        // clamped so that the look-ahead never leaves the item
@@ -498,8 +501,8 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                         tc_fence_after();
                     }
                     const uint32_t taddr = t_lane + (ts * UC) * BN;
-                    if (mu > 0) tc_ld_x64(taddr, va64);
-                    if (nch > 1) tc_ld_x64(taddr + BN, vb64);
+                    if (mu > 0) load_chunk(taddr, va64);
+                    if (nch > 1) load_chunk(taddr + BN, vb64);
                     const float sa0 = ra0 * rb0, sa1 = ra1 * rb1;
                     load_scales(unit_k(mu + 1));
                     tc_wait_ld();
@@ -512,14 +515,14 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                     {
                         const float2 sc2 = make_float2(sa0, sa0);
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
+                        for (int j = 0; j < CPT / 2; ++j)
                             acc[j] = __ffma2_rn(make_float2(__uint_as_float(va64[2 * j]), __uint_as_float(va64[2 * j + 1])),
                                                 sc2, acc[j]);
                     }
                     if (nch > 1) {
                         const float2 sc2 = make_float2(sa1, sa1);
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
+                        for (int j = 0; j < CPT / 2; ++j)
                             acc[j] = __ffma2_rn(make_float2(__uint_as_float(vb64[2 * j]), __uint_as_float(vb64[2 * j + 1])),
                                                 sc2, acc[j]);
                     }
@@ -613,8 +616,8 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
                     }
                 } else {
                     const bool vec_ok = (N % 8) == 0;
-                    for (int e = tid; e < rows_here * 16; e += kPromoThreads) {      // eight columns each
-                        const int i = e >> 4, k8 = e & 15, r_tile = me * R + i;
+                    for (int e = tid; e < rows_here * (BN / 8); e += kPromoThreads) {      // eight columns each
+                        const int i = e / (BN / 8), k8 = e % (BN / 8), r_tile = me * R + i;
                         const int64_t m = static_cast<int64_t>(it.p_idx) * kPRows + r_tile, n = static_cast<int64_t>(it.q_idx) * BN + 8 * k8;
                         if (m >= M || n >= N) continue;
                         float4 lo = make_float4(0.f, 0.f, 0.f, 0.f), hi = lo;
@@ -699,13 +702,13 @@ fp8_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_p, const __grid_cons
             }
             if (write_out) {
                 if constexpr (!kSwap) {
-                    if (C::kStoreBytes > 0 && p.tma_store) {
+                    if (BN == 128 && p.tma_store) {
                         // The four warps of a column half stage their 128 x 64 bf16 box in shared memory (128-byte
                         // swizzle: 16-byte slot c of row r sits at slot c ^ (r & 7), which also keeps the
                         // vector stores free of bank conflicts) and one thread hands it to the TMA, which clips
                         // rows beyond M and columns beyond N.  The store of the previous tile is only known to
                         // have read the buffer once its issuer has waited for it, hence the first barrier.
-                        static_assert(CPT == 64, "one 128-byte box row per thread");
+                        static_assert(BN != 128 || CPT == 64, "one 128-byte box row per thread");
                         const int half = (warp - kFirstPromoWarp) >> 2;
                         uint8_t* sbuf = store_buf + half * (kPRows * 128);
                         const bool issuer = ((threadIdx.x & 127) == 0);
@@ -928,7 +931,7 @@ int clusters_of(int dev, int splits) {
 }  // namespace
 
 static int64_t clusters_resident(int dev, int sms, bool swap, int bn, int splits) {
-    const int n = !swap ? clusters_of<128, false>(dev, splits)
+    const int n = !swap ? (bn == 64 ? clusters_of<64, false>(dev, splits) : clusters_of<128, false>(dev, splits))
                         : (bn == 16 ? clusters_of<16, true>(dev, splits) : (bn == 32 ? clusters_of<32, true>(dev, splits) : clusters_of<64, true>(dev, splits)));
     const int budget = sms / splits;
     return n < budget ? n : budget;
@@ -944,6 +947,12 @@ static double small_estimate(int bn, int64_t M, int chunks, int splits, int64_t 
     if (splits == 1) return 4.1 + 0.28 * chunks;
     const double per_tile = static_cast<double>(M) / static_cast<double>((M + 63) / 64);
     return 3.6 + 0.26 * chunks + 0.6 + 0.0125 * n + (per_tile > 33.0 ? 0.7 * (per_tile - 33.0) / 31.0 : 0.0);
+}
+
+// The same of token-major tiles of 64 weight rows (K up to 144 chunks).  Long K lies further from the L2: its chunks take longer.
+static double half_estimate(int kc, int chunks, int splits, int64_t ctas) {
+    const double n = static_cast<double>(ctas), far = kc <= 56 ? 0.0 : (kc >= 128 ? 0.04 : 0.04 * (kc - 56) / 72.0);
+    return splits == 1 ? 2.97 + (0.18 + far) * chunks + 0.0065 * n : 4.1 + (0.1955 + far) * chunks + 0.0078 * n + 0.123 * (splits - 2);
 }
 
 // Pinned values (dsv3_set_gemm_policy) are honoured or refused (pl.error), never rewritten; the automatic
@@ -967,6 +976,8 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
         pl.tiles_q = static_cast<int>((N + 127) / 128);
     }
     struct { int bn, tiles_q, splits; } chosen = {0, 0, 0};      // narrower token tiles than these
+    double chosen_estimate = 0.0;
+    int half_splits = 0;                                         // or token-major tiles of 64 weight rows
     const int64_t tiles = static_cast<int64_t>(pl.tiles_p) * pl.tiles_q;
     if (tiles * 64 >= (1ll << 31)) {     // the work-item counters are 32-bit (at most 64 splits)
         set_last_error("fp8_gemm: %lld output tiles are more than the work-item counter holds", static_cast<long long>(tiles));
@@ -1062,9 +1073,9 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
         // 512 -> 4096 at 64, 128 5.3 / 3.7, 5.1 / 4.1, 1536 -> 3072 at 128 7.0 / 5.6, 2048 -> 1408 at 256 7.45 / 6.3.  No gain: 7168 -> 2304 at 33
         // 7.9 / 8.5, 7168 -> 1536 at 256 11.3 / 13.1; with more weights, 16384 -> 7168 at 64 28.5 / 31.7.  (Weights in the L2.  From HBM the gain is smaller, and
         // up to 32 tokens it is a loss: two layers of a decode step, one rank of eight, 32 tokens 303.0 / 307.2, 48 356.3 / 353.2, 64 398.3 / 389.4.)
+        double now = best + 2.4 + (pl.cluster ? 0.017 * (static_cast<double>(tiles * splits) - 72.0) : 0.0);
         if (force_kernel == 0 && M > 32 && M <= 256 && N * K <= (24ll << 20)) {
             const int64_t rows = (N + kPRows - 1) / kPRows;
-            double now = best + 2.4 + (pl.cluster ? 0.017 * (static_cast<double>(tiles * splits) - 72.0) : 0.0);
             const double margin = pl.swap ? 0.15 : 0.5;     // (what the estimates are apart, of one kernel and of two)
             if (pl.swap) now = tiles * splits <= sms ? small_estimate(pl.bn, M, (pl.kc + splits - 1) / splits, splits, tiles * splits) : 1e30;
             for (int bn = 16; bn <= 64; bn *= 2) {
@@ -1077,10 +1088,39 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
                     if (t < now - margin) {
                         now = t + margin;                   // (once, not against one another)
                         chosen = {bn, static_cast<int>(q), sfac};
+                        chosen_estimate = t;
                     }
                 }
             }
+            if (chosen.bn) now = chosen_estimate;
         }
+        // Token-major tiles of 64 weight rows, which never lie in two weight blocks, where they fit one round: a chunk is 24 KB of loads for a CTA
+        // instead of 32, a part of a tile half as much to exchange, and there are more ways to come near 148 CTAs.  half_estimate() is
+        // fitted to 412 launches of 172 shapes of 70 to 2200 tokens (rms 5 %, weights from HBM, a replayed graph); against what the plan chose
+        // before, 59 of the shapes take them, two of these 2 % slower than before.  us, before / so: M 1003, N 576, K 7168 12.3 / 10.0; M 256, N 576, K 7168
+        // 9.3 / 7.4; M 1000, N 256, K 7168 10.2 / 8.2; M 200, N 2304, K 7168 12.4 / 10.1; M 529, N 1584, K 4224 11.5 / 9.3; M 70, N 7168, K 2304 8.6 / 7.1;
+        // M 650, N 800, K 896 5.6 / 4.7.  (Clusters of three and more that leave few SMs over wait for room: M 600, N 576, K 7168, 45 of three, 10.9.)
+        if (force_kernel == 0 && M > 64 && pl.kc <= 144) {
+            const int64_t narrow = static_cast<int64_t>(pl.tiles_p) * ((N + 63) / 64);
+            for (int sfac = 1; sfac <= kMaxClusterSplits && sfac <= pl.kc && narrow * sfac <= sms; ++sfac) {
+                if (sfac > 1 && (narrow > clusters_resident(dev, sms, false, 64, sfac) || (sfac > 2 && 10 * narrow * sfac > 9 * sms))) continue;
+                const double t = half_estimate(pl.kc, (pl.kc + sfac - 1) / sfac, sfac, narrow * sfac), floor = bytes / 6.0e6 + 2.4;
+                if (t < now - 0.4 && floor < now - 0.4) {
+                    now = t + 0.4;
+                    chosen = {0, 0, 0};
+                    half_splits = sfac;
+                }
+            }
+        }
+    }
+    if (half_splits) {
+        pl.swap = pl.pair = pl.wide = false;
+        pl.bn = 64;
+        pl.tiles_p = static_cast<int>((M + kPRows - 1) / kPRows);
+        pl.tiles_q = static_cast<int>((N + 63) / 64);
+        pl.splits = half_splits;
+        pl.cluster = half_splits > 1;
+        return pl;
     }
     if (chosen.bn) {
         pl.swap = true;
@@ -1190,7 +1230,7 @@ int launch_fp8_gemm_tc(const void* a, const float* a_s, const void* b, const flo
     } else {
         if ((rc = make_tmap(&tp, a, M, K, kPRows)) != DSV3_OK) return rc;
         if ((rc = make_tmap(&tq, b, N, K, pl.bn)) != DSV3_OK) return rc;
-        tma_store = (N % 8) == 0;   // row pitch of the result must be a multiple of 16 bytes for a tensor map
+        tma_store = pl.bn == 128 && !pl.cluster && (N % 8) == 0;   // row pitch of the result must be a multiple of 16 bytes for a tensor map
         if (tma_store && (rc = make_tmap_out(&tc, c, M, N)) != DSV3_OK) return rc;
     }
     TcParams prm;
@@ -1231,6 +1271,8 @@ int launch_fp8_gemm_tc(const void* a, const float* a_s, const void* b, const flo
         }
     } else if (pl.bn == 128) {
         return launch_variant<128, false>(tp, tq, tc, prm, stream);
+    } else if (pl.bn == 64) {
+        return launch_variant<64, false>(tp, tq, tc, prm, stream);
     }
     set_last_error("fp8_gemm: no tcgen05 variant for tile width %d", pl.bn);
     return DSV3_ERR_UNSUPPORTED;
