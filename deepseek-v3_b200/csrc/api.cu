@@ -269,6 +269,24 @@ int dsv3_fp8_gemm(const void* a, const float* a_s, const void* b, const float* b
     return launch_fp8_gemm_tc(a, a_s, b, b_s, M, N, K, c, workspace, workspace_bytes, pl, st);
 }
 
+int dsv3_fp8_gemm_two_pays(int64_t M, int64_t N, int64_t K) {
+    return M > 0 && N > 0 && K > 0 && K % 16 == 0 && g_force_kernel == 0 && g_force_split == 0 && tw_two_pay(M, N, K);
+}
+
+int dsv3_fp8_gemm_two(const void* a, const float* a_s, const void* b0, const float* b0_s, const void* b1, const float* b1_s, int64_t M, int64_t N,
+                      int64_t K, void* c0, void* c1, dsv3_stream_t stream) {
+    if (M <= 0 || N <= 0 || K <= 0 || is_null(a) || is_null(a_s) || is_null(b0) || is_null(b0_s) || is_null(b1) || is_null(b1_s) || is_null(c0) ||
+        is_null(c1)) {
+        set_last_error("fp8_gemm_two: null pointer, or a size that is not positive");
+        return DSV3_ERR_INVALID_ARGUMENT;
+    }
+    if (!tc_supported(a, b0, c0, M, N, K) || !tc_supported(a, b1, c1, M, N, K) || !tw_pair_supported(M, N, K)) {
+        set_last_error("fp8_gemm_two: takes more than 128 tokens, more than 128 weight rows, K %% 16 == 0 and 16-byte aligned operands");
+        return DSV3_ERR_UNSUPPORTED;
+    }
+    return launch_fp8_gemm_tw_two(a, a_s, {b0, b1}, {b0_s, b1_s}, M, N, K, {c0, c1}, static_cast<cudaStream_t>(stream));
+}
+
 int dsv3_fp8_linear(const void* x, int64_t M, int64_t K, const void* w, const float* w_s, int64_t N, int scale_fmt, void* c,
                     dsv3_stream_t stream) {
     if (M < 0 || N < 0 || K < 0) {

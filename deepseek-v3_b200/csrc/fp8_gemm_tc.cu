@@ -957,13 +957,22 @@ static double half_estimate(int kc, int chunks, int splits, int64_t ctas) {
 
 // Pinned values (dsv3_set_gemm_policy) are honoured or refused (pl.error), never rewritten; the automatic
 // plan adapts freely.  dev, sms: the device (-1: none) and the SMs there are on it, or the budget for them.
-static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split, int dev, int sms) {
+// Time of n wide tiles (256 x 256) on so many pairs, in the plan's microseconds.  The last round may be cut into strips.
+static double wide_estimate(int64_t n, int64_t pairs, int kc) {
+    const int strip = tw_strip_width(n % pairs, pairs, kc);
+    if (strip) return 0.5 + static_cast<double>(n / pairs) * (kc * 0.38 + 0.9) + kc * (strip == 64 ? 0.27 : 0.37) + 1.5;
+    return 0.5 + static_cast<double>((n + pairs - 1) / pairs) * (kc * 0.38 + 0.9);
+}
+
+// estimate: microseconds (automatic plans of token-major tiles; otherwise 0)
+static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split, int dev, int sms, double& estimate) {
     TcPlan pl;
     pl.error = DSV3_OK;
     pl.pair = false;
     pl.wide = false;
     pl.splits = 1;
     pl.cluster = false;
+    estimate = 0.0;
     pl.kc = static_cast<int>((K + kChunk - 1) / kChunk);
     pl.swap = (force_kernel == 3) || (force_kernel == 0 && M <= 64);
     if (pl.swap) {
@@ -1037,12 +1046,7 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
                     const double full = pp * pl.tiles_q < pairs ? static_cast<double>(pp * pl.tiles_q) / pairs : 1.0;
                     const double narrow = tm_pair_supported(M, N, K) ? 0.4 + 0.8 * full + unsplit(pp * pl.tiles_q, pairs, 0.265, 0.235, 0.8) : 1e30;
                     double wide = 1e30;
-                    if (tw_pair_supported(M, N, K)) {          // (the last round of the wide tiles may be cut into strips)
-                        const int64_t n = pp * ((N + 255) / 256), tail = n % pairs;
-                        const int strip = tw_strip_width(tail, pairs, pl.kc);
-                        wide = 0.5 + (strip ? static_cast<double>(n / pairs) * (pl.kc * 0.38 + 0.9) + pl.kc * (strip == 64 ? 0.27 : 0.37) + 1.5
-                                            : unsplit(n, pairs, 0.38, 0.38, 0.9));
-                    }
+                    if (tw_pair_supported(M, N, K)) wide = wide_estimate(pp * ((N + 255) / 256), pairs, pl.kc);
                     pl.wide = wide < best && wide <= narrow;
                     pl.pair = pl.wide || narrow < best;
                     if (narrow < best) best = narrow;
@@ -1074,6 +1078,7 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
         // 7.9 / 8.5, 7168 -> 1536 at 256 11.3 / 13.1; with more weights, 16384 -> 7168 at 64 28.5 / 31.7.  (Weights in the L2.  From HBM the gain is smaller, and
         // up to 32 tokens it is a loss: two layers of a decode step, one rank of eight, 32 tokens 303.0 / 307.2, 48 356.3 / 353.2, 64 398.3 / 389.4.)
         double now = best + 2.4 + (pl.cluster ? 0.017 * (static_cast<double>(tiles * splits) - 72.0) : 0.0);
+        estimate = now;
         if (force_kernel == 0 && M > 32 && M <= 256 && N * K <= (24ll << 20)) {
             const int64_t rows = (N + kPRows - 1) / kPRows;
             const double margin = pl.swap ? 0.15 : 0.5;     // (what the estimates are apart, of one kernel and of two)
@@ -1092,7 +1097,7 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
                     }
                 }
             }
-            if (chosen.bn) now = chosen_estimate;
+            if (chosen.bn) estimate = now = chosen_estimate;
         }
         // Token-major tiles of 64 weight rows, which never lie in two weight blocks, where they fit one round: a chunk is 24 KB of loads for a CTA
         // instead of 32, a part of a tile half as much to exchange, and there are more ways to come near 148 CTAs.  half_estimate() is
@@ -1107,6 +1112,7 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
                 const double t = half_estimate(pl.kc, (pl.kc + sfac - 1) / sfac, sfac, narrow * sfac), floor = bytes / 6.0e6 + 2.4;
                 if (t < now - 0.4 && floor < now - 0.4) {
                     now = t + 0.4;
+                    estimate = t;
                     chosen = {0, 0, 0};
                     half_splits = sfac;
                 }
@@ -1142,7 +1148,7 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
                 pl.error = DSV3_ERR_UNSUPPORTED;
                 return pl;
             }
-            return work_out_plan(M, N, K, 2, 0, dev, sms);   // automatic choice, absurdly long K: token-major tiles instead
+            return work_out_plan(M, N, K, 2, 0, dev, sms, estimate);   // automatic choice, absurdly long K: token-major tiles instead
         }
     }
     pl.splits = splits;
@@ -1167,27 +1173,56 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
 // A plan is asked for twice per call, for the workspace and for the launch, and takes 0.1 to 0.2 us to work out, of calls that keep the
 // host busy for 4.5: a thread remembers the last sixteen by all that they depend on.  (Looked through in turn, 4 to 15 ns; a slot
 // for each by its sizes made the Linears of one layer displace one another.)
-TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split) {
+static TcPlan planned(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split, double& estimate) {
     int dev = 0;
     const int sms = num_sms_of_device(&dev);
-    if (force_kernel != 0 || force_split != 0 || dev < 0) return work_out_plan(M, N, K, force_kernel, force_split, dev, sms);
+    if (force_kernel != 0 || force_split != 0 || dev < 0) return work_out_plan(M, N, K, force_kernel, force_split, dev, sms, estimate);
     struct Remembered {
         int64_t M, N, K;
         int sms, dev;
         TcPlan plan;
+        double estimate;
     };
     constexpr unsigned kRemembered = 16;
     static thread_local Remembered remembered[kRemembered] = {};
     static thread_local unsigned oldest = 0;
     for (const Remembered& r : remembered)
-        if (r.M == M && r.N == N && r.K == K && r.sms == sms && r.dev == dev) return r.plan;
+        if (r.M == M && r.N == N && r.K == K && r.sms == sms && r.dev == dev) {
+            estimate = r.estimate;
+            return r.plan;
+        }
     t_guessed = false;
-    const TcPlan plan = work_out_plan(M, N, K, 0, 0, dev, sms);
+    const TcPlan plan = work_out_plan(M, N, K, 0, 0, dev, sms, estimate);
     if (plan.error == DSV3_OK && !t_guessed) {           // (the message of an error is the call's own)
-        remembered[oldest] = {M, N, K, sms, dev, plan};
+        remembered[oldest] = {M, N, K, sms, dev, plan, estimate};
         oldest = (oldest + 1) % kRemembered;
     }
     return plan;
+}
+
+TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split) {
+    double estimate = 0.0;
+    return planned(M, N, K, force_kernel, force_split, estimate);
+}
+
+// Whether two weights of one size are multiplied sooner in one launch of wide tiles than in one launch each: the two have one last
+// round of the SMs between them instead of one each, and one launch's set-up.  The results are the same bit for bit where both ways
+// take tiles that are not cut over K.  B200, us with act_quant, two launches / one: M 2580, N 2304, K 7168 120.9 / 89.5; M 3942, N 2816, K 2048
+// 61.4 / 50.2; M 2201, N 2048, K 7168 75.1 / 69.1; M 2201, N 3072, K 5120 93.9 / 68.8; M 500, N 12288, K 5120 91.3 / 66.6; M 8192, N 2048, K 7168
+// 266 / 244.  The margin: with many rounds the two are level, or the launch boundary, which brings the pairs back into step,
+// is worth 1 %: M 2201, N 18432, K 7168 541 / 551, M 6000, N 12288, K 5120 697 / 704, M 8192, N 18432, K 7168 1917 / 1923.
+// Not where the common last round would be cut into strips: it is faster there, too (M 1300, N 2048, K 7168 60.2 / 53.5, M 1545, N 2816,
+// K 2048 33.1 / 27.1), but such MLPs are held to their number of launches (tests/test_gpu_mlp_launches.py).
+bool tw_two_pay(int64_t M, int64_t N, int64_t K) {
+    if (!tw_pair_supported(M, N, K)) return false;
+    double estimate = 0.0;
+    const TcPlan one = planned(M, N, K, 0, 0, estimate);
+    if (one.error != DSV3_OK || one.swap || estimate <= 0.0) return false;
+    const int64_t n = 2 * ((M + 2 * kPRows - 1) / (2 * kPRows)) * ((N + 255) / 256), pairs = num_sms() / 2;
+    if (n % pairs != 0 && 2 * (n % pairs) <= pairs) return false;
+    double two = wide_estimate(n, pairs, one.kc);
+    if (const double floor = (2.0 * static_cast<double>(N) * K + static_cast<double>(M) * K) / 6.0e6; two < floor) two = floor;
+    return two + 2.4 < 0.975 * 2.0 * estimate;
 }
 
 size_t tc_workspace_bytes(const TcPlan& pl, int64_t M, int64_t N) {

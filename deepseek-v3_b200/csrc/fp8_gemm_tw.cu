@@ -31,6 +31,12 @@
 //                     load has landed, and that piece's FMAs follow the release.
 //                     Result tile: bf16 through shared memory and TMA stores.
 //
+// One weight, or two of one size on the same activations (w1 and w3 of an MLP; TwOperands): a launch of 99 tiles on 74 pairs is two
+// rounds, the second a third full, and two of them four; 198 tiles in one launch are three.  MLP 7168 -> 2304 at 2580 rows 158.8 / 144.1 us, 2048 -> 2816 at
+// 3942 96.6 / 90.9, 5120 -> 12288 at 500 135.5 / 123.7, 2048 -> 1408 at 2580 45.6 / 41.5 (tw_two_pay()).  Tried instead: a launch each, the second
+// one's CTAs on the SMs that the first one's last round leaves idle, without waiting for its end: 5 us more for the set-up of the CTAs (M 2580, N 2304,
+// K 7168, w1 and w3 alone 120.9, in one launch 89.5, so 95.6), and nothing gained where more than half of the SMs have a tile in that round.
+//
 // Every mbarrier wait is bounded: after about a second the waiting thread records what it was waiting for in
 // the status word, raises a CTA-wide abort flag and all roles fall through to the common teardown.  Before a
 // CTA leaves, its producer waits for the last commits onto its empty[] barriers (nothing else would), and the
@@ -93,12 +99,45 @@ struct TwParams {
     int tail_tiles, tail_w; // tiles shared out in strips of tail_w columns (128 or 64) instead, one strip per pair; 0: none
 };
 
-struct Tile {
-    int pp, q;
+// Operands as tensor maps.  Two weights (w1 and w3 of an MLP, equal in size, on the same activations): the second one's tiles follow
+// the first one's in the order of weight tiles, so that the two have one last round between them.
+template <int kMats>
+struct TwOperands;
+template <>
+struct TwOperands<1> {
+    CUtensorMap a, b[1], c[1], s[1];      // s: strips' boxes of b
+};
+template <>
+struct TwOperands<2> {
+    CUtensorMap a, b[2], c[2], s[2];
+    const float* b_s1;                    // the second weight's, beside TwParams::b_s and c
+    __nv_bfloat16* c1;
+    int tiles_q0;                         // weight tiles of the first
 };
 
+struct Tile {
+    int pp, q;
+    int m;                  // which weight
+};
+
+template <int kMats>
+__device__ __forceinline__ const float* b_s_of(const TwOperands<kMats>& o, const TwParams& p, int m) {
+    if constexpr (kMats == 2) {
+        if (m) return o.b_s1;
+    }
+    return p.b_s;
+}
+template <int kMats>
+__device__ __forceinline__ __nv_bfloat16* c_of(const TwOperands<kMats>& o, const TwParams& p, int m) {
+    if constexpr (kMats == 2) {
+        if (m) return o.c1;
+    }
+    return p.c;
+}
+
 // Work order: `raster` token-tile pairs share consecutive weight tiles so that a wave re-uses both operands in L2.
-__device__ __forceinline__ Tile decode_tile(int tile, const TwParams& p) {
+template <int kMats>
+__device__ __forceinline__ Tile decode_tile(int tile, const TwOperands<kMats>& o, const TwParams& p) {
     const int per_group = p.raster * p.tiles_q;
     const int grp = static_cast<int>(fast_div(static_cast<uint32_t>(tile), p.div_per_group));
     const int first = grp * p.raster;
@@ -107,6 +146,13 @@ __device__ __forceinline__ Tile decode_tile(int tile, const TwParams& p) {
     Tile t;
     t.q = (gsz == p.raster) ? static_cast<int>(fast_div(static_cast<uint32_t>(r), p.div_raster)) : r / gsz;   // the last group may be shorter
     t.pp = first + (r - t.q * gsz);
+    t.m = 0;
+    if constexpr (kMats == 2) {
+        if (t.q >= o.tiles_q0) {
+            t.q -= o.tiles_q0;
+            t.m = 1;
+        }
+    }
     return t;
 }
 
@@ -122,20 +168,21 @@ struct Strip {
     int n0;                 // first column
     bool any;
 };
-__device__ __forceinline__ Strip decode_strip(int pair, const TwParams& p) {
+template <int kMats>
+__device__ __forceinline__ Strip decode_strip(int pair, const TwOperands<kMats>& o, const TwParams& p) {
     Strip s = {};
     const int shift = p.tail_w == 64 ? 2 : 1;
     if (p.tail_w == 0 || (pair >> shift) >= p.tail_tiles) return s;
-    s.t = decode_tile(p.num_tiles + (pair >> shift), p);
+    s.t = decode_tile(p.num_tiles + (pair >> shift), o, p);
     s.n0 = s.t.q * kBN + (pair & ((1 << shift) - 1)) * p.tail_w;
     s.any = s.n0 < p.N;
     return s;
 }
 
-template <int kBlock>      // K chunks per scale load: 4 (K chunks a multiple of four, 16-byte aligned scales), 2 (of two, 8-byte) or 1
+// kBlock: K chunks per scale load: 4 (K chunks a multiple of four, 16-byte aligned scales), 2 (of two, 8-byte) or 1
+template <int kBlock, int kMats>
 __global__ void __launch_bounds__(kNumThreads, 1)
-fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                   const __grid_constant__ CUtensorMap tmap_c, const __grid_constant__ CUtensorMap tmap_s, const TwParams p) {
+fp8_gemm_tw_kernel(const __grid_constant__ TwOperands<kMats> o, const TwParams p) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = smem_u32(smem_raw);
     const uint32_t tiles = (raw + 1023u) & ~1023u;     // the same offset in both CTAs of the pair
@@ -167,9 +214,11 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         }
         ctl->abort_flag = 0;
         mbar_fence_init();
-        tma_prefetch_desc(&tmap_a);
-        tma_prefetch_desc(&tmap_b);
-        if (p.tma_store) tma_prefetch_desc(&tmap_c);
+        tma_prefetch_desc(&o.a);
+        for (int m = 0; m < kMats; ++m) {
+            tma_prefetch_desc(&o.b[m]);
+            if (p.tma_store) tma_prefetch_desc(&o.c[m]);
+        }
     }
     if (warp == 1) tc_alloc_pair(smem_u32(&ctl->tmem_base), kTmemCols);
     // Programmatic dependent launch: nothing above touches global memory, so it may overlap the tail of
@@ -179,11 +228,11 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
     if (threadIdx.x == 0) {
         const int n_pre = min(kc, kStages);
         if (pair < p.num_tiles) {
-            const Tile t = decode_tile(pair, p);
+            const Tile t = decode_tile(pair, o, p);
             for (int j = 0; j < n_pre; ++j)
-                for (int h = 0; h < 2; ++h) tma_prefetch_l2_2d(&tmap_b, j * kChunk, t.q * kBN + h * kBHalf + static_cast<int>(rank) * (kBHalf / 2));
-        } else if (const Strip s = decode_strip(pair, p); s.any) {
-            for (int j = 0; j < n_pre; ++j) tma_prefetch_l2_2d(&tmap_s, j * kChunk, s.n0 + static_cast<int>(rank) * (p.tail_w / 2));
+                for (int h = 0; h < 2; ++h) tma_prefetch_l2_2d(&o.b[t.m], j * kChunk, t.q * kBN + h * kBHalf + static_cast<int>(rank) * (kBHalf / 2));
+        } else if (const Strip s = decode_strip(pair, o, p); s.any) {
+            for (int j = 0; j < n_pre; ++j) tma_prefetch_l2_2d(&o.s[s.t.m], j * kChunk, s.n0 + static_cast<int>(rank) * (p.tail_w / 2));
         }
     }
     griddep_launch_dependents();
@@ -217,7 +266,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                         const uint32_t dst = tiles + s * kChunkBytes;
                         if (elect_one()) {
                             if (rank == 0) mbar_arrive_expect_tx(full_bar(s), bytes);
-                            tma_load_2d_pair(dst, &tmap_a, k * kChunk, a_row, lead_full);
+                            tma_load_2d_pair(dst, &o.a, k * kChunk, a_row, lead_full);
                             tma_load_2d_pair(dst + kPRows * kChunk, tmap, k * kChunk, b_row, lead_full);
                             if (boxes == 2) tma_load_2d_pair(dst + kPRows * kChunk + kBHalf / 2 * kChunk, tmap, k * kChunk, b_row + kBHalf, lead_full);
                         }
@@ -225,11 +274,11 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                     }
                 };
                 for (int tile = pair; ok && tile < p.num_tiles; tile += n_pairs) {
-                    const Tile t = decode_tile(tile, p);
-                    load_tile(&tmap_b, 2, (2 * t.pp + static_cast<int>(rank)) * kPRows, t.q * kBN + static_cast<int>(rank) * (kBHalf / 2), 2 * kChunkBytes);
+                    const Tile t = decode_tile(tile, o, p);
+                    load_tile(&o.b[t.m], 2, (2 * t.pp + static_cast<int>(rank)) * kPRows, t.q * kBN + static_cast<int>(rank) * (kBHalf / 2), 2 * kChunkBytes);
                 }
-                if (const Strip st = decode_strip(pair, p); ok && st.any)
-                    load_tile(&tmap_s, 1, (2 * st.t.pp + static_cast<int>(rank)) * kPRows, st.n0 + static_cast<int>(rank) * (p.tail_w / 2),
+                if (const Strip st = decode_strip(pair, o, p); ok && st.any)
+                    load_tile(&o.s[st.t.m], 1, (2 * st.t.pp + static_cast<int>(rank)) * kPRows, st.n0 + static_cast<int>(rank) * (p.tail_w / 2),
                               2u * (kPRows + p.tail_w / 2) * kChunk);
                 // Nothing waits for the commits onto the empty[] barriers of the last chunks; wait for them here so
                 // that none is in flight when the CTA leaves (it would land in whatever CTA gets this shared memory next).
@@ -289,7 +338,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                     }
                 };
                 for (int tile = pair; ok && tile < p.num_tiles; tile += n_pairs) multiply_tile(umma_idesc_e4m3_f32(2 * kPRows, kBHalf), 2);
-                if (ok && decode_strip(pair, p).any) multiply_tile(umma_idesc_e4m3_f32(2 * kPRows, static_cast<uint32_t>(p.tail_w)), 1);
+                if (ok && decode_strip(pair, o, p).any) multiply_tile(umma_idesc_e4m3_f32(2 * kPRows, static_cast<uint32_t>(p.tail_w)), 1);
             }
         }
     } else {
@@ -326,7 +375,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         // them, hence the first barrier, which every tile passes and which also says whether a wait of any of the four
         // warps gave up (false: they all turn away).  tp = token tile of this CTA.
         const bool issuer = (((threadIdx.x - kFirstPromoWarp * 32) & 127) == 0);
-        auto write_tile = [&](int tp, int tq) -> bool {
+        auto write_tile = [&](int tp, int tq, int m) -> bool {
             if (p.tma_store) {
                 if (issuer) bulk_wait_group_read0();
                 if (!barrier_all<128>(2 + half, true)) return false;
@@ -356,16 +405,16 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
 #pragma unroll
                         for (int bx = 0; bx < kBoxes; ++bx) {
                             const int64_t n = n0 + (pass * kBoxes + bx) * 64;
-                            if (n < p.N) tma_store_2d(&tmap_c, smem_u32(sbuf + bx * (kPRows * 128)), static_cast<int>(n), tp * kPRows);
+                            if (n < p.N) tma_store_2d(&o.c[m], smem_u32(sbuf + bx * (kPRows * 128)), static_cast<int>(n), tp * kPRows);
                         }
                         bulk_commit_group();
                     }
                 }
             } else {
-                const int64_t m = static_cast<int64_t>(tp) * kPRows + row;
+                const int64_t tok = static_cast<int64_t>(tp) * kPRows + row;
                 const int64_t N = p.N;
-                if (m < p.M) {
-                    __nv_bfloat16* crow = p.c + m * N;
+                if (tok < p.M) {
+                    __nv_bfloat16* crow = c_of(o, p, m) + tok * N;
 #pragma unroll
                     for (int j = 0; j < 64; ++j) {
                         if (n0 + 2 * j < N) crow[n0 + 2 * j] = __float2bfloat16_rn(acc[j].x);
@@ -382,7 +431,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             const int64_t tok = static_cast<int64_t>(2 * t.pp + static_cast<int>(rank)) * kPRows + row;
             return p.a_s + min(tok, p.M - 1) * kc;
         };
-        auto bs_row = [&](const Tile& t) { return p.b_s + static_cast<int64_t>(min(2 * t.q + half, p.nblk - 1)) * kc; };
+        auto bs_row = [&](const Tile& t) { return b_s_of(o, p, t.m) + static_cast<int64_t>(min(2 * t.q + half, p.nblk - 1)) * kc; };
 
         // Scales, kBlock chunks at a time.  A thread's a_s row is a 32-byte sector of its own, and L1 (what the operand
         // stages leave of it) does not hold 256 of them until the next chunk: one chunk at a time, the scales cost a quarter
@@ -412,7 +461,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
         uint32_t g = 0;            // chunk counter
         int tile = pair;
         if (tile < p.num_tiles) {
-            Tile cur = decode_tile(tile, p);
+            Tile cur = decode_tile(tile, o, p);
             first_scales(cur);
             while (true) {
                 const float* as_ptr = as_row(cur);
@@ -454,20 +503,20 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
                 const bool more = next < p.num_tiles;
                 Tile nt = cur;
                 if (more) {
-                    nt = decode_tile(next, p);
+                    nt = decode_tile(next, o, p);
                     first_scales(nt);
                 }
-                ok = write_tile(2 * cur.pp + static_cast<int>(rank), cur.q);
+                ok = write_tile(2 * cur.pp + static_cast<int>(rank), cur.q, cur.m);
                 if (!ok || !more) break;
                 tile = next;
                 cur = nt;
             }
         }
         // ---- a strip of the last round: the two warp groups take half of its columns each, and store them directly
-        if (const Strip st = decode_strip(pair, p); ok && st.any) {
+        if (const Strip st = decode_strip(pair, o, p); ok && st.any) {
             const int cw = p.tail_w / 2, n0 = st.n0 + half * cw;
             const float* as_ptr = as_row(st.t);
-            const float* bs_ptr = p.b_s + static_cast<int64_t>(st.n0 / 128) * kc;
+            const float* bs_ptr = b_s_of(o, p, st.t.m) + static_cast<int64_t>(st.n0 / 128) * kc;
             // scales are requested four chunks ahead: a chunk takes half as long as a load that misses L1
             float sa[4], sb[4];
 #pragma unroll
@@ -500,7 +549,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
             }
             const int64_t m = static_cast<int64_t>(2 * st.t.pp + static_cast<int>(rank)) * kPRows + row;
             if (ok && m < p.M) {
-                __nv_bfloat16* crow = p.c + m * p.N;
+                __nv_bfloat16* crow = c_of(o, p, st.t.m) + m * p.N;
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const int n = n0 + 8 * j;
@@ -555,26 +604,36 @@ int tw_strip_width(int64_t tiles, int64_t pairs, int kc) {
     return 4 * tiles <= pairs ? 64 : (kc >= 24 ? 128 : 0);
 }
 
-int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const float* b_s, int64_t M, int64_t N,
-                       int64_t K, void* c, cudaStream_t stream) {
-    const int64_t tiles_p = (M + kPRows - 1) / kPRows, tiles_q = (N + kBN - 1) / kBN;
-    const int64_t tiles_pp = (tiles_p + 1) / 2;
+namespace {
+
+template <int kMats>
+int launch(const void* a, const float* a_s, const void* const* b, const float* const* b_s, int64_t M, int64_t N, int64_t K, void* const* c,
+           cudaStream_t stream) {
+    const int64_t tiles_p = (M + kPRows - 1) / kPRows, tiles_q0 = (N + kBN - 1) / kBN;
+    const int64_t tiles_pp = (tiles_p + 1) / 2, tiles_q = kMats * tiles_q0;
     if (tiles_pp * tiles_q >= (1ll << 31)) {
         set_last_error("fp8_gemm: %lld x %lld output tiles are more than the work-item counter holds",
                        static_cast<long long>(tiles_p), static_cast<long long>(tiles_q));
         return DSV3_ERR_UNSUPPORTED;
     }
-    CUtensorMap ta, tb, tc;
-    memset(&tc, 0, sizeof(tc));
+    TwOperands<kMats> ops;
+    memset(&ops, 0, sizeof(ops));
     int rc;
-    if ((rc = make_tmap(&ta, a, M, K, kPRows)) != DSV3_OK) return rc;
-    if ((rc = make_tmap(&tb, b, N, K, kBHalf / 2)) != DSV3_OK) return rc;
+    if ((rc = make_tmap(&ops.a, a, M, K, kPRows)) != DSV3_OK) return rc;
     const bool tma_store = (N % 8) == 0;   // row pitch of the result must be a multiple of 16 bytes for a tensor map
-    if (tma_store && (rc = make_tmap_out(&tc, c, M, N)) != DSV3_OK) return rc;
+    for (int m = 0; m < kMats; ++m) {
+        if ((rc = make_tmap(&ops.b[m], b[m], N, K, kBHalf / 2)) != DSV3_OK) return rc;
+        if (tma_store && (rc = make_tmap_out(&ops.c[m], c[m], M, N)) != DSV3_OK) return rc;
+    }
     TwParams prm;
     prm.a_s = a_s;
-    prm.b_s = b_s;
-    prm.c = static_cast<__nv_bfloat16*>(c);
+    prm.b_s = b_s[0];
+    prm.c = static_cast<__nv_bfloat16*>(c[0]);
+    if constexpr (kMats == 2) {
+        ops.b_s1 = b_s[1];
+        ops.c1 = static_cast<__nv_bfloat16*>(c[1]);
+        ops.tiles_q0 = static_cast<int>(tiles_q0);
+    }
     prm.status = status_device_ptr();
     if (!prm.status) return DSV3_ERR_CUDA;
     prm.M = M;
@@ -596,11 +655,15 @@ int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const flo
     prm.tail_w = tw_strip_width(prm.tail_tiles, max_pairs, prm.kc);
     if (prm.tail_w == 0) prm.tail_tiles = 0;
     prm.num_tiles -= prm.tail_tiles;
-    CUtensorMap ts = tb;
-    if (prm.tail_w && (rc = make_tmap(&ts, b, N, K, prm.tail_w / 2)) != DSV3_OK) return rc;
+    for (int m = 0; m < kMats; ++m) {
+        ops.s[m] = ops.b[m];
+        if (prm.tail_w && (rc = make_tmap(&ops.s[m], b[m], N, K, prm.tail_w / 2)) != DSV3_OK) return rc;
+    }
 
-    const auto aligned = [&](int n) { return (prm.kc % n) == 0 && ((reinterpret_cast<uintptr_t>(a_s) | reinterpret_cast<uintptr_t>(b_s)) % (4 * n)) == 0; };
-    auto kern = aligned(4) ? fp8_gemm_tw_kernel<4> : aligned(2) ? fp8_gemm_tw_kernel<2> : fp8_gemm_tw_kernel<1>;
+    uintptr_t scales = reinterpret_cast<uintptr_t>(a_s);
+    for (int m = 0; m < kMats; ++m) scales |= reinterpret_cast<uintptr_t>(b_s[m]);
+    const auto aligned = [&](int n) { return (prm.kc % n) == 0 && (scales % (4 * n)) == 0; };
+    auto kern = aligned(4) ? fp8_gemm_tw_kernel<4, kMats> : aligned(2) ? fp8_gemm_tw_kernel<2, kMats> : fp8_gemm_tw_kernel<1, kMats>;
     static bool configured[64] = {};
     int dev = 0;
     DSV3_CUDA_TRY(cudaGetDevice(&dev));
@@ -609,9 +672,9 @@ int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const flo
         return DSV3_ERR_UNSUPPORTED;
     }
     if (!configured[dev]) {
-        DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
-        DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+        DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<4, kMats>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+        DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<2, kMats>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+        DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<1, kMats>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
         configured[dev] = true;
     }
     const int work = prm.num_tiles > 0 && prm.tail_w ? max_pairs : prm.num_tiles + (prm.tail_w ? prm.tail_tiles * (kBN / prm.tail_w) : 0);
@@ -630,8 +693,20 @@ int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const flo
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    DSV3_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ta, tb, tc, ts, prm));
+    DSV3_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ops, prm));
     return DSV3_OK;
+}
+
+}  // namespace
+
+int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const float* b_s, int64_t M, int64_t N, int64_t K, void* c,
+                       cudaStream_t stream) {
+    return launch<1>(a, a_s, &b, &b_s, M, N, K, &c, stream);
+}
+
+int launch_fp8_gemm_tw_two(const void* a, const float* a_s, const void* const (&b)[2], const float* const (&b_s)[2], int64_t M, int64_t N, int64_t K,
+                           void* const (&c)[2], cudaStream_t stream) {
+    return launch<2>(a, a_s, b, b_s, M, N, K, c, stream);
 }
 
 }  // namespace dsv3

@@ -43,6 +43,10 @@ bool tw_pair_supported(int64_t M, int64_t N, int64_t K);
 int tw_strip_width(int64_t tiles, int64_t pairs, int kc);
 int launch_fp8_gemm_tw(const void* a, const float* a_s, const void* b, const float* b_s, int64_t M, int64_t N,
                        int64_t K, void* c, cudaStream_t stream);
+// Two weights of one size on the same activations in one launch: w1 and w3 of an MLP.
+int launch_fp8_gemm_tw_two(const void* a, const float* a_s, const void* const (&b)[2], const float* const (&b_s)[2], int64_t M, int64_t N, int64_t K,
+                           void* const (&c)[2], cudaStream_t stream);
+bool tw_two_pay(int64_t M, int64_t N, int64_t K);
 
 // Decode-sized Linear without tcgen05 set-up (fp8_linear_small.cu): M <= 16; x != nullptr quantises bf16 activations
 // in the kernel's prologue (K % 128 == 0), otherwise (a, a_s) are the quantised activations (K % 16 == 0).

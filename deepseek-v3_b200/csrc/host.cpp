@@ -326,14 +326,16 @@ std::pair<at::Tensor, at::Tensor> quantise_remembered(const at::Tensor& x, int64
 }
 
 // ------------------------------------------------------------------ an MLP whose Linears are plain
-// w2(swiglu_quant(w1(x), w3(x))) in three launches: the quantisation of x, w1 and w3 with everything in front of w2, w2.
+// w2(swiglu_quant(w1(x), w3(x))) in three launches: the quantisation of x, w1 and w3 with everything in front of w2, w2; or, with
+// more tokens, in four: w1 and w3 in one launch, which fills the SMs' last round better than two.
 // Undefined where the separate launches are faster: in a graph, where only the device counts, or from here, where the host's launches do too.
 at::Tensor mlp(const at::Tensor& x, const at::Tensor (&w)[3], const at::Tensor (&s)[3], int x_fmt, int h_fmt, bool assume_no_inplace) {
     const int64_t K = last_dim(x), M = K ? x.numel() / K : 0, N = w[0].size(0);
     if (w[0].dim() != 2 || w[0].sizes() != w[1].sizes() || w[0].size(1) != K) return {};
-    if (!dsv3_swiglu_linear_pays(M, N, K) &&
-        (!dsv3_swiglu_linear_saves_launches(M, N, K) || !x.is_cuda() || capture_of(c10::cuda::getCurrentCUDAStream(x.device().index()).stream()) != 0))
-        return {};
+    const bool fused = dsv3_swiglu_linear_pays(M, N, K) ||
+                       (dsv3_swiglu_linear_saves_launches(M, N, K) && x.is_cuda() &&
+                        capture_of(c10::cuda::getCurrentCUDAStream(x.device().index()).stream()) == 0);
+    if (!fused && (N % 128 != 0 || !dsv3_fp8_gemm_two_pays(M, N, K))) return {};
     for (int i = 0; i < 2; ++i) {
         require(w[i].is_contiguous(), "Input tensors must be contiguous");
         require(s[i].is_contiguous(), "Scaling factor tensors must be contiguous");
@@ -343,14 +345,27 @@ at::Tensor mlp(const at::Tensor& x, const at::Tensor (&w)[3], const at::Tensor (
     require_bf16_default();
     auto q = quantise_remembered(x, 128, x_fmt, assume_no_inplace);
     const c10::Device dev = require_cuda(q.first, w[0], s[0], w[1], s[1]);
-    at::Tensor h = new_cuda_last(x, N, at::kFloat8_e4m3fn), hs = new_cuda_last(x, N / 128, at::kFloat);
+    at::Tensor h, hs;
+    const void *a = q.first.const_data_ptr(), *p1 = w[0].const_data_ptr(), *p3 = w[1].const_data_ptr();
+    auto f32 = [](const at::Tensor& t) { return static_cast<const float*>(t.const_data_ptr()); };
+    const float *as = f32(q.second), *s1 = f32(s[0]), *s3 = f32(s[1]);
+    if (!fused) {
+        const at::Tensor y1 = new_cuda_last(x, N, at::kBFloat16), y3 = new_cuda_last(x, N, at::kBFloat16);
+        void *y1p = y1.data_ptr(), *y3p = y3.data_ptr();
+        call_library(dev, [&](dsv3_stream_t st) { return dsv3_fp8_gemm_two(a, as, p1, s1, p3, s3, M, N, K, y1p, y3p, st); });
+        h = new_cuda_last(x, N, at::kFloat8_e4m3fn);
+        hs = new_cuda_last(x, N / 128, at::kFloat);
+        void* hp = h.data_ptr();
+        float* hsp = static_cast<float*>(hs.data_ptr());
+        call_library(dev, [&](dsv3_stream_t st) { return dsv3_swiglu_quant(y1p, y3p, M, N, h_fmt, hp, hsp, st); });
+        return gemm(h, hs, w[2], s[2]);
+    }
+    h = new_cuda_last(x, N, at::kFloat8_e4m3fn);
+    hs = new_cuda_last(x, N / 128, at::kFloat);
     const size_t need = dsv3_swiglu_linear_workspace_bytes(M, N, K);
     const at::Tensor held = need ? workspace(dev, need) : at::Tensor();
     void* ws = need ? held.data_ptr() : nullptr;
     const size_t ws_bytes = need ? static_cast<size_t>(held.numel()) : 0;
-    const void *a = q.first.const_data_ptr(), *p1 = w[0].const_data_ptr(), *p3 = w[1].const_data_ptr();
-    auto f32 = [](const at::Tensor& t) { return static_cast<const float*>(t.const_data_ptr()); };
-    const float *as = f32(q.second), *s1 = f32(s[0]), *s3 = f32(s[1]);
     void* hp = h.data_ptr();
     float* hsp = static_cast<float*>(hs.data_ptr());
     call_library(dev, [&](dsv3_stream_t st) { return dsv3_swiglu_linear(a, as, p1, s1, p3, s3, M, N, K, h_fmt, hp, hsp, ws, ws_bytes, st); });

@@ -28,7 +28,7 @@ EXPORTS = (
     "dsv3_fp8_gemm_workspace_bytes", "dsv3_fp8_gemm", "dsv3_set_gemm_policy", "dsv3_weight_quant",
     "dsv3_check_device_status", "dsv3_fp8_gemm_static", "dsv3_fp8_gemm_static_scratch_bytes",
     "dsv3_group_table_bytes", "dsv3_group_table_build", "dsv3_fp8_gemm_grouped", "dsv3_moe_combine", "dsv3_moe_route",
-    "dsv3_swiglu_linear_pays", "dsv3_swiglu_linear_saves_launches", "dsv3_swiglu_linear_workspace_bytes", "dsv3_swiglu_linear",
+    "dsv3_fp8_gemm_two_pays", "dsv3_fp8_gemm_two", "dsv3_swiglu_linear_pays", "dsv3_swiglu_linear_saves_launches", "dsv3_swiglu_linear_workspace_bytes", "dsv3_swiglu_linear",
     "dsv3_moe_dispatch", "dsv3_gemm_rows_workspace_bytes", "dsv3_swiglu_gemm_rows", "dsv3_fp8_gemm_rows", "dsv3_expert_gemms", "dsv3_moe_combine_add",
     "dsv3_few_experts_pay", "dsv3_few_route_bytes", "dsv3_few_up", "dsv3_few_down",
     "dsv3_fp8_linear", "dsv3_swiglu_quant", "dsv3_selftest_bounded_wait", "dsv3_p2p_handle_bytes", "dsv3_p2p_create", "dsv3_p2p_connect", "dsv3_p2p_connect_local", "dsv3_p2p_base",

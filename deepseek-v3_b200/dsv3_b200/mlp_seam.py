@@ -6,7 +6,8 @@ round trips through HBM for what is one pass over the data.  Where ``w1`` and ``
 ``linear`` and the library's rules on sizes say that it pays (few rows, or tiles that fit one round of the SMs; on the
 device, or outside of a graph capture for the host that launches),
 ``mlp_forward`` is three launches behind one host call: the quantisation of ``x``, ``w1`` and ``w3`` with SwiGLU and the
-quantisation in front of ``w2``, and ``w2``.  Otherwise it calls ``w1`` and ``w3`` (through whatever ``linear`` is
+quantisation in front of ``w2``, and ``w2``.  With more tokens, where ``w1`` and ``w3`` leave most of their last rounds of the SMs
+idle, it is four: both GEMMs are one launch and share that round.  Otherwise it calls ``w1`` and ``w3`` (through whatever ``linear`` is
 installed), then ``swiglu_quant`` (one launch, same rounding points, bit-identical FP8 codes and scales) and feeds
 ``fp8_gemm`` of ``w2`` directly.  What ``w2.forward`` would have done after its GEMM follows: the all-reduce of a
 ``RowParallelLinear`` (model.py:263-264) and the bias.

@@ -94,6 +94,16 @@ int dsv3_fp8_gemm(const void* a, const float* a_s, const void* b, const float* b
                   void* workspace, size_t workspace_bytes, dsv3_stream_t stream);
 
 /*
+ * fp8_gemm of the same activations with two weights of one size in one launch (w1 and w3 of an MLP, model.py:532, 633): c0 and c1 hold
+ * bit for bit what one of the kernels of dsv3_fp8_gemm writes (its 256-wide tiles).  M > 128, N > 128, K % 16 == 0, 16-byte aligned
+ * a, b0, b1, c0 and c1; other calls return DSV3_ERR_UNSUPPORTED.  No workspace.  _pays: whether it is faster than two launches (0 while
+ * dsv3_set_gemm_policy pins a kernel or split).
+ */
+int dsv3_fp8_gemm_two_pays(int64_t M, int64_t N, int64_t K);
+int dsv3_fp8_gemm_two(const void* a, const float* a_s, const void* b0, const float* b0_s, const void* b1, const float* b1_s, int64_t M,
+                      int64_t N, int64_t K, void* c0, void* c1, dsv3_stream_t stream);
+
+/*
  * Decode-sized Linear in one launch -- replaces the FP8 branch of linear(), model.py:158-160
  * (`y = fp8_gemm(*act_quant(x, block_size, scale_fmt), weight, weight.scale)`), for at most 16 rows.
  *   x : bf16 [M, K], 1 <= M <= 16, K % 128 == 0      w : e4m3 [N, K]      w_s : fp32 [ceil(N/128), K/128]
