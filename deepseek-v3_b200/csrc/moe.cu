@@ -136,6 +136,9 @@ struct DispatchParams {
     float* xs;                            // [T, dim / 128]
     uint2* xq_rows;                       // e4m3 [P, dim]
     float* xs_rows;                       // [dim / 128, P]
+    int per_y;                            // blocks of a token row that a CTA along y has
+    uint32_t by_b[2];                     // 2^32 / that, rounded up; [1]: of the last along y, which may have fewer
+    FastDiv div_topk;
 };
 
 __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const DispatchParams p) {
@@ -144,13 +147,7 @@ __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const Dispat
     __shared__ int to_row[kDispPairs], to_rows[kDispPairs];       // a token's local rows, side by side, and how many
     __shared__ __align__(8) uint8_t in_warp[kDispThreads / 32][kDispMaxExperts];      // a warp's own pairs of each expert
     griddep_launch_dependents();
-    griddep_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int topk = p.topk;
-    const int64_t t0 = static_cast<int64_t>(blockIdx.x) * p.tpc;
-    const int tokens = static_cast<int>(min(static_cast<int64_t>(p.tpc), p.T - t0));
-    const int own = tokens * topk;
-    const int64_t own0 = t0 * topk;
     if (tid < kDispMaxExperts) {
         total[tid] = 0;
         before[tid] = 0;
@@ -158,6 +155,31 @@ __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const Dispat
     static_assert(sizeof(in_warp) == 8 * kDispThreads, "eight bytes per thread");
     reinterpret_cast<uint2*>(&in_warp[0][0])[tid] = make_uint2(0u, 0u);
     __syncthreads();
+    griddep_wait();
+    const int topk = p.topk;
+    const int64_t t0 = static_cast<int64_t>(blockIdx.x) * p.tpc;
+    const int tokens = static_cast<int>(min(static_cast<int64_t>(p.tpc), p.T - t0));
+    const int own = tokens * topk;
+    const int64_t own0 = t0 * topk;
+    const int nb = p.dim / 128;
+    const int b_lo = blockIdx.y * p.per_y, b_n = min(p.per_y, nb - b_lo);
+    const int items = b_n > 0 ? tokens * b_n : 0;
+    // i / b_n is the upper half of i * by_b_n, as long as items * b_n < 2^32 (and b_n > 1)
+    const uint32_t by_b_n = p.by_b[b_n == p.per_y ? 0 : 1];
+    const bool divide = b_n == 1 || static_cast<uint64_t>(items) * b_n >= (1ull << 32);
+    const int lane16 = tid & 15;
+    constexpr int kHalfWarps = kDispThreads / 16;
+    // With few tokens this kernel is a chain of short steps.  So shared memory is cleared before the wait, the divisions are the host's, and the
+    // first round's block, when there is only one round, is on its way while the pairs are counted.  us, one launch behind another, 4, 148 and 600 tokens 3.78 /
+    // 3.26, 4.57 / 4.06, 5.79 / 5.29; per layer, 64 experts of
+    // 2048 x 1408, 8 of them here, 62 and 300 tokens 37.5 / 36.7, 54.6 / 53.4; a decode layer in a graph, 6 and 16 sequences 70.9 / 70.0, 110.6 / 109.7.
+    // (Its own pairs' experts asked for here, too, instead of behind the loop: 0.5 to 1 us slower with 6 and 16; their weights: no change.)
+    const bool one_round = items <= kHalfWarps;
+    uint4 early = make_uint4(0u, 0u, 0u, 0u);
+    if (one_round && (tid >> 4) < items) {
+        const int i = tid >> 4, t = b_n == 1 ? i : static_cast<int>(__umulhi(static_cast<uint32_t>(i), by_b_n));
+        early = __ldg(p.x + ((t0 + t) * nb + b_lo + (i - t * b_n)) * 16 + lane16);
+    }
 #pragma unroll 4
     for (int64_t pr = tid; pr < p.P; pr += kDispThreads) {
         const int64_t e = __ldg(p.indices + pr) - p.start;
@@ -210,7 +232,7 @@ __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const Dispat
     int sorted = 0;
     if (tid < own) {
         const int i = tid;
-        const int t = i / topk, first = t * topk, e = own_e[i];
+        const int t = static_cast<int>(fast_div(static_cast<uint32_t>(i), p.div_topk)), first = t * topk, e = own_e[i];
         int local = 0;                                             // local rows of the token's pairs before this one
         for (int j = first; j < i; ++j) local += own_row[j] >= 0;
         if (own_row[i] >= 0) to_row[first + local] = own_row[i];
@@ -228,16 +250,6 @@ __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const Dispat
     // instructions: 32 warps go through every place of a round, whether there is a block or not, and went through all of a
     // token's pairs for every block, local or not.  us before / after: 32 of 256 experts of dim 7168, 4 tokens 5.7 / 5.1, 1024 14.6 / 12.6, 4096
     // 42.6 / 36.8; 20 of 160 of dim 5120, 2048 17.7 / 14.5; 128 of 256, 4096 53.5 / 52.6.
-    const int nb = p.dim / 128;
-    const int per_y = (nb + gridDim.y - 1) / gridDim.y;
-    const int b_lo = blockIdx.y * per_y, b_n = min(per_y, nb - b_lo);
-    if (b_n <= 0) return;
-    const int items = tokens * b_n;
-    // i / b_n is the upper half of i * by_b_n, as long as items * b_n < 2^32 (and b_n > 1)
-    const uint32_t by_b_n = 0xFFFFFFFFu / static_cast<uint32_t>(b_n) + 1u;
-    const bool divide = b_n == 1 || static_cast<uint64_t>(items) * b_n >= (1ull << 32);
-    const int lane16 = tid & 15;
-    constexpr int kHalfWarps = kDispThreads / 16;
     auto quantise = [&](int i0, auto unroll) {
         constexpr int kU = decltype(unroll)::value;
         uint4 v[kU];
@@ -248,7 +260,7 @@ __global__ void __launch_bounds__(kDispThreads) moe_dispatch_kernel(const Dispat
             tl[u] = divide ? i / b_n : static_cast<int>(__umulhi(static_cast<uint32_t>(i), by_b_n));
             bl[u] = b_lo + i - tl[u] * b_n;
             if (i >= items) tl[u] = -1;
-            v[u] = tl[u] >= 0 ? __ldg(p.x + ((t0 + tl[u]) * nb + bl[u]) * 16 + lane16) : make_uint4(0u, 0u, 0u, 0u);
+            v[u] = kU == 1 && one_round ? early : tl[u] >= 0 ? __ldg(p.x + ((t0 + tl[u]) * nb + bl[u]) * 16 + lane16) : make_uint4(0u, 0u, 0u, 0u);
         }
 #pragma unroll
         for (int u = 0; u < kU; ++u) {
@@ -675,6 +687,12 @@ int dsv3_moe_dispatch(const void* x, int64_t T, int64_t dim, const int64_t* indi
     const int64_t gx = (T + tpc - 1) / tpc;
     int gy = 1;                                                    // few tokens: share each token's blocks among CTAs
     while (gy < 8 && gx * gy * 2 <= wave && gy * 2 * 32 <= dim / 128) gy *= 2;
+    const int nb = static_cast<int>(dim / 128);
+    p.per_y = (nb + gy - 1) / gy;
+    const int last = nb - (nb - 1) / p.per_y * p.per_y;
+    p.div_topk = make_fast_div(static_cast<uint32_t>(topk));
+    p.by_b[0] = 0xFFFFFFFFu / static_cast<uint32_t>(p.per_y) + 1u;
+    p.by_b[1] = 0xFFFFFFFFu / static_cast<uint32_t>(last) + 1u;
     DSV3_CUDA_TRY(launch_dependent(moe_dispatch_kernel, dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), dim3(kDispThreads), 0,
                                    static_cast<cudaStream_t>(stream), p));
     return DSV3_OK;
