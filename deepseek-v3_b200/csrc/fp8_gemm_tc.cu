@@ -949,14 +949,13 @@ static double small_estimate(int bn, int64_t M, int chunks, int splits, int64_t 
     return 3.6 + 0.26 * chunks + 0.6 + 0.0125 * n + (per_tile > 33.0 ? 0.7 * (per_tile - 33.0) / 31.0 : 0.0);
 }
 
-// The same of token-major tiles of 64 weight rows (K up to 144 chunks).  Long K lies further from the L2: its chunks take longer.
+// The same of token-major tiles of 64 weight rows (K up to 144 chunks).  Long K lies further from the L2: its chunks take longer; so do those of rows that
+// lie multiples of 4 KB apart (N 1536, M 151, two splits: K 4096 8.8 us, K 5120 8.3; M 674, N 1360, K 8192 17.6, K 7680 13.9).
 static double half_estimate(int kc, int chunks, int splits, int64_t ctas) {
-    const double n = static_cast<double>(ctas), far = kc <= 56 ? 0.0 : (kc >= 128 ? 0.04 : 0.04 * (kc - 56) / 72.0);
+    const double n = static_cast<double>(ctas), far = (kc <= 56 ? 0.0 : (kc >= 128 ? 0.04 : 0.04 * (kc - 56) / 72.0)) + (kc % 32 ? 0.0 : 0.04);
     return splits == 1 ? 2.97 + (0.18 + far) * chunks + 0.0065 * n : 4.1 + (0.1955 + far) * chunks + 0.0078 * n + 0.123 * (splits - 2);
 }
 
-// Pinned values (dsv3_set_gemm_policy) are honoured or refused (pl.error), never rewritten; the automatic
-// plan adapts freely.  dev, sms: the device (-1: none) and the SMs there are on it, or the budget for them.
 // Time of n wide tiles (256 x 256) on so many pairs, in the plan's microseconds.  The last round may be cut into strips.
 static double wide_estimate(int64_t n, int64_t pairs, int kc) {
     const int strip = tw_strip_width(n % pairs, pairs, kc);
@@ -964,6 +963,8 @@ static double wide_estimate(int64_t n, int64_t pairs, int kc) {
     return 0.5 + static_cast<double>((n + pairs - 1) / pairs) * (kc * 0.38 + 0.9);
 }
 
+// Pinned values (dsv3_set_gemm_policy) are honoured or refused (pl.error), never rewritten; the automatic
+// plan adapts freely.  dev, sms: the device (-1: none) and the SMs there are on it, or the budget for them.
 // estimate: microseconds (automatic plans of token-major tiles; otherwise 0)
 static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split, int dev, int sms, double& estimate) {
     TcPlan pl;
@@ -1104,14 +1105,18 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
         // fitted to 412 launches of 172 shapes of 70 to 2200 tokens (rms 5 %, weights from HBM, a replayed graph); against what the plan chose
         // before, 59 of the shapes take them, two of these 2 % slower than before.  us, before / so: M 1003, N 576, K 7168 12.3 / 10.0; M 256, N 576, K 7168
         // 9.3 / 7.4; M 1000, N 256, K 7168 10.2 / 8.2; M 200, N 2304, K 7168 12.4 / 10.1; M 529, N 1584, K 4224 11.5 / 9.3; M 70, N 7168, K 2304 8.6 / 7.1;
-        // M 650, N 800, K 896 5.6 / 4.7.  (Clusters of three and more that leave few SMs over wait for room: M 600, N 576, K 7168, 45 of three, 10.9.)
-        if (force_kernel == 0 && M > 64 && pl.kc <= 144) {
+        // M 650, N 800, K 896 5.6 / 4.7.  Clusters of more than two that leave few SMs over wait for room, odd ones, which leave an SM of a pair over, sooner
+        // (behind act_quant, M 1328, N 256, K 7168, 44 of three, 15.9 / 18.0; M 1280, 40 of three, 15.7 / 13.4; M 301, N 688, K 7936, 33 of four, 14.0 / 11.2).
+        // Beyond 96 MB HBM bounds both (M 107, N 8688, K 14336 28.5 / 30.4).  Against narrow token tiles the estimates, and behind act_quant the
+        // launches, are further apart: of 45 shapes with 0.85 between them all but one gain, up to 2.2, of 21 with less seven lose 0.2 to 0.4.
+        if (force_kernel == 0 && M > 64 && pl.kc <= 144 && N * K <= (96ll << 20)) {
             const int64_t narrow = static_cast<int64_t>(pl.tiles_p) * ((N + 63) / 64);
+            const double margin = chosen.bn ? 0.85 : 0.4;
             for (int sfac = 1; sfac <= kMaxClusterSplits && sfac <= pl.kc && narrow * sfac <= sms; ++sfac) {
-                if (sfac > 1 && (narrow > clusters_resident(dev, sms, false, 64, sfac) || (sfac > 2 && 10 * narrow * sfac > 9 * sms))) continue;
+                if (sfac > 1 && (narrow > clusters_resident(dev, sms, false, 64, sfac) || (sfac > 2 && 20 * narrow * sfac > (sfac % 2 ? 17 : 18) * sms))) continue;
                 const double t = half_estimate(pl.kc, (pl.kc + sfac - 1) / sfac, sfac, narrow * sfac), floor = bytes / 6.0e6 + 2.4;
-                if (t < now - 0.4 && floor < now - 0.4) {
-                    now = t + 0.4;
+                if (t < now - margin && floor < now - margin) {
+                    now = t + margin;
                     estimate = t;
                     chosen = {0, 0, 0};
                     half_splits = sfac;
