@@ -956,11 +956,14 @@ static double half_estimate(int kc, int chunks, int splits, int64_t ctas) {
     return splits == 1 ? 2.97 + (0.18 + far) * chunks + 0.0065 * n : 4.1 + (0.1955 + far) * chunks + 0.0078 * n + 0.123 * (splits - 2);
 }
 
-// Time of n wide tiles (256 x 256) on so many pairs, in the plan's microseconds.  The last round may be cut into strips.
+// Time of n wide tiles (256 x 256) on so many pairs, in the plan's microseconds.  The last round may be cut into strips.  Scales that do not
+// come four chunks at a time lengthen the chunks, with long rows of them more: 256 x 256 tiles against 256 x 128, us, M 2048, N 7168, 56, 57 and 58 chunks
+// 102 / 115, 117 / 116, 111 / 116; M 4096, N 7168, 16 and 17 58 / 77, 69 / 76; M 8000, N 5120, 96 and 97 420 / 657, 613 / 520; M 1585, N 3936, 89 96 / 77.
 static double wide_estimate(int64_t n, int64_t pairs, int kc) {
+    const double chunk = kc % 4 == 0 ? 0.38 : 0.38 * ((kc % 2 ? 1.12 : 1.05) + (kc > 64 ? 0.003 * (kc - 64) : 0.0));
     const int strip = tw_strip_width(n % pairs, pairs, kc);
-    if (strip) return 0.5 + static_cast<double>(n / pairs) * (kc * 0.38 + 0.9) + kc * (strip == 64 ? 0.27 : 0.37) + 1.5;
-    return 0.5 + static_cast<double>((n + pairs - 1) / pairs) * (kc * 0.38 + 0.9);
+    if (strip) return 0.5 + static_cast<double>(n / pairs) * (kc * chunk + 0.9) + kc * (strip == 64 ? 0.27 : 0.37) + 1.5;
+    return 0.5 + static_cast<double>((n + pairs - 1) / pairs) * (kc * chunk + 0.9);
 }
 
 // Pinned values (dsv3_set_gemm_policy) are honoured or refused (pl.error), never rewritten; the automatic
