@@ -436,8 +436,8 @@ fp8_gemm_tw_kernel(const __grid_constant__ TwOperands<kMats> o, const TwParams p
         // Scales, kBlock chunks at a time.  A thread's a_s row is a 32-byte sector of its own, and L1 (what the operand
         // stages leave of it) does not hold 256 of them until the next chunk: one chunk at a time, the scales cost a quarter
         // as much L2 traffic as the operands and a wait in every chunk (M 4096, N 7168, K 16384: 465 us, with no scale loads
-        // at all 419, as here 430).  One 16-byte load brings four chunks; it is issued as soon as the fourth
-        // product is formed and has that chunk's time to arrive.  Rows that 16-byte loads cannot read (K chunks not a
+        // at all 419, as here 430; with products in halves 394, with no loads 367, eight chunks at a time 458).  One 16-byte load brings
+        // four chunks; it is issued as soon as the fourth product is formed and has that chunk's time to arrive.  Rows that 16-byte loads cannot read (K chunks not a
         // multiple of four) take 8-byte loads, kBlock = 2, or the scalar form; scalar / 8-byte, M 4096, N 7168, K 2304 64.2 / 62.6 us, M 8862,
         // N 2608, K 8960 195.4 / 190.7, M 2000, N 2048, K 2816 15.9 / 15.5.
         float ra[kBlock], rb[kBlock];
