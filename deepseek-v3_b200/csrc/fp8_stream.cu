@@ -1217,17 +1217,8 @@ int launch_stream(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMa
 }
 
 template <bool kSwiglu, bool kBoth>
-int launch_divided(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, StreamParams prm, int64_t most_large,
-                   int64_t most_small, int divide, int sms, cudaStream_t stream) {
-    CUtensorMap c0, c1;
-    memset(&c0, 0, sizeof(c0));
-    memset(&c1, 0, sizeof(c1));
-    if (!kSwiglu)
-        for (int i = 0; i < 2; ++i) {
-            const Side& d = prm.side[i];
-            int rc;
-            if (d.c && d.vec_store && (rc = make_tmap_out(i == kGroups ? &c0 : &c1, d.c, d.rows, d.N, 32)) != DSV3_OK) return rc;
-        }
+int launch_divided(const CUtensorMap& w0, const CUtensorMap& w1, const CUtensorMap& ta0, const CUtensorMap& ta1, const CUtensorMap& c0,
+                   const CUtensorMap& c1, StreamParams prm, int64_t most_large, int64_t most_small, int divide, int sms, cudaStream_t stream) {
     constexpr int kLarge = SCfg<128, true>::kSmemBytes, kSmall = SCfg<64, false>::kSmemBytes;
     static bool configured[64] = {};
     StreamParams small = prm;
@@ -1290,14 +1281,21 @@ static int fill_side(Side& d, CUtensorMap* map, const StreamSide& q, bool swiglu
     return DSV3_OK;
 }
 
-int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
+// A launch whose arguments have been looked at.
+namespace {
+struct StreamLaunch {
     StreamParams prm;
-    memset(&prm, 0, sizeof(prm));
-    CUtensorMap w0, w1, ta0, ta1;
-    memset(&w0, 0, sizeof(w0));
-    memset(&w1, 0, sizeof(w1));
-    memset(&ta0, 0, sizeof(ta0));
-    memset(&ta1, 0, sizeof(ta1));
+    CUtensorMap w0, w1, ta0, ta1, c0, c1;       // c0, c1: results of tiles of 128 tokens
+    int bn, sms, divide;
+    bool swiglu, ordinary, split;
+    int64_t bound, small;                       // tiles at most (cut tiles: K chunks); of groups of one token tile
+};
+}  // namespace
+
+static int plan_stream(const StreamGemm& q, StreamLaunch& l) {
+    memset(&l, 0, sizeof(l));
+    StreamParams& prm = l.prm;
+    CUtensorMap &w0 = l.w0, &w1 = l.w1, &ta0 = l.ta0, &ta1 = l.ta1;
     int rc;
     const bool ordinary = q.ordinary.rows > 0;
     const int64_t per_tile = q.n_groups > 0 ? (q.rows_expected + q.n_groups - 1) / q.n_groups : q.ordinary.rows;
@@ -1348,33 +1346,59 @@ int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
         set_last_error("fp8 stream GEMM: %lld K chunks are more than the work-item counter holds", static_cast<long long>(units));
         return DSV3_ERR_UNSUPPORTED;
     }
-    const int64_t bound = split ? units : tiles[0] + tiles[1];
+    if (bn == 128 && !q.swiglu)
+        for (int i = 0; i < 2; ++i) {
+            const Side& d = prm.side[i];
+            if (d.c && d.vec_store && (rc = make_tmap_out(i == kGroups ? &l.c0 : &l.c1, d.c, d.rows, d.N, 32)) != DSV3_OK) return rc;
+        }
+    if (bn != 16 && bn != 32 && bn != 64 && bn != 128) return DSV3_ERR_UNSUPPORTED;
+    l.bn = bn;
+    l.sms = sms;
+    l.divide = sm_budget_set() ? 0 : kDivide;       // under a budget both kinds' CTAs could be resident side by side
+    l.swiglu = q.swiglu;
+    l.ordinary = ordinary;
+    l.split = split;
+    l.bound = split ? units : tiles[0] + tiles[1];
+    l.small = (q.n_groups < q.groups.rows ? q.n_groups : q.groups.rows) * prm.side[kGroups].tiles_p;    // (a group of at most kDivide rows is one token tile)
+    return DSV3_OK;
+}
+
+static int launch_planned(const StreamLaunch& l, cudaStream_t stream) {
 #define DSV3_STREAM_LAUNCH(BN_, SW_, SPLIT_)                                                                               \
-    return ordinary ? launch_stream<BN_, SW_, true, SPLIT_>(w0, w1, ta0, ta1, prm, bound, sms, stream)                          \
-                    : launch_stream<BN_, SW_, false, SPLIT_>(w0, w1, ta0, ta1, prm, bound, sms, stream)
+    return l.ordinary ? launch_stream<BN_, SW_, true, SPLIT_>(l.w0, l.w1, l.ta0, l.ta1, l.prm, l.bound, l.sms, stream)          \
+                      : launch_stream<BN_, SW_, false, SPLIT_>(l.w0, l.w1, l.ta0, l.ta1, l.prm, l.bound, l.sms, stream)
 #define DSV3_STREAM_CASE(BN_)                                                                                              \
     case BN_:                                                                                                              \
-        if (q.swiglu) { if (split) DSV3_STREAM_LAUNCH(BN_, true, true); DSV3_STREAM_LAUNCH(BN_, true, false); }            \
-        if (split) DSV3_STREAM_LAUNCH(BN_, false, true);                                                                   \
+        if (l.swiglu) { if (l.split) DSV3_STREAM_LAUNCH(BN_, true, true); DSV3_STREAM_LAUNCH(BN_, true, false); }          \
+        if (l.split) DSV3_STREAM_LAUNCH(BN_, false, true);                                                                 \
         DSV3_STREAM_LAUNCH(BN_, false, false)
-    switch (bn) {
+#define DSV3_DIVIDED_LAUNCH(SW_)                                                                                           \
+    return l.ordinary ? launch_divided<SW_, true>(l.w0, l.w1, l.ta0, l.ta1, l.c0, l.c1, l.prm, l.bound, l.small, l.divide, l.sms, stream) \
+                      : launch_divided<SW_, false>(l.w0, l.w1, l.ta0, l.ta1, l.c0, l.c1, l.prm, l.bound, l.small, l.divide, l.sms, stream)
+    switch (l.bn) {
         DSV3_STREAM_CASE(16);
         DSV3_STREAM_CASE(32);
         DSV3_STREAM_CASE(64);
-        case 128: {
-            // a group of at most kDivide rows is one token tile
-            const int64_t small = (q.n_groups < q.groups.rows ? q.n_groups : q.groups.rows) * prm.side[kGroups].tiles_p;
-            const int divide = sm_budget_set() ? 0 : kDivide;       // under a budget both kinds' CTAs could be resident side by side
-            if (q.swiglu)
-                return ordinary ? launch_divided<true, true>(w0, w1, ta0, ta1, prm, bound, small, divide, sms, stream)
-                                : launch_divided<true, false>(w0, w1, ta0, ta1, prm, bound, small, divide, sms, stream);
-            return ordinary ? launch_divided<false, true>(w0, w1, ta0, ta1, prm, bound, small, divide, sms, stream)
-                            : launch_divided<false, false>(w0, w1, ta0, ta1, prm, bound, small, divide, sms, stream);
-        }
+        default:
+            if (l.swiglu) DSV3_DIVIDED_LAUNCH(true);
+            DSV3_DIVIDED_LAUNCH(false);
     }
 #undef DSV3_STREAM_LAUNCH
 #undef DSV3_STREAM_CASE
-    return DSV3_ERR_UNSUPPORTED;
+#undef DSV3_DIVIDED_LAUNCH
+}
+
+int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream) {
+    StreamLaunch l;
+    const int rc = plan_stream(q, l);
+    return rc != DSV3_OK ? rc : launch_planned(l, stream);
+}
+
+int launch_fp8_streams(const StreamGemm& first, const StreamGemm& second, cudaStream_t stream) {
+    StreamLaunch l[2];
+    int rc;
+    if ((rc = plan_stream(first, l[0])) != DSV3_OK || (rc = plan_stream(second, l[1])) != DSV3_OK) return rc;
+    return (rc = launch_planned(l[0], stream)) != DSV3_OK ? rc : launch_planned(l[1], stream);
 }
 
 // The table holds, in device memory, n tensor maps, n scale pointers and n weight pointers.

@@ -104,6 +104,8 @@ int stream_tile(int64_t rows_per_group);
 size_t stream_workspace_bytes(int64_t rows_per_group);
 size_t stream_tile_workspace_bytes(int bn);
 int launch_fp8_stream(const StreamGemm& q, cudaStream_t stream);
+// One after the other; nothing is launched where either is refused.
+int launch_fp8_streams(const StreamGemm& first, const StreamGemm& second, cudaStream_t stream);
 
 // Table of the weights of up to 256 groups: tensor maps, scale pointers and weight pointers, in device memory.
 constexpr int kMaxGroupsOfTable = 256;

@@ -453,23 +453,19 @@ int add_ordinary(StreamGemm& q, const dsv3_side_gemm_t* s) {
     return DSV3_OK;
 }
 
-int grouped_plain(const void* table, int n, const void* a, const float* a_s, bool transposed, const int32_t* seg, int64_t rows_total,
-                  int64_t rows_hint, int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace, size_t workspace_bytes,
-                  bool early, dsv3_stream_t stream) {
-    int rc = check_groups(n, a, K);
+int grouped_plain(StreamGemm& q, const void* table, int n, const void* a, const float* a_s, bool transposed, const int32_t* seg, int64_t rows_total,
+                  int64_t rows_hint, int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace, size_t workspace_bytes) {
+    const int rc = check_groups(n, a, K);
     if (rc != DSV3_OK) return rc;
-    StreamGemm q = {};
     q.groups = side_of(a, a_s, transposed, rows_total, N, K);
     q.groups.c = c;
     q.rows_expected = rows_hint > 0 && rows_hint < rows_total ? rows_hint : rows_total;
     q.n_groups = n;
     q.table0 = table;
     q.seg = seg;
-    q.early = early;
     q.workspace = workspace;
     q.workspace_bytes = workspace_bytes;
-    if ((rc = add_ordinary(q, side)) != DSV3_OK) return rc;
-    return launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
+    return add_ordinary(q, side);
 }
 
 }  // namespace
@@ -502,12 +498,15 @@ int dsv3_fp8_gemm_grouped(const void* table, int n_groups, const void* a, const 
         set_last_error("fp8_gemm_grouped: null pointer");
         return DSV3_ERR_INVALID_ARGUMENT;
     }
-    return grouped_plain(table, n_groups, a, a_s, false, seg, rows_total, rows_hint, N, K, c, nullptr, nullptr, 0, false, stream);
+    StreamGemm q = {};
+    const int rc = grouped_plain(q, table, n_groups, a, a_s, false, seg, rows_total, rows_hint, N, K, c, nullptr, nullptr, 0);
+    return rc != DSV3_OK ? rc : launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
 }
 
-static int gemm_rows(const void* table, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total, int64_t rows_hint,
-                     int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace, size_t workspace_bytes, bool early,
-                     dsv3_stream_t stream) {
+// The arguments of dsv3_fp8_gemm_rows and dsv3_swiglu_gemm_rows as a launch; any: whether there is one.
+static int gemm_rows(StreamGemm& q, bool& any, const void* table, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total,
+                     int64_t rows_hint, int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace, size_t workspace_bytes) {
+    any = false;
     if (rows_total < 0 || rows_hint < 0 || N < 0 || K <= 0) {
         set_last_error("fp8_gemm_rows: negative size");
         return DSV3_ERR_INVALID_ARGUMENT;
@@ -517,18 +516,23 @@ static int gemm_rows(const void* table, int n_groups, const void* a, const float
         set_last_error("fp8_gemm_rows: null pointer");
         return DSV3_ERR_INVALID_ARGUMENT;
     }
-    return grouped_plain(table, n_groups, a, a_s_t, true, seg, rows_total, rows_hint, N, K, c, side, workspace, workspace_bytes, early, stream);
+    any = true;
+    return grouped_plain(q, table, n_groups, a, a_s_t, true, seg, rows_total, rows_hint, N, K, c, side, workspace, workspace_bytes);
 }
 
 int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total,
                        int64_t rows_hint, int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace,
                        size_t workspace_bytes, dsv3_stream_t stream) {
-    return gemm_rows(table, n_groups, a, a_s_t, seg, rows_total, rows_hint, N, K, c, side, workspace, workspace_bytes, false, stream);
+    StreamGemm q = {};
+    bool any = false;
+    const int rc = gemm_rows(q, any, table, n_groups, a, a_s_t, seg, rows_total, rows_hint, N, K, c, side, workspace, workspace_bytes);
+    return rc != DSV3_OK || !any ? rc : launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
 }
 
-static int swiglu_rows(const void* table1, const void* table3, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total,
-                       int64_t rows_hint, int64_t N, int64_t K, int scale_fmt, void* hq, float* hs_t, const dsv3_side_gemm_t* side, void* workspace,
-                       size_t workspace_bytes, bool leads, dsv3_stream_t stream) {
+static int swiglu_rows(StreamGemm& q, bool& any, const void* table1, const void* table3, int n_groups, const void* a, const float* a_s_t, const int32_t* seg,
+                       int64_t rows_total, int64_t rows_hint, int64_t N, int64_t K, int scale_fmt, void* hq, float* hs_t, const dsv3_side_gemm_t* side,
+                       void* workspace, size_t workspace_bytes) {
+    any = false;
     if (rows_total < 0 || rows_hint < 0 || N < 0 || K <= 0) {
         set_last_error("swiglu_gemm_rows: negative size");
         return DSV3_ERR_INVALID_ARGUMENT;
@@ -546,9 +550,9 @@ static int swiglu_rows(const void* table1, const void* table3, int n_groups, con
         set_last_error("swiglu_gemm_rows: N = %lld is not divisible by 128", static_cast<long long>(N));
         return DSV3_ERR_UNSUPPORTED;
     }
-    int rc = check_groups(n_groups, a, K);
+    const int rc = check_groups(n_groups, a, K);
     if (rc != DSV3_OK) return rc;
-    StreamGemm q = {};
+    any = true;
     q.groups = side_of(a, a_s_t, true, rows_total, N, K);
     q.groups.hq = hq;
     q.groups.hs = hs_t;
@@ -560,30 +564,33 @@ static int swiglu_rows(const void* table1, const void* table3, int n_groups, con
     q.table1 = table3;
     q.seg = seg;
     q.swiglu = true;
-    q.leads = leads;
     q.scale_fmt = scale_fmt;
     q.workspace = workspace;
     q.workspace_bytes = workspace_bytes;
-    if ((rc = add_ordinary(q, side)) != DSV3_OK) return rc;
-    return launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
+    return add_ordinary(q, side);
 }
 
 int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, const void* a, const float* a_s_t, const int32_t* seg,
                           int64_t rows_total, int64_t rows_hint, int64_t N, int64_t K, int scale_fmt, void* hq, float* hs_t,
                           const dsv3_side_gemm_t* side, void* workspace, size_t workspace_bytes, dsv3_stream_t stream) {
-    return swiglu_rows(table1, table3, n_groups, a, a_s_t, seg, rows_total, rows_hint, N, K, scale_fmt, hq, hs_t, side, workspace, workspace_bytes, false,
-                       stream);
+    StreamGemm q = {};
+    bool any = false;
+    const int rc = swiglu_rows(q, any, table1, table3, n_groups, a, a_s_t, seg, rows_total, rows_hint, N, K, scale_fmt, hq, hs_t, side, workspace, workspace_bytes);
+    return rc != DSV3_OK || !any ? rc : launch_fp8_stream(q, static_cast<cudaStream_t>(stream));
 }
 
 // The second launch begins to read its weights while the CTAs of the first leave (StreamGemm::early).
 int dsv3_expert_gemms(const void* table1, const void* table3, const void* table2, int n_groups, const void* a, const float* a_s_t, const int32_t* seg,
                       int64_t rows_total, int64_t rows_hint, int64_t inter, int64_t dim, int scale_fmt, void* hq, float* hs_t, void* o,
                       const dsv3_side_gemm_t* up, const dsv3_side_gemm_t* down, void* workspace, size_t workspace_bytes, dsv3_stream_t stream) {
-    const int rc = swiglu_rows(table1, table3, n_groups, a, a_s_t, seg, rows_total, rows_hint, inter, dim, scale_fmt, hq, hs_t, up, workspace,
-                               workspace_bytes, true, stream);
-    if (rc != DSV3_OK) return rc;
-    return gemm_rows(table2, n_groups, hq, hs_t, seg, rows_total, rows_hint, dim, inter, o, down, workspace, workspace_bytes,
-                     rows_total > 0 && inter > 0, stream);
+    StreamGemm first = {}, second = {};
+    bool any_first = false, any_second = false;
+    int rc = swiglu_rows(first, any_first, table1, table3, n_groups, a, a_s_t, seg, rows_total, rows_hint, inter, dim, scale_fmt, hq, hs_t, up, workspace,
+                         workspace_bytes);
+    if (rc == DSV3_OK) rc = gemm_rows(second, any_second, table2, n_groups, hq, hs_t, seg, rows_total, rows_hint, dim, inter, o, down, workspace, workspace_bytes);
+    if (rc != DSV3_OK || !any_first || !any_second) return rc;      // (both or neither: rows and sizes are the same)
+    first.leads = second.early = true;
+    return launch_fp8_streams(first, second, static_cast<cudaStream_t>(stream));
 }
 
 // (a kernel or split that the host pinned is one of fp8_gemm's: the separate launches honour or refuse it)

@@ -65,3 +65,26 @@ def test_like_the_launches_one_after_the_other(counts, inter, dim, side_rows, wo
                 assert torch.equal(a.view(torch.uint8) if a.element_size() == 1 else a, b.view(torch.uint8) if b.element_size() == 1 else b)
     finally:
         dsv3_b200.set_num_sms(0)
+
+
+@pytest.mark.parametrize("wrong", ["table", "out", "dim"])
+def test_refused_as_one(wrong):
+    """An argument that only w2's launch is refused for leaves w1's and w3's results alone, too."""
+    from dsv3_b200 import _lib
+    i64, p = ctypes.c_int64, lambda t, at=0: ctypes.c_void_p(t.data_ptr() + at)
+    layer = _Layer([5, 3, 2], 256, 512, 9)
+    m, dim, (t1, t3, t2) = layer.side_rows, layer.dim, layer.tables
+    out = [torch.full((layer.rows * 2048,), 7, dtype=torch.uint8, device="cuda") for _ in range(6)]
+    hq, hs, o, zq, zs, z = out
+    up = _Side(layer.sq.data_ptr(), layer.ss.data_ptr(), 0, m, 256, dim, layer.s1.data_ptr(), layer.s1.scale.data_ptr(), layer.s3.data_ptr(),
+               layer.s3.scale.data_ptr(), zq.data_ptr(), zs.data_ptr())
+    down = _Side(zq.data_ptr(), zs.data_ptr(), 1, m, dim, 256, layer.s2.data_ptr(), layer.s2.scale.data_ptr(), None, None,
+                 z.data_ptr() + (2 if wrong == "out" else 0), None)
+    if wrong == "dim":
+        down.K = 8                     # no multiple of 16
+    rc = _lib.lib.dsv3_expert_gemms(p(t1), p(t3), None if wrong == "table" else p(t2), layer.n, p(layer.xq), p(layer.xs_t), p(layer.seg),
+                                    i64(layer.rows), i64(0), i64(layer.inter), i64(dim), 0, p(hq), p(hs), p(o), ctypes.byref(up), ctypes.byref(down),
+                                    None, ctypes.c_size_t(0), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc != _lib.OK
+    torch.cuda.synchronize()
+    assert all(bool((t == 7).all()) for t in out)
