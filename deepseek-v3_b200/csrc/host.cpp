@@ -350,14 +350,18 @@ at::Tensor mlp(const at::Tensor& x, const at::Tensor (&w)[3], const at::Tensor (
     auto f32 = [](const at::Tensor& t) { return static_cast<const float*>(t.const_data_ptr()); };
     const float *as = f32(q.second), *s1 = f32(s[0]), *s3 = f32(s[1]);
     if (!fused) {
-        const at::Tensor y1 = new_cuda_last(x, N, at::kBFloat16), y3 = new_cuda_last(x, N, at::kBFloat16);
+        // (what is no longer read is given back at once, as the separate launches give it back: w2's result may take its place)
+        at::Tensor y1 = new_cuda_last(x, N, at::kBFloat16), y3 = new_cuda_last(x, N, at::kBFloat16);
         void *y1p = y1.data_ptr(), *y3p = y3.data_ptr();
         call_library(dev, [&](dsv3_stream_t st) { return dsv3_fp8_gemm_two(a, as, p1, s1, p3, s3, M, N, K, y1p, y3p, st); });
+        q = {};
         h = new_cuda_last(x, N, at::kFloat8_e4m3fn);
         hs = new_cuda_last(x, N / 128, at::kFloat);
         void* hp = h.data_ptr();
         float* hsp = static_cast<float*>(hs.data_ptr());
         call_library(dev, [&](dsv3_stream_t st) { return dsv3_swiglu_quant(y1p, y3p, M, N, h_fmt, hp, hsp, st); });
+        y1.reset();
+        y3.reset();
         return gemm(h, hs, w[2], s[2]);
     }
     h = new_cuda_last(x, N, at::kFloat8_e4m3fn);

@@ -87,3 +87,34 @@ def test_an_mlp_of_four_launches(dim, inter, M, fmt):
         assert len(_kernels(lambda: mlp(x.view(x.shape)))) == 4
         y3 = mlp(x.view(1, M, dim))
         assert y3.shape == (1, M, dim) and torch.equal(y3[0], got)
+
+
+@pytest.mark.parametrize("dim,inter,M", [(7168, 2304, 2580), (2048, 2816, 3942)])
+def test_memory_of_an_mlp_of_four_launches(dim, inter, M):
+    """No more at its peak than the operators one by one, each of whose inputs is given back once it has been read."""
+    import kernel
+    from dsv3_b200 import swiglu_quant
+    from dsv3_b200._lib import host
+    mlp, model = _host(dim, inter)
+    w1, w3, w2 = mlp.w1.weight, mlp.w3.weight, mlp.w2.weight
+    x = _rows(M, dim)
+
+    def one_by_one():
+        q, s = kernel.act_quant(x)
+        y1, y3 = kernel.fp8_gemm(q, s, w1, w1.scale), kernel.fp8_gemm(q, s, w3, w3.scale)
+        del q, s
+        h = swiglu_quant(y1, y3)
+        del y1, y3
+        return kernel.fp8_gemm(*h, w2, w2.scale)
+
+    def peak(run):
+        run()                                     # workspaces
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        run()
+        return torch.cuda.max_memory_allocated() - before
+
+    with torch.inference_mode():                  # a tensor without a modification counter: its quantisation is not kept
+        x = x.clone()
+        assert peak(lambda: host.mlp(x, w1, w3, w2, None, None, False)) <= peak(one_by_one)
