@@ -88,3 +88,57 @@ def test_refused_as_one(wrong):
     assert rc != _lib.OK
     torch.cuda.synchronize()
     assert all(bool((t == 7).all()) for t in out)
+
+
+# 3, 10, 30 and 100 rows per group: every tile width, whole and cut
+@pytest.mark.parametrize("T,topk,n,inter,dim", [(6, 2, 4, 256, 512), (40, 2, 8, 2048, 1152), (120, 2, 8, 384, 1152), (400, 2, 8, 384, 512)])
+@pytest.mark.parametrize("workspace", [True, False])
+def test_routing_that_changes_from_pass_to_pass(T, topk, n, inter, dim, workspace):
+    """The row offsets, which w2's launch reads while w1's and w3's still runs, are written by the dispatch in front of both, to the same
+    memory in every pass and with other counts in each.  Reference: the launches with a synchronisation behind each."""
+    from dsv3_b200 import _lib
+    lib, i64, p = _lib.lib, ctypes.c_int64, lambda t: ctypes.c_void_p(t.data_ptr())
+    layer = _Layer([1] * n, inter, dim, 0)
+    t1, t3, t2 = layer.tables
+    g = torch.Generator(device="cuda").manual_seed(T)
+    E, P, start = n + 3, T * topk, 1
+    x = torch.randn(T, dim, generator=g, device="cuda", dtype=torch.float32).bfloat16()
+    w = torch.rand(T, topk, generator=g, device="cuda", dtype=torch.float32)
+    # all experts alike; the first and the last local one only; half of the pairs elsewhere; no local ones
+    prefer = [torch.zeros(E), torch.tensor([0.0, 9.0] + [0.0] * (n - 2) + [9.0] + [0.0] * (E - n - 1)), torch.tensor([9.0] + [0.0] * (E - 1)),
+              torch.tensor([9.0] + [0.0] * n + [1.0] * (E - n - 1))]
+    routings = [(torch.rand(T, E, generator=g, device="cuda") + q.cuda()).topk(topk, dim=-1).indices for q in prefer]
+    size = dict(seg=4 * (n + 1), pos=4 * P, ws=2 * P, xq=T * dim, xs=4 * T * (dim // 128), xr=P * dim, xst=4 * P * (dim // 128), hq=P * inter,
+                hs=4 * P * (inter // 128), o=2 * P * dim)
+    b = {k: torch.zeros(v, dtype=torch.uint8, device="cuda") for k, v in size.items()}
+    idx = torch.empty_like(routings[0])
+    need = lib.dsv3_gemm_rows_workspace_bytes(n, i64(P), i64(0))
+    space = torch.zeros(max(need, 1), dtype=torch.uint8, device="cuda") if workspace else None
+    tail = (p(space) if workspace else None, ctypes.c_size_t(need if workspace else 0))
+    results = ("seg", "hq", "hs", "o")
+
+    def one_pass(i, between):
+        stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        for k in results[1:]:
+            b[k].zero_()
+        idx.copy_(routings[i])
+        _lib.check(lib.dsv3_moe_dispatch(p(x), i64(T), i64(dim), p(idx), p(w), 0, topk, start, n, 0, p(b["seg"]), p(b["pos"]), p(b["ws"]), p(b["xq"]),
+                                         p(b["xs"]), p(b["xr"]), p(b["xst"]), stream))
+        rows = (p(b["seg"]), i64(P), i64(0))
+        if between:
+            between()
+            _lib.check(lib.dsv3_swiglu_gemm_rows(p(t1), p(t3), n, p(b["xr"]), p(b["xst"]), *rows, i64(inter), i64(dim), 0, p(b["hq"]), p(b["hs"]), None,
+                                                 *tail, stream))
+            between()
+            _lib.check(lib.dsv3_fp8_gemm_rows(p(t2), n, p(b["hq"]), p(b["hs"]), *rows, i64(dim), i64(inter), p(b["o"]), None, *tail, stream))
+            between()
+        else:
+            _lib.check(lib.dsv3_expert_gemms(p(t1), p(t3), p(t2), n, p(b["xr"]), p(b["xst"]), *rows, i64(inter), i64(dim), 0, p(b["hq"]), p(b["hs"]),
+                                             p(b["o"]), None, None, *tail, stream))
+        return [b[k].clone() for k in results]
+
+    want = [one_pass(i, torch.cuda.synchronize) for i in range(4)]
+    assert all(not torch.equal(want[i][0], want[j][0]) for i in range(4) for j in range(i))
+    got = [(i, one_pass(i, None)) for i in (0, 1, 2, 3, 1, 0, 3, 2, 0)]
+    for i, tensors in got:
+        assert all(torch.equal(a, c) for a, c in zip(tensors, want[i]))
