@@ -89,9 +89,8 @@ __global__ void __launch_bounds__(kThreads) act_quant_generic_kernel(const uint4
 
 // SwiGLU followed by act_quant in one pass: h = bf16(bf16(silu(a)) * b), then h is quantised per 128 values.
 // Replaces the three launches `F.silu(w1(x)) * w3(x)` + act_quant in front of w2 (model.py:532, 633 and 158-159) and
-// keeps their rounding points: silu is evaluated in fp32 and rounded to bf16 (swiglu8), the product is
-// formed in fp32 and rounded to bf16 (what the framework's bf16 kernels do), and the quantisation of h is the
-// arithmetic of act_quant128_kernel.  h itself is never written.
+// keeps their rounding points: silu is evaluated in fp32 and rounded to bf16, the product is rounded to bf16 (swiglu8: the values of
+// the framework's bf16 kernels), and the quantisation of h is the arithmetic of act_quant128_kernel.  h itself is never written.
 // Two blocks of each operand per thread and six CTAs per SM: with four and four (64 registers, as above) fewer warps have
 // loads in flight while others compute (2048 x 2048 6.7 us, so 6.15; 300 x 18432 8.0, 7.2; 8192 x 18432 134 either way).
 constexpr int kSwigluUnroll = 2;

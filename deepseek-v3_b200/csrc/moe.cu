@@ -29,8 +29,8 @@ constexpr int kThreads = 256;
 constexpr int kCombineManyTokens = 400, kCombineManyDim = 4096;
 
 // Two bf16 values to a word, each result rounded once to bf16: what a product or sum formed in fp32 and then rounded gives (a
-// product of two bf16 values is exact in fp32, and a sum that is not lies too far from a tie of bf16 to be rounded twice; below
-// 2^-126 a product need not be exact in fp32, and is rounded once here where the other form rounds it twice).
+// product of two bf16 values is exact in fp32, or below 2^-134, where either way ends at zero; a sum that is not exact lies too far from a
+// tie of bf16 for the first of two roundings to matter).
 __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
     uint32_t d;
     asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));

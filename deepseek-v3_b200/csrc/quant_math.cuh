@@ -106,7 +106,8 @@ static __device__ __noinline__ float silu_exact(float a) {
 // h = bf16(bf16(silu(a)) * b) for eight bf16 pairs.
 // silu's fast form, a * rcp(1 + ex2(-a log2 e)), is within 13 ulp of fp32 of the exact one, and rounds to the same bf16 value for every
 // bf16 a but -87.5, -88 and -88.5, whose reciprocals are flushed (all 65536 checked on a B200): those are a * exp(a / 2) * exp(a / 2).
-// The product of two bf16 values is rounded once, as by way of fp32, which holds it exactly unless it is below 2^-126.
+// The product of two bf16 values, rounded once, is what it is by way of fp32: of its at most 16 bits fp32 drops one only below 2^-134, where either
+// way ends at zero.
 // The exact form by a call where the fast one lay near a rounding boundary (0.05 % of values, 13 % of a warp's trips) cost the epilogue of a
 // 128-token tile 2300 of 9700 cycles, the check, the separate product and the maximum per word another 600.  us, with them / without: w1 and w3 of 64
 // experts of 2048 x 1408, 512 rows each 256 / 225, of 32 of 7168 x 2048 485 / 451; swiglu_quant 8192 x 18432 127 / 111, ue8m0 138 / 112,
