@@ -179,7 +179,9 @@ __device__ __forceinline__ Strip decode_strip(int pair, const TwOperands<kMats>&
     return s;
 }
 
-// kBlock: K chunks per scale load: 4 (K chunks a multiple of four, 16-byte aligned scales), 2 (of two, 8-byte) or 1
+// kBlock: K chunks per scale load: 4 (K chunks a multiple of four, 16-byte aligned scales), 2 (of two, 8-byte), else 1, or kShifted: in the
+// aligned groups of four that rows lie in, wherever they begin
+constexpr int kShifted = 0, kShiftedFrom = 11;
 template <int kBlock, int kMats>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_gemm_tw_kernel(const __grid_constant__ TwOperands<kMats> o, const TwParams p) {
@@ -438,9 +440,35 @@ fp8_gemm_tw_kernel(const __grid_constant__ TwOperands<kMats> o, const TwParams p
         // as much L2 traffic as the operands and a wait in every chunk (M 4096, N 7168, K 16384: 465 us, with no scale loads
         // at all 419, as here 430; with products in halves 394, with no loads 367, eight chunks at a time 458).  One 16-byte load brings
         // four chunks; it is issued as soon as the fourth product is formed and has that chunk's time to arrive.  Rows that 16-byte loads cannot read (K chunks not a
-        // multiple of four) take 8-byte loads, kBlock = 2, or the scalar form; scalar / 8-byte, M 4096, N 7168, K 2304 64.2 / 62.6 us, M 8862,
+        // multiple of four) take 8-byte loads, kBlock = 2, or others; scalar / 8-byte, M 4096, N 7168, K 2304 64.2 / 62.6 us, M 8862,
         // N 2608, K 8960 195.4 / 190.7, M 2000, N 2048, K 2816 15.9 / 15.5.
-        float ra[kBlock], rb[kBlock];
+        // From kShiftedFrom chunks rows that begin anywhere are read in aligned groups of four, too, two of which hold the next four chunks: a
+        // thread picks them out by its own row's offset, and the last one to three chunks come behind the groups of four.  A scalar load waits in every
+        // chunk, which products in halves had made longer than what it was before them.  us with act_quant, whole slots and scalar loads / halves and scalar / so: M 2456, N 5456,
+        // K 6272 102.9 / 104.6 / 97.7; M 4096, N 7168, K 7296 247.1 / 251.1 / 236.8; M 8192, N 5120, K 12416 631 / 630 / 551.  Shorter rows are over before it pays: with
+        // 3 to 9 chunks 1 to 5 % slower, with 11 to 17 1 % faster (ten shapes of each).  (Even numbers of chunks: 4 to 6 % slower than 8-byte loads.)
+        float ra[kBlock == kShifted ? 1 : kBlock], rb[kBlock == kShifted ? 4 : kBlock];
+        float4 a_cur, a_next;      // kShifted: the groups that hold the next four chunks' a_s
+        const float* const a_end = p.a_s + p.M * kc;
+        // group `grp` of a row; nothing outside of a_s is read
+        const auto offset_of = [](const float* row) { return static_cast<int>((reinterpret_cast<uintptr_t>(row) >> 2) & 3); };
+        auto a_group = [&](const float* row, int grp) -> float4 {
+            // (predicated, not branched around: behind a branch a load is waited for at once)
+            const float* q = row - offset_of(row) + 4 * grp;
+            const bool whole = q >= p.a_s && q + 4 <= a_end;
+            float4 e = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const auto one = [&](float& x, int i) {
+                asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %1, 0;\n @p ld.global.nc.f32 %0, [%2];\n}"
+                             : "+f"(x) : "r"(static_cast<int>(!whole && q + i >= p.a_s && q + i < a_end)), "l"(q + i));
+            };
+            asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n @p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%5];\n}"
+                         : "+f"(e.x), "+f"(e.y), "+f"(e.z), "+f"(e.w) : "r"(static_cast<int>(whole)), "l"(q));
+            one(e.x, 0);
+            one(e.y, 1);
+            one(e.z, 2);
+            one(e.w, 3);
+            return e;
+        };
         auto next_scales = [&](const float* as, const float* bs, int k) {
             if (k >= kc) return;
             if constexpr (kBlock == 4) {
@@ -451,10 +479,26 @@ fp8_gemm_tw_kernel(const __grid_constant__ TwOperands<kMats> o, const TwParams p
                 const float2 a2 = __ldg(reinterpret_cast<const float2*>(as + k)), b2 = __ldg(reinterpret_cast<const float2*>(bs + k));
                 ra[0] = a2.x; ra[1] = a2.y;
                 rb[0] = b2.x; rb[1] = b2.y;
-            } else {
+            } else if constexpr (kBlock == 1) {
                 ra[0] = __ldg(as + k);
                 rb[0] = __ldg(bs + k);
+            } else {
+                a_cur = k == 0 ? a_group(as, 0) : a_next;
+                a_next = a_group(as, k / 4 + 1);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) rb[i] = __ldg(bs + min(k + i, kc - 1));
             }
+        };
+        // kShifted: the products of the four
+        auto take_scales = [&](const float* as, float (&sc)[4]) {
+            const int m = offset_of(as);
+            const bool one = m & 1, two = m & 2;
+            const float t0 = one ? a_cur.y : a_cur.x, t1 = one ? a_cur.z : a_cur.y, t2 = one ? a_cur.w : a_cur.z;
+            const float t3 = one ? a_next.x : a_cur.w, t4 = one ? a_next.y : a_next.x, t5 = one ? a_next.z : a_next.y;
+            sc[0] = (two ? t2 : t0) * rb[0];
+            sc[1] = (two ? t3 : t1) * rb[1];
+            sc[2] = (two ? t4 : t2) * rb[2];
+            sc[3] = (two ? t5 : t3) * rb[3];
         };
         auto first_scales = [&](const Tile& t) { next_scales(as_row(t), bs_row(t), 0); };
         bool ok = true;
@@ -468,29 +512,58 @@ fp8_gemm_tw_kernel(const __grid_constant__ TwOperands<kMats> o, const TwParams p
                 const float* bs_ptr = bs_row(cur);
 #pragma unroll
                 for (int j = 0; j < 64; ++j) acc[j] = make_float2(0.0f, 0.0f);
-                for (int k0 = 0; ok && k0 < kc; k0 += kBlock) {
+                // one chunk; scale(): its scale, formed (and the next ones asked for) while its first columns are on their way
+                auto chunk = [&](auto scale) {
+                    const int slot = static_cast<int>(g & 1u);
+                    const bool mine = bounded_wait_lean(tfull_bar(half * kSlots + slot), (g >> 1) & 1u, ctl, p.status, 4, g);
+                    ++g;
+                    ok = __all_sync(0xffffffffu, mine);
+                    if (!ok) return;
+                    tc_fence_after();
+                    const uint32_t t_slot = t_lane + slot * kBN;
+                    // The first 64 columns are read back and folded, then the other 64 are read back and the half slot
+                    // returns to the issuer: two read-back latencies per chunk; the last fold follows the release.
+                    tc_ld_x64(t_slot, &v[0][0]);
+                    const float sc = scale();
+                    tc_wait_ld();
+                    fold(v[0], sc, 0);
+                    fold(v[1], sc, 1);
+                    tc_ld_x64(t_slot + 2 * kPiece, &v[0][0]);
+                    tc_wait_ld();
+                    release(slot);
+                    fold(v[0], sc, 2);
+                    fold(v[1], sc, 3);
+                };
+                if constexpr (kBlock == kShifted) {
+                    int k0 = 0;
+                    float sc[4];
+                    for (; ok && k0 + 4 <= kc; k0 += 4) {
 #pragma unroll
-                    for (int i = 0; i < kBlock; ++i) {
-                        const int slot = static_cast<int>(g & 1u);
-                        const bool mine = bounded_wait_lean(tfull_bar(half * kSlots + slot), (g >> 1) & 1u, ctl, p.status, 4, g);
-                        ++g;
-                        ok = __all_sync(0xffffffffu, mine);
-                        if (!ok) break;
-                        tc_fence_after();
-                        const uint32_t t_slot = t_lane + slot * kBN;
-                        // The first 64 columns are read back and folded, then the other 64 are read back and the half slot
-                        // returns to the issuer: two read-back latencies per chunk; the last fold follows the release.
-                        tc_ld_x64(t_slot, &v[0][0]);
-                        const float sc = ra[i] * rb[i];
-                        if (i == kBlock - 1) next_scales(as_ptr, bs_ptr, k0 + kBlock);
-                        tc_wait_ld();
-                        fold(v[0], sc, 0);
-                        fold(v[1], sc, 1);
-                        tc_ld_x64(t_slot + 2 * kPiece, &v[0][0]);
-                        tc_wait_ld();
-                        release(slot);
-                        fold(v[0], sc, 2);
-                        fold(v[1], sc, 3);
+                        for (int i = 0; i < 4; ++i) {
+                            chunk([&] {
+                                if (i == 0) take_scales(as_ptr, sc);
+                                if (i == 3) next_scales(as_ptr, bs_ptr, k0 + 4);
+                                return sc[i];
+                            });
+                            if (!ok) break;
+                        }
+                    }
+                    for (int i = 0; ok && i < kc - k0; ++i)
+                        chunk([&] {
+                            if (i == 0) take_scales(as_ptr, sc);
+                            return i == 0 ? sc[0] : (i == 1 ? sc[1] : sc[2]);
+                        });
+                } else {
+                    for (int k0 = 0; ok && k0 < kc; k0 += kBlock) {
+#pragma unroll
+                        for (int i = 0; i < kBlock; ++i) {
+                            chunk([&] {
+                                const float sc = ra[i] * rb[i];
+                                if (i == kBlock - 1) next_scales(as_ptr, bs_ptr, k0 + kBlock);
+                                return sc;
+                            });
+                            if (!ok) break;
+                        }
                     }
                 }
                 if (!ok) {
@@ -663,7 +736,8 @@ int launch(const void* a, const float* a_s, const void* const* b, const float* c
     uintptr_t scales = reinterpret_cast<uintptr_t>(a_s);
     for (int m = 0; m < kMats; ++m) scales |= reinterpret_cast<uintptr_t>(b_s[m]);
     const auto aligned = [&](int n) { return (prm.kc % n) == 0 && (scales % (4 * n)) == 0; };
-    auto kern = aligned(4) ? fp8_gemm_tw_kernel<4, kMats> : aligned(2) ? fp8_gemm_tw_kernel<2, kMats> : fp8_gemm_tw_kernel<1, kMats>;
+    auto kern = aligned(4) ? fp8_gemm_tw_kernel<4, kMats> : aligned(2) ? fp8_gemm_tw_kernel<2, kMats>
+              : prm.kc >= kShiftedFrom ? fp8_gemm_tw_kernel<kShifted, kMats> : fp8_gemm_tw_kernel<1, kMats>;
     static bool configured[64] = {};
     int dev = 0;
     DSV3_CUDA_TRY(cudaGetDevice(&dev));
@@ -674,6 +748,7 @@ int launch(const void* a, const float* a_s, const void* const* b, const float* c
     if (!configured[dev]) {
         DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<4, kMats>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
         DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<2, kMats>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
+        DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<kShifted, kMats>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
         DSV3_CUDA_TRY(cudaFuncSetAttribute(fp8_gemm_tw_kernel<1, kMats>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
         configured[dev] = true;
     }

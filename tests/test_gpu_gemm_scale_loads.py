@@ -32,3 +32,33 @@ def test_equal_whatever_the_loads(kc, offset):
         dsv3_b200.set_gemm_policy(0, 0)
         torch.set_default_dtype(torch.float32)
         dsv3_b200.check_device_status()
+
+
+# every remainder of four, every place of a row in the groups of four (rows begin at offset + row * kc), the first and the last row of the scales in
+# groups that lie partly outside of them
+@pytest.mark.parametrize("kc", [9, 11, 12, 13, 14, 15, 23])
+@pytest.mark.parametrize("offset", [1, 2, 3])
+@pytest.mark.parametrize("M", [129, 256])
+def test_rows_between_the_groups_of_four(kc, offset, M):
+    import dsv3_b200
+    import kernel
+    N, K = 264, 128 * kc
+    g = torch.Generator(device="cuda").manual_seed(kc)
+    torch.set_default_dtype(torch.bfloat16)
+    try:
+        a = torch.randn(M, K, generator=g, device="cuda", dtype=torch.float32).to(torch.float8_e4m3fn)
+        b = torch.randn(N, K, generator=g, device="cuda", dtype=torch.float32).to(torch.float8_e4m3fn)
+        # (NaN around the scales: a scale from beside them would show)
+        moved = []
+        for rows in (M, -(-N // 128)):
+            buf = torch.full((rows * kc + 8,), float("nan"), dtype=torch.float32, device="cuda")
+            moved.append(buf[offset:offset + rows * kc].view(rows, kc).copy_(torch.rand(rows, kc, generator=g, device="cuda", dtype=torch.float32) + 0.5))
+        out = []
+        for policy in (4, 6):
+            dsv3_b200.set_gemm_policy(policy, 0)
+            out.append(kernel.fp8_gemm(a, moved[0], b, moved[1]))
+        assert torch.equal(*out) and bool(out[0].isfinite().all())
+    finally:
+        dsv3_b200.set_gemm_policy(0, 0)
+        torch.set_default_dtype(torch.float32)
+        dsv3_b200.check_device_status()
