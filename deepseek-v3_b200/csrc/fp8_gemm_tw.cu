@@ -181,7 +181,7 @@ __device__ __forceinline__ Strip decode_strip(int pair, const TwOperands<kMats>&
 
 // kBlock: K chunks per scale load: 4 (K chunks a multiple of four, 16-byte aligned scales), 2 (of two, 8-byte), else 1, or kShifted: in the
 // aligned groups of four that rows lie in, wherever they begin
-constexpr int kShifted = 0, kShiftedFrom = 11;
+constexpr int kShifted = 0, kShiftedFrom = 19;
 template <int kBlock, int kMats>
 __global__ void __launch_bounds__(kNumThreads, 1)
 fp8_gemm_tw_kernel(const __grid_constant__ TwOperands<kMats> o, const TwParams p) {
@@ -446,7 +446,7 @@ fp8_gemm_tw_kernel(const __grid_constant__ TwOperands<kMats> o, const TwParams p
         // thread picks them out by its own row's offset, and the last one to three chunks come behind the groups of four.  A scalar load waits in every
         // chunk, which products in halves had made longer than what it was before them.  us with act_quant, whole slots and scalar loads / halves and scalar / so: M 2456, N 5456,
         // K 6272 102.9 / 104.6 / 97.7; M 4096, N 7168, K 7296 247.1 / 251.1 / 236.8; M 8192, N 5120, K 12416 631 / 630 / 551.  Shorter rows are over before it pays: with
-        // 3 to 9 chunks 1 to 5 % slower, with 11 to 17 1 % faster (ten shapes of each).  (Even numbers of chunks: 4 to 6 % slower than 8-byte loads.)
+        // 3 to 9 chunks 1 to 5 % slower, with 11, 13, 15 and 17 level, 1 to 2 % slower, 1 % faster and level, with 19 1 to 3 % faster.  (Even numbers of chunks: 4 to 6 % slower than 8-byte loads.)
         float ra[kBlock == kShifted ? 1 : kBlock], rb[kBlock == kShifted ? 4 : kBlock];
         float4 a_cur, a_next;      // kShifted: the groups that hold the next four chunks' a_s
         const float* const a_end = p.a_s + p.M * kc;
