@@ -957,13 +957,15 @@ static double half_estimate(int kc, int chunks, int splits, int64_t ctas) {
 }
 
 // Time of n wide tiles (256 x 256) on so many pairs, in the plan's microseconds.  The last round may be cut into strips.  Scales that do not
-// come four chunks at a time lengthen the chunks, with long rows of them more: 256 x 256 tiles against 256 x 128, us, M 2048, N 7168, 56, 57 and 58 chunks
-// 102 / 115, 117 / 116, 111 / 116; M 4096, N 7168, 16 and 17 58 / 77, 69 / 76; M 8000, N 5120, 96 and 97 420 / 657, 613 / 520; M 1585, N 3936, 89 96 / 77.
+// come four chunks at a time lengthen the chunks, with long rows of them more.  With act_quant, us, tiles of 256 x 256 / 256 x 128: chunks a multiple of
+// four, M 4172, N 7168, K 7168 210 / 243; of two, M 3475, N 6432, K 9856 219 / 242, two rounds and long rows, M 1336, N 4624, K 14080 138 / 115; odd, M 1709,
+// N 10384, K 5248 104 / 114, a round and a half, M 1418, N 4624, K 7040 69 / 59, strips behind one round, M 1937, N 2944, K 6016 50 / 46.5, long rows, M 5248,
+// N 2688, K 14464 286 / 251.
 static double wide_estimate(int64_t n, int64_t pairs, int kc) {
-    const double chunk = kc % 4 == 0 ? 0.38 : 0.38 * ((kc % 2 ? 1.12 : 1.05) + (kc > 64 ? 0.003 * (kc - 64) : 0.0));
+    const double more = kc % 4 == 0 ? 1.0 : (kc % 2 ? 1.16 : 1.10) + (kc > 64 ? 0.003 * (kc - 64) : 0.0);
     const int strip = tw_strip_width(n % pairs, pairs, kc);
-    if (strip) return 0.5 + static_cast<double>(n / pairs) * (kc * chunk + 0.9) + kc * (strip == 64 ? 0.27 : 0.37) + 1.5;
-    return 0.5 + static_cast<double>((n + pairs - 1) / pairs) * (kc * chunk + 0.9);
+    if (strip) return 0.5 + static_cast<double>(n / pairs) * (kc * 0.40 * more + 0.9) + kc * (strip == 64 ? 0.30 : 0.39) * more + 1.5;
+    return 0.5 + static_cast<double>((n + pairs - 1) / pairs) * (kc * 0.40 * more + 0.9);
 }
 
 // Pinned values (dsv3_set_gemm_policy) are honoured or refused (pl.error), never rewritten; the automatic
@@ -1036,19 +1038,21 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
                 // tile and hand-over, and 0.4 to 1.2 for the cluster launch.  (Chunk times in a full machine; a single round runs at
                 // higher clocks.  Chosen so, 277 shapes of 72 to 4000 tokens are within a few per cent of the best of the
                 // three; with K below 1536 excluded from the 256 x 128 tiles and no estimate for the single CTA, thirty
-                // were 4-39 % away.  The wide tiles' figures are those of products in halves: 198 shapes of 140 to 3000 tokens are 0.3 % from
-                // the best on average, with the figures from before, 0.41 and 1.3, 0.5 %: M 200, N 24576, K 1536 15.9 / 14.6 us, M 1500, N 4096,
-                // K 512 10.7 / 9.5, M 2048, N 3072, K 1536 18.5 / 17.5.)
+                // were 4-39 % away.  949 shapes of 129 to 8000 tokens for which the estimates of the pairs are within a quarter of one another: 0.24 %
+                // from the best of the three on average, 3 % of them by more than 3 %.  Estimates too low for wide tiles of odd chunk counts and in strips,
+                // and for a single CTA's later rounds (0.37 a chunk of a strip of 128, 0.38 of a tile, 1.12 and 1.05 times as much, 0.29): 0.72 %, and 10 %
+                // of them; M 1049, N 4720, K 5504 with act_quant 46.3 / 42.6 us, M 923, N 6464, K 2944 28.8 / 25.3.)
                 const int pairs = sms / 2;
                 const int64_t pp = (static_cast<int64_t>(pl.tiles_p) + 1) / 2;
                 const auto unsplit = [&](int64_t n, int64_t units, double chunk, double chunk1, double o) {
                     const int64_t rounds = (n + units - 1) / units;
                     return static_cast<double>(rounds) * (pl.kc * (rounds == 1 ? chunk1 : chunk) + o);
                 };
-                best = unsplit(tiles, sms, 0.29, 0.29, 1.0);
+                best = unsplit(tiles, sms, 0.305, 0.29, 1.0);
                 if (force_kernel == 0) {
                     const double full = pp * pl.tiles_q < pairs ? static_cast<double>(pp * pl.tiles_q) / pairs : 1.0;
-                    const double narrow = tm_pair_supported(M, N, K) ? 0.4 + 0.8 * full + unsplit(pp * pl.tiles_q, pairs, 0.265, 0.235, 0.8) : 1e30;
+                    const double pitch = pl.kc % 32 ? 1.0 : 1.1;       // (as in half_estimate())
+                    const double narrow = tm_pair_supported(M, N, K) ? pitch * (0.4 + 0.8 * full + unsplit(pp * pl.tiles_q, pairs, 0.265, 0.235, 0.8)) : 1e30;
                     double wide = 1e30;
                     if (tw_pair_supported(M, N, K)) wide = wide_estimate(pp * ((N + 255) / 256), pairs, pl.kc);
                     pl.wide = wide < best && wide <= narrow;

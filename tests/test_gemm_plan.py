@@ -53,3 +53,21 @@ def test_a_plan_beyond_the_scale_table_is_not_launched(bn, splits, chunks, fits)
     plan = Plan(0, True, False, False, splits > 1, bn, 1, 1, splits, chunks)
     rc = launch(None, None, None, None, bn, 128, 128 * chunks, None, None, 0, ctypes.byref(plan), None)
     assert rc != _lib.OK and (b"scale table" in _lib.lib.dsv3_last_error()) == (not fits)
+
+
+@pytest.mark.parametrize("M,N,K,wide", [
+    (1049, 4720, 5504, False),              # one round of 256 x 256 tiles and strips of 128, odd chunks
+    (722, 9088, 3968, False),
+    (923, 6464, 2944, False),               # a round and 40 % of one
+    (684, 8016, 2688, False),
+    (1845, 4736, 4096, True),               # rows 4 KB apart
+    (4096, 7168, 16384, True),              # many rounds
+    (2048, 7168, 7296, True),
+])
+def test_pair_tiles(M, N, K, wide):
+    """256 x 256 or 256 x 128, where 148 SMs decide it (both sum in the same order: no result tells them apart)."""
+    from dsv3_b200 import _lib
+    tc_plan = getattr(_lib.lib, "_ZN4dsv37tc_planElllii")
+    tc_plan.argtypes, tc_plan.restype = [ctypes.c_int64] * 3 + [ctypes.c_int] * 2, Plan
+    p = tc_plan(M, N, K, 0, 0)
+    assert p.pair and p.wide == wide and p.splits == 1
