@@ -970,7 +970,7 @@ static double wide_estimate(int64_t n, int64_t pairs, int kc) {
 
 // Pinned values (dsv3_set_gemm_policy) are honoured or refused (pl.error), never rewritten; the automatic
 // plan adapts freely.  dev, sms: the device (-1: none) and the SMs there are on it, or the budget for them.
-// estimate: microseconds (automatic plans of token-major tiles; otherwise 0)
+// estimate: microseconds of an automatic plan of token-major tiles; of others (pl.swap, or anything pinned) it says nothing
 static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_split, int dev, int sms, double& estimate) {
     TcPlan pl;
     pl.error = DSV3_OK;
@@ -1109,8 +1109,9 @@ static TcPlan work_out_plan(int64_t M, int64_t N, int64_t K, int force_kernel, i
         }
         // Token-major tiles of 64 weight rows, which never lie in two weight blocks, where they fit one round: a chunk is 24 KB of loads for a CTA
         // instead of 32, a part of a tile half as much to exchange, and there are more ways to come near 148 CTAs.  half_estimate() is
-        // fitted to 412 launches of 172 shapes of 70 to 2200 tokens (rms 5 %, weights from HBM, a replayed graph); against what the plan chose
-        // before, 59 of the shapes take them, two of these 2 % slower than before.  us, before / so: M 1003, N 576, K 7168 12.3 / 10.0; M 256, N 576, K 7168
+        // fitted to 412 launches of 172 shapes of 70 to 2200 tokens (rms 5 %, weights from HBM, a replayed graph).  Of 520 drawn shapes of 65 to
+        // 2200 tokens 176 take them, at 1.13 of the speed of the best of the other kinds by the plan, 1.11 behind act_quant; one is 6 % slower behind it (M 87,
+        // N 2240, K 3456 8.4 / 8.9); of 130 that would take narrow token tiles, at 1.10, one 3 %.  us, without them / so: M 1003, N 576, K 7168 12.3 / 10.0; M 256, N 576, K 7168
         // 9.3 / 7.4; M 1000, N 256, K 7168 10.2 / 8.2; M 200, N 2304, K 7168 12.4 / 10.1; M 529, N 1584, K 4224 11.5 / 9.3; M 70, N 7168, K 2304 8.6 / 7.1;
         // M 650, N 800, K 896 5.6 / 4.7.  Clusters of more than two that leave few SMs over wait for room, odd ones, which leave an SM of a pair over, sooner
         // (behind act_quant, M 1328, N 256, K 7168, 44 of three, 15.9 / 18.0; M 1280, 40 of three, 15.7 / 13.4; M 301, N 688, K 7936, 33 of four, 14.0 / 11.2).
@@ -1223,8 +1224,10 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
 // 61.4 / 50.2; M 2201, N 2048, K 7168 75.1 / 69.1; M 2201, N 3072, K 5120 93.9 / 68.8; M 500, N 12288, K 5120 91.3 / 66.6; M 8192, N 2048, K 7168
 // 266 / 244.  The margin: with many rounds the two are level, or the launch boundary, which brings the pairs back into step,
 // is worth 1 %: M 2201, N 18432, K 7168 541 / 551, M 6000, N 12288, K 5120 697 / 704, M 8192, N 18432, K 7168 1917 / 1923.
-// Not where the common last round would be cut into strips: it is faster there, too (M 1300, N 2048, K 7168 60.2 / 53.5, M 1545, N 2816,
-// K 2048 33.1 / 27.1), but such MLPs are held to their number of launches (tests/test_gpu_mlp_launches.py).
+// Not where the common last round would be half full or less (with 24 chunks, or up to a quarter, it would be cut into strips).  The line keeps
+// the launches that tests/test_gpu_mlp_launches.py counts, and leaves time there: of 99 such shapes of 11 MLPs two launches are ahead at a dozen, by up
+// to 1 %, with many rounds of long rows (M 8191, N 18432, K 7168 1910 / 1917), one launch by up to 40 % at the others: strips, M 2335, N 2304, K 7168
+// 111.9 / 87.3, M 1786, N 2816, K 2048 33.8 / 26.3; whole, M 2030, N 2816, K 2048 36.4 / 28.5, M 6910, N 1408, K 2048 59.3 / 49.7.
 bool tw_two_pay(int64_t M, int64_t N, int64_t K) {
     if (!tw_pair_supported(M, N, K)) return false;
     double estimate = 0.0;

@@ -1120,7 +1120,7 @@ __device__ __forceinline__ void rows_tiles(const CUtensorMap* tmap_w0, const CUt
                 float m = 0.0f;
                 // Rolled loops over a register file that turns by one group per trip: unrolled, this epilogue was longer
                 // than the instruction cache holds and cost 8000-14000 cycles per tile.  (Rows beyond the tile's hold
-                // products of weights with weights: not worth silu's exact path.)
+                // products of weights with weights, which nobody reads.)
                 if (row < s.ntok) {
 #pragma unroll 1
                     for (int c = 0; c < 8; ++c) {
