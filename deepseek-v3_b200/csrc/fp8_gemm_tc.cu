@@ -1223,7 +1223,8 @@ TcPlan tc_plan(int64_t M, int64_t N, int64_t K, int force_kernel, int force_spli
 // take tiles that are not cut over K.  B200, us with act_quant, two launches / one: M 2580, N 2304, K 7168 120.9 / 89.5; M 3942, N 2816, K 2048
 // 61.4 / 50.2; M 2201, N 2048, K 7168 75.1 / 69.1; M 2201, N 3072, K 5120 93.9 / 68.8; M 500, N 12288, K 5120 91.3 / 66.6; M 8192, N 2048, K 7168
 // 266 / 244.  The margin: with many rounds the two are level, or the launch boundary, which brings the pairs back into step,
-// is worth 1 %: M 2201, N 18432, K 7168 541 / 551, M 6000, N 12288, K 5120 697 / 704, M 8192, N 18432, K 7168 1917 / 1923.
+// is worth 1 %: M 2201, N 18432, K 7168 541 / 551, M 6000, N 12288, K 5120 697 / 704, M 8192, N 18432, K 7168 1917 / 1923.  (Odd numbers of chunks, half
+// of it: M 5121, N 2560, K 4992 152 / 148, M 5377, N 4096, K 2944 152 / 148.)
 // Not where the common last round would be half full or less (with 24 chunks, or up to a quarter, it would be cut into strips).  The line keeps
 // the launches that tests/test_gpu_mlp_launches.py counts, and leaves time there: of 99 such shapes of 11 MLPs two launches are ahead at a dozen, by up
 // to 1 %, with many rounds of long rows (M 8191, N 18432, K 7168 1910 / 1917), one launch by up to 40 % at the others: strips, M 2335, N 2304, K 7168
@@ -1237,7 +1238,7 @@ bool tw_two_pay(int64_t M, int64_t N, int64_t K) {
     if (n % pairs != 0 && 2 * (n % pairs) <= pairs) return false;
     double two = wide_estimate(n, pairs, one.kc);
     if (const double floor = (2.0 * static_cast<double>(N) * K + static_cast<double>(M) * K) / 6.0e6; two < floor) two = floor;
-    return two + 2.4 < 0.975 * 2.0 * estimate;
+    return two + 2.4 < (one.kc % 2 ? 0.98 : 0.975) * 2.0 * estimate;
 }
 
 size_t tc_workspace_bytes(const TcPlan& pl, int64_t M, int64_t N) {
