@@ -118,3 +118,25 @@ def test_memory_of_an_mlp_of_four_launches(dim, inter, M):
     with torch.inference_mode():                  # a tensor without a modification counter: its quantisation is not kept
         x = x.clone()
         assert peak(lambda: host.mlp(x, w1, w3, w2, None, None, False)) <= peak(one_by_one)
+
+
+@pytest.mark.parametrize("which", [0, 1])
+def test_weights_off_16_bytes_take_the_separate_launches(which):
+    import kernel
+    from dsv3_b200 import _lib, swiglu_quant
+    from dsv3_b200._lib import host
+    dim, inter, M = 2048, 1408, 2580
+    assert _lib.lib.dsv3_fp8_gemm_two_pays(_i64(M), _i64(inter), _i64(dim))
+    mlp, model = _host(dim, inter)
+    lin = (mlp.w1, mlp.w3)[which]
+    scale = lin.weight.scale
+    w = torch.empty(inter * dim + 1, dtype=torch.uint8, device="cuda")[1:].view(lin.weight.dtype).view(inter, dim)
+    w.view(torch.uint8).copy_(lin.weight.view(torch.uint8))
+    lin.weight = torch.nn.Parameter(w, requires_grad=False)
+    lin.weight.scale = scale
+    assert lin.weight.data_ptr() % 16
+    x = _rows(M, dim)
+    assert host.mlp(x, mlp.w1.weight, mlp.w3.weight, mlp.w2.weight, None, None, False) is None
+    q = kernel.act_quant(x)
+    h = swiglu_quant(*(kernel.fp8_gemm(*q, lin.weight, lin.weight.scale) for lin in (mlp.w1, mlp.w3)))
+    assert torch.equal(mlp(x), kernel.fp8_gemm(*h, mlp.w2.weight, mlp.w2.weight.scale))
