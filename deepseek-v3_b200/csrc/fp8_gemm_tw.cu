@@ -9,7 +9,7 @@
 // of 256 promotion threads), TMEM holds only two chunk products, and the read-back buffer shrinks to 64 registers per thread.
 //
 // Why each product in two halves (N128).  A slot handed back as a whole was away for 1100 cycles besides its own 512 (commit, wake-up,
-// two read-backs with the FMAs between them, arrivals from both CTAs, issue), so that two slots gave a product every 810 cycles.
+// two read-backs with the FMAs between them, arrivals from both CTAs, issue), so that two slots gave a product every 774 to 810 cycles.
 // As halves, one for either warp group, the next product's left half is computed while the right one is still being read: 675.  The tokens
 // are read from shared memory twice for that, 96 instead of 64 bytes per clock.  In a loop of launches the clock falls with the
 // work it does (1 kW): us, whole slots / halves, act_quant included, M 500, N 7168, K 7168 35.6 / 34.2; M 867, N 18432, K 7168 126.8 / 123.4; M 4096, N 7168,
