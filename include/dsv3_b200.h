@@ -275,7 +275,8 @@ int dsv3_swiglu_gemm_rows(const void* table1, const void* table3, int n_groups, 
 int dsv3_fp8_gemm_rows(const void* table, int n_groups, const void* a, const float* a_s_t, const int32_t* seg, int64_t rows_total,
                        int64_t rows_hint, int64_t N, int64_t K, void* c, const dsv3_side_gemm_t* side, void* workspace,
                        size_t workspace_bytes, dsv3_stream_t stream);
-/* Both, one after the other: w1 and w3 [inter, dim] into hq and hs_t, w2 [dim, inter] of those into o; up and down: their ordinary weights. */
+/* Both, one after the other: w1 and w3 [inter, dim] into hq and hs_t, w2 [dim, inter] of those into o; up and down: their ordinary weights. Nothing is
+ * launched where the arguments of either are refused. */
 int dsv3_expert_gemms(const void* table1, const void* table3, const void* table2, int n_groups, const void* a, const float* a_s_t,
                       const int32_t* seg, int64_t rows_total, int64_t rows_hint, int64_t inter, int64_t dim, int scale_fmt, void* hq,
                       float* hs_t, void* o, const dsv3_side_gemm_t* up, const dsv3_side_gemm_t* down, void* workspace,
